@@ -235,3 +235,103 @@ def tolerance(case):
         return {"rel": 1.5e-2, "max": 0.2, "differ": 1e-3}
     # fp16 operands and result, fp32 sums: half an fp16 step per operand and on the way out
     return {"rel": 1.5e-3, "max": 2e-2}
+
+
+def _expand(q, s, group, shape):
+    """The packed matrix in 64 bits: a byte row holds two groups, the even one in the high nibbles."""
+    q = q.reshape(-1, group)
+    codes = torch.cat(((q >> 4).double(), ((q << 4) >> 4).double()), dim=1).view(-1, group)
+    return (codes * s.reshape(-1, 1).double()).view(shape)
+
+
+def _attend(q, k, v, mask=None):
+    """softmax(q k^T / sqrt(d)) v over [..., rows, d] operands in 64 bits; `mask` is true where a key counts."""
+    sc = q @ k.transpose(-1, -2) / math.sqrt(HEAD_DIM)
+    if mask is not None:
+        sc = sc.masked_fill(~mask, -math.inf)
+    return torch.softmax(sc, dim=-1) @ v
+
+
+def _exact_model(case, seed):
+    """Logits of the prompt pass, or of the decode step after it, layer by layer in 64 bits."""
+    state = prepare(case, seed)
+    m, eps = state["model"], 1e-5
+    lin = lambda x, l: x @ _expand(l.w, l.s, 64, (int(l.shape[1]), int(l.shape[0])))
+    norm = lambda x, w: x / (x.square().mean(-1, keepdim=True) + eps).sqrt() * w.double()
+    freq = m.params.rope_theta ** (-torch.arange(0, HEAD_DIM, 2, device=DEV).double() / HEAD_DIM)
+
+    def rope(x, pos):                                  # value i turns with value i + 64, [rows, heads, 128]
+        ang = (pos.double()[:, None] * freq)[:, None]
+        lo, hi = x.chunk(2, dim=-1)
+        return torch.cat((lo * ang.cos() - hi * ang.sin(), hi * ang.cos() + lo * ang.sin()), dim=-1)
+
+    split = lambda x: x.view(x.shape[0], HEADS, HEAD_DIM)
+    decode = case["kind"] == "decode"
+    if decode:
+        gen = torch.Generator(device=DEV).manual_seed(int(seed))
+        torch.randint(0, 1 << 30, (1,), generator=gen, device=DEV)
+        prompt = torch.randint(0, VOCAB, (1, case["prompt"]), generator=gen, device=DEV).view(-1)
+    else:
+        prompt = state["tokens"].view(-1)
+    S = prompt.numel()
+    at = torch.arange(S, device=DEV)
+    causal = at[:, None] >= at[None, :]
+    h = m.tok_embeddings.weight[prompt].double()
+    if decode:
+        w, t = case["width"], case["suffix"]
+        d = m.tok_embeddings.weight[state["tokens"].view(-1)].double()
+        here = torch.full((w,), state["pos"], device=DEV)
+    heads = lambda x: x.transpose(0, 1)
+    for layer in m.layers:
+        att, ff = layer.attention, layer.feed_forward
+        feed = lambda x: lin(torch.nn.functional.silu(lin(x, ff.w1)) * lin(x, ff.w3), ff.w2)
+        x = norm(h, layer.attention_norm.weight)
+        k, v = rope(split(lin(x, att.wk)), at), split(lin(x, att.wv))
+        o = _attend(heads(rope(split(lin(x, att.wq)), at)), heads(k), heads(v), causal)
+        h = h + lin(heads(o).reshape(S, -1), att.wo)
+        h = h + feed(norm(h, layer.ffn_norm.weight))
+        if decode:
+            x = norm(d, layer.attention_norm.weight)
+            dq, dk, dv = rope(split(lin(x, att.wq)), here), rope(split(lin(x, att.wk)), here), split(lin(x, att.wv))
+            out = []
+            for b in range(w):
+                own = [torch.cat((p, _expand(c[b, :t], s[b, :t], 64, (t, HEADS, HEAD_DIM)), n[b:b + 1])) for p, c, s, n in
+                       ((k, att.cache_k, att.cache_k_s, dk), (v, att.cache_v, att.cache_v_s, dv))]
+                out.append(_attend(dq[b][:, None], heads(own[0]), heads(own[1])).reshape(1, -1))
+            d = d + lin(torch.cat(out), att.wo)
+            d = d + feed(norm(d, layer.ffn_norm.weight))
+    r = norm(d if decode else h, m.norm.weight) @ m.output.weight.double().t()
+    return r.view(w, 1, -1) if decode else r.view(1, S, -1)
+
+
+def exact(case, seed):
+    kind = case["kind"]
+    if kind == "pack":
+        return None                    # codes, and one rounding each way: compared bit for bit
+    if kind in ("decode", "prompt"):
+        logits = _exact_model(case, seed)
+        if kind == "prompt":
+            return {"logits": logits, "k": None, "v": None}
+        return {"logits": logits, "k": None, "k_scale": None, "v": None, "v_scale": None}
+    st = prepare(case, seed)
+    if kind == "matmul":
+        return st["x"].double() @ _expand(st["w"], st["s"], 64, st["shape"])
+    if kind == "linear":
+        return st["x"].double() @ _expand(st["w"], st["s"], st["group"], st["shape"]).t()
+    h, hkv = case["heads"], case["kv_heads"]
+    rep = h // hkv
+    out = []
+    for b in range(case["width"]):
+        if kind == "tree_attn":
+            n, page = int(st["lens"][b]), st["page"]
+            at = torch.arange(n, device=DEV)
+            slot = st["table"][b].long()[at // page] * page + at % page
+            k, v = (torch.cat((p.double().transpose(0, 1), s[:, slot].double()), dim=1)
+                    for p, s in ((st["pk"], st["k"]), (st["pv"], st["v"])))
+        elif st["paged"]:
+            k, v = (st[x][:, st["table"][b].long()].double() for x in ("k", "v"))
+        else:
+            k, v = st["k"][b].double(), st["v"][b].double()
+        q = st["q"][b].double()[:, None]
+        out.append(_attend(q, k.repeat_interleave(rep, 0), v.repeat_interleave(rep, 0)).view(h, HEAD_DIM))
+    return torch.stack(out)
