@@ -73,6 +73,27 @@ def test_quantize_random_vs_oracle(K, G):
     assert_bits_equal(host(d), O.dequantize_q40(qo, so, G, w.shape))
 
 
+@pytest.mark.parametrize("pairs", [1, 3, 63, 65, 257])
+@pytest.mark.parametrize("G", [64, 32])
+def test_quantize_and_back_ragged_piece_counts(K, pairs, G):
+    """Counts around a block's pieces, every magnitude of fp16, and groups with zeros, infinities and subnormals:
+    bit for bit, as the format is defined."""
+    rng = np.random.default_rng(pairs * G)
+    w = (rng.standard_normal((2 * pairs, G)) * 2.0 ** rng.integers(-24, 13, (2 * pairs, 1))).astype(np.float16)
+    w[0] = 0
+    w[1, ::3] = 0
+    if pairs > 1:
+        w[2] = np.float16(2 ** -24) * rng.integers(-40, 41, G)
+        w[3, 5] = np.inf
+    q, s = K.quantize_q40(dev(w), G)
+    qo, so = O.quantize_q40(w, G)
+    assert_bits_equal(host(q), qo)
+    assert_bits_equal(host(s), so)
+    fin = np.isfinite(so.astype(np.float32)).ravel()        # an infinite scale dequantises to NaN, whatever its bits
+    back = host(K.dequantize_q40(q, s, G, (2 * pairs, G)))
+    assert_bits_equal(back[fin], O.dequantize_q40(qo, so, G, (2 * pairs, G))[fin])
+
+
 def test_quantize_negative_values_round_like_torch(K):
     """The reference's Triton quantiser truncates toward zero; ours must round half-even."""
     w = np.tile(np.array([-7, -2.5, -1.5, -0.5, 0.5, 1.5, 2.5, 7], dtype=np.float16), 16).reshape(1, 128)
