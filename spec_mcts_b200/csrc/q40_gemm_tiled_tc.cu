@@ -134,6 +134,27 @@ __device__ __forceinline__ uint32_t deq_pair(uint32_t a72, __half2 scale) {
   return h2_as_u32(__hmul2(__hsub2(u32_as_h2(a72), u32_as_h2(0x54805480u)), scale));
 }
 
+// One 16-row step of a lane's two 16-row tiles: the tile words w0, w1 and the scales of k = 4t .. 4t + 3 to the
+// registers of columns 8 st + 2t, + 1 of st_16x256b_x4
+__device__ __forceinline__ void dequant_step(const unsigned char* w, const unsigned char* sc, uint32_t (&r)[2][16], int st) {
+  const uint2 wv = *reinterpret_cast<const uint2*>(w);
+  const uint2 sv = *reinterpret_cast<const uint2*>(sc);
+  const __half2 s01 = u32_as_h2(sv.x), s23 = u32_as_h2(sv.y);     // scales of k = 4t, 4t+1 and 4t+2, 4t+3
+  const uint32_t wds[2] = {wv.x, wv.y};
+#pragma unroll
+  for (int j2 = 0; j2 < 2; ++j2) {
+    const uint32_t v = wds[j2];
+    const uint32_t a0 = lop3_and_xor(v, 0x00F000F0u, 0x54805480u);        // row g,     k + 0, 1
+    const uint32_t a1 = lop3_and_xor(v << 4, 0x00F000F0u, 0x54805480u);   // row g + 8, k + 0, 1
+    const uint32_t a2 = lop3_and_xor(v >> 8, 0x00F000F0u, 0x54805480u);   // row g,     k + 2, 3
+    const uint32_t a3 = lop3_and_xor(v >> 4, 0x00F000F0u, 0x54805480u);   // row g + 8, k + 2, 3
+    r[j2][4 * st + 0] = deq_pair(a0, s01);      // row g,     column 8 st + 2t
+    r[j2][4 * st + 1] = deq_pair(a2, s23);      // row g,     column 8 st + 2t + 1
+    r[j2][4 * st + 2] = deq_pair(a1, s01);      // row g + 8, column 8 st + 2t
+    r[j2][4 * st + 3] = deq_pair(a3, s23);      // row g + 8, column 8 st + 2t + 1
+  }
+}
+
 // Tensor memory (all 512 columns of the SM): accumulators of the two 128-feature halves at columns
 // 0 and 128, A buffer ab of half hh at column 256 + 64 ab + 32 hh (64 k as 32 columns of fp16 pairs).
 constexpr int ACC_COLS = 128;
@@ -339,24 +360,8 @@ gemm_tiled_tc_kernel(const Params p, const __grid_constant__ CUtensorMap amap) {
       const size_t so = (size_t)s * stage_bytes;
       uint32_t r[2][16];
 #pragma unroll
-      for (int st = 0; st < 4; ++st) {
-        const uint2 w = *reinterpret_cast<const uint2*>(lane_w + so + st * STEP_BYTES);
-        const uint2 sc = *reinterpret_cast<const uint2*>(lane_s + so + st * STEP_BYTES);
-        const __half2 s01 = u32_as_h2(sc.x), s23 = u32_as_h2(sc.y);     // scales of k = 4t, 4t+1 and 4t+2, 4t+3
-        const uint32_t wds[2] = {w.x, w.y};
-#pragma unroll
-        for (int j2 = 0; j2 < 2; ++j2) {
-          const uint32_t v = wds[j2];
-          const uint32_t a0 = lop3_and_xor(v, 0x00F000F0u, 0x54805480u);        // row g,     k + 0, 1
-          const uint32_t a1 = lop3_and_xor(v << 4, 0x00F000F0u, 0x54805480u);   // row g + 8, k + 0, 1
-          const uint32_t a2 = lop3_and_xor(v >> 8, 0x00F000F0u, 0x54805480u);   // row g,     k + 2, 3
-          const uint32_t a3 = lop3_and_xor(v >> 4, 0x00F000F0u, 0x54805480u);   // row g + 8, k + 2, 3
-          r[j2][4 * st + 0] = deq_pair(a0, s01);      // row g,     column 8 st + 2t
-          r[j2][4 * st + 1] = deq_pair(a2, s23);      // row g,     column 8 st + 2t + 1
-          r[j2][4 * st + 2] = deq_pair(a1, s01);      // row g + 8, column 8 st + 2t
-          r[j2][4 * st + 3] = deq_pair(a3, s23);      // row g + 8, column 8 st + 2t + 1
-        }
-      }
+      for (int st = 0; st < 4; ++st)
+        dequant_step(lane_w + so + st * STEP_BYTES, lane_s + so + st * STEP_BYTES, r, st);
       const uint32_t ta = tmem + ((uint32_t)(32 * quad) << 16) + A_COL0 + ab * 64 + hh * 32;
       TTC_ROLE(2, i, 3);
       st_16x256b_x4(ta, r[0]);
@@ -442,6 +447,215 @@ gemm_tiled_tc_kernel(const Params p, const __grid_constant__ CUtensorMap amap) {
   Q40_TRACE_FLUSH(p.trace, 310);
 }
 
+// ---------------------------------------------------------------------------------------------------------
+// More than 128 rows (prompt pass, wide batches): 128 features x up to 256 batch rows per CTA.
+//
+// Same operands as above, other proportions.  A tcgen05.mma has a fixed cost of ~78 cycles whatever its width
+// (see gemm_tiled_tc_kernel), so the rows, which are the MMA's N, go up to 256, and one accumulator of 128
+// features takes half of tensor memory; the other half holds NA = 8 A buffers.  The activations of a k block
+// (32 KB at 256 rows) are read once per 128 features.  Sixteen dequantiser warps are four sets of four (one
+// warp per tensor-memory quadrant) that take the k blocks in turn; one thread issues all MMAs, in k order, so a
+// result depends on nothing but the operands and the k split.  Rows are cut into equal chunks of at most 256
+// inside ONE launch (grid z); a tile that is not split along k goes from tensor memory to the output
+// directly, otherwise the ranks of a cluster add their fp32 tiles in rank order.
+// ---------------------------------------------------------------------------------------------------------
+namespace wide {
+
+constexpr int FEATS = 128;                      // features per CTA: half a span of the tiled format
+constexpr int MAX_ROWS = 256;
+constexpr int NA = 8;                           // A buffers: 32 columns of tensor memory each
+constexpr int DSETS = 4;                        // dequantiser sets of four warps
+constexpr int DQ_WARP0 = 4;                     // warp 0: copies, warp 1: MMA issue, warps 4..19: dequantise
+constexpr int THREADS = (DQ_WARP0 + 4 * DSETS) * 32;
+constexpr int HSTEP = 1024 + 64;                // half a step: two 64-column groups and their scales
+constexpr int RAW_BYTES = 4 * HSTEP;
+constexpr int RAW_PAD = 5120;                   // next multiple of 1024 (the B tile wants that alignment)
+constexpr int A_COL0 = MAX_ROWS;
+
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_tiled_wide_kernel(const Params p, const __grid_constant__ CUtensorMap amap) {
+  extern __shared__ unsigned char smem_raw[];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int pi = 0, span = blockIdx.x >> 1;
+  const int half = blockIdx.x & 1;
+  while (pi < p.nprob - 1 && span >= p.spans[pi]) { span -= p.spans[pi]; ++pi; }
+  const int kb = blockIdx.y * p.rows_per_split;
+  const int ke = min(p.K, kb + p.rows_per_split);
+  const int nblk = (ke - kb) / BK;                           // host guarantees >= 1 and exact
+  const int m0 = blockIdx.z * p.Mpad;                        // first batch row of this chunk
+  const int rows = min(p.Mpad, p.M - m0);
+  const int S = p.stages;
+  const uint32_t b_bytes = (uint32_t)p.Mpad * 128u;          // B tile: Mpad rows x 64 k x 2 B
+  const uint32_t stage_bytes = RAW_PAD + b_bytes;
+
+  const uint32_t raw0 = smem_u32(smem_raw);
+  const uint32_t ring = (raw0 + 1023u) & ~1023u;
+  unsigned char* gbase = smem_raw + (ring - raw0);
+  const size_t ring_bytes = max((size_t)S * stage_bytes, ((size_t)p.Mpad * FEATS + 64) * 4);
+  // full[s]: the stage's copies have landed; afull / mdone [i % NA]: the A operand of block i is written / the MMAs
+  // of block i are complete (its stage and its A buffer may be refilled; S <= NA, so neither waiter can
+  // miss a phase); done: all MMAs complete
+  const uint32_t bar_full = ring + (uint32_t)ring_bytes, bar_afull = bar_full + 8 * MAX_STAGES;
+  const uint32_t bar_mdone = bar_afull + 8 * NA, bar_done = bar_mdone + 8 * NA;
+  unsigned char* tail = gbase + ring_bytes + 8 * MAX_STAGES + 16 * NA + 16;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail);
+  volatile int* s_failed = reinterpret_cast<volatile int*>(tail + 8);
+
+  if (tid == 0) {
+    *s_failed = 0;
+    for (int s = 0; s < MAX_STAGES; ++s) mbar_init(bar_full + 8 * s, 1);
+    for (int s = 0; s < NA; ++s) { mbar_init(bar_afull + 8 * s, 4); mbar_init(bar_mdone + 8 * s, 1); }
+    mbar_init(bar_done, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  asm volatile("griddepcontrol.launch_dependents;");
+
+  bool failed = false;
+  if (warp == 0) {
+    if (lane == 0) {
+      const int ksteps = p.K / 16;
+      const uint8_t* src = p.bw[pi] + ((int64_t)span * ksteps + kb / 16) * STEP_BYTES;
+      auto weights = [&](int i, int s) {
+#pragma unroll
+        for (int st = 0; st < 4; ++st) {
+          const uint8_t* step = src + (int64_t)(4 * i + st) * STEP_BYTES;
+          const uint32_t dst = ring + s * stage_bytes + st * HSTEP;
+          bulk_g2s(dst, step + half * 1024, 1024, bar_full + 8 * s);
+          bulk_g2s(dst + 1024, step + 2048 + half * 64, 64, bar_full + 8 * s);
+        }
+      };
+      // weights do not depend on the previous launch, the activations do
+      const int first = min(S, nblk);
+      for (int i = 0; i < first; ++i) {
+        mbar_expect_tx(bar_full + 8 * i, RAW_BYTES + b_bytes);
+        weights(i, i);
+      }
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      for (int i = 0; i < first; ++i)
+        tma_2d(ring + i * stage_bytes + RAW_PAD, &amap, kb + i * BK, m0, bar_full + 8 * i);
+      for (int i = first; i < nblk; ++i) {
+        const int s = i % S, j = i - S;                      // block j was the stage's last user
+        if (!mbar_wait(bar_mdone + 8 * (j % NA), (uint32_t)((j / NA) & 1))) { failed = true; break; }
+        mbar_expect_tx(bar_full + 8 * s, RAW_BYTES + b_bytes);
+        tma_2d(ring + s * stage_bytes + RAW_PAD, &amap, kb + i * BK, m0, bar_full + 8 * s);
+        weights(i, s);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    const uint32_t idesc = (1u << 4) | ((uint32_t)(p.Mpad >> 3) << 17) | ((uint32_t)(FEATS >> 4) << 24);
+    for (int i = 0; i < nblk; ++i) {
+      const int ab = i % NA;
+      // the dequantisers' arrival also covers the stage's copies, which they waited for
+      if (!mbar_wait(bar_afull + 8 * ab, (uint32_t)((i / NA) & 1))) { failed = true; break; }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (lane == 0) {
+        const uint64_t bd0 = kmajor_desc(ring + (i % S) * stage_bytes + RAW_PAD);
+#pragma unroll
+        for (int ks = 0; ks < BK / 16; ++ks)
+          mma_ts(tmem, tmem + A_COL0 + ab * 32 + ks * 8, bd0 + (uint64_t)((ks * 32) >> 4), idesc,
+                 (i > 0 || ks > 0) ? 1u : 0u);
+        commit(bar_mdone + 8 * ab);
+      }
+      __syncwarp();
+    }
+    if (lane == 0 && !failed) commit(bar_done);
+    __syncwarp();
+  } else if (warp >= DQ_WARP0) {
+    // warp = (set, quadrant): 32 feature rows = two 16-row tiles of one 64-column group, see above
+    const int quad = warp & 3, dset = (warp - DQ_WARP0) >> 2;
+    const int q = quad >> 1, t = lane & 3;
+    const unsigned char* lane_w = gbase + (q * 32 + lane) * 16 + (quad & 1) * 8;
+    const unsigned char* lane_s = gbase + 1024 + q * 32 + t * 8;
+    for (int i = dset; i < nblk; i += DSETS) {
+      const int s = i % S, ab = i % NA;
+      if (!mbar_wait(bar_full + 8 * s, (uint32_t)((i / S) & 1))) { failed = true; break; }
+      if (i >= NA && !mbar_wait(bar_mdone + 8 * ab, (uint32_t)((i / NA - 1) & 1))) { failed = true; break; }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const size_t so = (size_t)s * stage_bytes;
+      uint32_t r[2][16];
+#pragma unroll
+      for (int st = 0; st < 4; ++st) dequant_step(lane_w + so + st * HSTEP, lane_s + so + st * HSTEP, r, st);
+      const uint32_t ta = tmem + ((uint32_t)(32 * quad) << 16) + A_COL0 + ab * 32;
+      st_16x256b_x4(ta, r[0]);
+      st_16x256b_x4(ta + (16u << 16), r[1]);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_afull + 8 * ab);
+    }
+  }
+  if (failed) *s_failed = 1;
+  if (!failed && !mbar_wait(bar_done, 0)) *s_failed = 1;
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  __syncthreads();
+  failed = *s_failed != 0;
+  if (failed && tid == 0) atomicExch(p.err, 1);
+
+  const int nranks = (int)cluster.num_blocks();
+  const int n0 = span * SPAN + half * FEATS;
+  __half* c = p.c[pi] + (int64_t)m0 * p.ldc[pi] + n0;
+  float* tile_f = reinterpret_cast<float*>(gbase);
+  if (!failed && warp >= DQ_WARP0) {
+    const int quad = warp & 3, dset = (warp - DQ_WARP0) >> 2;
+    const int feat = 32 * quad + lane;                // MMA row = feature
+    for (int ch = dset; ch < p.Mpad / 16; ch += DSETS) {
+      uint32_t r[16];
+      ld16(tmem + ((uint32_t)(32 * quad) << 16) + ch * 16, r);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      if (nranks > 1) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) tile_f[(ch * 16 + j) * FEATS + feat] = __uint_as_float(r[j]);
+      } else {
+        // a warp's store is 64 contiguous bytes of one row: whole sectors, no staging
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (ch * 16 + j < rows) c[(int64_t)(ch * 16 + j) * p.ldc[pi] + feat] = __float2half_rn(__uint_as_float(r[j]));
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  cluster.sync();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512));
+  }
+  if (nranks == 1) return;
+  // split-K: rank r finishes the r-th slice of the (row, feature) pairs, adding the ranks' tiles in rank order
+  const int rank = (int)cluster.block_rank();
+  const int total = rows * FEATS;
+  const int per = ((total / 4 + nranks - 1) / nranks) * 4;
+  const int e0 = rank * per, e1 = min(total, e0 + per);
+  if (!failed) {
+    for (int e = e0 + tid * 4; e < e1; e += THREADS * 4) {
+      float4 tt[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+        tt[r] = (r < nranks) ? *reinterpret_cast<const float4*>(cluster.map_shared_rank(tile_f + e, r))
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int r = 0; r < 8; ++r) { v.x += tt[r].x; v.y += tt[r].y; v.z += tt[r].z; v.w += tt[r].w; }
+      __half2* dst = reinterpret_cast<__half2*>(c + (int64_t)(e / FEATS) * p.ldc[pi] + e % FEATS);
+      dst[0] = __floats2half2_rn(v.x, v.y);
+      dst[1] = __floats2half2_rn(v.z, v.w);
+    }
+  }
+  cluster.sync();       // every rank has read the tiles: shared memory may go away
+}
+
+}  // namespace wide
+
 }  // namespace ttc
 }  // namespace q40
 
@@ -466,17 +680,16 @@ static EncodeTiledFn ttc_encode_fn() {
 }
 
 // How many clusters of (1, nsplit) CTAs with this much dynamic shared memory run at once (cached per
-// device, split and padded row class; 0 when the runtime cannot tell).
-static int ttc_max_clusters(TtcKernel kern, int mpad, int nsplit, size_t smem) {
-  static int cache_all[16][9][17] = {};
+// device, kernel, split and padded row class; 0 when the runtime cannot tell).
+static int ttc_max_clusters(TtcKernel kern, bool wide, int threads, int mpad, int nsplit, size_t smem) {
+  static int cache_all[16][2][9][17] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) dev = 0;
-  int (*cache)[17] = cache_all[dev];
-  const int cls = mpad / 16;
-  if (cache[nsplit][cls]) return cache[nsplit][cls] - 1;
+  int* cached = &cache_all[dev][wide][nsplit][mpad / 16];
+  if (*cached) return *cached - 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(1024, nsplit, 1);
-  cfg.blockDim = dim3(q40::ttc::THREADS, 1, 1);
+  cfg.blockDim = dim3(threads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -490,7 +703,7 @@ static int ttc_max_clusters(TtcKernel kern, int mpad, int nsplit, size_t smem) {
     (void)cudaGetLastError();
     n = 0;
   }
-  cache[nsplit][cls] = n + 1;
+  *cached = n + 1;
   return n;
 }
 
@@ -498,6 +711,9 @@ static int ttc_max_clusters(TtcKernel kern, int mpad, int nsplit, size_t smem) {
 // 16 < M, K % 64 == 0, N_i % 256 == 0, on tcgen05.  `err` is a device int the kernel sets to 1 if one of its
 // bounded waits expires (results are then undefined); the caller zeroes it beforehand and may read it after
 // synchronising.
+// Up to 128 rows: gemm_tiled_tc_kernel, 256 features per CTA.  Above: gemm_tiled_wide_kernel, 128 features and up
+// to 256 rows per CTA, in equal row chunks (the first kernel's accumulators hold 128 rows: it read the
+// weights once per 128 rows and launched once per chunk).
 extern "C" int q40_gemm_tiled_tc_multi(int nmat, const void* a, int64_t lda, const void* const* bw_tiled,
                                        void* const* c, const int64_t* ldc, const int* n_cols, int M, int K, int* err,
                                        int use_pdl, void* stream) {
@@ -507,12 +723,17 @@ extern "C" int q40_gemm_tiled_tc_multi(int nmat, const void* a, int64_t lda, con
   if (nmat < 1 || nmat > 3) return Q40_E_UNSUPPORTED;
   if (M < 1 || K <= 0 || K % BK != 0 || lda < K || lda % 8 != 0) return Q40_E_SHAPE;
   if (!q40_aligned(a, 16)) return Q40_E_ALIGN;
-  int spans = 0;
+  int spans = 0, widest = 0;
+  Params p{};
   for (int i = 0; i < nmat; ++i) {
     if (!bw_tiled[i] || !c[i]) return Q40_E_NULL;
     if (n_cols[i] <= 0 || n_cols[i] % SPAN != 0 || ldc[i] < n_cols[i] || ldc[i] % 2 != 0) return Q40_E_SHAPE;
     if (!q40_aligned(bw_tiled[i], 16) || !q40_aligned(c[i], 4)) return Q40_E_ALIGN;
-    spans += n_cols[i] / SPAN;
+    p.bw[i] = (const uint8_t*)bw_tiled[i];
+    p.c[i] = (__half*)c[i]; p.ldc[i] = ldc[i];
+    p.N[i] = n_cols[i]; p.spans[i] = n_cols[i] / SPAN;
+    spans += p.spans[i];
+    widest = p.spans[i] > widest ? p.spans[i] : widest;
   }
   EncodeTiledFn encode = ttc_encode_fn();
   if (!encode) return Q40_E_UNSUPPORTED;
@@ -521,82 +742,85 @@ extern "C" int q40_gemm_tiled_tc_multi(int nmat, const void* a, int64_t lda, con
     return Q40_E_UNSUPPORTED;
   cudaStream_t st = (cudaStream_t)stream;
   const int kblocks = K / BK;
-  const __half* ah = (const __half*)a;
-  // the two accumulators hold 128 batch rows: wider batches go in chunks (the weights of the later chunks
-  // come from L2 when the matrix fits there)
-  for (int m0 = 0; m0 < M; m0 += ACC_COLS) {
-    const int mc = (M - m0) < ACC_COLS ? (M - m0) : ACC_COLS;
-    Params p{};
-    p.nprob = nmat;
-    for (int i = 0; i < nmat; ++i) {
-      p.bw[i] = (const uint8_t*)bw_tiled[i];
-      p.c[i] = (__half*)c[i] + (int64_t)m0 * ldc[i]; p.ldc[i] = ldc[i];
-      p.N[i] = n_cols[i]; p.spans[i] = n_cols[i] / SPAN;
-    }
-    p.M = mc; p.K = K; p.Mpad = (mc + 15) / 16 * 16;
-    p.split_acc = p.Mpad <= 64 ? 1 : 0;
-    p.err = err;
+  const bool wide = M > ACC_COLS;
+  const int max_rows = wide ? wide::MAX_ROWS : ACC_COLS;
+  const int chunks = (M + max_rows - 1) / max_rows;
+  if (chunks > 65535) return Q40_E_SHAPE;
+  p.nprob = nmat;
+  p.M = M; p.K = K; p.Mpad = ((M + chunks - 1) / chunks + 15) / 16 * 16;
+  p.split_acc = p.Mpad <= 64 ? 1 : 0;
+  p.err = err;
 #ifdef Q40_TRACE
-    p.trace = q40_trace_ptr;
+  p.trace = q40_trace_ptr;
 #endif
-    // activations [mc rows, K] as a 2-D tensor, box {64 k, Mpad rows}, 128-byte swizzle, zero fill beyond row mc
-    CUtensorMap amap;
-    const cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)mc};
-    const cuuint64_t gstride[1] = {(cuuint64_t)lda * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)p.Mpad};
-    const cuuint32_t estr[2] = {1, 1};
-    if (encode(&amap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)(ah + (int64_t)m0 * lda), gdim, gstride, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return Q40_E_UNSUPPORTED;
-    // ring depth: what fits, at most MAX_STAGES; the fp32 tile of the epilogue reuses the ring
-    const size_t stage_bytes = (size_t)RAW_PAD + (size_t)p.Mpad * 128;
-    const size_t fixed = 1024 /* alignment slack */ + 256 /* barriers, tmem slot, flag */;
-    int stages = (int)((227 * 1024 - fixed) / stage_bytes);
-    if (stages > MAX_STAGES) stages = MAX_STAGES;
-    if (stages < 2) return Q40_E_UNSUPPORTED;
-    p.stages = stages;
-    size_t ring_bytes = (size_t)stages * stage_bytes;
-    const size_t tile_f = ((size_t)p.Mpad * SPAN + 64) * 4;     // slices are rounded up to 4 elements per rank
-    if (tile_f > ring_bytes) ring_bytes = tile_f;
-    const size_t smem = fixed + ring_bytes;
-    TtcKernel kern = gemm_tiled_tc_kernel;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) { (void)cudaGetLastError(); return Q40_E_UNSUPPORTED; }
-    // split K over a cluster (<= 8 ranks, each with at least 4 k blocks): the split that minimises
-    // waves x (k blocks per rank + a fixed cost of about 10 k blocks for allocation and epilogue)
-    int best = 1;
-    double best_cost = 1e30;
-    for (int ns = 1; ns <= 8; ++ns) {
-      const int bps = (kblocks + ns - 1) / ns;
-      if (ns > 1 && (bps < 4 || (ns - 1) * bps >= kblocks)) continue;
-      int fit = sms / ns;
-      if (ns > 1) {
-        fit = ttc_max_clusters(kern, p.Mpad, ns, smem);
-        if (fit < 1) continue;
-      }
-      const int waves = (spans + fit - 1) / fit;
-      const double cost = (double)waves * (bps + 10.0 + 1.5 * ns);
-      if (cost < best_cost) { best_cost = cost; best = ns; }
+  // activations [M rows, K] as a 2-D tensor, box {64 k, Mpad rows}, 128-byte swizzle, zero fill beyond row M
+  CUtensorMap amap;
+  const cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)M};
+  const cuuint64_t gstride[1] = {(cuuint64_t)lda * 2};
+  const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)p.Mpad};
+  const cuuint32_t estr[2] = {1, 1};
+  if (encode(&amap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)a, gdim, gstride, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return Q40_E_UNSUPPORTED;
+  // ring depth: what fits, at most MAX_STAGES; the fp32 tile of the epilogue reuses the ring
+  const size_t stage_bytes = (size_t)(wide ? wide::RAW_PAD : RAW_PAD) + (size_t)p.Mpad * 128;
+  const size_t fixed = 1024 /* alignment slack */ + 256 /* barriers, tmem slot, flag */;
+  int stages = (int)((227 * 1024 - fixed) / stage_bytes);
+  if (stages > MAX_STAGES) stages = MAX_STAGES;
+  if (stages < 2) return Q40_E_UNSUPPORTED;
+  p.stages = stages;
+  size_t ring_bytes = (size_t)stages * stage_bytes;
+  const size_t tile_f = ((size_t)p.Mpad * (wide ? wide::FEATS : SPAN) + 64) * 4;   // slices are rounded up to 4 elements per rank
+  if (tile_f > ring_bytes) ring_bytes = tile_f;
+  const size_t smem = fixed + ring_bytes;
+  TtcKernel kern = wide ? wide::gemm_tiled_wide_kernel : gemm_tiled_tc_kernel;
+  const int threads = wide ? wide::THREADS : THREADS;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) { (void)cudaGetLastError(); return Q40_E_UNSUPPORTED; }
+  // split K over a cluster (<= 8 ranks, each with at least 4 k blocks).
+  // Up to 128 rows: the split that minimises waves x (k blocks per rank + a fixed cost of about 10 k blocks for
+  // allocation and epilogue).
+  // Above: the largest power of two with which all tiles of the widest matrix run at once at one row chunk.  That
+  // is how q40_gemm_kn_tc splits k, and as both sum a rank's k range in order, a prompt pass of whole
+  // 256-row chunks has the same bits on either layout (the 512-row prompt pass of the 7B geometry with the
+  // split of least cost takes 11.4 ms and flips greedy tokens at near-ties).
+  const int tiles = spans * (wide ? SPAN / wide::FEATS : 1);
+  int best = 1;
+  double best_cost = 1e30;
+  for (int ns = 1; ns <= 8; ++ns) {
+    const int bps = (kblocks + ns - 1) / ns;
+    if (ns > 1 && (bps < 4 || (ns - 1) * bps >= kblocks)) continue;
+    int fit = sms / ns;
+    if (ns > 1) {
+      fit = ttc_max_clusters(kern, wide, threads, p.Mpad, ns, smem);
+      if (fit < 1) continue;
     }
-    const int nsplit = best, bps = (kblocks + nsplit - 1) / nsplit;
-    p.rows_per_split = bps * BK;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(spans, nsplit, 1);
-    cfg.blockDim = dim3(THREADS, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1;
-    attr[0].val.clusterDim.y = nsplit;
-    attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = use_pdl ? 2 : 1;
-    e = cudaLaunchKernelEx(&cfg, kern, p, amap);
-    if (e != cudaSuccess) return (int)e;
+    if (wide) {
+      if (ns == 1 || ((ns & (ns - 1)) == 0 && fit >= widest * (SPAN / wide::FEATS))) best = ns;
+      continue;
+    }
+    const int waves = (tiles + fit - 1) / fit;
+    const double cost = (double)waves * (bps + 10.0 + 1.5 * ns);
+    if (cost < best_cost) { best_cost = cost; best = ns; }
   }
+  const int nsplit = best, bps = (kblocks + nsplit - 1) / nsplit;
+  p.rows_per_split = bps * BK;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(tiles, nsplit, chunks);
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = nsplit;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = use_pdl ? 2 : 1;
+  e = cudaLaunchKernelEx(&cfg, kern, p, amap);
+  if (e != cudaSuccess) return (int)e;
   return Q40_OK;
 }

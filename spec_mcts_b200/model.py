@@ -221,13 +221,15 @@ class Transformer(nn.Module):
         self.use_tp_fused_allreduce = True
         self.tp_wait_cycles = 0     # limit of the wait for a peer's rows in SM cycles (0: 2^31, about a second)
         self._tp_peer = None
-        # the prompt pass keeps the checkpoint-layout tensor-core matmul by default: the tiled-copy kernel sums
-        # k in a different order, which flips greedy tokens at near-ties against the 7B reference run
+        # the prompt pass above 16 rows reads the tiled copies too (the decode step needs them anyway); True: it
+        # reads the checkpoint layout, unless prefill_tiled_tc asks for the copies
+        self.prefill_checkpoint_layout = False
         self.prefill_tiled_tc = False
         # True: the prompt pass returns logits of the last position only, [1, 1, vocab] (all a caller that
         # samples the next token needs); False: of every position like the reference
         self.prefill_last_only = False
         self._tc_err = None         # device word the prompt pass's tensor-core launches set on a wait expiry
+        self._tc_err_host = None    # ... and its copy of the last finished pass
         # ... True: through the byte-balanced stream-K launch (one CTA per SM, bulk-copy ring, no clusters);
         # False: the cluster-reduced launch on the same tiled copies (faster on B200, the default)
         self.use_stream = False
@@ -281,47 +283,82 @@ class Transformer(nn.Module):
         bsz, S = tokens.shape
         assert bsz == 1, "the prompt is processed once and shared by all branches"
         assert S <= p.max_prompt_seq_len
+        self._check_tc_err()
         dev = self.device
         H, Hkv, D = self._H, self._Hkv, self._D
+        hid = self.layers[0].feed_forward.hidden_dim
+        # tiled copies are made ahead of the pass: a dependent launch reads its weights before it waits for the
+        # launch in front of it, which must not be the one that writes them
+        plan = []
+        for layer in self.layers:
+            att, ff = layer.attention, layer.feed_forward
+            plan.append([(lins, self._tiled_of(lins) if self._prefill_tiled(S, lins) else None)
+                         for lins in ([att.wq, att.wk, att.wv], [att.wo], [ff.w1, ff.w3], [ff.w2])])
         h = self.tok_embeddings(tokens.to(dev)).to(DTYPE).view(S, p.dim)
         pos = torch.arange(S, dtype=torch.int32, device=dev)
-        for li, layer in enumerate(self.layers):
-            att, ff = layer.attention, layer.feed_forward
-            xn = K.rmsnorm(h, layer.attention_norm.weight, p.norm_eps)
-            xq, xk, xv = self._mm(xn, [att.wq, att.wk, att.wv])
-            xq, xk, xv = xq.view(S, H, D), xk.view(S, Hkv, D), xv.view(S, Hkv, D)
-            K.rope_(xq, pos, self._cos, self._sin)
-            K.rope_(xk, pos, self._cos, self._sin)
-            att.cache_prompt_k[:S] = xk
-            att.cache_prompt_v[:S] = xv
+        st = torch.cuda.current_stream(dev).cuda_stream
+        e = lambda n: torch.empty((S, n), dtype=DTYPE, device=dev)
+        xn, q, ao, o, a1, a3, g, f = (e(n) for n in (p.dim, H * D, H * D, p.dim, hid, hid, hid, p.dim))
+        pending = None     # output of the previous sub-block, added to h by the next norm kernel
+        for layer, (qkv, wo, w13, w2) in zip(self.layers, plan):
+            att = layer.attention
+            # keys and values go straight to their place in the prompt cache
+            ck, cv = att.cache_prompt_k[:S], att.cache_prompt_v[:S]
+            self._norm(h, pending, layer.attention_norm.weight, xn, st)
+            self._mm(xn, qkv, [q, ck.view(S, Hkv * D), cv.view(S, Hkv * D)], st)
+            K.rope_(q.view(S, H, D), pos, self._cos, self._sin)
+            K.rope_(ck, pos, self._cos, self._sin)
             att.cache_prompt_len = S
             # causal attention over the prompt (grouped-query heads read their kv head directly)
-            o = K.causal_attn(xq, xk, xv).view(S, H * D)
-            ao = self._all_reduce(self._mm(o, [att.wo])[0])
-            hn, h = K.rmsnorm(h, layer.ffn_norm.weight, p.norm_eps, residual=ao)
-            a1, a3 = self._mm(hn, [ff.w1, ff.w3])
-            f2 = self._all_reduce(self._mm(K.silu_mul(a1, a3), [ff.w2])[0])
-            h = h + f2
+            K.causal_attn(q.view(S, H, D), ck, cv, out=ao.view(S, H, D))
+            self._mm(ao, wo, [o], st)
+            self._all_reduce(o)
+            self._norm(h, o, layer.ffn_norm.weight, xn, st)
+            self._mm(xn, w13, [a1, a3], st)
+            check(lib.q40_silu_mul(a1.data_ptr(), a3.data_ptr(), g.data_ptr(), g.numel(), st), "q40_silu_mul")
+            self._mm(g, w2, [f], st)
+            self._all_reduce(f)
+            pending = f
         self._prefix_len_dev.fill_(S)
-        if self._tc_err is not None and int(self._tc_err.item()) != 0:
-            raise K.Q40Error("prompt pass: a bounded wait inside a tensor-core matmul expired")
+        if self._tc_err is not None:
+            self._tc_err_host.copy_(self._tc_err, non_blocking=True)      # read by the next call, without a wait here
         if self.prefill_last_only:
             # the tree search reads the last position only (mcts.py:105); the reference computes all S rows
-            h = h[S - 1:]
-        hn = K.rmsnorm(h, self.norm.weight, p.norm_eps)
-        return F.linear(hn, self.output.weight).to(DTYPE).view(1, h.shape[0], -1)
+            h, xn, pending = h[S - 1:], xn[S - 1:], pending[S - 1:]
+        self._norm(h, pending, self.norm.weight, xn, st)
+        return F.linear(xn, self.output.weight).to(DTYPE).view(1, h.shape[0], -1)
 
-    def _mm(self, x, lins):
-        """[x @ deq(W_i)] for projections that share the activations x [M, K] (prompt pass): one tensor-core
-        launch on the tiled copies when the shapes allow it, matmul_q40 per projection otherwise."""
-        M = x.shape[0]
-        if (M > 16 and self.use_tiled and self.use_tiled_tc and self.prefill_tiled_tc and len(lins) <= 3 and
-                all(l.group_size == 64 and self._tileable(l) and l.kn()[0] % 64 == 0 for l in lins)):
+    def _check_tc_err(self):
+        if self._tc_err_host is not None and int(self._tc_err_host) != 0:
+            raise K.Q40Error("prompt pass: a bounded wait inside a tensor-core matmul expired")
+
+    def _prefill_tiled(self, M, lins):
+        """Whether the prompt pass multiplies these projections through their tiled copies."""
+        return (M > 16 and self.use_tiled and self.use_tiled_tc and len(lins) <= 3 and
+                (self.prefill_tiled_tc or not self.prefill_checkpoint_layout) and
+                all(l.group_size == 64 and self._tileable(l) and l.kn()[0] % 64 == 0 for l in lins))
+
+    def _mm(self, x, weights, outs, st):
+        """outs[i] = x @ deq(W_i) for projections that share the activations x [M, K] (prompt pass): one tensor-core
+        launch when they have tiled copies, matmul_q40 per projection otherwise."""
+        import ctypes
+        lins, tiled = weights
+        n = len(lins)
+        if tiled is not None:
             if self._tc_err is None:
                 self._tc_err = torch.zeros(1, dtype=torch.int32, device=self.device)
-            return K.gemm_tiled_tc(x, [(t, l.kn()) for t, l in zip(self._tiled_of(lins), lins)], err=self._tc_err)
-        # relayout=False: the checkpoint-layout kernels, whose summation order the 7B token parity was taken with
-        return [K.matmul_q40(x, l.w, l.s, l.kn(), group_size=l.group_size, relayout=False) for l in lins]
+                self._tc_err_host = torch.zeros(1, dtype=torch.int32, pin_memory=True)
+            P = ctypes.c_void_p * n
+            check(lib.q40_gemm_tiled_tc_multi(n, x.data_ptr(), x.stride(0), P(*[t.data_ptr() for t in tiled]),
+                                              P(*[o.data_ptr() for o in outs]),
+                                              (ctypes.c_int64 * n)(*[o.stride(0) for o in outs]),
+                                              (ctypes.c_int * n)(*[l.kn()[1] for l in lins]), x.shape[0], x.shape[1],
+                                              self._tc_err.data_ptr(), 1 if self.use_pdl else 0, st),
+                  "q40_gemm_tiled_tc_multi")
+            return
+        # relayout=False: the checkpoint-layout kernels
+        for l, o in zip(lins, outs):
+            K.matmul_q40(x, l.w, l.s, l.kn(), group_size=l.group_size, relayout=False, out=o)
 
     # ------------------------------------------------------------------ decode
     def _step_buffers(self, B):

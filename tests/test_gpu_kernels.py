@@ -187,6 +187,20 @@ def test_linear_nk_vs_oracle(K, M, NK, G):
     assert_close(host(y), O.linear_q40_nk(x, q, s, (N, Kd), G))
 
 
+@pytest.mark.parametrize("M", [17, 32, 33, 64, 65, 100])
+@pytest.mark.parametrize("NK,G", [((100, 2944), 64), ((1000, 640), 32), ((64, 11008), 64)])
+def test_linear_nk_more_rows_than_one_mma_tile_pair(K, M, NK, G):
+    """Above 16 rows a launch takes up to 64 of them and stages the activations piece by piece: ragged rows, k ranges
+    of whole and partial pieces.  Tolerance: fp16 result and operands, fp32 sums (the repository's for matmuls)."""
+    rng = np.random.default_rng(M + NK[0])
+    N, Kd = NK
+    x = (rng.standard_normal((M, Kd)) * 0.5).astype(np.float16)
+    w = (rng.standard_normal((N, Kd)) * 0.05).astype(np.float16)
+    q, s = O.quantize_q40(w, G)
+    y = K.linear_q40(dev(x), dev(q), dev(s), (N, Kd), group_size=G)
+    assert_close(host(y), O.linear_q40_nk(x, q, s, (N, Kd), G))
+
+
 @pytest.mark.parametrize("M", [17, 100, 300])
 def test_matmul_tc_multi_matches_oracle(K, M):
     """Three matrices that share the activations in one tensor-core launch (the q, k, v projections
@@ -311,6 +325,34 @@ def test_attn_paged_ragged_vs_oracle(K, page_size, idx):
     assert float(host(o)[0].astype(np.float32).max()) == 0.0   # empty branch -> zeros
 
 
+@pytest.mark.parametrize("B,H,Hkv,L", [(13, 34, 34, 70), (14, 32, 8, 130), (37, 32, 32, 33), (37, 33, 11, 70), (149, 8, 8, 5)])
+@pytest.mark.parametrize("paged", [False, True])
+def test_attn_branch_row_counts_around_the_splits(K, B, H, Hkv, L, paged):
+    """Row counts (branches x heads) on both sides of where the warps per row change, odd ones among them, and ragged
+    lengths with empty branches, against fp32 torch."""
+    g = torch.Generator(device="cuda").manual_seed(B * H + L)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").half()
+    q = rnd(B, H, 128)
+    if paged:
+        P = 3 * L + 1
+        k, v = rnd(Hkv, P, 128), rnd(Hkv, P, 128)
+        tbl = torch.randint(0, P, (B, L), generator=g, device="cuda", dtype=torch.int32)
+        lens = torch.randint(0, L + 1, (B,), generator=g, device="cuda", dtype=torch.int32)
+        lens[0], lens[-1] = 0, L
+        o = K.page_flash_attn(tbl, q, k, v, P, B, L, H, 128, seq_lens=lens)
+        kb, vb = (t[:, tbl.long()].permute(1, 0, 2, 3).float() for t in (k, v))         # [B, Hkv, L, 128]
+    else:
+        k, v = rnd(B, Hkv, L, 128), rnd(B, Hkv, L, 128)
+        lens = torch.full((B,), L, device="cuda")
+        o = K.flash_attn(q, k, v, B, L, H, 128)
+        kb, vb = k.float(), v.float()
+    kb, vb = (t.repeat_interleave(H // Hkv, 1) for t in (kb, vb))
+    sc = torch.einsum("bhd,bhld->bhl", q.float(), kb) / 128 ** 0.5
+    sc = sc.masked_fill(torch.arange(L, device="cuda")[None, None] >= lens[:, None, None], float("-inf"))
+    ref = torch.einsum("bhl,bhld->bhd", torch.softmax(sc, -1).nan_to_num(0.0), vb)      # no keys: zeros
+    assert_close(host(o.view(B, H, 128)), ref.cpu().numpy())
+
+
 @pytest.mark.parametrize("B,H,Hkv,prefix", [(5, 4, 4, 40), (64, 8, 8, 300), (100, 4, 4, 129), (9, 16, 2, 64),
                                             (1, 32, 32, 2048)])
 def test_attn_shared_prefix_vs_oracle(K, B, H, Hkv, prefix):
@@ -394,6 +436,33 @@ def test_rope_golden_bit_exact(K, golden):
         x = dev(golden[f"ep.rope.{name}"]).view(3, 4, 128).clone()
         K.rope_(x, torch.full((3,), pos, dtype=torch.int32, device="cuda"), cos, sin)
         assert_bits_equal(host(x).reshape(3, 1, 4, 128), golden[f"ep.rope.o{name}"])
+
+
+@pytest.mark.parametrize("rows,heads,D", [(1, 1, 128), (77, 3, 128), (5, 2, 64), (9, 2, 20)])
+@pytest.mark.parametrize("pad", [0, 8, 4])
+def test_rope_on_strided_rows_is_the_same_on_either_kernel(K, rows, heads, D, pad):
+    """Rows that are 16 bytes apart (vector kernel) and rows that are not (one pair per thread): the bits of the
+    reference's formula, as fp16 torch operations give them."""
+    g = torch.Generator(device="cuda").manual_seed(rows * D + pad)
+    buf = torch.randn((rows, heads * D + pad), generator=g, device="cuda").half()
+    cos, sin = (torch.randn((100, D // 2), generator=g, device="cuda").half() for _ in range(2))
+    pos = torch.randint(0, 100, (rows,), generator=g, device="cuda", dtype=torch.int32)
+    x = buf[:, :heads * D].unflatten(1, (heads, D))
+    c, s = cos[pos.long()][:, None], sin[pos.long()][:, None]
+    lo, hi = x[..., :D // 2].clone(), x[..., D // 2:].clone()
+    ref = torch.cat((lo * c + (-hi) * s, hi * c + lo * s), dim=-1)
+    tail = buf[:, heads * D:].clone()
+    K.rope_(x, pos, cos, sin)
+    assert torch.equal(x, ref) and torch.equal(buf[:, heads * D:], tail)
+
+
+@pytest.mark.parametrize("M,Kd,N", [(256, 4096, 4096), (512, 4096, 4096), (512, 4096, 11008), (512, 11008, 4096)])
+def test_matmul_256_row_chunks_have_the_same_bits_on_either_layout(K, M, Kd, N):
+    """Whole 256-row chunks: the tiled-copy kernel splits and sums k as the checkpoint-layout kernel does."""
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    q, s = K.quantize_q40((torch.randn((Kd, N), generator=g, device="cuda") * 0.02).half(), 64)
+    a = torch.randn((M, Kd), generator=g, device="cuda").half()
+    assert torch.equal(K.matmul_q40(a, q, s, (Kd, N), relayout=True), K.matmul_q40(a, q, s, (Kd, N), relayout=False))
 
 
 def test_silu_mul_golden(K, golden):
