@@ -106,14 +106,22 @@ int q40_gemm_kn_tc_multi(int nmat, const void* a, int64_t lda, const void* const
 /* The same operation on TILED copies of the weights (q40_relayout_tiled; N_i % 256 == 0, K % 64 == 0),
  * so that a caller that already holds tiled copies for the narrow decode path needs no second format:
  * the weight stream of a CTA is one contiguous run fetched by 1-D bulk copies, the activations arrive by
- * tiled TMA copies (a tensor map over `a` is encoded per call), both into a 3..6 stage ring; A operand
+ * tiled TMA copies (a tensor map over `a` is encoded per call), both into a 3..8 stage ring; A operand
  * value fp16(code * scale) as in the reference (triton_kernels.py:444-445), written to tensor memory.  Batches
- * above 128 rows run as consecutive launches of 128 rows.  Results are bit-identical from run to run.  Same
+ * above 128 rows run in equal row chunks of at most 256 inside one launch.  Results are bit-identical from run to run.  Same
  * `err` and `use_pdl` rules as q40_gemm_kn_tc_multi; Q40_E_UNSUPPORTED when the driver offers no tensor-map
  * encoder. */
 int q40_gemm_tiled_tc_multi(int nmat, const void* a, int64_t lda, const void* const* bw_tiled, void* const* c,
                             const int64_t* ldc, const int* n_cols, int M, int K, int* err, int use_pdl,
                             void* stream);
+
+/* C[M, N] = A @ deq(B) for one TILED copy: q40_gemv_tiled (mode 0) up to 16 rows, q40_gemm_tiled_tc_multi above,
+ * under their rules, for hosts that make one call per projection.  `max_cluster` is used up to 16 rows, `err` (which
+ * may be NULL there) above.
+ * Replaces: matmul_q40 (triton_kernels.py:471-500). */
+int q40_matmul_tiled(const void* bw_tiled, void* c, int64_t ldc, const void* a, int64_t lda, int M, int N, int K,
+                     int max_cluster, int* err, int use_pdl, void* stream);
+
 
 /* q40_gemm_kn without a caller-provided workspace, for hosts that cannot allocate device
  * memory themselves (all HBM already handed to their own planner, or a plug-in that only

@@ -110,6 +110,8 @@ SIGNATURES = {
     "q40_embed_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
     "q40_rmsnorm": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float,
                             c_void_p]),
+    "q40_matmul_tiled": (c_int, [c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_void_p,
+                                 c_int, c_void_p]),
     "q40_rope": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int64,
                          c_void_p]),
     "q40_silu_mul": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_void_p]),

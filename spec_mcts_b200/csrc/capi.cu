@@ -21,3 +21,13 @@ extern "C" const char* q40_strerror(int status) {
 void* q40_trace_ptr = nullptr;
 extern "C" void q40_debug_trace(void* buf) { q40_trace_ptr = buf; }
 #endif
+
+// One call per projection costs the host more than the launch when its arguments are arrays: the plain form.
+extern "C" int q40_matmul_tiled(const void* bw_tiled, void* c, int64_t ldc, const void* a, int64_t lda, int M, int N,
+                                int K, int max_cluster, int* err, int use_pdl, void* stream) {
+  const void* none = nullptr;
+  if (M <= 16)
+    return q40_gemv_tiled(0, 1, &bw_tiled, &none, &c, &N, ldc, a, lda, M, K, nullptr, nullptr, 0, 0.f, nullptr, 0,
+                          nullptr, 0, max_cluster, use_pdl, stream);
+  return q40_gemm_tiled_tc_multi(1, a, lda, &bw_tiled, &c, &ldc, &N, M, K, err, use_pdl, stream);
+}

@@ -22,6 +22,8 @@
 // stream is one sequential run.
 #include <cooperative_groups.h>
 
+#include <atomic>
+
 #include "q40_common.cuh"
 
 namespace cg = cooperative_groups;
@@ -176,62 +178,84 @@ gemv_tiled_kernel(const TiledParams p) {
   asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   Q40_STAMP(2);
-  // the residual value of the first output this thread finishes, fetched now instead of at the very end
-  __half h_first = __float2half(0.f);
-  if (EPI == EPI_RESIDUAL && warp < p.M && lane < slice && col_ok)
-    h_first = p.h_in[(int64_t)warp * p.ldh + f_span_col(span, rank * slice + lane)];
+  // the residual values of the first column this thread finishes, fetched now instead of at the very end
+  constexpr int RPW = (MT * 8 + FW - 1) / FW;      // rows of a warp
+  __half h_first[RPW];
+#pragma unroll
+  for (int r = 0; r < RPW; ++r)
+    h_first[r] = (EPI == EPI_RESIDUAL && warp + r * FW < p.M && lane < slice && col_ok)
+                     ? p.h_in[(int64_t)(warp + r * FW) * p.ldh + f_span_col(span, rank * slice + lane)]
+                     : __float2half(0.f);
 
   // ---- activations of this k range.  RMSNorm prologue with the reference's rounding points:
-  // fp16(fp16(float(a) * 1/rms) * norm_w).  The raw values are requested first, then the row statistics
-  // are summed while they are in flight ----
+  // fp16(fp16(float(a) * 1/rms) * norm_w).  A thread has XU 16-byte chunks (and their norm weights) in flight; the
+  // first of them are requested ahead of the row statistics, whose partials of all of a warp's rows are in
+  // flight together.  (One chunk and one row at a time, each a trip to L2, cost a 10-row launch 4 to 7 us.) ----
   {
+    constexpr int XU = (MT == 1) ? 2 : 4;
     const int chunks = p.rows_per_split / 8;
     const int total = MT * 8 * chunks;
-    auto load_chunk = [&](int idx) {
-      const int m = idx / chunks, k = kb + (idx % chunks) * 8;
-      return (m < p.M && k < ke) ? *reinterpret_cast<const uint4*>(p.a + (int64_t)m * p.lda + k)
-                                 : make_uint4(0, 0, 0, 0);
-    };
-    auto store_chunk = [&](int idx, uint4 v) {
-      const int m = idx / chunks, kk = (idx % chunks) * 8;
-      const int k = kb + kk;
-      if (PRO == PRO_NORM && m < p.M && k < ke) {
-        const uint4 wv = *reinterpret_cast<const uint4*>(p.norm_w + k);
-        const float inv = s_inv[m];
-        __half2* vh = reinterpret_cast<__half2*>(&v);
-        const __half2* wh = reinterpret_cast<const __half2*>(&wv);
+    uint4 xv[XU], wv[XU];
+    auto load_chunks = [&](int idx0) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 f = __half22float2(vh[j]);
-          vh[j] = __hmul2(__floats2half2_rn(f.x * inv, f.y * inv), wh[j]);
-        }
+      for (int u = 0; u < XU; ++u) {
+        const int idx = idx0 + u * FT;
+        const int m = idx / chunks, k = kb + (idx % chunks) * 8;
+        const bool ok = m < p.M && k < ke;
+        xv[u] = ok ? *reinterpret_cast<const uint4*>(p.a + (int64_t)m * p.lda + k) : make_uint4(0, 0, 0, 0);
+        if (PRO == PRO_NORM) wv[u] = ok ? *reinterpret_cast<const uint4*>(p.norm_w + k) : make_uint4(0, 0, 0, 0);
       }
-      *reinterpret_cast<uint4*>(xs + m * xs_ld + kk) = v;
     };
-    uint4 v_first = make_uint4(0, 0, 0, 0);
-    if (tid < total) v_first = load_chunk(tid);
+    auto store_chunks = [&](int idx0) {
+#pragma unroll
+      for (int u = 0; u < XU; ++u) {
+        const int idx = idx0 + u * FT;
+        if (idx >= total) break;
+        const int m = idx / chunks, kk = (idx % chunks) * 8;
+        if (PRO == PRO_NORM && m < p.M && kb + kk < ke) {
+          const float inv = s_inv[m];
+          __half2* vh = reinterpret_cast<__half2*>(&xv[u]);
+          const __half2* wh = reinterpret_cast<const __half2*>(&wv[u]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 f = __half22float2(vh[j]);
+            vh[j] = __hmul2(__floats2half2_rn(f.x * inv, f.y * inv), wh[j]);
+          }
+        }
+        *reinterpret_cast<uint4*>(xs + m * xs_ld + kk) = xv[u];
+      }
+    };
+    load_chunks(tid);
     if (PRO == PRO_NORM) {
-      for (int m = warp; m < p.M; m += FW) {
-        // all loads in flight before the first add (the partials sit in L2)
-        float s = 0.f;
-        const float* sp = p.ss_in + (int64_t)m * p.ss_in_count;
-        for (int i0 = 0; i0 < p.ss_in_count; i0 += 256) {
-          float part[8];
+      float s[RPW];
+#pragma unroll
+      for (int r = 0; r < RPW; ++r) s[r] = 0.f;
+      for (int i0 = 0; i0 < p.ss_in_count; i0 += 256) {
+        float part[RPW][8];
+#pragma unroll
+        for (int r = 0; r < RPW; ++r)
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
-            const int i = i0 + u * 32 + lane;
-            part[u] = (i < p.ss_in_count) ? __ldcg(sp + i) : 0.f;
+            const int m = warp + r * FW, i = i0 + u * 32 + lane;
+            part[r][u] = (m < p.M && i < p.ss_in_count) ? __ldcg(p.ss_in + (int64_t)m * p.ss_in_count + i) : 0.f;
           }
 #pragma unroll
-          for (int u = 0; u < 8; ++u) s += part[u];
-        }
-        s = warp_sum(s);
-        if (lane == 0) s_inv[m] = rsqrtf(s / (float)p.K + p.eps);
+        for (int r = 0; r < RPW; ++r)
+#pragma unroll
+          for (int u = 0; u < 8; ++u) s[r] += part[r][u];
+      }
+#pragma unroll
+      for (int r = 0; r < RPW; ++r) {
+        s[r] = warp_sum(s[r]);
+        if (lane == 0 && warp + r * FW < p.M) s_inv[warp + r * FW] = rsqrtf(s[r] / (float)p.K + p.eps);
       }
       __syncthreads();
     }
-    if (tid < total) store_chunk(tid, v_first);
-    for (int idx = tid + FT; idx < total; idx += FT) store_chunk(idx, load_chunk(idx));
+    store_chunks(tid);
+    for (int idx = tid + XU * FT; idx < total; idx += XU * FT) {
+      load_chunks(idx);
+      store_chunks(idx);
+    }
   }
   __syncthreads();
 
@@ -340,7 +364,10 @@ gemv_tiled_kernel(const TiledParams p) {
   // ---- split-K over the cluster: rank r finishes columns [r*slice, (r+1)*slice) of the span from the
   // partials it received (added in rank order) ----
   const int npart = (EPI == EPI_SILU) ? nranks / 2 : nranks;
-  for (int m = warp; m < p.M; m += FW) {
+#pragma unroll
+  for (int mr = 0; mr < RPW; ++mr) {
+    const int m = warp + mr * FW;
+    if (m >= p.M) break;
     float ssq = 0.f;
     for (int cidx = lane; cidx < slice; cidx += 32) {
       const int lc = rank * slice + cidx;
@@ -360,7 +387,7 @@ gemv_tiled_kernel(const TiledParams p) {
         if (EPI == EPI_STORE) {
           pr.out[(int64_t)m * p.ldc + n] = __float2half_rn(v0);
         } else if (EPI == EPI_RESIDUAL) {
-          const __half hres = (m == warp && cidx == lane) ? h_first : p.h_in[(int64_t)m * p.ldh + n];
+          const __half hres = cidx == lane ? h_first[mr] : p.h_in[(int64_t)m * p.ldh + n];
           const __half hn = __hadd_rn(hres, __float2half_rn(v0));
           pr.out[(int64_t)m * p.ldc + n] = hn;
           const float f = __half2float(hn);
@@ -393,16 +420,30 @@ static int launch_tiled(const TiledParams& p, int grid_x, int nsplit, int cluste
   TiledParams pp = p;
   pp.recv_off = (int)smem;
   smem += (size_t)p.M * F_SPAN_COLS * 4;        // receive buffer of the cluster reduction
+  // What this kernel was set up for on a device, so that a repeated call asks the runtime nothing (the cluster
+  // query alone costs more than the launch).  The attributes are the same for every call, so that threads that meet here
+  // do not undo each other's; the cluster answer holds up to the shared memory it was asked with.
+  constexpr int SMEM_MAX = 227 * 1024;
+  struct Ready { std::atomic<int> attrs{0}, cluster16{0}; };
+  static Ready ready_all[16];
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) dev = -1;
+  Ready* ready = dev >= 0 ? &ready_all[dev] : nullptr;
+  cudaError_t e;
   // a shape whose shared-memory need exceeds what a CTA of this device may have is refused with a
   // negative status (callers fall back to the workspace kernel), not reported as a CUDA error
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) {
-    (void)cudaGetLastError();
-    return Q40_E_UNSUPPORTED;
+  if (smem > (size_t)SMEM_MAX) return Q40_E_UNSUPPORTED;
+  if (!ready || !ready->attrs.load(std::memory_order_acquire)) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
+    if (e != cudaSuccess) {
+      (void)cudaGetLastError();
+      return Q40_E_UNSUPPORTED;
+    }
+    // set on every variant, not only those that need it (see the note at q40_gemv_tiled)
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return (int)e;
+    if (ready) ready->attrs.store(1, std::memory_order_release);
   }
-  // set on every variant, not only those that need it (see the note at q40_gemv_tiled)
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid_x, nsplit, 1);
   cfg.blockDim = dim3(FT, 1, 1);
@@ -417,7 +458,7 @@ static int launch_tiled(const TiledParams& p, int grid_x, int nsplit, int cluste
   attrs[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attrs;
   cfg.numAttrs = 1;
-  if (cluster_x * nsplit > 8) {
+  if (cluster_x * nsplit > 8 && (!ready || (int)smem > ready->cluster16.load(std::memory_order_acquire))) {
     // a 16-CTA cluster is outside the portable limit: ask whether this device can schedule one
     int nclusters = 0;
     e = cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg);
@@ -425,6 +466,7 @@ static int launch_tiled(const TiledParams& p, int grid_x, int nsplit, int cluste
       (void)cudaGetLastError();
       return Q40_E_UNSUPPORTED;
     }
+    if (ready) ready->cluster16.store((int)smem, std::memory_order_release);
   }
   cfg.numAttrs = pdl ? 2 : 1;
   e = cudaLaunchKernelEx(&cfg, kern, pp);
@@ -516,43 +558,65 @@ extern "C" int q40_gemv_tiled_ss_count(int N, int K, int max_cluster) {
 namespace q40 {
 namespace tiled {
 
-// One thread per output word (or per scale): gathers eight nibbles of the checkpoint layout into the
-// word of (span, k step, group, lane, tile) described at the top of this file.
+// A block rewrites four steps of a span (64 k rows x 128 packed bytes) through shared memory, so that both sides are
+// read and written in whole lines.  A thread takes, for k rows 4t .. 4t+3, four neighbouring columns g0 .. g0+3 of
+// a 16-column tile and the four columns 8 further, in both nibbles: eight words of the format described at the top
+// of this file.  (One thread per word, gathering eight bytes from eight lines: ~20 us for 4096 x 4096.)
+constexpr int RL_STEPS = 4;
 __global__ void __launch_bounds__(256)
 relayout_kernel(const uint8_t* __restrict__ bw, const __half* __restrict__ bs, uint8_t* __restrict__ out, int N,
                 int K) {
-  const int ksteps = K / 16;
-  const int64_t nsteps = (int64_t)(N / 256) * ksteps;
-  const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t stepi = gid / 576;            // 512 weight words + 64 scale slots per step
-  const int w = (int)(gid % 576);
-  if (stepi >= nsteps) return;
-  const int span = (int)(stepi / ksteps), ks = (int)(stepi % ksteps);
-  uint8_t* dst = out + stepi * T_STEP_BYTES;
+  __shared__ __align__(16) uint8_t in_s[RL_STEPS * 16][F_SPAN_BYTES];
+  __shared__ __align__(16) uint8_t out_s[RL_STEPS * T_STEP_BYTES];
+  const int ksteps = K / 16, tid = threadIdx.x;
+  const int per_span = (ksteps + RL_STEPS - 1) / RL_STEPS;
+  const int span = blockIdx.x / per_span, ks0 = (blockIdx.x % per_span) * RL_STEPS;
+  const int nst = min(RL_STEPS, ksteps - ks0);
   const int64_t w_ld = N / 2, s_ld = N / 64;
-  if (w < 512) {
-    const int q = w >> 7, lane = (w >> 2) & 31, jt = w & 3;
-    const int g = lane >> 2, t = lane & 3;
-    // native layout: group q of the span = block q/2 of the span's two 64-byte blocks, high nibble if q even
-    const int byte_col = span * 128 + (q >> 1) * 64 + jt * 16 + g;     // column g of the tile; column g+8 is 8 bytes on
-    const bool high = (q & 1) == 0;
-    uint32_t nib[2][4];
-#pragma unroll
-    for (int c = 0; c < 2; ++c)
-#pragma unroll
-      for (int kk = 0; kk < 4; ++kk) {
-        const uint8_t b = bw[(int64_t)(ks * 16 + 4 * t + kk) * w_ld + byte_col + 8 * c];
-        nib[c][kk] = high ? (b >> 4) : (b & 0xF);
-      }
-    // byte0 = A | B<<4, byte1 = C | D<<4, byte2 = E | F<<4, byte3 = G | H<<4 with
-    // B,F,D,H = column g at k+0,+1,+2,+3 and A,E,C,G = column g+8 at k+0,+1,+2,+3
-    const uint32_t word = (nib[1][0] | (nib[0][0] << 4)) | ((nib[1][2] | (nib[0][2] << 4)) << 8) |
-                          ((nib[1][1] | (nib[0][1] << 4)) << 16) | ((nib[1][3] | (nib[0][3] << 4)) << 24);
-    reinterpret_cast<uint32_t*>(dst)[w] = word;
+  const uint8_t* src = bw + (int64_t)ks0 * 16 * w_ld + span * F_SPAN_BYTES;
+  if (((uintptr_t)bw & 15) == 0) {
+    for (int i = tid; i < nst * 16 * (F_SPAN_BYTES / 16); i += 256)
+      *reinterpret_cast<uint4*>(&in_s[i >> 3][(i & 7) * 16]) = *reinterpret_cast<const uint4*>(src + (i >> 3) * w_ld + (i & 7) * 16);
   } else {
-    const int i = w - 512, q = i >> 4, kk = i & 15;
-    reinterpret_cast<__half*>(dst + 2048)[i] = bs[(int64_t)(ks * 16 + kk) * s_ld + span * 4 + q];
+    for (int i = tid; i < nst * 16 * F_SPAN_BYTES; i += 256) in_s[i >> 7][i & 127] = src[(i >> 7) * w_ld + (i & 127)];
   }
+  if (tid < nst * 64) {
+    const int st = tid >> 6, q = (tid >> 4) & 3, kk = tid & 15;
+    reinterpret_cast<__half*>(out_s + st * T_STEP_BYTES + 2048)[q * 16 + kk] =
+        bs[(int64_t)((ks0 + st) * 16 + kk) * s_ld + span * 4 + q];
+  }
+  __syncthreads();
+  const int st = tid >> 6;
+  if (st < nst) {
+    const int t = tid & 3, g0 = (tid >> 2 & 1) * 4, jt = tid >> 3 & 3, blk = tid >> 5 & 1;
+    uint32_t a[4], b[4];                       // columns g0.. and g0 + 8.. of the tile, rows k = 4t + kk
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      const uint8_t* row = in_s[st * 16 + 4 * t + kk] + blk * 64 + jt * 16 + g0;
+      a[kk] = *reinterpret_cast<const uint32_t*>(row);
+      b[kk] = *reinterpret_cast<const uint32_t*>(row + 8);
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+#pragma unroll
+      for (int lo = 0; lo < 2; ++lo) {
+        // byte 0 = k + 0, byte 1 = k + 2, byte 2 = k + 1, byte 3 = k + 3; column g in the high nibble, g + 8 in the low
+        uint32_t word = 0;
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+          const int kk = (y & 1) * 2 + (y >> 1);
+          const uint32_t na = (a[kk] >> (8 * c + (lo ? 0 : 4))) & 0xF, nb = (b[kk] >> (8 * c + (lo ? 0 : 4))) & 0xF;
+          word |= (nb | (na << 4)) << (8 * y);
+        }
+        const int q = blk * 2 + lo, lane = (g0 + c) * 4 + t;
+        *reinterpret_cast<uint32_t*>(out_s + st * T_STEP_BYTES + (q * 32 + lane) * 16 + jt * 4) = word;
+      }
+    }
+  }
+  __syncthreads();
+  uint8_t* dst = out + ((int64_t)span * ksteps + ks0) * T_STEP_BYTES;
+  for (int i = tid; i < nst * (T_STEP_BYTES / 16); i += 256)
+    reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(out_s)[i];
 }
 
 }  // namespace tiled
@@ -568,11 +632,10 @@ extern "C" int q40_relayout_tiled(const void* bw, const void* bs, void* out, int
   if (!bw || !bs || !out) return Q40_E_NULL;
   if (N <= 0 || K <= 0 || N % 256 != 0 || K % 16 != 0) return Q40_E_SHAPE;
   if (!q40_aligned(out, 16)) return Q40_E_ALIGN;
-  const int64_t threads = (int64_t)(N / 256) * (K / 16) * 576;
-  const int64_t grid = (threads + 255) / 256;
+  const int64_t grid = (int64_t)((K / 16 + q40::tiled::RL_STEPS - 1) / q40::tiled::RL_STEPS) * (N / 256);
   if (grid > 0x7fffffffLL) return Q40_E_SHAPE;
-  q40::tiled::relayout_kernel<<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>((const uint8_t*)bw, (const __half*)bs,
-                                                                              (uint8_t*)out, N, K);
+  q40::tiled::relayout_kernel<<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>((const uint8_t*)bw, (const __half*)bs, (uint8_t*)out,
+                                                                      N, K);
   Q40_LAUNCH_CHECK();
   return Q40_OK;
 }

@@ -9,6 +9,7 @@ There is no CPU path: a CPU tensor raises.
 from __future__ import annotations
 
 import math
+import weakref
 from typing import Optional, Sequence
 
 import torch
@@ -51,7 +52,8 @@ def _need_cuda(*ts: torch.Tensor) -> torch.device:
 
 
 def _stream(dev: torch.device) -> int:
-    return torch.cuda.current_stream(dev).cuda_stream
+    # the handle alone: a torch.cuda.Stream object costs more than the rest of a small call's checks
+    return torch._C._cuda_getCurrentRawStream(dev.index)
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -183,34 +185,18 @@ def matmul_q40(a: torch.Tensor, b_w: torch.Tensor, b_s: torch.Tensor, b_shape, *
     if M == 0:
         return c
     small = M <= 16 and group_size == 64 and K % 16 == 0 and K >= 64 and a.data_ptr() % 16 == 0 and c.stride(1) == 1
-    if small and N % 256 == 0 and (relayout if relayout is not None else _relayout_cfg["enabled"]):
+    wide = (M > 16 and group_size == 64 and N % 256 == 0 and K % 64 == 0 and a.data_ptr() % 16 == 0 and
+            c.stride(1) == 1 and c.stride(0) % 2 == 0 and c.data_ptr() % 4 == 0)
+    if (wide or (small and N % 256 == 0)) and (relayout if relayout is not None else _relayout_cfg["enabled"]):
         n_before = len(_relayout_cache)
         tiled = _tiled_copy_of(b_w, b_s, K, N)
         # programmatic launch (weights requested while the previous kernel drains) except right after the
         # kernel that wrote the copy
-        pdl = len(_relayout_cache) == n_before
-        if tiled is not None and (_tiled_gemv(dev, a, tiled, c, M, N, K, pdl) or
-                                  _stream_gemv(dev, a, tiled, c, M, N, K)):
+        if tiled is not None and (_tiled_matmul(dev, a, tiled, c, M, N, K, len(_relayout_cache) == n_before) or
+                                  (small and _stream_gemv(dev, a, tiled, c, M, N, K))):
             return c
     if small and N % 128 == 0 and _cluster_gemv(dev, a, b_w, b_s, c, M, N, K):
         return c
-    wide = (M > 16 and group_size == 64 and N % 256 == 0 and K % 64 == 0 and a.data_ptr() % 16 == 0 and
-            c.stride(1) == 1 and c.stride(0) % 2 == 0 and c.data_ptr() % 4 == 0)
-    if wide and (relayout if relayout is not None else _relayout_cfg["enabled"]):
-        n_before = len(_relayout_cache)
-        tiled = _tiled_copy_of(b_w, b_s, K, N)
-        if tiled is not None:
-            import ctypes
-            ws = _workspace("gemm", dev, 4096, zero=True)        # its last word is the error word of tc_error_flag()
-            P1 = ctypes.c_void_p * 1
-            rc = lib.q40_gemm_tiled_tc_multi(1, a.data_ptr(), a.stride(0), P1(tiled.data_ptr()), P1(c.data_ptr()),
-                                             (ctypes.c_int64 * 1)(c.stride(0)), (ctypes.c_int * 1)(N), M, K,
-                                             ws.data_ptr() + 4092, 1 if len(_relayout_cache) == n_before else 0,
-                                             _stream(dev))
-            if rc == 0:
-                return c
-            if rc != -5:        # Q40_E_UNSUPPORTED: no tensor-map encoder in this driver -> checkpoint layout
-                check(rc, "q40_gemm_tiled_tc_multi")
     nbytes = lib.q40_gemm_workspace_bytes(M, N, K)
     ws = _workspace("gemm", dev, nbytes, zero=True)
     check(lib.q40_gemm_kn(a.data_ptr(), a.stride(0), b_w.data_ptr(), b_s.data_ptr(), c.data_ptr(),
@@ -219,7 +205,7 @@ def matmul_q40(a: torch.Tensor, b_w: torch.Tensor, b_s: torch.Tensor, b_shape, *
     return c
 
 
-_cluster_size = {}      # device index -> largest cluster the device schedules for the decode matmul (16 or 8)
+_cluster_sizes = {}     # device index -> (largest cluster the device schedules for the decode matmul,): 16 or 8
 
 # tiled copies made for matmul_q40: id(b_w) -> (weakref to b_w, weakref to b_s, versions, (K, N), copy)
 _relayout_cfg = {"enabled": True, "max_bytes": 48 << 30}
@@ -253,7 +239,6 @@ def _versions(*ts):
 
 
 def _tiled_copy_of(b_w, b_s, K, N):
-    import weakref
     key = id(b_w)
     ent = _relayout_cache.get(key)
     if ent is not None:
@@ -279,20 +264,20 @@ def _tiled_copy_of(b_w, b_s, K, N):
     return copy
 
 
-def _tiled_gemv(dev, a, tiled, c, M, N, K, pdl=False) -> bool:
-    """Mode 0 of q40_gemv_tiled (cluster split-K) on a tiled copy; False if this device cannot schedule
-    the clusters."""
-    import ctypes
-    P = ctypes.c_void_p * 1
-    for cluster in ((_cluster_size.get(dev.index, 16),) if dev.index in _cluster_size else (16, 8)):
-        rc = lib.q40_gemv_tiled(0, 1, P(tiled.data_ptr()), P(0), P(c.data_ptr()), (ctypes.c_int * 1)(N), c.stride(0),
-                                a.data_ptr(), a.stride(0), M, K, None, None, 0, 0.0, None, 0, None, 0, cluster,
-                                1 if pdl else 0, _stream(dev))
+def _tiled_matmul(dev, a, tiled, c, M, N, K, pdl) -> bool:
+    """q40_matmul_tiled on a tiled copy; False if this device cannot schedule the clusters (up to 16 rows) or its
+    driver has no tensor-map encoder (above)."""
+    # the error word of tc_error_flag(); the narrow kernel has no wait that could expire
+    err = _workspace("gemm", dev, 4096, zero=True).data_ptr() + 4092 if M > 16 else None
+    for cluster in (_cluster_sizes.get(dev.index) or (16, 8)):
+        rc = lib.q40_matmul_tiled(tiled.data_ptr(), c.data_ptr(), c.stride(0), a.data_ptr(), a.stride(0), M, N, K, cluster,
+                                  err, 1 if pdl else 0, _stream(dev))
         if rc == 0:
-            _cluster_size[dev.index] = cluster
+            if M <= 16:
+                _cluster_sizes[dev.index] = (cluster,)
             return True
-        if rc > 0:
-            check(rc, "q40_gemv_tiled")
+        if rc > 0 or (M > 16 and rc != -5):      # -5: Q40_E_UNSUPPORTED
+            check(rc, "q40_matmul_tiled")
     return False
 
 
@@ -318,12 +303,12 @@ def _cluster_gemv(dev, a, b_w, b_s, c, M, N, K) -> bool:
     the workspace kernel behind q40_gemm_kn.  False if the launch was refused for this shape."""
     import ctypes
     P = ctypes.c_void_p * 1
-    for cluster in ((_cluster_size.get(dev.index, 16),) if dev.index in _cluster_size else (16, 8)):
+    for cluster in (_cluster_sizes.get(dev.index) or (16, 8)):
         rc = lib.q40_gemv_fused(0, 1, P(b_w.data_ptr()), P(b_s.data_ptr()), P(c.data_ptr()), (ctypes.c_int * 1)(N),
                                 c.stride(0), a.data_ptr(), a.stride(0), M, K, None, None, 0, 0.0, None, 0, None, 0,
                                 cluster, 0, _stream(dev))
         if rc == 0:
-            _cluster_size[dev.index] = cluster
+            _cluster_sizes[dev.index] = (cluster,)
             return True
         if rc > 0:
             check(rc, "q40_gemv_fused")
