@@ -44,18 +44,16 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
 }
 
 // Sum of one element over the split-K partials, in split order (so the result does not depend
-// on which CTA arrives last) but with eight L2 loads in flight at a time.
+// on which CTA arrives last) but with eight L2 loads in flight at a time, the last batch included.
 __device__ __forceinline__ float sum_partials(const float* __restrict__ p, int stride, int nsplit) {
   float v = 0.f;
-  int sp = 0;
-  for (; sp + 8 <= nsplit; sp += 8) {
+  for (int sp = 0; sp < nsplit; sp += 8) {
     float t[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) t[i] = __ldcg(p + (int64_t)(sp + i) * stride);
+    for (int i = 0; i < 8; ++i) t[i] = sp + i < nsplit ? __ldcg(p + (int64_t)(sp + i) * stride) : 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) v += t[i];
   }
-  for (; sp < nsplit; ++sp) v += __ldcg(p + (int64_t)sp * stride);
   return v;
 }
 
@@ -356,19 +354,21 @@ __device__ __forceinline__ void nk_compute(float (&acc)[MT][4], const NkRegs& r,
   }
 }
 
+// MT: 8-row tiles of the batch per launch, up to 8 (a 16-row limit read the weights M/16 times); the activations
+// are staged xch k rows at a time (a multiple of DEPTH steps, or the whole k range).
 template <int G, int MT>
-__global__ void __launch_bounds__(GEMV_THREADS, 4)
+__global__ void __launch_bounds__(GEMV_THREADS, MT <= 2 ? 5 : 3)
 gemv_nk_kernel(const __half* __restrict__ X, int64_t ldx, const uint8_t* __restrict__ wq,
                const __half* __restrict__ ws, __half* __restrict__ Y, int64_t ldy, int M, int N, int K,
-               int kchunk, float* __restrict__ part, unsigned int* __restrict__ counters) {
+               int kchunk, int xch, float* __restrict__ part, unsigned int* __restrict__ counters) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __half* xs = reinterpret_cast<__half*>(smem_raw);   // [MT*8][kchunk + pad], order x0,x2,x1,x3
+  __half* xs = reinterpret_cast<__half*>(smem_raw);   // [MT*8][xch + pad], order x0,x2,x1,x3
   __shared__ unsigned int ticket_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int nblk = blockIdx.x, split = blockIdx.y, nsplit = gridDim.y;
   const int kb = split * kchunk, ke = min(K, kb + kchunk);
-  const int xs_ld = kchunk + NK_XS_PAD;
+  const int xs_ld = xch + NK_XS_PAD;
   const int n0 = nblk * NK_ROWS + warp * 16 + g, n1 = n0 + 8;
   const bool ok0 = n0 < N, ok1 = n1 < N;
   const int64_t w_ld = K / 2, s_ld = K / G;
@@ -385,17 +385,18 @@ gemv_nk_kernel(const __half* __restrict__ X, int64_t ldx, const uint8_t* __restr
   for (int d = 0; d < DEPTH; ++d)
     if (d < nsteps) nk_load<G>(regs[d], w0, w1, s0, s1, cb0 + d * NK_STEP_BYTES, ok0, ok1);
 
-  for (int idx = tid; idx < MT * 8 * (kchunk / 4); idx += GEMV_THREADS) {
-    const int m = idx / (kchunk / 4), kk = (idx % (kchunk / 4)) * 4;
-    uint2 v = make_uint2(0, 0);
-    if (m < M && kb + kk < ke) {
-      const uint2 raw = *reinterpret_cast<const uint2*>(X + (int64_t)m * ldx + kb + kk);  // x0 x1 | x2 x3
-      v.x = prmt(raw.x, raw.y, 0x5410);   // x0 x2
-      v.y = prmt(raw.x, raw.y, 0x7632);   // x1 x3
+  auto stage = [&](int k0) {
+    for (int idx = tid; idx < MT * 8 * (xch / 4); idx += GEMV_THREADS) {
+      const int m = idx / (xch / 4), kk = (idx % (xch / 4)) * 4;
+      uint2 v = make_uint2(0, 0);
+      if (m < M && k0 + kk < ke) {
+        const uint2 raw = *reinterpret_cast<const uint2*>(X + (int64_t)m * ldx + k0 + kk);  // x0 x1 | x2 x3
+        v.x = prmt(raw.x, raw.y, 0x5410);   // x0 x2
+        v.y = prmt(raw.x, raw.y, 0x7632);   // x1 x3
+      }
+      *reinterpret_cast<uint2*>(xs + m * xs_ld + kk) = v;
     }
-    *reinterpret_cast<uint2*>(xs + m * xs_ld + kk) = v;
-  }
-  __syncthreads();
+  };
 
   float acc[MT][4];
 #pragma unroll
@@ -405,12 +406,19 @@ gemv_nk_kernel(const __half* __restrict__ X, int64_t ldx, const uint8_t* __restr
 
   // position of this lane's first high-nibble k inside a step: byte 16t of the step -> k offset
   const int koff = 2 * G * ((16 * t) / G) + (16 * t) % G;
+  const int xsteps = xch / NK_STEP_K;
   const __half* xlane = xs + g * xs_ld + koff;
-  for (int s = 0; s < nsteps; s += DEPTH) {
+  for (int s = 0, c0 = 0; s < nsteps; s += DEPTH) {
+    if (s == 0 || s - c0 >= xsteps) {
+      if (s) __syncthreads();               // every warp is done with the previous piece
+      c0 = s;
+      stage(kb + s * NK_STEP_K);
+      __syncthreads();
+    }
 #pragma unroll
     for (int d = 0; d < DEPTH; ++d) {
       if (s + d < nsteps) {
-        nk_compute<G, MT>(acc, regs[d], xlane + (s + d) * NK_STEP_K, xs_ld);
+        nk_compute<G, MT>(acc, regs[d], xlane + (s - c0 + d) * NK_STEP_K, xs_ld);
         if (s + d + DEPTH < nsteps)
           nk_load<G>(regs[d], w0, w1, s0, s1, cb0 + (s + d + DEPTH) * NK_STEP_BYTES, ok0, ok1);
       }
@@ -456,21 +464,33 @@ gemv_nk_kernel(const __half* __restrict__ X, int64_t ldx, const uint8_t* __restr
 
 struct NkPlan {
   int nblocks, nsplit, kchunk;
-  size_t smem_bytes(int MT) const { return ((size_t)MT * 8 * (kchunk + NK_XS_PAD) * 2 + 15) & ~(size_t)15; }
 };
 
+// One wave: five CTAs of 128 threads fit an SM, and a few CTAs more than that would cost a second pass
+// (11008 x 4096 at 10 rows, 688 CTAs: 23.9 us with four per SM).
 static NkPlan plan_nk(int N, int K) {
   NkPlan p;
   p.nblocks = (N + NK_ROWS - 1) / NK_ROWS;
-  int want = (148 * 4 + p.nblocks - 1) / p.nblocks;
+  int want = 148 * 5 / p.nblocks;
   if (want < 1) want = 1;
   int kchunk = (K + want - 1) / want;
   kchunk = ((kchunk + NK_STEP_K - 1) / NK_STEP_K) * NK_STEP_K;
   if (kchunk < 256) kchunk = 256;
-  if (kchunk > 2048) kchunk = 2048;
   if (kchunk > K) kchunk = K;
   p.kchunk = kchunk;
   p.nsplit = (K + kchunk - 1) / kchunk;
+  return p;
+}
+
+// The same for a launch of up to 8 mt > 16 rows: fewer splits, so that the partial sums need no more scratch
+// than those of 16 rows.
+static NkPlan plan_nk_rows(int N, int K, int mt) {
+  NkPlan p = plan_nk(N, K);
+  if (mt > 2) {
+    const int want = p.nsplit * 2 / mt > 1 ? p.nsplit * 2 / mt : 1;
+    p.kchunk = ((K + want - 1) / want + NK_STEP_K - 1) / NK_STEP_K * NK_STEP_K;
+    p.nsplit = (K + p.kchunk - 1) / p.kchunk;
+  }
   return p;
 }
 
@@ -556,9 +576,11 @@ extern "C" int q40_gemm_kn(const void* a, int64_t lda, const void* bw, const voi
 
 template <int G, int MT>
 static int launch_gemv_nk(const __half* x, int64_t ldx, const uint8_t* wq, const __half* ws, __half* y,
-                          int64_t ldy, int M, int N, int K, const q40::NkPlan& p, void* workspace,
-                          cudaStream_t st) {
-  const size_t smem = p.smem_bytes(MT);
+                          int64_t ldy, int M, int N, int K, void* workspace, cudaStream_t st) {
+  const q40::NkPlan p = q40::plan_nk_rows(N, K, MT);
+  const int xmax = MT <= 2 ? 1024 : 512;        // 33 to 66 KB: what lets the CTAs of a wave share the SMs
+  const int xch = p.kchunk < xmax ? p.kchunk : xmax;
+  const size_t smem = ((size_t)MT * 8 * (xch + q40::NK_XS_PAD) * 2 + 15) & ~(size_t)15;
   auto kern = q40::gemv_nk_kernel<G, MT>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -566,7 +588,7 @@ static int launch_gemv_nk(const __half* x, int64_t ldx, const uint8_t* wq, const
   }
   dim3 grid(p.nblocks, p.nsplit);
   kern<<<grid, q40::GEMV_THREADS, smem, st>>>(
-      x, ldx, wq, ws, y, ldy, M, N, K, p.kchunk,
+      x, ldx, wq, ws, y, ldy, M, N, K, p.kchunk, xch,
       reinterpret_cast<float*>((char*)workspace + q40::COUNTER_BYTES),
       reinterpret_cast<unsigned int*>(workspace));
   Q40_LAUNCH_CHECK();
@@ -595,21 +617,18 @@ extern "C" int q40_gemm_nk(const void* x, int64_t ldx, const void* wq, const voi
   cudaStream_t st = (cudaStream_t)stream;
   const __half* xh = (const __half*)x;
   __half* yh = (__half*)y;
-  for (int m0 = 0; m0 < M; m0 += 16) {
-    const int mc = (M - m0) < 16 ? (M - m0) : 16;
+  for (int m0 = 0; m0 < M;) {
+    const int left = M - m0, mc = left < 64 ? left : 64;
+    auto run = [&](auto launch) {
+      return launch(xh + m0 * ldx, ldx, (const uint8_t*)wq, (const __half*)ws, yh + m0 * ldy, ldy, mc, N, K, workspace, st);
+    };
     int rc;
-    if (group == 64) {
-      rc = (mc <= 8) ? launch_gemv_nk<64, 1>(xh + m0 * ldx, ldx, (const uint8_t*)wq, (const __half*)ws,
-                                            yh + m0 * ldy, ldy, mc, N, K, p, workspace, st)
-                     : launch_gemv_nk<64, 2>(xh + m0 * ldx, ldx, (const uint8_t*)wq, (const __half*)ws,
-                                            yh + m0 * ldy, ldy, mc, N, K, p, workspace, st);
-    } else {
-      rc = (mc <= 8) ? launch_gemv_nk<32, 1>(xh + m0 * ldx, ldx, (const uint8_t*)wq, (const __half*)ws,
-                                            yh + m0 * ldy, ldy, mc, N, K, p, workspace, st)
-                     : launch_gemv_nk<32, 2>(xh + m0 * ldx, ldx, (const uint8_t*)wq, (const __half*)ws,
-                                            yh + m0 * ldy, ldy, mc, N, K, p, workspace, st);
-    }
+    if (mc <= 8) rc = group == 64 ? run(launch_gemv_nk<64, 1>) : run(launch_gemv_nk<32, 1>);
+    else if (mc <= 16) rc = group == 64 ? run(launch_gemv_nk<64, 2>) : run(launch_gemv_nk<32, 2>);
+    else if (mc <= 32) rc = group == 64 ? run(launch_gemv_nk<64, 4>) : run(launch_gemv_nk<32, 4>);
+    else rc = group == 64 ? run(launch_gemv_nk<64, 8>) : run(launch_gemv_nk<32, 8>);
     if (rc != Q40_OK) return rc;
+    m0 += mc;
   }
   return Q40_OK;
 }
