@@ -105,6 +105,57 @@ __device__ __forceinline__ __half2 codes_hi_to_h2(uint32_t p) {
   return __hfma2(u32_as_h2(v), u32_as_h2(0x2C002C00u) /* 1/16 */, u32_as_h2(0xD480D480u) /* -72 */);
 }
 
+// The format's fp16(w / scale) without a division per element.  w and s are fp16: write w = A 2^i, s = S 2^j with
+// integers A, S < 2^11.  An fp16 rounding boundary of the quotient is M 2^g with an odd 12-bit M, and
+// A/S = M 2^h has no solution (S M has more significant bits than A), so |A 2^h' - S M| >= 1 and the quotient stays
+// at least 1 / (2047 * 4095) = 2^-23 * 1.0007 away from every boundary, relatively.  fl(w * fl(1/s)) in fp32 is at
+// most 2^-23 + 2^-48 off.  So it lies on the quotient's side of the boundary and rounds to the same fp16 value.
+// (Quotients below the normal fp16 range round to a code of 0 either way.)
+// x + 1536 in fp16 then rounds to the nearest integer, ties to even, and leaves the two's complement code in the low
+// bits; the clamp makes NaN and infinite quotients (NaN loses against a number in min/max) leave 0 there, which
+// is what the x86 float->int conversion of the reference makes of them.
+__device__ __forceinline__ uint32_t quant_pair(uint32_t w2, float inv) {
+  const float2 f = __half22float2(u32_as_h2(w2));
+  __half2 h = __floats2half2_rn(f.x * inv, f.y * inv);
+  h = __hmin2(__hmax2(h, u32_as_h2(0xE000E000u)), u32_as_h2(0x60006000u));   // [-512, 512]
+  return h2_as_u32(__hadd2(h, u32_as_h2(0x66006600u)));                      // 1536 + code
+}
+
+// Eight values of a pair's even group and the same of its odd group: their (even, odd) maxima.  max drops NaN like
+// torch.max would not, but NaN inputs are outside the format.
+__device__ __forceinline__ __half2 quant_max(const uint32_t (&ew)[4], const uint32_t (&ow)[4]) {
+  __half2 ae = __habs2(u32_as_h2(ew[0])), ao = __habs2(u32_as_h2(ow[0]));
+#pragma unroll
+  for (int i = 1; i < 4; ++i) {
+    ae = __hmax2(ae, __habs2(u32_as_h2(ew[i])));
+    ao = __hmax2(ao, __habs2(u32_as_h2(ow[i])));
+  }
+  return __hmax2(__lows2half2(ae, ao), __highs2half2(ae, ao));
+}
+
+// ... and, with the maxima m over the whole groups, their 8 finished bytes and the two scales
+__device__ __forceinline__ uint2 quant_codes(const uint32_t (&ew)[4], const uint32_t (&ow)[4], __half2 m, __half2& sc) {
+  const float me = fmaxf(0.f, __low2float(m)), mo = fmaxf(0.f, __high2float(m));    // all-NaN group: 0
+  // scale = fp16(absmax / 7): fp32 division, one rounding to fp16
+  const __half se = __float2half_rn(__fdiv_rn(me, 7.0f)), so = __float2half_rn(__fdiv_rn(mo, 7.0f));
+  // a scale of zero makes every code 0 (x/0 and 0/0 both do)
+  const float fe = __half2float(se), fo = __half2float(so);
+  const float ie = fe > 0.f ? __frcp_rn(fe) : 0.f, io = fo > 0.f ? __frcp_rn(fo) : 0.f;
+  uint32_t out[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    uint32_t b[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t ce = quant_pair(ew[2 * k + i], ie), co = quant_pair(ow[2 * k + i], io);
+      b[i] = ((ce << 4) & 0x00F000F0u) | (co & 0x000F000Fu);      // bytes 0 and 2 of the word
+    }
+    out[k] = prmt(b[0], b[1], 0x6420);
+  }
+  sc = __halves2half2(se, so);
+  return make_uint2(out[0], out[1]);
+}
+
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
