@@ -579,8 +579,11 @@ gemm_tiled_wide_kernel(const Params p, const __grid_constant__ CUtensorMap amap)
     const unsigned char* lane_s = gbase + 1024 + q * 32 + t * 8;
     for (int i = dset; i < nblk; i += DSETS) {
       const int s = i % S, ab = i % NA;
+      // block i - S first: its MMAs free this block's A buffer (S <= NA), and the full barrier, which tells only odd
+      // from even phases, has then left the phase of block i - S (the copies of different blocks land in any order)
+      const int w = i - S;
+      if (w >= 0 && !mbar_wait(bar_mdone + 8 * (w % NA), (uint32_t)((w / NA) & 1))) { failed = true; break; }
       if (!mbar_wait(bar_full + 8 * s, (uint32_t)((i / S) & 1))) { failed = true; break; }
-      if (i >= NA && !mbar_wait(bar_mdone + 8 * ab, (uint32_t)((i / NA - 1) & 1))) { failed = true; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const size_t so = (size_t)s * stage_bytes;
       uint32_t r[2][16];
