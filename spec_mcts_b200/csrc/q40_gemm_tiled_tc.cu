@@ -69,6 +69,13 @@ struct Params {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// One lane of a converged warp, chosen so that the compiler knows the branch to be taken by a single thread: operands
+// of copies and MMAs issued under `lane == 0` go through a loop that moves them to uniform registers.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
+  return pred != 0;
+}
 // K-major operand with 128-byte swizzle: rows of 128 bytes, groups of 8 rows 1024 bytes apart
 __device__ __forceinline__ uint64_t kmajor_desc(uint32_t saddr) {
   uint64_t d = 0;
@@ -258,7 +265,7 @@ gemm_tiled_tc_kernel(const Params p, const __grid_constant__ CUtensorMap amap) {
   bool failed = false;
   if (warp == 0) {
     // ================= the copy thread: weights and activations of block i into stage i % S =================
-    if (lane == 0) {
+    if (elect_one()) {
       const int ksteps = p.K / 16;
       const uint8_t* src = p.bw[pi] + ((int64_t)span * ksteps + kb / 16) * STEP_BYTES;
       // the weights do not depend on the previous launch: the first stages are requested before this
@@ -288,7 +295,7 @@ gemm_tiled_tc_kernel(const Params p, const __grid_constant__ CUtensorMap amap) {
     }
     __syncwarp();
   } else if (warp < DQ_WARP0 || warp >= DQ_WARP0 + DQ_WARPS) {
-    // ================= the four MMA warps: lane 0 issues, the warp stays converged =================
+    // ================= the four MMA warps: one elected thread each =================
     // Per k block an issuing warp spends ~800 cycles on fixed latencies (mbarrier test, fences, commit) and
     // 60-120 per tcgen05.mma, whatever the tile size, so one thread cannot feed eight small MMAs per k block.
     // Warp (hh, set) issues the four k steps of feature half hh for the k blocks of its set (even or odd).
@@ -305,21 +312,18 @@ gemm_tiled_tc_kernel(const Params p, const __grid_constant__ CUtensorMap amap) {
     const uint32_t idesc = (1u << 4) | ((uint32_t)(p.Mpad >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     TTC_ROLE_DECL
-    for (int i = mset; i < nblk && !failed; i += 2) {
-      const int s = i % S, ab = i % NA;
-      TTC_ROLE(1, i, 0);
-      if (!mbar_wait(bar_afull + 8 * ab, (uint32_t)((i / NA) & 1))) { failed = true; break; }
-      TTC_ROLE(1, i, 1);
-      int ok = 1;
-      if (lane == 0 && !p.split_acc) {
-        unsigned spins = 0;
-        while (s_issued[hh] != i && ++spins < (SPIN_LIMIT << 4)) { }
-        ok = s_issued[hh] == i;
-      }
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (!ok) { failed = true; break; }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (lane == 0) {
+    if (elect_one()) {
+      for (int i = mset; i < nblk; i += 2) {
+        const int s = i % S, ab = i % NA;
+        TTC_ROLE(1, i, 0);
+        if (!mbar_wait(bar_afull + 8 * ab, (uint32_t)((i / NA) & 1))) { failed = true; break; }
+        TTC_ROLE(1, i, 1);
+        if (!p.split_acc) {
+          unsigned spins = 0;
+          while (s_issued[hh] != i && ++spins < (SPIN_LIMIT << 4)) { }
+          if (s_issued[hh] != i) { failed = true; break; }
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint64_t bd0 = kmajor_desc(ring + s * stage_bytes + RAW_PAD);
         const uint32_t a0 = tmem + A_COL0 + ab * 64 + hh * 32;
 #pragma unroll
@@ -330,11 +334,10 @@ gemm_tiled_tc_kernel(const Params p, const __grid_constant__ CUtensorMap amap) {
         s_issued[hh] = i + 1;
         TTC_ROLE(1, i, 3);
         commit(bar_mdone + 8 * s);                  // the stage and the A buffer may be refilled when the MMAs
-      }                                             // of both accumulators are done
-      TTC_ROLE(1, i, 6);
-      __syncwarp();
+        TTC_ROLE(1, i, 6);                          // of both accumulators are done
+      }
+      if (!failed) commit(bar_done);                // all of this thread's MMAs
     }
-    if (lane == 0 && !failed) commit(bar_done);     // all of this thread's MMAs
     __syncwarp();
     if (warp == 1) TTC_ROLE_FLUSH(312);
   } else {
@@ -522,7 +525,7 @@ gemm_tiled_wide_kernel(const Params p, const __grid_constant__ CUtensorMap amap)
 
   bool failed = false;
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const int ksteps = p.K / 16;
       const uint8_t* src = p.bw[pi] + ((int64_t)span * ksteps + kb / 16) * STEP_BYTES;
       auto weights = [&](int i, int s) {
@@ -554,12 +557,12 @@ gemm_tiled_wide_kernel(const Params p, const __grid_constant__ CUtensorMap amap)
     __syncwarp();
   } else if (warp == 1) {
     const uint32_t idesc = (1u << 4) | ((uint32_t)(p.Mpad >> 3) << 17) | ((uint32_t)(FEATS >> 4) << 24);
-    for (int i = 0; i < nblk; ++i) {
-      const int ab = i % NA;
-      // the dequantisers' arrival also covers the stage's copies, which they waited for
-      if (!mbar_wait(bar_afull + 8 * ab, (uint32_t)((i / NA) & 1))) { failed = true; break; }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (lane == 0) {
+    if (elect_one()) {
+      for (int i = 0; i < nblk; ++i) {
+        const int ab = i % NA;
+        // the dequantisers' arrival also covers the stage's copies, which they waited for
+        if (!mbar_wait(bar_afull + 8 * ab, (uint32_t)((i / NA) & 1))) { failed = true; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint64_t bd0 = kmajor_desc(ring + (i % S) * stage_bytes + RAW_PAD);
 #pragma unroll
         for (int ks = 0; ks < BK / 16; ++ks)
@@ -567,9 +570,8 @@ gemm_tiled_wide_kernel(const Params p, const __grid_constant__ CUtensorMap amap)
                  (i > 0 || ks > 0) ? 1u : 0u);
         commit(bar_mdone + 8 * ab);
       }
-      __syncwarp();
+      if (!failed) commit(bar_done);
     }
-    if (lane == 0 && !failed) commit(bar_done);
     __syncwarp();
   } else if (warp >= DQ_WARP0) {
     // warp = (set, quadrant): 32 feature rows = two 16-row tiles of one 64-column group, see above
