@@ -1,8 +1,9 @@
 // Decode attention for one query token per branch over that branch's own keys: a
 // contiguous [B,Hkv,L,D] cache or a paged pool.  One CTA per (branch, query head).
 //
-// Eight lanes share a key: each lane owns 16 of the 128 head dims (two 16-byte loads of K,
-// two of V), the partial dot products are summed with three shuffles, and every group of
+// Eight lanes share a key: lane i owns dims 8i..8i+7 and 64+8i..64+8i+7 of the head (two 16-byte loads of K, two of
+// V, each of which covers 128 contiguous bytes over the lanes; in the Q4_0 cache the same dims are the two
+// nibbles of 8 bytes), the partial dot products are summed with three shuffles, and every group of
 // eight lanes keeps its own online-softmax state (running max, sum, 16 output dims) in
 // fp32.  The 16 groups of a CTA are merged through shared memory at the end; the same
 // merge can fold in partial results of a shared-prefix pass (see attn_prefix.cu), which is
@@ -17,57 +18,77 @@
 
 namespace q40 {
 
-constexpr int BR_THREADS = 128;
-constexpr int BR_GROUPS = BR_THREADS / 8;   // key groups per CTA
-constexpr int BR_UNROLL = 4;                // keys per group per iteration
+// Page ids are looked up one iteration ahead of the keys they lead to, and the shared-prefix pass's row maxima
+// and sums before the key loop, so that an iteration waits for one memory latency and not for two.
+//
+// A CTA has NW warps; WPR of them share a row (branch, head).  What bounds a row is latency (ids -> keys -> sums
+// -> merge), so the split is the one that keeps the warps of all rows resident at once: see launch_branch.
 
-
-template <int MODE>  // 0 contiguous, 1 paged with int16 ids, 2 paged with int32 ids
-__device__ __forceinline__ int64_t key_slot(const BranchArgs& a, int b, int hk, int t) {
-  if (MODE == 0 || MODE == 3) {
-    return ((int64_t)(b * a.Hkv + hk) * a.L + t);
-  } else {
-    const int pg = t / a.page_size, in = t - pg * a.page_size;
-    int64_t id;
-    if (MODE == 1)
-      id = (int64_t)(uint16_t) reinterpret_cast<const int16_t*>(a.tbl)[(int64_t)b * a.tbl_stride + pg];
-    else
-      id = (int64_t) reinterpret_cast<const int32_t*>(a.tbl)[(int64_t)b * a.tbl_stride + pg];
-    int64_t slot = id * a.page_size + in;
-    // a bad page id must not turn into a wild read: clamp into the pool
-    if (slot < 0) slot = 0;
-    if (slot >= a.P) slot = a.P - 1;
-    return (int64_t)hk * a.P + slot;
-  }
+// Slot of key t of branch b: in the pool (paged), or just t (contiguous)
+template <int MODE>  // 0 contiguous, 1 paged with int16 ids, 2 paged with int32 ids, 3 Q4_0 cache
+__device__ __forceinline__ int key_slot(const BranchArgs& a, int b, int t) {
+  if (MODE == 0 || MODE == 3) return t;
+  const int pg = t / a.page_size, in = t - pg * a.page_size;
+  int64_t id;
+  if (MODE == 1)
+    id = (int64_t)(uint16_t) reinterpret_cast<const int16_t*>(a.tbl)[(int64_t)b * a.tbl_stride + pg];
+  else
+    id = (int64_t) reinterpret_cast<const int32_t*>(a.tbl)[(int64_t)b * a.tbl_stride + pg];
+  const int64_t slot = id * a.page_size + in;
+  // a bad page id must not turn into a wild read: clamp into the pool
+  return (int)min(max(slot, (int64_t)0), (int64_t)a.P - 1);
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(BR_THREADS)
+// a row's two scales in one word
+__device__ __forceinline__ uint32_t load_scales(const __half* p, bool aligned4) {
+  if (aligned4) return __ldg(reinterpret_cast<const uint32_t*>(p));
+  return h2_as_u32(__halves2half2(__ldg(p), __ldg(p + 1)));
+}
+
+template <int MODE, int NW, int WPR, int U>    // U: keys per 8-lane group in flight
+__global__ void __launch_bounds__(NW * 32, U > 2 ? 16 / NW : NW == 8 ? 3 : 5)
 attn_branch_kernel(const BranchArgs a) {
   constexpr int D = ATTN_D;
+  constexpr int RT = WPR * 32;                // threads of a row
+  constexpr int NG = WPR * 4;                 // key groups of a row
   asm volatile("griddepcontrol.launch_dependents;");   // a dependent may start prefetching its weights
   asm volatile("griddepcontrol.wait;" ::: "memory");               // ... but nothing of the previous launch is read before it is done
-  const int bh = blockIdx.x;
-  const int b = bh / a.H, h = bh % a.H;
-  const int hk = h / (a.H / a.Hkv);
   const int tid = threadIdx.x, lane = tid & 31;
-  const int grp = tid >> 3, sub = tid & 7;
+  const int slot = (NW == WPR) ? 0 : (tid >> 5) / WPR;      // row of this CTA
+  const int64_t bh = (int64_t)blockIdx.x * (NW / WPR) + slot;
+  const int64_t rows = a.rows;
+  if (bh >= rows) return;                     // whole warps; rows of a CTA meet at no barrier unless NW == WPR
+  const int b = (int)(bh / a.H), h = (int)(bh % a.H);
+  const int hk = h / (a.H / a.Hkv);
+  const int tr = tid - slot * RT;             // thread of the row
+  const int grp = tr >> 3, sub = tid & 7;
   // the 8 lanes that share a key; groups of one warp may run different numbers of iterations,
   // so every shuffle names only its own group
   const unsigned gmask = 0xffu << (lane & 24);
+
+  // first page ids: table entries up to L exist whatever the branch's length is
+  int slots[U];
+  if (MODE == 1 || MODE == 2) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) slots[u] = (grp + u * NG < a.L) ? key_slot<MODE>(a, b, grp + u * NG) : 0;
+  }
   int len;
   if (MODE == 3) len = min(max(a.pos[b] - a.prefix_len[0], 0), a.max_t);
   else len = a.seq_lens ? min(max(a.seq_lens[b], 0), a.L) : a.L;
 
-  __shared__ float sm_m[BR_GROUPS], sm_l[BR_GROUPS];
-  __shared__ __align__(16) float sm_o[BR_GROUPS][D];
+  // prefix partials: lane sp holds the maximum and the sum of split sp (further splits are read at the merge)
+  const float pm_l = lane < a.nsp ? a.pm[(int64_t)lane * rows + bh] : -CUDART_INF_F;
+  const float pl_l = lane < a.nsp ? a.pl[(int64_t)lane * rows + bh] : 0.f;
+
+  __shared__ float sm_m[NW * 4], sm_l[NW * 4];
+  __shared__ __align__(16) float sm_o[NW * 4][D];
 
   // this lane's 16 query dims, pre-multiplied by scale*log2(e)
   float qf[16];
   {
-    const __half* qp = a.q + (int64_t)b * a.q_stride + h * D + sub * 16;
+    const __half* qp = a.q + (int64_t)b * a.q_stride + h * D + sub * 8;
     const uint4 q0 = *reinterpret_cast<const uint4*>(qp);
-    const uint4 q1 = *reinterpret_cast<const uint4*>(qp + 8);
+    const uint4 q1 = *reinterpret_cast<const uint4*>(qp + 64);
     const __half2* h0 = reinterpret_cast<const __half2*>(&q0);
     const __half2* h1 = reinterpret_cast<const __half2*>(&q1);
 #pragma unroll
@@ -83,26 +104,35 @@ attn_branch_kernel(const BranchArgs a) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) o[i] = 0.f;
 
+  // first key of this head and branch, at this lane's dims
+  const int64_t kv0 = (MODE == 0 ? (int64_t)(b * a.Hkv + hk) * a.L : (int64_t)hk * a.P) * D + sub * 8;
   if (MODE != 3)
-  for (int t0 = grp; t0 < len; t0 += BR_GROUPS * BR_UNROLL) {
-    uint4 kv[BR_UNROLL][4];
-    float s[BR_UNROLL];
+  for (int t0 = grp; t0 < len; t0 += NG * U) {
+    uint4 kv[U][4];
+    float s[U];
 #pragma unroll
-    for (int u = 0; u < BR_UNROLL; ++u) {
-      const int t = t0 + u * BR_GROUPS;
+    for (int u = 0; u < U; ++u) {
+      const int t = t0 + u * NG;
       if (t < len) {
-        const int64_t off = key_slot<MODE>(a, b, hk, t) * D + sub * 16;
+        const int64_t off = kv0 + (int64_t)(MODE == 0 ? t : slots[u]) * D;
         kv[u][0] = __ldg(reinterpret_cast<const uint4*>(a.k + off));
-        kv[u][1] = __ldg(reinterpret_cast<const uint4*>(a.k + off + 8));
+        kv[u][1] = __ldg(reinterpret_cast<const uint4*>(a.k + off + 64));
         kv[u][2] = __ldg(reinterpret_cast<const uint4*>(a.v + off));
-        kv[u][3] = __ldg(reinterpret_cast<const uint4*>(a.v + off + 8));
+        kv[u][3] = __ldg(reinterpret_cast<const uint4*>(a.v + off + 64));
       } else {
         kv[u][0] = kv[u][1] = kv[u][2] = kv[u][3] = make_uint4(0, 0, 0, 0);
       }
     }
+    if (MODE == 1 || MODE == 2) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int t = t0 + (U + u) * NG;
+        slots[u] = (t < len) ? key_slot<MODE>(a, b, t) : 0;
+      }
+    }
     float mnew = m;
 #pragma unroll
-    for (int u = 0; u < BR_UNROLL; ++u) {
+    for (int u = 0; u < U; ++u) {
       const __half2* kh = reinterpret_cast<const __half2*>(&kv[u][0]);  // 8 half2 = 16 dims
       float acc = 0.f;
 #pragma unroll
@@ -114,7 +144,7 @@ attn_branch_kernel(const BranchArgs a) {
       acc += __shfl_xor_sync(gmask, acc, 1);
       acc += __shfl_xor_sync(gmask, acc, 2);
       acc += __shfl_xor_sync(gmask, acc, 4);
-      s[u] = (t0 + u * BR_GROUPS < len) ? acc : -CUDART_INF_F;
+      s[u] = (t0 + u * NG < len) ? acc : -CUDART_INF_F;
       mnew = fmaxf(mnew, s[u]);
     }
     // t0 < len, so mnew is finite here
@@ -123,7 +153,7 @@ attn_branch_kernel(const BranchArgs a) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) o[i] *= corr;
 #pragma unroll
-    for (int u = 0; u < BR_UNROLL; ++u) {
+    for (int u = 0; u < U; ++u) {
       const float p = exp2f(s[u] - mnew);
       l += p;
       const __half2* vh = reinterpret_cast<const __half2*>(&kv[u][2]);
@@ -138,47 +168,51 @@ attn_branch_kernel(const BranchArgs a) {
   }
 
   if (MODE == 3) {
-    // Q4_0 cache: lane `sub` owns dims 16*sub..16*sub+15 = nibble half (sub>>2) of bytes 16*(sub&3)..+15
-    const int nib_lo = sub >> 2;                 // 0: high nibbles (dims 0..63), 1: low nibbles
-    const int boff = 16 * (sub & 3);
-    for (int t0 = grp; t0 < len; t0 += BR_GROUPS * BR_UNROLL) {
-      uint4 kb[BR_UNROLL], vb[BR_UNROLL];
-      __half ksv[BR_UNROLL], vsv[BR_UNROLL];
-      float s[BR_UNROLL];
+    // Q4_0 cache: lane `sub` owns bytes 8*sub..8*sub+7 of a row, both nibbles
+    const bool sc4 = (((uintptr_t)a.ksc | (uintptr_t)a.vsc) & 3) == 0;
+    for (int t0 = grp; t0 < len; t0 += NG * U) {
+      uint2 kb[U], vb[U];
+      uint32_t ksv[U], vsv[U];
+      float s[U];
 #pragma unroll
-      for (int u = 0; u < BR_UNROLL; ++u) {
-        const int t = t0 + u * BR_GROUPS;
+      for (int u = 0; u < U; ++u) {
+        const int t = t0 + u * NG;
         if (t < len) {
           const int64_t row = ((int64_t)b * a.max_t + t) * a.Hkv + hk;
-          kb[u] = __ldg(reinterpret_cast<const uint4*>(a.kq + row * 64 + boff));
-          vb[u] = __ldg(reinterpret_cast<const uint4*>(a.vq + row * 64 + boff));
-          ksv[u] = a.ksc[row * 2 + nib_lo];
-          vsv[u] = a.vsc[row * 2 + nib_lo];
+          kb[u] = __ldg(reinterpret_cast<const uint2*>(a.kq + row * 64 + 8 * sub));
+          vb[u] = __ldg(reinterpret_cast<const uint2*>(a.vq + row * 64 + 8 * sub));
+          ksv[u] = load_scales(a.ksc + row * 2, sc4);
+          vsv[u] = load_scales(a.vsc + row * 2, sc4);
         } else {
-          kb[u] = vb[u] = make_uint4(0, 0, 0, 0);
-          ksv[u] = vsv[u] = __float2half(0.f);
+          kb[u] = vb[u] = make_uint2(0, 0);
+          ksv[u] = vsv[u] = 0u;
         }
       }
       float mnew = m;
 #pragma unroll
-      for (int u = 0; u < BR_UNROLL; ++u) {
-        const uint32_t* wd = reinterpret_cast<const uint32_t*>(&kb[u]);
-        const __half2 sc = __half2half2(ksv[u]);
+      for (int u = 0; u < U; ++u) {
+        const __half2 sh = __low2half2(u32_as_h2(ksv[u])), sl = __high2half2(u32_as_h2(ksv[u]));
         float acc = 0.f;
 #pragma unroll
-        for (int wi = 0; wi < 4; ++wi) {
-          const uint32_t w = nib_lo ? wd[wi] : (wd[wi] >> 4);
-          const float2 f02 = __half22float2(__hmul2(codes_lo_to_h2(w), sc));        // bytes 0, 2
-          const float2 f13 = __half22float2(__hmul2(codes_lo_to_h2(w >> 8), sc));   // bytes 1, 3
-          acc = fmaf(qf[4 * wi + 0], f02.x, acc);
-          acc = fmaf(qf[4 * wi + 2], f02.y, acc);
-          acc = fmaf(qf[4 * wi + 1], f13.x, acc);
-          acc = fmaf(qf[4 * wi + 3], f13.y, acc);
+        for (int wi = 0; wi < 2; ++wi) {
+          const uint32_t w = wi ? kb[u].y : kb[u].x;
+          const float2 h02 = __half22float2(__hmul2(codes_hi_to_h2(w), sh));        // bytes 0, 2
+          const float2 h13 = __half22float2(__hmul2(codes_hi_to_h2(w >> 8), sh));   // bytes 1, 3
+          const float2 l02 = __half22float2(__hmul2(codes_lo_to_h2(w), sl));
+          const float2 l13 = __half22float2(__hmul2(codes_lo_to_h2(w >> 8), sl));
+          acc = fmaf(qf[4 * wi + 0], h02.x, acc);
+          acc = fmaf(qf[4 * wi + 2], h02.y, acc);
+          acc = fmaf(qf[4 * wi + 1], h13.x, acc);
+          acc = fmaf(qf[4 * wi + 3], h13.y, acc);
+          acc = fmaf(qf[8 + 4 * wi + 0], l02.x, acc);
+          acc = fmaf(qf[8 + 4 * wi + 2], l02.y, acc);
+          acc = fmaf(qf[8 + 4 * wi + 1], l13.x, acc);
+          acc = fmaf(qf[8 + 4 * wi + 3], l13.y, acc);
         }
         acc += __shfl_xor_sync(gmask, acc, 1);
         acc += __shfl_xor_sync(gmask, acc, 2);
         acc += __shfl_xor_sync(gmask, acc, 4);
-        s[u] = (t0 + u * BR_GROUPS < len) ? acc : -CUDART_INF_F;
+        s[u] = (t0 + u * NG < len) ? acc : -CUDART_INF_F;
         mnew = fmaxf(mnew, s[u]);
       }
       const float corr = exp2f(m - mnew);
@@ -186,20 +220,25 @@ attn_branch_kernel(const BranchArgs a) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) o[i] *= corr;
 #pragma unroll
-      for (int u = 0; u < BR_UNROLL; ++u) {
+      for (int u = 0; u < U; ++u) {
         const float p = exp2f(s[u] - mnew);
         l += p;
-        const uint32_t* wd = reinterpret_cast<const uint32_t*>(&vb[u]);
-        const __half2 sc = __half2half2(vsv[u]);
+        const __half2 sh = __low2half2(u32_as_h2(vsv[u])), sl = __high2half2(u32_as_h2(vsv[u]));
 #pragma unroll
-        for (int wi = 0; wi < 4; ++wi) {
-          const uint32_t w = nib_lo ? wd[wi] : (wd[wi] >> 4);
-          const float2 f02 = __half22float2(__hmul2(codes_lo_to_h2(w), sc));
-          const float2 f13 = __half22float2(__hmul2(codes_lo_to_h2(w >> 8), sc));
-          o[4 * wi + 0] = fmaf(p, f02.x, o[4 * wi + 0]);
-          o[4 * wi + 2] = fmaf(p, f02.y, o[4 * wi + 2]);
-          o[4 * wi + 1] = fmaf(p, f13.x, o[4 * wi + 1]);
-          o[4 * wi + 3] = fmaf(p, f13.y, o[4 * wi + 3]);
+        for (int wi = 0; wi < 2; ++wi) {
+          const uint32_t w = wi ? vb[u].y : vb[u].x;
+          const float2 h02 = __half22float2(__hmul2(codes_hi_to_h2(w), sh));
+          const float2 h13 = __half22float2(__hmul2(codes_hi_to_h2(w >> 8), sh));
+          const float2 l02 = __half22float2(__hmul2(codes_lo_to_h2(w), sl));
+          const float2 l13 = __half22float2(__hmul2(codes_lo_to_h2(w >> 8), sl));
+          o[4 * wi + 0] = fmaf(p, h02.x, o[4 * wi + 0]);
+          o[4 * wi + 2] = fmaf(p, h02.y, o[4 * wi + 2]);
+          o[4 * wi + 1] = fmaf(p, h13.x, o[4 * wi + 1]);
+          o[4 * wi + 3] = fmaf(p, h13.y, o[4 * wi + 3]);
+          o[8 + 4 * wi + 0] = fmaf(p, l02.x, o[8 + 4 * wi + 0]);
+          o[8 + 4 * wi + 2] = fmaf(p, l02.y, o[8 + 4 * wi + 2]);
+          o[8 + 4 * wi + 1] = fmaf(p, l13.x, o[8 + 4 * wi + 1]);
+          o[8 + 4 * wi + 3] = fmaf(p, l13.y, o[8 + 4 * wi + 3]);
         }
       }
       m = mnew;
@@ -207,10 +246,10 @@ attn_branch_kernel(const BranchArgs a) {
   }
   // the token being decoded attends to its own, un-quantised K/V: one extra key for group 0
   if (a.cur_k != nullptr && grp == 0) {
-    const __half* kp = a.cur_k + (int64_t)b * a.cur_stride + hk * D + sub * 16;
-    const __half* vp = a.cur_v + (int64_t)b * a.cur_stride + hk * D + sub * 16;
-    const uint4 k0 = *reinterpret_cast<const uint4*>(kp), k1 = *reinterpret_cast<const uint4*>(kp + 8);
-    const uint4 v0 = *reinterpret_cast<const uint4*>(vp), v1 = *reinterpret_cast<const uint4*>(vp + 8);
+    const __half* kp = a.cur_k + (int64_t)b * a.cur_stride + hk * D + sub * 8;
+    const __half* vp = a.cur_v + (int64_t)b * a.cur_stride + hk * D + sub * 8;
+    const uint4 k0 = *reinterpret_cast<const uint4*>(kp), k1 = *reinterpret_cast<const uint4*>(kp + 64);
+    const uint4 v0 = *reinterpret_cast<const uint4*>(vp), v1 = *reinterpret_cast<const uint4*>(vp + 64);
     const __half2* kh0 = reinterpret_cast<const __half2*>(&k0);
     const __half2* kh1 = reinterpret_cast<const __half2*>(&k1);
     float acc = 0.f;
@@ -241,47 +280,90 @@ attn_branch_kernel(const BranchArgs a) {
     m = mnew;
   }
 
-  if (sub == 0) { sm_m[grp] = m; sm_l[grp] = l; }
+  const int g0 = slot * NG;
+  if (sub == 0) { sm_m[g0 + grp] = m; sm_l[g0 + grp] = l; }
 #pragma unroll
   for (int i = 0; i < 16; i += 4)
-    *reinterpret_cast<float4*>(&sm_o[grp][sub * 16 + i]) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
-  __syncthreads();
+    *reinterpret_cast<float4*>(&sm_o[g0 + grp][(i & 8) * 8 + sub * 8 + (i & 4)]) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+  if (NW == WPR) __syncthreads();
+  else if (WPR == 1) __syncwarp();
+  else asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "n"(RT) : "memory");
 
-  // merge: thread d owns output dim d
-  const int d = tid;
+  // merge: thread tr owns output dims tr, tr + RT, ... (WPR = 8: the first four warps)
+  constexpr int DP = RT >= D ? 1 : D / RT;
+  if (RT > D && tr >= D) return;
   float M = -CUDART_INF_F;
 #pragma unroll
-  for (int gI = 0; gI < BR_GROUPS; ++gI) M = fmaxf(M, sm_m[gI]);
-  const int64_t rows = (int64_t)gridDim.x;
-  for (int sp = 0; sp < a.nsp; ++sp) M = fmaxf(M, a.pm[(int64_t)sp * rows + bh]);
-  float Lsum = 0.f, acc = 0.f;
+  for (int gI = 0; gI < NG; ++gI) M = fmaxf(M, sm_m[g0 + gI]);
+  M = fmaxf(M, warp_max(pm_l));
+  for (int sp = 32; sp < a.nsp; ++sp) M = fmaxf(M, a.pm[(int64_t)sp * rows + bh]);
+  float Lsum = 0.f, acc[DP];
+#pragma unroll
+  for (int j = 0; j < DP; ++j) acc[j] = 0.f;
   if (M > -CUDART_INF_F) {
 #pragma unroll
-    for (int gI = 0; gI < BR_GROUPS; ++gI) {
-      const float w = exp2f(sm_m[gI] - M);   // exp2(-inf) = 0 for empty groups
-      Lsum = fmaf(sm_l[gI], w, Lsum);
-      acc = fmaf(sm_o[gI][d], w, acc);
+    for (int gI = 0; gI < NG; ++gI) {
+      const float w = exp2f(sm_m[g0 + gI] - M);   // exp2(-inf) = 0 for empty groups
+      Lsum = fmaf(sm_l[g0 + gI], w, Lsum);
+#pragma unroll
+      for (int j = 0; j < DP; ++j) acc[j] = fmaf(sm_o[g0 + gI][tr + j * RT], w, acc[j]);
     }
-    for (int sp = 0; sp < a.nsp; ++sp) {
+    const float pw_l = exp2f(pm_l - M);
+#pragma unroll 4
+    for (int sp = 0; sp < min(a.nsp, 32); ++sp) {
+      const float w = __shfl_sync(0xffffffffu, pw_l, sp);
+      Lsum = fmaf(__shfl_sync(0xffffffffu, pl_l, sp), w, Lsum);
+#pragma unroll
+      for (int j = 0; j < DP; ++j) acc[j] = fmaf(a.po[((int64_t)sp * rows + bh) * D + tr + j * RT], w, acc[j]);
+    }
+    for (int sp = 32; sp < a.nsp; ++sp) {
       const int64_t r = (int64_t)sp * rows + bh;
       const float w = exp2f(a.pm[r] - M);
       Lsum = fmaf(a.pl[r], w, Lsum);
-      acc = fmaf(a.po[r * D + d], w, acc);
+#pragma unroll
+      for (int j = 0; j < DP; ++j) acc[j] = fmaf(a.po[r * D + tr + j * RT], w, acc[j]);
     }
   }
-  const float outv = (Lsum > 0.f) ? acc / Lsum : 0.f;
-  a.o[((int64_t)b * a.H + h) * D + d] = __float2half_rn(outv);
+#pragma unroll
+  for (int j = 0; j < DP; ++j)
+    a.o[bh * D + tr + j * RT] = __float2half_rn((Lsum > 0.f) ? acc[j] / Lsum : 0.f);
 }
 
-int launch_branch(const BranchArgs& a, int mode, int B, cudaStream_t st) {
-  const unsigned grid = (unsigned)(B * a.H);
-  cudaError_t e;
-  if (mode == 0) e = q40_launch_pdl(attn_branch_kernel<0>, dim3(grid), dim3(BR_THREADS), 0, st, a);
-  else if (mode == 1) e = q40_launch_pdl(attn_branch_kernel<1>, dim3(grid), dim3(BR_THREADS), 0, st, a);
-  else if (mode == 2) e = q40_launch_pdl(attn_branch_kernel<2>, dim3(grid), dim3(BR_THREADS), 0, st, a);
-  else e = q40_launch_pdl(attn_branch_kernel<3>, dim3(grid), dim3(BR_THREADS), 0, st, a);
-  if (e != cudaSuccess) return (int)e;
-  return Q40_OK;
+template <int MODE, int NW, int WPR, int U>
+static int launch_rows(const BranchArgs& a, cudaStream_t st) {
+  const unsigned grid = (unsigned)((a.rows + NW / WPR - 1) / (NW / WPR));
+  const cudaError_t e = q40_launch_pdl(attn_branch_kernel<MODE, NW, WPR, U>, dim3(grid), dim3(NW * 32), 0, st, a);
+  return e == cudaSuccess ? Q40_OK : (int)e;
+}
+
+// Warps per row by the number of rows, at 16 (U = 4), 20 or 24 (U = 2) warps an SM; microseconds on a B200, L2 flushed
+// unless a step is named:
+//   contiguous: four warps, four keys in flight; two warps a row are the same within 2 % at any width
+//   paged: eight warps while three CTAs an SM hold all rows (320 rows x 512 keys: 24.7 against 28.7) and there is
+//     more than a row per SM; then four warps with two keys in flight, which leaves room for a fifth CTA
+//     (1920 rows x 300 keys: 58.4 against 61.5 with four keys, 59.4 with two warps a row; 640 rows: 25.6 against
+//     27.6 and 31.7); above one wave of those two warps a row (3200 rows: 48.2 against 52.2)
+//   Q4_0 cache (a quarter of the bytes): two warps a row once four fill more than two waves (a decode step of 3200
+//     rows: 4.58 against 4.77 ms)
+template <int MODE>
+static int launch_branch_mode(const BranchArgs& a, cudaStream_t st) {
+  if constexpr (MODE == 1 || MODE == 2) {
+    if (a.rows > 148 && a.rows <= 3 * 148) return launch_rows<MODE, 8, 8, 2>(a, st);
+    if (a.rows > 16 * 148) return launch_rows<MODE, 4, 2, 4>(a, st);
+    if (a.rows > 148) return launch_rows<MODE, 4, 4, 2>(a, st);
+  }
+  if constexpr (MODE == 3) {
+    if (a.rows > 8 * 148) return launch_rows<MODE, 4, 2, 4>(a, st);
+  }
+  return launch_rows<MODE, 4, 4, 4>(a, st);
+}
+
+int launch_branch(BranchArgs a, int mode, int B, cudaStream_t st) {
+  a.rows = (int64_t)B * a.H;
+  if (mode == 0) return launch_branch_mode<0>(a, st);
+  if (mode == 1) return launch_branch_mode<1>(a, st);
+  if (mode == 2) return launch_branch_mode<2>(a, st);
+  return launch_branch_mode<3>(a, st);
 }
 
 }  // namespace q40

@@ -19,6 +19,7 @@ struct BranchArgs {
   const int32_t* seq_lens;  // per-branch length or nullptr (= L)
   int L, H, Hkv, P, page_size;
   // optional partial results of a prefix pass over rows (b, h), log2 domain, un-normalised
+  int64_t rows;           // B*H (set by launch_branch)
   const float* pm;        // [nsp][B*H]
   const float* pl;        // [nsp][B*H]
   const float* po;        // [nsp][B*H][128]
@@ -40,6 +41,6 @@ struct BranchArgs {
 };
 
 // defined in attn_branch.cu; mode 0 contiguous, 1 paged/int16 ids, 2 paged/int32 ids, 3 Q4_0 cache
-int launch_branch(const BranchArgs& a, int mode, int B, cudaStream_t st);
+int launch_branch(BranchArgs a, int mode, int B, cudaStream_t st);
 
 }  // namespace q40

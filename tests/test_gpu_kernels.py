@@ -325,7 +325,7 @@ def test_attn_paged_ragged_vs_oracle(K, page_size, idx):
     assert float(host(o)[0].astype(np.float32).max()) == 0.0   # empty branch -> zeros
 
 
-@pytest.mark.parametrize("B,H,Hkv,L", [(13, 34, 34, 70), (14, 32, 8, 130), (37, 32, 32, 33), (37, 33, 11, 70), (149, 8, 8, 5)])
+@pytest.mark.parametrize("B,H,Hkv,L", [(4, 37, 37, 70), (13, 34, 34, 70), (14, 32, 8, 130), (37, 33, 11, 70), (149, 8, 8, 5), (74, 32, 8, 40), (103, 23, 23, 33)])
 @pytest.mark.parametrize("paged", [False, True])
 def test_attn_branch_row_counts_around_the_splits(K, B, H, Hkv, L, paged):
     """Row counts (branches x heads) on both sides of where the warps per row change, odd ones among them, and ragged
