@@ -21,7 +21,7 @@
 //     k block, more than the operands themselves);
 //   * four warps issue the tcgen05.mma (A from tensor memory, B from the stage): a k block is 2 x 4 MMAs of
 //     128 x Mpad x 16, small enough that the issuing thread's fixed latencies (mbarrier test, fences, commit:
-//     ~800 cycles per k block measured) matter, so each accumulator has two issuing warps that alternate k
+//     ~800 cycles per k block measured under `lane == 0`, before the elected thread) matter, so each accumulator has two issuing warps that alternate k
 //     blocks and hand over in order through shared memory (every accumulator sees its MMAs in k order:
 //     results do not depend on which warp was faster).  A commit per warp arrives on the block's "MMAs done"
 //     mbarrier, which frees both the stage and the A buffer.
@@ -296,8 +296,9 @@ gemm_tiled_tc_kernel(const Params p, const __grid_constant__ CUtensorMap amap) {
     __syncwarp();
   } else if (warp < DQ_WARP0 || warp >= DQ_WARP0 + DQ_WARPS) {
     // ================= the four MMA warps: one elected thread each =================
-    // Per k block an issuing warp spends ~800 cycles on fixed latencies (mbarrier test, fences, commit) and
-    // 60-120 per tcgen05.mma, whatever the tile size, so one thread cannot feed eight small MMAs per k block.
+    // Under `lane == 0` an issuing warp spent ~800 cycles per k block on fixed latencies (mbarrier test, fences, commit)
+    // and 60-120 per tcgen05.mma, whatever the tile size; the elected thread takes less (100 rows x 4096 x 11008: 19.4 ->
+    // 16.9 us), and four of them still overlap their waits.
     // Warp (hh, set) issues the four k steps of feature half hh for the k blocks of its set (even or odd).
     // fp32 accumulation is not associative, and the result must not depend on which warp was faster, so every
     // accumulator has to see its MMAs in a fixed order.  Up to 64 padded batch rows tensor memory has room for
@@ -453,14 +454,16 @@ gemm_tiled_tc_kernel(const Params p, const __grid_constant__ CUtensorMap amap) {
 // ---------------------------------------------------------------------------------------------------------
 // More than 128 rows (prompt pass, wide batches): 128 features x up to 256 batch rows per CTA.
 //
-// Same operands as above, other proportions.  A tcgen05.mma has a fixed cost of ~78 cycles whatever its width
-// (see gemm_tiled_tc_kernel), so the rows, which are the MMA's N, go up to 256, and one accumulator of 128
+// Same operands as above, other proportions.  The rows, which are the MMA's N, go up to 256, so that a k block is four
+// large MMAs, and one accumulator of 128
 // features takes half of tensor memory; the other half holds NA = 8 A buffers.  The activations of a k block
 // (32 KB at 256 rows) are read once per 128 features.  Sixteen dequantiser warps are four sets of four (one
 // warp per tensor-memory quadrant) that take the k blocks in turn; one thread issues all MMAs, in k order, so a
 // result depends on nothing but the operands and the k split.  Rows are cut into equal chunks of at most 256
 // inside ONE launch (grid z); a tile that is not split along k goes from tensor memory to the output
 // directly, otherwise the ranks of a cluster add their fp32 tiles in rank order.
+// 512 x 4096 x 11008: 58.5 us = 0.79 PFLOP/s, about half the tensor rate (122.9 us on the checkpoint layout; 94.9 us with
+// the copies and MMAs under `lane == 0`).  36 KB a k block come through L2, which is what bounds it next.
 // ---------------------------------------------------------------------------------------------------------
 namespace wide {
 
