@@ -118,6 +118,8 @@ def quantize_q40_rows(w: torch.Tensor, q_out: torch.Tensor, s_out: torch.Tensor,
     check(lib.q40_quantize_rows(w.data_ptr(), w.stride(0), q_out.data_ptr(), q_out.stride(0),
                                 s_out.data_ptr(), s_out.stride(0), rows, row_len, group_size,
                                 _stream(dev)), "q40_quantize_rows")
+    # a write that torch did not make itself: counted, so that tiled copies of these tensors are made again
+    torch.autograd.graph.increment_version([t for t in (q_out, s_out) if not t.is_inference()])
 
 
 def triton_deq_int40(w: torch.Tensor, s: torch.Tensor, group_size, shape, ptdtype=torch.float16):
@@ -236,6 +238,25 @@ def _versions(*ts):
         except RuntimeError:
             out.append(-1)
     return tuple(out)
+
+
+class TiledCopy:
+    """A tiled copy a model keeps and what it was made from: tensors (weakly), their addresses and in-place
+    modification counters, and the (K, N) they were read as.  A write into a tensor made under inference_mode is not
+    seen, nor is one through `.data` or a raw pointer."""
+    __slots__ = ("data", "shape", "_refs", "_ptrs", "_versions")
+
+    def __init__(self, data: torch.Tensor, shape, *src: torch.Tensor):
+        self.data, self.shape = data, tuple(shape)
+        self._refs, self._ptrs, self._versions = [weakref.ref(t) for t in src], [t.data_ptr() for t in src], _versions(*src)
+
+    def is_of(self, shape, *src: torch.Tensor) -> bool:
+        """Whether the copy still holds these tensors' contents."""
+        return (self.shape == shape and len(src) == len(self._refs) and self._versions == _versions(*src) and
+                all(r() is t and p == t.data_ptr() for r, p, t in zip(self._refs, self._ptrs, src)))
+
+    def __reduce__(self):
+        return type(None), ()       # pickled or copied with its owner: made again on first use
 
 
 def _tiled_copy_of(b_w, b_s, K, N):

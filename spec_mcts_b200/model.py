@@ -154,6 +154,11 @@ class TransformerBlock(nn.Module):
         self.ffn_norm = RMSNorm(args.dim, eps=args.norm_eps)
 
 
+def _projections(layer: TransformerBlock):
+    att, ff = layer.attention, layer.feed_forward
+    return [att.wq, att.wk, att.wv, att.wo, ff.w1, ff.w3, ff.w2]
+
+
 class Transformer(nn.Module):
     """forward(tokens, start_pos): start_pos == 0 is the prompt (batch 1; fills the shared
     prompt cache), start_pos > 0 with one token per branch is a decode step
@@ -292,7 +297,7 @@ class Transformer(nn.Module):
         plan = []
         for layer in self.layers:
             att, ff = layer.attention, layer.feed_forward
-            plan.append([(lins, self._tiled_of(lins) if self._prefill_tiled(S, lins) else None)
+            plan.append([(lins, self._tiled_of(lins) if self._prefill_tiled(S, lins) else self._drop_stale(lins))
                          for lins in ([att.wq, att.wk, att.wv], [att.wo], [ff.w1, ff.w3], [ff.w2])])
         h = self.tok_embeddings(tokens.to(dev)).to(DTYPE).view(S, p.dim)
         pos = torch.arange(S, dtype=torch.int32, device=dev)
@@ -336,7 +341,9 @@ class Transformer(nn.Module):
         """Whether the prompt pass multiplies these projections through their tiled copies."""
         return (M > 16 and self.use_tiled and self.use_tiled_tc and len(lins) <= 3 and
                 (self.prefill_tiled_tc or not self.prefill_checkpoint_layout) and
-                all(l.group_size == 64 and self._tileable(l) and l.kn()[0] % 64 == 0 for l in lins))
+                all(l.group_size == 64 and self._tileable(l) and l.kn()[0] % 64 == 0 for l in lins) and
+                # a write into an inference tensor is not counted, so a copy of it could be old
+                (self.prefill_tiled_tc or not any(l.w.is_inference() or l.s.is_inference() for l in lins)))
 
     def _mm(self, x, weights, outs, st):
         """outs[i] = x @ deq(W_i) for projections that share the activations x [M, K] (prompt pass): one tensor-core
@@ -456,14 +463,42 @@ class Transformer(nn.Module):
         return lin.kn()[1] % 256 == 0 and lin.kn()[0] % 16 == 0
 
     def _tiled_of(self, lins):
-        """The rearranged copies of these layers' weights (made on first use)."""
+        """The rearranged copies of these layers' weights: made on first use, and again after `w` or `s` was assigned
+        or written in place."""
         out = []
         for l in lins:
-            if getattr(l, "_tiled", None) is None or l._tiled_src != l.w.data_ptr():
-                l._tiled = K.relayout_tiled(l.w, l.s, l.kn())     # one-time rearranged copy
-                l._tiled_src = l.w.data_ptr()
-            out.append(l._tiled)
+            c = getattr(l, "_tiled", None)
+            if c is None or not c.is_of(l.kn(), l.w, l.s):
+                if c is not None:
+                    self.release_graphs()         # captured steps hold the address of the copy that goes away
+                c = l._tiled = K.TiledCopy(K.relayout_tiled(l.w, l.s, l.kn()), l.kn(), l.w, l.s)
+            out.append(c.data)
         return out
+
+    def drop_tiled_copies(self):
+        """Forget the rearranged weight copies (made again on the next step): for weights written in a way torch
+        does not count, through `.data`, a raw pointer or under inference_mode."""
+        self.release_graphs()
+        for layer in self.layers:
+            for l in _projections(layer):
+                l._tiled = l._tiled_cat = None
+        if self._lm_head_q4 is not None:
+            self._lm_head_q4._tiled = None
+
+    def _drop_stale(self, lins):
+        """Drop these layers' copies, and the captured steps that read them, if their weights have changed."""
+        for l in lins:
+            c, cat = getattr(l, "_tiled", None), getattr(l, "_tiled_cat", None)
+            if c is not None and not c.is_of(l.kn(), l.w, l.s):
+                self.release_graphs()
+                l._tiled = None
+            if cat is not None and not cat.is_of(*self._concat_source(lins)):
+                self.release_graphs()
+                l._tiled_cat = None
+
+    @staticmethod
+    def _concat_source(lins):
+        return (tuple(l.kn() for l in lins), *[t for l in lins for t in (l.w, l.s)])
 
     @staticmethod
     def _concat_tileable(lins, outs):
@@ -484,15 +519,17 @@ class Transformer(nn.Module):
     def _tiled_concat(self, lins):
         """Tiled copy of [W_0 | W_1 | ...] (columns concatenated): packed rows and scale rows of the checkpoint
         layout concatenate block by block, so no code or scale changes.  Cached on the first matrix."""
-        key = tuple(l.w.data_ptr() for l in lins)
-        first = lins[0]
-        if getattr(first, "_tiled_cat_key", None) != key:
+        first, src = lins[0], self._concat_source(lins)
+        c = getattr(first, "_tiled_cat", None)
+        if c is None or not c.is_of(*src):
+            if c is not None:
+                self.release_graphs()
             Kd = first.kn()[0]
             w = torch.cat([l.w.reshape(Kd, l.kn()[1] // 2) for l in lins], dim=1).contiguous()
             sc = torch.cat([l.s.reshape(Kd, l.kn()[1] // 64) for l in lins], dim=1).contiguous()
-            first._tiled_cat = K.relayout_tiled(w, sc, (Kd, sum(l.kn()[1] for l in lins)))
-            first._tiled_cat_key = key
-        return first._tiled_cat
+            data = K.relayout_tiled(w, sc, (Kd, sum(l.kn()[1] for l in lins)))
+            c = first._tiled_cat = K.TiledCopy(data, *src)
+        return c.data
 
     def _streamable(self, lins, M):
         return self.use_tiled and self.use_stream and M <= 16 and all(self._tileable(l) for l in lins)

@@ -296,3 +296,85 @@ def test_wide_step_with_one_kv_head_uses_the_concatenated_tiled_copy():
                 assert not m._tileable(att.wk) and getattr(att.wq, "_tiled_cat", None) is not None
     rel = np.linalg.norm(logits[0] - logits[1], axis=-1) / np.linalg.norm(logits[1], axis=-1)
     assert rel.max() < 2e-2, rel
+
+
+def small_random(seed=5, **kw):
+    from spec_mcts_b200.model import ModelArgs, Transformer, random_init_
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    args = ModelArgs(**{**dict(dim=512, n_layers=2, n_heads=4, vocab_size=512, multiple_of=256, max_batch_size=24,
+                               max_seq_len=8, max_prompt_seq_len=160), **kw})
+    m = Transformer(args, device=torch.device("cuda", 0))
+    random_init_(m, seed=seed, std=0.05)
+    return m.to("cuda", torch.float16)
+
+
+def random_weights(seed, k, n):
+    from spec_mcts_b200 import kernels as KK
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    q, s = KK.quantize_q40((torch.randn((k, n), generator=g, device="cuda") * 0.05).half())
+    return q, s.view(-1)
+
+
+@pytest.mark.parametrize("n_kv_heads", [4, 1])       # one kv head: wk / wv are read as part of one concatenated copy
+@pytest.mark.parametrize("how", ["copy_", "scales", "assign", "packer", "data"])
+def test_prompt_and_step_follow_written_weights(how, n_kv_heads):
+    """Weights written after a prompt pass and two widths of steps: the next prompt pass and the steps after it give the
+    bits of a model that had those weights from the start."""
+    from spec_mcts_b200 import kernels as KK
+    prompt = torch.arange(40, device="cuda").view(1, -1) * 7 % 512
+    toks = {b: torch.arange(b, device="cuda").view(-1, 1) * 11 % 512 for b in (3, 20)}
+
+    def outputs(m):
+        out = [m(prompt, 0).clone()]
+        for b, t in toks.items():
+            m.fork(0, 1, b - 1)
+            out.append(m(t, 40).clone())
+        return out
+
+    def change(m, fresh):
+        for i, l in enumerate([m.layers[0].attention.wk, m.layers[1].feed_forward.w1, m.layers[1].attention.wo]):
+            k, n = l.kn()
+            q, s = random_weights(i, k, n)
+            if fresh or how == "assign":
+                l.w, l.s = q, s
+            elif how == "scales":
+                l.w = q
+                l.s.copy_(s)
+            elif how == "packer":                    # the library's own packer writes into the weight tensors
+                g = torch.Generator(device="cuda").manual_seed(i)
+                w = (torch.randn((k, n), generator=g, device="cuda") * 0.05).half()
+                KK.quantize_q40_rows(w, l.w.view(k, n // 2), l.s.view(k, n // 64))
+            elif how == "data":                      # not counted by torch: the host says so
+                l.w.data.copy_(q)
+                l.s.data.copy_(s)
+            else:
+                l.w.copy_(q)
+                l.s.copy_(s)
+        if how == "data" and not fresh:
+            m.drop_tiled_copies()
+
+    m, ref = small_random(n_kv_heads=n_kv_heads), small_random(n_kv_heads=n_kv_heads)
+    before = outputs(m)
+    change(m, False)
+    change(ref, True)
+    got, want = outputs(m), outputs(ref)
+    for x, y, z in zip(got, want, before):
+        assert torch.equal(x, y) and not torch.equal(x, z)
+
+
+def test_prompt_follows_weights_made_under_inference_mode():
+    """Tensors made under inference_mode keep no count of writes: the prompt pass reads them as they are."""
+    with torch.inference_mode():
+        m = small_random()
+        prompt = torch.arange(40, device="cuda").view(1, -1)
+        a = m(prompt, 0).clone()
+        l = m.layers[0].feed_forward.w2
+        q, s = random_weights(3, *l.kn())
+        l.w.copy_(q)
+        l.s.copy_(s)
+        b = m(prompt, 0).clone()
+        ref = small_random()
+        r = ref.layers[0].feed_forward.w2
+        r.w, r.s = q, s
+        assert torch.equal(b, ref(prompt, 0)) and not torch.equal(a, b)
