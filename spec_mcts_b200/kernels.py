@@ -336,8 +336,13 @@ def _cluster_gemv(dev, a, b_w, b_s, c, M, N, K) -> bool:
     return False
 
 
+def _tc_error_word(dev) -> torch.Tensor:
+    """The int32 device word behind tc_error_flag(), for this stream."""
+    return _workspace("gemm", dev, 4096, zero=True)[4092:4096].view(torch.int32)
+
+
 def tc_error_flag(dev=None) -> int:
-    """1 if a tensor-core matmul launched through matmul_q40 on the current stream of `dev` gave up
+    """1 if a tensor-core matmul launched through matmul_q40 or a prompt pass on the current stream of `dev` gave up
     on one of its bounded waits since the workspace was created (synchronises the device)."""
     dev = torch.device("cuda", torch.cuda.current_device()) if dev is None else dev
     buf = _workspaces.get(("gemm", dev.index, _stream(dev)))

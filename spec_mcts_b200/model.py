@@ -233,8 +233,11 @@ class Transformer(nn.Module):
         # True: the prompt pass returns logits of the last position only, [1, 1, vocab] (all a caller that
         # samples the next token needs); False: of every position like the reference
         self.prefill_last_only = False
-        self._tc_err = None         # device word the prompt pass's tensor-core launches set on a wait expiry
-        self._tc_err_host = None    # ... and its copy of the last finished pass
+        # device word that the last prompt pass's tensor-core launches set on a wait expiry (the one of
+        # kernels.tc_error_flag), its copy of the last finished pass, and whether nothing has waited for it yet
+        self._tc_err = None
+        self._tc_err_host = torch.zeros(1, dtype=torch.int32).pin_memory()
+        self._prompt_unchecked = False
         # ... True: through the byte-balanced stream-K launch (one CTA per SM, bulk-copy ring, no clusters);
         # False: the cluster-reduced launch on the same tiled copies (faster on B200, the default)
         self.use_stream = False
@@ -288,7 +291,8 @@ class Transformer(nn.Module):
         bsz, S = tokens.shape
         assert bsz == 1, "the prompt is processed once and shared by all branches"
         assert S <= p.max_prompt_seq_len
-        self._check_tc_err()
+        if self._prompt_unchecked and int(self._tc_err_host) != 0:      # without waiting for the pass before this one
+            self._prompt_failed()
         dev = self.device
         H, Hkv, D = self._H, self._Hkv, self._D
         hid = self.layers[0].feed_forward.hidden_dim
@@ -302,6 +306,7 @@ class Transformer(nn.Module):
         h = self.tok_embeddings(tokens.to(dev)).to(DTYPE).view(S, p.dim)
         pos = torch.arange(S, dtype=torch.int32, device=dev)
         st = torch.cuda.current_stream(dev).cuda_stream
+        err = K._tc_error_word(h.device)
         e = lambda n: torch.empty((S, n), dtype=DTYPE, device=dev)
         xn, q, ao, o, a1, a3, g, f = (e(n) for n in (p.dim, H * D, H * D, p.dim, hid, hid, hid, p.dim))
         pending = None     # output of the previous sub-block, added to h by the next norm kernel
@@ -310,32 +315,56 @@ class Transformer(nn.Module):
             # keys and values go straight to their place in the prompt cache
             ck, cv = att.cache_prompt_k[:S], att.cache_prompt_v[:S]
             self._norm(h, pending, layer.attention_norm.weight, xn, st)
-            self._mm(xn, qkv, [q, ck.view(S, Hkv * D), cv.view(S, Hkv * D)], st)
+            self._mm(xn, qkv, [q, ck.view(S, Hkv * D), cv.view(S, Hkv * D)], err, st)
             K.rope_(q.view(S, H, D), pos, self._cos, self._sin)
             K.rope_(ck, pos, self._cos, self._sin)
             att.cache_prompt_len = S
             # causal attention over the prompt (grouped-query heads read their kv head directly)
             K.causal_attn(q.view(S, H, D), ck, cv, out=ao.view(S, H, D))
-            self._mm(ao, wo, [o], st)
+            self._mm(ao, wo, [o], err, st)
             self._all_reduce(o)
             self._norm(h, o, layer.ffn_norm.weight, xn, st)
-            self._mm(xn, w13, [a1, a3], st)
+            self._mm(xn, w13, [a1, a3], err, st)
             check(lib.q40_silu_mul(a1.data_ptr(), a3.data_ptr(), g.data_ptr(), g.numel(), st), "q40_silu_mul")
-            self._mm(g, w2, [f], st)
+            self._mm(g, w2, [f], err, st)
             self._all_reduce(f)
             pending = f
         self._prefix_len_dev.fill_(S)
-        if self._tc_err is not None:
-            self._tc_err_host.copy_(self._tc_err, non_blocking=True)      # read by the next call, without a wait here
+        self._tc_err = K._tc_error_word(h.device)
+        if self._tc_err.data_ptr() != err.data_ptr():     # a larger workspace took the first one's place meanwhile
+            self._tc_err |= err
+        self._tc_err_host.copy_(self._tc_err, non_blocking=True)
+        self._prompt_unchecked = S > 16        # narrower passes run no kernel that waits
         if self.prefill_last_only:
             # the tree search reads the last position only (mcts.py:105); the reference computes all S rows
             h, xn, pending = h[S - 1:], xn[S - 1:], pending[S - 1:]
         self._norm(h, pending, self.norm.weight, xn, st)
-        return F.linear(xn, self.output.weight).to(DTYPE).view(1, h.shape[0], -1)
+        logits = F.linear(xn, self.output.weight).to(DTYPE).view(1, h.shape[0], -1)
+        if self.prefill_tiled_tc:
+            self._check_prompt()
+        return logits
 
-    def _check_tc_err(self):
-        if self._tc_err_host is not None and int(self._tc_err_host) != 0:
-            raise K.Q40Error("prompt pass: a bounded wait inside a tensor-core matmul expired")
+    def _check_prompt(self):
+        """Raise if a bounded wait inside a tensor-core matmul of the last prompt pass expired: waits for the pass, so
+        that nothing is built on an undefined prompt cache.  Once per pass, by what uses it first."""
+        if self._prompt_unchecked and not torch.cuda.is_current_stream_capturing():
+            if int(self._tc_err.item()) != 0:
+                self._prompt_failed()
+            self._prompt_unchecked = False
+
+    @torch.inference_mode()
+    def _prompt_failed(self):
+        self._tc_err.zero_()
+        torch.cuda.synchronize(self.device)      # copies of passes in flight have landed
+        self._tc_err_host.zero_()
+        self._prompt_unchecked = False
+        raise K.Q40Error("prompt pass: a bounded wait inside a tensor-core matmul expired")
+
+    def prompt_status(self) -> int:
+        """Non-zero if a bounded wait inside a tensor-core matmul of a prompt pass expired, which makes its logits and
+        prompt cache undefined (synchronises).  For hosts that take no decode step: the first step after such a pass
+        raises, and so does a later prompt pass once the word has reached the host."""
+        return 0 if self._tc_err is None else int(self._tc_err.item())
 
     def _prefill_tiled(self, M, lins):
         """Whether the prompt pass multiplies these projections through their tiled copies."""
@@ -345,22 +374,19 @@ class Transformer(nn.Module):
                 # a write into an inference tensor is not counted, so a copy of it could be old
                 (self.prefill_tiled_tc or not any(l.w.is_inference() or l.s.is_inference() for l in lins)))
 
-    def _mm(self, x, weights, outs, st):
+    def _mm(self, x, weights, outs, err, st):
         """outs[i] = x @ deq(W_i) for projections that share the activations x [M, K] (prompt pass): one tensor-core
         launch when they have tiled copies, matmul_q40 per projection otherwise."""
         import ctypes
         lins, tiled = weights
         n = len(lins)
         if tiled is not None:
-            if self._tc_err is None:
-                self._tc_err = torch.zeros(1, dtype=torch.int32, device=self.device)
-                self._tc_err_host = torch.zeros(1, dtype=torch.int32, pin_memory=True)
             P = ctypes.c_void_p * n
             check(lib.q40_gemm_tiled_tc_multi(n, x.data_ptr(), x.stride(0), P(*[t.data_ptr() for t in tiled]),
                                               P(*[o.data_ptr() for o in outs]),
                                               (ctypes.c_int64 * n)(*[o.stride(0) for o in outs]),
                                               (ctypes.c_int * n)(*[l.kn()[1] for l in lins]), x.shape[0], x.shape[1],
-                                              self._tc_err.data_ptr(), 1 if self.use_pdl else 0, st),
+                                              err.data_ptr(), 1 if self.use_pdl else 0, st),
                   "q40_gemm_tiled_tc_multi")
             return
         # relayout=False: the checkpoint-layout kernels
@@ -804,6 +830,7 @@ class Transformer(nn.Module):
     def decode_replay(self, B):
         """Run one decode step for B branches with the tokens/positions already in the device
         buffers (`_tok_dev`, `_pos_dev`); returns the static logits buffer [B, vocab]."""
+        self._check_prompt()
         fused = self.use_fused and B <= 16 and self.tp_world == 1
         self.launches_per_step = self.params.n_layers * ((5 if self._fused_attn_for(B) else 7) if fused else 13) + (2 if fused else 1)
         if not self.use_cuda_graph:

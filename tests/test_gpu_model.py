@@ -378,3 +378,39 @@ def test_prompt_follows_weights_made_under_inference_mode():
         r = ref.layers[0].feed_forward.w2
         r.w, r.s = q, s
         assert torch.equal(b, ref(prompt, 0)) and not torch.equal(a, b)
+
+
+def test_expired_wait_of_a_prompt_pass_is_reported_before_its_first_use():
+    """The error word set by hand, as a kernel whose wait ran out leaves it: the first decode step raises before it
+    gives a result, the status calls report it, and the next prompt pass and its steps work."""
+    from spec_mcts_b200 import kernels as KK
+    prompt, tok = torch.arange(40, device="cuda").view(1, -1), torch.zeros((1, 1), dtype=torch.int64, device="cuda")
+    m = small_random()
+
+    def expire():
+        with torch.inference_mode():
+            m._tc_err.fill_(1)
+
+    want = m(prompt, 0).clone(), m(tok, 40).clone()
+    for width in (1, 20):
+        m(prompt, 0)
+        assert m.prompt_status() == 0 and KK.tc_error_flag() == 0
+        expire()
+        assert m.prompt_status() != 0 and KK.tc_error_flag() != 0
+        with pytest.raises(KK.Q40Error):
+            m(tok.expand(width, 1), 40)
+        got = m(prompt, 0).clone(), m(tok, 40).clone()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    # prompts only: the next pass says so once the word is on the host, and the one after that works
+    expire()
+    m(prompt, 0)
+    torch.cuda.synchronize()
+    with pytest.raises(KK.Q40Error):
+        m(prompt, 0)
+    assert torch.equal(m(prompt, 0), want[0]) and m.prompt_status() == 0
+    # asked for by name, the pass itself waits
+    m.prefill_tiled_tc = True
+    assert torch.equal(m(prompt, 0), want[0])
+    expire()
+    with pytest.raises(KK.Q40Error):
+        m(prompt, 0)
