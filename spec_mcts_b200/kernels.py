@@ -190,11 +190,10 @@ def matmul_q40(a: torch.Tensor, b_w: torch.Tensor, b_s: torch.Tensor, b_shape, *
     wide = (M > 16 and group_size == 64 and N % 256 == 0 and K % 64 == 0 and a.data_ptr() % 16 == 0 and
             c.stride(1) == 1 and c.stride(0) % 2 == 0 and c.data_ptr() % 4 == 0)
     if (wide or (small and N % 256 == 0)) and (relayout if relayout is not None else _relayout_cfg["enabled"]):
-        n_before = len(_relayout_cache)
-        tiled = _tiled_copy_of(b_w, b_s, K, N)
+        tiled, fresh = _tiled_copy_of(b_w, b_s, K, N)
         # programmatic launch (weights requested while the previous kernel drains) except right after the
         # kernel that wrote the copy
-        if tiled is not None and (_tiled_matmul(dev, a, tiled, c, M, N, K, len(_relayout_cache) == n_before) or
+        if tiled is not None and (_tiled_matmul(dev, a, tiled, c, M, N, K, not fresh) or
                                   (small and _stream_gemv(dev, a, tiled, c, M, N, K))):
             return c
     if small and N % 128 == 0 and _cluster_gemv(dev, a, b_w, b_s, c, M, N, K):
@@ -260,18 +259,19 @@ class TiledCopy:
 
 
 def _tiled_copy_of(b_w, b_s, K, N):
+    """(copy or None, whether this call made it)."""
     key = id(b_w)
     ent = _relayout_cache.get(key)
     if ent is not None:
         rw, rs, ver, shape, ptrs, copy = ent
         if (rw() is b_w and rs() is b_s and ver == _versions(b_w, b_s) and shape == (K, N)
                 and ptrs == (b_w.data_ptr(), b_s.data_ptr())):
-            return copy
+            return copy, False
         _relayout_bytes[0] -= copy.numel()
         del _relayout_cache[key]
     nbytes = lib.q40_tiled_bytes(N, K)
     if nbytes == 0 or _relayout_bytes[0] + nbytes > _relayout_cfg["max_bytes"]:
-        return None
+        return None, False
     copy = relayout_tiled(b_w, b_s, (K, N))
 
     def _drop(_ref, key=key):
@@ -282,7 +282,7 @@ def _tiled_copy_of(b_w, b_s, K, N):
     _relayout_cache[key] = (weakref.ref(b_w, _drop), weakref.ref(b_s), _versions(b_w, b_s), (K, N),
                             (b_w.data_ptr(), b_s.data_ptr()), copy)
     _relayout_bytes[0] += nbytes
-    return copy
+    return copy, True
 
 
 def _tiled_matmul(dev, a, tiled, c, M, N, K, pdl) -> bool:

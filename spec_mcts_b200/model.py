@@ -301,7 +301,7 @@ class Transformer(nn.Module):
         plan = []
         for layer in self.layers:
             att, ff = layer.attention, layer.feed_forward
-            plan.append([(lins, self._tiled_of(lins) if self._prefill_tiled(S, lins) else self._drop_stale(lins))
+            plan.append([(lins, self._tiled_of(lins)[0] if self._prefill_tiled(S, lins) else self._drop_stale(lins))
                          for lins in ([att.wq, att.wk, att.wv], [att.wo], [ff.w1, ff.w3], [ff.w2])])
         h = self.tok_embeddings(tokens.to(dev)).to(DTYPE).view(S, p.dim)
         pos = torch.arange(S, dtype=torch.int32, device=dev)
@@ -434,13 +434,13 @@ class Transformer(nn.Module):
             if len(t_idx) < n and self._concat_tileable(lins, outs):
                 # widths that cannot be tiled one by one (a kv head per rank: 128 columns) but whose outputs are
                 # adjacent column ranges of one buffer: one tiled copy of the concatenated matrix, one launch
-                cat = self._tiled_concat(lins)
+                cat, pdl = self._tiled_concat(lins)
                 err = bufs["gemm_ws"].data_ptr() + 4096 - 4
                 P1 = ctypes.c_void_p * 1
                 check(lib.q40_gemm_tiled_tc_multi(1, x.data_ptr(), x.stride(0), P1(cat.data_ptr()),
                                                   P1(outs[0].data_ptr()), (ctypes.c_int64 * 1)(outs[0].stride(0)),
                                                   (ctypes.c_int * 1)(sum(l.kn()[1] for l in lins)), M,
-                                                  lins[0].kn()[0], err, 1 if self.use_pdl else 0, st),
+                                                  lins[0].kn()[0], err, 1 if pdl else 0, st),
                       "q40_gemm_tiled_tc_multi")
                 return
             if t_idx and len(t_idx) < n:
@@ -455,12 +455,12 @@ class Transformer(nn.Module):
             if t_idx and n <= 3 and all(l.kn()[0] == lins[0].kn()[0] for l in lins):
                 P = ctypes.c_void_p * n
                 err = bufs["gemm_ws"].data_ptr() + 4096 - 4      # the error word q40_gemm_kn also uses
-                check(lib.q40_gemm_tiled_tc_multi(n, x.data_ptr(), x.stride(0),
-                                                  P(*[t.data_ptr() for t in self._tiled_of(lins)]),
+                tiled, pdl = self._tiled_of(lins)
+                check(lib.q40_gemm_tiled_tc_multi(n, x.data_ptr(), x.stride(0), P(*[t.data_ptr() for t in tiled]),
                                                   P(*[o.data_ptr() for o in outs]),
                                                   (ctypes.c_int64 * n)(*[o.stride(0) for o in outs]),
                                                   (ctypes.c_int * n)(*[l.kn()[1] for l in lins]), M, lins[0].kn()[0],
-                                                  err, 1 if self.use_pdl else 0, st), "q40_gemm_tiled_tc_multi")
+                                                  err, 1 if pdl else 0, st), "q40_gemm_tiled_tc_multi")
                 return
         ok = M > 16 and n <= 3 and all(l.group_size == 64 and l.kn()[1] % 128 == 0 and l.kn()[0] % 64 == 0 and
                                        l.kn()[0] == lins[0].kn()[0] and o.stride(0) % 2 == 0
@@ -490,16 +490,18 @@ class Transformer(nn.Module):
 
     def _tiled_of(self, lins):
         """The rearranged copies of these layers' weights: made on first use, and again after `w` or `s` was assigned
-        or written in place."""
-        out = []
+        or written in place; and whether a launch may read them before it waits for the one in front of it (not if
+        that one writes a copy)."""
+        out, pdl = [], self.use_pdl
         for l in lins:
             c = getattr(l, "_tiled", None)
             if c is None or not c.is_of(l.kn(), l.w, l.s):
                 if c is not None:
                     self.release_graphs()         # captured steps hold the address of the copy that goes away
                 c = l._tiled = K.TiledCopy(K.relayout_tiled(l.w, l.s, l.kn()), l.kn(), l.w, l.s)
+                pdl = False
             out.append(c.data)
-        return out
+        return out, pdl
 
     def drop_tiled_copies(self):
         """Forget the rearranged weight copies (made again on the next step): for weights written in a way torch
@@ -544,7 +546,9 @@ class Transformer(nn.Module):
 
     def _tiled_concat(self, lins):
         """Tiled copy of [W_0 | W_1 | ...] (columns concatenated): packed rows and scale rows of the checkpoint
-        layout concatenate block by block, so no code or scale changes.  Cached on the first matrix."""
+        layout concatenate block by block, so no code or scale changes.  Cached on the first matrix.  Returns the copy
+        and the second value of _tiled_of."""
+        pdl = self.use_pdl
         first, src = lins[0], self._concat_source(lins)
         c = getattr(first, "_tiled_cat", None)
         if c is None or not c.is_of(*src):
@@ -555,7 +559,8 @@ class Transformer(nn.Module):
             sc = torch.cat([l.s.reshape(Kd, l.kn()[1] // 64) for l in lins], dim=1).contiguous()
             data = K.relayout_tiled(w, sc, (Kd, sum(l.kn()[1] for l in lins)))
             c = first._tiled_cat = K.TiledCopy(data, *src)
-        return c.data
+            pdl = False
+        return c.data, pdl
 
     def _streamable(self, lins, M):
         return self.use_tiled and self.use_stream and M <= 16 and all(self._tileable(l) for l in lins)
@@ -584,8 +589,10 @@ class Transformer(nn.Module):
         n = len(lins)
         P = ctypes.c_void_p * n
         tiled = self.use_tiled and M <= 16 and all(self._tileable(l) for l in lins)
+        pdl = self.use_pdl
         if tiled:
-            bw = P(*[t.data_ptr() for t in self._tiled_of(lins)])
+            copies, pdl = self._tiled_of(lins)
+            bw = P(*[t.data_ptr() for t in copies])
         else:
             bw = P(*[l.w.data_ptr() for l in lins])
         op = P(*[o.data_ptr() for o in outs])
@@ -599,14 +606,14 @@ class Transformer(nn.Module):
             ws = self._stream_ws(bufs, M)
             check(lib.q40_gemv_stream(mode, n, bw, op, nc, ldc, a.data_ptr(), lda, M, Kd, nw, si, ss_in_count,
                                       float(self.params.norm_eps), hi, ldh, so, ss_out_count, ws.data_ptr(),
-                                      ws.numel(), self.stream_smem_budget, 1 if self.use_pdl else 0, st),
+                                      ws.numel(), self.stream_smem_budget, 1 if pdl else 0, st),
                   "q40_gemv_stream")
             return
         bs = P(*[l.s.data_ptr() for l in lins])
         fn = lib.q40_gemv_tiled if tiled else lib.q40_gemv_fused
         check(fn(mode, n, bw, bs, op, nc, ldc, a.data_ptr(), lda, M, Kd, nw, si, ss_in_count,
                  float(self.params.norm_eps), hi, ldh, so, ss_out_count,
-                 self.max_cluster, 1 if self.use_pdl else 0, st), "q40_gemv_fused")
+                 self.max_cluster, 1 if pdl else 0, st), "q40_gemv_fused")
 
     def stream_status(self, B) -> int:
         """Non-zero if a bounded wait inside a stream-K launch of the last steps expired (synchronises)."""

@@ -109,3 +109,58 @@ def test_concatenated_projection_rule():
     sep = [torch.zeros((4, 1024), dtype=torch.float16), torch.zeros((4, 128), dtype=torch.float16),
            torch.zeros((4, 128), dtype=torch.float16)]
     assert not Transformer._concat_tileable([lin(1024), lin(128), lin(128)], sep)                # separate buffers
+
+
+@pytest.fixture
+def launches(monkeypatch):
+    """kernels.py with its device calls faked: a list of (rows, whether the matmul was launched with programmatic
+    dependent launch) of the matmul_q40 calls made, on CPU tensors."""
+    import torch
+    from types import SimpleNamespace
+    from spec_mcts_b200 import kernels as K
+    calls = []
+
+    def matmul_tiled(bw, c, ldc, a, lda, M, N, Kd, cluster, err, pdl, stream):
+        calls.append((M, bool(pdl)))
+        return 0
+
+    monkeypatch.setattr(K, "lib", SimpleNamespace(q40_matmul_tiled=matmul_tiled, q40_tiled_bytes=lambda N, Kd: 128))
+    monkeypatch.setattr(K, "_need_cuda", lambda *t: torch.device("cpu"))
+    monkeypatch.setattr(K, "_stream", lambda dev: 0)
+    monkeypatch.setattr(K, "relayout_tiled", lambda w, s, shape: torch.zeros(128, dtype=torch.uint8))
+    monkeypatch.setattr(K, "_workspaces", {})
+    monkeypatch.setattr(K, "_relayout_cache", {})
+    monkeypatch.setattr(K, "_relayout_bytes", [0])
+    monkeypatch.setattr(K, "_cluster_sizes", {})
+    return K, calls
+
+
+@pytest.mark.parametrize("rows", [1, 16, 17, 129])
+def test_a_matmul_right_behind_its_copy_is_no_dependent_launch(launches, rows):
+    """A dependent launch reads weights before it waits for the launch in front of it: not behind the one that writes
+    the copy, neither the first time nor when it is made again for weights written in place, or when another weight's
+    entry goes away meanwhile."""
+    import torch
+    K, calls = launches
+    Kd, N = 64, 256
+    w, s = torch.zeros((Kd * N // 128, 64), dtype=torch.int8), torch.zeros(Kd * N // 64, dtype=torch.float16)
+    a = torch.zeros((rows, Kd), dtype=torch.float16)
+    run = lambda w=w: K.matmul_q40(a, w, s, (Kd, N))
+    run(), run()
+    w.add_(1)
+    run(), run()
+    s.add_(1)
+    run(), run()
+    other = w.clone()
+    run(other)
+    relayout = K.relayout_tiled
+
+    def drop_other(*args):
+        nonlocal other
+        other = None                       # its entry is dropped while this weight's new copy is made
+        return relayout(*args)
+
+    K.relayout_tiled = drop_other
+    w.add_(1)
+    run(), run()
+    assert [p for _, p in calls] == [False, True, False, True, False, True, False, False, True]

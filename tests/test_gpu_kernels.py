@@ -657,3 +657,19 @@ def test_matmul_tiled_tc_short_and_long_k_ranges(K, M, Kd):
     ref = O.matmul_q40(a, q, s, (Kd, N))
     scale = max(1.0, float(np.abs(ref.astype(np.float32)).mean()))
     assert_close(host(c1), ref, atol=ATOL * scale)
+
+
+@pytest.mark.parametrize("M", [4, 16, 40, 200])
+def test_matmul_follows_weights_written_in_place(K, M):
+    """Each write is followed at once by the multiplication: its copy of the weight is read after it is written."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    Kd, N = 2048, 4096
+    mats = [K.quantize_q40((torch.randn((Kd, N), generator=g, device="cuda") * 0.05).half()) for _ in range(3)]
+    a = torch.randn((M, Kd), generator=g, device="cuda").half()
+    want = [K.matmul_q40(a, q, s, (Kd, N)) for q, s in mats]
+    w, sc = mats[0][0].clone(), mats[0][1].clone()
+    for i in range(30):
+        q, s = mats[i % 3]
+        w.copy_(q)
+        sc.copy_(s)
+        assert torch.equal(K.matmul_q40(a, w, sc, (Kd, N)), want[i % 3])
