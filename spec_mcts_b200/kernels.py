@@ -190,10 +190,11 @@ def matmul_q40(a: torch.Tensor, b_w: torch.Tensor, b_s: torch.Tensor, b_shape, *
     wide = (M > 16 and group_size == 64 and N % 256 == 0 and K % 64 == 0 and a.data_ptr() % 16 == 0 and
             c.stride(1) == 1 and c.stride(0) % 2 == 0 and c.data_ptr() % 4 == 0)
     if (wide or (small and N % 256 == 0)) and (relayout if relayout is not None else _relayout_cfg["enabled"]):
-        tiled, fresh = _tiled_copy_of(b_w, b_s, K, N)
+        st = _stream(dev)
+        tiled, plain = _tiled_copy_of(b_w, b_s, K, N, dev, st)
         # programmatic launch (weights requested while the previous kernel drains) except right after the
         # kernel that wrote the copy
-        if tiled is not None and (_tiled_matmul(dev, a, tiled, c, M, N, K, not fresh) or
+        if tiled is not None and (_tiled_matmul(dev, a, tiled, c, M, N, K, not plain, st) or
                                   (small and _stream_gemv(dev, a, tiled, c, M, N, K))):
             return c
     if small and N % 128 == 0 and _cluster_gemv(dev, a, b_w, b_s, c, M, N, K):
@@ -208,7 +209,8 @@ def matmul_q40(a: torch.Tensor, b_w: torch.Tensor, b_s: torch.Tensor, b_shape, *
 
 _cluster_sizes = {}     # device index -> (largest cluster the device schedules for the decode matmul,): 16 or 8
 
-# tiled copies made for matmul_q40: id(b_w) -> (weakref to b_w, weakref to b_s, versions, (K, N), copy)
+# tiled copies made for matmul_q40: id(b_w) -> (weakref to b_w, weakref to b_s, versions, (K, N), addresses, copy,
+# event behind the kernel that wrote it, streams that are behind that event)
 _relayout_cfg = {"enabled": True, "max_bytes": 48 << 30}
 _relayout_cache: dict = {}
 _relayout_bytes = [0]
@@ -258,15 +260,30 @@ class TiledCopy:
         return type(None), ()       # pickled or copied with its owner: made again on first use
 
 
-def _tiled_copy_of(b_w, b_s, K, N):
-    """(copy or None, whether this call made it)."""
+def _recorded_event():
+    e = torch.cuda.Event()
+    e.record()
+    return e
+
+
+def _tiled_copy_of(b_w, b_s, K, N, dev, st):
+    """(copy or None, whether the launch that reads it has to be a plain one: it follows the kernel that writes the
+    copy, or is the first on a stream that has just been put behind it)."""
     key = id(b_w)
     ent = _relayout_cache.get(key)
     if ent is not None:
-        rw, rs, ver, shape, ptrs, copy = ent
+        rw, rs, ver, shape, ptrs, copy, event, streams = ent
         if (rw() is b_w and rs() is b_s and ver == _versions(b_w, b_s) and shape == (K, N)
                 and ptrs == (b_w.data_ptr(), b_s.data_ptr())):
-            return copy, False
+            if st in streams:
+                return copy, False
+            # a capture cannot wait for an event from outside of it (and begins on a device that has been waited for)
+            if not torch.cuda.is_current_stream_capturing():
+                here = torch.cuda.current_stream(dev)
+                here.wait_event(event)
+                copy.record_stream(here)
+                streams.add(st)
+            return copy, True
         _relayout_bytes[0] -= copy.numel()
         del _relayout_cache[key]
     nbytes = lib.q40_tiled_bytes(N, K)
@@ -280,19 +297,19 @@ def _tiled_copy_of(b_w, b_s, K, N):
             _relayout_bytes[0] -= e[5].numel()
 
     _relayout_cache[key] = (weakref.ref(b_w, _drop), weakref.ref(b_s), _versions(b_w, b_s), (K, N),
-                            (b_w.data_ptr(), b_s.data_ptr()), copy)
+                            (b_w.data_ptr(), b_s.data_ptr()), copy, _recorded_event(), {st})
     _relayout_bytes[0] += nbytes
     return copy, True
 
 
-def _tiled_matmul(dev, a, tiled, c, M, N, K, pdl) -> bool:
+def _tiled_matmul(dev, a, tiled, c, M, N, K, pdl, st) -> bool:
     """q40_matmul_tiled on a tiled copy; False if this device cannot schedule the clusters (up to 16 rows) or its
     driver has no tensor-map encoder (above)."""
     # the error word of tc_error_flag(); the narrow kernel has no wait that could expire
     err = _workspace("gemm", dev, 4096, zero=True).data_ptr() + 4092 if M > 16 else None
     for cluster in (_cluster_sizes.get(dev.index) or (16, 8)):
         rc = lib.q40_matmul_tiled(tiled.data_ptr(), c.data_ptr(), c.stride(0), a.data_ptr(), a.stride(0), M, N, K, cluster,
-                                  err, 1 if pdl else 0, _stream(dev))
+                                  err, 1 if pdl else 0, st)
         if rc == 0:
             if M <= 16:
                 _cluster_sizes[dev.index] = (cluster,)

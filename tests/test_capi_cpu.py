@@ -127,6 +127,7 @@ def launches(monkeypatch):
     monkeypatch.setattr(K, "lib", SimpleNamespace(q40_matmul_tiled=matmul_tiled, q40_tiled_bytes=lambda N, Kd: 128))
     monkeypatch.setattr(K, "_need_cuda", lambda *t: torch.device("cpu"))
     monkeypatch.setattr(K, "_stream", lambda dev: 0)
+    monkeypatch.setattr(K, "_recorded_event", lambda: None, raising=False)
     monkeypatch.setattr(K, "relayout_tiled", lambda w, s, shape: torch.zeros(128, dtype=torch.uint8))
     monkeypatch.setattr(K, "_workspaces", {})
     monkeypatch.setattr(K, "_relayout_cache", {})
@@ -164,3 +165,33 @@ def test_a_matmul_right_behind_its_copy_is_no_dependent_launch(launches, rows):
     w.add_(1)
     run(), run()
     assert [p for _, p in calls] == [False, True, False, True, False, True, False, False, True]
+
+
+def test_a_matmul_on_another_stream_waits_for_the_copy(launches, monkeypatch):
+    """The copy is written on the stream that first used the weight: another stream waits for it once, by a plain
+    launch, and the copy's memory is not given back under it.  A capturing stream cannot wait."""
+    import torch
+    K, calls = launches
+    Kd, N = 64, 256
+    w, s = torch.zeros((Kd * N // 128, 64), dtype=torch.int8), torch.zeros(Kd * N // 64, dtype=torch.float16)
+    a = torch.zeros((20, Kd), dtype=torch.float16)
+    stream, capturing, log = [1], [False], []
+
+    class Stream:
+        def wait_event(self, e):
+            log.append((stream[0], "waits", e))
+
+    class Copy(torch.Tensor):
+        def record_stream(self, _):
+            log.append((stream[0], "holds"))
+
+    monkeypatch.setattr(K, "_stream", lambda dev: stream[0])
+    monkeypatch.setattr(K, "_recorded_event", lambda: "copied")
+    monkeypatch.setattr(K, "relayout_tiled", lambda *args: torch.zeros(128, dtype=torch.uint8).as_subclass(Copy))
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: Stream())
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing[0])
+    for st, capture in ((1, False), (1, False), (2, False), (2, False), (3, True), (3, True), (3, False), (3, False), (1, False)):
+        stream[0], capturing[0] = st, capture
+        K.matmul_q40(a, w, s, (Kd, N))
+    assert [p for _, p in calls] == [False, True, False, True, False, False, False, True, True]
+    assert log == [(2, "waits", "copied"), (2, "holds"), (3, "waits", "copied"), (3, "holds")]

@@ -673,3 +673,23 @@ def test_matmul_follows_weights_written_in_place(K, M):
         w.copy_(q)
         sc.copy_(s)
         assert torch.equal(K.matmul_q40(a, w, sc, (Kd, N)), want[i % 3])
+
+
+@pytest.mark.parametrize("M", [4, 40, 200])
+def test_matmul_on_a_second_stream_reads_a_finished_copy(K, M):
+    """The weight's first use is held up on one stream; a second stream multiplies by the same weight meanwhile."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    Kd, N = 2048, 4096
+    a = torch.randn((M, Kd), generator=g, device="cuda").half()
+    q, s = K.quantize_q40((torch.randn((Kd, N), generator=g, device="cuda") * 0.05).half())
+    want = K.matmul_q40(a, q, s, (Kd, N))
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    w, sc = q.clone(), s.clone()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(one):
+        torch.cuda._sleep(20_000_000)           # about 10 ms
+        first = K.matmul_q40(a, w, sc, (Kd, N))
+    with torch.cuda.stream(two):
+        second = [K.matmul_q40(a, w, sc, (Kd, N)) for _ in range(3)]
+    torch.cuda.synchronize()
+    assert all(torch.equal(x, want) for x in (first, *second))
