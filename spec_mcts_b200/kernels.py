@@ -284,6 +284,10 @@ def _tiled_copy_of(b_w, b_s, K, N, dev, st):
                 copy.record_stream(here)
                 streams.add(st)
             return copy, True
+    # a copy made inside a capture would hold nothing until the graph runs: the checkpoint layout is read there
+    if torch.cuda.is_current_stream_capturing():
+        return None, False
+    if ent is not None:
         _relayout_bytes[0] -= copy.numel()
         del _relayout_cache[key]
     nbytes = lib.q40_tiled_bytes(N, K)

@@ -298,10 +298,11 @@ class Transformer(nn.Module):
         hid = self.layers[0].feed_forward.hidden_dim
         # tiled copies are made ahead of the pass: a dependent launch reads its weights before it waits for the
         # launch in front of it, which must not be the one that writes them
-        plan = []
+        plan, capturing = [], torch.cuda.is_current_stream_capturing()
         for layer in self.layers:
             att, ff = layer.attention, layer.feed_forward
-            plan.append([(lins, self._tiled_of(lins)[0] if self._prefill_tiled(S, lins) else self._drop_stale(lins))
+            plan.append([(lins, self._tiled_of(lins)[0] if self._prefill_tiled(S, lins, capturing)
+                          else None if capturing else self._drop_stale(lins))
                          for lins in ([att.wq, att.wk, att.wv], [att.wo], [ff.w1, ff.w3], [ff.w2])])
         h = self.tok_embeddings(tokens.to(dev)).to(DTYPE).view(S, p.dim)
         pos = torch.arange(S, dtype=torch.int32, device=dev)
@@ -366,13 +367,15 @@ class Transformer(nn.Module):
         raises, and so does a later prompt pass once the word has reached the host."""
         return 0 if self._tc_err is None else int(self._tc_err.item())
 
-    def _prefill_tiled(self, M, lins):
-        """Whether the prompt pass multiplies these projections through their tiled copies."""
+    def _prefill_tiled(self, M, lins, capturing=False):
+        """Whether the prompt pass multiplies these projections through their tiled copies (a capture makes none: they
+        would hold nothing until the graph runs)."""
         return (M > 16 and self.use_tiled and self.use_tiled_tc and len(lins) <= 3 and
                 (self.prefill_tiled_tc or not self.prefill_checkpoint_layout) and
                 all(l.group_size == 64 and self._tileable(l) and l.kn()[0] % 64 == 0 for l in lins) and
                 # a write into an inference tensor is not counted, so a copy of it could be old
-                (self.prefill_tiled_tc or not any(l.w.is_inference() or l.s.is_inference() for l in lins)))
+                (self.prefill_tiled_tc or not any(l.w.is_inference() or l.s.is_inference() for l in lins)) and
+                not (capturing and any(self._tiled_copy(l) is None for l in lins)))
 
     def _mm(self, x, weights, outs, err, st):
         """outs[i] = x @ deq(W_i) for projections that share the activations x [M, K] (prompt pass): one tensor-core
@@ -494,14 +497,20 @@ class Transformer(nn.Module):
         that one writes a copy)."""
         out, pdl = [], self.use_pdl
         for l in lins:
-            c = getattr(l, "_tiled", None)
-            if c is None or not c.is_of(l.kn(), l.w, l.s):
-                if c is not None:
+            c = self._tiled_copy(l)
+            if c is None:
+                if getattr(l, "_tiled", None) is not None:
                     self.release_graphs()         # captured steps hold the address of the copy that goes away
                 c = l._tiled = K.TiledCopy(K.relayout_tiled(l.w, l.s, l.kn()), l.kn(), l.w, l.s)
                 pdl = False
             out.append(c.data)
         return out, pdl
+
+    @staticmethod
+    def _tiled_copy(l):
+        """The copy of a layer's weight that is there and up to date, or None."""
+        c = getattr(l, "_tiled", None)
+        return c if c is not None and c.is_of(l.kn(), l.w, l.s) else None
 
     def drop_tiled_copies(self):
         """Forget the rearranged weight copies (made again on the next step): for weights written in a way torch
@@ -516,8 +525,8 @@ class Transformer(nn.Module):
     def _drop_stale(self, lins):
         """Drop these layers' copies, and the captured steps that read them, if their weights have changed."""
         for l in lins:
-            c, cat = getattr(l, "_tiled", None), getattr(l, "_tiled_cat", None)
-            if c is not None and not c.is_of(l.kn(), l.w, l.s):
+            cat = getattr(l, "_tiled_cat", None)
+            if getattr(l, "_tiled", None) is not None and self._tiled_copy(l) is None:
                 self.release_graphs()
                 l._tiled = None
             if cat is not None and not cat.is_of(*self._concat_source(lins)):

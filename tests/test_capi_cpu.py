@@ -127,6 +127,7 @@ def launches(monkeypatch):
     monkeypatch.setattr(K, "lib", SimpleNamespace(q40_matmul_tiled=matmul_tiled, q40_tiled_bytes=lambda N, Kd: 128))
     monkeypatch.setattr(K, "_need_cuda", lambda *t: torch.device("cpu"))
     monkeypatch.setattr(K, "_stream", lambda dev: 0)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
     monkeypatch.setattr(K, "_recorded_event", lambda: None, raising=False)
     monkeypatch.setattr(K, "relayout_tiled", lambda w, s, shape: torch.zeros(128, dtype=torch.uint8))
     monkeypatch.setattr(K, "_workspaces", {})

@@ -693,3 +693,29 @@ def test_matmul_on_a_second_stream_reads_a_finished_copy(K, M):
         second = [K.matmul_q40(a, w, sc, (Kd, N)) for _ in range(3)]
     torch.cuda.synchronize()
     assert all(torch.equal(x, want) for x in (first, *second))
+
+
+@pytest.mark.parametrize("M", [4, 40])
+def test_matmul_whose_weight_is_first_seen_in_a_capture(K, M):
+    """The captured call, the graph's replay and the calls after the capture all multiply by the weight."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    Kd, N = 512, 1024
+    a = torch.randn((M, Kd), generator=g, device="cuda").half()
+    q, s = K.quantize_q40((torch.randn((Kd, N), generator=g, device="cuda") * 0.05).half())
+    deq = K.dequantize_q40(q, s, 64, (Kd, N)).float()
+    graph = torch.cuda.CUDAGraph()
+    out = torch.zeros((M, N), dtype=torch.float16, device="cuda")
+    for relayout in (True, False):               # workspaces and kernel attributes are set up ahead of a capture
+        K.matmul_q40(a, q.clone(), s.clone(), (Kd, N), relayout=relayout)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        K.matmul_q40(a, q.clone(), s.clone(), (Kd, N), relayout=False)
+        side.synchronize()
+        with torch.cuda.graph(graph, stream=side):
+            K.matmul_q40(a, q, s, (Kd, N), out=out)
+    eager = K.matmul_q40(a, q, s, (Kd, N))
+    graph.replay()
+    torch.cuda.synchronize()
+    ref = a.float() @ deq
+    for y in (eager, out, K.matmul_q40(a, q, s, (Kd, N))):
+        assert_close(host(y), ref.cpu().numpy())

@@ -414,3 +414,23 @@ def test_expired_wait_of_a_prompt_pass_is_reported_before_its_first_use():
     expire()
     with pytest.raises(KK.Q40Error):
         m(prompt, 0)
+
+
+def test_prompt_pass_first_seen_in_a_capture():
+    """A captured prompt pass of a model without tiled copies, the eager passes after it, and the graph's replay."""
+    prompt = torch.arange(40, device="cuda").view(1, -1)
+    want = small_random()(prompt, 0).clone()
+    m = small_random()
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.stream(side):
+        m.prefill_checkpoint_layout = True       # workspaces are made ahead of the capture, copies are not
+        checkpoint = m(prompt, 0).clone()
+        m.prefill_checkpoint_layout = False
+        side.synchronize()
+        with torch.cuda.graph(graph, stream=side):
+            out = m(prompt, 0)
+    torch.cuda.current_stream().wait_stream(side)
+    assert torch.equal(m(prompt, 0), want)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, checkpoint)
