@@ -280,7 +280,8 @@ int q40_attn_decode(const void* q, const void* k, const void* v, void* o, int B,
 /* Paged decode attention.  kpool/vpool [Hkv, P, D] fp16 hold P token slots per kv head.
  * page_tbl[B, tbl_stride] (idx_bytes = 2: int16, 4: int32) lists page ids; token t of
  * branch b is slot page_tbl[b][t / page_size] * page_size + t % page_size.  seq_lens[B]
- * int32 gives each branch's length, or NULL = every branch has length Lmax.
+ * int32 gives each branch's length, or NULL = every branch has length Lmax.  Entries of page_tbl beyond
+ * a branch's length are not read and need not exist.
  * page_size = 1 with an int16 table is the reference's layout.
  * Replaces: page_flash_attn (triton_kernels.py:700-789). */
 int q40_attn_paged(const void* page_tbl, int idx_bytes, int64_t tbl_stride, const int32_t* seq_lens,

@@ -719,3 +719,32 @@ def test_matmul_whose_weight_is_first_seen_in_a_capture(K, M):
     ref = a.float() @ deq
     for y in (eager, out, K.matmul_q40(a, q, s, (Kd, N))):
         assert_close(host(y), ref.cpu().numpy())
+
+
+@pytest.mark.parametrize("page_size,idx", [(1, torch.int16), (16, torch.int32)])
+@pytest.mark.parametrize("B,H", [(3, 8), (10, 32), (30, 32), (80, 32)])      # each split of the warps over a row
+def test_page_table_shorter_than_the_longest_suffix_allowed(K, page_size, idx, B, H):
+    """max_suffix beyond the table's width, on a table that is a column range of a wider buffer whose last row ends
+    with the storage: the lengths say what is read."""
+    g = torch.Generator(device="cuda").manual_seed(B)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").half()
+    pages, P, limit = 3, 64 * page_size, 40 * page_size
+    wide = torch.randint(0, 64, (B, 40), generator=g, device="cuda").to(idx)
+    tbl = wide.view(-1)[37:].as_strided((B, pages), (40, 1))
+    lens = torch.randint(0, pages * page_size + 1, (B,), generator=g, device="cuda", dtype=torch.int32)
+    lens[-1] = pages * page_size
+    q, k, v, pk, pv = rnd(B, H, 128), rnd(H, P, 128), rnd(H, P, 128), rnd(20, H, 128), rnd(20, H, 128)
+    full = tbl.contiguous()
+    want = K.shared_prefix_attn(q, pk, pv, 20, full, lens, k, v, page_size=page_size)
+    got = K.shared_prefix_attn(q, pk, pv, 20, tbl, lens, k, v, page_size=page_size, max_suffix=limit)
+    assert torch.equal(got, want)
+    alone = K.page_flash_attn(full, q, k, v, P, B, pages * page_size, H, 128, page_size=page_size, seq_lens=lens)
+    got = K.page_flash_attn(tbl, q, k, v, P, B, limit, H, 128, page_size=page_size, seq_lens=lens)
+    assert torch.equal(got, alone)
+    at = torch.arange(pages * page_size, device="cuda")
+    slot = full.long()[:, at // page_size] * page_size + at % page_size
+    kb, vb = (t[:, slot].permute(1, 0, 2, 3).float() for t in (k, v))
+    sc = torch.einsum("bhd,bhld->bhl", q.float(), kb) / 128 ** 0.5
+    sc = sc.masked_fill(at[None, None] >= lens[:, None, None], float("-inf"))
+    ref = torch.einsum("bhl,bhld->bhd", torch.softmax(sc, -1).nan_to_num(0.0), vb)
+    assert_close(host(alone.view(B, H, 128)), ref.cpu().numpy())
