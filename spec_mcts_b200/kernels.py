@@ -397,6 +397,10 @@ def relayout_tiled(b_w: torch.Tensor, b_s: torch.Tensor, b_shape) -> torch.Tenso
     """Tiled copy (uint8 tensor) of a packed [K, N] matrix for gemv_fused(..., tiled=True)."""
     dev = _need_cuda(b_w, b_s)
     K, N = int(b_shape[0]), int(b_shape[1])
+    if b_s.dtype != torch.float16 or b_w.element_size() != 1:
+        raise Q40Error(f"relayout_tiled: packed bytes and fp16 scales required, got {b_w.dtype} and {b_s.dtype}")
+    if b_w.numel() * 2 != K * N or b_s.numel() * GROUP_SIZE != K * N:
+        raise Q40Error("relayout_tiled: packed weight / scale sizes do not match b_shape")
     nbytes = lib.q40_tiled_bytes(N, K)
     if nbytes == 0:
         raise Q40Error(f"relayout_tiled: shape ({K}, {N}) needs N % 256 == 0 and K % 16 == 0")

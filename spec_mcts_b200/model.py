@@ -296,6 +296,8 @@ class Transformer(nn.Module):
         dev = self.device
         H, Hkv, D = self._H, self._Hkv, self._D
         hid = self.layers[0].feed_forward.hidden_dim
+        # what the launches below take as bare addresses: not loaded yet, or another device's
+        K._need_cuda(self.norm.weight, *[n.weight for l in self.layers for n in (l.attention_norm, l.ffn_norm)])
         # tiled copies are made ahead of the pass: a dependent launch reads its weights before it waits for the
         # launch in front of it, which must not be the one that writes them
         plan, capturing = [], torch.cuda.is_current_stream_capturing()
@@ -383,6 +385,9 @@ class Transformer(nn.Module):
         import ctypes
         lins, tiled = weights
         n = len(lins)
+        for l, o in zip(lins, outs):
+            if l.kn() != (x.shape[1], o.shape[1]):
+                raise K.Q40Error(f"prompt pass: a projection of shape {l.kn()} where {(x.shape[1], o.shape[1])} is expected")
         if tiled is not None:
             P = ctypes.c_void_p * n
             check(lib.q40_gemm_tiled_tc_multi(n, x.data_ptr(), x.stride(0), P(*[t.data_ptr() for t in tiled]),
@@ -832,7 +837,7 @@ class Transformer(nn.Module):
         """out = RMSNorm(h + residual) with h updated in place (residual may be None)."""
         p = self.params
         check(lib.q40_rmsnorm(h.data_ptr(), residual.data_ptr() if residual is not None else None,
-                              weight.data_ptr(), out.data_ptr(), h.data_ptr() if residual is not None else None,
+                              weight.contiguous().data_ptr(), out.data_ptr(), h.data_ptr() if residual is not None else None,
                               h.shape[0], p.dim, float(p.norm_eps), st), "q40_rmsnorm")
 
     def _decode(self, tokens, start_pos):

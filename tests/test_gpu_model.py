@@ -434,3 +434,40 @@ def test_prompt_pass_first_seen_in_a_capture():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, checkpoint)
+
+
+@pytest.mark.parametrize("S", [8, 40])
+@pytest.mark.parametrize("broken", ["norm on the host", "last norm on the host", "scales too few", "codes too few",
+                                    "scales in fp32", "shape turned round", "too narrow"])
+def test_prompt_pass_refuses_weights_it_cannot_read(broken, S):
+    """What a loader can get wrong is refused before the launch that would read it."""
+    from spec_mcts_b200 import kernels as KK
+    m = small_random()
+    l = m.layers[1].feed_forward.w1
+    if broken == "norm on the host":
+        m.layers[1].ffn_norm.weight = torch.nn.Parameter(torch.ones(512, dtype=torch.float16), requires_grad=False)
+    elif broken == "last norm on the host":
+        m.norm.weight = torch.nn.Parameter(torch.ones(512, dtype=torch.float16), requires_grad=False)
+    elif broken == "scales too few":
+        l.s = l.s[:-64].clone()
+    elif broken == "codes too few":
+        l.w = l.w[:-1].clone()
+    elif broken == "scales in fp32":
+        l.s = l.s.float()
+    elif broken == "shape turned round":
+        l.shape = (l.shape[1], l.shape[0])
+    else:
+        l.w, l.s = random_weights(0, 512, 1024)
+        l.shape = (1024, 512)
+    with pytest.raises(KK.Q40Error):
+        m(torch.arange(S, device="cuda").view(1, -1), 0)
+
+
+def test_prompt_pass_takes_strided_norm_weights():
+    prompt = torch.arange(40, device="cuda").view(1, -1)
+    m = small_random()
+    w = torch.rand(512, device="cuda").half()
+    m.norm.weight = m.layers[1].ffn_norm.weight = torch.nn.Parameter(w, requires_grad=False)
+    want = m(prompt, 0).clone()
+    m.norm.weight = m.layers[1].ffn_norm.weight = torch.nn.Parameter(w.repeat_interleave(2)[::2], requires_grad=False)
+    assert not m.norm.weight.is_contiguous() and torch.equal(m(prompt, 0), want)
