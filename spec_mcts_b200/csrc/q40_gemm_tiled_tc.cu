@@ -743,6 +743,18 @@ extern "C" int q40_gemm_tiled_tc_multi(int nmat, const void* a, int64_t lda, con
     spans += p.spans[i];
     widest = p.spans[i] > widest ? p.spans[i] : widest;
   }
+  // a grid has 65535 row chunks at most: more rows go in several launches
+  constexpr int LAUNCH_ROWS = 65535 * wide::MAX_ROWS;
+  if (M > LAUNCH_ROWS) {
+    for (int64_t m0 = 0; m0 < M; m0 += LAUNCH_ROWS) {
+      void* cm[3];
+      for (int i = 0; i < nmat; ++i) cm[i] = (__half*)c[i] + m0 * ldc[i];
+      const int rc = q40_gemm_tiled_tc_multi(nmat, (const __half*)a + m0 * lda, lda, bw_tiled, cm, ldc, n_cols,
+                                             M - m0 < LAUNCH_ROWS ? (int)(M - m0) : LAUNCH_ROWS, K, err, use_pdl, stream);
+      if (rc != Q40_OK) return rc;
+    }
+    return Q40_OK;
+  }
   EncodeTiledFn encode = ttc_encode_fn();
   if (!encode) return Q40_E_UNSUPPORTED;
   int sms = 0, dev = 0;
@@ -753,7 +765,6 @@ extern "C" int q40_gemm_tiled_tc_multi(int nmat, const void* a, int64_t lda, con
   const bool wide = M > ACC_COLS;
   const int max_rows = wide ? wide::MAX_ROWS : ACC_COLS;
   const int chunks = (M + max_rows - 1) / max_rows;
-  if (chunks > 65535) return Q40_E_SHAPE;
   p.nprob = nmat;
   p.M = M; p.K = K; p.Mpad = ((M + chunks - 1) / chunks + 15) / 16 * 16;
   p.split_acc = p.Mpad <= 64 ? 1 : 0;

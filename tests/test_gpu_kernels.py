@@ -748,3 +748,15 @@ def test_page_table_shorter_than_the_longest_suffix_allowed(K, page_size, idx, B
     sc = sc.masked_fill(at[None, None] >= lens[:, None, None], float("-inf"))
     ref = torch.einsum("bhl,bhld->bhd", torch.softmax(sc, -1).nan_to_num(0.0), vb)
     assert_close(host(alone.view(B, H, 128)), ref.cpu().numpy())
+
+
+def test_matmul_of_more_rows_than_one_launch_takes(K):
+    """65535 chunks of 256 rows fit a grid: rows on both sides of that, the last one alone in its launch."""
+    M, Kd, N = 65535 * 256 + 1, 64, 256
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q, s = K.quantize_q40((torch.randn((Kd, N), generator=g, device="cuda") * 0.3).half())
+    a = torch.randn((512, Kd), generator=g, device="cuda").half().repeat(M // 512 + 1, 1)[:M].contiguous()
+    c = K.matmul_q40(a, q, s, (Kd, N))
+    rows = torch.tensor([0, 255, 256, M // 2, M - 258, M - 257, M - 2, M - 1], device="cuda")
+    ref = a[rows].float() @ K.dequantize_q40(q, s, 64, (Kd, N)).float()
+    assert_close(host(c[rows]), ref.cpu().numpy())
