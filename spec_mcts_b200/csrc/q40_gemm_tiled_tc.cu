@@ -141,6 +141,14 @@ __device__ __forceinline__ uint32_t deq_pair(uint32_t a72, __half2 scale) {
   return h2_as_u32(__hmul2(__hsub2(u32_as_h2(a72), u32_as_h2(0x54805480u)), scale));
 }
 
+// A wait ran out: the error word, and a wait (with a limit as well) for the copies still on their way, the last S of the
+// `copied` k blocks at most: none may land in shared memory that this CTA has given back.  (The MMAs that were issued are
+// waited for through the `done` barrier, which every issuing thread commits to, also after giving up.)
+__device__ __noinline__ void give_up(int* err, uint32_t bar_full, int S, int copied) {
+  atomicExch(err, 1);
+  for (int i = max(0, copied - S); i < copied; ++i) mbar_wait(bar_full + 8 * (i % S), (uint32_t)((i / S) & 1));
+}
+
 // One 16-row step of a lane's two 16-row tiles: the tile words w0, w1 and the scales of k = 4t .. 4t + 3 to the
 // registers of columns 8 st + 2t, + 1 of st_16x256b_x4
 __device__ __forceinline__ void dequant_step(const unsigned char* w, const unsigned char* sc, uint32_t (&r)[2][16], int st) {
@@ -240,6 +248,7 @@ gemm_tiled_tc_kernel(const Params p, const __grid_constant__ CUtensorMap amap) {
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail);
   volatile int* s_failed = reinterpret_cast<volatile int*>(tail + 8);
   volatile int* s_issued = reinterpret_cast<volatile int*>(tail + 16);     // [2] k blocks issued per accumulator
+  volatile int* s_copied = reinterpret_cast<volatile int*>(tail + 24);     // k blocks whose copies were requested
 
   if (tid == 0) {
     *s_failed = 0;
@@ -280,7 +289,8 @@ gemm_tiled_tc_kernel(const Params p, const __grid_constant__ CUtensorMap amap) {
         tma_2d(ring + i * stage_bytes + RAW_PAD, &amap, kb + i * BK, 0, bar_full + 8 * i);
       Q40_STAMP(2);
       TTC_ROLE_DECL
-      for (int i = first; i < nblk; ++i) {
+      int i = first;
+      for (; i < nblk; ++i) {
         const int s = i % S;
         TTC_ROLE(0, i, 0);
         if (!mbar_wait(bar_mdone + 8 * s, (uint32_t)(((i / S) - 1) & 1))) { failed = true; break; }
@@ -290,6 +300,7 @@ gemm_tiled_tc_kernel(const Params p, const __grid_constant__ CUtensorMap amap) {
         tma_2d(ring + s * stage_bytes + RAW_PAD, &amap, kb + i * BK, 0, bar_full + 8 * s);
         TTC_ROLE(0, i, 2);
       }
+      *s_copied = i;
       TTC_ROLE_FLUSH(313);
       Q40_STAMP(3);
     }
@@ -337,7 +348,7 @@ gemm_tiled_tc_kernel(const Params p, const __grid_constant__ CUtensorMap amap) {
         commit(bar_mdone + 8 * s);                  // the stage and the A buffer may be refilled when the MMAs
         TTC_ROLE(1, i, 6);                          // of both accumulators are done
       }
-      if (!failed) commit(bar_done);                // all of this thread's MMAs
+      commit(bar_done);                             // all MMAs this thread has issued
     }
     __syncwarp();
     if (warp == 1) TTC_ROLE_FLUSH(312);
@@ -379,12 +390,11 @@ gemm_tiled_tc_kernel(const Params p, const __grid_constant__ CUtensorMap amap) {
     }
     if (warp == DQ_WARP0) TTC_ROLE_FLUSH(311);
   }
-  if (failed) *s_failed = 1;
-  if (!failed && !mbar_wait(bar_done, 0)) *s_failed = 1;
+  if (!mbar_wait(bar_done, 0) || failed) *s_failed = 1;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   __syncthreads();
   failed = *s_failed != 0;
-  if (failed && tid == 0) atomicExch(p.err, 1);
+  if (failed && tid == 0) give_up(p.err, bar_full, S, *s_copied);
   Q40_STAMP(4);
 
   // ---- accumulators -> fp32 tile [Mpad][256] in shared memory (over the ring, idle by now) -> split-K sum
@@ -507,6 +517,7 @@ gemm_tiled_wide_kernel(const Params p, const __grid_constant__ CUtensorMap amap)
   unsigned char* tail = gbase + ring_bytes + 8 * MAX_STAGES + 16 * NA + 16;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail);
   volatile int* s_failed = reinterpret_cast<volatile int*>(tail + 8);
+  volatile int* s_copied = reinterpret_cast<volatile int*>(tail + 12);     // k blocks whose copies were requested
 
   if (tid == 0) {
     *s_failed = 0;
@@ -549,13 +560,15 @@ gemm_tiled_wide_kernel(const Params p, const __grid_constant__ CUtensorMap amap)
       asm volatile("griddepcontrol.wait;" ::: "memory");
       for (int i = 0; i < first; ++i)
         tma_2d(ring + i * stage_bytes + RAW_PAD, &amap, kb + i * BK, m0, bar_full + 8 * i);
-      for (int i = first; i < nblk; ++i) {
+      int i = first;
+      for (; i < nblk; ++i) {
         const int s = i % S, j = i - S;                      // block j was the stage's last user
         if (!mbar_wait(bar_mdone + 8 * (j % NA), (uint32_t)((j / NA) & 1))) { failed = true; break; }
         mbar_expect_tx(bar_full + 8 * s, RAW_BYTES + b_bytes);
         tma_2d(ring + s * stage_bytes + RAW_PAD, &amap, kb + i * BK, m0, bar_full + 8 * s);
         weights(i, s);
       }
+      *s_copied = i;
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -573,7 +586,7 @@ gemm_tiled_wide_kernel(const Params p, const __grid_constant__ CUtensorMap amap)
                  (i > 0 || ks > 0) ? 1u : 0u);
         commit(bar_mdone + 8 * ab);
       }
-      if (!failed) commit(bar_done);
+      commit(bar_done);
     }
     __syncwarp();
   } else if (warp >= DQ_WARP0) {
@@ -603,12 +616,11 @@ gemm_tiled_wide_kernel(const Params p, const __grid_constant__ CUtensorMap amap)
       if (lane == 0) mbar_arrive(bar_afull + 8 * ab);
     }
   }
-  if (failed) *s_failed = 1;
-  if (!failed && !mbar_wait(bar_done, 0)) *s_failed = 1;
+  if (!mbar_wait(bar_done, 0) || failed) *s_failed = 1;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   __syncthreads();
   failed = *s_failed != 0;
-  if (failed && tid == 0) atomicExch(p.err, 1);
+  if (failed && tid == 0) give_up(p.err, bar_full, S, *s_copied);
 
   const int nranks = (int)cluster.num_blocks();
   const int n0 = span * SPAN + half * FEATS;
