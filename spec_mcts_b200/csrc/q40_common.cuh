@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/q40b200.h"
 
 #if defined(__CUDA_ARCH__) && (__CUDA_ARCH__ < 1000)
@@ -17,6 +19,19 @@
   } while (0)
 
 static inline bool q40_aligned(const void* p, size_t a) { return ((uintptr_t)p % a) == 0; }
+
+// Allow `kern` that much dynamic shared memory, once per device (`ready`: one bit each).  The limit is a property of the
+// kernel, not of a launch: set to the most any call needs, threads that meet here do not lower each other's.
+static inline cudaError_t q40_allow_smem(std::atomic<uint64_t>& ready, const void* kern, int bytes) {
+  int dev = -1;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+  if (ready.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) ready.fetch_or(bit, std::memory_order_release);
+  return e;
+}
 
 // Launch with programmatic stream serialization.  Kernels launched this way execute griddepcontrol.wait
 // before their first access to global memory, so for the caller the launch orders exactly like a plain

@@ -578,12 +578,14 @@ template <int G, int MT>
 static int launch_gemv_nk(const __half* x, int64_t ldx, const uint8_t* wq, const __half* ws, __half* y,
                           int64_t ldy, int M, int N, int K, void* workspace, cudaStream_t st) {
   const q40::NkPlan p = q40::plan_nk_rows(N, K, MT);
-  const int xmax = MT <= 2 ? 1024 : 512;        // 33 to 66 KB: what lets the CTAs of a wave share the SMs
-  const int xch = p.kchunk < xmax ? p.kchunk : xmax;
-  const size_t smem = ((size_t)MT * 8 * (xch + q40::NK_XS_PAD) * 2 + 15) & ~(size_t)15;
+  constexpr int XMAX = MT <= 2 ? 1024 : 512;    // 33 to 66 KB: what lets the CTAs of a wave share the SMs
+  constexpr auto smem_of = [](int x) { return ((size_t)MT * 8 * (x + q40::NK_XS_PAD) * 2 + 15) & ~(size_t)15; };
+  const int xch = p.kchunk < XMAX ? p.kchunk : XMAX;
+  const size_t smem = smem_of(xch);
   auto kern = q40::gemv_nk_kernel<G, MT>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if constexpr (smem_of(XMAX) > 48 * 1024) {
+    static std::atomic<uint64_t> ready;
+    const cudaError_t e = q40_allow_smem(ready, (const void*)kern, (int)smem_of(XMAX));
     if (e != cudaSuccess) return (int)e;
   }
   dim3 grid(p.nblocks, p.nsplit);

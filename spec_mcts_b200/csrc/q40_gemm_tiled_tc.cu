@@ -54,6 +54,7 @@ constexpr int RAW_BYTES = 4 * STEP_BYTES;       // 8704: a k block of a span in 
 constexpr int RAW_PAD = 9216;                   // next multiple of 1024 (the B tile wants that alignment)
 constexpr int NA = 4;                           // A buffers (in tensor memory)
 constexpr int MAX_STAGES = 8;                   // a multiple of NA: block i owns barrier i % MAX_STAGES
+constexpr int SMEM_MAX = 227 * 1024;            // of a CTA
 constexpr unsigned SPIN_LIMIT = 1u << 22;       // polls of ~50 ns each before giving up
 
 struct Params {
@@ -699,14 +700,14 @@ static EncodeTiledFn ttc_encode_fn() {
   return (EncodeTiledFn)fn;
 }
 
-// How many clusters of (1, nsplit) CTAs with this much dynamic shared memory run at once (cached per
-// device, kernel, split and padded row class; 0 when the runtime cannot tell).
+// How many clusters of (1, nsplit) CTAs with this much dynamic shared memory run at once (an answer is
+// kept per device, kernel, split and padded row class; 0, not kept, when the runtime cannot tell).
 static int ttc_max_clusters(TtcKernel kern, bool wide, int threads, int mpad, int nsplit, size_t smem) {
-  static int cache_all[16][2][9][17] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) dev = 0;
-  int* cached = &cache_all[dev][wide][nsplit][mpad / 16];
-  if (*cached) return *cached - 1;
+  static std::atomic<int> cache_all[16][2][9][17] = {};
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  std::atomic<int>* cached = dev < 16 ? &cache_all[dev][wide][nsplit][mpad / 16] : nullptr;
+  if (cached && cached->load(std::memory_order_relaxed)) return cached->load(std::memory_order_relaxed) - 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(1024, nsplit, 1);
   cfg.blockDim = dim3(threads, 1, 1);
@@ -721,9 +722,9 @@ static int ttc_max_clusters(TtcKernel kern, bool wide, int threads, int mpad, in
   int n = 0;
   if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
     (void)cudaGetLastError();
-    n = 0;
+    return 0;
   }
-  *cached = n + 1;
+  if (cached) cached->store(n + 1, std::memory_order_relaxed);
   return n;
 }
 
@@ -797,7 +798,7 @@ extern "C" int q40_gemm_tiled_tc_multi(int nmat, const void* a, int64_t lda, con
   // ring depth: what fits, at most MAX_STAGES; the fp32 tile of the epilogue reuses the ring
   const size_t stage_bytes = (size_t)(wide ? wide::RAW_PAD : RAW_PAD) + (size_t)p.Mpad * 128;
   const size_t fixed = 1024 /* alignment slack */ + 256 /* barriers, tmem slot, flag */;
-  int stages = (int)((227 * 1024 - fixed) / stage_bytes);
+  int stages = (int)((SMEM_MAX - fixed) / stage_bytes);
   if (stages > MAX_STAGES) stages = MAX_STAGES;
   if (stages < 2) return Q40_E_UNSUPPORTED;
   p.stages = stages;
@@ -807,7 +808,8 @@ extern "C" int q40_gemm_tiled_tc_multi(int nmat, const void* a, int64_t lda, con
   const size_t smem = fixed + ring_bytes;
   TtcKernel kern = wide ? wide::gemm_tiled_wide_kernel : gemm_tiled_tc_kernel;
   const int threads = wide ? wide::THREADS : THREADS;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static std::atomic<uint64_t> ready[2];
+  cudaError_t e = q40_allow_smem(ready[wide], (const void*)kern, SMEM_MAX);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return Q40_E_UNSUPPORTED; }
   // split K over a cluster (<= 8 ranks, each with at least 4 k blocks).
   // Up to 128 rows: the split that minimises waves x (k blocks per rank + a fixed cost of about 10 k blocks for

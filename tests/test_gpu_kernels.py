@@ -760,3 +760,38 @@ def test_matmul_of_more_rows_than_one_launch_takes(K):
     rows = torch.tensor([0, 255, 256, M // 2, M - 258, M - 257, M - 2, M - 1], device="cuda")
     ref = a[rows].float() @ K.dequantize_q40(q, s, 64, (Kd, N)).float()
     assert_close(host(c[rows]), ref.cpu().numpy())
+
+
+def test_calls_of_different_sizes_from_two_threads(K):
+    """What a launch sets up for a kernel serves every size: threads with few and with many rows (and k) do not undo
+    each other's."""
+    import threading
+    g = torch.Generator(device="cuda").manual_seed(1)
+    cases = []
+    for M, Kd, op in ((20, 512, "kn"), (128, 512, "kn"), (130, 512, "kn"), (256, 512, "kn"), (64, 384, "nk"), (64, 2048, "nk")):
+        shape = (Kd, 256) if op == "kn" else (256, Kd)
+        q, s = K.quantize_q40((torch.randn(shape, generator=g, device="cuda") * 0.1).half())
+        x = torch.randn((M, Kd), generator=g, device="cuda").half()
+        fn = K.matmul_q40 if op == "kn" else K.linear_q40
+        cases.append((fn, x, q, s, shape, fn(x, q, s, shape)))
+    bad = []
+
+    def work(case):
+        fn, x, q, s, shape, want = case
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(1500):
+                    y = fn(x, q, s, shape)
+                if not torch.equal(y, want):
+                    bad.append((fn.__name__, tuple(x.shape), "other result"))
+        except Exception as e:
+            bad.append((fn.__name__, tuple(x.shape), repr(e)))
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(c,)) for c in cases]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not bad, bad
