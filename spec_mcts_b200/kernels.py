@@ -357,6 +357,11 @@ def _cluster_gemv(dev, a, b_w, b_s, c, M, N, K) -> bool:
     return False
 
 
+def _indexed(dev) -> torch.device:
+    """`dev`, or the current device where it is None or names none."""
+    return torch.device("cuda", torch.cuda.current_device()) if dev is None or dev.index is None else dev
+
+
 def _tc_error_word(dev) -> torch.Tensor:
     """The int32 device word behind tc_error_flag(), for this stream."""
     return _workspace("gemm", dev, 4096, zero=True)[4092:4096].view(torch.int32)
@@ -365,7 +370,7 @@ def _tc_error_word(dev) -> torch.Tensor:
 def tc_error_flag(dev=None) -> int:
     """1 if a tensor-core matmul launched through matmul_q40 or a prompt pass on the current stream of `dev` gave up
     on one of its bounded waits since the workspace was created (synchronises the device)."""
-    dev = torch.device("cuda", torch.cuda.current_device()) if dev is None else dev
+    dev = _indexed(dev)
     buf = _workspaces.get(("gemm", dev.index, _stream(dev)))
     if buf is None:
         return 0
@@ -550,7 +555,7 @@ def gemv_stream(mode: int, a: torch.Tensor, weights, *, norm_w=None, ss_in=None,
 def stream_status(dev=None) -> int:
     """Status word of the stream-K launches made through this module on the current stream of `dev`
     (non-zero: a bounded wait inside a kernel expired; synchronises the device)."""
-    dev = torch.device("cuda", torch.cuda.current_device()) if dev is None else dev
+    dev = _indexed(dev)
     buf = _workspaces.get(("stream", dev.index, _stream(dev)))
     return 0 if buf is None else int(buf[:4].view(torch.int32).item())
 

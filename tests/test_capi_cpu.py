@@ -196,3 +196,23 @@ def test_a_matmul_on_another_stream_waits_for_the_copy(launches, monkeypatch):
         K.matmul_q40(a, w, s, (Kd, N))
     assert [p for _, p in calls] == [False, True, False, True, False, False, False, True, True]
     assert log == [(2, "waits", "copied"), (2, "holds"), (3, "waits", "copied"), (3, "holds")]
+
+
+@pytest.mark.parametrize("dev", [None, "cuda", "cuda:1"])
+def test_status_calls_take_a_device_without_an_index(monkeypatch, dev):
+    """torch.device("cuda") is the current device."""
+    import torch
+    from spec_mcts_b200 import kernels as K
+
+    def raw_stream(index):
+        if not isinstance(index, int):
+            raise TypeError("an index is required")
+        return 7
+
+    words = torch.zeros(4096, dtype=torch.uint8)
+    words.view(torch.int32)[-1], words.view(torch.int32)[0] = 3, 5
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", raw_stream, raising=False)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 1)
+    monkeypatch.setattr(K, "_workspaces", {("gemm", 1, 7): words, ("stream", 1, 7): words})
+    dev = None if dev is None else torch.device(dev)
+    assert K.tc_error_flag(dev) == 3 and K.stream_status(dev) == 5
