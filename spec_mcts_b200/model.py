@@ -226,9 +226,11 @@ class Transformer(nn.Module):
         self.use_tp_fused_allreduce = True
         self.tp_wait_cycles = 0     # limit of the wait for a peer's rows in SM cycles (0: 2^31, about a second)
         self._tp_peer = None
-        # the prompt pass above 16 rows reads the tiled copies too (the decode step needs them anyway); True: it
-        # reads the checkpoint layout, unless prefill_tiled_tc asks for the copies
+        # the prompt pass above 16 rows reads the tiled copies too (the decode step needs them anyway); True: it reads
+        # the checkpoint layout and makes no copies
         self.prefill_checkpoint_layout = False
+        # the copies are also made of weights whose writes torch does not count (made under inference_mode), and the
+        # call waits for the device and raises itself if a wait in it ran out
         self.prefill_tiled_tc = False
         # True: the prompt pass returns logits of the last position only, [1, 1, vocab] (all a caller that
         # samples the next token needs); False: of every position like the reference
@@ -373,7 +375,7 @@ class Transformer(nn.Module):
         """Whether the prompt pass multiplies these projections through their tiled copies (a capture makes none: they
         would hold nothing until the graph runs)."""
         return (M > 16 and self.use_tiled and self.use_tiled_tc and len(lins) <= 3 and
-                (self.prefill_tiled_tc or not self.prefill_checkpoint_layout) and
+                not self.prefill_checkpoint_layout and
                 all(l.group_size == 64 and self._tileable(l) and l.kn()[0] % 64 == 0 for l in lins) and
                 # a write into an inference tensor is not counted, so a copy of it could be old
                 (self.prefill_tiled_tc or not any(l.w.is_inference() or l.s.is_inference() for l in lins)) and

@@ -242,9 +242,9 @@ def test_q4_lm_head_option(small):
 
 
 def test_prefill_tiled_tc_matches_default_prefill(small):
-    """The prompt pass through the tiled-copy tensor-core matmul (prefill_tiled_tc) against the default
-    prompt pass on the same model and against the reference class's logits: same logits within the matmul
-    tolerance, same prompt cache."""
+    """The prompt pass through the tiled-copy tensor-core matmul, with prefill_tiled_tc and by default, against the
+    reference class's logits within the matmul tolerance; same prompt cache.  (The checkpoint layout against the
+    copies: test_prompt_pass_on_either_layout.)"""
     g = small
     outs = []
     for flag in (False, True):
@@ -471,3 +471,24 @@ def test_prompt_pass_takes_strided_norm_weights():
     want = m(prompt, 0).clone()
     m.norm.weight = m.layers[1].ffn_norm.weight = torch.nn.Parameter(w.repeat_interleave(2)[::2], requires_grad=False)
     assert not m.norm.weight.is_contiguous() and torch.equal(m(prompt, 0), want)
+
+
+@pytest.mark.parametrize("S", [17, 40, 129, 160])       # both tiled tensor-core kernels, at their smallest and beyond
+@pytest.mark.parametrize("n_kv_heads", [4, 2, 1])       # kv projections of 512, 256 and 128 columns (not tileable)
+def test_prompt_pass_on_either_layout(S, n_kv_heads):
+    """prefill_checkpoint_layout reads that layout and makes no copies, the other settings read the copies; logits and
+    prompt cache agree within fp16 rounding of two summation orders over two layers (the model tests' 2e-2)."""
+    prompt = torch.arange(S, device="cuda").view(1, -1) * 5 % 512
+    res = []
+    for flags in ({"prefill_checkpoint_layout": True}, {}, {"prefill_tiled_tc": True}):
+        m = small_random(n_kv_heads=n_kv_heads)
+        for name, value in flags.items():
+            setattr(m, name, value)
+        logits = m(prompt, 0).float()
+        made = [getattr(l, "_tiled", None) is not None for layer in m.layers
+                for l in (layer.attention.wo, layer.feed_forward.w1, layer.feed_forward.w2)]
+        assert all(made) if res else not any(made)
+        res.append((logits, m._caches["pk"][:, :S].float(), m._caches["pv"][:, :S].float()))
+    for x, y, z in zip(*res):
+        assert torch.equal(y, z)
+        assert (x - y).norm() / x.norm() < 2e-2
