@@ -71,6 +71,15 @@ def test_new_entry_points_check_their_arguments():
     assert lib.q40_gemm_tiled_tc_multi(1, p16, 128, P1(p16), P1(p16), one64, bad_n, 20, 128, p16, 0, None) == -2
     assert lib.q40_gemm_tiled_tc_multi(1, p16, 128, P1(p16), P1(p16), one64, one32, 20, 128, None, 0, None) == -1
     assert lib.q40_gemm_tiled_tc_multi(4, p16, 128, P1(p16), P1(p16), one64, one32, 20, 128, p16, 0, None) == -5
+    # one projection on its tiled copy: no rows, K % 16 and cluster size (up to 16 rows), K % 64, N % 256, NULL error
+    # word, output pitch (above)
+    mm = lambda M, N, Kd, ldc=512, cluster=16, err=p16: lib.q40_matmul_tiled(p16, p16, ldc, p16, 128, M, N, Kd, cluster, err, 0, None)
+    assert mm(0, 512, 128) == -2 and mm(16, 512, 120) == -2 and mm(16, 384, 128) == -2
+    assert mm(16, 512, 128, cluster=4) == -5
+    assert mm(17, 512, 80) == -2 and mm(17, 384, 128) == -2 and mm(17, 512, 128, ldc=256) == -2
+    assert mm(17, 512, 128, err=None) == -1
+    assert lib.q40_matmul_tiled(None, p16, 512, p16, 128, 17, 512, 128, 16, p16, 0, None) == -1
+    assert lib.q40_matmul_tiled(p16, p16, 512, p16 + 2, 128, 4, 512, 128, 16, None, 0, None) == -3
     # causal attention: head dim, H % Hkv, row strides
     assert lib.q40_attn_causal(p16, 256, p16, 256, p16, 256, p16, 256, 4, 2, 2, 64, None) == -5
     assert lib.q40_attn_causal(p16, 384, p16, 256, p16, 256, p16, 384, 4, 3, 2, 128, None) == -2

@@ -795,3 +795,85 @@ def test_calls_of_different_sizes_from_two_threads(K):
         t.join()
     torch.cuda.synchronize()
     assert not bad, bad
+
+
+@pytest.mark.parametrize("pad,off", [(0, 0), (8, 8), (4, 0), (0, 1), (3, 5)])
+def test_rope_kv_append_on_any_rows(K, pad, off):
+    """Rows, tables and caches that are 16-byte aligned take one kernel, any others the other: the rotated bits are the
+    fp16 formula's, the cache rows the packer's, and nothing else is written."""
+    from spec_mcts_b200._lib import check, lib
+    g = torch.Generator(device="cuda").manual_seed(pad * 8 + off)
+    B, H, Hkv, D, maxB, maxT, plen, n_pos = 5, 6, 3, 128, 6, 9, 20, 40
+    W = (H + 2 * Hkv) * D + pad
+
+    def odd(*shape, scale=1.0):              # the same values, `off` elements behind a 16-byte boundary
+        n = int(np.prod(shape))
+        t = torch.empty(n + off, dtype=torch.float16, device="cuda")[off:].view(shape)
+        return t.copy_(torch.randn(shape, generator=g, device="cuda") * scale)
+
+    qkv = odd(B, W)
+    qkv[1, (H + Hkv) * D:(H + Hkv) * D + 64] = 0                      # a group of zeros, one with an infinity
+    qkv[2, (H + Hkv) * D + 3] = float("inf")
+    q, k, v = qkv[:, :H * D], qkv[:, H * D:(H + Hkv) * D], qkv[:, (H + Hkv) * D:(H + 2 * Hkv) * D]
+    before = qkv.clone()
+    cos, sin = odd(n_pos, D // 2), odd(n_pos, D // 2)
+    kq = torch.full((maxB, maxT, Hkv, 64), 7, dtype=torch.int8, device="cuda")
+    ks = torch.full((maxB, maxT, Hkv, 2), 7.0, dtype=torch.float16, device="cuda")
+    vq, vs = kq.clone(), ks.clone()
+    t = torch.tensor([0, 8, 3, -1, 9], device="cuda")                 # the last two lie outside the cache
+    pos = (t + plen).to(torch.int32)
+    plen_d = torch.tensor([plen], dtype=torch.int32, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    check(lib.q40_rope_kv_append(q.data_ptr(), W, k.data_ptr(), W, v.data_ptr(), W, pos.data_ptr(), plen_d.data_ptr(),
+                                 cos.data_ptr(), sin.data_ptr(), n_pos, kq.data_ptr(), ks.data_ptr(), vq.data_ptr(),
+                                 vs.data_ptr(), B, H, Hkv, D, maxT, st))
+
+    def rotated(x, heads):
+        x = x.reshape(B, heads, D)
+        c, s = cos[pos.long()][:, None], sin[pos.long()][:, None]
+        lo, hi = x[..., :64], x[..., 64:]
+        return torch.cat((lo * c + (-hi) * s, hi * c + lo * s), dim=-1)
+
+    kr = rotated(before[:, H * D:(H + Hkv) * D], Hkv)
+    assert torch.equal(q.reshape(B, H, D), rotated(before[:, :H * D], H)) and torch.equal(k.reshape(B, Hkv, D), kr)
+    assert torch.equal(qkv[:, (H + Hkv) * D:], before[:, (H + Hkv) * D:])
+    for x, codes, scales in ((kr, kq, ks), (v.reshape(B, Hkv, D), vq, vs)):
+        cq, cs = (y.cpu().numpy() for y in (codes, scales))
+        wq, ws = O.quantize_q40(x.cpu().numpy().reshape(-1, D), 64)
+        want_q, want_s = np.full_like(cq, 7), np.full_like(cs, 7.0)
+        for b in range(B):
+            if 0 <= int(t[b]) < maxT:
+                want_q[b, int(t[b])] = wq.reshape(B, Hkv, 64)[b]
+                want_s[b, int(t[b])] = ws.reshape(B, Hkv, 2)[b]
+        np.testing.assert_array_equal(cq, want_q)
+        assert_bits_equal(cs, want_s)
+
+
+@pytest.mark.parametrize("B,H,Hkv,plen", [(37, 32, 32, 40), (38, 32, 8, 40), (74, 32, 8, 700), (38, 32, 32, 0)])
+def test_tree_decode_on_both_sides_of_the_warp_split(K, B, H, Hkv, plen):
+    """1184 rows take four warps a row, more take two: packed suffixes of every length, merged with the partial
+    results of the shared prompt, against fp32 torch."""
+    from spec_mcts_b200._lib import check, lib
+    g = torch.Generator(device="cuda").manual_seed(B + H)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").half()
+    D, maxT, maxP = 128, 21, plen + 8
+    q, ck, cv, pk, pv = rnd(B, H, D), rnd(B, Hkv, D), rnd(B, Hkv, D), rnd(maxP, Hkv, D), rnd(maxP, Hkv, D)
+    packed = [K.quantize_q40(rnd(B, maxT, Hkv, D)) for _ in range(2)]
+    sk, sv = (K.dequantize_q40(c, s, 64, (B, maxT, Hkv, D)).float() for c, s in packed)
+    t = torch.randint(0, maxT + 1, (B,), generator=g, device="cuda", dtype=torch.int32)
+    t[0], t[-1] = 0, maxT
+    pos, plen_d = t + plen, torch.tensor([plen], dtype=torch.int32, device="cuda")
+    ws = torch.empty(lib.q40_attn_shared_prefix_workspace_bytes(B, H, D, maxP), dtype=torch.uint8, device="cuda")
+    o = torch.empty((B, H, D), dtype=torch.float16, device="cuda")
+    (kq, ks), (vq, vs) = packed
+    check(lib.q40_attn_tree_decode(q.data_ptr(), H * D, pk.data_ptr(), pv.data_ptr(), maxP, plen_d.data_ptr(), pk.stride(0),
+                                   pk.stride(1), kq.data_ptr(), ks.data_ptr(), vq.data_ptr(), vs.data_ptr(), maxT,
+                                   pos.data_ptr(), ck.data_ptr(), cv.data_ptr(), Hkv * D, o.data_ptr(), B, H, Hkv, D,
+                                   ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream))
+    keys, vals = (torch.cat((p[:plen].float().expand(B, -1, -1, -1), s, c.float()[:, None]), 1).repeat_interleave(H // Hkv, 2)
+                  for p, s, c in ((pk, sk, ck), (pv, sv, cv)))
+    sc = torch.einsum("bhd,blhd->bhl", q.float(), keys) / D ** 0.5
+    at = torch.arange(plen + maxT + 1, device="cuda")[None]
+    dead = (at >= plen + t[:, None]) & (at < plen + maxT)
+    ref = torch.einsum("bhl,blhd->bhd", torch.softmax(sc.masked_fill(dead[:, None], float("-inf")), -1), vals)
+    assert_close(host(o), ref.cpu().numpy())
