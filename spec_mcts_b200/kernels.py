@@ -241,20 +241,32 @@ def _versions(*ts):
     return tuple(out)
 
 
+def writes_counted(*ts: torch.Tensor) -> bool:
+    """Whether torch counts in-place writes into all of these (not into tensors made under inference_mode)."""
+    for t in ts:
+        if t.is_inference():
+            return False
+    return True
+
+
 class TiledCopy:
     """A tiled copy a model keeps and what it was made from: tensors (weakly), their addresses and in-place
     modification counters, and the (K, N) they were read as.  A write into a tensor made under inference_mode is not
     seen, nor is one through `.data` or a raw pointer."""
-    __slots__ = ("data", "shape", "_refs", "_ptrs", "_versions")
+    __slots__ = ("data", "shape", "_src", "_versions")
 
     def __init__(self, data: torch.Tensor, shape, *src: torch.Tensor):
         self.data, self.shape = data, tuple(shape)
-        self._refs, self._ptrs, self._versions = [weakref.ref(t) for t in src], [t.data_ptr() for t in src], _versions(*src)
+        self._src, self._versions = [(weakref.ref(t), t.data_ptr()) for t in src], _versions(*src)
 
     def is_of(self, shape, *src: torch.Tensor) -> bool:
         """Whether the copy still holds these tensors' contents."""
-        return (self.shape == shape and len(src) == len(self._refs) and self._versions == _versions(*src) and
-                all(r() is t and p == t.data_ptr() for r, p, t in zip(self._refs, self._ptrs, src)))
+        if self.shape != shape or len(src) != len(self._src) or self._versions != _versions(*src):
+            return False
+        for (ref, ptr), t in zip(self._src, src):
+            if ref() is not t or ptr != t.data_ptr():
+                return False
+        return True
 
     def __reduce__(self):
         return type(None), ()       # pickled or copied with its owner: made again on first use

@@ -17,6 +17,7 @@ What differs from the reference is how a decode step executes, not what it compu
 """
 from __future__ import annotations
 
+import ctypes
 from dataclasses import dataclass
 from typing import Optional
 
@@ -81,6 +82,7 @@ class LinearQ4_0(nn.Module):
                              device="meta")
         self.s = torch.empty(in_features * out_features // group_size, dtype=DTYPE, device="meta")
         self.shape = (in_features, out_features)
+        self._tiled = self._tiled_cat = None       # rearranged copies (kernels.TiledCopy), made on first use
 
     def kn(self):
         """(K, N) of the stored [K, N] matrix."""
@@ -298,40 +300,45 @@ class Transformer(nn.Module):
         dev = self.device
         H, Hkv, D = self._H, self._Hkv, self._D
         hid = self.layers[0].feed_forward.hidden_dim
-        # what the launches below take as bare addresses: not loaded yet, or another device's
-        K._need_cuda(self.norm.weight, *[n.weight for l in self.layers for n in (l.attention_norm, l.ffn_norm)])
-        # tiled copies are made ahead of the pass: a dependent launch reads its weights before it waits for the
-        # launch in front of it, which must not be the one that writes them
+        # K and the widths of the four matmuls of a layer, and whether their shapes are multiplied through tiled copies
+        sites = ((p.dim, (H * D, Hkv * D, Hkv * D)), (H * D, (p.dim,)), (p.dim, (hid, hid)), (hid, (p.dim,)))
+        copies_read = S > 16 and self.use_tiled and self.use_tiled_tc and not self.prefill_checkpoint_layout
+        tiled = [copies_read and Kd % 64 == 0 and all(n % 256 == 0 for n in Ns) for Kd, Ns in sites]
+        # copies are made ahead of the pass: a dependent launch reads its weights before it waits for the launch in
+        # front of it, which must not be the one that writes them
         plan, capturing = [], torch.cuda.is_current_stream_capturing()
         for layer in self.layers:
             att, ff = layer.attention, layer.feed_forward
-            plan.append([(lins, self._tiled_of(lins)[0] if self._prefill_tiled(S, lins, capturing)
-                          else None if capturing else self._drop_stale(lins))
-                         for lins in ([att.wq, att.wk, att.wv], [att.wo], [ff.w1, ff.w3], [ff.w2])])
+            lins = ((att.wq, att.wk, att.wv), (att.wo,), (ff.w1, ff.w3), (ff.w2,))
+            plan.append((att, layer.attention_norm.weight, layer.ffn_norm.weight,
+                         [(ls, self._prefill_copies(ls, *site, ok, capturing)) for ls, site, ok in zip(lins, sites, tiled)]))
+        # the norm launches take bare addresses: not loaded yet, or another device's
+        K._need_cuda(self.norm.weight, *[w for _, *ws, _ in plan for w in ws])
         h = self.tok_embeddings(tokens.to(dev)).to(DTYPE).view(S, p.dim)
         pos = torch.arange(S, dtype=torch.int32, device=dev)
         st = torch.cuda.current_stream(dev).cuda_stream
         err = K._tc_error_word(h.device)
         e = lambda n: torch.empty((S, n), dtype=DTYPE, device=dev)
         xn, q, ao, o, a1, a3, g, f = (e(n) for n in (p.dim, H * D, H * D, p.dim, hid, hid, hid, p.dim))
+        args = [self._mm_args(Ns) for _, Ns in sites]
         pending = None     # output of the previous sub-block, added to h by the next norm kernel
-        for layer, (qkv, wo, w13, w2) in zip(self.layers, plan):
-            att = layer.attention
+        for att, attn_norm, ffn_norm, (qkv, wo, w13, w2) in plan:
             # keys and values go straight to their place in the prompt cache
             ck, cv = att.cache_prompt_k[:S], att.cache_prompt_v[:S]
-            self._norm(h, pending, layer.attention_norm.weight, xn, st)
-            self._mm(xn, qkv, [q, ck.view(S, Hkv * D), cv.view(S, Hkv * D)], err, st)
-            K.rope_(q.view(S, H, D), pos, self._cos, self._sin)
-            K.rope_(ck, pos, self._cos, self._sin)
+            self._norm(h, pending, attn_norm, xn, st)
+            self._mm(xn, qkv, [q, ck.view(S, Hkv * D), cv.view(S, Hkv * D)], args[0], err, st)
+            for x, heads in ((q, H), (ck, Hkv)):
+                check(lib.q40_rope(x.data_ptr(), pos.data_ptr(), self._cos.data_ptr(), self._sin.data_ptr(), S, heads, D,
+                                   heads * D, st), "q40_rope")
             att.cache_prompt_len = S
             # causal attention over the prompt (grouped-query heads read their kv head directly)
             K.causal_attn(q.view(S, H, D), ck, cv, out=ao.view(S, H, D))
-            self._mm(ao, wo, [o], err, st)
+            self._mm(ao, wo, [o], args[1], err, st)
             self._all_reduce(o)
-            self._norm(h, o, layer.ffn_norm.weight, xn, st)
-            self._mm(xn, w13, [a1, a3], err, st)
+            self._norm(h, o, ffn_norm, xn, st)
+            self._mm(xn, w13, [a1, a3], args[2], err, st)
             check(lib.q40_silu_mul(a1.data_ptr(), a3.data_ptr(), g.data_ptr(), g.numel(), st), "q40_silu_mul")
-            self._mm(g, w2, [f], err, st)
+            self._mm(g, w2, [f], args[3], err, st)
             self._all_reduce(f)
             pending = f
         self._prefix_len_dev.fill_(S)
@@ -371,31 +378,36 @@ class Transformer(nn.Module):
         raises, and so does a later prompt pass once the word has reached the host."""
         return 0 if self._tc_err is None else int(self._tc_err.item())
 
-    def _prefill_tiled(self, M, lins, capturing=False):
-        """Whether the prompt pass multiplies these projections through their tiled copies (a capture makes none: they
-        would hold nothing until the graph runs)."""
-        return (M > 16 and self.use_tiled and self.use_tiled_tc and len(lins) <= 3 and
-                not self.prefill_checkpoint_layout and
-                all(l.group_size == 64 and self._tileable(l) and l.kn()[0] % 64 == 0 for l in lins) and
-                # a write into an inference tensor is not counted, so a copy of it could be old
-                (self.prefill_tiled_tc or not any(l.w.is_inference() or l.s.is_inference() for l in lins)) and
-                not (capturing and any(self._tiled_copy(l) is None for l in lins)))
+    def _prefill_copies(self, lins, Kd, Ns, tiled, capturing):
+        """The tiled copies that a prompt pass multiplies these projections through, or None where it reads the
+        checkpoint layout: `tiled` is false, or a copy could be old (a write into an inference tensor is not counted),
+        or would have to be made inside a capture (it would hold nothing until the graph runs)."""
+        for l, n in zip(lins, Ns):
+            if l.kn() != (Kd, n):
+                raise K.Q40Error(f"prompt pass: a projection of shape {l.kn()} where {(Kd, n)} is expected")
+            if tiled and (l.group_size != 64 or not (self.prefill_tiled_tc or K.writes_counted(l.w, l.s)) or
+                          (capturing and self._tiled_copy(l) is None)):
+                tiled = False
+        if tiled:
+            return self._tiled_of(lins)[0]
+        if not capturing:
+            self._drop_stale(lins)
+        return None
 
-    def _mm(self, x, weights, outs, err, st):
+    @staticmethod
+    def _mm_args(Ns):
+        """What the launches of one matmul of every layer share: array types and the output widths."""
+        n = len(Ns)
+        return n, ctypes.c_void_p * n, (ctypes.c_int64 * n)(*Ns), (ctypes.c_int * n)(*Ns)
+
+    def _mm(self, x, weights, outs, args, err, st):
         """outs[i] = x @ deq(W_i) for projections that share the activations x [M, K] (prompt pass): one tensor-core
-        launch when they have tiled copies, matmul_q40 per projection otherwise."""
-        import ctypes
+        launch when they have tiled copies, matmul_q40 per projection otherwise.  All operands are contiguous."""
         lins, tiled = weights
-        n = len(lins)
-        for l, o in zip(lins, outs):
-            if l.kn() != (x.shape[1], o.shape[1]):
-                raise K.Q40Error(f"prompt pass: a projection of shape {l.kn()} where {(x.shape[1], o.shape[1])} is expected")
         if tiled is not None:
-            P = ctypes.c_void_p * n
-            check(lib.q40_gemm_tiled_tc_multi(n, x.data_ptr(), x.stride(0), P(*[t.data_ptr() for t in tiled]),
-                                              P(*[o.data_ptr() for o in outs]),
-                                              (ctypes.c_int64 * n)(*[o.stride(0) for o in outs]),
-                                              (ctypes.c_int * n)(*[l.kn()[1] for l in lins]), x.shape[0], x.shape[1],
+            n, P, widths64, widths = args
+            check(lib.q40_gemm_tiled_tc_multi(n, x.data_ptr(), x.shape[1], P(*[t.data_ptr() for t in tiled]),
+                                              P(*[o.data_ptr() for o in outs]), widths64, widths, x.shape[0], x.shape[1],
                                               err.data_ptr(), 1 if self.use_pdl else 0, st),
                   "q40_gemm_tiled_tc_multi")
             return
@@ -434,7 +446,6 @@ class Transformer(nn.Module):
     def _gemm_multi(self, bufs, x, lins, outs, st):
         """Several projections of the same activations: one tensor-core launch above 16 rows when the
         shapes allow it, one launch per matrix otherwise."""
-        import ctypes
         M, n = x.shape[0], len(lins)
         if M > 16 and self.use_tiled and self.use_tiled_tc and x.stride(0) % 8 == 0:
             # matrices that have a tiled copy (N % 256 == 0) go through the tensor-core kernel that reads it;
@@ -506,7 +517,7 @@ class Transformer(nn.Module):
         for l in lins:
             c = self._tiled_copy(l)
             if c is None:
-                if getattr(l, "_tiled", None) is not None:
+                if l._tiled is not None:
                     self.release_graphs()         # captured steps hold the address of the copy that goes away
                 c = l._tiled = K.TiledCopy(K.relayout_tiled(l.w, l.s, l.kn()), l.kn(), l.w, l.s)
                 pdl = False
@@ -516,7 +527,7 @@ class Transformer(nn.Module):
     @staticmethod
     def _tiled_copy(l):
         """The copy of a layer's weight that is there and up to date, or None."""
-        c = getattr(l, "_tiled", None)
+        c = l._tiled
         return c if c is not None and c.is_of(l.kn(), l.w, l.s) else None
 
     def drop_tiled_copies(self):
@@ -532,8 +543,8 @@ class Transformer(nn.Module):
     def _drop_stale(self, lins):
         """Drop these layers' copies, and the captured steps that read them, if their weights have changed."""
         for l in lins:
-            cat = getattr(l, "_tiled_cat", None)
-            if getattr(l, "_tiled", None) is not None and self._tiled_copy(l) is None:
+            cat = l._tiled_cat
+            if l._tiled is not None and self._tiled_copy(l) is None:
                 self.release_graphs()
                 l._tiled = None
             if cat is not None and not cat.is_of(*self._concat_source(lins)):
@@ -566,7 +577,7 @@ class Transformer(nn.Module):
         and the second value of _tiled_of."""
         pdl = self.use_pdl
         first, src = lins[0], self._concat_source(lins)
-        c = getattr(first, "_tiled_cat", None)
+        c = first._tiled_cat
         if c is None or not c.is_of(*src):
             if c is not None:
                 self.release_graphs()
@@ -601,7 +612,6 @@ class Transformer(nn.Module):
 
     def _fused(self, mode, lins, outs, ldc, a, lda, M, norm_w=None, ss_in=None, ss_in_count=0, h_in=None,
                ldh=0, ss_out=None, ss_out_count=0, st=None, bufs=None):
-        import ctypes
         n = len(lins)
         P = ctypes.c_void_p * n
         tiled = self.use_tiled and M <= 16 and all(self._tileable(l) for l in lins)
