@@ -466,20 +466,32 @@ struct NkPlan {
   int nblocks, nsplit, kchunk;
 };
 
-// One wave: five CTAs of 128 threads fit an SM, and a few CTAs more than that would cost a second pass
-// (11008 x 4096 at 10 rows, 688 CTAs: 23.9 us with four per SM).
-static NkPlan plan_nk(int N, int K) {
+static NkPlan plan_nk_want(int N, int K, int want) {
   NkPlan p;
   p.nblocks = (N + NK_ROWS - 1) / NK_ROWS;
-  int want = 148 * 5 / p.nblocks;
   if (want < 1) want = 1;
   int kchunk = (K + want - 1) / want;
   kchunk = ((kchunk + NK_STEP_K - 1) / NK_STEP_K) * NK_STEP_K;
+  // 256 k at least, 512 where that still gives the SMs three CTAs each: a split's partial sums cost about 40 k
+  // (16 x 2048 x 8192: 704 CTAs of 384 k 18.5 us, 512 of 512 k 17.5 us)
   if (kchunk < 256) kchunk = 256;
+  if (kchunk < 512 && p.nblocks * ((K + 511) / 512) >= 500) kchunk = 512;
   if (kchunk > K) kchunk = K;
   p.kchunk = kchunk;
   p.nsplit = (K + kchunk - 1) / kchunk;
   return p;
+}
+
+// One wave: five CTAs of 128 threads fit an SM, and a few CTAs more than that would cost a second pass
+// (11008 x 4096 at 10 rows, 688 CTAs: 23.9 us with four per SM).  Four, if whole steps of k leave the fullest SM more
+// to do with five (9472 x 4096 at 10 rows: 5 x 896 k 20.5 us, 4 x 1024 k 18.6 us).  Where no split fits the wave, two of
+// a long k range level the SMs (32000 x 11008: 500 CTAs 93 us at one row, 1000 88 us).
+static NkPlan plan_nk(int N, int K) {
+  const int nblocks = (N + NK_ROWS - 1) / NK_ROWS;
+  const auto busiest = [](const NkPlan& p) { return (int64_t)((p.nblocks * p.nsplit + 147) / 148) * p.kchunk; };
+  if (2 * nblocks > 148 * 5) return plan_nk_want(N, K, K >= 8192 && (2 * nblocks + 147) / 148 < 2 * ((nblocks + 147) / 148) ? 2 : 1);
+  const NkPlan five = plan_nk_want(N, K, 148 * 5 / nblocks), four = plan_nk_want(N, K, 148 * 4 / nblocks);
+  return busiest(five) * 50 > busiest(four) * 51 ? four : five;
 }
 
 // The same for a launch of up to 8 mt > 16 rows: fewer splits, so that the partial sums need no more scratch
