@@ -354,7 +354,7 @@ __device__ __forceinline__ void nk_compute(float (&acc)[MT][4], const NkRegs& r,
   }
 }
 
-// MT: 8-row tiles of the batch per launch, up to 8 (a 16-row limit read the weights M/16 times); the activations
+// MT: 8-row tiles of the batch per launch, up to 8 (see nk_launch_rows); the activations
 // are staged xch k rows at a time (a multiple of DEPTH steps, or the whole k range).
 template <int G, int MT>
 __global__ void __launch_bounds__(GEMV_THREADS, MT <= 2 ? 5 : 3)
@@ -506,6 +506,20 @@ static NkPlan plan_nk_rows(int N, int K, int mt) {
   return p;
 }
 
+// Rows of the next launch when `left` are to go.  A wider launch reads the weights less often but has fewer splits,
+// that is fewer and longer CTAs, at three per SM and not five: 64 rows while a CTA's k range stays short or is no longer
+// than with 32, 32 rows up to 4096 k.  Microseconds with 64 / 32 / 16 rows a launch: 48 rows x 4096 x 1024: 18.0 / 26.9 /
+// 30.8; x 4096 x 11008: 107 / 68 / 70; x 512 x 11008: 38.5 / 46.6 / 55.8; 64 rows x 14336 x 4096: 89 / 104 / 125;
+// 24 rows x 14336 x 11008: - / 154 / 106.
+static int nk_launch_rows(int N, int K, int left) {
+  if (left > 32) {
+    const int k64 = plan_nk_rows(N, K, 8).kchunk;
+    if (k64 <= 1152 || (left > 48 && k64 <= 4096 && k64 == plan_nk_rows(N, K, 4).kchunk)) return left < 64 ? left : 64;
+  }
+  if (left > 16 && plan_nk_rows(N, K, 4).kchunk <= 4096) return left < 32 ? left : 32;
+  return left < 16 ? left : 16;
+}
+
 }  // namespace q40
 
 extern "C" int q40_gemm_kn_tc(const void* a, int64_t lda, const void* bw, const void* bs, void* c, int64_t ldc,
@@ -632,7 +646,7 @@ extern "C" int q40_gemm_nk(const void* x, int64_t ldx, const void* wq, const voi
   const __half* xh = (const __half*)x;
   __half* yh = (__half*)y;
   for (int m0 = 0; m0 < M;) {
-    const int left = M - m0, mc = left < 64 ? left : 64;
+    const int mc = q40::nk_launch_rows(N, K, M - m0);
     auto run = [&](auto launch) {
       return launch(xh + m0 * ldx, ldx, (const uint8_t*)wq, (const __half*)ws, yh + m0 * ldy, ldy, mc, N, K, workspace, st);
     };

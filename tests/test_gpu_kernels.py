@@ -877,3 +877,15 @@ def test_tree_decode_on_both_sides_of_the_warp_split(K, B, H, Hkv, plen):
     dead = (at >= plen + t[:, None]) & (at < plen + maxT)
     ref = torch.einsum("bhl,blhd->bhd", torch.softmax(sc.masked_fill(dead[:, None], float("-inf")), -1), vals)
     assert_close(host(o), ref.cpu().numpy())
+
+
+@pytest.mark.parametrize("M", [33, 48, 49, 64, 81])
+@pytest.mark.parametrize("N,Kd,G", [(100, 1152, 64), (4096, 2048, 64), (4096, 1024, 32), (24000, 1024, 64), (24000, 5120, 32)])
+def test_linear_nk_rows_of_a_launch(K, M, N, Kd, G):
+    """Above 16 rows a launch takes 64, 32 or 16 of them by the k range of a CTA: sizes on both sides of each choice,
+    against fp32 torch (fp16 operands and result, fp32 sums)."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    q, s = K.quantize_q40((torch.randn((N, Kd), generator=g, device="cuda") * 0.05).half(), G)
+    x = (torch.randn((M, Kd), generator=g, device="cuda") * 0.5).half()
+    ref = x.float() @ K.dequantize_q40(q, s, G, (N, Kd)).float().t()
+    assert_close(host(K.linear_q40(x, q, s, (N, Kd), group_size=G)), ref.cpu().numpy())
