@@ -364,7 +364,8 @@ gemv_tiled_kernel(const TiledParams p) {
   // ---- split-K over the cluster: rank r finishes columns [r*slice, (r+1)*slice) of the span from the
   // partials it received (added in rank order) ----
   const int npart = (EPI == EPI_SILU) ? nranks / 2 : nranks;
-#pragma unroll
+  // unrolled only where a row's residual values wait in registers: 10 x 11008 x 4096, plain: 16.4 us, unrolled 16.7
+#pragma unroll (EPI == EPI_RESIDUAL ? RPW : 1)
   for (int mr = 0; mr < RPW; ++mr) {
     const int m = warp + mr * FW;
     if (m >= p.M) break;
