@@ -342,9 +342,10 @@ static int launch_rows(const BranchArgs& a, cudaStream_t st) {
 // unless a step is named:
 //   contiguous: four warps, four keys in flight; two warps a row are the same within 2 % at any width
 //   paged: eight warps while three CTAs an SM hold all rows (320 rows x 512 keys: 24.7 against 28.7) and there is
-//     more than a row per SM; then four warps with two keys in flight, which leaves room for a fifth CTA
-//     (1920 rows x 300 keys: 58.4 against 61.5 with four keys, 59.4 with two warps a row; 640 rows: 25.6 against
-//     27.6 and 31.7); above one wave of those two warps a row (3200 rows: 48.2 against 52.2)
+//     more than a row per SM; then four warps with four keys in flight while four CTAs an SM hold all rows (512 rows x
+//     512 keys: 23.5 against 25.8 with two keys), with long rows of different lengths a fifth, for the short ones make room
+//     (608 rows of up to 768 keys: 31.0 against 34.9; of up to 128: 9.4 against 7.8); then two keys, which lets a fifth CTA in (608 rows x 512 keys: 26.5 against 36.5;
+//     1920 rows x 300 keys: 58.4 against 61.5); two warps a row above 16 rows an SM (3200 rows: 48.2 against 52.2)
 //   Q4_0 cache (a quarter of the bytes): two warps a row once four fill more than two waves (a decode step of 3200
 //     rows: 4.58 against 4.77 ms)
 template <int MODE>
@@ -352,7 +353,7 @@ static int launch_branch_mode(const BranchArgs& a, cudaStream_t st) {
   if constexpr (MODE == 1 || MODE == 2) {
     if (a.rows > 148 && a.rows <= 3 * 148) return launch_rows<MODE, 8, 8, 2>(a, st);
     if (a.rows > 16 * 148) return launch_rows<MODE, 4, 2, 4>(a, st);
-    if (a.rows > 148) return launch_rows<MODE, 4, 4, 2>(a, st);
+    if (a.rows > (a.seq_lens && a.L > 256 ? 5 : 4) * 148) return launch_rows<MODE, 4, 4, 2>(a, st);
   }
   if constexpr (MODE == 3) {
     if (a.rows > 8 * 148) return launch_rows<MODE, 4, 2, 4>(a, st);
