@@ -311,12 +311,24 @@ attn_branch_kernel(const BranchArgs a) {
       for (int j = 0; j < DP; ++j) acc[j] = fmaf(sm_o[g0 + gI][tr + j * RT], w, acc[j]);
     }
     const float pw_l = exp2f(pm_l - M);
-#pragma unroll 4
-    for (int sp = 0; sp < min(a.nsp, 32); ++sp) {
-      const float w = __shfl_sync(0xffffffffu, pw_l, sp);
-      Lsum = fmaf(__shfl_sync(0xffffffffu, pl_l, sp), w, Lsum);
+    // four splits' outputs requested together (splits from nsp on: weight and sum are 0): between the shuffles the loads
+    // waited for one another (a branch over 1000 shared keys of 8 kv heads, 16 splits: 20.7 us)
+    constexpr int PB = 4;
+    const int nsp32 = min(a.nsp, 32);
+    for (int sp0 = 0; sp0 < nsp32; sp0 += PB) {
+      float po[PB][DP];
 #pragma unroll
-      for (int j = 0; j < DP; ++j) acc[j] = fmaf(a.po[((int64_t)sp * rows + bh) * D + tr + j * RT], w, acc[j]);
+      for (int i = 0; i < PB; ++i)
+#pragma unroll
+        for (int j = 0; j < DP; ++j)
+          po[i][j] = sp0 + i < nsp32 ? a.po[((int64_t)(sp0 + i) * rows + bh) * D + tr + j * RT] : 0.f;
+#pragma unroll
+      for (int i = 0; i < PB; ++i) {
+        const float w = __shfl_sync(0xffffffffu, pw_l, sp0 + i);
+        Lsum = fmaf(__shfl_sync(0xffffffffu, pl_l, sp0 + i), w, Lsum);
+#pragma unroll
+        for (int j = 0; j < DP; ++j) acc[j] = fmaf(po[i][j], w, acc[j]);
+      }
     }
     for (int sp = 32; sp < a.nsp; ++sp) {
       const int64_t r = (int64_t)sp * rows + bh;
