@@ -137,7 +137,7 @@ def launches(monkeypatch):
     monkeypatch.setattr(K, "_need_cuda", lambda *t: torch.device("cpu"))
     monkeypatch.setattr(K, "_stream", lambda dev: 0)
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
-    monkeypatch.setattr(K, "_recorded_event", lambda: None, raising=False)
+    monkeypatch.setattr(K, "_recorded_event", lambda dev, st: None, raising=False)
     monkeypatch.setattr(K, "relayout_tiled", lambda w, s, shape: torch.zeros(128, dtype=torch.uint8))
     monkeypatch.setattr(K, "_workspaces", {})
     monkeypatch.setattr(K, "_relayout_cache", {})
@@ -196,7 +196,7 @@ def test_a_matmul_on_another_stream_waits_for_the_copy(launches, monkeypatch):
             log.append((stream[0], "holds"))
 
     monkeypatch.setattr(K, "_stream", lambda dev: stream[0])
-    monkeypatch.setattr(K, "_recorded_event", lambda: "copied")
+    monkeypatch.setattr(K, "_recorded_event", lambda dev, st: "copied")
     monkeypatch.setattr(K, "relayout_tiled", lambda *args: torch.zeros(128, dtype=torch.uint8).as_subclass(Copy))
     monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: Stream())
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing[0])

@@ -684,13 +684,15 @@ def test_matmul_on_a_second_stream_reads_a_finished_copy(K, M):
     q, s = K.quantize_q40((torch.randn((Kd, N), generator=g, device="cuda") * 0.05).half())
     want = K.matmul_q40(a, q, s, (Kd, N))
     one, two = torch.cuda.Stream(), torch.cuda.Stream()
-    w, sc = q.clone(), s.clone()
+    w, sc, w2, sc2 = q.clone(), s.clone(), q.clone(), s.clone()
     torch.cuda.synchronize()
     with torch.cuda.stream(one):
         torch.cuda._sleep(20_000_000)           # about 10 ms
         first = K.matmul_q40(a, w, sc, (Kd, N))
+        torch.cuda._sleep(20_000_000)
+        K.matmul_q40(a, w2, sc2, (Kd, N))       # the stream's event moves on
     with torch.cuda.stream(two):
-        second = [K.matmul_q40(a, w, sc, (Kd, N)) for _ in range(3)]
+        second = [K.matmul_q40(a, x, y, (Kd, N)) for x, y in ((w, sc), (w, sc), (w2, sc2))]
     torch.cuda.synchronize()
     assert all(torch.equal(x, want) for x in (first, *second))
 
