@@ -1,11 +1,12 @@
 // Decode attention for one query token per branch over that branch's own keys: a
-// contiguous [B,Hkv,L,D] cache or a paged pool.  One CTA per (branch, query head).
+// contiguous [B,Hkv,L,D] cache, a paged pool or the packed Q4_0 cache.  Two, four or eight warps per row
+// (branch, query head), one or two rows per CTA: see launch_branch_mode.
 //
 // Eight lanes share a key: lane i owns dims 8i..8i+7 and 64+8i..64+8i+7 of the head (two 16-byte loads of K, two of
 // V, each of which covers 128 contiguous bytes over the lanes; in the Q4_0 cache the same dims are the two
 // nibbles of 8 bytes), the partial dot products are summed with three shuffles, and every group of
 // eight lanes keeps its own online-softmax state (running max, sum, 16 output dims) in
-// fp32.  The 16 groups of a CTA are merged through shared memory at the end; the same
+// fp32.  A row's groups (four per warp) are merged through shared memory at the end; the same
 // merge can fold in partial results of a shared-prefix pass (see attn_prefix.cu), which is
 // how the shared-prefix entry point finishes.
 //

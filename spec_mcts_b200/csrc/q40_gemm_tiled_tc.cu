@@ -2,9 +2,10 @@
 // TILED copy of the weights (the format of q40_gemv_tiled.cu: [span of 256 columns][16 k rows] steps of
 // 2176 contiguous bytes), so that the decode step's wide path and its narrow path share one weight copy.
 //
-// Swap-AB as in q40_gemm_tc.cu: the 256 output features of a span are the M dimension of two
-// tcgen05.mma accumulators (128 features each, in tensor memory), the batch rows the N dimension
-// (padded to a multiple of 16, up to 128 per launch; wider batches go in row chunks).  What differs is how
+// Swap-AB as in q40_gemm_tc.cu: the output features are the M dimension of the tcgen05.mma accumulators (128 features
+// each, in tensor memory), the batch rows the N dimension (padded to a multiple of 16).  Up to 128 rows a CTA takes
+// the 256 features of a span, two accumulators: gemm_tiled_tc_kernel, described here; above, 128 features and up to
+// 256 rows: gemm_tiled_wide_kernel, described there.  What differs from q40_gemm_tc.cu is how
 // the operands arrive:
 //   * one elected thread streams the weights: a 64-row k block of a span is 4 steps = 8704 contiguous
 //     bytes = ONE cp.async.bulk into a ring stage, and the matching 64-wide slice of the activations is
@@ -20,14 +21,15 @@
 //     dequantised weights never touch shared memory (through shared memory they cost 64 KB of traffic per
 //     k block, more than the operands themselves);
 //   * four warps issue the tcgen05.mma (A from tensor memory, B from the stage): a k block is 2 x 4 MMAs of
-//     128 x Mpad x 16, small enough that the issuing thread's fixed latencies (mbarrier test, fences, commit:
-//     ~800 cycles per k block measured under `lane == 0`, before the elected thread) matter, so each accumulator has two issuing warps that alternate k
+//     128 x Mpad x 16, small enough that an issuing thread's fixed latencies (mbarrier test, fences, commit) matter,
+//     so each accumulator has two issuing warps that alternate k
 //     blocks and hand over in order through shared memory (every accumulator sees its MMAs in k order:
 //     results do not depend on which warp was faster).  A commit per warp arrives on the block's "MMAs done"
 //     mbarrier, which frees both the stage and the A buffer.
 // The k range is split over a thread-block cluster; partial accumulators meet through distributed
 // shared memory (no global scratch).  Every mbarrier wait is bounded: on expiry the kernel records an
-// error code, skips the remaining work, frees its tensor memory and returns.
+// error code, skips the remaining work, waits (bounded too) for its own copies and MMAs, frees its tensor memory and
+// returns.
 //
 // Replaces matmul_q40_kernel (triton_kernels.py:357-469) for M > 16 when the caller holds tiled weights.
 #include <cooperative_groups.h>
@@ -71,7 +73,8 @@ struct Params {
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // One lane of a converged warp, chosen so that the compiler knows the branch to be taken by a single thread: operands
-// of copies and MMAs issued under `lane == 0` go through a loop that moves them to uniform registers.
+// of copies and MMAs issued under `lane == 0` go through a loop that moves them to uniform registers, which bound a
+// k block (100 rows x 4096 x 11008: 19.4 -> 16.9 us; 512 rows: 94.9 -> 58.5 us).
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
@@ -308,9 +311,6 @@ gemm_tiled_tc_kernel(const Params p, const __grid_constant__ CUtensorMap amap) {
     __syncwarp();
   } else if (warp < DQ_WARP0 || warp >= DQ_WARP0 + DQ_WARPS) {
     // ================= the four MMA warps: one elected thread each =================
-    // Under `lane == 0` an issuing warp spent ~800 cycles per k block on fixed latencies (mbarrier test, fences, commit)
-    // and 60-120 per tcgen05.mma, whatever the tile size; the elected thread takes less (100 rows x 4096 x 11008: 19.4 ->
-    // 16.9 us), and four of them still overlap their waits.
     // Warp (hh, set) issues the four k steps of feature half hh for the k blocks of its set (even or odd).
     // fp32 accumulation is not associative, and the result must not depend on which warp was faster, so every
     // accumulator has to see its MMAs in a fixed order.  Up to 64 padded batch rows tensor memory has room for
@@ -466,15 +466,15 @@ gemm_tiled_tc_kernel(const Params p, const __grid_constant__ CUtensorMap amap) {
 // More than 128 rows (prompt pass, wide batches): 128 features x up to 256 batch rows per CTA.
 //
 // Same operands as above, other proportions.  The rows, which are the MMA's N, go up to 256, so that a k block is four
-// large MMAs, and one accumulator of 128
-// features takes half of tensor memory; the other half holds NA = 8 A buffers.  The activations of a k block
+// large MMAs, and one accumulator of 128 features takes half of tensor memory; the other half holds NA = 8 A buffers.  The activations of a k block
 // (32 KB at 256 rows) are read once per 128 features.  Sixteen dequantiser warps are four sets of four (one
 // warp per tensor-memory quadrant) that take the k blocks in turn; one thread issues all MMAs, in k order, so a
 // result depends on nothing but the operands and the k split.  Rows are cut into equal chunks of at most 256
 // inside ONE launch (grid z); a tile that is not split along k goes from tensor memory to the output
 // directly, otherwise the ranks of a cluster add their fp32 tiles in rank order.
-// 512 x 4096 x 11008: 58.5 us = 0.79 PFLOP/s, about half the tensor rate (122.9 us on the checkpoint layout; 94.9 us with
-// the copies and MMAs under `lane == 0`).  36 KB a k block come through L2, which is what bounds it next.
+// 512 x 4096 x 11008: 58.5 us = 0.79 PFLOP/s, about half the tensor rate (122.9 us on the checkpoint layout).  Bound by
+// waves and a CTA's fixed cost, not by L2 (16 % of its rate): 172 tiles of 64 k blocks on 148 SMs are two waves, the second
+// for 24 of them, and an SM is active 53 % of the launch.
 // ---------------------------------------------------------------------------------------------------------
 namespace wide {
 
