@@ -294,14 +294,13 @@ def _tiled_copy_of(b_w, b_s, K, N, dev, st):
         rw, rs, ver, shape, ptrs, copy, event, streams = ent
         if (rw() is b_w and rs() is b_s and ver == _versions(b_w, b_s) and shape == (K, N)
                 and ptrs == (b_w.data_ptr(), b_s.data_ptr())):
-            if st in streams:
+            # a capture cannot wait for an event from outside of it, and begins on a device that has been waited for
+            if st in streams or torch.cuda.is_current_stream_capturing():
                 return copy, False
-            # a capture cannot wait for an event from outside of it (and begins on a device that has been waited for)
-            if not torch.cuda.is_current_stream_capturing():
-                here = torch.cuda.current_stream(dev)
-                here.wait_event(event)
-                copy.record_stream(here)
-                streams.add(st)
+            here = torch.cuda.current_stream(dev)
+            here.wait_event(event)
+            copy.record_stream(here)
+            streams.add(st)
             return copy, True
     # a copy made inside a capture would hold nothing until the graph runs: the checkpoint layout is read there
     if torch.cuda.is_current_stream_capturing():
