@@ -108,7 +108,8 @@ int q40_gemm_kn_tc_multi(int nmat, const void* a, int64_t lda, const void* const
  * the weight stream of a CTA is one contiguous run fetched by 1-D bulk copies, the activations arrive by
  * tiled TMA copies (a tensor map over `a` is encoded per call), both into a 3..8 stage ring; A operand
  * value fp16(code * scale) as in the reference (triton_kernels.py:444-445), written to tensor memory.  Batches
- * above 128 rows run in equal row chunks of at most 256 inside one launch.  Results are bit-identical from run to run.  Same
+ * above 128 rows run in equal row chunks of at most 256, up to 65535 of them in one launch.  Results are bit-identical from
+ * run to run.  Same
  * `err` and `use_pdl` rules as q40_gemm_kn_tc_multi; Q40_E_UNSUPPORTED when the driver offers no tensor-map
  * encoder. */
 int q40_gemm_tiled_tc_multi(int nmat, const void* a, int64_t lda, const void* const* bw_tiled, void* const* c,
@@ -121,7 +122,6 @@ int q40_gemm_tiled_tc_multi(int nmat, const void* a, int64_t lda, const void* co
  * Replaces: matmul_q40 (triton_kernels.py:471-500). */
 int q40_matmul_tiled(const void* bw_tiled, void* c, int64_t ldc, const void* a, int64_t lda, int M, int N, int K,
                      int max_cluster, int* err, int use_pdl, void* stream);
-
 
 /* q40_gemm_kn without a caller-provided workspace, for hosts that cannot allocate device
  * memory themselves (all HBM already handed to their own planner, or a plug-in that only
