@@ -105,20 +105,28 @@ int q40_gemm_kn_tc_multi(int nmat, const void* a, int64_t lda, const void* const
 
 /* The same operation on TILED copies of the weights (q40_relayout_tiled; N_i % 256 == 0, K % 64 == 0),
  * so that a caller that already holds tiled copies for the narrow decode path needs no second format:
- * the weight stream of a CTA is one contiguous run fetched by 1-D bulk copies, the activations arrive by
- * tiled TMA copies (a tensor map over `a` is encoded per call), both into a 3..8 stage ring; A operand
- * value fp16(code * scale) as in the reference (triton_kernels.py:444-445), written to tensor memory.  Batches
- * above 128 rows run in equal row chunks of at most 256, up to 65535 of them in one launch.  Results are bit-identical from
- * run to run.  Same
- * `err` and `use_pdl` rules as q40_gemm_kn_tc_multi; Q40_E_UNSUPPORTED when the driver offers no tensor-map
- * encoder. */
+ * weights and activations arrive by tensor copies (tensor maps are encoded per call) into a ring of shared-memory
+ * stages; A operand value fp16(code * scale) as in the reference (triton_kernels.py:444-445), written to tensor memory.
+ * Any number of rows; results are bit-identical from run to run.  Same `err` and `use_pdl` rules as
+ * q40_gemm_kn_tc_multi; Q40_E_UNSUPPORTED when the driver offers no tensor-map encoder. */
 int q40_gemm_tiled_tc_multi(int nmat, const void* a, int64_t lda, const void* const* bw_tiled, void* const* c,
                             const int64_t* ldc, const int* n_cols, int M, int K, int* err, int use_pdl,
                             void* stream);
 
-/* C[M, N] = A @ deq(B) for one TILED copy: q40_gemv_tiled (mode 0) up to 16 rows, q40_gemm_tiled_tc_multi above,
- * under their rules, for hosts that make one call per projection.  `max_cluster` is used up to 16 rows, `err` (which
- * may be NULL there) above.
+/* q40_gemm_tiled_tc_multi with scratch and, if silu_mul != 0, an epilogue: c[0] = silu(A @ deq(B_0)) * (A @ deq(B_1)) for
+ * two matrices of one width, every step rounded to fp16 like the separate launches (hf_model_q40_kv_shared.py:434); c[1]
+ * and ldc[1] have to be valid but are not written.  Up to 128 rows the k range of a tile may then be shared between
+ * pairs of SMs, whose sums meet in the scratch: q40_gemm_tiled_tc_ws_bytes(M) bytes (0 above 128 rows: no scratch
+ * needed), 16-byte aligned, zeroed before its first use; the kernels leave it ready for the next call.  Calls that
+ * overlap on the GPU need scratch of their own.  After an expired wait (`err`) it has to be zeroed again. */
+size_t q40_gemm_tiled_tc_ws_bytes(int M);
+int q40_gemm_tiled_tc_ws(int nmat, const void* a, int64_t lda, const void* const* bw_tiled, void* const* c, const int64_t* ldc,
+                         const int* n_cols, int M, int K, int silu_mul, void* workspace, size_t workspace_bytes, int* err,
+                         int use_pdl, void* stream);
+
+/* C[M, N] = A @ deq(B) for one TILED copy, for hosts that make one call per projection: q40_gemv_tiled (mode 0) up to 8
+ * rows, q40_gemm_tiled_tc_multi above, under their rules.  `max_cluster` is used up to 16 rows, where
+ * q40_gemv_tiled also takes 9..16 rows that the other does not (K % 64 != 0, `err` NULL, an odd ldc, no encoder).
  * Replaces: matmul_q40 (triton_kernels.py:471-500). */
 int q40_matmul_tiled(const void* bw_tiled, void* c, int64_t ldc, const void* a, int64_t lda, int M, int N, int K,
                      int max_cluster, int* err, int use_pdl, void* stream);

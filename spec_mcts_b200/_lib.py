@@ -58,6 +58,9 @@ SIGNATURES = {
     "q40_tp_status": (c_int, [c_void_p, c_void_p, c_int, c_void_p]),
     "q40_gemm_tiled_tc_multi": (c_int, [c_int, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p,
                                         c_int, c_int, c_void_p, c_int, c_void_p]),
+    "q40_gemm_tiled_tc_ws_bytes": (c_size_t, [c_int]),
+    "q40_gemm_tiled_tc_ws": (c_int, [c_int, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                                     c_void_p, c_size_t, c_void_p, c_int, c_void_p]),
     "q40_gemm_kn_static": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int,
                                    c_int, c_int, c_void_p]),
     "q40_gemm_kn_static_max_workspace": (c_size_t, []),

@@ -1,0 +1,899 @@
+// Q4_0 dequant-matmul on the tiled weight copies (format: q40_gemv_tiled.cu) for two CTAs that work as a pair: the
+// MMAs are tcgen05 cta_group::2, 256 features of a span x up to 256 batch rows, each CTA of the pair holding 128
+// features (its half of the A operand and of the accumulators, both in its tensor memory) and HALF of the batch rows
+// of a k block in its shared memory.
+//
+// Why pairs: a CTA that does 128 features x 256 rows by itself loads 32 KB of activations and 4.3 KB of weights per
+// 512 tensor cycles of a k block, 72 bytes a cycle, more than an SM gets from L2 (64 at most); a pair loads 16 KB of
+// activations per CTA instead.  The batch rows are the MMA's N, so that a k block is four MMAs whatever the rows.
+//
+// Persistent: a pair takes a contiguous share of all (tile, k block) units and runs through it without a break, weights
+// and activations of the next tile on their way while the last one is finished by warps of its own, out of the second
+// of two accumulators (one, if they do not fit tensor memory beside the A buffers).  Roles of a CTA's 24 warps:
+//   warp 0        weights: two tensor copies per k block into a ring stage
+//   warp 1        issues the MMAs (the even CTA's, for both)
+//   warp 2        activations: a TMA copy per 64 k (half of the rows, 128-byte swizzle)
+//   warps 4..19   dequantise: four sets of four (one warp per 32 tensor-memory lanes) that take the k blocks in turn
+//                 and write fp16(code * scale), the reference's operand value (triton_kernels.py:444-445), to
+//                 tensor memory (see q40_gemm_tiled_tc.cu)
+//   warps 20..23  accumulators -> output
+// The pair's last tile is finished by the dequantiser warps as well.
+//
+// A tile whose k range is cut between pairs: all but the last leave their fp32 sums in a scratch slot (first thing,
+// each has one at most) and raise flags; the pair with the last k blocks does them last and adds the slots in order.  A
+// pair waits for lower-numbered pairs only, and those publish before they wait, so that no order of scheduling can make
+// them wait for each other.  Results depend on nothing but operands and grid.
+//
+// What bounds it, per 128 k of a tile (cycles): up to 96 rows the dequantisers' instructions (460; two thousand issue slots of
+// four schedulers), at 112 and 128 rows the MMAs (500 and 545 with their gaps, 450 and 512 without), above, with all SMs
+// busy, activations from L2 (28 to 33 bytes a cycle and SM).  A launch adds 4 to 5.4 us: set-up and the first stages'
+// latency 2, the last accumulator's way out 1 to 2, draining.  Microseconds, here and by the kernels before (one CTA per
+// tile, k split over clusters; up to 16 rows q40_gemv_tiled): 10 rows x 11008 x 4096 13.0 and 16.8, two x 4096 x 11008 16.9 and
+// 22.9; 100 rows x 11008 x 4096 15.7 and 20.8, two x 4096 x 11008 21.8 and 34.1; 512 rows x 4096 x 11008 39.5 and 61.4,
+// three x 4096 x 4096 45.5 and 82.5, x 11008 x 4096 37.2 and 48.6.
+//
+// Every wait is bounded: on expiry an error word is set, the remaining work skipped, copies and MMAs in flight
+// waited for, tensor memory freed.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+
+#include "q40_tc_common.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace q40 {
+namespace ttc {
+namespace pair {
+
+constexpr int FEATS = 128;                      // features of a CTA
+constexpr int MAX_ROWS = 256;
+constexpr int DSETS = 4;                        // dequantiser sets, of one warp per tensor-memory quadrant
+constexpr int DQ_WARP0 = 4, EPI_WARP0 = DQ_WARP0 + 4 * DSETS;
+constexpr int THREADS = (EPI_WARP0 + 4) * 32;
+constexpr int BLK = 2;                          // 64-row k steps of a block: 8 MMAs per wait and commit (with 4 the issuing
+                                                // thread's own latencies, 390 cycles, bound the loop)
+constexpr int RAW_W = 8 * 1024, RAW_S = 8 * 64; // of a block: eight half steps (two 64-column groups each) and their scales
+constexpr int RAW_BYTES = RAW_W + RAW_S;
+constexpr int RAW_PAD = 9216;                   // next multiple of 1024 (the B tiles want that alignment)
+constexpr int S_MAX = 16;                       // ring stages
+constexpr int A_COLS = 32 * BLK;                // tensor-memory columns of an A buffer
+constexpr int NA_MAX = 4;
+constexpr int TMEM_COLS = 512;
+constexpr int CUT = 2;                          // a k range is cut at multiples of so many blocks
+constexpr int GROUPS = 1 + DSETS;               // of four warps, one per tensor-memory quadrant, that finish a pair's last tile
+constexpr int BAR_BYTES = 16 * S_MAX + 8 * NA_MAX + 64;
+constexpr int OUT_LD = FEATS + 8;              // halves between rows that wait in shared memory
+constexpr int MAX_PAIRS = 128;
+constexpr int FLAG_BYTES = MAX_PAIRS * 64;      // at the start of the scratch, per pair: [half][quadrant] arrivals, then departures
+
+// Tensor maps: the activations, and per matrix the weights (box 1024 bytes x 8 steps) and scales (64 bytes x 8 steps) of a
+// tiled copy read as rows of one step
+struct Maps { CUtensorMap act, w[3], s[3]; };
+
+struct Params {
+  __half* c[3];
+  int64_t ldc[3];
+  int spans[3], nprob;
+  int M, K, npad;          // npad: rows of a tile, a multiple of 16
+  int chunks;              // row chunks; tile = span * chunks + chunk
+  int ntiles, nblk;        // blocks of a tile: up to BLK 64-row k steps of one range
+  int k64, range, rblk;    // k steps of a tile and of a range, and blocks of a range.  A range is summed in tensor memory;
+                           // the sums of a tile's ranges are added in order
+  int cut;                 // tiles may be shared between pairs along k (scratch given)
+  int share, rest;         // cut: a pair has share units of CUT blocks, the first `rest` pairs one more
+  int bps;                 // SPLIT: blocks of a rank
+  int stages, nacc;        // ring stages, accumulators
+  int run_off, x_off, out_off, bar_off;    // byte offsets in the aligned shared memory
+  int silu;                // c[0] = silu(A @ deq(B_0)) * (A @ deq(B_1)): a tile is half a span of both
+  int vec;                 // outputs take 16-byte stores
+  float* part;             // scratch slots: [pair][half][npad][128]
+  int* flags;              // per pair: see FLAG_BYTES
+  int* err;
+};
+
+// A bounded wait as one instruction to the compiler, and without a way out of the loop around it: what that loop computes
+// stays uniform, so that MMA operands are kept in uniform registers (an MMA issues in 15 cycles instead of 53).  `limit` is
+// what remains of the polls; it is 0 once a wait has run out, and later ones then ask once.
+__device__ __forceinline__ void wait_limited(uint32_t bar, uint32_t parity, uint32_t& limit) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\tmov.u32 n, %3;\n\t"
+      "TRY:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %4;\n\t@p bra DONE;\n\t"
+      "setp.eq.u32 q, n, 0;\n\t@q bra DONE;\n\tsub.u32 n, n, 1;\n\tbra TRY;\n\t"
+      "DONE:\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit), "r"(POLL_NS) : "memory");
+  limit = ok ? limit : 0;
+}
+// A position in a ring of n slots and the parity of its turn
+struct Slot {
+  int i = 0;
+  uint32_t turn = 0;
+  __device__ __forceinline__ void next(int n) { if (++i == n) { i = 0; turn ^= 1; } }
+  __device__ __forceinline__ void next4(int n) { i += 4; if (i >= n) { i -= n; turn ^= 1; } }     // n >= 4
+};
+__device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+// An arrival in the even CTA's shared memory.  It publishes no ordinary stores (tensor-memory accesses are ordered by the
+// tcgen05 waits and fences, copies by their own barrier), so it goes without a cluster-wide release, which costs a
+// dequantiser warp 1100 cycles
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void commit2(uint32_t bar, uint16_t mask) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(bar), "h"(mask) : "memory");
+}
+__device__ __forceinline__ void mma2_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accum) : "memory");
+}
+
+// Waits for tensor-memory loads; naming the registers keeps their uses behind it
+__device__ __forceinline__ void wait_ld16(uint32_t (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                 "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]) :: "memory");
+}
+
+// `n` finished rows of 128 features from shared memory to the output, by the 128 threads t of a group
+__device__ __forceinline__ void store_rows(const __half* o, __half* c, int64_t ldc, int n, int t, int vec) {
+  if (vec) {
+    for (int row = t >> 4; row < n; row += 8)
+      *reinterpret_cast<uint4*>(c + row * ldc + (t & 15) * 8) = *reinterpret_cast<const uint4*>(o + row * OUT_LD + (t & 15) * 8);
+  } else {
+    for (int row = t >> 6; row < n; row += 2)
+      *reinterpret_cast<uint32_t*>(c + row * ldc + (t & 63) * 2) = *reinterpret_cast<const uint32_t*>(o + row * OUT_LD + (t & 63) * 2);
+  }
+}
+
+// First block of pair q
+__device__ __forceinline__ int first_block(const Params& p, int q, int npairs) {
+  if (q >= npairs) return p.ntiles * p.nblk;
+  if (!p.cut) return (int)((int64_t)p.ntiles * q / npairs) * p.nblk;
+  return CUT * (q * p.share + min(q, p.rest));
+}
+
+// The k steps of block b of a tile, and of those behind it
+struct KCursor {
+  int k, end;                                  // first k step; end of the range it belongs to
+  __device__ __forceinline__ KCursor(const Params& p, int b) {
+    const int r = b / p.rblk;
+    k = r * p.range + (b - r * p.rblk) * BLK;
+    end = min(p.k64, (r + 1) * p.range);
+  }
+  __device__ __forceinline__ bool next(const Params& p) {      // true: the range has ended
+    k = min(k + BLK, end);
+    if (k < end) return false;
+    end = min(p.k64, end + p.range);
+    return true;
+  }
+};
+
+// The pieces of tiles that a pair works on, in the order it takes them: the one it publishes first (the last tile, if its
+// k range goes on beyond the pair's share), the one it may have to wait for last (the first tile)
+struct Work {
+  int u0, u1, nblk, t0, t1, np;
+  bool pub;
+  __device__ __forceinline__ Work(int a, int b, int n) : u0(a), u1(b), nblk(n) {
+    t0 = u0 / n;
+    t1 = u1 > u0 ? (u1 - 1) / n : t0;
+    np = u1 > u0 ? t1 - t0 + 1 : 0;
+    pub = u1 > u0 && u1 < (t1 + 1) * n;
+  }
+  __device__ __forceinline__ void piece(int k, int& tile, int& b0, int& b1) const {
+    tile = k == np - 1 ? t0 : (pub ? (k == 0 ? t1 : t0 + k) : t0 + 1 + k);
+    b0 = tile == t0 ? u0 - tile * nblk : 0;
+    b1 = tile == t1 ? u1 - tile * nblk : nblk;
+  }
+};
+
+// SPLIT: the k range of one tile is spread over the pairs of a cluster (grid y), whose fp32 sums meet through
+// distributed shared memory.  Otherwise a cluster is a pair.
+// CUT: tiles may be shared between pairs along k; SILU: see Params (compiled for each, to keep the registers of all roles
+// below the 80 that 24 warps leave)
+template <bool SPLIT, int NA, bool CUT_K, bool SILU>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
+  extern __shared__ unsigned char smem_raw[];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int half = blockIdx.x & 1, me = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+  const uint32_t lead = SPLIT ? 2 * blockIdx.y : 0;          // rank of the pair's even CTA in the cluster
+  const int S = p.stages;                                    // at least as many as A buffers, and four
+  const uint32_t b_bytes = (uint32_t)p.npad * 64u;           // B tile of a k step: npad / 2 rows x 64 k x 2 B
+  const uint32_t stage_bytes = RAW_PAD + BLK * b_bytes;
+
+  const uint32_t raw0 = smem_u32(smem_raw);
+  const uint32_t ring = (raw0 + 1023u) & ~1023u;
+  unsigned char* gbase = smem_raw + (ring - raw0);
+  // Block i has stage and barriers i % S and A buffer i % NA.  full: its weights and activations have landed in this
+  // CTA; mdone: its MMAs are complete, in both CTAs; accfull[b]: an accumulator is complete.  In the even CTA, for both:
+  // afull: the A operand is written (and the activations have landed); accfree[b]: an accumulator has been read.
+  const uint32_t bar_full = ring + (uint32_t)p.bar_off, bar_mdone = bar_full + 8 * S_MAX, bar_afull = bar_mdone + 8 * S_MAX, bar_accfull = bar_afull + 8 * NA_MAX,
+                 bar_accfree = bar_accfull + 16, bar_x = bar_accfree + 16, bar_xfree = bar_x + 8, bar_done = bar_xfree + 8, bar_last = bar_done + 8;
+  unsigned char* tail = gbase + p.bar_off + BAR_BYTES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail);
+  volatile int* s_failed = reinterpret_cast<volatile int*>(tail + 8);
+  volatile int* s_acc = reinterpret_cast<volatile int*>(tail + 24);        // of a pair's last tile: accumulator, SiLU tiles before
+  volatile int* s_tiles = reinterpret_cast<volatile int*>(tail + 28);
+  volatile int* s_copied = reinterpret_cast<volatile int*>(tail + 16);     // [2] blocks whose copies were requested
+  float* run = reinterpret_cast<float*>(gbase + p.run_off);                // [npad][128] sums of earlier ranges
+  __half* out_s = reinterpret_cast<__half*>(gbase + p.out_off);            // [2][16][OUT_LD] finished rows on their way out
+  // SiLU: [npad / 16][128] halves of 16 rows that this CTA finishes, its own and the other CTA's
+  uint4* own = reinterpret_cast<uint4*>(gbase + p.x_off);
+  uint4* other = own + p.npad / 16 * FEATS;
+
+  const int sb0 = SPLIT ? blockIdx.y * p.bps : 0, sb1 = SPLIT ? min(p.nblk, sb0 + p.bps) : 0;
+  const Work wk(SPLIT ? me * p.nblk + sb0 : first_block(p, me, npairs),
+                SPLIT ? me * p.nblk + sb1 : first_block(p, me + 1, npairs), p.nblk);
+  const int total = wk.u1 - wk.u0;                    // blocks of this pair
+  // matrix, span, 128-feature half of this CTA and first row of a tile
+  auto decode = [&](int tile, int& pi, int& span, int& fh, int& m0) {
+    span = tile / p.chunks;
+    m0 = (tile - span * p.chunks) * p.npad;
+    if (SILU) {
+      pi = half;
+      fh = span & 1;
+      span >>= 1;
+      return;
+    }
+    pi = 0;
+    fh = half;
+    while (pi < p.nprob - 1 && span >= p.spans[pi]) { span -= p.spans[pi]; ++pi; }
+  };
+  bool failed = false;
+  uint32_t limit = SPIN_LIMIT;                               // see wait_limited
+
+  // ---- weights: they do not depend on the previous launch, so the first stages are requested before anything else ----
+  int wi = 0;                                                // blocks requested
+  Slot wslot;
+  auto stream_weights = [&](int limit) {
+    int i = 0;
+    for (int k = 0; k < wk.np && wi < limit && !failed; ++k) {
+      int tile, b0, b1, pi, span, fh, m0;
+      wk.piece(k, tile, b0, b1);
+      if (i + b1 - b0 <= wi) { i += b1 - b0; continue; }
+      decode(tile, pi, span, fh, m0);
+      KCursor kc(p, b0 + (wi - i));
+      for (int b = b0 + (wi - i); b < b1 && wi < limit; ++b, kc.next(p)) {
+        const int s = wslot.i;
+        if (wi >= S && !mbar_wait(bar_mdone + 8 * s, wslot.turn ^ 1)) { failed = true; break; }
+        const uint32_t dst = ring + s * stage_bytes;
+        const int step = (span * p.k64 + kc.k) * 4;
+        mbar_expect_tx(bar_full + 8 * s, RAW_BYTES);
+        tma_2d(dst, &maps.w[pi], fh * 256, step, bar_full + 8 * s);               // x in words of four bytes
+        tma_2d(dst + RAW_W, &maps.s[pi], 512 + fh * 16, step, bar_full + 8 * s);
+        wslot.next(S);
+        ++wi;
+      }
+      i += b1 - b0;
+    }
+  };
+  if (warp == 0) {
+    if (lane == 0) {
+      *s_failed = 0;
+      for (int s = 0; s < S; ++s) {
+        mbar_init(bar_full + 8 * s, 2);
+        mbar_init(bar_mdone + 8 * s, 1);
+      }
+      for (int s = 0; s < NA; ++s) mbar_init(bar_afull + 8 * s, 8);
+      for (int s = 0; s < 2; ++s) { mbar_init(bar_accfull + 8 * s, 1); mbar_init(bar_accfree + 8 * s, 8); }
+      mbar_init(bar_x, 1);
+      mbar_init(bar_xfree, 4);
+      mbar_init(bar_done, 1);
+      mbar_init(bar_last, 4);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(TMEM_COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  if (warp == 0) {
+    if (elect_one()) stream_weights(min(S, total));
+    __syncwarp();
+  }
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");     // both CTAs' barriers and tensor memory are there
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  constexpr uint32_t A_COL0 = TMEM_COLS - A_COLS * NA;
+  asm volatile("griddepcontrol.launch_dependents;");
+
+  if (warp == 0) {
+    if (elect_one()) {
+      wi = min(S, total);
+      wslot.i = wi % S;
+      wslot.turn = wi / S;
+      stream_weights(total);
+      s_copied[0] = wi;
+    }
+    __syncwarp();
+  } else if (warp == 2) {
+    if (elect_one()) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      int i = 0;
+      Slot sl;
+      for (int k = 0; k < wk.np && !failed; ++k) {
+        int tile, b0, b1, pi, span, fh, m0;
+        wk.piece(k, tile, b0, b1);
+        decode(tile, pi, span, fh, m0);
+        KCursor kc(p, b0);
+        for (int b = b0; b < b1; ++b, kc.next(p)) {
+          const int s = sl.i;
+          if (i >= S && !mbar_wait(bar_mdone + 8 * s, sl.turn ^ 1)) { failed = true; break; }
+          // the second k step of a range's last block may be the next range's or beyond K (zeros): not multiplied
+          mbar_expect_tx(bar_full + 8 * s, BLK * b_bytes);
+#pragma unroll
+          for (int h = 0; h < BLK; ++h)
+            tma_2d(ring + s * stage_bytes + RAW_PAD + h * b_bytes, &maps.act, (kc.k + h) * BK, m0 + half * (p.npad / 2),
+                   bar_full + 8 * s);
+          sl.next(S);
+          ++i;
+        }
+      }
+      s_copied[1] = i;
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (half == 0) {
+      // instruction descriptor: D fp32, A and B fp16 and K-major, N = npad, M = 256 over the two CTAs
+      const uint32_t idesc = (1u << 4) | ((uint32_t)(p.npad >> 3) << 17) | ((uint32_t)(2 * FEATS >> 4) << 24);
+      const uint16_t both = (uint16_t)(3u << lead);
+      const uint64_t bdesc = kmajor_desc(ring + RAW_PAD);
+      if (elect_one()) {
+        Slot sl, sa, sc;                                     // stage, A buffer, accumulator
+        int g = 0;
+        for (int k = 0; k < wk.np; ++k) {
+          int tile, b, b1;
+          wk.piece(k, tile, b, b1);
+          KCursor kc(p, b);
+          while (b < b1) {                                   // a range, or the pair's share of it
+            if (g >= p.nacc) wait_limited(bar_accfree + 8 * sc.i, sc.turn ^ 1, limit);
+            const uint32_t acc = tmem + sc.i * p.npad;
+            uint32_t accum = 0;
+            for (bool last = false; b < b1 && !last; ++b) {
+              wait_limited(bar_afull + 8 * sa.i, sa.turn, limit);
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              const uint64_t bd0 = bdesc + (uint64_t)((sl.i * stage_bytes) >> 4), bd1 = bd0 + (uint64_t)(b_bytes >> 4);
+              const uint32_t ta = tmem + A_COL0 + sa.i * A_COLS;
+#pragma unroll
+              for (int ks = 0; ks < BK / 16; ++ks) mma2_ts(acc, ta + ks * 8, bd0 + (uint64_t)(ks * 2), idesc, ks ? 1u : accum);
+              if (kc.end - kc.k >= BLK) {
+#pragma unroll
+                for (int ks = 0; ks < BK / 16; ++ks) mma2_ts(acc, ta + 32 + ks * 8, bd1 + (uint64_t)(ks * 2), idesc, 1);
+              }
+              commit2(bar_mdone + 8 * sl.i, both);
+              accum = 1;
+              sl.next(S);
+              sa.next(NA);
+              last = kc.next(p);
+            }
+            commit2(bar_accfull + 8 * sc.i, both);
+            sc.next(p.nacc);
+            ++g;
+          }
+        }
+        failed = limit == 0;
+        commit2(bar_done, both);
+      }
+      __syncwarp();
+    }
+  } else if (warp >= DQ_WARP0 && warp < EPI_WARP0) {
+    // warp = (set, quadrant): 32 feature rows = two 16-row tiles of one 64-column group, all k of a block.  Lane (g, t) holds, per
+    // 16-row tile and 16 k, rows g and g + 8 at k = 4t .. 4t + 3
+    const int quad = warp & 3, dset = (warp - DQ_WARP0) >> 2;
+    const int q = quad >> 1, t = lane & 3;
+    const unsigned char* lane_w = gbase + (q * 32 + lane) * 16 + (quad & 1) * 8;
+    const unsigned char* lane_s = gbase + RAW_W + q * 32 + t * 8;
+    const uint32_t afull_lead = mapa(bar_afull, lead) + 8 * (dset % NA);
+    const uint32_t ta = tmem + ((uint32_t)(32 * quad) << 16) + A_COL0 + dset % NA * A_COLS;
+    Slot sl, sw;                                 // stage of this block, and of the one that used its A buffer before
+    sl.i = dset;
+    const int w0 = dset >= NA ? dset - NA : dset + DSETS - NA;
+    sw.i = w0 % S;
+    sw.turn = w0 / S;
+    for (int i = dset; i < total; i += DSETS) {
+      // The MMAs of the block that last used this A buffer are complete.  As the ring has at least NA stages, the block that
+      // last used this stage is through as well, and the stage's barrier, which tells only odd from even phases, is in one
+      // of the two phases that it can tell apart
+      if (i >= NA) {
+        wait_limited(bar_mdone + 8 * sw.i, sw.turn, limit);
+        sw.next4(S);
+      }
+      wait_limited(bar_full + 8 * sl.i, sl.turn, limit);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t so = sl.i * stage_bytes;
+#pragma unroll
+      for (int h = 0; h < BLK; ++h) {
+        uint32_t r[2][16];
+#pragma unroll
+        for (int st = 0; st < 4; ++st) dequant_step(lane_w + so + (4 * h + st) * 1024, lane_s + so + (4 * h + st) * 64, r, st);
+        st_16x256b_x4(ta + 32 * h, r[0]);
+        st_16x256b_x4(ta + 32 * h + (16u << 16), r[1]);
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(afull_lead);
+      sl.next4(S);
+    }
+    failed = limit == 0;
+  }
+  if (!SPLIT && warp >= DQ_WARP0) {
+    // ================= accumulators -> output =================
+    // Group 0 (warps 20..23) finishes every tile but the pair's last beside the main loop; the last one (the last range of it)
+    // falls to all groups, the dequantisers having come to their end: 16-row chunks group, group + GROUPS, ...
+    // No wait leaves these loops early, so that the warps of a group always meet at its (plain) barrier.
+    const int group = warp >= EPI_WARP0 ? 0 : 1 + ((warp - DQ_WARP0) >> 2);
+    const int quad = warp & 3, feat = 32 * quad + lane;
+    const uint32_t lane_base = tmem + ((uint32_t)(32 * quad) << 16);
+    // two buffers of 16 finished rows per group; those of groups 1.. over the ring, which is idle by then
+    __half* out_g = group == 0 ? out_s : reinterpret_cast<__half*>(gbase) + (group - 1) * 2 * 16 * OUT_LD;
+    const int nchunk = p.npad / 16;
+    Slot sc;                                                 // accumulator
+    int turn = 0, tiles = 0;                                 // output buffer; finished tiles (SiLU)
+    // outputs, scratch and flags may still be in use by the launch in front of this one
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int k = group == 0 ? 0 : max(0, wk.np - 1); k < wk.np; ++k) {
+      int tile, b0, b1, pi, span, fh, m0;
+      wk.piece(k, tile, b0, b1);
+      decode(tile, pi, span, fh, m0);
+      const bool whole = !CUT_K || b1 == p.nblk;                       // this pair has the tile's last blocks and finishes it
+      const int rows = min(p.npad, p.M - m0);
+      const int64_t ldc = p.ldc[SILU ? 0 : pi];
+      __half* c = p.c[SILU ? 0 : pi] + (int64_t)m0 * ldc + span * SPAN + fh * FEATS;
+      // the pairs with its first blocks, whose sums are added in k order
+      int q0 = me;
+      if (CUT_K && whole && b0 > 0) {
+        --q0;
+        while (q0 > 0 && first_block(p, q0, npairs) > wk.u0 - b0) --q0;
+      }
+      bool all = false;
+      for (int b = b0; b < b1;) {
+        const int e = CUT_K ? b1 : min(b1, (b / p.rblk + 1) * p.rblk);    // a range, or the pair's share of it
+        const bool add_run = b > b0;
+        b = e;
+        all = e == b1 && k == wk.np - 1;
+        if (group > 0 && !all) continue;
+        const int ch0 = all ? group : 0, step = all ? GROUPS : 1;
+        const float* first = p.part + ((int64_t)(q0 * 2 + half) * p.npad) * FEATS + feat;
+        float v[16];
+        if (CUT_K && e == b1 && q0 < me) {
+          for (int q = q0; q < me; ++q) {
+            const int* flag = p.flags + q * 16 + half * 4 + quad;
+            int arrived;
+            do {
+              asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(arrived) : "l"(flag) : "memory");
+              if (arrived < GROUPS) { __nanosleep(64); limit = limit ? limit - 1 : 0; }
+            } while (arrived < GROUPS && limit);
+          }
+          if (ch0 < nchunk) {                                // while the last MMAs run
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = __ldcg(first + (ch0 * 16 + j) * FEATS);
+          }
+        }
+        // (a barrier's parity tells a phase from its neighbours only: the other groups, which have not followed accfull and xfree,
+        // wait for the end of all MMAs and for group 0, which has)
+        if (group == 0) {
+          wait_limited(bar_accfull + 8 * sc.i, sc.turn, limit);
+          if (SILU && whole && e == b1) {
+            if (tiles > 0) wait_limited(bar_xfree, (tiles - 1) & 1, limit);
+            if (warp == EPI_WARP0 && lane == 0) mbar_expect_tx(bar_x, nchunk * FEATS * 16);
+          }
+          __syncwarp();
+          if (all && lane == 0) {
+            *s_acc = sc.i;
+            *s_tiles = tiles;
+            mbar_arrive(bar_last);
+          }
+        } else {
+          wait_limited(bar_done, 0, limit);
+          wait_limited(bar_last, 0, limit);
+          sc.i = *s_acc;
+        }
+        limit = __all_sync(0xffffffffu, limit != 0) ? limit : 0;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t acc = lane_base + sc.i * p.npad;
+        uint32_t nx[16];                                     // the next chunk (CUT_K has no registers for it)
+        if (!CUT_K && ch0 < nchunk) ld16(acc + ch0 * 16, nx);
+#pragma unroll 1
+        for (int ch = ch0; ch < nchunk; ch += step) {
+          uint32_t r[16];
+          if constexpr (CUT_K) {
+            ld16(acc + ch * 16, r);
+            wait_ld16(r);
+          } else {
+            wait_ld16(nx);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) r[j] = nx[j];
+            if (ch + step < nchunk) ld16(acc + (ch + step) * 16, nx);
+          }
+          if (CUT_K && q0 < me) {
+            for (int q = q0 + 1; q < me; ++q) {
+              const float* src = first + ((int64_t)(q - q0) * 2 * p.npad + ch * 16) * FEATS;
+#pragma unroll
+              for (int j = 0; j < 16; ++j) v[j] += __ldcg(src + j * FEATS);
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(v[j] + __uint_as_float(r[j]));
+            if (ch + step < nchunk) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) v[j] = __ldcg(first + ((ch + step) * 16 + j) * FEATS);
+            }
+          }
+          if (!CUT_K && add_run) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(run[(ch * 16 + j) * FEATS + feat] + __uint_as_float(r[j]));
+          }
+          if (!CUT_K && e < b1) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) run[(ch * 16 + j) * FEATS + feat] = __uint_as_float(r[j]);
+          } else if (CUT_K && !whole) {
+            float* dst = p.part + ((int64_t)(me * 2 + half) * p.npad + ch * 16) * FEATS + feat;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) __stcg(dst + j * FEATS, __uint_as_float(r[j]));
+          } else if (SILU) {
+            // the even CTA has silu's argument (matrix 0), the odd one the factor (matrix 1); each finishes eight of the 16 rows
+            // and sends the other what it needs for its own
+            union { uint4 v; __half2 h[4]; } keep, send;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const __half2 lo = __floats2half2_rn(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+              const __half2 hi = __floats2half2_rn(__uint_as_float(r[8 + 2 * j]), __uint_as_float(r[9 + 2 * j]));
+              keep.h[j] = half ? hi : lo;
+              send.h[j] = half ? lo : hi;
+            }
+            own[ch * FEATS + feat] = keep.v;
+            asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+                         ::"r"(mapa(smem_u32(other + ch * FEATS + feat), half ^ 1)), "r"(send.v.x), "r"(send.v.y), "r"(send.v.z),
+                           "r"(send.v.w), "r"(mapa(bar_x, half ^ 1)) : "memory");
+          } else {
+            // 16 rows x 128 features meet in shared memory, so that rows leave in 16-byte stores of 16 lanes (a warp's own
+            // 64 bytes of a row at a time: 85 cycles each, 11000 for a tile of 128 rows)
+            __half* o = out_g + (turn ^= 1) * 16 * OUT_LD;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) o[j * OUT_LD + feat] = __float2half_rn(__uint_as_float(r[j]));
+            asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+            store_rows(o, c + (int64_t)ch * 16 * ldc, ldc, min(16, rows - ch * 16), feat, p.vec);
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (!all && lane == 0) mbar_arrive_cluster(mapa(bar_accfree, lead) + 8 * sc.i);
+        sc.next(p.nacc);
+      }
+      if (CUT_K && q0 < me) {
+        // read: the last group makes the flags ready for the next launch
+        __syncwarp();
+        for (int q = q0 + lane; q < me; q += 32) {
+          int* flag = p.flags + q * 16 + half * 4 + quad;
+          if (atomicAdd(flag + 8, 1) == GROUPS - 1) { flag[0] = 0; flag[8] = 0; }
+        }
+      }
+      if (CUT_K && !whole) {
+        // published: GROUPS arrivals per flag, whoever drained the accumulator
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) atomicAdd(p.flags + me * 16 + half * 4 + quad, all ? 1 : GROUPS);
+      } else if (SILU) {
+        wait_limited(bar_x, group == 0 ? tiles & 1 : *s_tiles & 1, limit);
+        ++tiles;
+        for (int ch = all ? group : 0; ch < nchunk; ch += all ? GROUPS : 1) {
+          union { uint4 v; __half2 h[4]; } mine, theirs;
+          mine.v = own[ch * FEATS + feat];
+          theirs.v = other[ch * FEATS + feat];
+          __half* o = out_g + (turn ^= 1) * 16 * OUT_LD;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 f = __half22float2(half ? theirs.h[j] : mine.h[j]);
+            const __half2 sg = __floats2half2_rn(f.x / (1.0f + expf(-f.x)), f.y / (1.0f + expf(-f.y)));
+            const __half2 y = __hmul2(sg, half ? mine.h[j] : theirs.h[j]);
+            o[2 * j * OUT_LD + feat] = __low2half(y);
+            o[(2 * j + 1) * OUT_LD + feat] = __high2half(y);
+          }
+          asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+          const int row0 = ch * 16 + 8 * half;
+          store_rows(o, c + (int64_t)row0 * ldc, ldc, min(8, rows - row0), feat, p.vec);
+        }
+        __syncwarp();
+        if (!all && lane == 0) mbar_arrive_cluster(mapa(bar_xfree, half ^ 1));      // the other CTA may send its next tile's
+      }
+    }
+    failed = failed || limit == 0;
+  }
+  if (!mbar_wait(bar_done, 0) || failed) *s_failed = 1;
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  __syncthreads();
+  failed = *s_failed != 0;
+  if (failed && tid == 0) {
+    // the copies still on their way, those of the last S blocks at most: none may land in shared memory that has been given back
+    atomicExch(p.err, 1);
+    const int n = max(s_copied[0], s_copied[1]);
+    for (int i = max(0, n - S); i < n; ++i) mbar_wait(bar_full + 8 * (i % S), (uint32_t)((i / S) & 1));
+  }
+
+  if (SPLIT && !failed && warp >= DQ_WARP0) {
+    // accumulators -> fp32 tile [npad][128] over the ring, which is idle by now
+    float* tile_f = reinterpret_cast<float*>(gbase);
+    const int quad = warp & 3, set = (warp - DQ_WARP0) >> 2, feat = 32 * quad + lane;
+    for (int ch = set; ch < p.npad / 16; ch += (THREADS / 32 - DQ_WARP0) / 4) {
+      uint32_t r[16];
+      ld16(tmem + ((uint32_t)(32 * quad) << 16) + ch * 16, r);
+      wait_ld16(r);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) tile_f[(ch * 16 + j) * FEATS + feat] = __uint_as_float(r[j]);
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  cluster.sync();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TMEM_COLS));
+  }
+  if (!SPLIT) return;
+  // split-K: the r-th CTA of this half finishes the r-th slice of the (row, feature) pairs, adding the tiles in k order
+  float* tile_f = reinterpret_cast<float*>(gbase);
+  int pi, span, fh, m0;
+  decode(me, pi, span, fh, m0);
+  const int nranks = (int)gridDim.y, rank = (int)blockIdx.y;
+  const int rows = min(p.npad, p.M - m0), n_el = rows * FEATS;
+  const int per = ((n_el / 4 + nranks - 1) / nranks) * 4;
+  const int e0 = rank * per, e1 = min(n_el, e0 + per);
+  __half* c = p.c[pi] + (int64_t)m0 * p.ldc[pi] + span * SPAN + fh * FEATS;
+  if (!failed) {
+    for (int e = e0 + tid * 4; e < e1; e += THREADS * 4) {
+      float4 tt[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        tt[r] = (r < nranks) ? *reinterpret_cast<const float4*>(cluster.map_shared_rank(tile_f + e, 2 * r + half))
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
+      float4 v = tt[0];
+#pragma unroll
+      for (int r = 1; r < 4; ++r) { v.x += tt[r].x; v.y += tt[r].y; v.z += tt[r].z; v.w += tt[r].w; }
+      __half2* dst = reinterpret_cast<__half2*>(c + (int64_t)(e / FEATS) * p.ldc[pi] + e % FEATS);
+      dst[0] = __floats2half2_rn(v.x, v.y);
+      dst[1] = __floats2half2_rn(v.z, v.w);
+    }
+  }
+  cluster.sync();       // every rank has read the tiles: shared memory may go away
+}
+
+}  // namespace pair
+}  // namespace ttc
+}  // namespace q40
+
+using PairKernel = void (*)(const q40::ttc::pair::Params, const q40::ttc::pair::Maps);
+
+// [0] SPLIT; else 1 + NA == 4, + 2 SiLU, + 4 cut
+static PairKernel pair_kernel(int which) {
+  using namespace q40::ttc::pair;
+  switch (which) {
+    case 0: return gemm_pair_kernel<true, 4, false, false>;
+    case 1: return gemm_pair_kernel<false, 2, false, false>;
+    case 2: return gemm_pair_kernel<false, 4, false, false>;
+    case 3: return gemm_pair_kernel<false, 2, false, true>;
+    case 4: return gemm_pair_kernel<false, 4, false, true>;
+    case 6: return gemm_pair_kernel<false, 4, true, false>;
+    default: return gemm_pair_kernel<false, 4, true, true>;
+  }
+}
+
+// How many clusters of (2, nsplit) CTAs run at once, one CTA per SM (an answer is kept per device and split; 0, not kept,
+// when the runtime cannot tell)
+static int pair_max_clusters(PairKernel kern, int nsplit) {
+  using namespace q40::ttc;
+  static std::atomic<int> cache[16][5];
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  std::atomic<int>* kept = dev < 16 ? &cache[dev][nsplit] : nullptr;
+  if (kept && kept->load(std::memory_order_relaxed)) return kept->load(std::memory_order_relaxed) - 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(2048, nsplit, 1);
+  cfg.blockDim = dim3(pair::THREADS, 1, 1);
+  cfg.dynamicSmemBytes = SMEM_MAX;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = nsplit;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  if (kept) kept->store(n + 1, std::memory_order_relaxed);
+  return n;
+}
+
+namespace q40 {
+namespace ttc {
+namespace pair {
+
+// Shared memory of a launch, or 0 if it does not fit: [ring][run][SiLU halves][rows on their way out][barriers]
+static size_t layout(Params& p, int na, bool split) {
+  const size_t tile = (size_t)p.npad * FEATS * 4, stage = RAW_PAD + (size_t)p.npad * 64 * BLK;
+  const size_t run = p.range < p.k64 ? tile : 0, x = p.silu ? (size_t)p.npad / 16 * FEATS * 32 : 0, out = split ? 0 : 2 * 16 * OUT_LD * 2;
+  const size_t fixed = 1024 /* alignment */ + BAR_BYTES + 64 /* tail */ + run + x + out;
+  if (fixed + NA_MAX * stage > (size_t)SMEM_MAX) return 0;
+  p.stages = (int)((SMEM_MAX - fixed) / stage);
+  if (p.stages > S_MAX) p.stages = S_MAX;
+  size_t off = p.stages * stage;
+  if (split && off < tile) off = tile;                       // the fp32 tile of a split takes the ring's place
+  p.run_off = (int)off;
+  p.x_off = (int)(off + run);
+  p.out_off = (int)(off + run + x);
+  p.bar_off = (int)(off + run + x + out);
+  // more than half of an SM's: two pairs of different launches that each got one SM's tensor memory would wait for the other's
+  const size_t smem = off + fixed;
+  return smem < 116 * 1024 ? 116 * 1024 : smem;
+}
+
+// Rows of a tile -> accumulators and A buffers: two accumulators where they fit tensor memory beside at least two A buffers
+static int tile_rows(Params& p, int npad) {
+  p.npad = npad;
+  p.chunks = (p.M + npad - 1) / npad;
+  p.nacc = 2 * npad + 2 * A_COLS <= TMEM_COLS ? 2 : 1;
+  return TMEM_COLS - p.nacc * npad >= NA_MAX * A_COLS ? NA_MAX : 2;
+}
+
+// k steps -> blocks; `range` k steps are summed in tensor memory
+static void k_blocks(Params& p, int range) {
+  p.range = range;
+  p.rblk = (range + BLK - 1) / BLK;
+  const int nr = (p.k64 + range - 1) / range;
+  p.nblk = (nr - 1) * p.rblk + (p.k64 - (nr - 1) * range + BLK - 1) / BLK;
+}
+
+}  // namespace pair
+}  // namespace ttc
+}  // namespace q40
+
+// The launch that q40_gemm_tiled_tc_multi and q40_gemm_tiled_tc_ws make: see q40_tc_common.cuh.  Arguments are checked.
+//
+// Which launch: the one of least estimated time.  Nanoseconds on a B200, weights from HBM, launches in a row; npad = rows
+// of a tile, a block = 128 k of 256 features:
+//   a block           232 + npad / 4, or the MMAs' 2.2 npad (one tile per pair; 16 rows 236, 112 rows 258, 128 rows 283);
+//                     165 + 1.8 npad, 2.8 npad beyond 128, while all SMs draw activations from L2 (64 rows 287, 128 rows 390, 256 rows 710)
+//   a launch          3900 + 12 npad; with shared tiles 3800 + 28 npad more; with k split over the pairs of a cluster 700 more per
+//                     pair, and all of it once per wave of clusters (they are not persistent); a range after the first 16 npad for its sums where the next one's MMAs do not hide it
+// 10 rows x 4096 x 11008, two matrices: 16.8 us shared, 21.9 not, 29.3 split in two; 100 rows x 11008 x 4096: 15.7 split in
+// three, 17.6 in two, 27.5 not; 512 rows x 4096 x 11008: 128-row tiles 41.3, 112 39.5, 176 45.7, 256 57.2.
+int q40_pair_gemm(int nmat, const void* a, int64_t lda, const void* const* bw_tiled, void* const* c, const int64_t* ldc,
+                  const int* n_cols, int M, int K, int ranges, int silu, void* workspace, size_t workspace_bytes, double beat_ns,
+                  int* err, int use_pdl, void* stream) {
+  using namespace q40;
+  using namespace q40::ttc;
+  pair::Params p{};
+  int spans = 0;
+  p.vec = 1;
+  for (int i = 0; i < nmat; ++i) {
+    p.c[i] = (__half*)c[i]; p.ldc[i] = ldc[i];
+    p.spans[i] = n_cols[i] / SPAN;
+    p.vec &= q40_aligned(c[i], 16) && ldc[i] % 8 == 0;
+    spans += p.spans[i];
+  }
+  EncodeTiledFn encode = ttc_encode_fn();
+  if (!encode) return Q40_E_UNSUPPORTED;
+  p.nprob = nmat; p.M = M; p.K = K; p.err = err; p.silu = silu;
+  p.k64 = K / BK;
+  pair::k_blocks(p, ranges > 1 ? (p.k64 + ranges - 1) / ranges : p.k64);
+  if ((int64_t)spans * ((M + 63) / 64) * p.nblk > 0x7fffffffLL) return Q40_E_UNSUPPORTED;
+  // the kernels' attributes come first: the runtime is asked how many fit with the shared memory that they allow
+  static std::atomic<uint64_t> ready[9];
+  auto kernel = [&](int which) -> PairKernel {
+    PairKernel k = pair_kernel(which);
+    if (q40_allow_smem(ready[which], (const void*)k, SMEM_MAX) == cudaSuccess) return k;
+    (void)cudaGetLastError();
+    return nullptr;
+  };
+  PairKernel plain = kernel(2), in_clusters = kernel(0);
+  if (!plain || !in_clusters) return Q40_E_UNSUPPORTED;
+  const int fit = pair_max_clusters(plain, 1) < pair::MAX_PAIRS ? pair_max_clusters(plain, 1) : pair::MAX_PAIRS;
+  if (fit < 1) return Q40_E_UNSUPPORTED;
+
+  double best = beat_ns;
+  int npad = 0, split = 1, cut = 0;
+  if (M <= 128) {
+    const int n = (M + 15) / 16 * 16;
+    const double block = std::max(232.0 + 0.25 * n, 2.21 * n), launch = 3900 + 12.0 * n;
+    auto consider = [&](double ns, int sp, int ct) { if (ns < best) { best = ns; npad = n; split = sp; cut = ct; } };
+    consider(launch + (double)((spans + fit - 1) / fit) * p.nblk * block, 1, 0);
+    const int64_t units = (int64_t)spans * p.nblk / pair::CUT;
+    if (workspace && workspace_bytes >= q40_gemm_tiled_tc_ws_bytes(M) && units * 2 * pair::CUT >= (int64_t)fit * p.nblk)
+      consider(launch + 3800 + 28.0 * n + (double)spans * p.nblk / fit * block, 1, 1);
+    for (int sp = 2; sp <= 4 && !silu; ++sp) {
+      const int bps = (p.nblk + sp - 1) / sp, f = (sp - 1) * bps < p.nblk ? pair_max_clusters(in_clusters, sp) : 0;
+      if (f > 0) consider((double)((spans + f - 1) / f) * (launch + 700.0 * (sp - 1) + bps * block), sp, 0);
+    }
+  } else {
+    for (int n = 64; n <= pair::MAX_ROWS; n += 16) {
+      const int chunks = (M + n - 1) / n;
+      if (((M + chunks - 1) / chunks + 15) / 16 * 16 != n) continue;           // the same chunks with fewer rows of padding
+      const int na = pair::tile_rows(p, n);
+      if (pair::layout(p, na, false) == 0) continue;
+      const double waves = (double)(((int64_t)spans * chunks + fit - 1) / fit);
+      const double block = n <= 128 ? 165 + 1.8 * n : 395 + 2.8 * (n - 128);
+      const int nr = (p.k64 + p.range - 1) / p.range;
+      const double tile = nr > 1 ? nr * std::max(p.rblk * block + 1000, 16.5 * n) : p.nblk * block;
+      const double ns = 3900 + 12.0 * n + waves * tile;
+      if (ns < best) { best = ns; npad = n; }
+    }
+  }
+  if (npad == 0) return Q40_E_UNSUPPORTED;
+
+  const int na = pair::tile_rows(p, npad);
+  p.ntiles = spans * p.chunks;                   // SiLU: as many, of half a span of both matrices
+  p.cut = cut;
+  if (cut) {
+    p.flags = (int*)workspace;
+    p.part = (float*)((char*)workspace + pair::FLAG_BYTES);
+  }
+  int npairs = p.ntiles;
+  if (split > 1) {
+    p.bps = (p.nblk + split - 1) / split;
+  } else {
+    const int units = cut ? p.ntiles * p.nblk / pair::CUT : p.ntiles;
+    npairs = units < fit ? (units < 1 ? 1 : units) : fit;
+    p.share = units / npairs;
+    p.rest = units % npairs;
+  }
+  const size_t smem = pair::layout(p, na, split > 1);
+  if (smem == 0 || smem > (size_t)SMEM_MAX) return Q40_E_UNSUPPORTED;
+  PairKernel kern = kernel(split > 1 ? 0 : 1 + (na == pair::NA_MAX) + 2 * silu + 4 * cut);      // shared tiles have at most 128 rows: four A buffers
+  if (!kern) return Q40_E_UNSUPPORTED;
+  pair::Maps maps;
+  const cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)M};
+  const cuuint64_t gstride[1] = {(cuuint64_t)lda * 2};
+  const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)p.npad / 2};
+  const cuuint32_t estr[2] = {1, 1};
+  if (encode(&maps.act, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)a, gdim, gstride, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return Q40_E_UNSUPPORTED;
+  for (int i = 0; i < nmat; ++i) {
+    const cuuint64_t wdim[2] = {STEP_BYTES / 4, (cuuint64_t)p.spans[i] * (K / 16)};
+    const cuuint64_t wstride[1] = {STEP_BYTES};
+    const cuuint32_t wbox[2] = {256, 4 * pair::BLK}, sbox[2] = {16, 4 * pair::BLK};
+    for (int j = 0; j < 2; ++j)
+      if (encode(j ? &maps.s[i] : &maps.w[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, (void*)bw_tiled[i], wdim, wstride, j ? sbox : wbox,
+                 estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return Q40_E_UNSUPPORTED;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(2 * npairs, split, 1);
+  cfg.blockDim = dim3(pair::THREADS, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = (cudaStream_t)stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = split;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = use_pdl ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p, maps);
+  if (e != cudaSuccess) return (int)e;
+  return Q40_OK;
+}
+
+// Scratch of q40_gemm_tiled_tc_ws: flags and one slot of sums per pair (0: none is used for so many rows)
+extern "C" size_t q40_gemm_tiled_tc_ws_bytes(int M) {
+  using namespace q40::ttc::pair;
+  if (M < 1 || M > 128) return 0;
+  return (size_t)FLAG_BYTES + (size_t)MAX_PAIRS * 2 * ((M + 15) / 16 * 16) * FEATS * 4;
+}

@@ -327,8 +327,8 @@ def _tiled_copy_of(b_w, b_s, K, N, dev, st):
 def _tiled_matmul(dev, a, tiled, c, M, N, K, pdl, st) -> bool:
     """q40_matmul_tiled on a tiled copy; False if this device cannot schedule the clusters (up to 16 rows) or its
     driver has no tensor-map encoder (above)."""
-    # the error word of tc_error_flag(); the narrow kernel has no wait that could expire
-    err = _workspace("gemm", dev, 4096, zero=True).data_ptr() + 4092 if M > 16 else None
+    # the error word of tc_error_flag(); the narrow kernel (up to 8 rows) has no wait that could expire
+    err = _workspace("gemm", dev, 4096, zero=True).data_ptr() + 4092 if M > 8 else None
     for cluster in (_cluster_sizes.get(dev.index) or (16, 8)):
         rc = lib.q40_matmul_tiled(tiled.data_ptr(), c.data_ptr(), c.stride(0), a.data_ptr(), a.stride(0), M, N, K, cluster,
                                   err, 1 if pdl else 0, st)
@@ -373,6 +373,27 @@ def _cluster_gemv(dev, a, b_w, b_s, c, M, N, K) -> bool:
         if rc > 0:
             check(rc, "q40_gemv_fused")
     return False
+
+
+_TILED_TC_FLAGS = 8192      # bytes at the start of that scratch that have to be zero
+
+
+def _tiled_tc_workspace(dev, M: int) -> Optional[torch.Tensor]:
+    """Scratch of q40_gemm_tiled_tc_ws for M rows on this stream, or None where it uses none."""
+    nbytes = lib.q40_gemm_tiled_tc_ws_bytes(M)
+    if nbytes and torch.cuda.is_current_stream_capturing():
+        # the graph's own, made ready by each replay: one kept for later calls would not be until the first
+        buf = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+        buf[:_TILED_TC_FLAGS].zero_()
+        return buf
+    return _workspace("tiled_tc", dev, nbytes, zero=True) if nbytes else None
+
+
+def _reset_tiled_tc_workspaces(dev) -> None:
+    """After an expired wait: the launches in flight may have left their scratch in any state."""
+    for (kind, index, _), buf in list(_workspaces.items()):
+        if kind == "tiled_tc" and index == dev.index:
+            buf.zero_()
 
 
 def _indexed(dev) -> torch.device:

@@ -211,17 +211,16 @@ class Transformer(nn.Module):
         # when set, a decode step also writes argmax(logits) back as the next input token and
         # advances the positions on the device, so steps can be replayed without the host
         self.greedy_feedback = False
-        # kernels of this library enqueued by one decode step (per layer: 2 norms, 7 matmuls,
-        # rope+append, 2 attention, SiLU-mul; plus the final norm)
-        self.launches_per_step = params.n_layers * 13 + 1
-        # B <= 16 uses the fused, cluster-reduced, dependent-launch-chained matmuls
+        # kernels of this library enqueued by one decode step (set by it)
+        self.launches_per_step = params.n_layers * 9 + 1
+        # B <= 8 uses the fused, cluster-reduced, dependent-launch-chained matmuls; up to 16 what `_fused_body` says
         self.use_fused = True
         self.use_pdl = True
         self.max_cluster = 16
         # B <= 16: the fused matmuls read a rearranged ("tiled") copy of each weight, made on first use
         self.use_tiled = True
-        # B > 16 and the prompt pass: the tensor-core matmul that reads the same tiled copies (A operand
-        # written to tensor memory); False: the tensor-core matmul on the checkpoint layout
+        # B > 8 and the prompt pass: the tensor-core matmul that reads the same tiled copies (A operand
+        # written to tensor memory); False: B <= 16 as B <= 8, above the tensor-core matmul on the checkpoint layout
         self.use_tiled_tc = True
         # tensor parallel: all-reduce + residual add + RMSNorm as one launch over peer-mapped buffers (plain
         # stores into the peers' memory); False: torch.distributed all_reduce + the norm kernel
@@ -336,8 +335,11 @@ class Transformer(nn.Module):
             self._mm(ao, wo, [o], args[1], err, st)
             self._all_reduce(o)
             self._norm(h, o, ffn_norm, xn, st)
-            self._mm(xn, w13, [a1, a3], args[2], err, st)
-            check(lib.q40_silu_mul(a1.data_ptr(), a3.data_ptr(), g.data_ptr(), g.numel(), st), "q40_silu_mul")
+            if w13[1] is not None:
+                self._mm_silu(xn, w13[1], g, args[2], err, st)
+            else:
+                self._mm(xn, w13, [a1, a3], args[2], err, st)
+                check(lib.q40_silu_mul(a1.data_ptr(), a3.data_ptr(), g.data_ptr(), g.numel(), st), "q40_silu_mul")
             self._mm(g, w2, [f], args[3], err, st)
             self._all_reduce(f)
             pending = f
@@ -367,6 +369,7 @@ class Transformer(nn.Module):
     @torch.inference_mode()
     def _prompt_failed(self):
         self._tc_err.zero_()
+        K._reset_tiled_tc_workspaces(self.device)
         torch.cuda.synchronize(self.device)      # copies of passes in flight have landed
         self._tc_err_host.zero_()
         self._prompt_unchecked = False
@@ -415,6 +418,17 @@ class Transformer(nn.Module):
         for l, o in zip(lins, outs):
             K.matmul_q40(x, l.w, l.s, l.kn(), group_size=l.group_size, relayout=False, out=o)
 
+    def _mm_silu(self, x, tiled, g, args, err, st, ws=None, pdl=None):
+        """g = silu(x @ deq(W_1)) * (x @ deq(W_3)) for the tiled copies of the two: one launch, with the scratch `ws` (of
+        this stream, if none is given)."""
+        _, P, widths64, widths = args
+        if ws is None:
+            ws = K._tiled_tc_workspace(x.device, x.shape[0])
+        check(lib.q40_gemm_tiled_tc_ws(2, x.data_ptr(), x.stride(0), P(*[t.data_ptr() for t in tiled]), P(*[g.data_ptr()] * 2),
+                                       widths64, widths, x.shape[0], x.shape[1], 1, ws.data_ptr() if ws is not None else None,
+                                       ws.numel() if ws is not None else 0, err.data_ptr() if isinstance(err, torch.Tensor) else err,
+                                       1 if (self.use_pdl if pdl is None else pdl) else 0, st), "q40_gemm_tiled_tc_ws")
+
     # ------------------------------------------------------------------ decode
     def _step_buffers(self, B):
         b = self._bufs.get(B)
@@ -430,6 +444,7 @@ class Transformer(nn.Module):
                      ao=e(B, H * D), o=e(B, p.dim), a1=e(B, hid), a3=e(B, hid), g=e(B, hid), f=e(B, p.dim),
                      attn_ws=torch.empty(nb_attn, dtype=torch.uint8, device=dev),
                      gemm_ws=torch.zeros(nb_gemm, dtype=torch.uint8, device=dev),
+                     tc_ws=torch.zeros(lib.q40_gemm_tiled_tc_ws_bytes(B) if B > 8 else 0, dtype=torch.uint8, device=dev),
                      logits=e(B, p.vocab_size), qkv=e(B, (H + 2 * Hkv) * D),
                      ss_attn=torch.zeros((B, 1024), dtype=torch.float32, device=dev),
                      ss_ffn=torch.zeros((B, 1024), dtype=torch.float32, device=dev))
@@ -444,10 +459,10 @@ class Transformer(nn.Module):
               "q40_gemm_kn")
 
     def _gemm_multi(self, bufs, x, lins, outs, st):
-        """Several projections of the same activations: one tensor-core launch above 16 rows when the
+        """Several projections of the same activations: one tensor-core launch above 8 rows when the
         shapes allow it, one launch per matrix otherwise."""
         M, n = x.shape[0], len(lins)
-        if M > 16 and self.use_tiled and self.use_tiled_tc and x.stride(0) % 8 == 0:
+        if M > 8 and self.use_tiled and self.use_tiled_tc and x.stride(0) % 8 == 0:
             # matrices that have a tiled copy (N % 256 == 0) go through the tensor-core kernel that reads it;
             # the others (e.g. one kv head per rank under 8-way tensor parallelism) keep the checkpoint layout
             t_idx = [i for i, (l, o) in enumerate(zip(lins, outs))
@@ -499,9 +514,26 @@ class Transformer(nn.Module):
                                        1 if self.use_pdl else 0, st),
               "q40_gemm_kn_tc_multi")
 
+    def _fused_body(self, B):
+        """Whether a step of B branches takes the narrow matmuls with their fused neighbours.  From 9 branches on the
+        tensor-core matmuls make up for two norm launches a layer (10 branches: 2.75 ms a step with the narrow ones), where the
+        shapes and switches allow them."""
+        if not self.use_fused or B > 16 or self.tp_world > 1:
+            return False
+        if B <= 8 or self.use_stream or self._lm_head_q4 is not None or not (self.use_tiled and self.use_tiled_tc):
+            return True
+        layer = self.layers[0]
+        return not all(l.group_size == 64 and self._tileable(l) and l.kn()[0] % 64 == 0 for l in _projections(layer))
+
+    def _silu_pair(self, B, ff):
+        """Whether w1 and w3 of a step of B branches are one launch with the SiLU product."""
+        lins = (ff.w1, ff.w3)
+        return (B > 8 and self.use_tiled and self.use_tiled_tc and lins[0].kn() == lins[1].kn() and
+                all(l.group_size == 64 and self._tileable(l) and l.kn()[0] % 64 == 0 for l in lins))
+
     def _decode_body(self, B):
         """Enqueue one decode step for B branches on the current stream (captured into a graph)."""
-        if self.use_fused and B <= 16 and self.tp_world == 1:
+        if self._fused_body(B):
             return self._decode_body_fused(B)
         return self._decode_body_unfused(B)
 
@@ -654,7 +686,7 @@ class Transformer(nn.Module):
                 p.max_prompt_seq_len + p.max_seq_len <= self.fused_attn_max_keys)
 
     def _decode_body_fused(self, B):
-        """Decode step for B <= 16 branches: 7 launches per layer (qkv with RMSNorm prologue,
+        """Decode step for B <= 8 branches (16: see `_fused_body`): 7 launches per layer (qkv with RMSNorm prologue,
         rope+append, 2 attention, wo with residual epilogue, w1/w3 with RMSNorm prologue and
         SiLU-mul epilogue, w2 with residual epilogue), chained with programmatic dependent launch."""
         p, bufs = self.params, self._step_buffers(B)
@@ -792,9 +824,14 @@ class Transformer(nn.Module):
             else:
                 self._all_reduce(bufs["o"])
                 self._norm(h, bufs["o"], layer.ffn_norm.weight, xn, st)
-            self._gemm_multi(bufs, xn, [ff.w1, ff.w3], [bufs["a1"], bufs["a3"]], st)
-            check(lib.q40_silu_mul(bufs["a1"].data_ptr(), bufs["a3"].data_ptr(), bufs["g"].data_ptr(),
-                                   bufs["g"].numel(), st), "q40_silu_mul")
+            if self._silu_pair(B, ff):
+                tiled, pdl = self._tiled_of((ff.w1, ff.w3))
+                self._mm_silu(xn, tiled, bufs["g"], self._mm_args([l.kn()[1] for l in (ff.w1, ff.w3)]),
+                              bufs["gemm_ws"].data_ptr() + 4096 - 4, st, bufs["tc_ws"] if bufs["tc_ws"].numel() else None, pdl)
+            else:
+                self._gemm_multi(bufs, xn, [ff.w1, ff.w3], [bufs["a1"], bufs["a3"]], st)
+                check(lib.q40_silu_mul(bufs["a1"].data_ptr(), bufs["a3"].data_ptr(), bufs["g"].data_ptr(),
+                                       bufs["g"].numel(), st), "q40_silu_mul")
             self._gemm_multi(bufs, bufs["g"], [ff.w2], [bufs["f"]], st)
             if peer is not None:
                 # ... of the partial w2 outputs + residual add + the next layer's attention norm (or the final norm)
@@ -864,8 +901,9 @@ class Transformer(nn.Module):
         """Run one decode step for B branches with the tokens/positions already in the device
         buffers (`_tok_dev`, `_pos_dev`); returns the static logits buffer [B, vocab]."""
         self._check_prompt()
-        fused = self.use_fused and B <= 16 and self.tp_world == 1
-        self.launches_per_step = self.params.n_layers * ((5 if self._fused_attn_for(B) else 7) if fused else 13) + (2 if fused else 1)
+        fused = self._fused_body(B)
+        per_layer = (5 if self._fused_attn_for(B) else 7) if fused else (9 if self._silu_pair(B, self.layers[0].feed_forward) else 10)
+        self.launches_per_step = self.params.n_layers * per_layer + (2 if fused else 1)
         if not self.use_cuda_graph:
             return self._decode_body(B)
         key = (B, self.greedy_feedback, self.use_fused, self.use_pdl, self.max_cluster, self.use_stream,
@@ -901,7 +939,7 @@ class Transformer(nn.Module):
                 self._pos_dev[:B] -= 1
                 self._tok_dev[:B].copy_(tok_saved)
         g.replay()
-        if self._lm_head_q4 is not None and fused:
+        if self._lm_head_q4 is not None and fused:      # only narrow steps compute with it
             return self._bufs[B]["logits_pad"][:, :self.params.vocab_size]
         return self._bufs[B]["logits"]
 

@@ -1,0 +1,103 @@
+"""GPU tests of the tensor-core matmul by pairs of CTAs (q40_gemm_tiled_tc_ws): edges of its tiles, of its k blocks and of
+the shares that pairs take of a tile, against the numpy oracle."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import q40_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def K():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from spec_mcts_b200 import kernels
+    return kernels
+
+
+def mats(K, rng, Kd, Ns):
+    packed = [O.quantize_q40((rng.standard_normal((Kd, n)) * 0.1).astype(np.float16), 64) for n in Ns]
+    tiled = [K.relayout_tiled(torch.from_numpy(q).cuda(), torch.from_numpy(s).cuda(), (Kd, n)) for (q, s), n in zip(packed, Ns)]
+    return packed, tiled
+
+
+def scratch(K, M):
+    from spec_mcts_b200._lib import lib
+    return torch.zeros(max(lib.q40_gemm_tiled_tc_ws_bytes(M), 16), dtype=torch.uint8, device="cuda")
+
+
+def launch(a, tiled, outs, Ns, silu, ws, pdl=0):
+    from spec_mcts_b200._lib import check, lib
+    n = len(tiled)
+    P = ctypes.c_void_p * n
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    check(lib.q40_gemm_tiled_tc_ws(n, a.data_ptr(), a.stride(0), P(*[t.data_ptr() for t in tiled]), P(*[o.data_ptr() for o in outs]),
+                                   (ctypes.c_int64 * n)(*[o.stride(0) for o in outs]), (ctypes.c_int * n)(*Ns), a.shape[0],
+                                   a.shape[1], silu, ws.data_ptr(), ws.numel(), err.data_ptr(), pdl,
+                                   torch.cuda.current_stream().cuda_stream), "q40_gemm_tiled_tc_ws")
+    assert int(err.item()) == 0
+
+
+def close(got, want):
+    # fp32 sums of fp16 operands in any order: rel 2^-11 for the rounded result and 2^-24 per addition, against the
+    # oracle's own fp16 result; the floor is that of cancelled sums (a few fp16 steps of the mean magnitude)
+    want = want.astype(np.float32)
+    scale = float(np.abs(want).mean())
+    np.testing.assert_allclose(got.float().cpu().numpy(), want, rtol=2e-3, atol=4e-3 * max(scale, 1e-6))
+
+
+# rows at the edges of 16-row tiles, of the two ways of tensor memory (192, 256) and of the row chunks; k of one step, an odd
+# number of steps, and whole blocks; one span and several; enough tiles for pairs to share them (75 spans)
+@pytest.mark.parametrize("M,Kd,Ns", [(9, 64, (256,)), (16, 192, (256, 512)), (17, 128, (256,)), (100, 4160, (512,)), (128, 320, (256, 256, 256)),
+                                     (129, 64, (512,)), (192, 320, (256,)), (193, 256, (512, 256)), (256, 192, (256,)), (257, 1024, (256,)),
+                                     (10, 256, (9728, 9728)), (112, 448, (19200,)), (300, 192, (19200,))])
+def test_products_at_the_edges(K, M, Kd, Ns):
+    rng = np.random.default_rng(M * 100 + Kd)
+    packed, tiled = mats(K, rng, Kd, Ns)
+    a = rng.standard_normal((M, Kd)).astype(np.float16)
+    a_d, ws = torch.from_numpy(a).cuda(), scratch(K, M)
+    outs = [torch.full((M, n), float("nan"), dtype=torch.float16, device="cuda") for n in Ns]
+    launch(a_d, tiled, outs, Ns, 0, ws)
+    for o, (q, s), n in zip(outs, packed, Ns):
+        close(o, O.matmul_q40(a, q, s, (Kd, n)))
+    # once more behind a dependent launch of the same scratch: the same bits, and the flags as they were found
+    again = [torch.empty_like(o) for o in outs]
+    launch(a_d, tiled, again, Ns, 0, ws, 1)
+    assert all(torch.equal(x, y) for x, y in zip(outs, again))
+    assert not ws[:8192].any()
+
+
+def test_rows_and_strides_outside_stay(K):
+    """Outputs that are column ranges of a wider buffer, at 16-byte and at 4-byte alignment, and activations with a row pitch:
+    nothing around them is written."""
+    rng = np.random.default_rng(5)
+    M, Kd, n = 21, 192, 256
+    packed, tiled = mats(K, rng, Kd, (n,))
+    wide = torch.from_numpy(rng.standard_normal((M, Kd + 8)).astype(np.float16)).cuda()
+    a = wide[:, :Kd]
+    want = O.matmul_q40(np.ascontiguousarray(a.cpu().numpy()), *packed[0], (Kd, n))
+    for first, pitch in ((8, 272), (2, 262)):
+        buf = torch.full((M + 1, pitch), 7.0, dtype=torch.float16, device="cuda")
+        launch(a, tiled, [buf[:M, first:first + n]], (n,), 0, scratch(K, M))
+        close(buf[:M, first:first + n], want)
+        assert (buf[:M, :first] == 7).all() and (buf[:M, first + n:] == 7).all() and (buf[M] == 7).all()
+
+
+@pytest.mark.parametrize("M,Kd,n", [(9, 64, 256), (16, 192, 512), (77, 1088, 512), (128, 256, 256), (129, 320, 512), (300, 192, 1024),
+                                    (20, 256, 9728)])
+def test_silu_product_is_that_of_the_separate_launches(K, M, Kd, n):
+    rng = np.random.default_rng(M + Kd)
+    _, tiled = mats(K, rng, Kd, (n, n))
+    a, ws = torch.from_numpy(rng.standard_normal((M, Kd)).astype(np.float16)).cuda(), scratch(K, M)
+    outs = [torch.empty((M, n), dtype=torch.float16, device="cuda") for _ in range(2)]
+    launch(a, tiled, outs, (n, n), 0, ws)
+    g = torch.full((M, n), float("nan"), dtype=torch.float16, device="cuda")
+    launch(a, tiled, [g, g], (n, n), 1, ws, 1)
+    want = K.silu_mul(*outs)
+    # k may be cut at other places, which moves a sum by its last fp32 bits and a product by an fp16 step of either factor
+    np.testing.assert_allclose(g.float().cpu().numpy(), want.float().cpu().numpy(), rtol=4e-3, atol=1e-4)
+    assert (g == want).float().mean() > 0.97
