@@ -13,16 +13,11 @@
 // cat(prompt.expand(B), suffix) for SDPA (hf_model_q40_kv_shared.py:375-376, 405).
 //
 // Algorithmic traffic: prefix K/V once per (kv head, row block); Q and the partials are
-// small next to it.
-#include <math_constants.h>
-
-#include "attn_common.cuh"
+// small next to it.  What bounds it: a warp's chain of MMAs and softmax per tile (2.1 us; see attn_tile.cuh), start, first
+// tile and partials around it.
+#include "attn_tile.cuh"
 
 namespace q40 {
-
-constexpr int PF_KT = 64;                      // keys per tile
-constexpr int PF_ROW_BYTES = ATTN_D * 2;       // 256 B per key
-constexpr int PF_TILE_BYTES = PF_KT * PF_ROW_BYTES;  // 16 KB
 
 struct PrefixArgs {
   const __half* q;    // branch b, head h at q + b*q_stride + h*D
@@ -38,43 +33,6 @@ struct PrefixArgs {
   float scale_log2;
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool pred) {
-  const int sz = pred ? 16 : 0;  // size 0 = write zeros
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(sz));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N)); }
-
-__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
-}
-__device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
-}
-__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                        uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// byte offset of 16-byte chunk `chunk` (0..15) of row `row` in a [rows][256 B] tile, XOR-swizzled so
-// that the 8 rows of an ldmatrix 8x8 block fall in different bank groups
-__device__ __forceinline__ uint32_t tile_off(int row, int chunk) {
-  return (uint32_t)(row * PF_ROW_BYTES + ((chunk ^ (row & 7)) << 4));
-}
-__device__ __forceinline__ uint32_t pack_h2(float a, float b) {
-  __half2 h = __floats2half2_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&h);
-}
-
 // grid: (nsp, Hkv, row blocks); block: NWARPS*32 threads, 16 query rows per warp.
 template <int NWARPS>
 __global__ void __launch_bounds__(NWARPS * 32)
@@ -83,10 +41,11 @@ attn_prefix_kernel(const PrefixArgs a) {
   constexpr int RB = NWARPS * 16;
   constexpr int NT = NWARPS * 32;
   extern __shared__ __align__(128) unsigned char smem[];
-  // [stage][K tile | V tile]; the Q rows are staged through the same memory first
+  // [Q rows][stage][K tile | V tile]
   const uint32_t sbase = smem_u32(smem);
-  asm volatile("griddepcontrol.launch_dependents;");   // a dependent may start prefetching its weights
-  asm volatile("griddepcontrol.wait;" ::: "memory");               // ... but nothing of the previous launch is read before it is done
+  asm volatile("griddepcontrol.wait;" ::: "memory");               // nothing of the previous launch is read before it is done
+  // the branch kernel behind this one starts when that holds for all of these CTAs, and walks its own keys beside them
+  asm volatile("griddepcontrol.launch_dependents;");
 
   const int sp = blockIdx.x, hk = blockIdx.y, rblk = blockIdx.z;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -97,9 +56,16 @@ attn_prefix_kernel(const PrefixArgs a) {
   const int plen = a.prefix_len_dev ? min(max(a.prefix_len_dev[0], 0), a.prefix_len) : a.prefix_len;
   const int k_begin = sp * a.keys_per_split;
   const int k_end = min(plen, k_begin + a.keys_per_split);
-  const int ntiles = (k_end > k_begin) ? (k_end - k_begin + PF_KT - 1) / PF_KT : 0;
+  const int ntiles = (k_end > k_begin) ? (k_end - k_begin + TILE_KEYS - 1) / TILE_KEYS : 0;
 
-  // ---- Q rows -> shared (swizzled) -> A fragments in registers ----
+  const uint32_t stages = sbase + RB * TILE_ROW_BYTES;
+  auto load = [&](int tile, int stage) {
+    const int key0 = k_begin + tile * TILE_KEYS;
+    const uint32_t kdst = stages + stage * 2 * TILE_BYTES;
+    const int64_t off = (int64_t)key0 * a.key_stride + (int64_t)hk * a.head_stride;
+    load_tile<NT>(kdst, kdst + TILE_BYTES, a.pk + off, a.pv + off, a.key_stride, a.key_stride, k_end - key0, tid);
+  };
+  // ---- Q rows -> shared (swizzled) -> A fragments in registers, with the first tile on its way ----
   for (int idx = tid; idx < RB * 16; idx += NT) {
     const int r = idx >> 4, ch = idx & 15;
     const int gr = row0 + r;
@@ -109,134 +75,33 @@ attn_prefix_kernel(const PrefixArgs a) {
     cp_async16(sbase + tile_off(r, ch), src, ok);
   }
   cp_async_commit();
-  cp_async_wait<0>();
-  __syncthreads();
-  uint32_t qa[8][4];
-  {
-    const int mi = lane >> 3, r8 = lane & 7;
-    const int row = warp * 16 + r8 + (mi & 1) * 8;
-#pragma unroll
-    for (int ks = 0; ks < 8; ++ks)
-      ldsm_x4(sbase + tile_off(row, 2 * ks + (mi >> 1)), qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3]);
-  }
-  __syncthreads();  // Q staging area is free again
-
-  auto load_tile = [&](int tile, int stage) {
-    const int key0 = k_begin + tile * PF_KT;
-    const uint32_t kdst = sbase + stage * 2 * PF_TILE_BYTES;
-    const uint32_t vdst = kdst + PF_TILE_BYTES;
-    for (int idx = tid; idx < PF_KT * 16; idx += NT) {
-      const int r = idx >> 4, ch = idx & 15;
-      const int key = key0 + r;
-      const bool ok = key < k_end;
-      const int64_t off = (int64_t)(ok ? key : k_begin) * a.key_stride + (int64_t)hk * a.head_stride + ch * 8;
-      cp_async16(kdst + tile_off(r, ch), a.pk + off, ok);
-      cp_async16(vdst + tile_off(r, ch), a.pv + off, ok);
-    }
-  };
-
-  float m_run[2] = {-CUDART_INF_F, -CUDART_INF_F}, l_run[2] = {0.f, 0.f};
-  float oacc[16][4];
-#pragma unroll
-  for (int i = 0; i < 16; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) oacc[i][j] = 0.f;
-
-  if (ntiles > 0) load_tile(0, 0);
+  if (ntiles > 0) load(0, 0);
   cp_async_commit();
+  cp_async_wait<1>();
+  __syncthreads();
+  WarpRows w;
+  w.init();
+  w.load_q(sbase, warp * 16, lane);
 
+  const bool any_row = row0 + warp * 16 < rows;      // a warp without rows only helps to load
   for (int tile = 0; tile < ntiles; ++tile) {
     const int stage = tile & 1;
-    if (tile + 1 < ntiles) load_tile(tile + 1, stage ^ 1);
+    if (tile + 1 < ntiles) load(tile + 1, stage ^ 1);
     cp_async_commit();
     cp_async_wait<1>();   // the tile for this iteration has landed
     __syncthreads();
-    const uint32_t kt = sbase + stage * 2 * PF_TILE_BYTES;
-    const uint32_t vt = kt + PF_TILE_BYTES;
-
-    // ---- S = Q K^T for 16 rows x 64 keys ----
-    float sacc[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) sacc[i][j] = 0.f;
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      const int krow = nt * 8 + (lane & 7);
-#pragma unroll
-      for (int ks = 0; ks < 8; ks += 2) {
-        uint32_t b0, b1, b2, b3;
-        ldsm_x4(kt + tile_off(krow, 2 * ks + (lane >> 3)), b0, b1, b2, b3);
-        mma_f16(sacc[nt], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b0, b1);
-        mma_f16(sacc[nt], qa[ks + 1][0], qa[ks + 1][1], qa[ks + 1][2], qa[ks + 1][3], b2, b3);
-      }
-    }
-    // ---- scale, mask the tail, online softmax (rows g and g+8 of this warp) ----
-    const int key0 = k_begin + tile * PF_KT;
-    float mx[2] = {-CUDART_INF_F, -CUDART_INF_F};
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int key = key0 + nt * 8 + 2 * t + (j & 1);
-        const float v = (key < k_end) ? sacc[nt][j] * a.scale_log2 : -CUDART_INF_F;
-        sacc[nt][j] = v;
-        mx[j >> 1] = fmaxf(mx[j >> 1], v);
-      }
-    }
-    float corr[2];
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
-      mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
-      const float mnew = fmaxf(m_run[r], mx[r]);   // finite: every tile holds at least one key
-      corr[r] = exp2f(m_run[r] - mnew);
-      m_run[r] = mnew;
-      l_run[r] *= corr[r];
-    }
-    float ls[2] = {0.f, 0.f};
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float p = exp2f(sacc[nt][j] - m_run[j >> 1]);
-        sacc[nt][j] = p;
-        ls[j >> 1] += p;
-      }
-    }
-    l_run[0] += ls[0];   // per-lane partial sums; combined across the quad at the end
-    l_run[1] += ls[1];
-#pragma unroll
-    for (int dt = 0; dt < 16; ++dt) {
-      oacc[dt][0] *= corr[0]; oacc[dt][1] *= corr[0];
-      oacc[dt][2] *= corr[1]; oacc[dt][3] *= corr[1];
-    }
-    // ---- O += P V ----
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-      const uint32_t a0 = pack_h2(sacc[2 * kk][0], sacc[2 * kk][1]);
-      const uint32_t a1 = pack_h2(sacc[2 * kk][2], sacc[2 * kk][3]);
-      const uint32_t a2 = pack_h2(sacc[2 * kk + 1][0], sacc[2 * kk + 1][1]);
-      const uint32_t a3 = pack_h2(sacc[2 * kk + 1][2], sacc[2 * kk + 1][3]);
-      const int vrow = kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
-#pragma unroll
-      for (int dt = 0; dt < 16; dt += 2) {
-        uint32_t b0, b1, b2, b3;
-        ldsm_x4_t(vt + tile_off(vrow, dt + (lane >> 4)), b0, b1, b2, b3);
-        mma_f16(oacc[dt], a0, a1, a2, a3, b0, b1);
-        mma_f16(oacc[dt + 1], a0, a1, a2, a3, b2, b3);
-      }
+    const uint32_t kt = stages + stage * 2 * TILE_BYTES, vt = kt + TILE_BYTES;
+    const int n = k_end - k_begin - tile * TILE_KEYS;          // every tile holds at least one key
+    if (any_row) {
+      if (n >= TILE_KEYS) w.step<false>(kt, vt, a.scale_log2, 0, 0, lane);
+      else w.step<true>(kt, vt, a.scale_log2, n, n, lane);
     }
     __syncthreads();  // all warps are done with this stage before it is refilled
   }
   cp_async_wait<0>();
 
   // ---- write the partial (m, l, O) of rows g and g+8 ----
-#pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 1);
-    l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 2);
-  }
+  w.finish();
   const int64_t total_rows = (int64_t)a.B * a.H;
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
@@ -244,11 +109,11 @@ attn_prefix_kernel(const PrefixArgs a) {
     if (gr >= rows) continue;
     const int b = gr / rep, j = gr % rep;
     const int64_t ridx = (int64_t)sp * total_rows + (int64_t)b * a.H + hk * rep + j;
-    if (t == 0) { a.pm[ridx] = m_run[r]; a.pl[ridx] = l_run[r]; }
+    if (t == 0) { a.pm[ridx] = w.m[r]; a.pl[ridx] = w.l[r]; }
     float* dst = a.po + ridx * D;
 #pragma unroll
     for (int dt = 0; dt < 16; ++dt)
-      *reinterpret_cast<float2*>(dst + dt * 8 + 2 * t) = make_float2(oacc[dt][2 * r], oacc[dt][2 * r + 1]);
+      *reinterpret_cast<float2*>(dst + dt * 8 + 2 * t) = make_float2(w.o[dt][2 * r], w.o[dt][2 * r + 1]);
   }
 }
 
@@ -256,7 +121,7 @@ static int prefix_splits(int B, int H, int Hkv, int prefix_len) {
   const int rep = H / Hkv;
   const int rows = B * rep;
   const int rblocks = (rows + 127) / 128;
-  const int tiles = (prefix_len + PF_KT - 1) / PF_KT;
+  const int tiles = (prefix_len + TILE_KEYS - 1) / TILE_KEYS;
   // CTAs per SM to aim for: two for the 64-row variant (128 threads; measured best for 2048 keys x 64
   // rows), one for the 128-row variant; never round up past whole waves (a 149th CTA doubles the time
   // of one SM)
@@ -271,21 +136,20 @@ static int prefix_splits(int B, int H, int Hkv, int prefix_len) {
 
 // pa.prefix_len is the (maximum) prefix length the grid is sized for
 static int launch_prefix(PrefixArgs& pa, int nsp, cudaStream_t st) {
-  const int tiles = (pa.prefix_len + PF_KT - 1) / PF_KT;
-  pa.keys_per_split = ((tiles + nsp - 1) / nsp) * PF_KT;
+  const int tiles = (pa.prefix_len + TILE_KEYS - 1) / TILE_KEYS;
+  pa.keys_per_split = ((tiles + nsp - 1) / nsp) * TILE_KEYS;
   const int rep = pa.H / pa.Hkv, rows = pa.B * rep;
-  const size_t smem = 4 * PF_TILE_BYTES;  // two stages of K and V (also covers 128 staged Q rows)
+  const auto smem = [](int warps) { return (size_t)warps * 16 * TILE_ROW_BYTES + 4 * TILE_BYTES; };      // the Q rows, two stages of K and V
+  static std::atomic<uint64_t> ready[2];
+  cudaError_t e;
   if (rows <= 64) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefix_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    e = q40_launch_pdl(attn_prefix_kernel<4>, dim3(nsp, pa.Hkv, 1), dim3(128), smem, st, pa);
-    if (e != cudaSuccess) return (int)e;
+    e = q40_allow_smem(ready[0], (const void*)attn_prefix_kernel<4>, (int)smem(4));
+    if (e == cudaSuccess) e = q40_launch_pdl(attn_prefix_kernel<4>, dim3(nsp, pa.Hkv, 1), dim3(128), smem(4), st, pa);
   } else {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefix_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    e = q40_launch_pdl(attn_prefix_kernel<8>, dim3(nsp, pa.Hkv, (rows + 127) / 128), dim3(256), smem, st, pa);
-    if (e != cudaSuccess) return (int)e;
+    e = q40_allow_smem(ready[1], (const void*)attn_prefix_kernel<8>, (int)smem(8));
+    if (e == cudaSuccess) e = q40_launch_pdl(attn_prefix_kernel<8>, dim3(nsp, pa.Hkv, (rows + 127) / 128), dim3(256), smem(8), st, pa);
   }
+  if (e != cudaSuccess) return (int)e;
   return Q40_OK;
 }
 
@@ -294,7 +158,7 @@ static int launch_prefix(PrefixArgs& pa, int nsp, cudaStream_t st) {
 extern "C" size_t q40_attn_shared_prefix_workspace_bytes(int B, int H, int D, int prefix_len) {
   if (B <= 0 || H <= 0 || D != q40::ATTN_D || prefix_len <= 0) return 0;
   // the split count depends on Hkv; Hkv = 1 with 128-row blocks gives the largest count
-  const int tiles = (prefix_len + q40::PF_KT - 1) / q40::PF_KT;
+  const int tiles = (prefix_len + q40::TILE_KEYS - 1) / q40::TILE_KEYS;
   const int max_sp = tiles < 296 ? tiles : 296;
   return (size_t)max_sp * B * H * (D + 2) * sizeof(float);
 }

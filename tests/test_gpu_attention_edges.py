@@ -1,0 +1,51 @@
+"""GPU tests of the attention kernels at the edges of their tiles, pages and row splits, against the numpy oracle."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import q40_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+# fp16 operands and result, fp32 sums and softmax: an fp16 step of the result and the hardware's 2^x (2 ulp of fp32)
+TOL = dict(rtol=2e-3, atol=1e-3)
+
+
+@pytest.fixture(scope="module")
+def K():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from spec_mcts_b200 import kernels
+    return kernels
+
+
+def normal(rng, *shape):
+    return rng.standard_normal(shape).astype(np.float16)
+
+
+# one tile, a tile's last and first key, ragged splits; one row block, its edge (64 rows) and two, with branches of no own keys
+@pytest.mark.parametrize("B,prefix,Hkv", [(1, 1, 2), (3, 64, 2), (5, 65, 1), (64, 130, 2), (65, 63, 2), (130, 500, 2)])
+def test_prefix_beside_own_keys(K, B, prefix, Hkv):
+    rng = np.random.default_rng(B + prefix)
+    H, page, pages = 2, 16, 3
+    q, pk, pv = normal(rng, B, H, 128), normal(rng, prefix, Hkv, 128), normal(rng, prefix, Hkv, 128)
+    kp, vp = normal(rng, Hkv, B * pages * page, 128), normal(rng, Hkv, B * pages * page, 128)
+    table = rng.permutation(B * pages).reshape(B, pages).astype(np.int32)
+    lens = rng.integers(0, pages * page + 1, B).astype(np.int32)
+    d = lambda x: torch.from_numpy(x).cuda()
+    args = (d(q), d(pk), d(pv), prefix, d(table), d(lens), d(kp), d(vp))
+    want = O.attn_shared_prefix(q, pk, pv, prefix, table, lens, kp, vp, page)
+    outs = [K.shared_prefix_attn(*args, page_size=page) for _ in range(3)]      # the scratch of one is the next one's
+    for o in outs:
+        np.testing.assert_allclose(o.float().cpu().numpy(), want.astype(np.float32), **TOL)
+        assert torch.equal(o, outs[0])
+
+
+@pytest.mark.parametrize("S", [1, 16, 63, 65, 127, 193])
+def test_causal_blocks(K, S):
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, k, v = (torch.randn((S, h, 128), generator=g, device="cuda").half() for h in (4, 2, 2))
+    s = torch.einsum("ihd,jhd->hij", q.double(), k.double().repeat_interleave(2, 1)) / 128 ** 0.5
+    s = s.masked_fill(torch.ones((S, S), device="cuda", dtype=torch.bool).triu(1), float("-inf"))
+    want = torch.einsum("hij,jhd->ihd", torch.softmax(s, -1), v.double().repeat_interleave(2, 1))
+    np.testing.assert_allclose(K.causal_attn(q, k, v).float().cpu().numpy(), want.float().cpu().numpy(), **TOL)
