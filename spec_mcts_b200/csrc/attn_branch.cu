@@ -19,25 +19,35 @@
 
 namespace q40 {
 
-// Page ids are looked up one iteration ahead of the keys they lead to, and the shared-prefix pass's row maxima
-// and sums before the key loop, so that an iteration waits for one memory latency and not for two.
+// Page ids are looked up one iteration ahead of the keys they lead to, so that an iteration waits for one memory latency
+// and not for two.
 //
 // A CTA has NW warps; WPR of them share a row (branch, head).  What bounds a row is latency (ids -> keys -> sums
-// -> merge), so the split is the one that keeps the warps of all rows resident at once: see launch_branch.
+// -> merge), so the split is the one that keeps the warps of all rows resident at once: see launch_branch_mode.
 
-// Slot of key t of branch b: in the pool (paged), or just t (contiguous)
+// Slot of key t of branch b: in the pool (paged), or just t (contiguous).  `row` is the branch's first page id.  (With a division
+// by the page size and 64-bit products per key, slots were a third of a paged row's instructions.)
 template <int MODE>  // 0 contiguous, 1 paged with int16 ids, 2 paged with int32 ids, 3 Q4_0 cache
-__device__ __forceinline__ int key_slot(const BranchArgs& a, int b, int t) {
+__device__ __forceinline__ int key_slot(const BranchArgs& a, const void* row, int t) {
   if (MODE == 0 || MODE == 3) return t;
-  const int pg = t / a.page_size, in = t - pg * a.page_size;
-  int64_t id;
-  if (MODE == 1)
-    id = (int64_t)(uint16_t) reinterpret_cast<const int16_t*>(a.tbl)[(int64_t)b * a.tbl_stride + pg];
-  else
-    id = (int64_t) reinterpret_cast<const int32_t*>(a.tbl)[(int64_t)b * a.tbl_stride + pg];
-  const int64_t slot = id * a.page_size + in;
+  const int pg = a.page_shift >= 0 ? t >> a.page_shift : t / a.page_size, in = t - pg * a.page_size;
+  const int id = MODE == 1 ? (int)(uint16_t) reinterpret_cast<const int16_t*>(row)[pg] : reinterpret_cast<const int32_t*>(row)[pg];
   // a bad page id must not turn into a wild read: clamp into the pool
-  return (int)min(max(slot, (int64_t)0), (int64_t)a.P - 1);
+  return min(min(max(id, 0), a.last_page) * a.page_size + in, a.P - 1);
+}
+
+// 2^x as the hardware gives it: exp2f without its detour for results below 2^-126, which are nothing beside a row's largest, 1
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// acc + a.x b.x + a.y b.y: the products of fp16 values are exact, each sum rounds once
+__device__ __forceinline__ float dot2(__half2 a, __half2 b, float acc) {
+  asm("{\n\t.reg .b16 a0, a1, b0, b1;\n\tmov.b32 {a0, a1}, %1;\n\tmov.b32 {b0, b1}, %2;\n\t"
+      "fma.rn.f32.f16 %0, a0, b0, %0;\n\tfma.rn.f32.f16 %0, a1, b1, %0;\n\t}" : "+f"(acc) : "r"(h2_as_u32(a)), "r"(h2_as_u32(b)));
+  return acc;
 }
 
 // a row's two scales in one word
@@ -53,7 +63,9 @@ attn_branch_kernel(const BranchArgs a) {
   constexpr int RT = WPR * 32;                // threads of a row
   constexpr int NG = WPR * 4;                 // key groups of a row
   asm volatile("griddepcontrol.launch_dependents;");   // a dependent may start prefetching its weights
-  asm volatile("griddepcontrol.wait;" ::: "memory");               // ... but nothing of the previous launch is read before it is done
+  // ... but nothing of the previous launch is read before it is done.  Behind a prefix pass, which lets this launch start only
+  // when everything in front of it is done, that is the pass's results alone: the branch's own keys are read beside it
+  if (!a.beside_prefix) asm volatile("griddepcontrol.wait;" ::: "memory");
   const int tid = threadIdx.x, lane = tid & 31;
   const int slot = (NW == WPR) ? 0 : (tid >> 5) / WPR;      // row of this CTA
   const int64_t bh = (int64_t)blockIdx.x * (NW / WPR) + slot;
@@ -73,35 +85,22 @@ attn_branch_kernel(const BranchArgs a) {
   // first page ids.  They wait for the length: entries beyond it need not exist (the last row of a table that is a
   // column range of a wider one ends with the allocation).  Ids of every row but the last ahead of the length, by a
   // branch around two copies of these loads: 2 to 9 % slower on short rows, also without lengths
+  const void* const table = MODE == 1 ? (const void*)(reinterpret_cast<const int16_t*>(a.tbl) + (int64_t)b * a.tbl_stride)
+                                      : (const void*)(reinterpret_cast<const int32_t*>(a.tbl) + (int64_t)b * a.tbl_stride);
   int slots[U];
   if (MODE == 1 || MODE == 2) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) slots[u] = (grp + u * NG < len) ? key_slot<MODE>(a, b, grp + u * NG) : 0;
+    for (int u = 0; u < U; ++u) slots[u] = (grp + u * NG < len) ? key_slot<MODE>(a, table, grp + u * NG) : 0;
   }
-
-  // prefix partials: lane sp holds the maximum and the sum of split sp (further splits are read at the merge)
-  const float pm_l = lane < a.nsp ? a.pm[(int64_t)lane * rows + bh] : -CUDART_INF_F;
-  const float pl_l = lane < a.nsp ? a.pl[(int64_t)lane * rows + bh] : 0.f;
 
   __shared__ float sm_m[NW * 4], sm_l[NW * 4];
   __shared__ __align__(16) float sm_o[NW * 4][D];
 
-  // this lane's 16 query dims, pre-multiplied by scale*log2(e)
-  float qf[16];
+  __half2 qh[8];                              // this lane's 16 query dims
   {
     const __half* qp = a.q + (int64_t)b * a.q_stride + h * D + sub * 8;
-    const uint4 q0 = *reinterpret_cast<const uint4*>(qp);
-    const uint4 q1 = *reinterpret_cast<const uint4*>(qp + 64);
-    const __half2* h0 = reinterpret_cast<const __half2*>(&q0);
-    const __half2* h1 = reinterpret_cast<const __half2*>(&q1);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 f0 = __half22float2(h0[i]), f1 = __half22float2(h1[i]);
-      qf[2 * i] = f0.x * a.scale_log2;
-      qf[2 * i + 1] = f0.y * a.scale_log2;
-      qf[8 + 2 * i] = f1.x * a.scale_log2;
-      qf[8 + 2 * i + 1] = f1.y * a.scale_log2;
-    }
+    *reinterpret_cast<uint4*>(qh) = *reinterpret_cast<const uint4*>(qp);
+    *reinterpret_cast<uint4*>(qh + 4) = *reinterpret_cast<const uint4*>(qp + 64);
   }
   float m = -CUDART_INF_F, l = 0.f, o[16];
 #pragma unroll
@@ -130,7 +129,7 @@ attn_branch_kernel(const BranchArgs a) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int t = t0 + (U + u) * NG;
-        slots[u] = (t < len) ? key_slot<MODE>(a, b, t) : 0;
+        slots[u] = (t < len) ? key_slot<MODE>(a, table, t) : 0;
       }
     }
     float mnew = m;
@@ -139,25 +138,21 @@ attn_branch_kernel(const BranchArgs a) {
       const __half2* kh = reinterpret_cast<const __half2*>(&kv[u][0]);  // 8 half2 = 16 dims
       float acc = 0.f;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float2 f = __half22float2(kh[i]);
-        acc = fmaf(qf[2 * i], f.x, acc);
-        acc = fmaf(qf[2 * i + 1], f.y, acc);
-      }
+      for (int i = 0; i < 8; ++i) acc = dot2(qh[i], kh[i], acc);
       acc += __shfl_xor_sync(gmask, acc, 1);
       acc += __shfl_xor_sync(gmask, acc, 2);
       acc += __shfl_xor_sync(gmask, acc, 4);
-      s[u] = (t0 + u * NG < len) ? acc : -CUDART_INF_F;
+      s[u] = (t0 + u * NG < len) ? acc * a.scale_log2 : -CUDART_INF_F;
       mnew = fmaxf(mnew, s[u]);
     }
     // t0 < len, so mnew is finite here
-    const float corr = exp2f(m - mnew);
+    const float corr = ex2(m - mnew);
     l *= corr;
 #pragma unroll
     for (int i = 0; i < 16; ++i) o[i] *= corr;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const float p = exp2f(s[u] - mnew);
+      const float p = ex2(s[u] - mnew);
       l += p;
       const __half2* vh = reinterpret_cast<const __half2*>(&kv[u][2]);
 #pragma unroll
@@ -171,7 +166,13 @@ attn_branch_kernel(const BranchArgs a) {
   }
 
   if (MODE == 3) {
-    // Q4_0 cache: lane `sub` owns bytes 8*sub..8*sub+7 of a row, both nibbles
+    // Q4_0 cache: lane `sub` owns bytes 8*sub..8*sub+7 of a row, both nibbles; a word's bytes come out as (0, 2) and (1, 3)
+    __half2 q4[8];
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+      q4[i] = __lows2half2(qh[i], qh[i + 1]);
+      q4[i + 1] = __highs2half2(qh[i], qh[i + 1]);
+    }
     const bool sc4 = (((uintptr_t)a.ksc | (uintptr_t)a.vsc) & 3) == 0;
     for (int t0 = grp; t0 < len; t0 += NG * U) {
       uint2 kb[U], vb[U];
@@ -199,32 +200,24 @@ attn_branch_kernel(const BranchArgs a) {
 #pragma unroll
         for (int wi = 0; wi < 2; ++wi) {
           const uint32_t w = wi ? kb[u].y : kb[u].x;
-          const float2 h02 = __half22float2(__hmul2(codes_hi_to_h2(w), sh));        // bytes 0, 2
-          const float2 h13 = __half22float2(__hmul2(codes_hi_to_h2(w >> 8), sh));   // bytes 1, 3
-          const float2 l02 = __half22float2(__hmul2(codes_lo_to_h2(w), sl));
-          const float2 l13 = __half22float2(__hmul2(codes_lo_to_h2(w >> 8), sl));
-          acc = fmaf(qf[4 * wi + 0], h02.x, acc);
-          acc = fmaf(qf[4 * wi + 2], h02.y, acc);
-          acc = fmaf(qf[4 * wi + 1], h13.x, acc);
-          acc = fmaf(qf[4 * wi + 3], h13.y, acc);
-          acc = fmaf(qf[8 + 4 * wi + 0], l02.x, acc);
-          acc = fmaf(qf[8 + 4 * wi + 2], l02.y, acc);
-          acc = fmaf(qf[8 + 4 * wi + 1], l13.x, acc);
-          acc = fmaf(qf[8 + 4 * wi + 3], l13.y, acc);
+          acc = dot2(q4[2 * wi], __hmul2(codes_hi_to_h2(w), sh), acc);                // bytes 0, 2
+          acc = dot2(q4[2 * wi + 1], __hmul2(codes_hi_to_h2(w >> 8), sh), acc);       // bytes 1, 3
+          acc = dot2(q4[4 + 2 * wi], __hmul2(codes_lo_to_h2(w), sl), acc);
+          acc = dot2(q4[4 + 2 * wi + 1], __hmul2(codes_lo_to_h2(w >> 8), sl), acc);
         }
         acc += __shfl_xor_sync(gmask, acc, 1);
         acc += __shfl_xor_sync(gmask, acc, 2);
         acc += __shfl_xor_sync(gmask, acc, 4);
-        s[u] = (t0 + u * NG < len) ? acc : -CUDART_INF_F;
+        s[u] = (t0 + u * NG < len) ? acc * a.scale_log2 : -CUDART_INF_F;
         mnew = fmaxf(mnew, s[u]);
       }
-      const float corr = exp2f(m - mnew);
+      const float corr = ex2(m - mnew);
       l *= corr;
 #pragma unroll
       for (int i = 0; i < 16; ++i) o[i] *= corr;
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const float p = exp2f(s[u] - mnew);
+        const float p = ex2(s[u] - mnew);
         l += p;
         const __half2 sh = __low2half2(u32_as_h2(vsv[u])), sl = __high2half2(u32_as_h2(vsv[u]));
 #pragma unroll
@@ -257,18 +250,13 @@ attn_branch_kernel(const BranchArgs a) {
     const __half2* kh1 = reinterpret_cast<const __half2*>(&k1);
     float acc = 0.f;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 f0 = __half22float2(kh0[i]), f1 = __half22float2(kh1[i]);
-      acc = fmaf(qf[2 * i], f0.x, acc);
-      acc = fmaf(qf[2 * i + 1], f0.y, acc);
-      acc = fmaf(qf[8 + 2 * i], f1.x, acc);
-      acc = fmaf(qf[8 + 2 * i + 1], f1.y, acc);
-    }
+    for (int i = 0; i < 4; ++i) acc = dot2(qh[4 + i], kh1[i], dot2(qh[i], kh0[i], acc));
     acc += __shfl_xor_sync(0x000000ffu, acc, 1);
     acc += __shfl_xor_sync(0x000000ffu, acc, 2);
     acc += __shfl_xor_sync(0x000000ffu, acc, 4);
+    acc *= a.scale_log2;
     const float mnew = fmaxf(m, acc);
-    const float corr = exp2f(m - mnew), p = exp2f(acc - mnew);
+    const float corr = ex2(m - mnew), p = ex2(acc - mnew);
     l = l * corr + p;
     const __half2* vh0 = reinterpret_cast<const __half2*>(&v0);
     const __half2* vh1 = reinterpret_cast<const __half2*>(&v1);
@@ -283,6 +271,21 @@ attn_branch_kernel(const BranchArgs a) {
     m = mnew;
   }
 
+  if (a.beside_prefix) asm volatile("griddepcontrol.wait;" ::: "memory");
+  // prefix partials: lane sp holds the maximum and the sum of split sp (further splits are read at the merge)
+  const float pm_l = lane < a.nsp ? a.pm[(int64_t)lane * rows + bh] : -CUDART_INF_F;
+  const float pl_l = lane < a.nsp ? a.pl[(int64_t)lane * rows + bh] : 0.f;
+  // ... and the first splits' outputs at this thread's dims, all requested together and before the groups meet
+  constexpr int DP = RT >= D ? 1 : D / RT, PB = 16 / DP;
+  float po[PB][DP];
+  if (a.nsp > 0) {
+#pragma unroll
+    for (int i = 0; i < PB; ++i)
+#pragma unroll
+      for (int j = 0; j < DP; ++j)
+        po[i][j] = i < a.nsp && (RT <= D || tr < D) ? a.po[((int64_t)i * rows + bh) * D + tr + j * RT] : 0.f;
+  }
+
   const int g0 = slot * NG;
   if (sub == 0) { sm_m[g0 + grp] = m; sm_l[g0 + grp] = l; }
 #pragma unroll
@@ -293,7 +296,6 @@ attn_branch_kernel(const BranchArgs a) {
   else asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "n"(RT) : "memory");
 
   // merge: thread tr owns output dims tr, tr + RT, ... (WPR = 8: the first four warps)
-  constexpr int DP = RT >= D ? 1 : D / RT;
   if (RT > D && tr >= D) return;
   float M = -CUDART_INF_F;
 #pragma unroll
@@ -306,34 +308,30 @@ attn_branch_kernel(const BranchArgs a) {
   if (M > -CUDART_INF_F) {
 #pragma unroll
     for (int gI = 0; gI < NG; ++gI) {
-      const float w = exp2f(sm_m[g0 + gI] - M);   // exp2(-inf) = 0 for empty groups
+      const float w = ex2(sm_m[g0 + gI] - M);   // exp2(-inf) = 0 for empty groups
       Lsum = fmaf(sm_l[g0 + gI], w, Lsum);
 #pragma unroll
       for (int j = 0; j < DP; ++j) acc[j] = fmaf(sm_o[g0 + gI][tr + j * RT], w, acc[j]);
     }
-    const float pw_l = exp2f(pm_l - M);
-    // four splits' outputs requested together (splits from nsp on: weight and sum are 0): between the shuffles the loads
-    // waited for one another (a branch over 1000 shared keys of 8 kv heads, 16 splits: 20.7 us)
-    constexpr int PB = 4;
-    const int nsp32 = min(a.nsp, 32);
-    for (int sp0 = 0; sp0 < nsp32; sp0 += PB) {
-      float po[PB][DP];
+    if (a.nsp > 0) {
+      const float pw_l = ex2(pm_l - M);
 #pragma unroll
-      for (int i = 0; i < PB; ++i)
-#pragma unroll
-        for (int j = 0; j < DP; ++j)
-          po[i][j] = sp0 + i < nsp32 ? a.po[((int64_t)(sp0 + i) * rows + bh) * D + tr + j * RT] : 0.f;
-#pragma unroll
-      for (int i = 0; i < PB; ++i) {
-        const float w = __shfl_sync(0xffffffffu, pw_l, sp0 + i);
-        Lsum = fmaf(__shfl_sync(0xffffffffu, pl_l, sp0 + i), w, Lsum);
+      for (int i = 0; i < PB; ++i) {                // splits from nsp on: weight and sum are 0
+        const float w = __shfl_sync(0xffffffffu, pw_l, i);
+        Lsum = fmaf(__shfl_sync(0xffffffffu, pl_l, i), w, Lsum);
 #pragma unroll
         for (int j = 0; j < DP; ++j) acc[j] = fmaf(po[i][j], w, acc[j]);
+      }
+      for (int sp = PB; sp < min(a.nsp, 32); ++sp) {
+        const float w = __shfl_sync(0xffffffffu, pw_l, sp);
+        Lsum = fmaf(__shfl_sync(0xffffffffu, pl_l, sp), w, Lsum);
+#pragma unroll
+        for (int j = 0; j < DP; ++j) acc[j] = fmaf(a.po[((int64_t)sp * rows + bh) * D + tr + j * RT], w, acc[j]);
       }
     }
     for (int sp = 32; sp < a.nsp; ++sp) {
       const int64_t r = (int64_t)sp * rows + bh;
-      const float w = exp2f(a.pm[r] - M);
+      const float w = ex2(a.pm[r] - M);
       Lsum = fmaf(a.pl[r], w, Lsum);
 #pragma unroll
       for (int j = 0; j < DP; ++j) acc[j] = fmaf(a.po[r * D + tr + j * RT], w, acc[j]);
@@ -351,30 +349,43 @@ static int launch_rows(const BranchArgs& a, cudaStream_t st) {
   return e == cudaSuccess ? Q40_OK : (int)e;
 }
 
-// Warps per row by the number of rows, at 16 (U = 4), 20 or 24 (U = 2) warps an SM; microseconds on a B200, L2 flushed
-// unless a step is named:
-//   contiguous: four warps, four keys in flight; two warps a row are the same within 2 % at any width
-//   paged: eight warps while three CTAs an SM hold all rows (320 rows x 512 keys: 24.7 against 28.7) and there is
-//     more than a row per SM; then four warps with four keys in flight while four CTAs an SM hold all rows (512 rows x
-//     512 keys: 23.5 against 25.8 with two keys), with long rows of different lengths a fifth, for the short ones make room
-//     (608 rows of up to 768 keys: 31.0 against 34.9; of up to 128: 9.4 against 7.8); then two keys, which lets a fifth CTA in (608 rows x 512 keys: 26.5 against 36.5;
-//     1920 rows x 300 keys: 58.4 against 61.5); two warps a row above 16 rows an SM (3200 rows: 48.2 against 52.2)
-//   Q4_0 cache (a quarter of the bytes): two warps a row once four fill more than two waves (a decode step of 3200
-//     rows: 4.58 against 4.77 ms)
+// Warps per row and keys per 8-lane group by the number of rows; CTAs an SM at 128 registers a thread: two of eight warps with
+// four keys, three with two keys, four of four warps with four keys, five with two.  A row's chain of iterations is its
+// time while all rows are resident: eight warps while they are, then four; then what counts is that a row's start and
+// merge occupy few warps: two, with two rows a CTA.  Microseconds, written warps / keys (2 / 4 has two rows a CTA):
+//   paged, 512 keys: 256 rows 8 / 4 10.2, 8 / 2 13.3, 4 / 4 14.7; 416 rows 8 / 2 15.2, 4 / 4 16.7, 8 / 4 18.2; 256 keys: 512 rows
+//     4 / 4 10.1, 4 / 2 12.3, 8 / 4 12.0; 608 rows 4 / 2 13.1, 4 / 4 14.9, 2 / 4 15.3; 1024 rows 2 / 4 17.0, 4 / 4 19.0; 3200 rows
+//     2 / 4 50, 4 / 4 53.8; of up to 64: 768 rows 2 / 4 5.8, 4 / 4 6.5, 4 / 2 7.4.  Behind a prefix: 3200 rows of up to 64
+//     2 / 4 23.2, 4 / 4 30.1, of up to 256 49.7 and 52.1
+//   contiguous, 512 keys: 256 rows 8 / 4 12.6, 4 / 4 14.7; 416 rows 8 / 2 19.3, 4 / 4 19.9; 768 rows 4 / 4 35.9, 2 / 4 36.1; 3200 rows
+//     of 256 4 / 4 63.1, 2 / 4 67.0; of 64: 64 rows 4 / 4 2.6, 8 / 4 3.1; 768 rows 2 / 4 5.1, 4 / 4 5.9
+//   Q4_0 cache, whose length the host does not know, 20 / 64 / 200 keys, with the prefix pass: 64 rows 4 / 4 6.2 / 6.3 / 8.8, 8 / 2
+//     6.5 / 6.8 / 8.7; 320 rows 8 / 2 8.5 / 9.1 / 12.7, 4 / 4 8.8 / 9.0 / 13.5, 2 / 4 8.1 / 10.2 / 18.6; 640 rows 2 / 4 8.2 / 9.9 /
+//     18.4, 4 / 4 10.5 / 10.9 / 16.6; 960 rows 9.3 / 11.4 / 20.2 and 12.7 / 13.1 / 20.7; 3200 rows 19.3 / 23.8 / 46.8 and 29.5 / 30.4 / 53.5
+//     (a whole step of 320 rows with 64 keys: 8 / 2 2280, 4 / 4 2251)
 template <int MODE>
 static int launch_branch_mode(const BranchArgs& a, cudaStream_t st) {
+  const int64_t rows = a.rows;
   if constexpr (MODE == 1 || MODE == 2) {
-    if (a.rows > 148 && a.rows <= 3 * 148) return launch_rows<MODE, 8, 8, 2>(a, st);
-    if (a.rows > 16 * 148) return launch_rows<MODE, 4, 2, 4>(a, st);
-    if (a.rows > (a.seq_lens && a.L > 256 ? 5 : 4) * 148) return launch_rows<MODE, 4, 4, 2>(a, st);
-  }
-  if constexpr (MODE == 3) {
-    if (a.rows > 8 * 148) return launch_rows<MODE, 4, 2, 4>(a, st);
+    if (rows <= 2 * 148) return launch_rows<MODE, 8, 8, 4>(a, st);
+    if (rows <= 3 * 148) return launch_rows<MODE, 8, 8, 2>(a, st);
+    if (rows > 5 * 148 || (rows > 4 * 148 && a.L <= 128)) return launch_rows<MODE, 4, 2, 4>(a, st);
+    if (rows > 4 * 148) return launch_rows<MODE, 4, 4, 2>(a, st);
+  } else if constexpr (MODE == 0) {
+    if (a.L > 128 && rows <= 2 * 148) return launch_rows<MODE, 8, 8, 4>(a, st);
+    if (a.L > 128 && rows <= 3 * 148) return launch_rows<MODE, 8, 8, 2>(a, st);
+    if (a.L <= 128 && rows > 4 * 148) return launch_rows<MODE, 4, 2, 4>(a, st);
+  } else {
+    if (rows > 4 * 148) return launch_rows<MODE, 4, 2, 4>(a, st);
   }
   return launch_rows<MODE, 4, 4, 4>(a, st);
 }
 
 int launch_branch(BranchArgs a, int mode, int B, cudaStream_t st) {
+  a.page_shift = -1;
+  if (a.page_size > 0 && (a.page_size & (a.page_size - 1)) == 0)
+    for (a.page_shift = 0; (1 << a.page_shift) < a.page_size;) ++a.page_shift;
+  a.last_page = a.page_size > 0 && a.P > 0 ? (a.P - 1) / a.page_size : 0;
   a.rows = (int64_t)B * a.H;
   if (mode == 0) return launch_branch_mode<0>(a, st);
   if (mode == 1) return launch_branch_mode<1>(a, st);

@@ -18,12 +18,14 @@ struct BranchArgs {
   int64_t tbl_stride;
   const int32_t* seq_lens;  // per-branch length or nullptr (= L)
   int L, H, Hkv, P, page_size;
+  int page_shift, last_page;   // log2 of the page size or -1; id of the pool's last page (set by launch_branch)
   // optional partial results of a prefix pass over rows (b, h), log2 domain, un-normalised
   int64_t rows;           // B*H (set by launch_branch)
   const float* pm;        // [nsp][B*H]
   const float* pl;        // [nsp][B*H]
   const float* po;        // [nsp][B*H][128]
   int nsp;
+  int beside_prefix;      // the prefix pass is the launch in front of this one: its results are waited for at the merge
   float scale_log2;       // 1/sqrt(D) * log2(e)
   // Q4_0 suffix cache (mode 3): packed rows [B, max_t, Hkv, 64] + scales [B, max_t, Hkv, 2];
   // the branch's suffix length is pos[b] - prefix_len[0] (device values)

@@ -209,7 +209,7 @@ extern "C" int q40_attn_shared_prefix(const void* q, const void* prefix_k, const
     pa.scale_log2 = br.scale_log2;
     int rc = launch_prefix(pa, nsp, st);
     if (rc != Q40_OK) return rc;
-    br.pm = pm; br.pl = pl; br.po = po; br.nsp = nsp;
+    br.pm = pm; br.pl = pl; br.po = po; br.nsp = nsp; br.beside_prefix = 1;
   }
   // Lmax == 0: the branch kernel only merges the prefix partials
   const int mode = (Lmax == 0) ? 0 : (idx_bytes == 2 ? 1 : 2);
@@ -261,7 +261,7 @@ extern "C" int q40_attn_tree_decode(const void* q, int64_t q_stride, const void*
   br.q = (const __half*)q; br.q_stride = q_stride; br.o = (__half*)o;
   br.H = H; br.Hkv = Hkv; br.L = max_t;
   br.scale_log2 = pa.scale_log2;
-  br.pm = pm; br.pl = pl; br.po = po; br.nsp = nsp;
+  br.pm = pm; br.pl = pl; br.po = po; br.nsp = nsp; br.beside_prefix = 1;
   br.kq = (const int8_t*)cache_kq; br.ksc = (const __half*)cache_ks;
   br.vq = (const int8_t*)cache_vq; br.vsc = (const __half*)cache_vs;
   br.pos = pos_dev; br.prefix_len = prefix_len_dev; br.max_t = max_t;

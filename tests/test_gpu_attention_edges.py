@@ -23,6 +23,32 @@ def normal(rng, *shape):
     return rng.standard_normal(shape).astype(np.float16)
 
 
+# rows on either side of every split of warps (32 heads: 296, 444, 592, 740 rows), page sizes that are and are not powers of two
+@pytest.mark.parametrize("B,L,Hkv,page,idx", [(1, 1, 32, 1, np.int16), (9, 130, 32, 16, np.int32), (10, 65, 8, 3, np.int32), (14, 129, 32, 1, np.int16),
+                                              (19, 128, 32, 5, np.int32), (19, 140, 32, 1, np.int16), (24, 33, 32, 20, np.int32)])
+def test_paged_rows(K, B, L, Hkv, page, idx):
+    rng = np.random.default_rng(B * 7 + L)
+    H, pages = 32, -(-L // page)
+    P = B * pages * page
+    table = rng.permutation(B * pages).reshape(B, pages).astype(idx)
+    lens = rng.integers(0, L + 1, B).astype(np.int32)
+    lens[0], lens[-1] = L, L
+    q, k, v = normal(rng, B, H, 128), normal(rng, Hkv, P, 128), normal(rng, Hkv, P, 128)
+    d = lambda x: torch.from_numpy(x).cuda()
+    o = K.page_flash_attn(d(table), d(q), d(k), d(v), P, B, L, H, 128, page_size=page, seq_lens=d(lens)).float().cpu().numpy()
+    for b in range(B):
+        n = int(lens[b])
+        if n == 0:
+            assert not o[b].any()
+            continue
+        at = np.arange(n)
+        slot = table[b].astype(np.int64)[at // page] * page + at % page
+        kb, vb = (np.repeat(x[:, slot].astype(np.float64), H // Hkv, axis=0) for x in (k, v))
+        s = np.einsum("hd,hnd->hn", q[b].astype(np.float64), kb) / np.sqrt(128.0)
+        w = np.exp(s - s.max(axis=1, keepdims=True))
+        np.testing.assert_allclose(o[b], np.einsum("hn,hnd->hd", w / w.sum(axis=1, keepdims=True), vb), **TOL)
+
+
 # one tile, a tile's last and first key, ragged splits; one row block, its edge (64 rows) and two, with branches of no own keys
 @pytest.mark.parametrize("B,prefix,Hkv", [(1, 1, 2), (3, 64, 2), (5, 65, 1), (64, 130, 2), (65, 63, 2), (130, 500, 2)])
 def test_prefix_beside_own_keys(K, B, prefix, Hkv):
