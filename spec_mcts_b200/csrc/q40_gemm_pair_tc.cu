@@ -67,8 +67,8 @@ constexpr int OUT_LD = FEATS + 8;              // halves between rows that wait 
 constexpr int MAX_PAIRS = 128;
 constexpr int FLAG_BYTES = MAX_PAIRS * 64;      // at the start of the scratch, per pair: [half][quadrant] arrivals, then departures
 
-// Tensor maps: the activations, and per matrix the weights (box 1024 bytes x 8 steps) and scales (64 bytes x 8 steps) of a
-// tiled copy read as rows of one step
+// Tensor maps: the activations, and per matrix the weights (box 1024 bytes x 8 steps, half of it with SiLU) and scales (64 bytes x
+// 8 steps, or half) of a tiled copy read as rows of one step
 struct Maps { CUtensorMap act, w[3], s[3]; };
 
 struct Params {
@@ -84,8 +84,9 @@ struct Params {
   int share, rest;         // cut: a pair has share units of CUT blocks, the first `rest` pairs one more
   int bps;                 // SPLIT: blocks of a rank
   int stages, nacc;        // ring stages, accumulators
-  int run_off, x_off, out_off, bar_off;    // byte offsets in the aligned shared memory
-  int silu;                // c[0] = silu(A @ deq(B_0)) * (A @ deq(B_1)): a tile is half a span of both
+  int run_off, out_off, bar_off;           // byte offsets in the aligned shared memory
+  int silu;                // c[0] = silu(A @ deq(B_0)) * (A @ deq(B_1)): a tile is 128 features of
+                           // both, of which a CTA has 64 (its A rows 0..63 those of matrix 0)
   int vec;                 // outputs take 16-byte stores
   float* part;             // scratch slots: [pair][half][npad][128]
   int* flags;              // per pair: see FLAG_BYTES
@@ -142,14 +143,17 @@ __device__ __forceinline__ void wait_ld16(uint32_t (&r)[16]) {
                  "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]) :: "memory");
 }
 
-// `n` finished rows of 128 features from shared memory to the output, by the 128 threads t of a group
+// `n` finished rows of W features from shared memory to the output, by the 128 threads t of a group
+template <int W>
 __device__ __forceinline__ void store_rows(const __half* o, __half* c, int64_t ldc, int n, int t, int vec) {
   if (vec) {
-    for (int row = t >> 4; row < n; row += 8)
-      *reinterpret_cast<uint4*>(c + row * ldc + (t & 15) * 8) = *reinterpret_cast<const uint4*>(o + row * OUT_LD + (t & 15) * 8);
+    const int col = t % (W / 8) * 8;
+    for (int row = t / (W / 8); row < n; row += 1024 / W)
+      *reinterpret_cast<uint4*>(c + row * ldc + col) = *reinterpret_cast<const uint4*>(o + row * OUT_LD + col);
   } else {
-    for (int row = t >> 6; row < n; row += 2)
-      *reinterpret_cast<uint32_t*>(c + row * ldc + (t & 63) * 2) = *reinterpret_cast<const uint32_t*>(o + row * OUT_LD + (t & 63) * 2);
+    const int col = t % (W / 2) * 2;
+    for (int row = t / (W / 2); row < n; row += 256 / W)
+      *reinterpret_cast<uint32_t*>(c + row * ldc + col) = *reinterpret_cast<const uint32_t*>(o + row * OUT_LD + col);
   }
 }
 
@@ -216,30 +220,26 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
   // Block i has stage and barriers i % S and A buffer i % NA.  full: its weights and activations have landed in this
   // CTA; mdone: its MMAs are complete, in both CTAs; accfull[b]: an accumulator is complete.  In the even CTA, for both:
   // afull: the A operand is written (and the activations have landed); accfree[b]: an accumulator has been read.
-  const uint32_t bar_full = ring + (uint32_t)p.bar_off, bar_mdone = bar_full + 8 * S_MAX, bar_afull = bar_mdone + 8 * S_MAX, bar_accfull = bar_afull + 8 * NA_MAX,
-                 bar_accfree = bar_accfull + 16, bar_x = bar_accfree + 16, bar_xfree = bar_x + 8, bar_done = bar_xfree + 8, bar_last = bar_done + 8;
+  const uint32_t bar_full = ring + (uint32_t)p.bar_off, bar_mdone = bar_full + 8 * S_MAX, bar_afull = bar_mdone + 8 * S_MAX,
+                 bar_accfull = bar_afull + 8 * NA_MAX, bar_accfree = bar_accfull + 16, bar_done = bar_accfree + 16, bar_last = bar_done + 8;
   unsigned char* tail = gbase + p.bar_off + BAR_BYTES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail);
   volatile int* s_failed = reinterpret_cast<volatile int*>(tail + 8);
-  volatile int* s_acc = reinterpret_cast<volatile int*>(tail + 24);        // of a pair's last tile: accumulator, SiLU tiles before
-  volatile int* s_tiles = reinterpret_cast<volatile int*>(tail + 28);
+  volatile int* s_acc = reinterpret_cast<volatile int*>(tail + 24);        // accumulator of a pair's last tile
   volatile int* s_copied = reinterpret_cast<volatile int*>(tail + 16);     // [2] blocks whose copies were requested
   float* run = reinterpret_cast<float*>(gbase + p.run_off);                // [npad][128] sums of earlier ranges
   __half* out_s = reinterpret_cast<__half*>(gbase + p.out_off);            // [2][16][OUT_LD] finished rows on their way out
-  // SiLU: [npad / 16][128] halves of 16 rows that this CTA finishes, its own and the other CTA's
-  uint4* own = reinterpret_cast<uint4*>(gbase + p.x_off);
-  uint4* other = own + p.npad / 16 * FEATS;
 
   const int sb0 = SPLIT ? blockIdx.y * p.bps : 0, sb1 = SPLIT ? min(p.nblk, sb0 + p.bps) : 0;
   const Work wk(SPLIT ? me * p.nblk + sb0 : first_block(p, me, npairs),
                 SPLIT ? me * p.nblk + sb1 : first_block(p, me + 1, npairs), p.nblk);
   const int total = wk.u1 - wk.u0;                    // blocks of this pair
-  // matrix, span, 128-feature half of this CTA and first row of a tile
+  // matrix, span, 128-feature half of this CTA (SiLU: of the tile, in both matrices) and first row of a tile
   auto decode = [&](int tile, int& pi, int& span, int& fh, int& m0) {
     span = tile / p.chunks;
     m0 = (tile - span * p.chunks) * p.npad;
     if (SILU) {
-      pi = half;
+      pi = 0;
       fh = span & 1;
       span >>= 1;
       return;
@@ -268,8 +268,16 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
         const uint32_t dst = ring + s * stage_bytes;
         const int step = (span * p.k64 + kc.k) * 4;
         mbar_expect_tx(bar_full + 8 * s, RAW_BYTES);
-        tma_2d(dst, &maps.w[pi], fh * 256, step, bar_full + 8 * s);               // x in words of four bytes
-        tma_2d(dst + RAW_W, &maps.s[pi], 512 + fh * 16, step, bar_full + 8 * s);
+        if constexpr (SILU) {                                                    // a 64-column group of each matrix
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            tma_2d(dst + m * (RAW_W / 2), &maps.w[m], fh * 256 + half * 128, step, bar_full + 8 * s);    // x in words of four bytes
+            tma_2d(dst + RAW_W + m * (RAW_S / 2), &maps.s[m], 512 + fh * 16 + half * 8, step, bar_full + 8 * s);
+          }
+        } else {
+          tma_2d(dst, &maps.w[pi], fh * 256, step, bar_full + 8 * s);
+          tma_2d(dst + RAW_W, &maps.s[pi], 512 + fh * 16, step, bar_full + 8 * s);
+        }
         wslot.next(S);
         ++wi;
       }
@@ -285,8 +293,6 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
       }
       for (int s = 0; s < NA; ++s) mbar_init(bar_afull + 8 * s, 8);
       for (int s = 0; s < 2; ++s) { mbar_init(bar_accfull + 8 * s, 1); mbar_init(bar_accfree + 8 * s, 8); }
-      mbar_init(bar_x, 1);
-      mbar_init(bar_xfree, 4);
       mbar_init(bar_done, 1);
       mbar_init(bar_last, 4);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -393,8 +399,10 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
     // 16-row tile and 16 k, rows g and g + 8 at k = 4t .. 4t + 3
     const int quad = warp & 3, dset = (warp - DQ_WARP0) >> 2;
     const int q = quad >> 1, t = lane & 3;
-    const unsigned char* lane_w = gbase + (q * 32 + lane) * 16 + (quad & 1) * 8;
-    const unsigned char* lane_s = gbase + RAW_W + q * 32 + t * 8;
+    // bytes between half steps of a group, and between groups: of one matrix, side by side; with SiLU each of its own
+    constexpr int WSTEP = SILU ? 512 : 1024, SSTEP = SILU ? 32 : 64, WGRP = SILU ? RAW_W / 2 : 512, SGRP = SILU ? RAW_S / 2 : 32;
+    const unsigned char* lane_w = gbase + q * WGRP + lane * 16 + (quad & 1) * 8;
+    const unsigned char* lane_s = gbase + RAW_W + q * SGRP + t * 8;
     const uint32_t afull_lead = mapa(bar_afull, lead) + 8 * (dset % NA);
     const uint32_t ta = tmem + ((uint32_t)(32 * quad) << 16) + A_COL0 + dset % NA * A_COLS;
     Slot sl, sw;                                 // stage of this block, and of the one that used its A buffer before
@@ -417,7 +425,7 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
       for (int h = 0; h < BLK; ++h) {
         uint32_t r[2][16];
 #pragma unroll
-        for (int st = 0; st < 4; ++st) dequant_step(lane_w + so + (4 * h + st) * 1024, lane_s + so + (4 * h + st) * 64, r, st);
+        for (int st = 0; st < 4; ++st) dequant_step(lane_w + so + (4 * h + st) * WSTEP, lane_s + so + (4 * h + st) * SSTEP, r, st);
         st_16x256b_x4(ta + 32 * h, r[0]);
         st_16x256b_x4(ta + 32 * h + (16u << 16), r[1]);
       }
@@ -441,7 +449,7 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
     __half* out_g = group == 0 ? out_s : reinterpret_cast<__half*>(gbase) + (group - 1) * 2 * 16 * OUT_LD;
     const int nchunk = p.npad / 16;
     Slot sc;                                                 // accumulator
-    int turn = 0, tiles = 0;                                 // output buffer; finished tiles (SiLU)
+    int turn = 0;                                            // output buffer
     // outputs, scratch and flags may still be in use by the launch in front of this one
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (int k = group == 0 ? 0 : max(0, wk.np - 1); k < wk.np; ++k) {
@@ -450,8 +458,8 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
       decode(tile, pi, span, fh, m0);
       const bool whole = !CUT_K || b1 == p.nblk;                       // this pair has the tile's last blocks and finishes it
       const int rows = min(p.npad, p.M - m0);
-      const int64_t ldc = p.ldc[SILU ? 0 : pi];
-      __half* c = p.c[SILU ? 0 : pi] + (int64_t)m0 * ldc + span * SPAN + fh * FEATS;
+      const int64_t ldc = p.ldc[pi];
+      __half* c = p.c[pi] + (int64_t)m0 * ldc + span * SPAN + fh * FEATS + (SILU ? half * (FEATS / 2) : 0);
       // the pairs with its first blocks, whose sums are added in k order
       int q0 = me;
       if (CUT_K && whole && b0 > 0) {
@@ -482,18 +490,13 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
             for (int j = 0; j < 16; ++j) v[j] = __ldcg(first + (ch0 * 16 + j) * FEATS);
           }
         }
-        // (a barrier's parity tells a phase from its neighbours only: the other groups, which have not followed accfull and xfree,
+        // (a barrier's parity tells a phase from its neighbours only: the other groups, which have not followed accfull,
         // wait for the end of all MMAs and for group 0, which has)
         if (group == 0) {
           wait_limited(bar_accfull + 8 * sc.i, sc.turn, limit);
-          if (SILU && whole && e == b1) {
-            if (tiles > 0) wait_limited(bar_xfree, (tiles - 1) & 1, limit);
-            if (warp == EPI_WARP0 && lane == 0) mbar_expect_tx(bar_x, nchunk * FEATS * 16);
-          }
           __syncwarp();
           if (all && lane == 0) {
             *s_acc = sc.i;
-            *s_tiles = tiles;
             mbar_arrive(bar_last);
           }
         } else {
@@ -504,12 +507,13 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
         limit = __all_sync(0xffffffffu, limit != 0) ? limit : 0;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = lane_base + sc.i * p.npad;
-        uint32_t nx[16];                                     // the next chunk (CUT_K has no registers for it)
-        if (!CUT_K && ch0 < nchunk) ld16(acc + ch0 * 16, nx);
+        constexpr bool AHEAD = !CUT_K && !SILU;              // the others have no registers for it
+        uint32_t nx[16];                                     // the next chunk
+        if (AHEAD && ch0 < nchunk) ld16(acc + ch0 * 16, nx);
 #pragma unroll 1
         for (int ch = ch0; ch < nchunk; ch += step) {
           uint32_t r[16];
-          if constexpr (CUT_K) {
+          if constexpr (!AHEAD) {
             ld16(acc + ch * 16, r);
             wait_ld16(r);
           } else {
@@ -543,20 +547,32 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) __stcg(dst + j * FEATS, __uint_as_float(r[j]));
           } else if (SILU) {
-            // the even CTA has silu's argument (matrix 0), the odd one the factor (matrix 1); each finishes eight of the 16 rows
-            // and sends the other what it needs for its own
-            union { uint4 v; __half2 h[4]; } keep, send;
+            // warps 0 and 1 of a group have silu's argument (matrix 0), 2 and 3 the factor of the same features; each finish eight
+            // of the 16 rows and give the others, through the unused half of the output buffer, what they need for theirs
+            const int hi = quad >> 1, f64 = feat & 63;
+            union { uint4 v; __half2 h[4]; } mine, x;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              const __half2 lo = __floats2half2_rn(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
-              const __half2 hi = __floats2half2_rn(__uint_as_float(r[8 + 2 * j]), __uint_as_float(r[9 + 2 * j]));
-              keep.h[j] = half ? hi : lo;
-              send.h[j] = half ? lo : hi;
+              const __half2 r_lo = __floats2half2_rn(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+              const __half2 r_hi = __floats2half2_rn(__uint_as_float(r[8 + 2 * j]), __uint_as_float(r[9 + 2 * j]));
+              mine.h[j] = hi ? r_hi : r_lo;
+              x.h[j] = hi ? r_lo : r_hi;
             }
-            own[ch * FEATS + feat] = keep.v;
-            asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
-                         ::"r"(mapa(smem_u32(other + ch * FEATS + feat), half ^ 1)), "r"(send.v.x), "r"(send.v.y), "r"(send.v.z),
-                           "r"(send.v.w), "r"(mapa(bar_x, half ^ 1)) : "memory");
+            __half* o = out_g + (turn ^= 1) * 16 * OUT_LD;
+            const auto xchg = [&](int i) { return reinterpret_cast<uint4*>(o + (i >> 3) * OUT_LD + FEATS / 2 + (i & 7) * 8); };
+            *xchg(feat ^ 64) = x.v;
+            asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+            x.v = *xchg(feat);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float2 f = __half22float2(hi ? x.h[j] : mine.h[j]);
+              const __half2 sg = __floats2half2_rn(f.x / (1.0f + expf(-f.x)), f.y / (1.0f + expf(-f.y)));
+              const __half2 y = __hmul2(sg, hi ? mine.h[j] : x.h[j]);
+              o[(8 * hi + 2 * j) * OUT_LD + f64] = __low2half(y);
+              o[(8 * hi + 2 * j + 1) * OUT_LD + f64] = __high2half(y);
+            }
+            asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+            store_rows<FEATS / 2>(o, c + (int64_t)ch * 16 * ldc, ldc, min(16, rows - ch * 16), feat, p.vec);
           } else {
             // 16 rows x 128 features meet in shared memory, so that rows leave in 16-byte stores of 16 lanes (a warp's own
             // 64 bytes of a row at a time: 85 cycles each, 11000 for a tile of 128 rows)
@@ -564,7 +580,7 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) o[j * OUT_LD + feat] = __float2half_rn(__uint_as_float(r[j]));
             asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
-            store_rows(o, c + (int64_t)ch * 16 * ldc, ldc, min(16, rows - ch * 16), feat, p.vec);
+            store_rows<FEATS>(o, c + (int64_t)ch * 16 * ldc, ldc, min(16, rows - ch * 16), feat, p.vec);
           }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -585,28 +601,6 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
         __threadfence();
         __syncwarp();
         if (lane == 0) atomicAdd(p.flags + me * 16 + half * 4 + quad, all ? 1 : GROUPS);
-      } else if (SILU) {
-        wait_limited(bar_x, group == 0 ? tiles & 1 : *s_tiles & 1, limit);
-        ++tiles;
-        for (int ch = all ? group : 0; ch < nchunk; ch += all ? GROUPS : 1) {
-          union { uint4 v; __half2 h[4]; } mine, theirs;
-          mine.v = own[ch * FEATS + feat];
-          theirs.v = other[ch * FEATS + feat];
-          __half* o = out_g + (turn ^= 1) * 16 * OUT_LD;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float2 f = __half22float2(half ? theirs.h[j] : mine.h[j]);
-            const __half2 sg = __floats2half2_rn(f.x / (1.0f + expf(-f.x)), f.y / (1.0f + expf(-f.y)));
-            const __half2 y = __hmul2(sg, half ? mine.h[j] : theirs.h[j]);
-            o[2 * j * OUT_LD + feat] = __low2half(y);
-            o[(2 * j + 1) * OUT_LD + feat] = __high2half(y);
-          }
-          asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
-          const int row0 = ch * 16 + 8 * half;
-          store_rows(o, c + (int64_t)row0 * ldc, ldc, min(8, rows - row0), feat, p.vec);
-        }
-        __syncwarp();
-        if (!all && lane == 0) mbar_arrive_cluster(mapa(bar_xfree, half ^ 1));      // the other CTA may send its next tile's
       }
     }
     failed = failed || limit == 0;
@@ -721,20 +715,19 @@ namespace q40 {
 namespace ttc {
 namespace pair {
 
-// Shared memory of a launch, or 0 if it does not fit: [ring][run][SiLU halves][rows on their way out][barriers]
+// Shared memory of a launch, or 0 if it does not fit: [ring][run][rows on their way out][barriers]
 static size_t layout(Params& p, int na, bool split) {
   const size_t tile = (size_t)p.npad * FEATS * 4, stage = RAW_PAD + (size_t)p.npad * 64 * BLK;
-  const size_t run = p.range < p.k64 ? tile : 0, x = p.silu ? (size_t)p.npad / 16 * FEATS * 32 : 0, out = split ? 0 : 2 * 16 * OUT_LD * 2;
-  const size_t fixed = 1024 /* alignment */ + BAR_BYTES + 64 /* tail */ + run + x + out;
+  const size_t run = p.range < p.k64 ? tile : 0, out = split ? 0 : 2 * 16 * OUT_LD * 2;
+  const size_t fixed = 1024 /* alignment */ + BAR_BYTES + 64 /* tail */ + run + out;
   if (fixed + NA_MAX * stage > (size_t)SMEM_MAX) return 0;
   p.stages = (int)((SMEM_MAX - fixed) / stage);
   if (p.stages > S_MAX) p.stages = S_MAX;
   size_t off = p.stages * stage;
   if (split && off < tile) off = tile;                       // the fp32 tile of a split takes the ring's place
   p.run_off = (int)off;
-  p.x_off = (int)(off + run);
-  p.out_off = (int)(off + run + x);
-  p.bar_off = (int)(off + run + x + out);
+  p.out_off = (int)(off + run);
+  p.bar_off = (int)(off + run + out);
   // more than half of an SM's: two pairs of different launches that each got one SM's tensor memory would wait for the other's
   const size_t smem = off + fixed;
   return smem < 116 * 1024 ? 116 * 1024 : smem;
@@ -865,7 +858,7 @@ int q40_pair_gemm(int nmat, const void* a, int64_t lda, const void* const* bw_ti
   for (int i = 0; i < nmat; ++i) {
     const cuuint64_t wdim[2] = {STEP_BYTES / 4, (cuuint64_t)p.spans[i] * (K / 16)};
     const cuuint64_t wstride[1] = {STEP_BYTES};
-    const cuuint32_t wbox[2] = {256, 4 * pair::BLK}, sbox[2] = {16, 4 * pair::BLK};
+    const cuuint32_t wbox[2] = {silu ? 128u : 256u, 4 * pair::BLK}, sbox[2] = {silu ? 8u : 16u, 4 * pair::BLK};
     for (int j = 0; j < 2; ++j)
       if (encode(j ? &maps.s[i] : &maps.w[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, (void*)bw_tiled[i], wdim, wstride, j ? sbox : wbox,
                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
