@@ -30,7 +30,9 @@
 // latency 2, the last accumulator's way out 1 to 2, draining.  Microseconds, here and by the kernels before (one CTA per
 // tile, k split over clusters; up to 16 rows q40_gemv_tiled): 10 rows x 11008 x 4096 13.0 and 16.8, two x 4096 x 11008 16.9 and
 // 22.9; 100 rows x 11008 x 4096 15.7 and 20.8, two x 4096 x 11008 21.8 and 34.1; 512 rows x 4096 x 11008 39.5 and 61.4,
-// three x 4096 x 4096 45.5 and 82.5, x 11008 x 4096 37.2 and 48.6.
+// three x 4096 x 4096 45.5 and 82.5, x 11008 x 4096 37.2 and 48.6.  With the SiLU product: 10 rows 17.1 (18.8 while w1's and w3's
+// sums met through the other CTA's shared memory), 77 rows 21.9 (23.0), 100 rows 25.0 (27.7), 512 rows 72 (76); expf and the
+// division are half of what it costs (100 rows: 22.6 with approximate ones).
 //
 // Every wait is bounded: on expiry an error word is set, the remaining work skipped, copies and MMAs in flight
 // waited for, tensor memory freed.
@@ -565,6 +567,8 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
             x.v = *xchg(feat);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
+              if (ch * 16 + 8 * hi + 2 * j >= rows) break;   // padding: its share of exponentials and divisions is issue slots
+                                                             // the dequantisers want (100 rows 25.0 us, with it 27.0)
               const float2 f = __half22float2(hi ? x.h[j] : mine.h[j]);
               const __half2 sg = __floats2half2_rn(f.x / (1.0f + expf(-f.x)), f.y / (1.0f + expf(-f.y)));
               const __half2 y = __hmul2(sg, hi ? mine.h[j] : x.h[j]);
