@@ -5,7 +5,67 @@
 
 namespace q40 {
 
-// One CTA per row.  h = fp16(x + residual) (optional), y = fp16(fp16(h32 * rsqrt(mean(h32^2)+eps)) * w)
+// The same sums in the same order as rmsnorm_kernel below, for rows of up to NV vectors of eight per thread: a row stays in
+// registers and all of it is requested at once, the weights ahead of the previous launch's end.  One trip to L2 instead
+// of one per vector.  4096 wide, what a pass waits for it: 10 rows 2.8 and 3.7 us before, 1.9 and 1.6 now; 512 rows 6.8 and 4.9.
+template <int NV>
+__global__ void __launch_bounds__(256)
+rmsnorm_reg_kernel(const __half* __restrict__ x, const __half* __restrict__ residual, const __half* __restrict__ w,
+                   __half* __restrict__ y, __half* __restrict__ h_out, int dim, float eps) {
+  __shared__ float red[8];
+  const int tid = threadIdx.x;
+  uint4 wv[NV], v[NV], u[NV];
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    const int i = (n * 256 + tid) * 8;
+    wv[n] = i < dim ? __ldg(reinterpret_cast<const uint4*>(w + i)) : make_uint4(0, 0, 0, 0);
+  }
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int64_t at = (int64_t)blockIdx.x * dim + tid * 8;
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    const bool in = (n * 256 + tid) * 8 < dim;
+    v[n] = in ? *reinterpret_cast<const uint4*>(x + at + n * 2048) : make_uint4(0, 0, 0, 0);
+    if (residual) u[n] = in ? *reinterpret_cast<const uint4*>(residual + at + n * 2048) : make_uint4(0, 0, 0, 0);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    __half2* vh = reinterpret_cast<__half2*>(&v[n]);
+    const __half2* uh = reinterpret_cast<const __half2*>(&u[n]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (residual) vh[j] = __hadd2(vh[j], uh[j]);           // fp16 add, one rounding
+      const float2 f = __half22float2(vh[j]);
+      ss = fmaf(f.x, f.x, ss);
+      ss = fmaf(f.y, f.y, ss);
+    }
+  }
+  ss = warp_sum(ss);
+  if ((tid & 31) == 0) red[tid >> 5] = ss;
+  __syncthreads();
+  float tot = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) tot += red[i];
+  const float inv = rsqrtf(tot / (float)dim + eps);
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    if ((n * 256 + tid) * 8 >= dim) break;
+    if (residual && h_out) *reinterpret_cast<uint4*>(h_out + at + n * 2048) = v[n];
+    __half2* vh = reinterpret_cast<__half2*>(&v[n]);
+    const __half2* wh = reinterpret_cast<const __half2*>(&wv[n]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __half22float2(vh[j]);
+      const __half2 nn = __floats2half2_rn(f.x * inv, f.y * inv);   // round to fp16 first
+      vh[j] = __hmul2(nn, wh[j]);                                   // then * weight in fp16
+    }
+    *reinterpret_cast<uint4*>(y + at + n * 2048) = v[n];
+  }
+}
+
+// Rows of any width.  One CTA per row.  h = fp16(x + residual) (optional), y = fp16(fp16(h32 * rsqrt(mean(h32^2)+eps)) * w)
 __global__ void __launch_bounds__(256)
 rmsnorm_kernel(const __half* __restrict__ x, const __half* __restrict__ residual,
                const __half* __restrict__ w, __half* __restrict__ y, __half* __restrict__ h_out,
@@ -191,6 +251,11 @@ extern "C" int q40_rmsnorm(const void* x, const void* residual, const void* w, v
   if (!q40_aligned(x, 16) || !q40_aligned(w, 16) || !q40_aligned(y, 16) ||
       (residual && !q40_aligned(residual, 16)) || (h_out && !q40_aligned(h_out, 16)))
     return Q40_E_ALIGN;
+  // up to four vectors a thread in registers (beyond, what a thread holds no longer leaves room for eight CTAs on an SM)
+  auto reg = dim <= 2048 ? q40::rmsnorm_reg_kernel<1> : dim <= 4096 ? q40::rmsnorm_reg_kernel<2> : q40::rmsnorm_reg_kernel<4>;
+  if (dim <= 8192)
+    return (int)q40_launch_pdl(reg, dim3(rows), dim3(256), 0, (cudaStream_t)stream, (const __half*)x, (const __half*)residual,
+                               (const __half*)w, (__half*)y, (__half*)h_out, dim, eps);
   const size_t smem = (size_t)dim * 2;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(q40::rmsnorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
