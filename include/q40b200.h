@@ -384,6 +384,11 @@ int q40_rmsnorm(const void* x, const void* residual, const void* w, void* y, voi
 int q40_rope(void* x, const int32_t* pos, const void* cos_tbl, const void* sin_tbl, int rows,
              int n_heads, int D, int64_t row_stride, void* stream);
 
+/* q40_rope of queries [rows, q_heads, D] and keys [rows, k_heads, D] of the same positions; one launch where both meet
+ * the vector kernel's alignment (D % 16 == 0, strides % 8 == 0, 16-byte addresses). */
+int q40_rope_qk(void* q, int q_heads, int64_t q_stride, void* k, int k_heads, int64_t k_stride, const int32_t* pos,
+                const void* cos_tbl, const void* sin_tbl, int rows, int D, void* stream);
+
 /* y = fp16(fp16(silu(a)) * b), n elements.
  * Replaces: F.silu(w1(x)) * w3(x) in FeedForward.forward (hf_model_q40_kv_shared.py:434). */
 int q40_silu_mul(const void* a, const void* b, void* y, int64_t n, void* stream);

@@ -326,9 +326,8 @@ class Transformer(nn.Module):
             ck, cv = att.cache_prompt_k[:S], att.cache_prompt_v[:S]
             self._norm(h, pending, attn_norm, xn, st)
             self._mm(xn, qkv, [q, ck.view(S, Hkv * D), cv.view(S, Hkv * D)], args[0], err, st)
-            for x, heads in ((q, H), (ck, Hkv)):
-                check(lib.q40_rope(x.data_ptr(), pos.data_ptr(), self._cos.data_ptr(), self._sin.data_ptr(), S, heads, D,
-                                   heads * D, st), "q40_rope")
+            check(lib.q40_rope_qk(q.data_ptr(), H, H * D, ck.data_ptr(), Hkv, Hkv * D, pos.data_ptr(), self._cos.data_ptr(),
+                                  self._sin.data_ptr(), S, D, st), "q40_rope_qk")
             att.cache_prompt_len = S
             # causal attention over the prompt (grouped-query heads read their kv head directly)
             K.causal_attn(q.view(S, H, D), ck, cv, out=ao.view(S, H, D))

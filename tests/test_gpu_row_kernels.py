@@ -38,3 +38,20 @@ def test_rmsnorm_widths(K, dim, in_place):
         # fp32 sums in another order: a result on a rounding edge may fall to the other side, by one step of each rounding
         d = np.abs(got.cpu().numpy().view(np.int16).astype(np.int32) - want.view(np.int16).astype(np.int32))
         assert d.max() <= 2 and (d > 0).mean() < 0.01
+
+
+# one launch; unequal heads; a tensor that only the one-pair kernel takes
+@pytest.mark.parametrize("rows,Hq,Hk,D,pad_q,pad_k", [(1, 1, 1, 128, 0, 0), (77, 8, 2, 128, 0, 8), (33, 3, 5, 64, 16, 0), (5, 2, 2, 128, 0, 4),
+                                                      (9, 2, 1, 20, 0, 0)])
+def test_rope_of_queries_and_keys_has_the_bits_of_two_launches(K, rows, Hq, Hk, D, pad_q, pad_k):
+    from spec_mcts_b200._lib import check, lib
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    q, k = (torch.randn((rows, h * D + p), generator=g, device="cuda").half() for h, p in ((Hq, pad_q), (Hk, pad_k)))
+    cos, sin = (torch.randn((100, D // 2), generator=g, device="cuda").half() for _ in range(2))
+    pos = torch.randint(0, 100, (rows,), generator=g, device="cuda", dtype=torch.int32)
+    want = [x.clone() for x in (q, k)]
+    for x, h in zip(want, (Hq, Hk)):
+        K.rope_(x[:, :h * D].unflatten(1, (h, D)), pos, cos, sin)
+    check(lib.q40_rope_qk(q.data_ptr(), Hq, q.stride(0), k.data_ptr(), Hk, k.stride(0), pos.data_ptr(), cos.data_ptr(), sin.data_ptr(),
+                          rows, D, torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(q, want[0]) and torch.equal(k, want[1])
