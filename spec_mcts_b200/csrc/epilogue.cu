@@ -6,8 +6,8 @@
 namespace q40 {
 
 // The same sums in the same order as rmsnorm_kernel below, for rows of up to NV vectors of eight per thread: a row stays in
-// registers and all of it is requested at once, the weights ahead of the previous launch's end.  One trip to L2 instead
-// of one per vector.  4096 wide, what a pass waits for it: 10 rows 2.8 and 3.7 us before, 1.9 and 1.6 now; 512 rows 6.8 and 4.9.
+// registers and all of it is requested at once, with its weights: one trip to L2 instead of one per vector.  4096 wide, what
+// a pass waits for it: 10 rows 2.8 and 3.7 us before, 1.8 and 1.7 now; 512 rows 6.8 and 5.2.
 template <int NV>
 __global__ void __launch_bounds__(256)
 rmsnorm_reg_kernel(const __half* __restrict__ x, const __half* __restrict__ residual, const __half* __restrict__ w,
@@ -15,19 +15,19 @@ rmsnorm_reg_kernel(const __half* __restrict__ x, const __half* __restrict__ resi
   __shared__ float red[8];
   const int tid = threadIdx.x;
   uint4 wv[NV], v[NV], u[NV];
-#pragma unroll
-  for (int n = 0; n < NV; ++n) {
-    const int i = (n * 256 + tid) * 8;
-    wv[n] = i < dim ? __ldg(reinterpret_cast<const uint4*>(w + i)) : make_uint4(0, 0, 0, 0);
-  }
   asm volatile("griddepcontrol.launch_dependents;");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");     // the weights, too, may be the previous launch's
   const int64_t at = (int64_t)blockIdx.x * dim + tid * 8;
 #pragma unroll
   for (int n = 0; n < NV; ++n) {
     const bool in = (n * 256 + tid) * 8 < dim;
     v[n] = in ? *reinterpret_cast<const uint4*>(x + at + n * 2048) : make_uint4(0, 0, 0, 0);
     if (residual) u[n] = in ? *reinterpret_cast<const uint4*>(residual + at + n * 2048) : make_uint4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    const int i = (n * 256 + tid) * 8;
+    wv[n] = i < dim ? *reinterpret_cast<const uint4*>(w + i) : make_uint4(0, 0, 0, 0);
   }
   float ss = 0.f;
 #pragma unroll
