@@ -55,3 +55,29 @@ def test_rope_of_queries_and_keys_has_the_bits_of_two_launches(K, rows, Hq, Hk, 
     check(lib.q40_rope_qk(q.data_ptr(), Hq, q.stride(0), k.data_ptr(), Hk, k.stride(0), pos.data_ptr(), cos.data_ptr(), sin.data_ptr(),
                           rows, D, torch.cuda.current_stream().cuda_stream))
     assert torch.equal(q, want[0]) and torch.equal(k, want[1])
+
+
+
+# activations 16 and 8 bytes apart; rows at the edges of a tile of eight and of a launch; a k range that ends inside a piece
+@pytest.mark.parametrize("M,Kd,N", [(1, 128, 192), (7, 1152, 192), (9, 4096, 192), (16, 2176, 192), (33, 1152, 192),
+                                    (1, 2176, 11904), (9, 2176, 11904)])          # these: 768 k in a piece, 640 in the last
+def test_linear_on_rows_of_any_alignment(K, M, Kd, N):
+    from spec_mcts_b200._lib import check, lib
+    rng = np.random.default_rng(M + Kd)
+    q, s = O.quantize_q40((rng.standard_normal((N, Kd)) * 0.1).astype(np.float16), 64)
+    x = rng.standard_normal((M, Kd)).astype(np.float16)
+    want = O.linear_q40_nk(x, q, s, (N, Kd), 64).astype(np.float32)
+    qd, sd = torch.from_numpy(q).cuda(), torch.from_numpy(s).cuda()
+    ws = torch.zeros(lib.q40_gemm_workspace_bytes(M, N, Kd), dtype=torch.uint8, device="cuda")
+    bits = []
+    for first, pad in ((0, 0), (0, 4), (4, 8), (8, 8)):                  # halves before the first row and behind each
+        buf = torch.zeros(first + M * (Kd + pad), dtype=torch.float16, device="cuda")
+        view = buf[first:].view(M, Kd + pad)[:, :Kd]
+        view.copy_(torch.from_numpy(x))
+        y = torch.empty((M, N), dtype=torch.float16, device="cuda")
+        check(lib.q40_gemm_nk(view.data_ptr(), Kd + pad, qd.data_ptr(), sd.data_ptr(), y.data_ptr(), N, M, N, Kd, 64, ws.data_ptr(),
+                              ws.numel(), torch.cuda.current_stream().cuda_stream))
+        # fp16 result of fp32 sums: half a step, and a step more where the sums' order moves one across an edge
+        np.testing.assert_allclose(y.float().cpu().numpy(), want, rtol=2e-3, atol=2e-3)
+        bits.append(y)
+    assert all(torch.equal(b, bits[0]) for b in bits)
