@@ -356,7 +356,7 @@ __device__ __forceinline__ void nk_compute(float (&acc)[MT][4], const NkRegs& r,
 
 // MT: 8-row tiles of the batch per launch, up to 8 (see nk_launch_rows); the activations
 // are staged xch k rows at a time (a multiple of DEPTH steps, or the whole k range).
-template <int G, int MT>
+template <int G, int MT, bool BATCHES>
 __global__ void __launch_bounds__(GEMV_THREADS, MT <= 2 ? 5 : 3)
 gemv_nk_kernel(const __half* __restrict__ X, int64_t ldx, const uint8_t* __restrict__ wq,
                const __half* __restrict__ ws, __half* __restrict__ Y, int64_t ldy, int M, int N, int K,
@@ -389,13 +389,11 @@ gemv_nk_kernel(const __half* __restrict__ X, int64_t ldx, const uint8_t* __restr
     *reinterpret_cast<uint2*>(xs + at) = make_uint2(prmt(x01, x23, 0x5410), prmt(x01, x23, 0x7632));   // x0 x2 | x1 x3
   };
   // Nothing is multiplied before the activations are there: five 16-byte loads of a thread on their way at once, where rows
-  // are aligned to that (10 x 4096 x 11008, 1024 k of 16 rows per CTA in 8-byte loads, one after the other: 20.5 us; so: 17.3;
+  // are aligned to that (10 x 4096 x 11008, 1024 k of 16 rows per CTA in 8-byte loads, one after the other: 20.5 us; so: 18.1;
   // 10 x 4096 x 32000 50.9 and 42.1).  A short piece of few rows is as soon there by single loads, without the set-up of
   // batches and padding (384 k of one row 7.5 us, batches 7.8; 256 k of 10 rows 8.0 and 8.3, 384 k 11.6 and 10.7).
-  const bool batches = xch > (MT == 1 ? 512 : MT == 2 ? 256 : 0) &&
-                       ((reinterpret_cast<uintptr_t>(X) | ((uintptr_t)ldx * 2)) & 15) == 0;
   auto stage = [&](int k0) {
-    if (batches) {
+    if constexpr (BATCHES) {
       // piece i = (row m, k 8 j) of tid, tid + GEMV_THREADS, ...: the next one without a division
       const int per = xch / 8, dm = GEMV_THREADS / per, dj = GEMV_THREADS - dm * per;
       int m = tid / per, j = tid - m * per;
@@ -428,7 +426,7 @@ gemv_nk_kernel(const __half* __restrict__ X, int64_t ldx, const uint8_t* __restr
       }
     }
   };
-  if (batches)                                // rows of padding
+  if constexpr (BATCHES)                      // rows of padding
     for (int at = M * xs_ld + tid * 4; at < MT * 8 * xs_ld; at += GEMV_THREADS * 4) put(at, 0, 0);
 
   float acc[MT][4];
@@ -641,10 +639,11 @@ static int launch_gemv_nk(const __half* x, int64_t ldx, const uint8_t* wq, const
   constexpr auto smem_of = [](int x) { return ((size_t)MT * 8 * (x + q40::NK_XS_PAD) * 2 + 15) & ~(size_t)15; };
   const int xch = p.kchunk < XMAX ? p.kchunk : XMAX;
   const size_t smem = smem_of(xch);
-  auto kern = q40::gemv_nk_kernel<G, MT>;
+  const bool batches = xch > (MT == 1 ? 512 : MT == 2 ? 256 : 0) && q40_aligned(x, 16) && ldx % 8 == 0;
+  auto kern = batches ? q40::gemv_nk_kernel<G, MT, true> : q40::gemv_nk_kernel<G, MT, false>;
   if constexpr (smem_of(XMAX) > 48 * 1024) {
-    static std::atomic<uint64_t> ready;
-    const cudaError_t e = q40_allow_smem(ready, (const void*)kern, (int)smem_of(XMAX));
+    static std::atomic<uint64_t> ready[2];
+    const cudaError_t e = q40_allow_smem(ready[batches], (const void*)kern, (int)smem_of(XMAX));
     if (e != cudaSuccess) return (int)e;
   }
   dim3 grid(p.nblocks, p.nsplit);
