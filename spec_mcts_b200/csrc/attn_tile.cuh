@@ -90,7 +90,7 @@ struct WarpRows {
   }
 
   // One tile: S = Q K^T, online softmax, O += P V.  With MASK, key i of the tile counts for row g below n0 and for row g + 8
-  // below n1.  A row has seen a key by the end of its first tile.
+  // below n1.  A row all of whose scores so far are -inf keeps its sum and outputs at zero.
   template <bool MASK>
   __device__ __forceinline__ void step(uint32_t kt, uint32_t vt, float scale_log2, int n0, int n1, int lane) {
     const int t = lane & 3;
@@ -121,13 +121,14 @@ struct WarpRows {
         if (MASK && nt * 8 + 2 * t + (j & 1) >= ((j >> 1) ? n1 : n0)) s[nt][j] = -CUDART_INF_F;
         mx[j >> 1] = fmaxf(mx[j >> 1], s[nt][j]);
       }
-    float corr[2];
+    float corr[2], base[2];                          // base: the maximum, or 0 while that is -inf (-inf - -inf is no number)
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
       mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
       const float mnew = fmaxf(m[r], mx[r]);
-      corr[r] = ex2(m[r] - mnew);
+      base[r] = mnew == -CUDART_INF_F ? 0.f : mnew;
+      corr[r] = ex2(m[r] - base[r]);
       m[r] = mnew;
       l[r] *= corr[r];
     }
@@ -136,7 +137,7 @@ struct WarpRows {
     for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float p = ex2(s[nt][j] - m[j >> 1]);
+        const float p = ex2(s[nt][j] - base[j >> 1]);
         s[nt][j] = p;
         ls[j >> 1] += p;
       }

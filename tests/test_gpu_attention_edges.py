@@ -75,3 +75,18 @@ def test_causal_blocks(K, S):
     s = s.masked_fill(torch.ones((S, S), device="cuda", dtype=torch.bool).triu(1), float("-inf"))
     want = torch.einsum("hij,jhd->ihd", torch.softmax(s, -1), v.double().repeat_interleave(2, 1))
     np.testing.assert_allclose(K.causal_attn(q, k, v).float().cpu().numpy(), want.float().cpu().numpy(), **TOL)
+
+
+def test_causal_rows_whose_first_tile_of_scores_is_minus_infinity(K):
+    """Rows with a finite score later on attend to those keys alone; rows without one are zero."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    S, blocked = 193, 70                              # more than a tile of 64 keys
+    q, k, v = (torch.randn((S, h, 128), generator=g, device="cuda").half() for h in (4, 2, 2))
+    q[..., 0], k[:blocked, :, 0] = 1.0, float("-inf")
+    got = K.causal_attn(q, k, v)
+    s = torch.einsum("ihd,jhd->hij", q[blocked:].double(), k[blocked:].double().repeat_interleave(2, 1)) / 128 ** 0.5
+    n = S - blocked
+    s = s.masked_fill(torch.ones((n, n), device="cuda", dtype=torch.bool).triu(1), float("-inf"))
+    want = torch.einsum("hij,jhd->ihd", torch.softmax(s, -1), v[blocked:].double().repeat_interleave(2, 1))
+    np.testing.assert_allclose(got[blocked:].float().cpu().numpy(), want.float().cpu().numpy(), **TOL)
+    assert not got[:blocked].any()
