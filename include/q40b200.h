@@ -37,6 +37,9 @@ extern "C" {
 const char* q40_strerror(int status);
 /* Library/ABI version, bumped when a signature changes. */
 int q40_abi_version(void);
+/* The capture that `stream` takes part in, or 0: for hosts that keep scratch per stream, where what is made inside a
+ * capture is ready in that graph's replays only. */
+int q40_capture_id(void* stream, uint64_t* id);
 
 /* ---- Q4_0 pack / unpack ------------------------------------------------------------ */
 

@@ -35,6 +35,7 @@ lib = _load()
 SIGNATURES = {
     "q40_strerror": (c_char_p, [c_int]),
     "q40_abi_version": (c_int, []),
+    "q40_capture_id": (c_int, [c_void_p, c_void_p]),
     "q40_quantize": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_void_p]),
     "q40_quantize_rows": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int64,
                                   c_int, c_int, c_void_p]),

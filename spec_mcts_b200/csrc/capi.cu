@@ -17,6 +17,16 @@ extern "C" const char* q40_strerror(int status) {
   return "q40: unknown status";
 }
 
+extern "C" int q40_capture_id(void* stream, uint64_t* id) {
+  if (!id) return Q40_E_NULL;
+  cudaStreamCaptureStatus status;
+  unsigned long long of = 0;
+  const cudaError_t e = cudaStreamGetCaptureInfo((cudaStream_t)stream, &status, &of);
+  if (e != cudaSuccess) return (int)e;
+  *id = status == cudaStreamCaptureStatusNone ? 0 : of;
+  return Q40_OK;
+}
+
 #ifdef Q40_TRACE
 void* q40_trace_ptr = nullptr;
 extern "C" void q40_debug_trace(void* buf) { q40_trace_ptr = buf; }

@@ -8,6 +8,7 @@ There is no CPU path: a CPU tensor raises.
 """
 from __future__ import annotations
 
+import ctypes
 import math
 import weakref
 from typing import Optional, Sequence
@@ -61,18 +62,30 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 _workspaces: dict = {}
+_capture_workspaces: dict = {}      # the same keys -> (id of the stream's last capture, buffer made in it)
 
 
 def _workspace(kind: str, dev: torch.device, nbytes: int, zero: bool) -> torch.Tensor:
     """Per (kind, device, stream) scratch buffer, grown on demand.  Split-K GEMM scratch
     must start zeroed (the kernels restore that); calls on different streams get
-    different buffers so that they may overlap."""
+    different buffers so that they may overlap.  One that is made inside a capture serves that capture only: until the
+    graph runs it holds nothing, and each replay makes it ready again."""
     key = (kind, dev.index, _stream(dev))
     buf = _workspaces.get(key)
     if buf is None or buf.numel() < nbytes:
         n = max(int(nbytes), 1 << 20)
+        capture = None
+        if torch.cuda.is_current_stream_capturing():
+            capture = ctypes.c_uint64()
+            check(lib.q40_capture_id(key[2], ctypes.byref(capture)), "q40_capture_id")
+            made_in, buf = _capture_workspaces.get(key, (None, None))
+            if made_in == capture.value and buf.numel() >= nbytes:
+                return buf
         buf = (torch.zeros if zero else torch.empty)(n, dtype=torch.uint8, device=dev)
-        _workspaces[key] = buf
+        if capture is None:
+            _workspaces[key] = buf
+        else:
+            _capture_workspaces[key] = (capture.value, buf)
     return buf
 
 
@@ -327,8 +340,9 @@ def _tiled_copy_of(b_w, b_s, K, N, dev, st):
 def _tiled_matmul(dev, a, tiled, c, M, N, K, pdl, st) -> bool:
     """q40_matmul_tiled on a tiled copy; False if this device cannot schedule the clusters (up to 16 rows) or its
     driver has no tensor-map encoder (above)."""
-    # the error word of tc_error_flag(); the narrow kernel (up to 8 rows) has no wait that could expire
-    err = _workspace("gemm", dev, 4096, zero=True).data_ptr() + 4092 if M > 8 else None
+    # the narrow kernel (up to 8 rows) has no wait that could expire
+    page = _tc_error_page(dev, st) if M > 8 else None
+    err = page.data_ptr() + 4092 if M > 8 else None
     for cluster in (_cluster_sizes.get(dev.index) or (16, 8)):
         rc = lib.q40_matmul_tiled(tiled.data_ptr(), c.data_ptr(), c.stride(0), a.data_ptr(), a.stride(0), M, N, K, cluster,
                                   err, 1 if pdl else 0, st)
@@ -343,7 +357,6 @@ def _tiled_matmul(dev, a, tiled, c, M, N, K, pdl, st) -> bool:
 
 def _stream_gemv(dev, a, tiled, c, M, N, K) -> bool:
     """Mode 0 of q40_gemv_stream on a tiled copy; False if the launch was refused for this shape."""
-    import ctypes
     P = ctypes.c_void_p * 1
     nbytes = lib.q40_gemv_stream_workspace_bytes(M, N, K)
     if nbytes == 0:
@@ -361,7 +374,6 @@ def _cluster_gemv(dev, a, b_w, b_s, c, M, N, K) -> bool:
     """Up to 16 rows: the decode step's cluster-reduced kernel in its plain form (mode 0 of
     q40_gemv_fused: no scratch, split-K summed through distributed shared memory), 2-4x faster than
     the workspace kernel behind q40_gemm_kn.  False if the launch was refused for this shape."""
-    import ctypes
     P = ctypes.c_void_p * 1
     for cluster in (_cluster_sizes.get(dev.index) or (16, 8)):
         rc = lib.q40_gemv_fused(0, 1, P(b_w.data_ptr()), P(b_s.data_ptr()), P(c.data_ptr()), (ctypes.c_int * 1)(N),
@@ -406,9 +418,25 @@ def _tc_error_word(dev) -> torch.Tensor:
     return _workspace("gemm", dev, 4096, zero=True)[4092:4096].view(torch.int32)
 
 
+def _tc_error_word_lasts(dev) -> bool:
+    """Whether that word is there outside of a capture as well."""
+    return ("gemm", dev.index, _stream(dev)) in _workspaces
+
+
+def _tc_error_page(dev, st) -> torch.Tensor:
+    """The 4096 bytes that end with that word, or under a capture on a stream that has none yet, bytes that nobody reads."""
+    page = _workspaces.get(("gemm", dev.index, st))
+    if page is None:
+        if torch.cuda.is_current_stream_capturing():
+            return torch.empty(4096, dtype=torch.uint8, device=dev)
+        page = _workspace("gemm", dev, 4096, zero=True)
+    return page
+
+
 def tc_error_flag(dev=None) -> int:
     """1 if a tensor-core matmul launched through matmul_q40 or a prompt pass on the current stream of `dev` gave up
-    on one of its bounded waits since the workspace was created (synchronises the device)."""
+    on one of its bounded waits since the workspace was created (synchronises the device).  Not reported: matmuls
+    captured on a stream on which no call that needs a workspace was made outside of a capture before."""
     dev = _indexed(dev)
     buf = _workspaces.get(("gemm", dev.index, _stream(dev)))
     if buf is None:
@@ -460,7 +488,6 @@ def gemv_fused(mode: int, a: torch.Tensor, weights, *, norm_w=None, ss_in=None, 
     `weights` is a list of 1-3 (b_w, b_s, (K, N)) triples sharing the activations a [M <= 16, K].
     mode 0: [a @ deq(B_i)]; 1: RMSNorm(a; norm_w, ss_in) first; 2: returns (h_in + a @ deq(B),
     ss_out [M, count]); 3: silu(RMSNorm(a) @ deq(B_0)) * (RMSNorm(a) @ deq(B_1))."""
-    import ctypes
     dev = _need_cuda(a, norm_w, ss_in, h_in, *[w[0] for w in weights], *[w[1] for w in weights if w[1] is not None])
     M, K = a.shape
     n = len(weights)
@@ -521,7 +548,6 @@ def gemm_tiled_tc(a: torch.Tensor, weights, use_pdl: bool = False, err: Optional
     cores (q40_gemm_tiled_tc_multi in include/q40b200.h); the outputs are column slices of one buffer.
     Raises if a bounded wait inside the kernel expired — unless the caller passes its own int32 device word
     `err` (zeroed by the caller), which the kernel sets instead and the caller reads when it synchronises."""
-    import ctypes
     dev = _need_cuda(a, *[w[0] for w in weights])
     M, K = a.shape
     n = len(weights)
@@ -552,7 +578,6 @@ def gemv_stream(mode: int, a: torch.Tensor, weights, *, norm_w=None, ss_in=None,
     `weights` is a list of 1-3 (tiled copy, (K, N)) pairs sharing the activations a [M <= 16, K];
     same modes and return values as gemv_fused.  Also returns nothing else: the kernel's status word
     is the first int of `workspace` (a zero-filled uint8 tensor of q40_gemv_stream_workspace_bytes)."""
-    import ctypes
     dev = _need_cuda(a, norm_w, ss_in, h_in, *[w[0] for w in weights])
     M, K = a.shape
     n = len(weights)

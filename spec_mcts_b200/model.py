@@ -239,6 +239,7 @@ class Transformer(nn.Module):
         # device word that the last prompt pass's tensor-core launches set on a wait expiry (the one of
         # kernels.tc_error_flag), its copy of the last finished pass, and whether nothing has waited for it yet
         self._tc_err = None
+        self._tc_err_own = torch.zeros(1, dtype=torch.int32, device=dev)      # ... in place of a captured pass's own word
         self._tc_err_host = torch.zeros(1, dtype=torch.int32).pin_memory()
         self._prompt_unchecked = False
         # ... True: through the byte-balanced stream-K launch (one CTA per SM, bulk-copy ring, no clusters);
@@ -346,6 +347,10 @@ class Transformer(nn.Module):
         self._tc_err = K._tc_error_word(h.device)
         if self._tc_err.data_ptr() != err.data_ptr():     # a larger workspace took the first one's place meanwhile
             self._tc_err |= err
+        if capturing and not K._tc_error_word_lasts(h.device):
+            # the word is the capture's, and holds nothing until the graph runs
+            self._tc_err_own |= self._tc_err
+            self._tc_err = self._tc_err_own
         self._tc_err_host.copy_(self._tc_err, non_blocking=True)
         self._prompt_unchecked = S > 16        # narrower passes run no kernel that waits
         if self.prefill_last_only:
@@ -368,6 +373,7 @@ class Transformer(nn.Module):
     @torch.inference_mode()
     def _prompt_failed(self):
         self._tc_err.zero_()
+        self._tc_err_own.zero_()
         K._reset_tiled_tc_workspaces(self.device)
         torch.cuda.synchronize(self.device)      # copies of passes in flight have landed
         self._tc_err_host.zero_()

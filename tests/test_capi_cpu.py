@@ -208,6 +208,46 @@ def test_a_matmul_on_another_stream_waits_for_the_copy(launches, monkeypatch):
     assert log == [(2, "waits", "copied"), (2, "holds"), (3, "waits", "copied"), (3, "holds")]
 
 
+def test_scratch_made_in_a_capture_is_not_kept(launches, monkeypatch):
+    """It holds nothing until that graph runs: launches of one capture share it, and neither another capture on the stream
+    nor a call after the capture finds it.  Scratch that was there before serves captures too."""
+    import torch
+    K, _ = launches
+    capture = [0]
+
+    def capture_id(st, out):
+        out._obj.value = capture[0]
+        return 0
+
+    monkeypatch.setattr(K.lib, "q40_capture_id", capture_id, raising=False)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capture[0] != 0)
+    monkeypatch.setattr(K, "_capture_workspaces", {}, raising=False)
+    cpu, stream = torch.device("cpu"), [1]
+    monkeypatch.setattr(K, "_stream", lambda dev: stream[0])
+    get = lambda n=4096: K._workspace("gemm", cpu, n, zero=True)
+    # a matmul of 9 to 16 rows (or more) passes an error word of that scratch
+    Kd, N = 64, 256
+    w, s = torch.zeros((Kd * N // 128, 64), dtype=torch.int8), torch.zeros(Kd * N // 64, dtype=torch.float16)
+    for rows in (10, 20):
+        K.matmul_q40(torch.zeros((rows, Kd), dtype=torch.float16), w, s, (Kd, N))
+    kept = get()
+    stream[0], capture[0] = 2, 7
+    for rows in (10, 20):
+        K.matmul_q40(torch.zeros((rows, Kd), dtype=torch.float16), w, s, (Kd, N))
+    first, large = get(), get(3 << 20)
+    assert get() is large and large is not first
+    capture[0] = 8
+    second = get()
+    assert second is not large and second is not first and not second.any()
+    capture[0] = 0
+    after = get()
+    assert all(after is not b for b in (first, large, second)) and get() is after
+    capture[0] = 9
+    assert get() is after
+    stream[0] = 1
+    assert get() is kept
+
+
 @pytest.mark.parametrize("dev", [None, "cuda", "cuda:1"])
 def test_status_calls_take_a_device_without_an_index(monkeypatch, dev):
     """torch.device("cuda") is the current device."""

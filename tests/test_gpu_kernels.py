@@ -723,6 +723,29 @@ def test_matmul_whose_weight_is_first_seen_in_a_capture(K, M):
         assert_close(host(y), ref.cpu().numpy())
 
 
+@pytest.mark.parametrize("M", [10, 40])
+def test_graphs_captured_on_one_fresh_stream_run_in_any_order(K, M):
+    """The second graph's split-K scratch is ready without the first one's replay, and calls outside of them have their own."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    Kd, N = 4096, 1024
+    a, x = (torch.randn((m, Kd), generator=g, device="cuda").half() for m in (M, 3))
+    q, s = K.quantize_q40((torch.randn((Kd, N), generator=g, device="cuda") * 0.05).half())
+    wq, ws = K.quantize_q40((torch.randn((N, Kd), generator=g, device="cuda") * 0.05).half())
+    want = K.matmul_q40(a, q, s, (Kd, N)), K.linear_q40(x, wq, ws, (N, Kd))
+    side, graphs, outs = torch.cuda.Stream(), [torch.cuda.CUDAGraph() for _ in range(2)], []
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        with torch.cuda.graph(graphs[0], stream=side):
+            outs.append(K.matmul_q40(a, q, s, (Kd, N)))
+        with torch.cuda.graph(graphs[1], stream=side):
+            outs.append(K.linear_q40(x, wq, ws, (N, Kd)))
+        for _ in range(2):
+            for i in (1, 0):
+                graphs[i].replay()
+                assert torch.equal(K.linear_q40(x, wq, ws, (N, Kd)), want[1])
+                assert torch.equal(outs[i], want[i])
+
+
 @pytest.mark.parametrize("page_size,idx", [(1, torch.int16), (16, torch.int32)])
 @pytest.mark.parametrize("B,H", [(3, 8), (10, 32), (30, 32), (80, 32)])      # each split of the warps over a row
 def test_page_table_shorter_than_the_longest_suffix_allowed(K, page_size, idx, B, H):

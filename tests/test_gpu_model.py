@@ -436,6 +436,34 @@ def test_prompt_pass_first_seen_in_a_capture():
     assert torch.equal(out, checkpoint)
 
 
+def test_prompt_pass_captured_on_a_fresh_stream():
+    """No workspace was made on the stream before, and the copies are there (the short prompt shares tiles through scratch):
+    steps before the replay find no error word of it, and the replay gives the pass's results, once and again."""
+    prompt, tok = torch.arange(40, device="cuda").view(1, -1), torch.zeros((1, 1), dtype=torch.int64, device="cuda")
+    m = small_random()
+    want = m(prompt, 0).clone(), m(tok, 40).clone()
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        with torch.cuda.graph(graph, stream=side):
+            out = m(prompt, 0)
+    torch.cuda.current_stream().wait_stream(side)
+    assert m.prompt_status() == 0 and torch.equal(m(tok, 40), want[1])
+    for _ in range(2):
+        m._caches["pk"].zero_()
+        graph.replay()
+        assert torch.equal(out, want[0]) and torch.equal(m(tok, 40), want[1])
+    # its word, set as a kernel whose wait ran out leaves it, is reported until the pass is known to have failed
+    from spec_mcts_b200 import kernels as KK
+    with torch.inference_mode():
+        m._tc_err.fill_(1)
+    m._prompt_unchecked = True
+    with pytest.raises(KK.Q40Error):
+        m(tok, 40)
+    graph.replay()
+    assert m.prompt_status() == 0 and torch.equal(m(tok, 40), want[1])
+
+
 @pytest.mark.parametrize("S", [8, 40])
 @pytest.mark.parametrize("broken", ["norm on the host", "last norm on the host", "scales too few", "codes too few",
                                     "scales in fp32", "shape turned round", "too narrow"])
