@@ -62,6 +62,8 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 _workspaces: dict = {}
+_in_graphs: set = set()             # keys of those whose address a graph has
+_outgrown: list = []                # ... when a larger one had taken their place
 _capture_workspaces: dict = {}      # the same keys -> (id of the stream's last capture, buffer made in it)
 
 
@@ -69,10 +71,14 @@ def _workspace(kind: str, dev: torch.device, nbytes: int, zero: bool) -> torch.T
     """Per (kind, device, stream) scratch buffer, grown on demand.  Split-K GEMM scratch
     must start zeroed (the kernels restore that); calls on different streams get
     different buffers so that they may overlap.  One that is made inside a capture serves that capture only: until the
-    graph runs it holds nothing, and each replay makes it ready again."""
+    graph runs it holds nothing, and each replay makes it ready again.  One that a graph has the address of is not given
+    back; the next is at least twice its size, so that all of these take no more than the last."""
     key = (kind, dev.index, _stream(dev))
     buf = _workspaces.get(key)
-    if buf is None or buf.numel() < nbytes:
+    if buf is not None and buf.numel() >= nbytes:
+        if torch.cuda.is_current_stream_capturing():
+            _in_graphs.add(key)
+    else:
         n = max(int(nbytes), 1 << 20)
         capture = None
         if torch.cuda.is_current_stream_capturing():
@@ -81,6 +87,10 @@ def _workspace(kind: str, dev: torch.device, nbytes: int, zero: bool) -> torch.T
             made_in, buf = _capture_workspaces.get(key, (None, None))
             if made_in == capture.value and buf.numel() >= nbytes:
                 return buf
+        elif key in _in_graphs:
+            _in_graphs.discard(key)
+            _outgrown.append(buf)
+            n = max(n, 2 * buf.numel())
         buf = (torch.zeros if zero else torch.empty)(n, dtype=torch.uint8, device=dev)
         if capture is None:
             _workspaces[key] = buf
@@ -425,12 +435,9 @@ def _tc_error_word_lasts(dev) -> bool:
 
 def _tc_error_page(dev, st) -> torch.Tensor:
     """The 4096 bytes that end with that word, or under a capture on a stream that has none yet, bytes that nobody reads."""
-    page = _workspaces.get(("gemm", dev.index, st))
-    if page is None:
-        if torch.cuda.is_current_stream_capturing():
-            return torch.empty(4096, dtype=torch.uint8, device=dev)
-        page = _workspace("gemm", dev, 4096, zero=True)
-    return page
+    if torch.cuda.is_current_stream_capturing() and ("gemm", dev.index, st) not in _workspaces:
+        return torch.empty(4096, dtype=torch.uint8, device=dev)
+    return _workspace("gemm", dev, 4096, zero=True)
 
 
 def tc_error_flag(dev=None) -> int:

@@ -248,6 +248,28 @@ def test_scratch_made_in_a_capture_is_not_kept(launches, monkeypatch):
     assert get() is kept
 
 
+def test_scratch_whose_address_a_graph_has_is_not_given_back(launches, monkeypatch):
+    import torch
+    import weakref
+    K, _ = launches
+    capturing = [False]
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing[0])
+    for name, empty in (("_in_graphs", set()), ("_outgrown", [])):
+        monkeypatch.setattr(K, name, empty, raising=False)
+    get = lambda n: K._workspace("gemm", torch.device("cpu"), n, zero=True)
+    plain = weakref.ref(get(4096))
+    in_graph = weakref.ref(get(2 << 20))
+    assert plain() is None
+    capturing[0] = True
+    assert get(4096) is in_graph()
+    capturing[0] = False
+    assert get(3 << 20) is not in_graph() and in_graph() is not None
+    last = weakref.ref(get(4096))
+    assert last().numel() >= 4 << 20
+    get(8 << 20)
+    assert last() is None and in_graph() is not None
+
+
 @pytest.mark.parametrize("dev", [None, "cuda", "cuda:1"])
 def test_status_calls_take_a_device_without_an_index(monkeypatch, dev):
     """torch.device("cuda") is the current device."""
