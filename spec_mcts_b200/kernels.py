@@ -349,7 +349,7 @@ def _tiled_copy_of(b_w, b_s, K, N, dev, st):
 
 def _tiled_matmul(dev, a, tiled, c, M, N, K, pdl, st) -> bool:
     """q40_matmul_tiled on a tiled copy; False if this device cannot schedule the clusters (up to 16 rows) or its
-    driver has no tensor-map encoder (above)."""
+    driver has no tensor-map encoder (above).  Only up to 8 rows is a launch sure to have used the cluster size."""
     # the narrow kernel (up to 8 rows) has no wait that could expire
     page = _tc_error_page(dev, st) if M > 8 else None
     err = page.data_ptr() + 4092 if M > 8 else None
@@ -357,7 +357,7 @@ def _tiled_matmul(dev, a, tiled, c, M, N, K, pdl, st) -> bool:
         rc = lib.q40_matmul_tiled(tiled.data_ptr(), c.data_ptr(), c.stride(0), a.data_ptr(), a.stride(0), M, N, K, cluster,
                                   err, 1 if pdl else 0, st)
         if rc == 0:
-            if M <= 16:
+            if M <= 8:
                 _cluster_sizes[dev.index] = (cluster,)
             return True
         if rc > 0 or (M > 16 and rc != -5):      # -5: Q40_E_UNSUPPORTED

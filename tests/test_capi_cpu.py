@@ -208,6 +208,27 @@ def test_a_matmul_on_another_stream_waits_for_the_copy(launches, monkeypatch):
     assert log == [(2, "waits", "copied"), (2, "holds"), (3, "waits", "copied"), (3, "holds")]
 
 
+def test_rows_that_need_no_cluster_do_not_choose_its_size(launches, monkeypatch):
+    """On a device that schedules clusters of 8 and not of 16: 9 to 16 rows run on a kernel without them, and what they are
+    given must not be taken for what the device can do."""
+    import torch
+    K, _ = launches
+    ran = []
+
+    def matmul_tiled(bw, c, ldc, a, lda, M, N, Kd, cluster, err, pdl, stream):
+        if M <= 8 and cluster == 16:
+            return -5
+        ran.append((M, cluster))
+        return 0
+
+    monkeypatch.setattr(K.lib, "q40_matmul_tiled", matmul_tiled)
+    Kd, N = 64, 256
+    w, s = torch.zeros((Kd * N // 128, 64), dtype=torch.int8), torch.zeros(Kd * N // 64, dtype=torch.float16)
+    for rows in (10, 1, 16, 8):
+        K.matmul_q40(torch.zeros((rows, Kd), dtype=torch.float16), w, s, (Kd, N))
+    assert [M for M, _ in ran] == [10, 1, 16, 8] and ran[1][1] == ran[3][1] == 8
+
+
 def test_scratch_made_in_a_capture_is_not_kept(launches, monkeypatch):
     """It holds nothing until that graph runs: launches of one capture share it, and neither another capture on the stream
     nor a call after the capture finds it.  Scratch that was there before serves captures too."""
