@@ -412,10 +412,14 @@ def _tiled_tc_workspace(dev, M: int) -> Optional[torch.Tensor]:
 
 
 def _reset_tiled_tc_workspaces(dev) -> None:
-    """After an expired wait: the launches in flight may have left their scratch in any state."""
+    """After an expired wait: the launches in flight may have left their scratch in any state.  Waits for the device, so
+    that no launch, of whatever stream, is using its scratch meanwhile or finds it as it was."""
+    dev = _indexed(dev)
+    torch.cuda.synchronize(dev)
     for (kind, index, _), buf in list(_workspaces.items()):
         if kind == "tiled_tc" and index == dev.index:
             buf.zero_()
+    torch.cuda.synchronize(dev)
 
 
 def _indexed(dev) -> torch.device:

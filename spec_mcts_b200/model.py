@@ -372,9 +372,9 @@ class Transformer(nn.Module):
 
     @torch.inference_mode()
     def _prompt_failed(self):
+        K._reset_tiled_tc_workspaces(self.device)
         self._tc_err.zero_()
         self._tc_err_own.zero_()
-        K._reset_tiled_tc_workspaces(self.device)
         torch.cuda.synchronize(self.device)      # copies of passes in flight have landed
         self._tc_err_host.zero_()
         self._prompt_unchecked = False

@@ -229,6 +229,20 @@ def test_rows_that_need_no_cluster_do_not_choose_its_size(launches, monkeypatch)
     assert [M for M, _ in ran] == [10, 1, 16, 8] and ran[1][1] == ran[3][1] == 8
 
 
+@pytest.mark.parametrize("dev", ["cuda", "cuda:1"])
+def test_scratch_of_an_expired_wait_is_reset_on_an_idle_device(monkeypatch, dev):
+    """Of every stream of that device, named with an index or without one, and only while nothing uses it."""
+    import torch
+    from spec_mcts_b200 import kernels as K
+    here, there = (torch.ones(64, dtype=torch.uint8) for _ in range(2))
+    monkeypatch.setattr(K, "_workspaces", {("tiled_tc", 1, 7): here, ("tiled_tc", 0, 7): there})
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 1)
+    waits = []
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda d=None: waits.append((torch.device(d).index, bool(here.any()))))
+    K._reset_tiled_tc_workspaces(torch.device(dev))
+    assert not here.any() and there.all() and waits == [(1, True), (1, False)]
+
+
 def test_scratch_made_in_a_capture_is_not_kept(launches, monkeypatch):
     """It holds nothing until that graph runs: launches of one capture share it, and neither another capture on the stream
     nor a call after the capture finds it.  Scratch that was there before serves captures too."""
