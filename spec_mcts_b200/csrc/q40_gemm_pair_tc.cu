@@ -34,8 +34,8 @@
 // sums met through the other CTA's shared memory), 77 rows 21.9 (23.0), 100 rows 25.0 (27.7), 512 rows 72 (76); expf and the
 // division are half of what it costs (100 rows: 22.6 with approximate ones).
 //
-// Every wait is bounded: on expiry an error word is set, the remaining work skipped, copies and MMAs in flight
-// waited for, tensor memory freed.
+// Every wait is bounded (by seconds): on expiry an error word is set and no more copies are requested; what is still
+// multiplied and stored is undefined, as is the scratch.  Copies and MMAs in flight are waited for, tensor memory is freed.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -65,6 +65,7 @@ constexpr int TMEM_COLS = 512;
 constexpr int CUT = 2;                          // a k range is cut at multiples of so many blocks
 constexpr int GROUPS = 1 + DSETS;               // of four warps, one per tensor-memory quadrant, that finish a pair's last tile
 constexpr int BAR_BYTES = 16 * S_MAX + 8 * NA_MAX + 64;
+constexpr uint32_t FLAG_POLLS = 1u << 22;       // of one flag, before giving up: seconds, like the other waits
 constexpr int OUT_LD = FEATS + 8;              // halves between rows that wait in shared memory
 constexpr int MAX_PAIRS = 128;
 constexpr int FLAG_BYTES = MAX_PAIRS * 64;      // at the start of the scratch, per pair: [half][quadrant] arrivals, then departures
@@ -482,10 +483,12 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
           for (int q = q0; q < me; ++q) {
             const int* flag = p.flags + q * 16 + half * 4 + quad;
             int arrived;
+            uint32_t polls = FLAG_POLLS;
             do {
               asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(arrived) : "l"(flag) : "memory");
-              if (arrived < GROUPS) { __nanosleep(64); limit = limit ? limit - 1 : 0; }
-            } while (arrived < GROUPS && limit);
+              if (arrived < GROUPS) { __nanosleep(64); --polls; }
+            } while (arrived < GROUPS && polls && limit);
+            if (arrived < GROUPS) limit = 0;
           }
           if (ch0 < nchunk) {                                // while the last MMAs run
 #pragma unroll
