@@ -207,6 +207,7 @@ class Transformer(nn.Module):
         self._tok_dev = torch.zeros(p.max_batch_size, dtype=torch.int64, device=dev)
         self._graphs = {}
         self._bufs = {}
+        self._tc_ws = None          # see _step_tc_ws
         self.use_cuda_graph = True
         # when set, a decode step also writes argmax(logits) back as the next input token and
         # advances the positions on the device, so steps can be replayed without the host
@@ -425,7 +426,7 @@ class Transformer(nn.Module):
 
     def _mm_silu(self, x, tiled, g, args, err, st, ws=None, pdl=None):
         """g = silu(x @ deq(W_1)) * (x @ deq(W_3)) for the tiled copies of the two: one launch, with the scratch `ws` (of
-        this stream, if none is given)."""
+        this stream or capture, if none is given)."""
         _, P, widths64, widths = args
         if ws is None:
             ws = K._tiled_tc_workspace(x.device, x.shape[0])
@@ -449,12 +450,24 @@ class Transformer(nn.Module):
                      ao=e(B, H * D), o=e(B, p.dim), a1=e(B, hid), a3=e(B, hid), g=e(B, hid), f=e(B, p.dim),
                      attn_ws=torch.empty(nb_attn, dtype=torch.uint8, device=dev),
                      gemm_ws=torch.zeros(nb_gemm, dtype=torch.uint8, device=dev),
-                     tc_ws=torch.zeros(lib.q40_gemm_tiled_tc_ws_bytes(B) if B > 8 else 0, dtype=torch.uint8, device=dev),
                      logits=e(B, p.vocab_size), qkv=e(B, (H + 2 * Hkv) * D),
                      ss_attn=torch.zeros((B, 1024), dtype=torch.float32, device=dev),
                      ss_ffn=torch.zeros((B, 1024), dtype=torch.float32, device=dev))
             self._bufs[B] = b
         return b
+
+    def _step_tc_ws(self, B):
+        """Scratch of q40_gemm_tiled_tc_ws for a step of B branches, or None where it uses none: one for all widths, whose
+        steps run one after the other."""
+        if lib.q40_gemm_tiled_tc_ws_bytes(B) == 0:
+            return None
+        if self._tc_ws is None:
+            if torch.cuda.is_current_stream_capturing():
+                return None                       # not ready outside of that graph
+            nbytes = lib.q40_gemm_tiled_tc_ws_bytes(min(self.params.max_batch_size, 128))
+            self._tc_ws = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+            self._tc_ws[:K._TILED_TC_FLAGS].zero_()
+        return self._tc_ws
 
     def _gemm(self, bufs, x, lin: LinearQ4_0, out, st):
         Kd, N = lin.kn()
@@ -832,7 +845,7 @@ class Transformer(nn.Module):
             if self._silu_pair(B, ff):
                 tiled, pdl = self._tiled_of((ff.w1, ff.w3))
                 self._mm_silu(xn, tiled, bufs["g"], self._mm_args([l.kn()[1] for l in (ff.w1, ff.w3)]),
-                              bufs["gemm_ws"].data_ptr() + 4096 - 4, st, bufs["tc_ws"] if bufs["tc_ws"].numel() else None, pdl)
+                              bufs["gemm_ws"].data_ptr() + 4096 - 4, st, self._step_tc_ws(B), pdl)
             else:
                 self._gemm_multi(bufs, xn, [ff.w1, ff.w3], [bufs["a1"], bufs["a3"]], st)
                 check(lib.q40_silu_mul(bufs["a1"].data_ptr(), bufs["a3"].data_ptr(), bufs["g"].data_ptr(),

@@ -464,6 +464,21 @@ def test_prompt_pass_captured_on_a_fresh_stream():
     assert m.prompt_status() == 0 and torch.equal(m(tok, 40), want[1])
 
 
+def test_widths_share_the_scratch_of_shared_tiles():
+    """A further width allocates its activations and no scratch of its own, and widths in turn give the same logits again."""
+    from spec_mcts_b200._lib import lib
+    m = small_random()
+    m.use_cuda_graph = False
+    m(torch.arange(40, device="cuda").view(1, -1), 0)
+    m.fork(0, 1, 15)
+    step = lambda b: m(torch.arange(b, device="cuda").view(-1, 1), 40).clone()
+    first = step(9)
+    before = torch.cuda.memory_allocated()
+    wide = step(16)
+    assert torch.cuda.memory_allocated() - before < lib.q40_gemm_tiled_tc_ws_bytes(16)
+    assert torch.equal(step(9), first) and torch.equal(step(16), wide)
+
+
 @pytest.mark.parametrize("S", [8, 40])
 @pytest.mark.parametrize("broken", ["norm on the host", "last norm on the host", "scales too few", "codes too few",
                                     "scales in fp32", "shape turned round", "too narrow"])
