@@ -243,6 +243,9 @@ class Transformer(nn.Module):
         self._tc_err_own = torch.zeros(1, dtype=torch.int32, device=dev)      # ... in place of a captured pass's own word
         self._tc_err_host = torch.zeros(1, dtype=torch.int32).pin_memory()
         self._prompt_unchecked = False
+        # per width, the error word (in gemm_ws) that the width's last finished step left
+        self._step_err_host = torch.zeros(p.max_batch_size + 1, dtype=torch.int32).pin_memory()
+        self._step_errs = self._step_err_host.numpy()
         # ... True: through the byte-balanced stream-K launch (one CTA per SM, bulk-copy ring, no clusters);
         # False: the cluster-reduced launch on the same tiled copies (faster on B200, the default)
         self.use_stream = False
@@ -455,6 +458,34 @@ class Transformer(nn.Module):
                      ss_ffn=torch.zeros((B, 1024), dtype=torch.float32, device=dev))
             self._bufs[B] = b
         return b
+
+    @staticmethod
+    def _step_err(bufs):
+        """The device word that a step's tensor-core matmuls set on a wait expiry (q40_gemm_kn's own, in its scratch)."""
+        return bufs["gemm_ws"][4092:4096].view(torch.int32)
+
+    def _check_steps(self):
+        """Raise if a bounded wait inside a matmul of an earlier step expired, as far as the host has heard: without waiting
+        for steps in flight."""
+        if self._step_errs.any() and not torch.cuda.is_current_stream_capturing():
+            self._steps_failed()
+
+    @torch.inference_mode()
+    def _steps_failed(self):
+        torch.cuda.synchronize(self.device)
+        for bufs in self._bufs.values():
+            bufs["gemm_ws"].zero_()
+        if self._tc_ws is not None:
+            self._tc_ws[:K._TILED_TC_FLAGS].zero_()
+        torch.cuda.synchronize(self.device)
+        self._step_errs.fill(0)
+        raise K.Q40Error("decode step: a bounded wait inside a tensor-core matmul expired")
+
+    def decode_status(self) -> int:
+        """Non-zero if a bounded wait inside a tensor-core matmul of a decode step expired, which makes its logits and cache
+        rows undefined (synchronises).  The first step after the word has reached the host raises."""
+        torch.cuda.synchronize(self.device)
+        return int(self._step_errs.any())
 
     def _step_tc_ws(self, B):
         """Scratch of q40_gemm_tiled_tc_ws for a step of B branches, or None where it uses none: one for all widths, whose
@@ -862,6 +893,8 @@ class Transformer(nn.Module):
         if not normed:
             self._norm(h, pending, self.norm.weight, xn, st)
         torch.matmul(xn, self.output.weight.t(), out=bufs["logits"])
+        if B > 8:                      # narrower matmuls have no wait that could expire
+            self._step_err_host[B:B + 1].copy_(self._step_err(bufs), non_blocking=True)
         if self.greedy_feedback:
             self._tok_dev[:B].copy_(bufs["logits"].argmax(dim=-1))
             self._pos_dev[:B] += 1
@@ -919,6 +952,7 @@ class Transformer(nn.Module):
         """Run one decode step for B branches with the tokens/positions already in the device
         buffers (`_tok_dev`, `_pos_dev`); returns the static logits buffer [B, vocab]."""
         self._check_prompt()
+        self._check_steps()
         fused = self._fused_body(B)
         per_layer = (5 if self._fused_attn_for(B) else 7) if fused else (9 if self._silu_pair(B, self.layers[0].feed_forward) else 10)
         self.launches_per_step = self.params.n_layers * per_layer + (2 if fused else 1)

@@ -89,6 +89,8 @@ class mcts:
             torch.cuda.current_stream(dev).synchronize()
             if t == 0 and hasattr(model, "_check_prompt"):
                 model._check_prompt()
+            if hasattr(model, "_check_steps"):
+                model._check_steps()
             new_curr, n_forks, stop = int(ctl_host[0]), int(ctl_host[1]), int(ctl_host[3])
             if n_forks and (self.record_forks or not hasattr(model, "_caches")):
                 src = fork_src[curr:new_curr].tolist()

@@ -479,6 +479,31 @@ def test_widths_share_the_scratch_of_shared_tiles():
     assert torch.equal(step(9), first) and torch.equal(step(16), wide)
 
 
+@pytest.mark.parametrize("use_graph", [True, False])
+@pytest.mark.parametrize("width", [9, 24])
+def test_expired_wait_of_a_step_is_reported(width, use_graph):
+    """The error word set by hand, and the scratch left as by a pair that arrived late: the status says so, the next step, of
+    whatever width, raises, and steps after that start from clean scratch."""
+    from spec_mcts_b200 import kernels as KK
+    m = small_random()
+    m.use_cuda_graph = use_graph
+    m(torch.arange(40, device="cuda").view(1, -1), 0)
+    m.fork(0, 1, 23)
+    step = lambda b: m(torch.arange(b, device="cuda").view(-1, 1), 40).clone()
+    want = step(width), step(1)
+    for after in (width, 1):
+        assert m.decode_status() == 0
+        with torch.inference_mode():
+            m._step_err(m._bufs[width]).fill_(1)
+            m._tc_ws[:8192].fill_(5)
+        step(width)
+        assert m.decode_status() != 0
+        with pytest.raises(KK.Q40Error):
+            step(after)
+        assert m.decode_status() == 0 and not m._tc_ws[:8192].any()
+        assert torch.equal(step(width), want[0]) and torch.equal(step(1), want[1])
+
+
 @pytest.mark.parametrize("S", [8, 40])
 @pytest.mark.parametrize("broken", ["norm on the host", "last norm on the host", "scales too few", "codes too few",
                                     "scales in fp32", "shape turned round", "too narrow"])
