@@ -563,11 +563,14 @@ class Transformer(nn.Module):
                                        1 if self.use_pdl else 0, st),
               "q40_gemm_kn_tc_multi")
 
+    def _narrow(self, B):
+        return self.use_fused and B <= 16 and self.tp_world == 1
+
     def _fused_body(self, B):
         """Whether a step of B branches takes the narrow matmuls with their fused neighbours.  From 9 branches on the
         tensor-core matmuls make up for two norm launches a layer (10 branches: 2.75 ms a step with the narrow ones), where the
         shapes and switches allow them."""
-        if not self.use_fused or B > 16 or self.tp_world > 1:
+        if not self._narrow(B):
             return False
         if B <= 8 or self.use_stream or self._lm_head_q4 is not None or not (self.use_tiled and self.use_tiled_tc):
             return True
@@ -838,7 +841,12 @@ class Transformer(nn.Module):
         self._check_loaded()
         st = torch.cuda.current_stream(self.device).cuda_stream
         h, xn = bufs["h"], bufs["xn"]
-        h.copy_(self.tok_embeddings(self._tok_dev[:B]).to(DTYPE))
+        if self._narrow(B):
+            # one launch, which clamps token ids, as in the other body (the sums of squares are not used)
+            check(lib.q40_embed_rows(self.tok_embeddings.weight.data_ptr(), self._tok_dev.data_ptr(), h.data_ptr(),
+                                     bufs["ss_ffn"].data_ptr(), 1, B, p.dim, p.vocab_size, st), "q40_embed_rows")
+        else:
+            h.copy_(self.tok_embeddings(self._tok_dev[:B]).to(DTYPE))
         pos, plen = self._pos_dev, self._prefix_len_dev
         aws = bufs["attn_ws"]
         pending = None     # output of the previous sub-block, added to h by the next norm kernel
@@ -955,7 +963,7 @@ class Transformer(nn.Module):
         self._check_steps()
         fused = self._fused_body(B)
         per_layer = (5 if self._fused_attn_for(B) else 7) if fused else (9 if self._silu_pair(B, self.layers[0].feed_forward) else 10)
-        self.launches_per_step = self.params.n_layers * per_layer + (2 if fused else 1)
+        self.launches_per_step = self.params.n_layers * per_layer + (2 if self._narrow(B) else 1)
         if not self.use_cuda_graph:
             return self._decode_body(B)
         key = (B, self.greedy_feedback, self.use_fused, self.use_pdl, self.max_cluster, self.use_stream,

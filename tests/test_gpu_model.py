@@ -504,6 +504,23 @@ def test_expired_wait_of_a_step_is_reported(width, use_graph):
         assert torch.equal(step(width), want[0]) and torch.equal(step(1), want[1])
 
 
+@pytest.mark.parametrize("width", [3, 9, 16])
+def test_token_ids_of_narrow_steps_are_clamped(width):
+    """Rows of the embedding are read by the library's launch, which clamps ids: those beside the vocabulary give the logits of
+    its first and last token."""
+    m = small_random()
+    m(torch.arange(40, device="cuda").view(1, -1), 0)
+    m.fork(0, 1, width - 1)
+    toks = torch.arange(width, device="cuda").view(-1, 1)
+    toks[0], toks[-1] = 0, 511
+    want = m(toks, 40).clone()
+    assert m._fused_body(width) == (width <= 8)
+    m.tok_embeddings.forward = None              # not the library's way through torch
+    toks[0], toks[-1] = -1, 512
+    m.release_graphs()
+    assert torch.equal(m(toks, 40), want)
+
+
 @pytest.mark.parametrize("S", [8, 40])
 @pytest.mark.parametrize("broken", ["norm on the host", "last norm on the host", "scales too few", "codes too few",
                                     "scales in fp32", "shape turned round", "too narrow"])
