@@ -427,16 +427,17 @@ class Transformer(nn.Module):
         for l, o in zip(lins, outs):
             K.matmul_q40(x, l.w, l.s, l.kn(), group_size=l.group_size, relayout=False, out=o)
 
-    def _mm_silu(self, x, tiled, g, args, err, st, ws=None, pdl=None):
-        """g = silu(x @ deq(W_1)) * (x @ deq(W_3)) for the tiled copies of the two: one launch, with the scratch `ws` (of
-        this stream or capture, if none is given)."""
+    @staticmethod
+    def _tc_ws_args(ws):
+        return (ws.data_ptr(), ws.numel()) if ws is not None else (None, 0)
+
+    def _mm_silu(self, x, tiled, g, args, err, st):
+        """g = silu(x @ deq(W_1)) * (x @ deq(W_3)) for the tiled copies of the two: one launch (prompt pass)."""
         _, P, widths64, widths = args
-        if ws is None:
-            ws = K._tiled_tc_workspace(x.device, x.shape[0])
+        ws = K._tiled_tc_workspace(x.device, x.shape[0])
         check(lib.q40_gemm_tiled_tc_ws(2, x.data_ptr(), x.stride(0), P(*[t.data_ptr() for t in tiled]), P(*[g.data_ptr()] * 2),
-                                       widths64, widths, x.shape[0], x.shape[1], 1, ws.data_ptr() if ws is not None else None,
-                                       ws.numel() if ws is not None else 0, err.data_ptr() if isinstance(err, torch.Tensor) else err,
-                                       1 if (self.use_pdl if pdl is None else pdl) else 0, st), "q40_gemm_tiled_tc_ws")
+                                       widths64, widths, x.shape[0], x.shape[1], 1, *self._tc_ws_args(ws), err.data_ptr(),
+                                       1 if self.use_pdl else 0, st), "q40_gemm_tiled_tc_ws")
 
     # ------------------------------------------------------------------ decode
     def _step_buffers(self, B):
@@ -506,6 +507,43 @@ class Transformer(nn.Module):
         check(lib.q40_gemm_kn(x.data_ptr(), x.stride(0), lin.w.data_ptr(), lin.s.data_ptr(), out.data_ptr(),
                               out.stride(0), x.shape[0], N, Kd, lin.group_size, ws.data_ptr(), ws.numel(), st),
               "q40_gemm_kn")
+
+    def _step_site(self, x, lins, outs):
+        """What the launches of one tensor-core matmul on tiled copies share in all layers of a step, or None where `lins`,
+        the first layer's projections, are not multiplied that way.  Laid out once a step: with the rules of _gemm_multi
+        asked, and its arrays made, in every layer, the first step at a width took 16.0 ms for 10 branches and 19.4 for 100
+        (now 12.3 and 15.9)."""
+        kns = [l.kn() for l in lins]
+        if not (x.shape[0] > 8 and self.use_tiled and self.use_tiled_tc and x.stride(0) % 8 == 0 and
+                all(l.group_size == 64 and self._tileable(l) and kn[0] == x.shape[1] and kn[0] % 64 == 0 and
+                    o.stride(0) % 2 == 0 for l, kn, o in zip(lins, kns, outs))):
+            return None
+        n = len(lins)
+        P = ctypes.c_void_p * n
+        return (kns, n, x.data_ptr(), x.stride(0), P, P(*[o.data_ptr() for o in outs]),
+                (ctypes.c_int64 * n)(*[o.stride(0) for o in outs]), (ctypes.c_int * n)(*[kn[1] for kn in kns]), *x.shape)
+
+    def _step_mm(self, bufs, site, lins, st, silu=False):
+        """One layer's launch of a prepared matmul (`silu`: of silu(x @ W_1) * (x @ W_3)); False if its projections are not
+        like the first layer's."""
+        if site is None:
+            return False
+        kns, n, x, ldx, P, outs, ldc, widths, M, Kd = site
+        for l, kn in zip(lins, kns):
+            if l.kn() != kn or l.group_size != 64:
+                return False
+        tiled, pdl = self._tiled_of(lins)
+        tiled, err = P(*[t.data_ptr() for t in tiled]), bufs["gemm_ws"].data_ptr() + 4096 - 4    # q40_gemm_kn's error word
+        if silu:
+            ws = self._step_tc_ws(M)
+            if ws is None:
+                ws = K._tiled_tc_workspace(self.device, M)
+            check(lib.q40_gemm_tiled_tc_ws(n, x, ldx, tiled, outs, ldc, widths, M, Kd, 1, *self._tc_ws_args(ws), err,
+                                           1 if pdl else 0, st), "q40_gemm_tiled_tc_ws")
+        else:
+            check(lib.q40_gemm_tiled_tc_multi(n, x, ldx, tiled, outs, ldc, widths, M, Kd, err, 1 if pdl else 0, st),
+                  "q40_gemm_tiled_tc_multi")
+        return True
 
     def _gemm_multi(self, bufs, x, lins, outs, st):
         """Several projections of the same activations: one tensor-core launch above 8 rows when the
@@ -852,14 +890,20 @@ class Transformer(nn.Module):
         pending = None     # output of the previous sub-block, added to h by the next norm kernel
         peer = self._tp_peer_buffers() if self.tp_world > 1 and self.use_tp_fused_allreduce else None
         normed = False     # xn already holds the attention norm of h (written by the fused all-reduce)
+        qkv, ao, g = bufs["qkv"], bufs["ao"], bufs["g"]
+        Wq = (H + 2 * Hkv) * D
+        bq, bk, bv = qkv[:, :H * D], qkv[:, H * D:(H + Hkv) * D], qkv[:, (H + Hkv) * D:]
+        att, ff = self.layers[0].attention, self.layers[0].feed_forward
+        q_site = self._step_site(xn, (att.wq, att.wk, att.wv), (bq, bk, bv))
+        o_site = self._step_site(ao, (att.wo,), (bufs["o"],))
+        f_site = self._step_site(g, (ff.w2,), (bufs["f"],))
+        silu_site = self._step_site(xn, (ff.w1, ff.w3), (g, g)) if self._silu_pair(B, ff) else None
         for li, layer in enumerate(self.layers):
             att, ff = layer.attention, layer.feed_forward
             if not normed:
                 self._norm(h, pending, layer.attention_norm.weight, xn, st)
-            qkv = bufs["qkv"]
-            Wq = (H + 2 * Hkv) * D
-            bq, bk, bv = qkv[:, :H * D], qkv[:, H * D:(H + Hkv) * D], qkv[:, (H + Hkv) * D:]
-            self._gemm_multi(bufs, xn, [att.wq, att.wk, att.wv], [bq, bk, bv], st)
+            if not self._step_mm(bufs, q_site, (att.wq, att.wk, att.wv), st):
+                self._gemm_multi(bufs, xn, [att.wq, att.wk, att.wv], [bq, bk, bv], st)
             check(lib.q40_rope_kv_append(bq.data_ptr(), Wq, bk.data_ptr(), Wq,
                                          bv.data_ptr(), Wq, pos.data_ptr(), plen.data_ptr(),
                                          self._cos.data_ptr(), self._sin.data_ptr(), self._n_pos,
@@ -872,24 +916,22 @@ class Transformer(nn.Module):
                                            att.cache_k.data_ptr(), att.cache_k_s.data_ptr(),
                                            att.cache_v.data_ptr(), att.cache_v_s.data_ptr(), p.max_seq_len,
                                            pos.data_ptr(), bk.data_ptr(), bv.data_ptr(), Wq,
-                                           bufs["ao"].data_ptr(), B, H, Hkv, D, aws.data_ptr(), aws.numel(), st),
+                                           ao.data_ptr(), B, H, Hkv, D, aws.data_ptr(), aws.numel(), st),
                   "q40_attn_tree_decode")
-            self._gemm_multi(bufs, bufs["ao"], [att.wo], [bufs["o"]], st)
+            if not self._step_mm(bufs, o_site, (att.wo,), st):
+                self._gemm_multi(bufs, ao, [att.wo], [bufs["o"]], st)
             if peer is not None:
                 # all-reduce of the partial wo outputs + residual add + ffn norm: one launch
                 peer.allreduce_norm(bufs["o"], h, layer.ffn_norm.weight, xn, p.norm_eps, st, self.tp_wait_cycles)
             else:
                 self._all_reduce(bufs["o"])
                 self._norm(h, bufs["o"], layer.ffn_norm.weight, xn, st)
-            if self._silu_pair(B, ff):
-                tiled, pdl = self._tiled_of((ff.w1, ff.w3))
-                self._mm_silu(xn, tiled, bufs["g"], self._mm_args([l.kn()[1] for l in (ff.w1, ff.w3)]),
-                              bufs["gemm_ws"].data_ptr() + 4096 - 4, st, self._step_tc_ws(B), pdl)
-            else:
+            if not self._step_mm(bufs, silu_site, (ff.w1, ff.w3), st, True):
                 self._gemm_multi(bufs, xn, [ff.w1, ff.w3], [bufs["a1"], bufs["a3"]], st)
-                check(lib.q40_silu_mul(bufs["a1"].data_ptr(), bufs["a3"].data_ptr(), bufs["g"].data_ptr(),
-                                       bufs["g"].numel(), st), "q40_silu_mul")
-            self._gemm_multi(bufs, bufs["g"], [ff.w2], [bufs["f"]], st)
+                check(lib.q40_silu_mul(bufs["a1"].data_ptr(), bufs["a3"].data_ptr(), g.data_ptr(), g.numel(), st),
+                      "q40_silu_mul")
+            if not self._step_mm(bufs, f_site, (ff.w2,), st):
+                self._gemm_multi(bufs, g, [ff.w2], [bufs["f"]], st)
             if peer is not None:
                 # ... of the partial w2 outputs + residual add + the next layer's attention norm (or the final norm)
                 nxt = self.layers[li + 1].attention_norm.weight if li + 1 < len(self.layers) else self.norm.weight
