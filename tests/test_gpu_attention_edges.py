@@ -90,3 +90,20 @@ def test_causal_rows_whose_first_tile_of_scores_is_minus_infinity(K):
     want = torch.einsum("hij,jhd->ihd", torch.softmax(s, -1), v[blocked:].double().repeat_interleave(2, 1))
     np.testing.assert_allclose(got[blocked:].float().cpu().numpy(), want.float().cpu().numpy(), **TOL)
     assert not got[:blocked].any()
+
+
+@pytest.mark.parametrize("blocked", [70, 130])        # of 130 shared keys: a split of 64 and part of the next, then all
+def test_shared_keys_whose_scores_are_minus_infinity(K, blocked):
+    """They weigh nothing beside a branch's own keys and the other shared ones; a branch without any has zeros."""
+    rng = np.random.default_rng(blocked)
+    B, H, prefix = 3, 4, 130
+    q, pk, pv = normal(rng, B, H, 128), normal(rng, prefix, H, 128), normal(rng, prefix, H, 128)
+    kp, vp = normal(rng, H, 32, 128), normal(rng, H, 32, 128)
+    q[..., 0], pk[:blocked, :, 0] = 1.0, -np.inf
+    table, lens = np.arange(6, dtype=np.int32).reshape(3, 2) % 4, np.array([0, 5, 16], dtype=np.int32)
+    d = lambda x: torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    got = K.shared_prefix_attn(d(q), d(pk), d(pv), prefix, d(table), d(lens), d(kp), d(vp), page_size=8).float().cpu().numpy()
+    some = slice(1, None) if blocked == prefix else slice(None)       # branches with a finite score
+    want = O.attn_shared_prefix(q[some], pk[blocked:], pv[blocked:], prefix - blocked, table[some], lens[some], kp, vp, 8)
+    np.testing.assert_allclose(got[some], want.astype(np.float32), **TOL)
+    assert blocked < prefix or not got[0].any()
