@@ -87,8 +87,8 @@ int q40_gemm_kn(const void* a, int64_t lda, const void* bw, const void* bs, void
 
 /* The tensor-core form q40_gemm_kn selects for M > 16 (group 64, K % 64 == 0, N % 128 == 0, even ldc, lda % 8 == 0):
  * tcgen05.mma with the 128 output features of a packed block as the MMA M dimension and the
- * batch as N, accumulator in tensor memory, split-K over a thread-block cluster.  `err` is a
- * device int (zeroed by the caller) that the kernel sets to 1 if one of its bounded waits
+ * batch as N, accumulator in tensor memory, split-K over a thread-block cluster.  `err` is an
+ * int (zeroed by the caller) in device or mapped host memory that the kernel sets to 1 if one of its bounded waits
  * expired, in which case the output is undefined; through q40_gemm_kn it is the last int of the
  * first 4096 bytes of the workspace.
  * Replaces: matmul_q40 (triton_kernels.py:357-500) at batch 100 and for the prompt pass. */

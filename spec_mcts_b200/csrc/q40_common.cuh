@@ -18,6 +18,9 @@
     if (e__ != cudaSuccess) return (int)e__;        \
   } while (0)
 
+// A bounded wait has run out: the caller's error word, which may be mapped host memory (all writers store the same)
+__device__ __forceinline__ void q40_set_error(int* err) { *reinterpret_cast<volatile int*>(err) = 1; }
+
 static inline bool q40_aligned(const void* p, size_t a) { return ((uintptr_t)p % a) == 0; }
 
 // Allow `kern` that much dynamic shared memory, once per device (`ready`: one bit each).  The limit is a property of the

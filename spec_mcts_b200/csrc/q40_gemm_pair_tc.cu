@@ -618,7 +618,7 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
   failed = *s_failed != 0;
   if (failed && tid == 0) {
     // the copies still on their way, those of the last S blocks at most: none may land in shared memory that has been given back
-    atomicExch(p.err, 1);
+    q40_set_error(p.err);
     const int n = max(s_copied[0], s_copied[1]);
     for (int i = max(0, n - S); i < n; ++i) mbar_wait(bar_full + 8 * (i % S), (uint32_t)((i / S) & 1));
   }

@@ -286,7 +286,7 @@ gemm_tc_kernel(const TcParams p) {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   __syncthreads();
   failed = *s_failed != 0;
-  if (failed && tid == 0) atomicExch(p.err, 1);
+  if (failed && tid == 0) q40_set_error(p.err);
   Q40_STAMP(4);
 
   // ---- accumulator -> fp32 tile in shared memory, [Mpad][128] with features in natural order ----

@@ -54,7 +54,7 @@ struct Params {
 // `copied` k blocks at most: none may land in shared memory that this CTA has given back.  (The MMAs that were issued are
 // waited for through the `done` barrier, which the issuing thread commits to, also after giving up.)
 __device__ __noinline__ void give_up(int* err, uint32_t bar_full, int S, int copied) {
-  atomicExch(err, 1);
+  q40_set_error(err);
   for (int i = max(0, copied - S); i < copied; ++i) mbar_wait(bar_full + 8 * (i % S), (uint32_t)((i / S) & 1));
 }
 

@@ -58,6 +58,18 @@ def precompute_freqs_cis(dim: int, end: int, theta: float = 10000.0):
     return torch.polar(torch.ones_like(freqs), freqs)
 
 
+class HostWord:
+    """An int32 in host memory that kernels can write; copies of its owner have one of their own."""
+    __slots__ = ("host", "ptr", "_pinned")
+
+    def __init__(self):
+        self._pinned = torch.zeros(1, dtype=torch.int32).pin_memory()
+        self.host, self.ptr = self._pinned.numpy(), self._pinned.data_ptr()
+
+    def __reduce__(self):
+        return HostWord, ()
+
+
 class RMSNorm(nn.Module):
     def __init__(self, dim: int, eps: float = 1e-6):
         super().__init__()
@@ -243,9 +255,9 @@ class Transformer(nn.Module):
         self._tc_err_own = torch.zeros(1, dtype=torch.int32, device=dev)      # ... in place of a captured pass's own word
         self._tc_err_host = torch.zeros(1, dtype=torch.int32).pin_memory()
         self._prompt_unchecked = False
-        # per width, the error word (in gemm_ws) that the width's last finished step left
-        self._step_err_host = torch.zeros(p.max_batch_size + 1, dtype=torch.int32).pin_memory()
-        self._step_errs = self._step_err_host.numpy()
+        # the error word of the steps' tensor-core matmuls: host memory that they can write, so that nothing has to be copied
+        # (a copy behind each step: 12 us of one of 100 branches)
+        self._step_err = HostWord()
         # ... True: through the byte-balanced stream-K launch (one CTA per SM, bulk-copy ring, no clusters);
         # False: the cluster-reduced launch on the same tiled copies (faster on B200, the default)
         self.use_stream = False
@@ -460,15 +472,10 @@ class Transformer(nn.Module):
             self._bufs[B] = b
         return b
 
-    @staticmethod
-    def _step_err(bufs):
-        """The device word that a step's tensor-core matmuls set on a wait expiry (q40_gemm_kn's own, in its scratch)."""
-        return bufs["gemm_ws"][4092:4096].view(torch.int32)
-
     def _check_steps(self):
         """Raise if a bounded wait inside a matmul of an earlier step expired, as far as the host has heard: without waiting
         for steps in flight."""
-        if self._step_errs.any() and not torch.cuda.is_current_stream_capturing():
+        if self._step_err.host[0] and not torch.cuda.is_current_stream_capturing():
             self._steps_failed()
 
     @torch.inference_mode()
@@ -479,14 +486,14 @@ class Transformer(nn.Module):
         if self._tc_ws is not None:
             self._tc_ws[:K._TILED_TC_FLAGS].zero_()
         torch.cuda.synchronize(self.device)
-        self._step_errs.fill(0)
+        self._step_err.host[0] = 0
         raise K.Q40Error("decode step: a bounded wait inside a tensor-core matmul expired")
 
     def decode_status(self) -> int:
         """Non-zero if a bounded wait inside a tensor-core matmul of a decode step expired, which makes its logits and cache
-        rows undefined (synchronises).  The first step after the word has reached the host raises."""
+        rows undefined (synchronises).  The first step that finds the word set raises."""
         torch.cuda.synchronize(self.device)
-        return int(self._step_errs.any())
+        return int(self._step_err.host[0])
 
     def _step_tc_ws(self, B):
         """Scratch of q40_gemm_tiled_tc_ws for a step of B branches, or None where it uses none: one for all widths, whose
@@ -523,7 +530,7 @@ class Transformer(nn.Module):
         return (kns, n, x.data_ptr(), x.stride(0), P, P(*[o.data_ptr() for o in outs]),
                 (ctypes.c_int64 * n)(*[o.stride(0) for o in outs]), (ctypes.c_int * n)(*[kn[1] for kn in kns]), *x.shape)
 
-    def _step_mm(self, bufs, site, lins, st, silu=False):
+    def _step_mm(self, site, lins, st, silu=False):
         """One layer's launch of a prepared matmul (`silu`: of silu(x @ W_1) * (x @ W_3)); False if its projections are not
         like the first layer's."""
         if site is None:
@@ -533,7 +540,7 @@ class Transformer(nn.Module):
             if l.kn() != kn or l.group_size != 64:
                 return False
         tiled, pdl = self._tiled_of(lins)
-        tiled, err = P(*[t.data_ptr() for t in tiled]), bufs["gemm_ws"].data_ptr() + 4096 - 4    # q40_gemm_kn's error word
+        tiled, err = P(*[t.data_ptr() for t in tiled]), self._step_err.ptr
         if silu:
             ws = self._step_tc_ws(M)
             if ws is None:
@@ -558,7 +565,7 @@ class Transformer(nn.Module):
                 # widths that cannot be tiled one by one (a kv head per rank: 128 columns) but whose outputs are
                 # adjacent column ranges of one buffer: one tiled copy of the concatenated matrix, one launch
                 cat, pdl = self._tiled_concat(lins)
-                err = bufs["gemm_ws"].data_ptr() + 4096 - 4
+                err = self._step_err.ptr
                 P1 = ctypes.c_void_p * 1
                 check(lib.q40_gemm_tiled_tc_multi(1, x.data_ptr(), x.stride(0), P1(cat.data_ptr()),
                                                   P1(outs[0].data_ptr()), (ctypes.c_int64 * 1)(outs[0].stride(0)),
@@ -577,7 +584,7 @@ class Transformer(nn.Module):
                 return
             if t_idx and n <= 3 and all(l.kn()[0] == lins[0].kn()[0] for l in lins):
                 P = ctypes.c_void_p * n
-                err = bufs["gemm_ws"].data_ptr() + 4096 - 4      # the error word q40_gemm_kn also uses
+                err = self._step_err.ptr
                 tiled, pdl = self._tiled_of(lins)
                 check(lib.q40_gemm_tiled_tc_multi(n, x.data_ptr(), x.stride(0), P(*[t.data_ptr() for t in tiled]),
                                                   P(*[o.data_ptr() for o in outs]),
@@ -593,7 +600,7 @@ class Transformer(nn.Module):
                 self._gemm(bufs, x, l, o, st)
             return
         P = ctypes.c_void_p * n
-        err = bufs["gemm_ws"].data_ptr() + 4096 - 4      # the error word q40_gemm_kn also uses
+        err = self._step_err.ptr
         check(lib.q40_gemm_kn_tc_multi(n, x.data_ptr(), x.stride(0), P(*[l.w.data_ptr() for l in lins]),
                                        P(*[l.s.data_ptr() for l in lins]), P(*[o.data_ptr() for o in outs]),
                                        (ctypes.c_int64 * n)(*[o.stride(0) for o in outs]),
@@ -902,7 +909,7 @@ class Transformer(nn.Module):
             att, ff = layer.attention, layer.feed_forward
             if not normed:
                 self._norm(h, pending, layer.attention_norm.weight, xn, st)
-            if not self._step_mm(bufs, q_site, (att.wq, att.wk, att.wv), st):
+            if not self._step_mm(q_site, (att.wq, att.wk, att.wv), st):
                 self._gemm_multi(bufs, xn, [att.wq, att.wk, att.wv], [bq, bk, bv], st)
             check(lib.q40_rope_kv_append(bq.data_ptr(), Wq, bk.data_ptr(), Wq,
                                          bv.data_ptr(), Wq, pos.data_ptr(), plen.data_ptr(),
@@ -918,7 +925,7 @@ class Transformer(nn.Module):
                                            pos.data_ptr(), bk.data_ptr(), bv.data_ptr(), Wq,
                                            ao.data_ptr(), B, H, Hkv, D, aws.data_ptr(), aws.numel(), st),
                   "q40_attn_tree_decode")
-            if not self._step_mm(bufs, o_site, (att.wo,), st):
+            if not self._step_mm(o_site, (att.wo,), st):
                 self._gemm_multi(bufs, ao, [att.wo], [bufs["o"]], st)
             if peer is not None:
                 # all-reduce of the partial wo outputs + residual add + ffn norm: one launch
@@ -926,11 +933,11 @@ class Transformer(nn.Module):
             else:
                 self._all_reduce(bufs["o"])
                 self._norm(h, bufs["o"], layer.ffn_norm.weight, xn, st)
-            if not self._step_mm(bufs, silu_site, (ff.w1, ff.w3), st, True):
+            if not self._step_mm(silu_site, (ff.w1, ff.w3), st, True):
                 self._gemm_multi(bufs, xn, [ff.w1, ff.w3], [bufs["a1"], bufs["a3"]], st)
                 check(lib.q40_silu_mul(bufs["a1"].data_ptr(), bufs["a3"].data_ptr(), g.data_ptr(), g.numel(), st),
                       "q40_silu_mul")
-            if not self._step_mm(bufs, f_site, (ff.w2,), st):
+            if not self._step_mm(f_site, (ff.w2,), st):
                 self._gemm_multi(bufs, g, [ff.w2], [bufs["f"]], st)
             if peer is not None:
                 # ... of the partial w2 outputs + residual add + the next layer's attention norm (or the final norm)
@@ -943,8 +950,6 @@ class Transformer(nn.Module):
         if not normed:
             self._norm(h, pending, self.norm.weight, xn, st)
         torch.matmul(xn, self.output.weight.t(), out=bufs["logits"])
-        if B > 8:                      # narrower matmuls have no wait that could expire
-            self._step_err_host[B:B + 1].copy_(self._step_err(bufs), non_blocking=True)
         if self.greedy_feedback:
             self._tok_dev[:B].copy_(bufs["logits"].argmax(dim=-1))
             self._pos_dev[:B] += 1

@@ -1,6 +1,7 @@
 """Model-level parity on the GPU: the q40b200 model class against logits and greedy tokens
 produced by the reference's own model class (run on CPU by tests/golden/make_golden_model.py)
 for prefill -> fork -> 12 decode steps on 3 branches of a small geometry."""
+import copy
 import os
 
 import numpy as np
@@ -489,14 +490,14 @@ def test_expired_wait_of_a_step_is_reported(width, use_graph):
     m.use_cuda_graph = use_graph
     m(torch.arange(40, device="cuda").view(1, -1), 0)
     m.fork(0, 1, 23)
+    assert copy.deepcopy(m._step_err).ptr != m._step_err.ptr
     step = lambda b: m(torch.arange(b, device="cuda").view(-1, 1), 40).clone()
     want = step(width), step(1)
     for after in (width, 1):
         assert m.decode_status() == 0
+        m._step_err.host[0] = 1
         with torch.inference_mode():
-            m._step_err(m._bufs[width]).fill_(1)
             m._tc_ws[:8192].fill_(5)
-        step(width)
         assert m.decode_status() != 0
         with pytest.raises(KK.Q40Error):
             step(after)

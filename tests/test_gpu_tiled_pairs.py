@@ -105,7 +105,8 @@ def test_silu_product_is_that_of_the_separate_launches(K, M, Kd, n):
 
 def test_a_share_that_never_comes_is_given_up_after_seconds(K):
     """Arrivals of the first pair start so low that the wait for its sums runs out: an error word instead of a result, not
-    before the time that the kernel's other waits allow, and the next launch on zeroed scratch works."""
+    before the time that the kernel's other waits allow, and the next launch on zeroed scratch works.  The word may be host
+    memory, as that of a model's steps is."""
     from spec_mcts_b200._lib import check, lib
     rng = np.random.default_rng(1)
     M, Kd, n = 16, 8064, 5120                       # 40 tiles: all are shared, on 60 to 74 pairs
@@ -115,13 +116,14 @@ def test_a_share_that_never_comes_is_given_up_after_seconds(K):
     launch(a, tiled, [want, want], (n, n), 1, ws)
     assert ws[8192:].any()                          # sums went through the scratch
     ws[:8192].view(torch.int32)[:8] = -1000
-    P, err = ctypes.c_void_p * 2, torch.zeros(1, dtype=torch.int32, device="cuda")
+    P, err = ctypes.c_void_p * 2, torch.zeros(1, dtype=torch.int32).pin_memory()
     t0, t1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
     t0.record()
     check(lib.q40_gemm_tiled_tc_ws(2, a.data_ptr(), a.stride(0), P(*[t.data_ptr() for t in tiled]), P(*[g.data_ptr()] * 2),
                                    (ctypes.c_int64 * 2)(n, n), (ctypes.c_int * 2)(n, n), M, Kd, 1, ws.data_ptr(), ws.numel(),
                                    err.data_ptr(), 0, torch.cuda.current_stream().cuda_stream), "q40_gemm_tiled_tc_ws")
     t1.record()
+    t1.synchronize()
     assert int(err.item()) == 1 and 1000 < t0.elapsed_time(t1) < 20000
     ws[:8192].zero_()
     launch(a, tiled, [g, g], (n, n), 1, ws, 1)
