@@ -51,7 +51,7 @@ def close(got, want):
 
 
 # rows at the edges of 16-row tiles, of the two ways of tensor memory (192, 256) and of the row chunks; k of one step, an odd
-# number of steps, and whole blocks; one span and several; enough tiles for pairs to share them (75 spans)
+# number of steps, and whole blocks; one span, several, and more than there are pairs
 @pytest.mark.parametrize("M,Kd,Ns", [(9, 64, (256,)), (16, 192, (256, 512)), (17, 128, (256,)), (100, 4160, (512,)), (128, 320, (256, 256, 256)),
                                      (129, 64, (512,)), (192, 320, (256,)), (193, 256, (512, 256)), (256, 192, (256,)), (257, 1024, (256,)),
                                      (10, 256, (9728, 9728)), (112, 448, (19200,)), (300, 192, (19200,))])
@@ -101,6 +101,42 @@ def test_silu_product_is_that_of_the_separate_launches(K, M, Kd, n):
     # k may be cut at other places, which moves a sum by its last fp32 bits and a product by an fp16 step of either factor
     np.testing.assert_allclose(g.float().cpu().numpy(), want.float().cpu().numpy(), rtol=4e-3, atol=1e-4)
     assert (g == want).float().mean() > 0.97
+
+
+# as many tiles as take more than a wave of pairs, or less than one, with k ranges long enough to be worth sharing, whether 60 or
+# 74 pairs run: a tile on two pairs or on three (40 tiles), blocks that do and do not divide among them, one and several
+# 16-row chunks
+@pytest.mark.parametrize("M,Kd,Ns,silu", [(10, 4096, (11008, 11008), 1), (16, 8320, (5120, 5120), 1), (16, 8064, (10240,), 0), (9, 4160, (19456,), 0),
+                                          (33, 6144, (10240, 10240), 0)])
+def test_tiles_shared_between_pairs(K, M, Kd, Ns, silu):
+    rng = np.random.default_rng(M * 100 + Kd)
+    packed, tiled = mats(K, rng, Kd, Ns)
+    acts = [rng.standard_normal((M, Kd)).astype(np.float16) for _ in range(2)]
+    acts_d, ws = [torch.from_numpy(a).cuda() for a in acts], scratch(K, M)
+
+    def run(a, pdl=0):
+        outs = [torch.full((M, n), float("nan"), dtype=torch.float16, device="cuda") for n in (Ns[:1] if silu else Ns)]
+        launch(a, tiled, outs * 2 if silu else outs, Ns, silu, ws, pdl)
+        return outs
+
+    first = [run(a) for a in acts_d]
+    assert ws[8192:].any(), "no sums went through the scratch"
+    for a, outs in zip(acts, first):
+        want = [O.matmul_q40(a, q, s, (Kd, n)) for (q, s), n in zip(packed, Ns)]
+        if not silu:
+            for o, w in zip(outs, want):
+                close(o, w)
+            continue
+        # the bounds of `close` for either factor f (df = 2e-3 |f| + 4e-3 mean|f|), and two more roundings to fp16
+        x, y = (w.astype(np.float64) for w in want)
+        dx, dy = (2e-3 * np.abs(f) + 4e-3 * np.abs(f).mean() for f in (x, y))
+        g = x / (1 + np.exp(-x))
+        bound = 1.1 * dx * np.abs(y) + np.abs(g) * dy + dx * dy + 2e-3 * np.abs(g * y) + 1e-4       # |silu'| < 1.1
+        assert (np.abs(outs[0].double().cpu().numpy() - g * y) <= bound).all()
+    # scratch and flags of one launch are the next one's, launched while it drains
+    for i in (0, 1, 1, 0, 1):
+        assert all(torch.equal(o, f) for o, f in zip(run(acts_d[i], 1), first[i]))
+    assert not ws[:8192].any()
 
 
 def test_a_share_that_never_comes_is_given_up_after_seconds(K):
