@@ -697,7 +697,7 @@ def test_matmul_on_a_second_stream_reads_a_finished_copy(K, M):
     assert all(torch.equal(x, want) for x in (first, *second))
 
 
-@pytest.mark.parametrize("M", [4, 40])
+@pytest.mark.parametrize("M", [4, 12, 40])
 def test_matmul_whose_weight_is_first_seen_in_a_capture(K, M):
     """The captured call, the graph's replay and the calls after the capture all multiply by the weight."""
     g = torch.Generator(device="cuda").manual_seed(M)

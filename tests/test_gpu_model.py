@@ -522,6 +522,40 @@ def test_token_ids_of_narrow_steps_are_clamped(width):
     assert torch.equal(m(toks, 40), want)
 
 
+@pytest.mark.parametrize("B", [9, 16])
+@pytest.mark.parametrize("variant", ["default", "no graph", "stream", "q4 head", "one kv head", "no tc", "no copies"])
+def test_steps_of_9_to_16_branches_by_either_body(variant, B):
+    """Which body such a step takes, and its logits against one launch per operation on the checkpoint layout: within the
+    matmul tolerance (no cached code takes part in a first step)."""
+    from spec_mcts_b200 import kernels as KK
+    kw = dict(n_kv_heads=1) if variant == "one kv head" else {}
+    logits = []
+    for plain in (True, False):
+        m = small_random(**kw)
+        m(torch.arange(40, device="cuda").view(1, -1), 0)
+        m.fork(0, 1, B - 1)
+        if plain:
+            m.use_fused = m.use_tiled = False
+        elif variant == "no graph":
+            m.use_cuda_graph = False
+        elif variant == "stream":
+            m.use_stream = True
+        elif variant == "q4 head":
+            m.quantize_lm_head()
+        elif variant == "no tc":
+            m.use_tiled_tc = False
+        elif variant == "no copies":
+            m.use_tiled = False
+        logits.append(m(torch.arange(B, device="cuda").view(-1, 1) * 7, 40)[:, -1].float().cpu().numpy())
+    assert m._fused_body(B) == (variant not in ("default", "no graph"))
+    if variant == "q4 head":
+        lin = m._lm_head_q4
+        with torch.inference_mode():
+            xn = KK.rmsnorm(m._step_buffers(B)["h"].clone(), m.norm.weight, m.params.norm_eps)
+            logits[0] = KK.matmul_q40(xn, lin.w, lin.s, lin.kn())[:, :512].float().cpu().numpy()
+    assert rel_l2(logits[1], logits[0]).max() < 2e-2
+
+
 @pytest.mark.parametrize("S", [8, 40])
 @pytest.mark.parametrize("broken", ["norm on the host", "last norm on the host", "scales too few", "codes too few",
                                     "scales in fp32", "shape turned round", "too narrow"])
