@@ -62,8 +62,7 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 _workspaces: dict = {}
-_in_graphs: set = set()             # keys of those whose address a graph has
-_outgrown: list = []                # ... when a larger one had taken their place
+_outgrown: list = []                # ... whose place a larger one has taken
 _capture_workspaces: dict = {}      # the same keys -> (id of the stream's last capture, buffer made in it)
 
 
@@ -71,31 +70,24 @@ def _workspace(kind: str, dev: torch.device, nbytes: int, zero: bool) -> torch.T
     """Per (kind, device, stream) scratch buffer, grown on demand.  Split-K GEMM scratch
     must start zeroed (the kernels restore that); calls on different streams get
     different buffers so that they may overlap.  One that is made inside a capture serves that capture only: until the
-    graph runs it holds nothing, and each replay makes it ready again.  One that a graph has the address of is not given
-    back; the next is at least twice its size, so that all of these take no more than the last."""
+    graph runs it holds nothing, and each replay makes it ready again.  One that is outgrown is not given back, since a graph
+    may have its address; the next is at least twice its size, so that all of these take no more than the last."""
     key = (kind, dev.index, _stream(dev))
     buf = _workspaces.get(key)
-    if buf is not None and buf.numel() >= nbytes:
-        if torch.cuda.is_current_stream_capturing():
-            _in_graphs.add(key)
-    else:
-        n = max(int(nbytes), 1 << 20)
-        capture = None
+    if buf is None or buf.numel() < nbytes:
+        n, make = max(int(nbytes), 1 << 20), torch.zeros if zero else torch.empty
         if torch.cuda.is_current_stream_capturing():
             capture = ctypes.c_uint64()
             check(lib.q40_capture_id(key[2], ctypes.byref(capture)), "q40_capture_id")
             made_in, buf = _capture_workspaces.get(key, (None, None))
-            if made_in == capture.value and buf.numel() >= nbytes:
-                return buf
-        elif key in _in_graphs:
-            _in_graphs.discard(key)
+            if made_in != capture.value or buf.numel() < nbytes:
+                buf = make(n, dtype=torch.uint8, device=dev)
+                _capture_workspaces[key] = (capture.value, buf)
+            return buf
+        if buf is not None:
             _outgrown.append(buf)
             n = max(n, 2 * buf.numel())
-        buf = (torch.zeros if zero else torch.empty)(n, dtype=torch.uint8, device=dev)
-        if capture is None:
-            _workspaces[key] = buf
-        else:
-            _capture_workspaces[key] = (capture.value, buf)
+        buf = _workspaces[key] = make(n, dtype=torch.uint8, device=dev)
     return buf
 
 
@@ -439,9 +431,12 @@ def _tc_error_word_lasts(dev) -> bool:
 
 def _tc_error_page(dev, st) -> torch.Tensor:
     """The 4096 bytes that end with that word, or under a capture on a stream that has none yet, bytes that nobody reads."""
-    if torch.cuda.is_current_stream_capturing() and ("gemm", dev.index, st) not in _workspaces:
-        return torch.empty(4096, dtype=torch.uint8, device=dev)
-    return _workspace("gemm", dev, 4096, zero=True)
+    page = _workspaces.get(("gemm", dev.index, st))
+    if page is None:
+        if torch.cuda.is_current_stream_capturing():
+            return torch.empty(4096, dtype=torch.uint8, device=dev)
+        page = _workspace("gemm", dev, 4096, zero=True)
+    return page
 
 
 def tc_error_flag(dev=None) -> int:

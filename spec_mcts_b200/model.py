@@ -337,6 +337,9 @@ class Transformer(nn.Module):
         e = lambda n: torch.empty((S, n), dtype=DTYPE, device=dev)
         xn, q, ao, o, a1, a3, g, f = (e(n) for n in (p.dim, H * D, H * D, p.dim, hid, hid, hid, p.dim))
         args = [self._mm_args(Ns) for _, Ns in sites]
+        # of all layers' launches with the SiLU product
+        scratch = K._tiled_tc_workspace(h.device, S) if any(mm[2][1] is not None for *_, mm in plan) else None
+        silu_ws = self._tc_ws_args(scratch)
         pending = None     # output of the previous sub-block, added to h by the next norm kernel
         for att, attn_norm, ffn_norm, (qkv, wo, w13, w2) in plan:
             # keys and values go straight to their place in the prompt cache
@@ -352,7 +355,7 @@ class Transformer(nn.Module):
             self._all_reduce(o)
             self._norm(h, o, ffn_norm, xn, st)
             if w13[1] is not None:
-                self._mm_silu(xn, w13[1], g, args[2], err, st)
+                self._mm_silu(xn, w13[1], g, args[2], silu_ws, err, st)
             else:
                 self._mm(xn, w13, [a1, a3], args[2], err, st)
                 check(lib.q40_silu_mul(a1.data_ptr(), a3.data_ptr(), g.data_ptr(), g.numel(), st), "q40_silu_mul")
@@ -443,12 +446,12 @@ class Transformer(nn.Module):
     def _tc_ws_args(ws):
         return (ws.data_ptr(), ws.numel()) if ws is not None else (None, 0)
 
-    def _mm_silu(self, x, tiled, g, args, err, st):
-        """g = silu(x @ deq(W_1)) * (x @ deq(W_3)) for the tiled copies of the two: one launch (prompt pass)."""
+    def _mm_silu(self, x, tiled, g, args, ws, err, st):
+        """g = silu(x @ deq(W_1)) * (x @ deq(W_3)) for the tiled copies of the two: one launch (prompt pass).  `ws`: address
+        and size of its scratch."""
         _, P, widths64, widths = args
-        ws = K._tiled_tc_workspace(x.device, x.shape[0])
         check(lib.q40_gemm_tiled_tc_ws(2, x.data_ptr(), x.stride(0), P(*[t.data_ptr() for t in tiled]), P(*[g.data_ptr()] * 2),
-                                       widths64, widths, x.shape[0], x.shape[1], 1, *self._tc_ws_args(ws), err.data_ptr(),
+                                       widths64, widths, x.shape[0], x.shape[1], 1, *ws, err.data_ptr(),
                                        1 if self.use_pdl else 0, st), "q40_gemm_tiled_tc_ws")
 
     # ------------------------------------------------------------------ decode

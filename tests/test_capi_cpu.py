@@ -283,26 +283,23 @@ def test_scratch_made_in_a_capture_is_not_kept(launches, monkeypatch):
     assert get() is kept
 
 
-def test_scratch_whose_address_a_graph_has_is_not_given_back(launches, monkeypatch):
+def test_outgrown_scratch_is_not_given_back(launches, monkeypatch):
+    """A graph may have its address.  Sizes at least double, so that what is held stays below the last one's size."""
     import torch
     import weakref
     K, _ = launches
-    capturing = [False]
-    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing[0])
-    for name, empty in (("_in_graphs", set()), ("_outgrown", [])):
-        monkeypatch.setattr(K, name, empty, raising=False)
+    monkeypatch.setattr(K, "_outgrown", [], raising=False)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
     get = lambda n: K._workspace("gemm", torch.device("cpu"), n, zero=True)
-    plain = weakref.ref(get(4096))
-    in_graph = weakref.ref(get(2 << 20))
-    assert plain() is None
-    capturing[0] = True
-    assert get(4096) is in_graph()
-    capturing[0] = False
-    assert get(3 << 20) is not in_graph() and in_graph() is not None
-    last = weakref.ref(get(4096))
-    assert last().numel() >= 4 << 20
-    get(8 << 20)
-    assert last() is None and in_graph() is not None
+    seen = []
+    for n in (4096, 2 << 20, (2 << 20) + 1, 3 << 20, 40 << 20, (40 << 20) + 1):
+        buf = get(n)
+        assert buf.numel() >= n and get(n) is buf and not buf.any()
+        if not seen or seen[-1]() is not buf:
+            seen.append(weakref.ref(buf))
+        del buf
+    sizes = [r().numel() for r in seen]
+    assert sum(sizes[:-1]) <= sizes[-1] and len(sizes) == 5
 
 
 @pytest.mark.parametrize("dev", [None, "cuda", "cuda:1"])
