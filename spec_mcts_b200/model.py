@@ -469,6 +469,7 @@ class Transformer(nn.Module):
                      ao=e(B, H * D), o=e(B, p.dim), a1=e(B, hid), a3=e(B, hid), g=e(B, hid), f=e(B, p.dim),
                      attn_ws=torch.empty(nb_attn, dtype=torch.uint8, device=dev),
                      gemm_ws=torch.zeros(nb_gemm, dtype=torch.uint8, device=dev),
+                     tc_ws=self._step_tc_ws(B) if B > 8 else None,
                      logits=e(B, p.vocab_size), qkv=e(B, (H + 2 * Hkv) * D),
                      ss_attn=torch.zeros((B, 1024), dtype=torch.float32, device=dev),
                      ss_ffn=torch.zeros((B, 1024), dtype=torch.float32, device=dev))
@@ -533,9 +534,9 @@ class Transformer(nn.Module):
         return (kns, n, x.data_ptr(), x.stride(0), P, P(*[o.data_ptr() for o in outs]),
                 (ctypes.c_int64 * n)(*[o.stride(0) for o in outs]), (ctypes.c_int * n)(*[kn[1] for kn in kns]), *x.shape)
 
-    def _step_mm(self, site, lins, st, silu=False):
-        """One layer's launch of a prepared matmul (`silu`: of silu(x @ W_1) * (x @ W_3)); False if its projections are not
-        like the first layer's."""
+    def _step_mm(self, site, lins, st, silu_ws=None):
+        """One layer's launch of a prepared matmul (`silu_ws`: of silu(x @ W_1) * (x @ W_3), with that scratch); False if its
+        projections are not like the first layer's."""
         if site is None:
             return False
         kns, n, x, ldx, P, outs, ldc, widths, M, Kd = site
@@ -544,11 +545,8 @@ class Transformer(nn.Module):
                 return False
         tiled, pdl = self._tiled_of(lins)
         tiled, err = P(*[t.data_ptr() for t in tiled]), self._step_err.ptr
-        if silu:
-            ws = self._step_tc_ws(M)
-            if ws is None:
-                ws = K._tiled_tc_workspace(self.device, M)
-            check(lib.q40_gemm_tiled_tc_ws(n, x, ldx, tiled, outs, ldc, widths, M, Kd, 1, *self._tc_ws_args(ws), err,
+        if silu_ws is not None:
+            check(lib.q40_gemm_tiled_tc_ws(n, x, ldx, tiled, outs, ldc, widths, M, Kd, 1, *silu_ws, err,
                                            1 if pdl else 0, st), "q40_gemm_tiled_tc_ws")
         else:
             check(lib.q40_gemm_tiled_tc_multi(n, x, ldx, tiled, outs, ldc, widths, M, Kd, err, 1 if pdl else 0, st),
@@ -908,6 +906,10 @@ class Transformer(nn.Module):
         o_site = self._step_site(ao, (att.wo,), (bufs["o"],))
         f_site = self._step_site(g, (ff.w2,), (bufs["f"],))
         silu_site = self._step_site(xn, (ff.w1, ff.w3), (g, g)) if self._silu_pair(B, ff) else None
+        scratch = bufs["tc_ws"]
+        if scratch is None and silu_site is not None:
+            scratch = K._tiled_tc_workspace(self.device, B)
+        silu_ws = self._tc_ws_args(scratch)
         for li, layer in enumerate(self.layers):
             att, ff = layer.attention, layer.feed_forward
             if not normed:
@@ -936,7 +938,7 @@ class Transformer(nn.Module):
             else:
                 self._all_reduce(bufs["o"])
                 self._norm(h, bufs["o"], layer.ffn_norm.weight, xn, st)
-            if not self._step_mm(silu_site, (ff.w1, ff.w3), st, True):
+            if not self._step_mm(silu_site, (ff.w1, ff.w3), st, silu_ws):
                 self._gemm_multi(bufs, xn, [ff.w1, ff.w3], [bufs["a1"], bufs["a3"]], st)
                 check(lib.q40_silu_mul(bufs["a1"].data_ptr(), bufs["a3"].data_ptr(), g.data_ptr(), g.numel(), st),
                       "q40_silu_mul")
