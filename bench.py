@@ -406,8 +406,8 @@ def reference_class_on_drop_in(model, dev, steps=16):
 def gemv_roofline(model, width, reps):
     """The dominant kernel alone: every Q4_0 matmul of the model in layer order (3.4 GB of
     distinct weights per pass, so nothing is served from L2), launched exactly as a decode step
-    launches them (for width <= 16 the cluster-reduced kernel, [wq,wk,wv] and [w1,w3] sharing a
-    launch) but with nothing in between, replayed from a CUDA graph so that the host does not
+    of up to 8 branches launches them (the cluster-reduced kernel, [wq,wk,wv] and [w1,w3] sharing a
+    launch; replayed for up to 16, where steps have the tensor-core kernel) but with nothing in between, replayed from a CUDA graph so that the host does not
     pace the launches; CUDA events around the replays on the replaying stream."""
     import torch
     from spec_mcts_b200 import kernels as K

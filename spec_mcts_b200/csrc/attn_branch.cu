@@ -36,13 +36,6 @@ __device__ __forceinline__ int key_slot(const BranchArgs& a, const void* row, in
   return min(min(max(id, 0), a.last_page) * a.page_size + in, a.P - 1);
 }
 
-// 2^x as the hardware gives it: exp2f without its detour for results below 2^-126, which are nothing beside a row's largest, 1
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // acc + a.x b.x + a.y b.y: the products of fp16 values are exact, each sum rounds once
 __device__ __forceinline__ float dot2(__half2 a, __half2 b, float acc) {
   asm("{\n\t.reg .b16 a0, a1, b0, b1;\n\tmov.b32 {a0, a1}, %1;\n\tmov.b32 {b0, b1}, %2;\n\t"

@@ -8,6 +8,13 @@ constexpr int ATTN_D = 128;  // head dim of every supported model (CodeLlama 7B/
 
 inline float attn_scale_log2(int D) { return (1.0f / sqrtf((float)D)) * 1.4426950408889634f; }
 
+// 2^x by the approximate instruction; results below 2^-126, which are nothing beside a row's largest weight, 1, become 0
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 struct BranchArgs {
   const __half* q;        // branch b, head h at q + b*q_stride + h*D
   int64_t q_stride;

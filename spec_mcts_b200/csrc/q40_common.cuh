@@ -37,7 +37,8 @@ static inline cudaError_t q40_allow_smem(std::atomic<uint64_t>& ready, const voi
 }
 
 // Launch with programmatic stream serialization.  Kernels launched this way execute griddepcontrol.wait
-// before their first access to global memory, so for the caller the launch orders exactly like a plain
+// before their first access to global memory (the branch attention behind a prefix pass: before the first to what that
+// pass writes, see attn_branch_kernel), so for the caller the launch orders exactly like a plain
 // one; what changes is that the CTAs may become resident while the previous launch on the stream drains
 // (and, where that launch triggered early, while it runs), which takes the launch latency off the
 // critical path of a chain of small dependent launches.

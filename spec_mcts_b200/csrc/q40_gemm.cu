@@ -389,7 +389,7 @@ gemv_nk_kernel(const __half* __restrict__ X, int64_t ldx, const uint8_t* __restr
     *reinterpret_cast<uint2*>(xs + at) = make_uint2(prmt(x01, x23, 0x5410), prmt(x01, x23, 0x7632));   // x0 x2 | x1 x3
   };
   // Nothing is multiplied before the activations are there: five 16-byte loads of a thread on their way at once, where rows
-  // are aligned to that (10 x 4096 x 11008, 1024 k of 16 rows per CTA in 8-byte loads, one after the other: 20.5 us; so: 18.1;
+  // are aligned to that (10 x 4096 x 11008, 1024 k of 16 rows per CTA in 8-byte loads, one after the other: 20.5 us; so: 18.4;
   // 10 x 4096 x 32000 50.9 and 42.1).  A short piece of few rows is as soon there by single loads, without the set-up of
   // batches and padding (256 k of 10 rows 8.0 us, batches 8.3; 384 k 11.6 and 10.7).  Padding is stored, not rearranged:
   // four rows x 512 x 11008 6.8 us, 7.25 with it going through the rearrangement.

@@ -26,7 +26,7 @@
 //
 // What bounds it, per 128 k of a tile (cycles): up to 96 rows the dequantisers' instructions (460; two thousand issue slots of
 // four schedulers), at 112 and 128 rows the MMAs (500 and 545 with their gaps, 450 and 512 without), above, with all SMs
-// busy, activations from L2 (28 to 33 bytes a cycle and SM).  A launch adds 4 to 5.4 us: set-up and the first stages'
+// busy, loads from L2 (512 rows x 4096 x 11008: 26 bytes a cycle and SM over a launch).  A launch adds 4 to 5.4 us: set-up and the first stages'
 // latency 2, the last accumulator's way out 1 to 2, draining.  Microseconds, here and by the kernels before (one CTA per
 // tile, k split over clusters; up to 16 rows q40_gemv_tiled): 10 rows x 11008 x 4096 13.0 and 16.8, two x 4096 x 11008 16.9 and
 // 22.9; 100 rows x 11008 x 4096 15.7 and 20.8, two x 4096 x 11008 21.8 and 34.1; 512 rows x 4096 x 11008 39.5 and 61.4,

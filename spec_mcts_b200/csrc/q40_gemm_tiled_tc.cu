@@ -1,4 +1,4 @@
-// Q4_0 dequant-matmul for batches above 16 rows on the 5th-generation tensor cores, reading the
+// Q4_0 dequant-matmul for batches above 8 rows on the 5th-generation tensor cores, reading the
 // TILED copy of the weights (the format of q40_gemv_tiled.cu: [span of 256 columns][16 k rows] steps of
 // 2176 contiguous bytes), so that the decode step's wide path and its narrow path share one weight copy.
 //
@@ -19,7 +19,7 @@
 // Every mbarrier wait is bounded: on expiry the kernel records an error code, skips the remaining work, waits (bounded too) for
 // its own copies and MMAs, frees its tensor memory and returns.
 //
-// Replaces matmul_q40_kernel (triton_kernels.py:357-469) for M > 16 when the caller holds tiled weights.
+// Replaces matmul_q40_kernel (triton_kernels.py:357-469) for M > 8 when the caller holds tiled weights.
 #include <cooperative_groups.h>
 
 #include "q40_tc_common.cuh"

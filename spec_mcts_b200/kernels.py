@@ -183,8 +183,8 @@ def matmul_q40(a: torch.Tensor, b_w: torch.Tensor, b_s: torch.Tensor, b_shape, *
     With N % 256 == 0 the weight is read through a tiled copy that is made the first time a given
     (b_w, b_s) pair of tensors is seen and kept while those tensor objects live and are not written in
     place (the reference's LinearQ4_0 passes the same `.w` / `.s` attributes on every call,
-    hf_model_q40_kv_shared.py:228-236): up to 16 rows by the decode step's tiled kernel, above (with
-    K % 64 == 0) by the tensor-core kernel that writes the dequantised operand to tensor memory.  The copy
+    hf_model_q40_kv_shared.py:228-236): up to 8 rows by the decode step's tiled kernel, above (with
+    K % 64 == 0; else up to 16 rows by the former) by the tensor-core kernel that writes the dequantised operand to tensor memory.  The copy
     doubles the device memory of that weight; `relayout=False` (or relayout_cache_config(enabled=False))
     reads the checkpoint layout instead."""
     dev = _need_cuda(a, b_w, b_s)

@@ -230,7 +230,7 @@ class Transformer(nn.Module):
         self.use_fused = True
         self.use_pdl = True
         self.max_cluster = 16
-        # B <= 16: the fused matmuls read a rearranged ("tiled") copy of each weight, made on first use
+        # the fused matmuls read a rearranged ("tiled") copy of each weight, made on first use
         self.use_tiled = True
         # B > 8 and the prompt pass: the tensor-core matmul that reads the same tiled copies (A operand
         # written to tensor memory); False: B <= 16 as B <= 8, above the tensor-core matmul on the checkpoint layout
@@ -256,7 +256,7 @@ class Transformer(nn.Module):
         self._tc_err_host = torch.zeros(1, dtype=torch.int32).pin_memory()
         self._prompt_unchecked = False
         # the error word of the steps' tensor-core matmuls: host memory that they can write, so that nothing has to be copied
-        # (a copy behind each step: 12 us of one of 100 branches)
+        # (a copy behind each step: 11 us of one of 10 branches)
         self._step_err = HostWord()
         # ... True: through the byte-balanced stream-K launch (one CTA per SM, bulk-copy ring, no clusters);
         # False: the cluster-reduced launch on the same tiled copies (faster on B200, the default)
