@@ -29,7 +29,7 @@
 // busy, loads from L2 (512 rows x 4096 x 11008: 26 bytes a cycle and SM over a launch).  A launch adds 4 to 5.4 us: set-up and the first stages'
 // latency 2, the last accumulator's way out 1 to 2, draining.  Microseconds, here and by the kernels before (one CTA per
 // tile, k split over clusters; up to 16 rows q40_gemv_tiled): 10 rows x 11008 x 4096 13.0 and 16.8, two x 4096 x 11008 16.9 and
-// 22.9; 100 rows x 11008 x 4096 15.7 and 20.8, two x 4096 x 11008 21.8 and 34.1; 512 rows x 4096 x 11008 39.5 and 61.4,
+// 22.9; 100 rows x 11008 x 4096 15.7 and 20.8, two x 4096 x 11008 21.8 and 34.1; 512 rows x 4096 x 11008 45.4 and 61.4,
 // three x 4096 x 4096 45.5 and 82.5, x 11008 x 4096 37.2 and 48.6.  With the SiLU product: 10 rows 17.1 (18.8 while w1's and w3's
 // sums met through the other CTA's shared memory), 77 rows 21.9 (23.0), 100 rows 25.0 (27.7), 512 rows 72 (76); expf and the
 // division are half of what it costs (100 rows: 22.6 with approximate ones).
@@ -769,7 +769,8 @@ static void k_blocks(Params& p, int range) {
 //   a launch          3900 + 12 npad; with shared tiles 3800 + 28 npad more; with k split over the pairs of a cluster 700 more per
 //                     pair, and all of it once per wave of clusters (they are not persistent); a range after the first 16 npad for its sums where the next one's MMAs do not hide it
 // 10 rows x 4096 x 11008, two matrices: 16.8 us shared, 21.9 not, 29.3 split in two; 100 rows x 11008 x 4096: 15.7 split in
-// three, 17.6 in two, 27.5 not; 512 rows x 4096 x 11008: 128-row tiles 41.3, 112 39.5, 176 45.7, 256 57.2.
+// three, 17.6 in two, 27.5 not; 512 rows x 4096 x 11008: 128-row tiles 41.3, 112 39.5, 176 45.4, 256 57.2: there the
+// estimate, 39.9 for 176 rows and 40.4 for 112, takes the slower one.
 int q40_pair_gemm(int nmat, const void* a, int64_t lda, const void* const* bw_tiled, void* const* c, const int64_t* ldc,
                   const int* n_cols, int M, int K, int ranges, int silu, void* workspace, size_t workspace_bytes, double beat_ns,
                   int* err, int use_pdl, void* stream) {
