@@ -908,7 +908,7 @@ class Transformer(nn.Module):
         silu_site = self._step_site(xn, (ff.w1, ff.w3), (g, g)) if self._silu_pair(B, ff) else None
         scratch = bufs["tc_ws"]
         if scratch is None and silu_site is not None:
-            scratch = K._tiled_tc_workspace(self.device, B)
+            scratch = K._tiled_tc_workspace(h.device, B)
         silu_ws = self._tc_ws_args(scratch)
         for li, layer in enumerate(self.layers):
             att, ff = layer.attention, layer.feed_forward

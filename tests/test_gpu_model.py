@@ -465,6 +465,35 @@ def test_prompt_pass_captured_on_a_fresh_stream():
     assert m.prompt_status() == 0 and torch.equal(m(tok, 40), want[1])
 
 
+def test_step_first_taken_in_a_capture_of_a_model_without_a_device_index():
+    """Its scratch for shared tiles is the capture's; the steps outside of it look theirs up by the stream's device."""
+    from spec_mcts_b200.model import Transformer
+    m = small_random()
+    other = Transformer(m.params, device="cuda")
+    other.load_state_dict(m.state_dict(), assign=True)
+    for a, b in zip(other.layers, m.layers):
+        for x, y in ((a.attention, b.attention), (a.feed_forward, b.feed_forward)):
+            for n, l in y.named_children():
+                getattr(x, n).w, getattr(x, n).s, getattr(x, n).shape = l.w, l.s, l.shape
+    prompt, toks = torch.arange(40, device="cuda").view(1, -1), torch.arange(12, device="cuda").view(-1, 1)
+    side, graph, out = torch.cuda.Stream(), torch.cuda.CUDAGraph(), []
+    for x in (m, other):
+        x.use_cuda_graph = False
+        x(prompt, 0)
+        x.fork(0, 1, 11)
+    want = m(toks, 40).clone()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        with torch.cuda.graph(graph, stream=side):
+            out = other(toks, 40)
+    torch.cuda.current_stream().wait_stream(side)
+    assert other._tc_ws is None and torch.equal(other(toks, 40), want)
+    with torch.inference_mode():
+        out.zero_()
+    graph.replay()
+    assert torch.equal(out, want)
+
+
 def test_widths_share_the_scratch_of_shared_tiles():
     """A further width allocates its activations and no scratch of its own, and widths in turn give the same logits again."""
     from spec_mcts_b200._lib import lib
