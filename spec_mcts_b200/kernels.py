@@ -62,7 +62,9 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 _workspaces: dict = {}
-_outgrown: list = []                # ... whose place a larger one has taken
+_outgrown: list = []                # ... whose place a larger one has taken, and whose address a graph may have
+_SMALL_WORKSPACE = 64 << 20
+_large_in_graphs: set = set()       # keys of larger ones that a capture has used
 _capture_workspaces: dict = {}      # the same keys -> (id of the stream's last capture, buffer made in it)
 
 
@@ -71,10 +73,12 @@ def _workspace(kind: str, dev: torch.device, nbytes: int, zero: bool) -> torch.T
     must start zeroed (the kernels restore that); calls on different streams get
     different buffers so that they may overlap.  One that is made inside a capture serves that capture only: until the
     graph runs it holds nothing, and each replay makes it ready again.  One that is outgrown is not given back, since a graph
-    may have its address; the next is at least twice its size, so that all of these take no more than the last."""
+    may have its address; the next is at least twice its size, so that all of these take no more than the last.  Beyond
+    64 MB it is given back unless a capture has used it (asking that in every call costs small calls 0.3 us)."""
     key = (kind, dev.index, _stream(dev))
     buf = _workspaces.get(key)
-    if buf is None or buf.numel() < nbytes:
+    size = 0 if buf is None else buf.numel()
+    if buf is None or size < nbytes:
         n, make = max(int(nbytes), 1 << 20), torch.zeros if zero else torch.empty
         if torch.cuda.is_current_stream_capturing():
             capture = ctypes.c_uint64()
@@ -84,10 +88,15 @@ def _workspace(kind: str, dev: torch.device, nbytes: int, zero: bool) -> torch.T
                 buf = make(n, dtype=torch.uint8, device=dev)
                 _capture_workspaces[key] = (capture.value, buf)
             return buf
-        if buf is not None:
+        if buf is not None and size <= _SMALL_WORKSPACE:
             _outgrown.append(buf)
-            n = max(n, 2 * buf.numel())
+            n = max(n, 2 * size)
+        elif key in _large_in_graphs:
+            _outgrown.append(buf)
+            _large_in_graphs.discard(key)
         buf = _workspaces[key] = make(n, dtype=torch.uint8, device=dev)
+    elif size > _SMALL_WORKSPACE and torch.cuda.is_current_stream_capturing():
+        _large_in_graphs.add(key)
     return buf
 
 

@@ -300,6 +300,18 @@ def test_outgrown_scratch_is_not_given_back(launches, monkeypatch):
         del buf
     sizes = [r().numel() for r in seen]
     assert sum(sizes[:-1]) <= sizes[-1] and len(sizes) == 5
+    # beyond what is always held: given back, unless a capture has used it
+    capturing = [False]
+    monkeypatch.setattr(K, "_SMALL_WORKSPACE", 1 << 20)
+    monkeypatch.setattr(K, "_large_in_graphs", set())
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing[0])
+    for used, n in ((False, 81 << 20), (True, 82 << 20), (False, 83 << 20)):
+        old = seen[-1]
+        capturing[0] = used
+        get(4096)
+        capturing[0] = False
+        seen.append(weakref.ref(get(n)))
+        assert (old() is not None) == used and seen[-1]().numel() == n
 
 
 @pytest.mark.parametrize("dev", [None, "cuda", "cuda:1"])
