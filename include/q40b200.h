@@ -352,6 +352,27 @@ int q40_attn_tree_fused(void* qkv, int64_t W, const void* pk, const void* pv, vo
                         const void* sin_tbl, int n_pos, void* ao, int B, int H, int Hkv, int D, int max_t,
                         int max_p, int use_pdl, void* stream);
 
+/* All layers of a decode step of B = 1 or 2 branches as one launch: embedding rows of tok[b] (ids clamped to the
+ * vocabulary), then per layer RMSNorm, q/k/v, rotary embedding, Q4_0 append, attention over prompt and suffix, wo, residual,
+ * RMSNorm, SiLU(w1) * w3, w2, residual, all with the reference's rounding points of activations; h_out [B, dim] is the residual
+ * stream after the last layer and ss_out[b] its sum of squares (what q40_lm_head takes).  Head size 128.
+ *
+ * `layers` (device memory, L records of 16 addresses, int64): tiled copies (q40_relayout_tiled) of wq, wk, wv, wo, w1, w3, w2,
+ * the fp16 weights of the two norms (8-byte aligned), prompt keys and values [max_p, Hkv, 128], suffix codes and scales of the
+ * keys, then of the values (as in q40_attn_tree_fused), 0.  Everything they address was complete before this launch.
+ *
+ * A cooperative launch of one CTA per SM in clusters of four that wait for one another through `workspace`:
+ * q40_decode_chain_ws_bytes bytes, zeroed before the first call and left ready for the next one; one workspace per stream of calls.
+ * The bytes are 0, and the call Q40_E_UNSUPPORTED, where the sizes do not suit (every matmul needs as many 64-column groups as there
+ * are clusters, 33 on a B200; dim <= 4096; dim, hid and the widths of q and k multiples of 256) or the device takes no such launch.
+ * Waits are bounded: on expiry *err (may be mapped host memory) is set, results and workspace are undefined.
+ * Replaces: the layer loop of Transformer.forward (hf_model_q40_kv_shared.py:303-409, 431-436, 456-466, 505-510). */
+size_t q40_decode_chain_ws_bytes(int B, int L, int dim, int hid, int H, int Hkv);
+int q40_decode_chain(const void* layers, int L, int B, int dim, int hid, int H, int Hkv, const int64_t* tok,
+                     const void* emb, int vocab, const int32_t* pos, const int32_t* prefix_len, const void* cos_tbl,
+                     const void* sin_tbl, int n_pos, int max_t, int max_p, float eps, void* h_out, float* ss_out,
+                     void* workspace, size_t workspace_bytes, int* err, void* stream);
+
 /* Rotary embedding of the new token's q [B, H*D] and k [B, Hkv*D] in place (position
  * pos_dev[b], tables cos/sin [n_pos, D/2] fp16) and Q4_0 append of the rotated k and of v to
  * the suffix cache at slot (b, pos_dev[b] - *prefix_len_dev); k and v stay un-quantised in

@@ -329,9 +329,9 @@ __global__ void __launch_bounds__(THREADS, MT == 1 ? 2 : 1) gemv_stream_kernel(c
           const uint32_t v = wds[jt];
           // nibble -> fp16 value 72 + code (see q40_gemv_tiled.cu)
           const uint32_t a0 = lop3_and_xor(v, 0x00F000F0u, 0x54805480u);
-          const uint32_t a1 = lop3_and_xor(v << 4, 0x00F000F0u, 0x54805480u);
+          const uint32_t a1 = lop3_and_xor(v << 4, 0x00F000F0u, 0x54005400u);
           const uint32_t a2 = lop3_and_xor(v >> 8, 0x00F000F0u, 0x54805480u);
-          const uint32_t a3 = lop3_and_xor(v >> 4, 0x00F000F0u, 0x54805480u);
+          const uint32_t a3 = lop3_and_xor(v >> 4, 0x00F000F0u, 0x54005400u);
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt) mma16816(acc[mt][q * 4 + jt], a0, a1, a2, a3, yb[mt][0], yb[mt][1]);
         }

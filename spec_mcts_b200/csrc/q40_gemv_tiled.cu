@@ -10,7 +10,9 @@
 //     4 groups of 64 columns x 32 lanes x 16 bytes   one 32-bit word per 16x16 MMA tile and lane,
 //                                                    nibbles placed so that four mask operations
 //                                                    (three after a shift) yield the four A-fragment
-//                                                    registers of mma.m16n8k16 as fp16 values 72 + code
+//                                                    registers of mma.m16n8k16 as fp16 values 72 + code; a high
+//                                                    nibble is the code, a low one code + 8, so that a byte, as a
+//                                                    signed number, is 16 code + (other code + 8)
 //     4 groups x 16 fp16 scales                      the scales of the 16 k rows
 // The scale is applied to the activations instead of the weights (B operand = fp16(scale * x),
 // one multiply per k and group instead of one per weight), and the constant 72 is removed exactly
@@ -301,11 +303,12 @@ gemv_tiled_kernel(const TiledParams p) {
 #pragma unroll
       for (int jt = 0; jt < 4; ++jt) {
         const uint32_t v = wds[jt];
-        // nibble -> fp16 value 72 + code: bits 4..7 of each 16-bit half under exponent 0x5400, sign bit flipped
+        // nibble -> fp16 value 72 + code: bits 4..7 of each 16-bit half under exponent 0x5400, sign bit flipped (of the low
+        // nibbles it is so already)
         const uint32_t a0 = lop3_and_xor(v, 0x00F000F0u, 0x54805480u);          // column g,   k 4t, 4t+1
-        const uint32_t a1 = lop3_and_xor(v << 4, 0x00F000F0u, 0x54805480u);     // column g+8, k 4t, 4t+1
+        const uint32_t a1 = lop3_and_xor(v << 4, 0x00F000F0u, 0x54005400u);     // column g+8, k 4t, 4t+1
         const uint32_t a2 = lop3_and_xor(v >> 8, 0x00F000F0u, 0x54805480u);     // column g,   k 4t+2, 4t+3
-        const uint32_t a3 = lop3_and_xor(v >> 4, 0x00F000F0u, 0x54805480u);     // column g+8, k 4t+2, 4t+3
+        const uint32_t a3 = lop3_and_xor(v >> 4, 0x00F000F0u, 0x54005400u);     // column g+8, k 4t+2, 4t+3
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt) f_mma(acc[mt][q * 4 + jt], a0, a1, a2, a3, yb[mt][0], yb[mt][1]);
       }
@@ -602,12 +605,12 @@ relayout_kernel(const uint8_t* __restrict__ bw, const __half* __restrict__ bs, u
 #pragma unroll
       for (int lo = 0; lo < 2; ++lo) {
         // byte 0 = k + 0, byte 1 = k + 2, byte 2 = k + 1, byte 3 = k + 3; column g in the high nibble, g + 8 in the low
-        uint32_t word = 0;
+        uint32_t word = 0x08080808u;      // low nibbles: code + 8
 #pragma unroll
         for (int y = 0; y < 4; ++y) {
           const int kk = (y & 1) * 2 + (y >> 1);
           const uint32_t na = (a[kk] >> (8 * c + (lo ? 0 : 4))) & 0xF, nb = (b[kk] >> (8 * c + (lo ? 0 : 4))) & 0xF;
-          word |= (nb | (na << 4)) << (8 * y);
+          word ^= (nb | (na << 4)) << (8 * y);
         }
         const int q = blk * 2 + lo, lane = (g0 + c) * 4 + t;
         *reinterpret_cast<uint32_t*>(out_s + st * T_STEP_BYTES + (q * 32 + lane) * 16 + jt * 4) = word;

@@ -98,13 +98,13 @@ __device__ __forceinline__ void dequant_step(const unsigned char* w, const unsig
   for (int j2 = 0; j2 < 2; ++j2) {
     const uint32_t v = wds[j2];
     // bits 4..7 of a 16-bit half under the exponent of 64: 72 + code; bits 0..3 under that of 1024: 1032 + code (the
-    // sign bit of the code flipped).  One shift a word instead of three
-    constexpr uint32_t HI = 0x54805480u, LO = 0x64086408u;
+    // sign bit of the code flipped; in the low nibbles of a copy it is so already).  One shift a word instead of three
+    constexpr uint32_t HI = 0x54805480u, LO = 0x64086408u, LO_EXP = 0x64006400u;
     const uint32_t v8 = v >> 8;
     r[j2][4 * st + 0] = deq_pair<HI>(lop3_and_xor(v, 0x00F000F0u, HI), s01);      // row g,     k + 0, 1: column 8 st + 2t
     r[j2][4 * st + 1] = deq_pair<HI>(lop3_and_xor(v8, 0x00F000F0u, HI), s23);     // row g,     k + 2, 3: column 8 st + 2t + 1
-    r[j2][4 * st + 2] = deq_pair<LO>(lop3_and_xor(v, 0x000F000Fu, LO), s01);      // row g + 8, column 8 st + 2t
-    r[j2][4 * st + 3] = deq_pair<LO>(lop3_and_xor(v8, 0x000F000Fu, LO), s23);     // row g + 8, column 8 st + 2t + 1
+    r[j2][4 * st + 2] = deq_pair<LO>(lop3_and_xor(v, 0x000F000Fu, LO_EXP), s01);      // row g + 8, column 8 st + 2t
+    r[j2][4 * st + 3] = deq_pair<LO>(lop3_and_xor(v8, 0x000F000Fu, LO_EXP), s23);     // row g + 8, column 8 st + 2t + 1
   }
 }
 

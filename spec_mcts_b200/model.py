@@ -273,6 +273,10 @@ class Transformer(nn.Module):
         # ... and while prompt + suffix fit in two register batches of its clusters (640 keys each);
         # longer contexts go through the tensor-core prefix pass
         self.fused_attn_max_keys = 1280
+        # ... and all layers of a step of up to two branches as one launch, while the same limit holds
+        self.use_chain = True
+        self._chain_tables = {}     # its layers' addresses, as the kernel reads them
+        self._chained = {}          # by width: whether the last step that was enqueued (or captured) was such a launch
         self._lm_head_q4 = None     # set by quantize_lm_head()
 
     # ------------------------------------------------------------------ reference API
@@ -304,6 +308,7 @@ class Transformer(nn.Module):
         captured its work is alive: call this before torch.distributed.destroy_process_group()."""
         torch.cuda.synchronize(self.device)
         self._graphs.clear()
+        self._chain_tables.clear()
 
     # ------------------------------------------------------------------ prompt
     def _prefill(self, tokens):
@@ -487,6 +492,8 @@ class Transformer(nn.Module):
         torch.cuda.synchronize(self.device)
         for bufs in self._bufs.values():
             bufs["gemm_ws"].zero_()
+            if "chain_ws" in bufs:
+                bufs["chain_ws"].zero_()
         if self._tc_ws is not None:
             self._tc_ws[:K._TILED_TC_FLAGS].zero_()
         torch.cuda.synchronize(self.device)
@@ -783,8 +790,52 @@ class Transformer(nn.Module):
         return (self.use_fused_attn and B <= self.fused_attn_max_width and
                 p.max_prompt_seq_len + p.max_seq_len <= self.fused_attn_max_keys)
 
+    def _chain_ws_bytes(self, B):
+        """Bytes of scratch of the launch that does all layers of a step of B branches, or 0 where a step is a chain of launches."""
+        p = self.params
+        if not (self.use_chain and self.use_tiled and not self.use_stream and self.use_fused_attn and B <= 2 and
+                self.tp_world == 1 and p.max_prompt_seq_len + p.max_seq_len <= self.fused_attn_max_keys):
+            return 0
+        return lib.q40_decode_chain_ws_bytes(B, p.n_layers, p.dim, self.layers[0].feed_forward.hidden_dim, self._H, self._Hkv)
+
+    def _chain(self, B, bufs, st):
+        """Enqueue all layers of a step as one launch: bufs["h"] and the sums of squares in bufs["ss_ffn"], one per row, as the
+        last layer leaves them.  False, and nothing is enqueued, where that cannot be."""
+        nbytes = self._chain_ws_bytes(B)
+        if nbytes == 0:
+            return False
+        p, hid = self.params, self.layers[0].feed_forward.hidden_dim
+        H, Hkv = self._H, self._Hkv
+        shapes = [(p.dim, H * 128), (p.dim, Hkv * 128), (p.dim, Hkv * 128), (H * 128, p.dim), (p.dim, hid), (p.dim, hid), (hid, p.dim)]
+        for layer in self.layers:
+            norms = (layer.attention_norm.weight, layer.ffn_norm.weight)
+            if (any(l.group_size != 64 or l.kn() != kn for l, kn in zip(_projections(layer), shapes)) or
+                    any(w.dtype != DTYPE or not w.is_contiguous() or w.data_ptr() % 8 for w in norms)):
+                return False
+        rows = []
+        for layer in self.layers:
+            att = layer.attention
+            tensors = (*self._tiled_of(_projections(layer))[0], layer.attention_norm.weight, layer.ffn_norm.weight, att.cache_prompt_k,
+                       att.cache_prompt_v, att.cache_k, att.cache_k_s, att.cache_v, att.cache_v_s)
+            rows.append([t.data_ptr() for t in tensors] + [0])
+        key = tuple(a for r in rows for a in r)
+        table, ws = self._chain_tables.get(key), bufs.get("chain_ws")
+        if table is None or ws is None:
+            if torch.cuda.is_current_stream_capturing():
+                return False                      # neither may be made inside a graph
+            table = self._chain_tables[key] = torch.tensor(rows, dtype=torch.int64).to(self.device)
+            if ws is None:
+                ws = bufs["chain_ws"] = torch.zeros(nbytes, dtype=torch.uint8, device=self.device)
+        check(lib.q40_decode_chain(table.data_ptr(), p.n_layers, B, p.dim, hid, H, Hkv, self._tok_dev.data_ptr(),
+                                   self.tok_embeddings.weight.data_ptr(), p.vocab_size, self._pos_dev.data_ptr(),
+                                   self._prefix_len_dev.data_ptr(), self._cos.data_ptr(), self._sin.data_ptr(), self._n_pos,
+                                   p.max_seq_len, p.max_prompt_seq_len, float(p.norm_eps), bufs["h"].data_ptr(),
+                                   bufs["ss_ffn"].data_ptr(), ws.data_ptr(), ws.numel(), self._step_err.ptr, st),
+              "q40_decode_chain")
+        return True
+
     def _decode_body_fused(self, B):
-        """Decode step for B <= 8 branches (16: see `_fused_body`): 7 launches per layer (qkv with RMSNorm prologue,
+        """Decode step for B <= 8 branches (16: see `_fused_body`): one launch for all layers (see `_chain`), or 7 per layer (qkv with RMSNorm prologue,
         rope+append, 2 attention, wo with residual epilogue, w1/w3 with RMSNorm prologue and
         SiLU-mul epilogue, w2 with residual epilogue), chained with programmatic dependent launch."""
         p, bufs = self.params, self._step_buffers(B)
@@ -800,9 +851,13 @@ class Transformer(nn.Module):
         W = (H + 2 * Hkv) * D
         q, k, v = qkv[:, :H * D], qkv[:, H * D:(H + Hkv) * D], qkv[:, (H + Hkv) * D:]
         pos, plen, aws = self._pos_dev, self._prefix_len_dev, bufs["attn_ws"]
-        check(lib.q40_embed_rows(self.tok_embeddings.weight.data_ptr(), self._tok_dev.data_ptr(), h.data_ptr(),
-                                 ss_ffn.data_ptr(), c_ffn, B, p.dim, p.vocab_size, st), "q40_embed_rows")
-        for layer in self.layers:
+        chained = self._chained[B] = self._chain(B, bufs, st)
+        if chained:
+            c_ffn = 1
+        else:
+            check(lib.q40_embed_rows(self.tok_embeddings.weight.data_ptr(), self._tok_dev.data_ptr(), h.data_ptr(),
+                                     ss_ffn.data_ptr(), c_ffn, B, p.dim, p.vocab_size, st), "q40_embed_rows")
+        for layer in () if chained else self.layers:
             att, ff = layer.attention, layer.feed_forward
             self._fused(1, [att.wq, att.wk, att.wv], [q, k, v], W, h, p.dim, B,
                         norm_w=layer.attention_norm.weight, ss_in=ss_ffn, ss_in_count=c_ffn, st=st, bufs=bufs)
@@ -1017,10 +1072,13 @@ class Transformer(nn.Module):
         per_layer = (5 if self._fused_attn_for(B) else 7) if fused else (9 if self._silu_pair(B, self.layers[0].feed_forward) else 10)
         self.launches_per_step = self.params.n_layers * per_layer + (2 if self._narrow(B) else 1)
         if not self.use_cuda_graph:
-            return self._decode_body(B)
+            logits = self._decode_body(B)
+            if fused and self._chained.get(B):
+                self.launches_per_step = 2
+            return logits
         key = (B, self.greedy_feedback, self.use_fused, self.use_pdl, self.max_cluster, self.use_stream,
                self.use_tiled, self.use_fused_attn, self.fused_attn_max_width, self.stream_smem_budget,
-               self.use_fused_tail, self.use_tiled_tc, self.use_tp_fused_allreduce)
+               self.use_fused_tail, self.use_tiled_tc, self.use_tp_fused_allreduce, self.use_chain)
         g = self._graphs.get(key)
         if g is None:
             # torch requires capture on a side stream after a warm-up run; with greedy feedback that run
@@ -1038,7 +1096,7 @@ class Transformer(nn.Module):
                     self.max_cluster = 8
                     key = (B, self.greedy_feedback, self.use_fused, self.use_pdl, self.max_cluster, self.use_stream,
                            self.use_tiled, self.use_fused_attn, self.fused_attn_max_width, self.stream_smem_budget,
-                           self.use_fused_tail, self.use_tiled_tc, self.use_tp_fused_allreduce)
+                           self.use_fused_tail, self.use_tiled_tc, self.use_tp_fused_allreduce, self.use_chain)
                     self._decode_body(B)
             torch.cuda.current_stream(self.device).wait_stream(s)
             torch.cuda.synchronize(self.device)
@@ -1051,6 +1109,8 @@ class Transformer(nn.Module):
                 self._pos_dev[:B] -= 1
                 self._tok_dev[:B].copy_(tok_saved)
         g.replay()
+        if fused and self._chained.get(B):
+            self.launches_per_step = 2
         if self._lm_head_q4 is not None and fused:      # only narrow steps compute with it
             return self._bufs[B]["logits_pad"][:, :self.params.vocab_size]
         return self._bufs[B]["logits"]
