@@ -636,6 +636,9 @@ extern "C" int q40_gemm_kn(const void* a, int64_t lda, const void* bw, const voi
   return Q40_OK;
 }
 
+// q40_linear.cu
+int q40_linear(const void* x, int64_t ldx, const void* wq, const void* ws, void* y, int64_t ldy, int M, int N, int K, void* stream);
+
 template <int G, int MT>
 static int launch_gemv_nk(const __half* x, int64_t ldx, const uint8_t* wq, const __half* ws, __half* y,
                           int64_t ldy, int M, int N, int K, void* workspace, cudaStream_t st) {
@@ -682,6 +685,10 @@ extern "C" int q40_gemm_nk(const void* x, int64_t ldx, const void* wq, const voi
   cudaStream_t st = (cudaStream_t)stream;
   const __half* xh = (const __half*)x;
   __half* yh = (__half*)y;
+  if (group == 64) {
+    const int rc = q40_linear(x, ldx, wq, ws, y, ldy, M, N, K, stream);
+    if (rc != Q40_E_UNSUPPORTED) return rc;
+  }
   for (int m0 = 0; m0 < M;) {
     const int mc = q40::nk_launch_rows(N, K, M - m0);
     auto run = [&](auto launch) {
