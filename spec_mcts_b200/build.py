@@ -11,12 +11,15 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 BUILD = os.path.join(PKG_DIR, "build")
 LIB = os.path.join(PKG_DIR, "libq40b200.so")
+HOST_SRC = os.path.join(CSRC, "host_calls.cpp")          # Python extension: see there
+HOST = os.path.join(PKG_DIR, "_host_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -42,7 +45,7 @@ def _sources_digest() -> str:
     """Content hash of everything the library is built from (file times do not survive a
     copy of the tree to another machine, contents do)."""
     import hashlib
-    files = sources() + sorted(glob.glob(os.path.join(CSRC, "*.cuh"))) + \
+    files = sources() + [HOST_SRC] + sorted(glob.glob(os.path.join(CSRC, "*.cuh"))) + \
         sorted(glob.glob(os.path.join(PKG_DIR, "..", "include", "*.h")))
     h = hashlib.sha256(" ".join(NVCC_FLAGS).encode())
     for f in files:
@@ -52,9 +55,23 @@ def _sources_digest() -> str:
 
 
 def needs_build() -> bool:
-    if not os.path.exists(LIB) or not os.path.exists(STAMP):
+    if not (os.path.exists(LIB) and os.path.exists(HOST) and os.path.exists(STAMP)):
         return True
     return open(STAMP).read().strip() != _sources_digest()
+
+
+def _build_host() -> None:
+    import torch
+    t = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I" + os.path.join(t, "include"),
+           "-I" + os.path.join(t, "include", "torch", "csrc", "api", "include"), "-I" + sysconfig.get_paths()["include"],
+           "-I" + os.path.join(cuda, "include"), HOST_SRC, "-o", HOST, "-L" + os.path.join(t, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu",
+           "-ltorch", "-ltorch_python"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"building {HOST_SRC} failed:\n{r.stdout}\n{r.stderr}")
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -84,6 +101,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    _build_host()
     with open(STAMP, "w") as f:
         f.write(_sources_digest())
     return LIB

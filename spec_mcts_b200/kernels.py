@@ -15,7 +15,10 @@ from typing import Optional, Sequence
 
 import torch
 
+from . import _host_calls
 from ._lib import Q40Error, check, lib
+
+_host_calls.init(*[ctypes.cast(f, ctypes.c_void_p).value for f in (lib.q40_matmul_tiled, lib.q40_gemm_nk)])
 
 DTYPE_torch = torch.float16
 GROUP_SIZE = 64
@@ -196,6 +199,12 @@ def matmul_q40(a: torch.Tensor, b_w: torch.Tensor, b_s: torch.Tensor, b_shape, *
     K % 64 == 0; else up to 16 rows by the former) by the tensor-core kernel that writes the dequantised operand to tensor memory.  The copy
     doubles the device memory of that weight; `relayout=False` (or relayout_cache_config(enabled=False))
     reads the checkpoint layout instead."""
+    if out is None and relayout is None and group_size == 64 and _relayout_cfg["enabled"]:
+        ent = _relayout_cache.get(id(b_w))
+        if ent is not None:
+            c = _host_calls.matmul(a, b_w, b_s, b_shape, ent, _cluster_sizes, _workspaces)     # None: not the plain repeated call
+            if c is not None:
+                return c
     dev = _need_cuda(a, b_w, b_s)
     assert a.is_contiguous(), "Matrix A must be contiguous"
     M, K = a.shape
@@ -463,6 +472,9 @@ def linear_q40(x: torch.Tensor, w_q: torch.Tensor, w_s: torch.Tensor, w_shape, *
                group_size: int = GROUP_SIZE):
     """y = x @ deq(W)^T for W [N,K] quantised along K — the fused form of the reference's
     dequantize_q40 + F.linear (quantize.py:235-246, hf_model_q40.py:222-233)."""
+    y = _host_calls.linear(x, w_q, w_s, w_shape, group_size, _workspaces)         # None: not a plain call
+    if y is not None:
+        return y
     dev = _need_cuda(x, w_q, w_s)
     N, K = int(w_shape[0]), int(w_shape[1])
     lead = x.shape[:-1]
