@@ -117,7 +117,7 @@ attn_prefix_kernel(const PrefixArgs a) {
   }
 }
 
-static int prefix_splits(int B, int H, int Hkv, int prefix_len) {
+static int prefix_splits(int B, int H, int Hkv, int prefix_len, int64_t suffix) {
   const int rep = H / Hkv;
   const int rows = B * rep;
   const int rblocks = (rows + 127) / 128;
@@ -125,10 +125,18 @@ static int prefix_splits(int B, int H, int Hkv, int prefix_len) {
   // CTAs per SM to aim for: two for the 64-row variant (128 threads; measured best for 2048 keys x 64
   // rows), one for the 128-row variant; never round up past whole waves (a 149th CTA doubles the time
   // of one SM)
-  const int per_sm = rows <= 64 ? 2 : 1;
+  // ... one, too, where the branches' own keys (`suffix` of a head, about; 0: not known) are so many that the pass is over long before they
+  // are: it then gets by with half of the partials and leaves SMs to them (64 branches of up to 256 own keys behind 512: 34.6 us
+  // with two, 31.4; 34 behind 471 22.2 and 21.4; at four times the prefix no difference, below it one is slower: 10 behind 2048
+  // 16.6 and 18.5; and with fewer than eight tiles: 64 branches of up to 100 behind 300 17.9 and 18.7)
+  const bool hidden = tiles >= 8 && suffix > 6 * (int64_t)prefix_len;
+  const int per_sm = rows <= 64 && !hidden ? 2 : 1;
   int want = (148 * per_sm) / (Hkv * rblocks);
   if (want < 1) want = 1;
   if (want > tiles) want = tiles;
+  // the merge has 16 splits of a row on their way at once and reads further ones one by one (8 kv heads, 2048 keys: 4 branches 11.5 us
+  // with 32 splits, 7.9; 16 branches 17.0 and 13.8)
+  if (want > 16) want = 16;
   if (want < 1) want = 1;
   const int tiles_per = (tiles + want - 1) / want;
   return (tiles + tiles_per - 1) / tiles_per;               // every split is non-empty
@@ -194,7 +202,7 @@ extern "C" int q40_attn_shared_prefix(const void* q, const void* prefix_k, const
   br.scale_log2 = attn_scale_log2(D);
 
   if (prefix_len > 0) {
-    const int nsp = prefix_splits(B, H, Hkv, prefix_len);
+    const int nsp = prefix_splits(B, H, Hkv, prefix_len, (int64_t)B * Lmax / 2);
     const size_t need = (size_t)nsp * rows_total * (D + 2) * sizeof(float);
     if (!workspace || workspace_bytes < need) return Q40_E_WORKSPACE;
     if (!q40_aligned(workspace, 16)) return Q40_E_ALIGN;
@@ -241,7 +249,7 @@ extern "C" int q40_attn_tree_decode(const void* q, int64_t q_stride, const void*
     return Q40_E_ALIGN;
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t rows_total = (int64_t)B * H;
-  const int nsp = prefix_splits(B, H, Hkv, max_prefix_len);
+  const int nsp = prefix_splits(B, H, Hkv, max_prefix_len, 0);
   const size_t need = (size_t)nsp * rows_total * (D + 2) * sizeof(float);
   if (!workspace || workspace_bytes < need) return Q40_E_WORKSPACE;
   if (!q40_aligned(workspace, 16)) return Q40_E_ALIGN;
