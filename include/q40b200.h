@@ -338,6 +338,16 @@ int q40_attn_tree_decode(const void* q, int64_t q_stride, const void* prefix_k, 
                          const void* cur_v, int64_t cur_stride, void* o, int B, int H, int Hkv, int D,
                          void* workspace, size_t workspace_bytes, void* stream);
 
+/* q40_rope_kv_append + q40_attn_tree_decode as the latter's two launches: q [B, H*D] and k [B, Hkv*D] (rows of q_stride and kv_stride elements)
+ * come un-rotated and stay so; the launches rotate what they read (tables [n_pos, D/2] fp16, 16-byte aligned), and the branch pass appends
+ * the rotated key and the value to the cache.  Everything else, and every result, as in the two calls.
+ * Replaces: the decode branch of Attention.forward (hf_model_q40_kv_shared.py:313-317, 330-405). */
+int q40_attn_tree_step(const void* q, int64_t q_stride, const void* k, const void* v, int64_t kv_stride, const void* prefix_k,
+                       const void* prefix_v, int max_prefix_len, const int32_t* prefix_len_dev, int64_t prefix_key_stride,
+                       int64_t prefix_head_stride, void* cache_kq, void* cache_ks, void* cache_vq, void* cache_vs, int max_t,
+                       const int32_t* pos_dev, const void* cos_tbl, const void* sin_tbl, int n_pos, void* o, int B, int H, int Hkv, int D,
+                       void* workspace, size_t workspace_bytes, void* stream);
+
 /* q40_rope_kv_append + q40_attn_tree_decode as one launch for small widths (a cluster of 8 CTAs
  * per (branch, head) splits the keys; no workspace): qkv [B, W] holds the new token's q heads, k
  * heads and v heads (un-rotated, W >= (H + 2 Hkv) * 128); the rotated key and the value are

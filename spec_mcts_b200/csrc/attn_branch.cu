@@ -49,6 +49,12 @@ __device__ __forceinline__ uint32_t load_scales(const __half* p, bool aligned4) 
   return h2_as_u32(__halves2half2(__ldg(p), __ldg(p + 1)));
 }
 
+// Rotary embedding of a lane's 16 dims at branch b's position
+__device__ __forceinline__ void rotate_at(const BranchArgs& a, int b, int sub, uint4& lo, uint4& hi) {
+  const int64_t at = (int64_t)min(max(a.pos[b], 0), a.n_pos - 1) * 64 + 8 * sub;
+  rotate_dims(lo, hi, __ldg(reinterpret_cast<const uint4*>(a.cos_tbl + at)), __ldg(reinterpret_cast<const uint4*>(a.sin_tbl + at)));
+}
+
 template <int MODE, int NW, int WPR, int U>    // U: keys per 8-lane group in flight
 __global__ void __launch_bounds__(NW * 32, U > 2 ? 16 / NW : NW == 8 ? 3 : 5)
 attn_branch_kernel(const BranchArgs a) {
@@ -95,6 +101,7 @@ attn_branch_kernel(const BranchArgs a) {
     *reinterpret_cast<uint4*>(qh) = *reinterpret_cast<const uint4*>(qp);
     *reinterpret_cast<uint4*>(qh + 4) = *reinterpret_cast<const uint4*>(qp + 64);
   }
+  if (MODE == 3 && a.cos_tbl) rotate_at(a, b, sub, *reinterpret_cast<uint4*>(qh), *reinterpret_cast<uint4*>(qh + 4));
   float m = -CUDART_INF_F, l = 0.f, o[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) o[i] = 0.f;
@@ -237,8 +244,17 @@ attn_branch_kernel(const BranchArgs a) {
   if (a.cur_k != nullptr && grp == 0) {
     const __half* kp = a.cur_k + (int64_t)b * a.cur_stride + hk * D + sub * 8;
     const __half* vp = a.cur_v + (int64_t)b * a.cur_stride + hk * D + sub * 8;
-    const uint4 k0 = *reinterpret_cast<const uint4*>(kp), k1 = *reinterpret_cast<const uint4*>(kp + 64);
+    uint4 k0 = *reinterpret_cast<const uint4*>(kp), k1 = *reinterpret_cast<const uint4*>(kp + 64);
     const uint4 v0 = *reinterpret_cast<const uint4*>(vp), v1 = *reinterpret_cast<const uint4*>(vp + 64);
+    if (MODE == 3 && a.cos_tbl) {
+      rotate_at(a, b, sub, k0, k1);
+      const int t = min(max(a.pos[b], 0), a.n_pos - 1) - a.prefix_len[0];
+      if (h % (a.H / a.Hkv) == 0 && t >= 0 && t < a.max_t) {             // the first query head of a kv head
+        const int64_t row = ((int64_t)b * a.max_t + t) * a.Hkv + hk;
+        append_row(k0, k1, const_cast<int8_t*>(a.kq) + row * 64, const_cast<__half*>(a.ksc) + row * 2, sub, 0xffu);
+        append_row(v0, v1, const_cast<int8_t*>(a.vq) + row * 64, const_cast<__half*>(a.vsc) + row * 2, sub, 0xffu);
+      }
+    }
     const __half2* kh0 = reinterpret_cast<const __half2*>(&k0);
     const __half2* kh1 = reinterpret_cast<const __half2*>(&k1);
     float acc = 0.f;

@@ -47,6 +47,11 @@ struct BranchArgs {
   const __half* cur_k;
   const __half* cur_v;
   int64_t cur_stride;
+  // mode 3, optional: q and cur_k come before their rotary embedding (tables [n_pos, 64], 16-byte aligned), which is done here, and the
+  // token's key and value are appended to the cache
+  const __half* cos_tbl;
+  const __half* sin_tbl;
+  int n_pos;
 };
 
 // defined in attn_branch.cu; mode 0 contiguous, 1 paged/int16 ids, 2 paged/int32 ids, 3 Q4_0 cache

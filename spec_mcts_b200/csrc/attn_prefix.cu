@@ -31,10 +31,14 @@ struct PrefixArgs {
   const int32_t* prefix_len_dev;     // optional device scalar overriding prefix_len (<= prefix_len)
   int B, H, Hkv, prefix_len, keys_per_split;
   float scale_log2;
+  const __half* cos_tbl;             // ROT: q is rotated here, at its branch's position
+  const __half* sin_tbl;
+  const int32_t* pos;
+  int n_pos;
 };
 
 // grid: (nsp, Hkv, row blocks); block: NWARPS*32 threads, 16 query rows per warp.
-template <int NWARPS>
+template <int NWARPS, bool ROT>
 __global__ void __launch_bounds__(NWARPS * 32)
 attn_prefix_kernel(const PrefixArgs a) {
   constexpr int D = ATTN_D;
@@ -66,7 +70,7 @@ attn_prefix_kernel(const PrefixArgs a) {
     load_tile<NT>(kdst, kdst + TILE_BYTES, a.pk + off, a.pv + off, a.key_stride, a.key_stride, k_end - key0, tid);
   };
   // ---- Q rows -> shared (swizzled) -> A fragments in registers, with the first tile on its way ----
-  for (int idx = tid; idx < RB * 16; idx += NT) {
+  for (int idx = tid; !ROT && idx < RB * 16; idx += NT) {
     const int r = idx >> 4, ch = idx & 15;
     const int gr = row0 + r;
     const bool ok = gr < rows;
@@ -77,6 +81,24 @@ attn_prefix_kernel(const PrefixArgs a) {
   cp_async_commit();
   if (ntiles > 0) load(0, 0);
   cp_async_commit();
+  if constexpr (ROT) {
+    // eight dims of a row and the eight 64 further
+#pragma unroll
+    for (int i = 0; i < RB * 8 / NT; ++i) {
+      const int idx = tid + i * NT, r = idx >> 3, ch = idx & 7, gr = row0 + r;
+      uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
+      if (gr < rows) {
+        const int b = gr / rep, j = gr % rep;
+        const __half* src = a.q + (int64_t)b * a.q_stride + (hk * rep + j) * D + ch * 8;
+        const int64_t at = (int64_t)min(max(a.pos[b], 0), a.n_pos - 1) * 64 + ch * 8;
+        lo = *reinterpret_cast<const uint4*>(src);
+        hi = *reinterpret_cast<const uint4*>(src + 64);
+        rotate_dims(lo, hi, __ldg(reinterpret_cast<const uint4*>(a.cos_tbl + at)), __ldg(reinterpret_cast<const uint4*>(a.sin_tbl + at)));
+      }
+      *reinterpret_cast<uint4*>(smem + tile_off(r, ch)) = lo;
+      *reinterpret_cast<uint4*>(smem + tile_off(r, ch + 8)) = hi;
+    }
+  }
   cp_async_wait<1>();
   __syncthreads();
   WarpRows w;
@@ -148,15 +170,14 @@ static int launch_prefix(PrefixArgs& pa, int nsp, cudaStream_t st) {
   pa.keys_per_split = ((tiles + nsp - 1) / nsp) * TILE_KEYS;
   const int rep = pa.H / pa.Hkv, rows = pa.B * rep;
   const auto smem = [](int warps) { return (size_t)warps * 16 * TILE_ROW_BYTES + 4 * TILE_BYTES; };      // the Q rows, two stages of K and V
-  static std::atomic<uint64_t> ready[2];
+  const auto launch = [&](std::atomic<uint64_t>& ready, auto kern, int warps) {
+    const cudaError_t e = q40_allow_smem(ready, (const void*)kern, (int)smem(warps));
+    return e != cudaSuccess ? e : q40_launch_pdl(kern, dim3(nsp, pa.Hkv, (rows + warps * 16 - 1) / (warps * 16)), dim3(warps * 32), smem(warps), st, pa);
+  };
+  static std::atomic<uint64_t> ready[4];
   cudaError_t e;
-  if (rows <= 64) {
-    e = q40_allow_smem(ready[0], (const void*)attn_prefix_kernel<4>, (int)smem(4));
-    if (e == cudaSuccess) e = q40_launch_pdl(attn_prefix_kernel<4>, dim3(nsp, pa.Hkv, 1), dim3(128), smem(4), st, pa);
-  } else {
-    e = q40_allow_smem(ready[1], (const void*)attn_prefix_kernel<8>, (int)smem(8));
-    if (e == cudaSuccess) e = q40_launch_pdl(attn_prefix_kernel<8>, dim3(nsp, pa.Hkv, (rows + 127) / 128), dim3(256), smem(8), st, pa);
-  }
+  if (rows <= 64) e = pa.cos_tbl ? launch(ready[0], attn_prefix_kernel<4, true>, 4) : launch(ready[1], attn_prefix_kernel<4, false>, 4);
+  else e = pa.cos_tbl ? launch(ready[2], attn_prefix_kernel<8, true>, 8) : launch(ready[3], attn_prefix_kernel<8, false>, 8);
   if (e != cudaSuccess) return (int)e;
   return Q40_OK;
 }
@@ -225,14 +246,12 @@ extern "C" int q40_attn_shared_prefix(const void* q, const void* prefix_k, const
   return launch_branch(br, mode, B, st);
 }
 
-extern "C" int q40_attn_tree_decode(const void* q, int64_t q_stride, const void* prefix_k, const void* prefix_v,
-                                    int max_prefix_len, const int32_t* prefix_len_dev,
-                                    int64_t prefix_key_stride, int64_t prefix_head_stride,
-                                    const void* cache_kq, const void* cache_ks, const void* cache_vq,
-                                    const void* cache_vs, int max_t, const int32_t* pos_dev,
-                                    const void* cur_k, const void* cur_v, int64_t cur_stride, void* o, int B,
-                                    int H, int Hkv, int D, void* workspace, size_t workspace_bytes,
-                                    void* stream) {
+// cos_tbl != NULL: q and cur_k are rotated and the token is appended (q40_attn_tree_step)
+static int tree_decode(const void* q, int64_t q_stride, const void* prefix_k, const void* prefix_v, int max_prefix_len,
+                       const int32_t* prefix_len_dev, int64_t prefix_key_stride, int64_t prefix_head_stride, const void* cache_kq,
+                       const void* cache_ks, const void* cache_vq, const void* cache_vs, int max_t, const int32_t* pos_dev, const void* cur_k,
+                       const void* cur_v, int64_t cur_stride, const void* cos_tbl, const void* sin_tbl, int n_pos, void* o, int B, int H,
+                       int Hkv, int D, void* workspace, size_t workspace_bytes, void* stream) {
   using namespace q40;
   if (!q || !o || !prefix_k || !prefix_v || !prefix_len_dev || !pos_dev) return Q40_E_NULL;
   if (!cache_kq || !cache_ks || !cache_vq || !cache_vs) return Q40_E_NULL;
@@ -263,9 +282,11 @@ extern "C" int q40_attn_tree_decode(const void* q, int64_t q_stride, const void*
   pa.prefix_len_dev = prefix_len_dev;
   pa.B = B; pa.H = H; pa.Hkv = Hkv; pa.prefix_len = max_prefix_len;
   pa.scale_log2 = attn_scale_log2(D);
+  pa.cos_tbl = (const __half*)cos_tbl; pa.sin_tbl = (const __half*)sin_tbl; pa.n_pos = n_pos; pa.pos = pos_dev;
   int rc = launch_prefix(pa, nsp, st);
   if (rc != Q40_OK) return rc;
   BranchArgs br{};
+  br.cos_tbl = pa.cos_tbl; br.sin_tbl = pa.sin_tbl; br.n_pos = n_pos;
   br.q = (const __half*)q; br.q_stride = q_stride; br.o = (__half*)o;
   br.H = H; br.Hkv = Hkv; br.L = max_t;
   br.scale_log2 = pa.scale_log2;
@@ -275,4 +296,32 @@ extern "C" int q40_attn_tree_decode(const void* q, int64_t q_stride, const void*
   br.pos = pos_dev; br.prefix_len = prefix_len_dev; br.max_t = max_t;
   br.cur_k = (const __half*)cur_k; br.cur_v = (const __half*)cur_v; br.cur_stride = cur_stride;
   return launch_branch(br, 3, B, st);
+}
+
+extern "C" int q40_attn_tree_decode(const void* q, int64_t q_stride, const void* prefix_k, const void* prefix_v,
+                                    int max_prefix_len, const int32_t* prefix_len_dev,
+                                    int64_t prefix_key_stride, int64_t prefix_head_stride,
+                                    const void* cache_kq, const void* cache_ks, const void* cache_vq,
+                                    const void* cache_vs, int max_t, const int32_t* pos_dev,
+                                    const void* cur_k, const void* cur_v, int64_t cur_stride, void* o, int B,
+                                    int H, int Hkv, int D, void* workspace, size_t workspace_bytes,
+                                    void* stream) {
+  return tree_decode(q, q_stride, prefix_k, prefix_v, max_prefix_len, prefix_len_dev, prefix_key_stride, prefix_head_stride, cache_kq,
+                     cache_ks, cache_vq, cache_vs, max_t, pos_dev, cur_k, cur_v, cur_stride, nullptr, nullptr, 0, o, B, H, Hkv, D,
+                     workspace, workspace_bytes, stream);
+}
+
+// A launch of its own for rotation and append (rope_kv_append_kernel), and the wait for it, took 2.5 us a layer and step of 10 branches
+// and 3.8 of 100
+extern "C" int q40_attn_tree_step(const void* q, int64_t q_stride, const void* k, const void* v, int64_t kv_stride, const void* prefix_k,
+                                  const void* prefix_v, int max_prefix_len, const int32_t* prefix_len_dev, int64_t prefix_key_stride,
+                                  int64_t prefix_head_stride, void* cache_kq, void* cache_ks, void* cache_vq, void* cache_vs, int max_t,
+                                  const int32_t* pos_dev, const void* cos_tbl, const void* sin_tbl, int n_pos, void* o, int B, int H,
+                                  int Hkv, int D, void* workspace, size_t workspace_bytes, void* stream) {
+  if (!k || !v || !cos_tbl || !sin_tbl) return Q40_E_NULL;
+  if (n_pos <= 0 || kv_stride < (int64_t)Hkv * D) return Q40_E_SHAPE;
+  if (!q40_aligned(cos_tbl, 16) || !q40_aligned(sin_tbl, 16) || !q40_aligned(cache_ks, 4) || !q40_aligned(cache_vs, 4)) return Q40_E_ALIGN;
+  return tree_decode(q, q_stride, prefix_k, prefix_v, max_prefix_len, prefix_len_dev, prefix_key_stride, prefix_head_stride, cache_kq,
+                     cache_ks, cache_vq, cache_vs, max_t, pos_dev, k, v, kv_stride, cos_tbl, sin_tbl, n_pos, o, B, H, Hkv, D, workspace,
+                     workspace_bytes, stream);
 }

@@ -101,18 +101,6 @@ rope_kv_append_any_kernel(const AppendArgs a) {
 constexpr int AP_THREADS = 128;
 constexpr int AP_UNITS = AP_THREADS / 8;
 
-// dims 8i.. (high nibbles) and 64 + 8i.. (low nibbles) of a head -> 8 packed bytes per lane and the row's two scales
-__device__ __forceinline__ void append_row(const uint4& lo, const uint4& hi, int8_t* codes, __half* scales, int i,
-                                           unsigned gmask) {
-  const uint32_t ew[4] = {lo.x, lo.y, lo.z, lo.w}, ow[4] = {hi.x, hi.y, hi.z, hi.w};
-  __half2 m = quant_max(ew, ow);
-#pragma unroll
-  for (int off = 4; off > 0; off >>= 1) m = __hmax2(m, u32_as_h2(__shfl_xor_sync(gmask, h2_as_u32(m), off)));
-  __half2 sc;
-  *reinterpret_cast<uint2*>(codes + 8 * i) = quant_codes(ew, ow, m, sc);
-  if (i == 0) *reinterpret_cast<__half2*>(scales) = sc;
-}
-
 __global__ void __launch_bounds__(AP_THREADS)
 rope_kv_append_kernel(const AppendArgs a, int units) {
   constexpr int D = 128, HD = 64;
@@ -135,14 +123,7 @@ rope_kv_append_kernel(const AppendArgs a, int units) {
   const int p = min(max(a.pos[b], 0), a.n_pos - 1);
   const uint4 c = *reinterpret_cast<const uint4*>(a.cos_tbl + (int64_t)p * HD + 8 * i);
   const uint4 s = *reinterpret_cast<const uint4*>(a.sin_tbl + (int64_t)p * HD + 8 * i);
-  const __half2 *ch = reinterpret_cast<const __half2*>(&c), *sh = reinterpret_cast<const __half2*>(&s);
-  __half2 *l2 = reinterpret_cast<__half2*>(&lo), *h2 = reinterpret_cast<__half2*>(&hi);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const __half2 x1 = l2[j], x2 = h2[j];
-    l2[j] = __hadd2_rn(__hmul2_rn(x1, ch[j]), __hmul2_rn(__hneg2(x2), sh[j]));
-    h2[j] = __hadd2_rn(__hmul2_rn(x2, ch[j]), __hmul2_rn(x1, sh[j]));
-  }
+  rotate_dims(lo, hi, c, s);
   *reinterpret_cast<uint4*>(px) = lo;
   *reinterpret_cast<uint4*>(px + HD) = hi;
   if (!is_k) return;                      // a query head: rotate only (the eight lanes leave together)

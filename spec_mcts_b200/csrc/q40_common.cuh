@@ -175,6 +175,30 @@ __device__ __forceinline__ uint2 quant_codes(const uint32_t (&ew)[4], const uint
   return make_uint2(out[0], out[1]);
 }
 
+// Rotary embedding of eight dims (lo) and the eight 64 further (hi), with their cosines and sines, in fp16: the reference's roundings
+__device__ __forceinline__ void rotate_dims(uint4& lo, uint4& hi, const uint4& c, const uint4& s) {
+  const __half2 *ch = reinterpret_cast<const __half2*>(&c), *sh = reinterpret_cast<const __half2*>(&s);
+  __half2 *l2 = reinterpret_cast<__half2*>(&lo), *h2 = reinterpret_cast<__half2*>(&hi);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const __half2 x1 = l2[j], x2 = h2[j];
+    l2[j] = __hadd2_rn(__hmul2_rn(x1, ch[j]), __hmul2_rn(__hneg2(x2), sh[j]));
+    h2[j] = __hadd2_rn(__hmul2_rn(x2, ch[j]), __hmul2_rn(x1, sh[j]));
+  }
+}
+
+// dims 8i.. (high nibbles) and 64 + 8i.. (low nibbles) of a head -> 8 packed bytes per lane and the row's two scales
+__device__ __forceinline__ void append_row(const uint4& lo, const uint4& hi, int8_t* codes, __half* scales, int i,
+                                           unsigned gmask) {
+  const uint32_t ew[4] = {lo.x, lo.y, lo.z, lo.w}, ow[4] = {hi.x, hi.y, hi.z, hi.w};
+  __half2 m = quant_max(ew, ow);
+#pragma unroll
+  for (int off = 4; off > 0; off >>= 1) m = __hmax2(m, u32_as_h2(__shfl_xor_sync(gmask, h2_as_u32(m), off)));
+  __half2 sc;
+  *reinterpret_cast<uint2*>(codes + 8 * i) = quant_codes(ew, ow, m, sc);
+  if (i == 0) *reinterpret_cast<__half2*>(scales) = sc;
+}
+
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));

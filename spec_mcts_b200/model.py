@@ -225,16 +225,17 @@ class Transformer(nn.Module):
         # advances the positions on the device, so steps can be replayed without the host
         self.greedy_feedback = False
         # kernels of this library enqueued by one decode step (set by it)
-        self.launches_per_step = params.n_layers * 9 + 1
-        # B <= 8 uses the fused, cluster-reduced, dependent-launch-chained matmuls; up to 16 what `_fused_body` says
+        self.launches_per_step = params.n_layers * 8 + 1
+        # B <= narrow_max uses the fused, cluster-reduced, dependent-launch-chained matmuls; up to 16 what `_fused_body` says
         self.use_fused = True
         self.use_pdl = True
         self.max_cluster = 16
         # the fused matmuls read a rearranged ("tiled") copy of each weight, made on first use
         self.use_tiled = True
-        # B > 8 and the prompt pass: the tensor-core matmul that reads the same tiled copies (A operand
-        # written to tensor memory); False: B <= 16 as B <= 8, above the tensor-core matmul on the checkpoint layout
+        # above, and the prompt pass: the tensor-core matmul that reads the same tiled copies (A operand
+        # written to tensor memory); False: B <= 16 as B <= narrow_max, above the tensor-core matmul on the checkpoint layout
         self.use_tiled_tc = True
+        self.narrow_max = 8
         # tensor parallel: all-reduce + residual add + RMSNorm as one launch over peer-mapped buffers (plain
         # stores into the peers' memory); False: torch.distributed all_reduce + the norm kernel
         self.use_tp_fused_allreduce = True
@@ -474,7 +475,7 @@ class Transformer(nn.Module):
                      ao=e(B, H * D), o=e(B, p.dim), a1=e(B, hid), a3=e(B, hid), g=e(B, hid), f=e(B, p.dim),
                      attn_ws=torch.empty(nb_attn, dtype=torch.uint8, device=dev),
                      gemm_ws=torch.zeros(nb_gemm, dtype=torch.uint8, device=dev),
-                     tc_ws=self._step_tc_ws(B) if B > 8 else None,
+                     tc_ws=self._step_tc_ws(B) if B > self.narrow_max else None,
                      logits=e(B, p.vocab_size), qkv=e(B, (H + 2 * Hkv) * D),
                      ss_attn=torch.zeros((B, 1024), dtype=torch.float32, device=dev),
                      ss_ffn=torch.zeros((B, 1024), dtype=torch.float32, device=dev))
@@ -532,7 +533,7 @@ class Transformer(nn.Module):
         asked, and its arrays made, in every layer, the first step at a width took 16.0 ms for 10 branches and 19.4 for 100
         (now 12.3 and 15.9)."""
         kns = [l.kn() for l in lins]
-        if not (x.shape[0] > 8 and self.use_tiled and self.use_tiled_tc and x.stride(0) % 8 == 0 and
+        if not (x.shape[0] > self.narrow_max and self.use_tiled and self.use_tiled_tc and x.stride(0) % 8 == 0 and
                 all(l.group_size == 64 and self._tileable(l) and kn[0] == x.shape[1] and kn[0] % 64 == 0 and
                     o.stride(0) % 2 == 0 for l, kn, o in zip(lins, kns, outs))):
             return None
@@ -564,7 +565,7 @@ class Transformer(nn.Module):
         """Several projections of the same activations: one tensor-core launch above 8 rows when the
         shapes allow it, one launch per matrix otherwise."""
         M, n = x.shape[0], len(lins)
-        if M > 8 and self.use_tiled and self.use_tiled_tc and x.stride(0) % 8 == 0:
+        if M > self.narrow_max and self.use_tiled and self.use_tiled_tc and x.stride(0) % 8 == 0:
             # matrices that have a tiled copy (N % 256 == 0) go through the tensor-core kernel that reads it;
             # the others (e.g. one kv head per rank under 8-way tensor parallelism) keep the checkpoint layout
             t_idx = [i for i, (l, o) in enumerate(zip(lins, outs))
@@ -620,12 +621,12 @@ class Transformer(nn.Module):
         return self.use_fused and B <= 16 and self.tp_world == 1
 
     def _fused_body(self, B):
-        """Whether a step of B branches takes the narrow matmuls with their fused neighbours.  From 9 branches on the
+        """Whether a step of B branches takes the narrow matmuls with their fused neighbours.  Beyond `narrow_max` the
         tensor-core matmuls make up for two norm launches a layer (10 branches: 2.75 ms a step with the narrow ones), where the
         shapes and switches allow them."""
         if not self._narrow(B):
             return False
-        if B <= 8 or self.use_stream or self._lm_head_q4 is not None or not (self.use_tiled and self.use_tiled_tc):
+        if B <= self.narrow_max or self.use_stream or self._lm_head_q4 is not None or not (self.use_tiled and self.use_tiled_tc):
             return True
         layer = self.layers[0]
         return not all(l.group_size == 64 and self._tileable(l) and l.kn()[0] % 64 == 0 for l in _projections(layer))
@@ -633,7 +634,7 @@ class Transformer(nn.Module):
     def _silu_pair(self, B, ff):
         """Whether w1 and w3 of a step of B branches are one launch with the SiLU product."""
         lins = (ff.w1, ff.w3)
-        return (B > 8 and self.use_tiled and self.use_tiled_tc and lins[0].kn() == lins[1].kn() and
+        return (B > self.narrow_max and self.use_tiled and self.use_tiled_tc and lins[0].kn() == lins[1].kn() and
                 all(l.group_size == 64 and self._tileable(l) and l.kn()[0] % 64 == 0 for l in lins))
 
     def _decode_body(self, B):
@@ -834,9 +835,34 @@ class Transformer(nn.Module):
               "q40_decode_chain")
         return True
 
+    def _rotates_in_attention(self, B):
+        return B * self._H <= 1536
+
+    def _attn_step(self, att, q, k, v, ld, ao, B, ws, st):
+        """Rotary embedding, cache append and attention of a step's new tokens (rows of `ld` values).  Up to 1536 (branch, head) pairs as two
+        launches, prompt and branches; with more of them each would rotate in too many places, and a launch of its own does as well or
+        better.  Us a layer, in three launches and two (32 heads, prompt 512, 64 own keys): 6 branches 68.0 and 64.1, 20 69.2 and
+        68.0, 40 75.1 and 74.0, 50 79.4 and 79.8, 100 100.8 and 101.3."""
+        p, pk, pv = self.params, att.cache_prompt_k, att.cache_prompt_v
+        if not self._rotates_in_attention(B):
+            caches = [t.data_ptr() for t in (att.cache_k, att.cache_k_s, att.cache_v, att.cache_v_s)]
+            pos, plen = self._pos_dev.data_ptr(), self._prefix_len_dev.data_ptr()
+            check(lib.q40_rope_kv_append(q.data_ptr(), ld, k.data_ptr(), ld, v.data_ptr(), ld, pos, plen, self._cos.data_ptr(),
+                                         self._sin.data_ptr(), self._n_pos, *caches, B, self._H, self._Hkv, self._D, p.max_seq_len, st),
+                  "q40_rope_kv_append")
+            check(lib.q40_attn_tree_decode(q.data_ptr(), ld, pk.data_ptr(), pv.data_ptr(), p.max_prompt_seq_len, plen, pk.stride(0),
+                                           pk.stride(1), *caches, p.max_seq_len, pos, k.data_ptr(), v.data_ptr(), ld, ao.data_ptr(), B,
+                                           self._H, self._Hkv, self._D, ws.data_ptr(), ws.numel(), st), "q40_attn_tree_decode")
+            return
+        check(lib.q40_attn_tree_step(q.data_ptr(), ld, k.data_ptr(), v.data_ptr(), ld, pk.data_ptr(), pv.data_ptr(), p.max_prompt_seq_len,
+                                     self._prefix_len_dev.data_ptr(), pk.stride(0), pk.stride(1), att.cache_k.data_ptr(),
+                                     att.cache_k_s.data_ptr(), att.cache_v.data_ptr(), att.cache_v_s.data_ptr(), p.max_seq_len,
+                                     self._pos_dev.data_ptr(), self._cos.data_ptr(), self._sin.data_ptr(), self._n_pos, ao.data_ptr(), B,
+                                     self._H, self._Hkv, self._D, ws.data_ptr(), ws.numel(), st), "q40_attn_tree_step")
+
     def _decode_body_fused(self, B):
-        """Decode step for B <= 8 branches (16: see `_fused_body`): one launch for all layers (see `_chain`), or 7 per layer (qkv with RMSNorm prologue,
-        rope+append, 2 attention, wo with residual epilogue, w1/w3 with RMSNorm prologue and
+        """Decode step for few branches (see `_fused_body`): one launch for all layers (see `_chain`), or 6 per layer (qkv with RMSNorm prologue,
+        2 of attention with rotary embedding and append, wo with residual epilogue, w1/w3 with RMSNorm prologue and
         SiLU-mul epilogue, w2 with residual epilogue), chained with programmatic dependent launch."""
         p, bufs = self.params, self._step_buffers(B)
         H, Hkv, D = self._H, self._Hkv, self._D
@@ -871,18 +897,7 @@ class Transformer(nn.Module):
                                               1 if self.use_pdl else 0, st),
                       "q40_attn_tree_fused")
             else:
-                check(lib.q40_rope_kv_append(q.data_ptr(), W, k.data_ptr(), W, v.data_ptr(), W, pos.data_ptr(),
-                                             plen.data_ptr(), self._cos.data_ptr(), self._sin.data_ptr(), self._n_pos,
-                                             att.cache_k.data_ptr(), att.cache_k_s.data_ptr(),
-                                             att.cache_v.data_ptr(), att.cache_v_s.data_ptr(), B, H, Hkv, D,
-                                             p.max_seq_len, st), "q40_rope_kv_append")
-                pk, pv = att.cache_prompt_k, att.cache_prompt_v
-                check(lib.q40_attn_tree_decode(q.data_ptr(), W, pk.data_ptr(), pv.data_ptr(), p.max_prompt_seq_len,
-                                               plen.data_ptr(), pk.stride(0), pk.stride(1), att.cache_k.data_ptr(),
-                                               att.cache_k_s.data_ptr(), att.cache_v.data_ptr(),
-                                               att.cache_v_s.data_ptr(), p.max_seq_len, pos.data_ptr(), k.data_ptr(),
-                                               v.data_ptr(), W, ao.data_ptr(), B, H, Hkv, D, aws.data_ptr(),
-                                               aws.numel(), st), "q40_attn_tree_decode")
+                self._attn_step(att, q, k, v, W, ao, B, aws, st)
             self._fused(2, [att.wo], [h], p.dim, ao, H * D, B, h_in=h, ldh=p.dim, ss_out=ss_attn,
                         ss_out_count=c_attn, st=st, bufs=bufs)
             self._fused(3, [ff.w1, ff.w3], [gbuf, gbuf], hid, h, p.dim, B, norm_w=layer.ffn_norm.weight,
@@ -948,7 +963,6 @@ class Transformer(nn.Module):
                                      bufs["ss_ffn"].data_ptr(), 1, B, p.dim, p.vocab_size, st), "q40_embed_rows")
         else:
             h.copy_(self.tok_embeddings(self._tok_dev[:B]).to(DTYPE))
-        pos, plen = self._pos_dev, self._prefix_len_dev
         aws = bufs["attn_ws"]
         pending = None     # output of the previous sub-block, added to h by the next norm kernel
         peer = self._tp_peer_buffers() if self.tp_world > 1 and self.use_tp_fused_allreduce else None
@@ -971,20 +985,7 @@ class Transformer(nn.Module):
                 self._norm(h, pending, layer.attention_norm.weight, xn, st)
             if not self._step_mm(q_site, (att.wq, att.wk, att.wv), st):
                 self._gemm_multi(bufs, xn, [att.wq, att.wk, att.wv], [bq, bk, bv], st)
-            check(lib.q40_rope_kv_append(bq.data_ptr(), Wq, bk.data_ptr(), Wq,
-                                         bv.data_ptr(), Wq, pos.data_ptr(), plen.data_ptr(),
-                                         self._cos.data_ptr(), self._sin.data_ptr(), self._n_pos,
-                                         att.cache_k.data_ptr(), att.cache_k_s.data_ptr(),
-                                         att.cache_v.data_ptr(), att.cache_v_s.data_ptr(), B, H, Hkv, D,
-                                         p.max_seq_len, st), "q40_rope_kv_append")
-            pk, pv = att.cache_prompt_k, att.cache_prompt_v
-            check(lib.q40_attn_tree_decode(bq.data_ptr(), Wq, pk.data_ptr(), pv.data_ptr(),
-                                           p.max_prompt_seq_len, plen.data_ptr(), pk.stride(0), pk.stride(1),
-                                           att.cache_k.data_ptr(), att.cache_k_s.data_ptr(),
-                                           att.cache_v.data_ptr(), att.cache_v_s.data_ptr(), p.max_seq_len,
-                                           pos.data_ptr(), bk.data_ptr(), bv.data_ptr(), Wq,
-                                           ao.data_ptr(), B, H, Hkv, D, aws.data_ptr(), aws.numel(), st),
-                  "q40_attn_tree_decode")
+            self._attn_step(att, bq, bk, bv, Wq, ao, B, aws, st)
             if not self._step_mm(o_site, (att.wo,), st):
                 self._gemm_multi(bufs, ao, [att.wo], [bufs["o"]], st)
             if peer is not None:
@@ -1069,7 +1070,9 @@ class Transformer(nn.Module):
         self._check_prompt()
         self._check_steps()
         fused = self._fused_body(B)
-        per_layer = (5 if self._fused_attn_for(B) else 7) if fused else (9 if self._silu_pair(B, self.layers[0].feed_forward) else 10)
+        per_layer = (5 if self._fused_attn_for(B) else 6) if fused else (8 if self._silu_pair(B, self.layers[0].feed_forward) else 9)
+        if not (fused and per_layer == 5 or self._rotates_in_attention(B)):
+            per_layer += 1
         self.launches_per_step = self.params.n_layers * per_layer + (2 if self._narrow(B) else 1)
         if not self.use_cuda_graph:
             logits = self._decode_body(B)
