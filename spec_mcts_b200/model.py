@@ -235,7 +235,10 @@ class Transformer(nn.Module):
         # above, and the prompt pass: the tensor-core matmul that reads the same tiled copies (A operand
         # written to tensor memory); False: B <= 16 as B <= narrow_max, above the tensor-core matmul on the checkpoint layout
         self.use_tiled_tc = True
-        self.narrow_max = 8
+        # steps of more branches than this take it: where a layer's launches, three more of them, have enough to do.  Us a step of 8
+        # layers (prompt 512, 64 own keys), the narrow matmuls and it: dim 4096, 4 branches 534 and 551, 5 565 and 545, 8 608 and 557;
+        # dim 2048, 5 branches 390 and 333; dim 1024, 5 255 and 269, 8 291 and 270; dim 512, 5 212 and 257, 8 233 and 256
+        self.narrow_max = 4 if tp_world == 1 and params.dim >= 2048 else 8
         # tensor parallel: all-reduce + residual add + RMSNorm as one launch over peer-mapped buffers (plain
         # stores into the peers' memory); False: torch.distributed all_reduce + the norm kernel
         self.use_tp_fused_allreduce = True
