@@ -685,11 +685,19 @@ extern "C" int q40_gemm_nk(const void* x, int64_t ldx, const void* wq, const voi
   cudaStream_t st = (cudaStream_t)stream;
   const __half* xh = (const __half*)x;
   __half* yh = (__half*)y;
-  if (group == 64) {
-    const int rc = q40_linear(x, ldx, wq, ws, y, ldy, M, N, K, stream);
-    if (rc != Q40_E_UNSUPPORTED) return rc;
+  int m0 = 0;
+  // 32 rows at a time with one CTA per SM, where the tiles allow it.  Above 32 rows a short k range over many CTAs is the exception, for which
+  // 64 rows a launch keep the SMs busy.  Microseconds by launches of 32 and by the launches below: 64 rows x 2048 x 2048 14.5 and 27.9,
+  // x 4096 x 5500 29.6 and 46.3; 100 rows x 1280 x 9000 30.9 and 57.5, x 3072 x 11008 59.6 and 92.6; 64 rows x 1024 x 6000 13.0 and 14.2, x
+  // 8000 14.5 and 14.0, x 11008 18.3 and 17.3
+  if (group == 64 && (M <= 32 || K > 1152 || N <= 6500)) {
+    for (; m0 < M; m0 += 32) {
+      const int rc = q40_linear(xh + m0 * ldx, ldx, wq, ws, yh + m0 * ldy, ldy, M - m0 < 32 ? M - m0 : 32, N, K, stream);
+      if (rc == Q40_E_UNSUPPORTED) break;
+      if (rc != Q40_OK) return rc;
+    }
   }
-  for (int m0 = 0; m0 < M;) {
+  while (m0 < M) {
     const int mc = q40::nk_launch_rows(N, K, M - m0);
     auto run = [&](auto launch) {
       return launch(xh + m0 * ldx, ldx, (const uint8_t*)wq, (const __half*)ws, yh + m0 * ldy, ldy, mc, N, K, workspace, st);

@@ -1,4 +1,5 @@
-// y[M, N] = x[M, K] @ deq(W)^T for W [N, K] with groups of 64 along K (the layout of quantize_q40 on a Linear weight), up to 32 rows.
+// y[M, N] = x[M, K] @ deq(W)^T for W [N, K] with groups of 64 along K (the layout of quantize_q40 on a Linear weight), up to 32 rows a
+// launch.
 //
 // One CTA per SM: up to five 16-row tiles of W over the whole k range, or, where the activations do not fit shared memory or
 // tiles are few, a cluster of two or four CTAs that share it.  The activations are staged once, W comes straight into the
