@@ -892,5 +892,9 @@ extern "C" int q40_decode_chain(const void* layers, int L, int B, int dim, int h
   cfg.attrs = attr;
   cfg.numAttrs = 2;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {              // a part of the SMs is not this context's
+    (void)cudaGetLastError();
+    return Q40_E_UNSUPPORTED;
+  }
   return e == cudaSuccess ? Q40_OK : (int)e;
 }

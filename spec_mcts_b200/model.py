@@ -830,12 +830,15 @@ class Transformer(nn.Module):
             table = self._chain_tables[key] = torch.tensor(rows, dtype=torch.int64).to(self.device)
             if ws is None:
                 ws = bufs["chain_ws"] = torch.zeros(nbytes, dtype=torch.uint8, device=self.device)
-        check(lib.q40_decode_chain(table.data_ptr(), p.n_layers, B, p.dim, hid, H, Hkv, self._tok_dev.data_ptr(),
-                                   self.tok_embeddings.weight.data_ptr(), p.vocab_size, self._pos_dev.data_ptr(),
-                                   self._prefix_len_dev.data_ptr(), self._cos.data_ptr(), self._sin.data_ptr(), self._n_pos,
-                                   p.max_seq_len, p.max_prompt_seq_len, float(p.norm_eps), bufs["h"].data_ptr(),
-                                   bufs["ss_ffn"].data_ptr(), ws.data_ptr(), ws.numel(), self._step_err.ptr, st),
-              "q40_decode_chain")
+        rc = lib.q40_decode_chain(table.data_ptr(), p.n_layers, B, p.dim, hid, H, Hkv, self._tok_dev.data_ptr(),
+                                  self.tok_embeddings.weight.data_ptr(), p.vocab_size, self._pos_dev.data_ptr(),
+                                  self._prefix_len_dev.data_ptr(), self._cos.data_ptr(), self._sin.data_ptr(), self._n_pos,
+                                  p.max_seq_len, p.max_prompt_seq_len, float(p.norm_eps), bufs["h"].data_ptr(),
+                                  bufs["ss_ffn"].data_ptr(), ws.data_ptr(), ws.numel(), self._step_err.ptr, st)
+        if rc == -5:                              # Q40_E_UNSUPPORTED: the device does not give it all SMs
+            self.use_chain = False
+            return False
+        check(rc, "q40_decode_chain")
         return True
 
     def _rotates_in_attention(self, B):
