@@ -406,8 +406,8 @@ def reference_class_on_drop_in(model, dev, steps=16):
 def gemv_roofline(model, width, reps):
     """The dominant kernel alone: every Q4_0 matmul of the model in layer order (3.4 GB of
     distinct weights per pass, so nothing is served from L2), launched exactly as a decode step
-    of up to 8 branches launches them (the cluster-reduced kernel, [wq,wk,wv] and [w1,w3] sharing a
-    launch; replayed for up to 16, where steps have the tensor-core kernel) but with nothing in between, replayed from a CUDA graph so that the host does not
+    of three or four branches launches them (the cluster-reduced kernel, [wq,wk,wv] and [w1,w3] sharing a
+    launch; one and two branches have one launch for all layers, more than four the tensor-core kernel) but with nothing in between, replayed from a CUDA graph so that the host does not
     pace the launches; CUDA events around the replays on the replaying stream."""
     import torch
     from spec_mcts_b200 import kernels as K
@@ -958,7 +958,12 @@ def main():
             model.use_tiled = False
             sec_ref = timed_decode(model, widths[0], min(steps, 32), warmup, PROMPT_LEN)
             model.use_tiled = True
-            by_path = {"tiled (default)": {"ms_per_step": results[widths[0]] / steps * 1e3},
+            # ... and as a chain of launches, five a layer
+            model.use_chain = False
+            sec_launches = timed_decode(model, widths[0], min(steps, 32), warmup, PROMPT_LEN)
+            model.use_chain = True
+            by_path = {"chain of launches, tiled": {"ms_per_step": sec_launches / min(steps, 32) * 1e3},
+                       "tiled (default)": {"ms_per_step": results[widths[0]] / steps * 1e3},
                        "checkpoint layout, reference operand rounding": {"ms_per_step": sec_ref / min(steps, 32) * 1e3}}
         drop_in = reference_class_on_drop_in(model, dev) if rank == 0 and world == 1 and not args.no_extras else None
         tree_step = tree_step_timing(dev, max(widths)) if rank == 0 and world == 1 and not args.no_extras else None
