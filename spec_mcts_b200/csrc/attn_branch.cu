@@ -27,9 +27,9 @@ namespace q40 {
 
 // Slot of key t of branch b: in the pool (paged), or just t (contiguous).  `row` is the branch's first page id.  (With a division
 // by the page size and 64-bit products per key, slots were a third of a paged row's instructions.)
-template <int MODE>  // 0 contiguous, 1 paged with int16 ids, 2 paged with int32 ids, 3 Q4_0 cache
+template <int MODE>  // 0 contiguous, 1 paged with int16 ids, 2 paged with int32 ids, 3 Q4_0 cache, 4 the same with rotation and append (see BranchArgs)
 __device__ __forceinline__ int key_slot(const BranchArgs& a, const void* row, int t) {
-  if (MODE == 0 || MODE == 3) return t;
+  if (MODE == 0 || MODE >= 3) return t;
   const int pg = a.page_shift >= 0 ? t >> a.page_shift : t / a.page_size, in = t - pg * a.page_size;
   const int id = MODE == 1 ? (int)(uint16_t) reinterpret_cast<const int16_t*>(row)[pg] : reinterpret_cast<const int32_t*>(row)[pg];
   // a bad page id must not turn into a wild read: clamp into the pool
@@ -79,7 +79,7 @@ attn_branch_kernel(const BranchArgs a) {
   const unsigned gmask = 0xffu << (lane & 24);
 
   int len;
-  if (MODE == 3) len = min(max(a.pos[b] - a.prefix_len[0], 0), a.max_t);
+  if (MODE >= 3) len = min(max(a.pos[b] - a.prefix_len[0], 0), a.max_t);
   else len = a.seq_lens ? min(max(a.seq_lens[b], 0), a.L) : a.L;
   // first page ids.  They wait for the length: entries beyond it need not exist (the last row of a table that is a
   // column range of a wider one ends with the allocation).  Ids of every row but the last ahead of the length, by a
@@ -101,14 +101,14 @@ attn_branch_kernel(const BranchArgs a) {
     *reinterpret_cast<uint4*>(qh) = *reinterpret_cast<const uint4*>(qp);
     *reinterpret_cast<uint4*>(qh + 4) = *reinterpret_cast<const uint4*>(qp + 64);
   }
-  if (MODE == 3 && a.cos_tbl) rotate_at(a, b, sub, *reinterpret_cast<uint4*>(qh), *reinterpret_cast<uint4*>(qh + 4));
+  if (MODE == 4) rotate_at(a, b, sub, *reinterpret_cast<uint4*>(qh), *reinterpret_cast<uint4*>(qh + 4));
   float m = -CUDART_INF_F, l = 0.f, o[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) o[i] = 0.f;
 
   // first key of this head and branch, at this lane's dims
   const int64_t kv0 = (MODE == 0 ? (int64_t)(b * a.Hkv + hk) * a.L : (int64_t)hk * a.P) * D + sub * 8;
-  if (MODE != 3)
+  if (MODE < 3)
   for (int t0 = grp; t0 < len; t0 += NG * U) {
     uint4 kv[U][4];
     float s[U];
@@ -165,7 +165,7 @@ attn_branch_kernel(const BranchArgs a) {
     m = mnew;
   }
 
-  if (MODE == 3) {
+  if (MODE >= 3) {
     // Q4_0 cache: lane `sub` owns bytes 8*sub..8*sub+7 of a row, both nibbles; a word's bytes come out as (0, 2) and (1, 3)
     __half2 q4[8];
 #pragma unroll
@@ -246,7 +246,7 @@ attn_branch_kernel(const BranchArgs a) {
     const __half* vp = a.cur_v + (int64_t)b * a.cur_stride + hk * D + sub * 8;
     uint4 k0 = *reinterpret_cast<const uint4*>(kp), k1 = *reinterpret_cast<const uint4*>(kp + 64);
     const uint4 v0 = *reinterpret_cast<const uint4*>(vp), v1 = *reinterpret_cast<const uint4*>(vp + 64);
-    if (MODE == 3 && a.cos_tbl) {
+    if (MODE == 4) {
       rotate_at(a, b, sub, k0, k1);
       const int t = min(max(a.pos[b], 0), a.n_pos - 1) - a.prefix_len[0];
       if (h % (a.H / a.Hkv) == 0 && t >= 0 && t < a.max_t) {             // the first query head of a kv head
@@ -399,7 +399,7 @@ int launch_branch(BranchArgs a, int mode, int B, cudaStream_t st) {
   if (mode == 0) return launch_branch_mode<0>(a, st);
   if (mode == 1) return launch_branch_mode<1>(a, st);
   if (mode == 2) return launch_branch_mode<2>(a, st);
-  return launch_branch_mode<3>(a, st);
+  return a.cos_tbl ? launch_branch_mode<4>(a, st) : launch_branch_mode<3>(a, st);
 }
 
 }  // namespace q40

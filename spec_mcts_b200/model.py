@@ -842,13 +842,14 @@ class Transformer(nn.Module):
         return True
 
     def _rotates_in_attention(self, B):
-        return B * self._H <= 1536
+        return B * self._H <= 1408
 
     def _attn_step(self, att, q, k, v, ld, ao, B, ws, st):
-        """Rotary embedding, cache append and attention of a step's new tokens (rows of `ld` values).  Up to 1536 (branch, head) pairs as two
+        """Rotary embedding, cache append and attention of a step's new tokens (rows of `ld` values).  Up to 1408 (branch, head) pairs as two
         launches, prompt and branches; with more of them each would rotate in too many places, and a launch of its own does as well or
-        better.  Us a layer, in three launches and two (32 heads, prompt 512, 64 own keys): 6 branches 68.0 and 64.1, 20 69.2 and
-        68.0, 40 75.1 and 74.0, 50 79.4 and 79.8, 100 100.8 and 101.3."""
+        better.  Us of a step of 32 layers with 32 heads, in three launches and two a layer, prompt 512 and 64 own keys / 100 and 200:
+        6 branches 2067 and 2026 / 2186 and 2107, 20 2266 and 2215 / 2486 and 2445, 44 2482 and 2435 / 2920 and 2898, 48 2512 and
+        2503 / 2964 and 3003, 64 2703 and 2692 / 3212 and 3198, 100 3218 and 3239 / 3982 and 3990."""
         p, pk, pv = self.params, att.cache_prompt_k, att.cache_prompt_v
         if not self._rotates_in_attention(B):
             caches = [t.data_ptr() for t in (att.cache_k, att.cache_k_s, att.cache_v, att.cache_v_s)]
