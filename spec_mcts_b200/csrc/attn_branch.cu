@@ -15,6 +15,8 @@
 // tail instead of the reference's fp16 state and multiple-of-32 length requirement.
 #include <math_constants.h>
 
+#include <type_traits>
+
 #include "attn_common.cuh"
 
 namespace q40 {
@@ -27,7 +29,7 @@ namespace q40 {
 
 // Slot of key t of branch b: in the pool (paged), or just t (contiguous).  `row` is the branch's first page id.  (With a division
 // by the page size and 64-bit products per key, slots were a third of a paged row's instructions.)
-template <int MODE>  // 0 contiguous, 1 paged with int16 ids, 2 paged with int32 ids, 3 Q4_0 cache, 4 the same with rotation and append (see BranchArgs)
+template <int MODE>  // 0 contiguous, 1 paged with int16 ids, 2 paged with int32 ids, 3 Q4_0 cache, 4 the same with rotation and append (see BranchRotArgs)
 __device__ __forceinline__ int key_slot(const BranchArgs& a, const void* row, int t) {
   if (MODE == 0 || MODE >= 3) return t;
   const int pg = a.page_shift >= 0 ? t >> a.page_shift : t / a.page_size, in = t - pg * a.page_size;
@@ -50,14 +52,17 @@ __device__ __forceinline__ uint32_t load_scales(const __half* p, bool aligned4) 
 }
 
 // Rotary embedding of a lane's 16 dims at branch b's position
-__device__ __forceinline__ void rotate_at(const BranchArgs& a, int b, int sub, uint4& lo, uint4& hi) {
+__device__ __forceinline__ void rotate_at(const BranchRotArgs& a, int b, int sub, uint4& lo, uint4& hi) {
   const int64_t at = (int64_t)min(max(a.pos[b], 0), a.n_pos - 1) * 64 + 8 * sub;
   rotate_dims(lo, hi, __ldg(reinterpret_cast<const uint4*>(a.cos_tbl + at)), __ldg(reinterpret_cast<const uint4*>(a.sin_tbl + at)));
 }
 
+template <int MODE>
+using ModeArgs = std::conditional_t<MODE == 4, BranchRotArgs, BranchArgs>;
+
 template <int MODE, int NW, int WPR, int U>    // U: keys per 8-lane group in flight
 __global__ void __launch_bounds__(NW * 32, U > 2 ? 16 / NW : NW == 8 ? 3 : 5)
-attn_branch_kernel(const BranchArgs a) {
+attn_branch_kernel(const ModeArgs<MODE> a) {
   constexpr int D = ATTN_D;
   constexpr int RT = WPR * 32;                // threads of a row
   constexpr int NG = WPR * 4;                 // key groups of a row
@@ -101,7 +106,7 @@ attn_branch_kernel(const BranchArgs a) {
     *reinterpret_cast<uint4*>(qh) = *reinterpret_cast<const uint4*>(qp);
     *reinterpret_cast<uint4*>(qh + 4) = *reinterpret_cast<const uint4*>(qp + 64);
   }
-  if (MODE == 4) rotate_at(a, b, sub, *reinterpret_cast<uint4*>(qh), *reinterpret_cast<uint4*>(qh + 4));
+  if constexpr (MODE == 4) rotate_at(a, b, sub, *reinterpret_cast<uint4*>(qh), *reinterpret_cast<uint4*>(qh + 4));
   float m = -CUDART_INF_F, l = 0.f, o[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) o[i] = 0.f;
@@ -246,7 +251,7 @@ attn_branch_kernel(const BranchArgs a) {
     const __half* vp = a.cur_v + (int64_t)b * a.cur_stride + hk * D + sub * 8;
     uint4 k0 = *reinterpret_cast<const uint4*>(kp), k1 = *reinterpret_cast<const uint4*>(kp + 64);
     const uint4 v0 = *reinterpret_cast<const uint4*>(vp), v1 = *reinterpret_cast<const uint4*>(vp + 64);
-    if (MODE == 4) {
+    if constexpr (MODE == 4) {
       rotate_at(a, b, sub, k0, k1);
       const int t = min(max(a.pos[b], 0), a.n_pos - 1) - a.prefix_len[0];
       if (h % (a.H / a.Hkv) == 0 && t >= 0 && t < a.max_t) {             // the first query head of a kv head
@@ -352,7 +357,7 @@ attn_branch_kernel(const BranchArgs a) {
 }
 
 template <int MODE, int NW, int WPR, int U>
-static int launch_rows(const BranchArgs& a, cudaStream_t st) {
+static int launch_rows(const ModeArgs<MODE>& a, cudaStream_t st) {
   const unsigned grid = (unsigned)((a.rows + NW / WPR - 1) / (NW / WPR));
   const cudaError_t e = q40_launch_pdl(attn_branch_kernel<MODE, NW, WPR, U>, dim3(grid), dim3(NW * 32), 0, st, a);
   return e == cudaSuccess ? Q40_OK : (int)e;
@@ -373,7 +378,7 @@ static int launch_rows(const BranchArgs& a, cudaStream_t st) {
 //     18.4, 4 / 4 10.5 / 10.9 / 16.6; 960 rows 9.3 / 11.4 / 20.2 and 12.7 / 13.1 / 20.7; 3200 rows 19.3 / 23.8 / 46.8 and 29.5 / 30.4 / 53.5
 //     (a whole step of 320 rows with 64 keys: 8 / 2 2280, 4 / 4 2251)
 template <int MODE>
-static int launch_branch_mode(const BranchArgs& a, cudaStream_t st) {
+static int launch_branch_mode(const ModeArgs<MODE>& a, cudaStream_t st) {
   const int64_t rows = a.rows;
   if constexpr (MODE == 1 || MODE == 2) {
     if (rows <= 2 * 148) return launch_rows<MODE, 8, 8, 4>(a, st);
@@ -390,16 +395,25 @@ static int launch_branch_mode(const BranchArgs& a, cudaStream_t st) {
   return launch_rows<MODE, 4, 4, 4>(a, st);
 }
 
-int launch_branch(BranchArgs a, int mode, int B, cudaStream_t st) {
+static void fill_derived(BranchArgs& a, int B) {
   a.page_shift = -1;
   if (a.page_size > 0 && (a.page_size & (a.page_size - 1)) == 0)
     for (a.page_shift = 0; (1 << a.page_shift) < a.page_size;) ++a.page_shift;
   a.last_page = a.page_size > 0 && a.P > 0 ? (a.P - 1) / a.page_size : 0;
   a.rows = (int64_t)B * a.H;
+}
+
+int launch_branch(BranchArgs a, int mode, int B, cudaStream_t st) {
+  fill_derived(a, B);
   if (mode == 0) return launch_branch_mode<0>(a, st);
   if (mode == 1) return launch_branch_mode<1>(a, st);
   if (mode == 2) return launch_branch_mode<2>(a, st);
-  return a.cos_tbl ? launch_branch_mode<4>(a, st) : launch_branch_mode<3>(a, st);
+  return launch_branch_mode<3>(a, st);
+}
+
+int launch_branch(BranchRotArgs a, int B, cudaStream_t st) {
+  fill_derived(a, B);
+  return launch_branch_mode<4>(a, st);
 }
 
 }  // namespace q40

@@ -285,7 +285,7 @@ static int tree_decode(const void* q, int64_t q_stride, const void* prefix_k, co
   pa.cos_tbl = (const __half*)cos_tbl; pa.sin_tbl = (const __half*)sin_tbl; pa.n_pos = n_pos; pa.pos = pos_dev;
   int rc = launch_prefix(pa, nsp, st);
   if (rc != Q40_OK) return rc;
-  BranchArgs br{};
+  BranchRotArgs br{};
   br.cos_tbl = pa.cos_tbl; br.sin_tbl = pa.sin_tbl; br.n_pos = n_pos;
   br.q = (const __half*)q; br.q_stride = q_stride; br.o = (__half*)o;
   br.H = H; br.Hkv = Hkv; br.L = max_t;
@@ -295,7 +295,7 @@ static int tree_decode(const void* q, int64_t q_stride, const void* prefix_k, co
   br.vq = (const int8_t*)cache_vq; br.vsc = (const __half*)cache_vs;
   br.pos = pos_dev; br.prefix_len = prefix_len_dev; br.max_t = max_t;
   br.cur_k = (const __half*)cur_k; br.cur_v = (const __half*)cur_v; br.cur_stride = cur_stride;
-  return launch_branch(br, 3, B, st);
+  return cos_tbl ? launch_branch(br, B, st) : launch_branch((const BranchArgs&)br, 3, B, st);
 }
 
 extern "C" int q40_attn_tree_decode(const void* q, int64_t q_stride, const void* prefix_k, const void* prefix_v,
