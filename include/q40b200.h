@@ -374,7 +374,8 @@ int q40_attn_tree_fused(void* qkv, int64_t W, const void* pk, const void* pv, vo
  * A cooperative launch of one CTA per SM in clusters of four that wait for one another through `workspace`:
  * q40_decode_chain_ws_bytes bytes, zeroed before the first call and left ready for the next one; one workspace per stream of calls.
  * The bytes are 0, and the call Q40_E_UNSUPPORTED, where the sizes do not suit (every matmul needs as many 64-column groups as there
- * are clusters, 33 on a B200; dim <= 4096; dim, hid and the widths of q and k multiples of 256) or the device takes no such launch.
+ * are clusters, 33 on a B200, and the groups that every cluster gets, of w1 and w3 together, times k at least 2048; dim <= 4096; dim, hid
+ * and the widths of q and k multiples of 256) or the device takes no such launch.
  * Waits are bounded: on expiry *err (may be mapped host memory) is set, results and workspace are undefined.
  * Replaces: the layer loop of Transformer.forward (hf_model_q40_kv_shared.py:303-409, 431-436, 456-466, 505-510). */
 size_t q40_decode_chain_ws_bytes(int B, int L, int dim, int hid, int H, int Hkv);

@@ -779,9 +779,10 @@ static int plan(Params& p, int B, int clusters, Plan& pl) {
   pl.clusters = clusters;
   int passes = 0;
   for (int i = 0; i < 4; ++i) {
-    // a cluster has work in every matmul (see the note on words that are written again), its segments fit, a warp has two at most
+    // a cluster has work in every matmul (see the note on words that are written again), and so has each of its warps (the sums over warps
+    // take every slab between a segment's first and last); its segments fit, a warp has two at most
     const int mul = i == 2 ? 2 : 1, most = (p.units[i] + clusters - 1) / clusters * mul;
-    if (p.units[i] < clusters || most > SEGS || most * B * 16 > THREADS || (most * p.kpairs[i] + WARPS - 1) / WARPS > p.kpairs[i]) return Q40_E_UNSUPPORTED;
+    if (p.units[i] / clusters * mul * p.kpairs[i] < WARPS || most > SEGS || most * B * 16 > THREADS || (most * p.kpairs[i] + WARPS - 1) / WARPS > p.kpairs[i]) return Q40_E_UNSUPPORTED;
     p.most[i] = most;
     passes += ((most * p.kpairs[i] + WARPS - 1) / WARPS + PASS - 1) / PASS + 1;      // a warp's share of two segments
     p.recv0[i] = i ? p.recv0[i - 1] + CL * p.most[i - 1] * B * 16 : 0;

@@ -134,3 +134,14 @@ def test_sizes_that_it_does_not_take():
     for B, dim, hid, H, Hkv in [(1, 8192, 28672, 64, 8), (3, 4096, 11008, 32, 32), (1, 4096, 11008, 32, 1), (1, 4096, 11000, 32, 32)]:
         assert lib.q40_decode_chain_ws_bytes(B, 32, dim, hid, H, Hkv) == 0
     assert lib.q40_decode_chain_ws_bytes(1, 32, 4096, 11008, 32, 32) > 0
+
+
+def test_sizes_that_leave_warps_without_work():
+    """Fewer 32-row pairs of a matmul in a cluster than it has warps: wo with one 64-column group of 6 to 14 pairs.  Not taken: sums over
+    warps would read slabs that nobody wrote.  One with 16 pairs or more is."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from spec_mcts_b200._lib import lib
+    for H, Hkv in [(14, 14), (14, 2), (6, 6), (12, 12)]:
+        assert lib.q40_decode_chain_ws_bytes(1, 2, 2304, 6144, H, Hkv) == 0
+    assert lib.q40_decode_chain_ws_bytes(1, 2, 2304, 6144, 16, 16) > 0
