@@ -340,7 +340,9 @@ int q40_attn_tree_decode(const void* q, int64_t q_stride, const void* prefix_k, 
 
 /* q40_rope_kv_append + q40_attn_tree_decode as the latter's two launches: q [B, H*D] and k [B, Hkv*D] (rows of q_stride and kv_stride elements)
  * come un-rotated and stay so; the launches rotate what they read (tables [n_pos, D/2] fp16, 16-byte aligned), and the branch pass appends
- * the rotated key and the value to the cache.  Everything else, and every result, as in the two calls.
+ * the rotated key and the value to the cache.  Everything else, and every result, as in the two calls, for positions below n_pos.  A position
+ * from n_pos on counts as n_pos - 1 in all that the call does, as in q40_attn_tree_fused and q40_decode_chain; of the two calls the first
+ * rotates and appends at n_pos - 1 too, but the second, which knows no tables, takes the length from the position as it is.
  * Replaces: the decode branch of Attention.forward (hf_model_q40_kv_shared.py:313-317, 330-405). */
 int q40_attn_tree_step(const void* q, int64_t q_stride, const void* k, const void* v, int64_t kv_stride, const void* prefix_k,
                        const void* prefix_v, int max_prefix_len, const int32_t* prefix_len_dev, int64_t prefix_key_stride,

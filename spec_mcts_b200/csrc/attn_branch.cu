@@ -84,7 +84,9 @@ attn_branch_kernel(const ModeArgs<MODE> a) {
   const unsigned gmask = 0xffu << (lane & 24);
 
   int len;
-  if (MODE >= 3) len = min(max(a.pos[b] - a.prefix_len[0], 0), a.max_t);
+  // mode 4 appends at the position that the tables allow, so that is the length too: the row that is written is never one that is read
+  if constexpr (MODE == 4) len = min(max(min(max(a.pos[b], 0), a.n_pos - 1) - a.prefix_len[0], 0), a.max_t);
+  else if (MODE == 3) len = min(max(a.pos[b] - a.prefix_len[0], 0), a.max_t);
   else len = a.seq_lens ? min(max(a.seq_lens[b], 0), a.L) : a.L;
   // first page ids.  They wait for the length: entries beyond it need not exist (the last row of a table that is a
   // column range of a wider one ends with the allocation).  Ids of every row but the last ahead of the length, by a

@@ -60,3 +60,43 @@ def test_refusals():
     assert lib.q40_attn_tree_step(*args(np=0)) == -2 and lib.q40_attn_tree_step(*args(ldk=128)) == -2
     assert lib.q40_attn_tree_step(*args(cos=p + 8)) == -3 and lib.q40_attn_tree_step(*args(kss=p + 2)) == -3
     assert lib.q40_attn_tree_step(*args(D=64)) == -5 and lib.q40_attn_tree_step(*args(wsb=16)) < 0
+
+
+@pytest.mark.parametrize("B,H,Hkv,own", [(3, 4, 4, 39), (3, 8, 2, 40), (5, 4, 1, 48), (40, 32, 8, 40)])
+def test_positions_past_the_tables_behind_a_full_prompt(B, H, Hkv, own):
+    """The appended row is then the cache's last, and within the length that the position as it is would give.  Such a position counts as the
+    tables' last one: the bits of the two calls there, the same ones every time, the caches of every call alike."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from spec_mcts_b200._lib import check, lib
+    D, maxP, maxT = 128, 128, 40
+    n_pos = maxP + maxT
+    g = torch.Generator(device="cuda").manual_seed(own)
+    normal = lambda *s: torch.randn(s, generator=g, device="cuda").half()
+    W = (H + 2 * Hkv) * D
+    qkv, pk, pv = normal(B, W), normal(maxP, Hkv, D), normal(maxP, Hkv, D)
+    ang = torch.rand((n_pos, 64), generator=g, device="cuda") * 6.28
+    cos, sin = ang.cos().half(), ang.sin().half()
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    plen, pos, last = i32(maxP), i32(*[maxP + own] * B), i32(*[n_pos - 1] * B)
+    ws = torch.zeros(lib.q40_attn_shared_prefix_workspace_bytes(B, H, D, maxP), dtype=torch.uint8, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    cache = [torch.randint(-128, 128, (B, maxT, Hkv, 64), generator=g, device="cuda", dtype=torch.int8),
+             (torch.rand((B, maxT, Hkv, 2), generator=g, device="cuda") * 0.3).half()]
+    cache += [cache[0].flip(0).contiguous(), cache[1].flip(0).contiguous()]
+    p = lambda c: [t.data_ptr() for t in c]
+    two, x, want = [c.clone() for c in cache], qkv.clone(), torch.empty((B, H * D), dtype=torch.float16, device="cuda")
+    q, k, v = x[:, :H * D], x[:, H * D:(H + Hkv) * D], x[:, (H + Hkv) * D:]
+    check(lib.q40_rope_kv_append(q.data_ptr(), W, k.data_ptr(), W, v.data_ptr(), W, last.data_ptr(), plen.data_ptr(), cos.data_ptr(), sin.data_ptr(),
+                                 n_pos, *p(two), B, H, Hkv, D, maxT, st))
+    check(lib.q40_attn_tree_decode(q.data_ptr(), W, pk.data_ptr(), pv.data_ptr(), maxP, plen.data_ptr(), pk.stride(0), pk.stride(1), *p(two), maxT,
+                                   last.data_ptr(), k.data_ptr(), v.data_ptr(), W, want.data_ptr(), B, H, Hkv, D, ws.data_ptr(), ws.numel(), st))
+    q, k, v = qkv[:, :H * D], qkv[:, H * D:(H + Hkv) * D], qkv[:, (H + Hkv) * D:]
+    for _ in range(20):
+        one, got = [c.clone() for c in cache], torch.empty_like(want)
+        check(lib.q40_attn_tree_step(q.data_ptr(), W, k.data_ptr(), v.data_ptr(), W, pk.data_ptr(), pv.data_ptr(), maxP, plen.data_ptr(), pk.stride(0),
+                                     pk.stride(1), *p(one), maxT, pos.data_ptr(), cos.data_ptr(), sin.data_ptr(), n_pos, got.data_ptr(), B, H, Hkv, D,
+                                     ws.data_ptr(), ws.numel(), st))
+        assert torch.equal(got, want)
+        for a, b in zip(one, two):
+            assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
