@@ -265,7 +265,7 @@ struct GemvPlan {
 
 static GemvPlan plan_kn(int N, int K) {
   GemvPlan p;
-  p.nspans = (N / 2 + SPAN_BYTES - 1) / SPAN_BYTES;
+  p.nspans = N > 1 ? (N / 2 + SPAN_BYTES - 1) / SPAN_BYTES : 1;      // a single column: scratch is asked for it through the other orientation
   const int target_ctas = 148 * 3;
   int want = (target_ctas + p.nspans - 1) / p.nspans;
   if (want < 1) want = 1;

@@ -47,6 +47,14 @@ def test_argument_errors_are_status_codes():
     assert lib.q40_gemm_workspace_bytes(0, 4096, 4096) == 0
 
 
+def test_workspace_of_a_single_output():
+    """linear_q40 asks for the scratch of a layer with one output."""
+    from spec_mcts_b200._lib import lib
+    for M in (1, 8, 16, 100):
+        for Kd in (128, 4096):
+            assert lib.q40_gemm_workspace_bytes(M, 1, Kd) >= lib.q40_gemm_workspace_bytes(M, 2, Kd) > 4096
+
+
 def test_python_api_refuses_cpu_tensors():
     import torch
     from spec_mcts_b200 import kernels as K

@@ -6,7 +6,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("M,K,N", [(1, 128, 2), (8, 128, 17), (9, 256, 16), (16, 384, 33), (17, 640, 15), (32, 1152, 100), (33, 1152, 100), (64, 1280, 7000), (65, 1152, 7000), (97, 2048, 2050),
+@pytest.mark.parametrize("M,K,N", [(1, 128, 1), (10, 4096, 1), (40, 384, 1), (1, 128, 2), (8, 128, 17), (9, 256, 16), (16, 384, 33), (17, 640, 15), (32, 1152, 100), (33, 1152, 100), (64, 1280, 7000), (65, 1152, 7000), (97, 2048, 2050),
                                    (10, 4096, 11008), (1, 11008, 4099), (10, 11008, 4096), (16, 11008, 1000), (32, 8320, 80), (3, 896, 11841),
                                    (13, 2944, 2368), (5, 2048, 2369)])
 def test_against_64_bits(M, K, N):
