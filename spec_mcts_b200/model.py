@@ -270,7 +270,9 @@ class Transformer(nn.Module):
         # single-launch attention (rotary + append + attention) up to this width; wider steps read the
         # shared prompt once for all branches with the three-launch path
         # width <= 8: final RMSNorm, fp16 lm_head, arg-max and position bump as one launch (above, the
-        # library GEMM is faster than the streaming kernel)
+        # library GEMM is faster than the streaming kernel).  Us of a step of 8 layers behind the
+        # tensor-core matmuls, with torch's product and arg-max and with it: dim 4096, 5 branches 545 and 549, with feedback
+        # 559 and 553, 8 branches 555 and 561, 571 and 565; its sums are fp32 and a tie goes to the smaller index
         self.use_fused_tail = True
         self.use_fused_attn = True
         self.fused_attn_max_width = 1
@@ -920,18 +922,8 @@ class Transformer(nn.Module):
             self._fused(1, [lin], [bufs["logits_pad"]], vp, h, p.dim, B, norm_w=self.norm.weight, ss_in=ss_ffn,
                         ss_in_count=c_ffn, st=st, bufs=bufs)
             logits = bufs["logits_pad"][:, :p.vocab_size]
-        elif self.use_fused_tail and p.dim % 128 == 0 and B <= 8:
-            # final RMSNorm + fp16 lm_head + (greedy feedback) arg-max and position bump: one launch
-            logits = bufs["logits"]
-            if "lm_scratch" not in bufs:
-                bufs["lm_scratch"] = torch.zeros(lib.q40_lm_head_scratch_bytes(), dtype=torch.uint8, device=self.device)
-            fb = self.greedy_feedback
-            check(lib.q40_lm_head(h.data_ptr(), p.dim, ss_ffn.data_ptr(), c_ffn, self.norm.weight.data_ptr(),
-                                  float(p.norm_eps), self.output.weight.data_ptr(), p.vocab_size, p.dim,
-                                  logits.data_ptr(), logits.stride(0), B,
-                                  self._tok_dev.data_ptr() if fb else None, self._pos_dev.data_ptr() if fb else None,
-                                  bufs["lm_scratch"].data_ptr(), 1 if self.use_pdl else 0, st), "q40_lm_head")
-            return logits
+        elif self._fused_tail(B):
+            return self._lm_head(B, bufs, ss_ffn, c_ffn, st)
         else:
             self._norm(h, None, self.norm.weight, bufs["xn"], st)
             logits = bufs["logits"]
@@ -939,6 +931,22 @@ class Transformer(nn.Module):
         if self.greedy_feedback:
             self._tok_dev[:B].copy_(logits.argmax(dim=-1))
             self._pos_dev[:B] += 1
+        return logits
+
+    def _fused_tail(self, B):
+        return self.use_fused_tail and self._narrow(B) and B <= 8 and self.params.dim % 128 == 0
+
+    def _lm_head(self, B, bufs, ss, ss_count, st):
+        """Final RMSNorm of bufs["h"], fp16 lm_head and (greedy feedback) arg-max and position bump: one launch.  `ss`: partial
+        sums of squares of the rows, or None."""
+        p, h, logits, fb = self.params, bufs["h"], bufs["logits"], self.greedy_feedback
+        if "lm_scratch" not in bufs:
+            bufs["lm_scratch"] = torch.zeros(lib.q40_lm_head_scratch_bytes(), dtype=torch.uint8, device=self.device)
+        check(lib.q40_lm_head(h.data_ptr(), p.dim, ss.data_ptr() if ss is not None else None, ss_count, self.norm.weight.data_ptr(),
+                              float(p.norm_eps), self.output.weight.data_ptr(), p.vocab_size, p.dim,
+                              logits.data_ptr(), logits.stride(0), B,
+                              self._tok_dev.data_ptr() if fb else None, self._pos_dev.data_ptr() if fb else None,
+                              bufs["lm_scratch"].data_ptr(), 1 if self.use_pdl else 0, st), "q40_lm_head")
         return logits
 
     def quantize_lm_head(self):
@@ -1017,6 +1025,9 @@ class Transformer(nn.Module):
                 pending = bufs["f"]
         if not normed:
             self._norm(h, pending, self.norm.weight, xn, st)
+        if self._fused_tail(B):
+            # the launch in front has added the last sub-block to h
+            return self._lm_head(B, bufs, None, 0, st)
         torch.matmul(xn, self.output.weight.t(), out=bufs["logits"])
         if self.greedy_feedback:
             self._tok_dev[:B].copy_(bufs["logits"].argmax(dim=-1))
@@ -1080,7 +1091,7 @@ class Transformer(nn.Module):
         per_layer = (5 if self._fused_attn_for(B) else 6) if fused else (8 if self._silu_pair(B, self.layers[0].feed_forward) else 9)
         if not (fused and per_layer == 5 or self._rotates_in_attention(B)):
             per_layer += 1
-        self.launches_per_step = self.params.n_layers * per_layer + (2 if self._narrow(B) else 1)
+        self.launches_per_step = self.params.n_layers * per_layer + (2 if self._narrow(B) else 1) + (not fused and self._fused_tail(B))
         if not self.use_cuda_graph:
             logits = self._decode_body(B)
             if fused and self._chained.get(B):
