@@ -15,6 +15,8 @@
 // Algorithmic traffic: prefix K/V once per (kv head, row block); Q and the partials are
 // small next to it.  What bounds it: a warp's chain of MMAs and softmax per tile (2.1 us; see attn_tile.cuh), start, first
 // tile and partials around it.
+#include <climits>
+
 #include "attn_tile.cuh"
 
 namespace q40 {
@@ -139,7 +141,8 @@ attn_prefix_kernel(const PrefixArgs a) {
   }
 }
 
-static int prefix_splits(int B, int H, int Hkv, int prefix_len, int64_t suffix) {
+// `own`: keys that the branches have of their own in front of a head, about; 0: not known
+static int prefix_splits(int B, int H, int Hkv, int prefix_len, int64_t own) {
   const int rep = H / Hkv;
   const int rows = B * rep;
   const int rblocks = (rows + 127) / 128;
@@ -147,21 +150,27 @@ static int prefix_splits(int B, int H, int Hkv, int prefix_len, int64_t suffix) 
   // CTAs per SM to aim for: two for the 64-row variant (128 threads; measured best for 2048 keys x 64
   // rows), one for the 128-row variant; never round up past whole waves (a 149th CTA doubles the time
   // of one SM)
-  // ... one, too, where the branches' own keys (`suffix` of a head, about; 0: not known) are so many that the pass is over long before they
-  // are: it then gets by with half of the partials and leaves SMs to them (64 branches of up to 256 own keys behind 512: 34.6 us
-  // with two, 31.4; 34 behind 471 22.2 and 21.4; at four times the prefix no difference, below it one is slower: 10 behind 2048
-  // 16.6 and 18.5; and with fewer than eight tiles: 64 branches of up to 100 behind 300 17.9 and 18.7)
-  const bool hidden = tiles >= 8 && suffix > 6 * (int64_t)prefix_len;
+  // ... one, too, where the branches' own keys are so many that the pass is over long before they are: it then gets by with half of the
+  // partials and leaves SMs to them (64 branches of up to 256 own keys behind 512: 34.6 us with two, 31.4; 34 behind 471 22.2 and 21.4; at four
+  // times the prefix no difference, below it one is slower: 10 behind 2048 16.6 and 18.5; and with fewer than eight tiles: 64 branches
+  // of up to 100 behind 300 17.9 and 18.7)
+  const bool hidden = tiles >= 8 && own > 6 * (int64_t)prefix_len;
   const int per_sm = rows <= 64 && !hidden ? 2 : 1;
   int want = (148 * per_sm) / (Hkv * rblocks);
   if (want < 1) want = 1;
   if (want > tiles) want = tiles;
-  // the merge has 16 splits of a row on their way at once and reads further ones one by one (8 kv heads, 2048 keys: 4 branches 11.5 us
-  // with 32 splits, 7.9; 16 branches 17.0 and 13.8)
-  if (want > 16) want = 16;
-  if (want < 1) want = 1;
-  const int tiles_per = (tiles + want - 1) / want;
-  return (tiles + tiles_per - 1) / tiles_per;               // every split is non-empty
+  // How many tiles a split has.  A tile costs it 1.0 us (1.9 with eight warps); the merge has 16 splits of a row on their way at once and reads further ones one by
+  // one, 0.07 us each; a second CTA on an SM costs 2.3 us that matter less the longer splits are.  Us by splits, 8 query heads a kv head:
+  // 1 kv head, 1 branch, 2048 keys 16 splits 6.1, 32 7.3; 8192 keys 16 12.4, 32 10.4, 128 14.1; 32768 keys 16 37.3, 64 16.8, 256 24.9; 8 kv heads
+  // x 4, 4 branches, 2048 keys 16 7.7, 32 10.6; 32768 keys 16 44.1, 32 30.5.  Over 448 sizes of 1 to 32 kv heads and 512 to 32768 keys 5 % less
+  // time than with as many splits as SMs take, four of them 3 to 9 % more (1 kv head x 4, 34 branches, 8192 keys 15.9 and 17.3)
+  int best = tiles, least = INT_MAX;
+  for (int per = (tiles + want - 1) / want;; ++per) {
+    const int n = (tiles + per - 1) / per;                  // every split is non-empty
+    const int cost = 14 * per + (n > 16 ? n - 16 : 0) + (n * Hkv * rblocks > 148 ? 32 / per : 0);
+    if (cost < least) { least = cost; best = n; }
+    if (n <= 16) return best;
+  }
 }
 
 // pa.prefix_len is the (maximum) prefix length the grid is sized for
@@ -223,7 +232,10 @@ extern "C" int q40_attn_shared_prefix(const void* q, const void* prefix_k, const
   br.scale_log2 = attn_scale_log2(D);
 
   if (prefix_len > 0) {
-    const int nsp = prefix_splits(B, H, Hkv, prefix_len, (int64_t)B * Lmax / 2);
+    // lengths are on the device; Lmax is taken for twice their mean up to 256 keys.  A wider table is more likely one that branches can grow
+    // into (64 branches of 64 keys with room for 4096, behind 8192: 71 us if they count as 2048 each, 47), and long rows gain nothing (34
+    // branches of 1000 behind 512: 89.7 and 89.9)
+    const int nsp = prefix_splits(B, H, Hkv, prefix_len, Lmax <= 256 ? (int64_t)B * Lmax / 2 : 0);
     const size_t need = (size_t)nsp * rows_total * (D + 2) * sizeof(float);
     if (!workspace || workspace_bytes < need) return Q40_E_WORKSPACE;
     if (!q40_aligned(workspace, 16)) return Q40_E_ALIGN;

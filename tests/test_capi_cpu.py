@@ -55,6 +55,32 @@ def test_workspace_of_a_single_output():
             assert lib.q40_gemm_workspace_bytes(M, 1, Kd) >= lib.q40_gemm_workspace_bytes(M, 2, Kd) > 4096
 
 
+def prefix_splits(B, H, Hkv, prefix, Lmax):
+    """Splits of q40_attn_shared_prefix: the scratch that it asks for is theirs.  The scratch handed over is off its boundary, so nothing is launched."""
+    from spec_mcts_b200._lib import lib
+    buf = ctypes.create_string_buffer(4096)
+    p16 = (ctypes.addressof(buf) + 15) // 16 * 16
+    status = lambda n: lib.q40_attn_shared_prefix(p16, p16, p16, prefix, Hkv * 128, 128, p16, 4, 1 << 20, p16, p16, p16, p16, 1 << 20, B, Lmax, H, Hkv, 128,
+                                                  16, p16 + 4, n * B * H * 130 * 4, None)
+    n = next(n for n in range(1, 400) if status(n) != -4)
+    assert status(n) == -3
+    assert n * B * H * 130 * 4 <= lib.q40_attn_shared_prefix_workspace_bytes(B, H, 128, prefix)
+    return n
+
+
+def test_prefix_splits():
+    # a merge has 16 splits on their way at once: no more for up to 2048 keys ...
+    assert [prefix_splits(B, 8 * Hkv, Hkv, 2048, 64) for B in (1, 4, 16) for Hkv in (1, 2)] == [16] * 6
+    # ... but a longer prefix goes to as many SMs as its time is worth
+    assert prefix_splits(16, 8, 1, 32768, 64) >= 64 and prefix_splits(1, 8, 1, 8192, 64) >= 32 and prefix_splits(4, 32, 8, 32768, 64) >= 32
+    # one an SM behind many own keys; a table with room for many more says nothing about them
+    assert prefix_splits(64, 32, 32, 1024, 256) == 4 and prefix_splits(64, 32, 32, 1024, 100) == 8
+    assert prefix_splits(64, 32, 32, 8192, 4096) == prefix_splits(64, 32, 32, 8192, 64) >= 8
+    for prefix in (1, 64, 65, 1024, 1025, 2049, 9999, 32768, 100000):
+        for B, Hkv, rep in ((1, 1, 1), (3, 1, 8), (100, 1, 8), (1, 32, 1), (100, 32, 1), (7, 5, 3), (500, 8, 4)):
+            assert 1 <= prefix_splits(B, Hkv * rep, Hkv, prefix, 64) <= min(296, -(-prefix // 64))
+
+
 def test_python_api_refuses_cpu_tensors():
     import torch
     from spec_mcts_b200 import kernels as K

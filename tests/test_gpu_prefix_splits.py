@@ -30,3 +30,10 @@ def test_against_64_bits(B, H, Hkv, prefix, suffix, page):
         # weights of the prefix pass are fp16 operands (2^-11 of each product), sums fp32, the result fp16 (2^-11)
         bound = 2 ** -10 * (w @ vv.abs())[:, 0] + 2 ** -11 * (w @ vv).abs()[:, 0] + 1e-5
         assert ((got[b] - (w @ vv)[:, 0]).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("B,H,Hkv,prefix", [(1, 4, 1, 8192), (10, 8, 1, 16390), (34, 4, 1, 4097), (4, 32, 8, 32768 - 63)])
+def test_long_prefixes(B, H, Hkv, prefix):
+    """More splits than a merge has on their way at once, up to more than a warp has lanes; a last split that is shorter, or a single key."""
+    test_against_64_bits(B, H, Hkv, prefix, 40, 16)
+
