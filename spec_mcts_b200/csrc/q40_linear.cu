@@ -279,7 +279,7 @@ int q40_linear(const void* x, int64_t ldx, const void* wq, const void* ws, void*
   p.x = (const __half*)x; p.ldx = ldx; p.w = (const uint8_t*)wq; p.s = (const __half*)ws; p.y = (__half*)y; p.ldy = ldy;
   p.M = M; p.N = N; p.K = K;
   double best = 1e30;
-  int bc = 0, bclusters = 0;
+  int bc = 0, bclusters = 0, busiest = 0;
   size_t bsmem = 0;
   Args bp{};
   for (int c = 1; c <= 4; c *= 2) {
@@ -297,13 +297,22 @@ int q40_linear(const void* x, int64_t ldx, const void* wq, const void* ws, void*
       p.off_slab = (int)off; off += (size_t)p.kw * TILES * mt * 8 * M_LD * 4;
       p.off_out = (int)off; off += c > 1 ? (size_t)TILES * mt * 8 * 16 * 4 : 0;
       if (off > (size_t)SMEM_MAX) continue;
-      // steps of the busiest warp, staging, sums over warps, what a cluster's exchange costs
-      const int tw = WARPS / p.kw;
-      const double ns = ((p.tiles + tw - 1) / tw) * ((p.ksteps + p.kw - 1) / p.kw) * (160.0 + 110.0 * mt) + p.xk * M * 0.03 + p.kw * 20.0 + (c > 1 ? 1200 : 0);
-      if (ns < best) { best = ns; bc = c; bclusters = clusters; bsmem = off; bp = p; }
+      // steps of the busiest warp (which come in pairs: an odd one counts a quarter more), staging, sums over warps, what a cluster's exchange
+      // costs.  (Without the quarter 1 row x 2048 x 10711, where a warp had five single steps, 10.2 us, 8.8 by gemv_nk_kernel; now 7.3)
+      const int tw = WARPS / p.kw, warp_tiles = (p.tiles + tw - 1) / tw, warp_steps = (p.ksteps + p.kw - 1) / p.kw;
+      const double ns = warp_tiles * (warp_steps + 0.25 * (warp_steps & 1)) * (160.0 + 110.0 * mt) + p.xk * M * 0.03 + p.kw * 20.0 + (c > 1 ? 1200 : 0);
+      if (ns < best) { best = ns; busiest = warp_tiles * warp_steps; bc = c; bclusters = clusters; bsmem = off; bp = p; }
     }
   }
   if (bc == 0) return Q40_E_UNSUPPORTED;
+  // gemv_nk_kernel instead, where it is the faster one with weights from HBM (us here and there).  Above eight rows, where activations leave room for
+  // few warps' sums, so that one has a long chain of steps: 16 rows x 7040 x 9825 45.4 and 31.9, 55 steps; 9 x 11008 x 11008 43.5 and 36.9, 43; 24 x
+  // 8320 x 3197 29.7 and 28.1, 33; but 12 x 8704 x 8754 27.8 and 31.1, 34, with tiles spread evenly; 16 x 6528 x 8146 25.9 and 27.7, 26.  Up to four,
+  // where CTAs have a quarter less to do on average than the busiest and scales lie so that a step's come in two loads: 1 row x 4224 x 4963 10.0
+  // and 9.0, 4 rows x 10880 x 2893 14.2 and 12.3, x 6016 x 5185 12.6 and 12.1; but 1 x 1152 x 2596, 2 steps, 4.3 and 5.0.  (From L2 this
+  // kernel is the faster one of most of these: 32.3 and 28.6, 30.6 and 33.4, 22.8 and 24.2 above eight rows, 8.2 and 8.6, 11.7 and 11.5, 10.2 and 10.9.)
+  const double even = (double)tiles * ksteps / (148.0 * bp.tiles * bp.ksteps);
+  if (M > 8 ? busiest >= (even < 0.9 ? 30 : 40) : M <= 4 && K % 256 != 0 && even < 0.75 && busiest >= 6) return Q40_E_UNSUPPORTED;
   if (mt == 1) return launch<1>(bp, bc, bclusters, bsmem, (cudaStream_t)stream);
   if (mt == 2) return launch<2>(bp, bc, bclusters, bsmem, (cudaStream_t)stream);
   return launch<4>(bp, bc, bclusters, bsmem, (cudaStream_t)stream);

@@ -8,7 +8,10 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("M,K,N", [(1, 128, 1), (10, 4096, 1), (40, 384, 1), (1, 128, 2), (8, 128, 17), (9, 256, 16), (16, 384, 33), (17, 640, 15), (32, 1152, 100), (33, 1152, 100), (64, 1280, 7000), (65, 1152, 7000), (97, 2048, 2050),
                                    (10, 4096, 11008), (1, 11008, 4099), (10, 11008, 4096), (16, 11008, 1000), (32, 8320, 80), (3, 896, 11841),
-                                   (13, 2944, 2368), (5, 2048, 2369)])
+                                   (13, 2944, 2368), (5, 2048, 2369),
+                                   # what the other kernel takes, and its neighbours: long chains of steps above eight rows, uneven CTAs up to four, a remainder of 32
+                                   (16, 7040, 9825), (17, 6144, 6165), (33, 6144, 6165), (1, 4224, 4963), (4, 4224, 4963), (5, 4224, 4963), (36, 4224, 4963),
+                                   (2, 1152, 2596), (1, 2048, 10711)])
 def test_against_64_bits(M, K, N):
     """What is rounded: operands fp16(code * scale), by half a step (2^-11) of each product; sums in fp32 (1e-5 of the sum of magnitudes
     covers 2^-24 per addition over K); the result, by half an fp16 step (2^-11, subnormals 2^-25)."""
