@@ -35,18 +35,24 @@ bool two(PyObject* t, int64_t& a, int64_t& b) {
   return true;
 }
 int64_t version(const at::Tensor& t) { return t.is_inference() ? -1 : (int64_t)t._version(); }
-// kernels._workspaces[("gemm", device, stream)], borrowed, or null
-const at::Tensor* workspace(PyObject* dict, int dev, PyObject* stream) {
+// kernels._workspaces[("gemm", device, stream)] or an undefined tensor
+at::Tensor workspace(PyObject* dict, int dev, PyObject* stream) {
   static PyObject* kind = PyUnicode_InternFromString("gemm");
   PyObject* key = Py_BuildValue("(OiO)", kind, dev, stream);
   if (!key) {
     PyErr_Clear();
-    return nullptr;
+    return {};
   }
   PyObject* t = PyDict_GetItem(dict, key);
   Py_DECREF(key);
-  return t && THPVariable_Check(t) ? &THPVariable_Unpack(t) : nullptr;
+  return t && THPVariable_Check(t) ? THPVariable_Unpack(t) : at::Tensor();
 }
+// Other Python threads run meanwhile: an allocation may wait for the device, a launch for room in its queue (behind a host function that
+// needs the interpreter, say).  What is used in there is owned here
+struct WithoutInterpreter {
+  PyThreadState* state = PyEval_SaveThread();
+  ~WithoutInterpreter() { PyEval_RestoreThread(state); }
+};
 at::Tensor output(int64_t rows, int64_t cols, int dev) {
   return at::empty({rows, cols}, at::TensorOptions().dtype(at::kHalf).device(at::kCUDA, (c10::DeviceIndex)dev));
 }
@@ -76,7 +82,7 @@ PyObject* matmul(PyObject*, PyObject* const* args, Py_ssize_t n) {
   PyObject* st = PyLong_FromVoidPtr(stream);
   if (!st) return nullptr;
   const int known = PySet_Contains(PyTuple_GET_ITEM(e, 7), st);
-  const at::Tensor* page = known == 1 && M > 8 ? workspace(args[6], dev, st) : nullptr;
+  const at::Tensor page = known == 1 && M > 8 ? workspace(args[6], dev, st) : at::Tensor();
   Py_DECREF(st);
   if (known != 1) {
     PyErr_Clear();
@@ -88,11 +94,17 @@ PyObject* matmul(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Py_XDECREF(d);
   if (sizes && PyTuple_Check(sizes) && PyTuple_GET_SIZE(sizes)) cluster = (int)PyLong_AsLong(PyTuple_GET_ITEM(sizes, 0));
   else if (M <= 8) Py_RETURN_NONE;
-  if (M > 8 && !page) Py_RETURN_NONE;
-  at::Tensor c = output(M, N, dev);
-  if (matmul_tiled(THPVariable_Unpack(PyTuple_GET_ITEM(e, 5)).data_ptr(), c.data_ptr(), N, a->data_ptr(), K, (int)M, (int)N, (int)K, cluster,
-                   page ? (char*)page->data_ptr() + 4092 : nullptr, 1, stream) != 0)
-    Py_RETURN_NONE;
+  if (M > 8 && !page.defined()) Py_RETURN_NONE;
+  const at::Tensor copy = THPVariable_Unpack(PyTuple_GET_ITEM(e, 5)), x = *a;
+  at::Tensor c;
+  int rc;
+  {
+    WithoutInterpreter w;
+    c = output(M, N, dev);
+    rc = matmul_tiled(copy.data_ptr(), c.data_ptr(), N, x.data_ptr(), K, (int)M, (int)N, (int)K, cluster,
+                      page.defined() ? (char*)page.data_ptr() + 4092 : nullptr, 1, stream);
+  }
+  if (rc != 0) Py_RETURN_NONE;
   return THPVariable_Wrap(std::move(c));
   END_HANDLE_TH_ERRORS
 }
@@ -113,15 +125,23 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const auto stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
   PyObject* st = PyLong_FromVoidPtr(stream);
   if (!st) return nullptr;
-  const at::Tensor* ws = workspace(args[5], dev, st);
+  const at::Tensor ws = workspace(args[5], dev, st);
   Py_DECREF(st);
-  if (!ws || ws->numel() > 64 << 20) Py_RETURN_NONE;        // a large one is noted where a capture uses it
-  at::Tensor y = output(M, N, dev);
-  if (gemm_nk(x->data_ptr(), K, w->data_ptr(), s->data_ptr(), y.data_ptr(), N, (int)M, (int)N, (int)K, (int)PyLong_AsLong(args[4]), ws->data_ptr(),
-              (size_t)ws->numel(), stream) != 0) {
+  if (!ws.defined() || ws.numel() > 64 << 20) Py_RETURN_NONE;        // a large one is noted where a capture uses it
+  const int group = (int)PyLong_AsLong(args[4]);
+  if (PyErr_Occurred()) {
     PyErr_Clear();
     Py_RETURN_NONE;
   }
+  const at::Tensor in = *x, codes = *w, scales = *s;
+  at::Tensor y;
+  int rc;
+  {
+    WithoutInterpreter w;
+    y = output(M, N, dev);
+    rc = gemm_nk(in.data_ptr(), K, codes.data_ptr(), scales.data_ptr(), y.data_ptr(), N, (int)M, (int)N, (int)K, group, ws.data_ptr(), (size_t)ws.numel(), stream);
+  }
+  if (rc != 0) Py_RETURN_NONE;
   return THPVariable_Wrap(std::move(y));
   END_HANDLE_TH_ERRORS
 }

@@ -104,3 +104,22 @@ def test_linear(K, monkeypatch, M, group):
     with pytest.raises(K.Q40Error):
         K.linear_q40(x, q, s, (300, 512), group_size=48)
     assert K.linear_q40(x[:0], q, s, (300, 512), group_size=group).shape == (0, 300)
+
+
+def test_interpreter_is_free_meanwhile(K, monkeypatch):
+    """In the place of the library's functions, one that returns 0 if the thread does not hold the interpreter's lock."""
+    import ctypes
+    a, q, s, shape = data(K)
+    K.matmul_q40(a, q, s, shape)
+    y = K.linear_q40(a, q, s, (512, 256))
+    taken = count(monkeypatch, K)
+    from spec_mcts_b200 import _host_calls
+    address = lambda f: ctypes.cast(f, ctypes.c_void_p).value
+    try:
+        _host_calls.init(*[address(ctypes.pythonapi.PyGILState_Check)] * 2)
+        K.matmul_q40(a, q, s, shape)
+        K.linear_q40(a, q, s, (512, 256))
+    finally:
+        _host_calls.init(address(K.lib.q40_matmul_tiled), address(K.lib.q40_gemm_nk))
+    assert taken == [True, True]
+    assert torch.equal(K.linear_q40(a, q, s, (512, 256)), y)
