@@ -39,39 +39,62 @@ def sources():
 
 
 STAMP = LIB + ".sha"
+HOST_STAMP = HOST + ".sha"
 
 
-def _sources_digest() -> str:
-    """Content hash of everything the library is built from (file times do not survive a
-    copy of the tree to another machine, contents do)."""
+def _digest(files, *words: str) -> str:
+    """Content hash of what something is built from (file times do not survive a copy of the tree to another machine,
+    contents do)."""
     import hashlib
-    files = sources() + [HOST_SRC] + sorted(glob.glob(os.path.join(CSRC, "*.cuh"))) + \
-        sorted(glob.glob(os.path.join(PKG_DIR, "..", "include", "*.h")))
-    h = hashlib.sha256(" ".join(NVCC_FLAGS).encode())
+    h = hashlib.sha256(" ".join(words).encode())
     for f in files:
         h.update(os.path.basename(f).encode())
         h.update(open(f, "rb").read())
     return h.hexdigest()
 
 
-def needs_build() -> bool:
-    if not (os.path.exists(LIB) and os.path.exists(HOST) and os.path.exists(STAMP)):
-        return True
-    return open(STAMP).read().strip() != _sources_digest()
+def _sources_digest() -> str:
+    return _digest(sources() + sorted(glob.glob(os.path.join(CSRC, "*.cuh"))) +
+                   sorted(glob.glob(os.path.join(PKG_DIR, "..", "include", "*.h"))), *NVCC_FLAGS)
 
 
-def _build_host() -> None:
+def _host_digest() -> str:
+    """... of the Python extension, which uses torch's C++ interface: that differs from version to version."""
     import torch
-    t = os.path.dirname(torch.__file__)
+    return _digest([HOST_SRC], torch.__version__, str(torch.version.cuda), str(int(torch._C._GLIBCXX_USE_CXX11_ABI)))
+
+
+def _is_built(path: str, stamp: str, digest: str) -> bool:
+    return os.path.exists(path) and os.path.exists(stamp) and open(stamp).read().strip() == digest
+
+
+def needs_build() -> bool:
+    return not _is_built(LIB, STAMP, _sources_digest())
+
+
+def host_needs_build() -> bool:
+    return not _is_built(HOST, HOST_STAMP, _host_digest())
+
+
+def build_host(force: bool = False) -> str:
+    """Compile the Python extension, with the host's C++ compiler."""
+    if not force and not host_needs_build():
+        return HOST
+    import torch
+    t, new = os.path.dirname(torch.__file__), f"{HOST}.{os.getpid()}"
     cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I" + os.path.join(t, "include"),
            "-I" + os.path.join(t, "include", "torch", "csrc", "api", "include"), "-I" + sysconfig.get_paths()["include"],
-           "-I" + os.path.join(cuda, "include"), HOST_SRC, "-o", HOST, "-L" + os.path.join(t, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu",
+           "-I" + os.path.join(cuda, "include"), HOST_SRC, "-o", new, "-L" + os.path.join(t, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu",
            "-ltorch", "-ltorch_python"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"building {HOST_SRC} failed:\n{r.stdout}\n{r.stderr}")
+    os.replace(new, HOST)              # a process that has the old one loaded keeps it
+    with open(HOST_STAMP, "w") as f:
+        f.write(_host_digest())
+    return HOST
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -101,7 +124,6 @@ def build(force: bool = False, verbose: bool = False) -> str:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
-    _build_host()
     with open(STAMP, "w") as f:
         f.write(_sources_digest())
     return LIB
@@ -110,3 +132,4 @@ def build(force: bool = False, verbose: bool = False) -> str:
 if __name__ == "__main__":
     path = build(force="--force" in sys.argv, verbose="-v" in sys.argv)
     print(path)
+    print(build_host(force="--force" in sys.argv))

@@ -15,10 +15,25 @@ from typing import Optional, Sequence
 
 import torch
 
-from . import _host_calls
+from . import build as _build
 from ._lib import Q40Error, check, lib
 
-_host_calls.init(*[ctypes.cast(f, ctypes.c_void_p).value for f in (lib.q40_matmul_tiled, lib.q40_gemm_nk)])
+
+def _load_host_calls():
+    """The Python extension of csrc/host_calls.cpp, or None where there is none for this torch and none can be built: it
+    saves host time and nothing else, every call has its way without it."""
+    try:
+        _build.build_host()
+        from . import _host_calls as m
+    except Exception as e:
+        import warnings
+        warnings.warn(f"calls of matmul_q40 and linear_q40 take longer without {_build.HOST}: {e}")
+        return None
+    m.init(*[ctypes.cast(f, ctypes.c_void_p).value for f in (lib.q40_matmul_tiled, lib.q40_gemm_nk)])
+    return m
+
+
+_host_calls = _load_host_calls()
 
 DTYPE_torch = torch.float16
 GROUP_SIZE = 64
@@ -199,7 +214,7 @@ def matmul_q40(a: torch.Tensor, b_w: torch.Tensor, b_s: torch.Tensor, b_shape, *
     K % 64 == 0; else up to 16 rows by the former) by the tensor-core kernel that writes the dequantised operand to tensor memory.  The copy
     doubles the device memory of that weight; `relayout=False` (or relayout_cache_config(enabled=False))
     reads the checkpoint layout instead."""
-    if out is None and relayout is None and group_size == 64 and _relayout_cfg["enabled"]:
+    if out is None and relayout is None and group_size == 64 and _host_calls is not None and _relayout_cfg["enabled"]:
         ent = _relayout_cache.get(id(b_w))
         if ent is not None:
             c = _host_calls.matmul(a, b_w, b_s, b_shape, ent, _cluster_sizes, _workspaces)     # None: not the plain repeated call
@@ -472,9 +487,10 @@ def linear_q40(x: torch.Tensor, w_q: torch.Tensor, w_s: torch.Tensor, w_shape, *
                group_size: int = GROUP_SIZE):
     """y = x @ deq(W)^T for W [N,K] quantised along K — the fused form of the reference's
     dequantize_q40 + F.linear (quantize.py:235-246, hf_model_q40.py:222-233)."""
-    y = _host_calls.linear(x, w_q, w_s, w_shape, group_size, _workspaces)         # None: not a plain call
-    if y is not None:
-        return y
+    if _host_calls is not None:
+        y = _host_calls.linear(x, w_q, w_s, w_shape, group_size, _workspaces)         # None: not a plain call
+        if y is not None:
+            return y
     dev = _need_cuda(x, w_q, w_s)
     N, K = int(w_shape[0]), int(w_shape[1])
     lead = x.shape[:-1]

@@ -55,6 +55,30 @@ def test_workspace_of_a_single_output():
             assert lib.q40_gemm_workspace_bytes(M, 1, Kd) >= lib.q40_gemm_workspace_bytes(M, 2, Kd) > 4096
 
 
+def test_extension_is_built_for_this_torch(monkeypatch):
+    import torch
+    from spec_mcts_b200 import build
+    build.build_host()
+    assert not build.host_needs_build() and not build.needs_build()
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    assert build.host_needs_build() and not build.needs_build()
+
+
+def test_without_extension(monkeypatch):
+    """No compiler, or another torch's extension: a warning that names it, and the general way."""
+    from spec_mcts_b200 import build
+    from spec_mcts_b200 import kernels as K
+
+    def fails(force=False):
+        raise RuntimeError("no headers here")
+
+    monkeypatch.setattr(build, "build_host", fails)
+    with pytest.warns(UserWarning, match="_host_calls.*no headers here"):
+        assert K._load_host_calls() is None
+    monkeypatch.undo()
+    assert K._load_host_calls() is not None
+
+
 def prefix_splits(B, H, Hkv, prefix, Lmax):
     """Splits of q40_attn_shared_prefix: the scratch that it asks for is theirs.  The scratch handed over is off its boundary, so nothing is launched."""
     from spec_mcts_b200._lib import lib

@@ -123,3 +123,12 @@ def test_interpreter_is_free_meanwhile(K, monkeypatch):
         _host_calls.init(address(K.lib.q40_matmul_tiled), address(K.lib.q40_gemm_nk))
     assert taken == [True, True]
     assert torch.equal(K.linear_q40(a, q, s, (512, 256)), y)
+
+
+def test_without_the_extension(K, monkeypatch):
+    a, q, s, shape = data(K, 9)
+    K.matmul_q40(a[:1].contiguous(), q, s, shape)
+    K.matmul_q40(a, q, s, shape)
+    c, y = K.matmul_q40(a, q, s, shape), K.linear_q40(a, q, s, (512, 256))
+    monkeypatch.setattr(K, "_host_calls", None)
+    assert torch.equal(K.matmul_q40(a, q, s, shape), c) and torch.equal(K.linear_q40(a, q, s, (512, 256)), y)
