@@ -282,7 +282,7 @@ class Transformer(nn.Module):
         # ... and all layers of a step of up to two branches as one launch, while the same limit holds
         self.use_chain = True
         self._chain_tables = {}     # its layers' addresses, as the kernel reads them
-        self._chained = {}          # by width: whether the last step that was enqueued (or captured) was such a launch
+        self._chained = {}          # by width: whether the last step was such a launch
         self._lm_head_q4 = None     # set by quantize_lm_head()
 
     # ------------------------------------------------------------------ reference API
@@ -644,6 +644,7 @@ class Transformer(nn.Module):
 
     def _decode_body(self, B):
         """Enqueue one decode step for B branches on the current stream (captured into a graph)."""
+        self._chained[B] = False
         if self._fused_body(B):
             return self._decode_body_fused(B)
         return self._decode_body_unfused(B)
@@ -1088,20 +1089,12 @@ class Transformer(nn.Module):
         self._check_prompt()
         self._check_steps()
         fused = self._fused_body(B)
-        per_layer = (5 if self._fused_attn_for(B) else 6) if fused else (8 if self._silu_pair(B, self.layers[0].feed_forward) else 9)
-        if not (fused and per_layer == 5 or self._rotates_in_attention(B)):
-            per_layer += 1
-        self.launches_per_step = self.params.n_layers * per_layer + (2 if self._narrow(B) else 1) + (not fused and self._fused_tail(B))
         if not self.use_cuda_graph:
             logits = self._decode_body(B)
-            if fused and self._chained.get(B):
-                self.launches_per_step = 2
+            self._count_launches(B, fused)
             return logits
-        key = (B, self.greedy_feedback, self.use_fused, self.use_pdl, self.max_cluster, self.use_stream,
-               self.use_tiled, self.use_fused_attn, self.fused_attn_max_width, self.stream_smem_budget,
-               self.use_fused_tail, self.use_tiled_tc, self.use_tp_fused_allreduce, self.use_chain)
-        g = self._graphs.get(key)
-        if g is None:
+        key = self._graph_key(B)
+        if key not in self._graphs:
             # torch requires capture on a side stream after a warm-up run; with greedy feedback that run
             # overwrites the input token and advances the position, so both are put back afterwards
             tok_saved = self._tok_dev[:B].clone() if self.greedy_feedback else None
@@ -1115,26 +1108,40 @@ class Transformer(nn.Module):
                         raise
                     # this device cannot schedule 16-CTA clusters: use the portable size
                     self.max_cluster = 8
-                    key = (B, self.greedy_feedback, self.use_fused, self.use_pdl, self.max_cluster, self.use_stream,
-                           self.use_tiled, self.use_fused_attn, self.fused_attn_max_width, self.stream_smem_budget,
-                           self.use_fused_tail, self.use_tiled_tc, self.use_tp_fused_allreduce, self.use_chain)
                     self._decode_body(B)
+            key = self._graph_key(B)              # with what the warm-up run has found out about the device
             torch.cuda.current_stream(self.device).wait_stream(s)
             torch.cuda.synchronize(self.device)
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g):
                 self._decode_body(B)
-            self._graphs[key] = g
+            self._graphs[key] = g, self._chained.get(B)
             if self.greedy_feedback:
                 # capture itself executes nothing
                 self._pos_dev[:B] -= 1
                 self._tok_dev[:B].copy_(tok_saved)
+        g, self._chained[B] = self._graphs[key]
         g.replay()
-        if fused and self._chained.get(B):
-            self.launches_per_step = 2
+        self._count_launches(B, fused)
         if self._lm_head_q4 is not None and fused:      # only narrow steps compute with it
             return self._bufs[B]["logits_pad"][:, :self.params.vocab_size]
         return self._bufs[B]["logits"]
+
+    def _graph_key(self, B):
+        """What decides the launches of a step of B branches."""
+        return (B, self.greedy_feedback, self.use_fused, self.use_pdl, self.max_cluster, self.use_stream,
+                self.use_tiled, self.use_fused_attn, self.fused_attn_max_width, self.stream_smem_budget,
+                self.use_fused_tail, self.use_tiled_tc, self.use_tp_fused_allreduce, self.use_chain, self.narrow_max)
+
+    def _count_launches(self, B, fused):
+        """launches_per_step of the step just enqueued."""
+        if fused and self._chained.get(B):
+            self.launches_per_step = 2
+            return
+        per_layer = (5 if self._fused_attn_for(B) else 6) if fused else (8 if self._silu_pair(B, self.layers[0].feed_forward) else 9)
+        if not (fused and per_layer == 5 or self._rotates_in_attention(B)):
+            per_layer += 1
+        self.launches_per_step = self.params.n_layers * per_layer + (2 if self._narrow(B) else 1) + (not fused and self._fused_tail(B))
 
 
 def random_init_(model: Transformer, seed: int = 0, std: float = 0.02) -> None:

@@ -9,7 +9,7 @@ def model(dim=2048, layers=2, max_b=9):
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     from spec_mcts_b200.model import ModelArgs, Transformer, random_init_
-    m = Transformer(ModelArgs(dim=dim, n_layers=layers, n_heads=dim // 128, n_kv_heads=4, vocab_size=1000, multiple_of=256, max_batch_size=max_b,
+    m = Transformer(ModelArgs(dim=dim, n_layers=layers, n_heads=dim // 128, n_kv_heads=4 if dim % 512 == 0 else None, vocab_size=1000, multiple_of=256, max_batch_size=max_b,
                               max_seq_len=32, max_prompt_seq_len=64))
     random_init_(m, seed=11, std=0.03)
     m(tokens(1, 1, 21), 0)
@@ -77,3 +77,28 @@ def test_ties_and_tail_switch(graph):
     m.use_fused_tail = False
     b = m(toks, 21).float().view(8, -1)
     assert ((a - b).norm() / b.norm()).item() < 1e-3
+
+
+def test_switches_choose_among_captured_steps():
+    """A graph is replayed for the switches that it was captured with, and the launches that are reported are its own."""
+    m = model(dim=2304, layers=2, max_b=6)              # 18 heads: one launch for all layers at widths 1 and 2
+    toks = tokens(7, 1, 1)
+    seen = {}
+    for chain in (True, False, True, False):
+        m.use_chain = chain
+        out = m(toks, 21).clone()
+        assert m._chained[1] == chain
+        assert seen.setdefault(chain, m.launches_per_step) == m.launches_per_step and torch.equal(seen.setdefault(("out", chain), out), out)
+    assert seen[True] == 2 < seen[False]
+    m.use_chain = True
+    m(toks, 21)
+    m.use_fused = False                                 # the launch-per-operation body, at a width that has just been one launch
+    m(toks, 21)
+    assert m.launches_per_step > 2 and not m._chained[1]
+    m.use_fused = True
+    toks, counts = tokens(8, 5, 1), {}
+    for most in (4, 8, 4):
+        m.narrow_max = most
+        m(toks, 21)
+        assert counts.setdefault(most, m.launches_per_step) == m.launches_per_step
+    assert counts[4] == 2 * 8 + 3 and counts[8] == 2 * 6 + 2
