@@ -314,6 +314,11 @@ class Transformer(nn.Module):
         captured its work is alive: call this before torch.distributed.destroy_process_group()."""
         torch.cuda.synchronize(self.device)
         self._graphs.clear()
+
+    def _forget_copies(self):
+        """... before tiled copies go away, and with them the tables that hold their addresses.  (Tables stay where graphs alone are released: a
+        graph that the caller has captured may read them.)"""
+        self.release_graphs()
         self._chain_tables.clear()
 
     # ------------------------------------------------------------------ prompt
@@ -662,7 +667,7 @@ class Transformer(nn.Module):
             c = self._tiled_copy(l)
             if c is None:
                 if l._tiled is not None:
-                    self.release_graphs()         # captured steps hold the address of the copy that goes away
+                    self._forget_copies()         # captured steps hold the address of the copy that goes away
                 c = l._tiled = K.TiledCopy(K.relayout_tiled(l.w, l.s, l.kn()), l.kn(), l.w, l.s)
                 pdl = False
             out.append(c.data)
@@ -677,7 +682,7 @@ class Transformer(nn.Module):
     def drop_tiled_copies(self):
         """Forget the rearranged weight copies (made again on the next step): for weights written in a way torch
         does not count, through `.data`, a raw pointer or under inference_mode."""
-        self.release_graphs()
+        self._forget_copies()
         for layer in self.layers:
             for l in _projections(layer):
                 l._tiled = l._tiled_cat = None
@@ -689,7 +694,7 @@ class Transformer(nn.Module):
         for l in lins:
             cat = l._tiled_cat
             if l._tiled is not None and self._tiled_copy(l) is None:
-                self.release_graphs()
+                self._forget_copies()
                 l._tiled = None
             if cat is not None and not cat.is_of(*self._concat_source(lins)):
                 self.release_graphs()

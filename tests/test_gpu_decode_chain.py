@@ -145,3 +145,27 @@ def test_sizes_that_leave_warps_without_work():
     for H, Hkv in [(14, 14), (14, 2), (6, 6), (12, 12)]:
         assert lib.q40_decode_chain_ws_bytes(1, 2, 2304, 6144, H, Hkv) == 0
     assert lib.q40_decode_chain_ws_bytes(1, 2, 2304, 6144, 16, 16) > 0
+
+
+def test_table_outlives_released_graphs():
+    """A graph that the caller captured reads the table of the layers' addresses: it goes with the tiled copies, not with the model's own graphs."""
+    m = model(layers=2)
+    m.use_cuda_graph = False
+    m(tokens(3, 1, 40), 0)
+    toks = tokens(4, 1, 1)
+    want = m(toks, 40).clone()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        m.decode_replay(1)
+    assert m._chained[1]
+    (table,) = m._chain_tables.values()
+    m.release_graphs()
+    assert next(iter(m._chain_tables.values())) is table
+    with torch.inference_mode():
+        m._bufs[1]["logits"].zero_()
+    g.replay()
+    assert torch.equal(m._bufs[1]["logits"].view(-1), want.view(-1))
+    del g
+    m.drop_tiled_copies()
+    assert not m._chain_tables
+    assert torch.equal(m(toks, 40), want)
