@@ -820,9 +820,10 @@ class Transformer(nn.Module):
         H, Hkv = self._H, self._Hkv
         shapes = [(p.dim, H * 128), (p.dim, Hkv * 128), (p.dim, Hkv * 128), (H * 128, p.dim), (p.dim, hid), (p.dim, hid), (hid, p.dim)]
         for layer in self.layers:
-            norms = (layer.attention_norm.weight, layer.ffn_norm.weight)
+            att, norms = layer.attention, (layer.attention_norm.weight, layer.ffn_norm.weight)
             if (any(l.group_size != 64 or l.kn() != kn for l, kn in zip(_projections(layer), shapes)) or
-                    any(w.dtype != DTYPE or not w.is_contiguous() or w.data_ptr() % 8 for w in norms)):
+                    any(w.dtype != DTYPE or not w.is_contiguous() or w.data_ptr() % 8 for w in norms) or
+                    any(c.stride() != (Hkv * 128, 128, 1) or c.data_ptr() % 16 for c in (att.cache_prompt_k, att.cache_prompt_v))):
                 return False
         rows = []
         for layer in self.layers:

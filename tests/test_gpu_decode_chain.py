@@ -169,3 +169,22 @@ def test_table_outlives_released_graphs():
     m.drop_tiled_copies()
     assert not m._chain_tables
     assert torch.equal(m(toks, 40), want)
+
+
+def test_prompt_caches_with_strides():
+    """Prompt caches that are views of something wider, head by head: the launches take their strides, the one launch leaves them to those."""
+    m = model(layers=2, kv_heads=8)
+    m(tokens(3, 1, 40), 0)
+    toks = tokens(4, 2, 1)
+    want = m(toks, 40).float()
+    assert m._chained[2]
+    for layer in m.layers:
+        att = layer.attention
+        for name in ("cache_prompt_k", "cache_prompt_v"):
+            old = getattr(att, name)
+            wide = torch.full((old.shape[1], old.shape[0] + 3, 128), float("nan"), dtype=old.dtype, device="cuda")
+            wide[:, :old.shape[0]] = old.transpose(0, 1)
+            setattr(att, name, wide[:, :old.shape[0]].transpose(0, 1))
+    m.release_graphs()
+    got = m(toks, 40).float()
+    assert not m._chained[2] and ((got - want).norm() / want.norm()).item() < 5e-3
