@@ -35,7 +35,7 @@ extern "C" {
 #define Q40_E_UNSUPPORTED (-5)
 
 const char* q40_strerror(int status);
-/* Library/ABI version, bumped when a signature changes. */
+/* Library/ABI version, bumped when a signature or what q40_relayout_tiled writes changes (2: low nibbles hold code + 8). */
 int q40_abi_version(void);
 /* The capture that `stream` takes part in, or 0: for hosts that keep scratch per stream, where what is made inside a
  * capture is ready in that graph's replays only. */
@@ -191,8 +191,9 @@ int q40_gemv_fused(int mode, int nmat, const void* const* bw, const void* const*
 int q40_gemv_fused_ss_count(int N, int K, int max_cluster);
 
 /* Tiled copy of a packed [K, N] matrix for q40_gemv_tiled (N % 256 == 0, K % 16 == 0): a one-time
- * device pass that rearranges codes and scales (none is changed) so that the decode matmul needs
- * about one instruction per weight.  `out` has q40_tiled_bytes(N, K) bytes (= packed + scales).
+ * device pass that rearranges codes and scales (codes in low nibbles are stored plus 8, scales as they are) so that the decode
+ * matmul needs about one instruction per weight.  `out` has q40_tiled_bytes(N, K) bytes (= packed + scales).  A copy is for the
+ * library that made it, or one of the same q40_abi_version: keep the packed matrix, not the copy.
  * No counterpart in the reference (its Triton kernel reads the checkpoint layout directly). */
 size_t q40_tiled_bytes(int N, int K);
 int q40_relayout_tiled(const void* bw, const void* bs, void* out, int N, int K, void* stream);

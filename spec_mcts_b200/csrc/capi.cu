@@ -1,7 +1,7 @@
 // Status strings and ABI version of the q40b200 library.
 #include "q40_common.cuh"
 
-extern "C" int q40_abi_version(void) { return 1; }
+extern "C" int q40_abi_version(void) { return 2; }
 
 extern "C" const char* q40_strerror(int status) {
   switch (status) {

@@ -55,6 +55,12 @@ def test_workspace_of_a_single_output():
             assert lib.q40_gemm_workspace_bytes(M, 1, Kd) >= lib.q40_gemm_workspace_bytes(M, 2, Kd) > 4096
 
 
+def test_abi_version_covers_the_tiled_layout():
+    """Low nibbles of a tiled copy hold code + 8 since version 2."""
+    from spec_mcts_b200._lib import lib
+    assert lib.q40_abi_version() == 2
+
+
 def test_extension_is_built_for_this_torch(monkeypatch):
     import torch
     from spec_mcts_b200 import build
