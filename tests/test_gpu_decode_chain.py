@@ -188,3 +188,47 @@ def test_prompt_caches_with_strides():
     m.release_graphs()
     got = m(toks, 40).float()
     assert not m._chained[2] and ((got - want).norm() / want.norm()).item() < 5e-3
+
+
+def layer64(m, tok, pos):
+    """One layer's step of one branch without own keys, sums and weights in 64 bits, activations rounded where the reference rounds them."""
+    from spec_mcts_b200 import kernels as K
+    layer, S = m.layers[0], int(m._prefix_len_dev)
+    att, ff, H = layer.attention, layer.feed_forward, m._H
+
+    def lin(x, l):
+        q = l.w.reshape(-1, 64)
+        w = torch.cat((q >> 4, (q << 4) >> 4), 1).view(-1, 64).double() * l.s.reshape(-1, 1).double()
+        return (x.double() @ w.view(l.kn())).half()
+
+    def norm(h, w):
+        return (h.double() * (h.double().square().mean() + m.params.norm_eps).rsqrt()).half() * w
+
+    h = m.tok_embeddings.weight[tok]
+    x, p = norm(h, layer.attention_norm.weight), torch.tensor([pos], device="cuda")
+    q, k = (K.rope_(lin(x, l).view(1, H, 128), p, m._cos, m._sin)[0] for l in (att.wq, att.wk))
+    keys, values = (torch.cat((c[:S], new[None])).double() for c, new in ((att.cache_prompt_k, k), (att.cache_prompt_v, lin(x, att.wv).view(H, 128))))
+    w = torch.softmax(torch.einsum("hd,khd->hk", q.double(), keys) / 128 ** 0.5, -1)
+    h = h + lin(torch.einsum("hk,khd->hd", w, values).reshape(-1).half(), att.wo)
+    x = norm(h, layer.ffn_norm.weight)
+    a = lin(x, ff.w1)
+    return h + lin((a.double() * torch.sigmoid(a.double())).half() * lin(x, ff.w3), ff.w2)
+
+
+@pytest.mark.parametrize("ratio", [1, 1000, 10000])
+def test_one_activation_far_above_the_rest(ratio):
+    """128 activations share an exponent: with one of them `ratio` times the rest, the layer's result in all other columns is no further from 64 bits
+    than that of the launches, which round each scale * x to fp16."""
+    m = model()
+    m(tokens(3, 1, 20), 0)
+    with torch.no_grad():
+        m.tok_embeddings.weight[7, 100] = 0.03 * ratio
+    want = layer64(m, 7, 20).double()
+    rest = torch.arange(4096, device="cuda") != 100
+    change, errors = (want - m.tok_embeddings.weight[7].double())[rest].norm(), {}
+    for chain in (False, True):
+        m.use_chain = chain
+        m(torch.tensor([[7]], device="cuda"), 20)
+        assert m._chained[1] == chain
+        errors[chain] = ((m._bufs[1]["h"][0].double() - want)[rest].norm() / change).item()
+    assert errors[True] < 1.05 * errors[False] < 5e-3
