@@ -10,8 +10,9 @@ by all branches, then greedy decode steps at tree width 1 (headline), 10 and 100
 A "step" is one decode step of all `width` branches; value = width * steps / time.
 
 Printed line (rank 0): the driver's JSON contract, plus
-  roofline      the fused dequant-matmul kernel on the model's own 224 weight matrices
-                (larger than L2, streamed in layer order), algorithmic bytes / CUDA-event time
+  roofline      the kernel of the headline step: all layers in one launch, algorithmic bytes of its matmuls / CUDA-event time
+  roofline_matmul_launches  the fused dequant-matmul kernel of 3 and 4 branches on the model's own 224 weight matrices
+                (larger than L2, streamed in layer order), likewise
   cpu_baseline  the reference's CPU path (torch unpack + matmul) on the host cores, bounded
                 sample: the 7 linears of one layer, extrapolated to a token
   e2e           the same metric through model(tokens, start_pos) with host tokens in pinned
@@ -403,8 +404,45 @@ def reference_class_on_drop_in(model, dev, steps=16):
             "tokens_per_s": steps / sec, "ms_per_step": sec / steps * 1e3}
 
 
+def timed_graph(dev, one_pass, reps):
+    """Seconds of `reps` replays of the captured work, by CUDA events on the replaying stream."""
+    import torch
+    side = torch.cuda.Stream(dev)
+    side.wait_stream(torch.cuda.current_stream(dev))
+    with torch.cuda.stream(side):
+        one_pass()
+    torch.cuda.current_stream(dev).wait_stream(side)
+    torch.cuda.synchronize(dev)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        one_pass()
+    for _ in range(3):
+        g.replay()
+    torch.cuda.synchronize(dev)
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    e0.record()
+    for _ in range(reps):
+        g.replay()
+    e1.record()
+    torch.cuda.synchronize(dev)
+    return e0.elapsed_time(e1) * 1e-3
+
+
+def chain_roofline(model, width, reps):
+    """The launch that does all layers of a step of `width` branches, alone, 64 tokens behind the prompt; None where a step is several."""
+    import torch
+    from spec_mcts_b200.model import _projections
+    bufs = model._step_buffers(width)
+    model._pos_dev[:width] = PROMPT_LEN + 64
+    if not model._chain(width, bufs, torch.cuda.current_stream(model.device).cuda_stream):
+        return None
+    sec = timed_graph(model.device, lambda: model._chain(width, bufs, torch.cuda.current_stream(model.device).cuda_stream), reps)
+    nbytes = sum(q4_bytes(l.kn()[1], l.kn()[0], width) for layer in model.layers for l in _projections(layer))
+    return reps * nbytes / sec / 1e9, sec / reps, nbytes, "decode_chain_kernel<%d>" % width
+
+
 def gemv_roofline(model, width, reps):
-    """The dominant kernel alone: every Q4_0 matmul of the model in layer order (3.4 GB of
+    """The dominant kernel of a step by launches alone: every Q4_0 matmul of the model in layer order (3.4 GB of
     distinct weights per pass, so nothing is served from L2), launched exactly as a decode step
     of three or four branches launches them (the cluster-reduced kernel, [wq,wk,wv] and [w1,w3] sharing a
     launch; one and two branches have one launch for all layers, more than four the tensor-core kernel) but with nothing in between, replayed from a CUDA graph so that the host does not
@@ -436,25 +474,7 @@ def gemv_roofline(model, width, reps):
                 check(lib.q40_gemm_kn(xs[k].data_ptr(), k, grp[0].w.data_ptr(), grp[0].s.data_ptr(), out.data_ptr(),
                                       3 * FFN, width, n, k, 64, ws.data_ptr(), ws.numel(), st))
 
-    side = torch.cuda.Stream(dev)
-    side.wait_stream(torch.cuda.current_stream(dev))
-    with torch.cuda.stream(side):
-        one_pass()
-    torch.cuda.current_stream(dev).wait_stream(side)
-    torch.cuda.synchronize(dev)
-    g = torch.cuda.CUDAGraph()
-    with torch.cuda.graph(g):
-        one_pass()
-    for _ in range(3):
-        g.replay()
-    torch.cuda.synchronize(dev)
-    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    e0.record()
-    for _ in range(reps):
-        g.replay()
-    e1.record()
-    torch.cuda.synchronize(dev)
-    sec = e0.elapsed_time(e1) * 1e-3
+    sec = timed_graph(dev, one_pass, reps)
     passes = (width + 15) // 16 if not fused else 1
     launches = reps * len(groups) * passes
     total_bytes = reps * sum(q4_bytes(l.kn()[1], l.kn()[0], width) for grp in groups for l in grp)
@@ -951,7 +971,8 @@ def main():
                 dist.all_reduce(t, op=dist.ReduceOp.MAX)
                 sec = float(t.item())
             e2e_res[w] = (sec, h2d, d2h)
-        roof = gemv_roofline(model, widths[0], reps=5) if rank == 0 else None
+        roof_launches = gemv_roofline(model, widths[0], reps=5) if rank == 0 else None
+        roof = (chain_roofline(model, widths[0], reps=20) or roof_launches) if rank == 0 else None
         by_path = None
         if rank == 0 and world == 1 and not args.no_extras:
             # the same step with the kernels that keep the reference's operand rounding, fp16(code * scale)
@@ -987,7 +1008,12 @@ def main():
         w0 = widths[0]
         tok_s = {w: world * w * steps / results[w] for w in widths}
         e2e_tok_s = {w: world * w * steps / e2e_res[w][0] for w in widths}
-        ach, sec_per_launch, bytes_per_launch, roof_kernel = roof
+
+        def roof_entry(ach, sec_per_launch, bytes_per_launch, kernel):
+            return {"bound": "hbm", "kernel": kernel, "achieved": ach, "peak": hbm_peak, "peak_kind": peak_kind, "unit": "GB/s",
+                    "frac": ach / hbm_peak, "avg_launch_us": sec_per_launch * 1e6, "alg_bytes_per_launch": bytes_per_launch,
+                    "traffic": measured_traffic(kernel.split("<")[0])}
+
         step_bytes = step_weight_bytes()
         line = {
             "metric": METRIC, "value": tok_s[w0], "unit": UNIT, "n_gpus": world, "steps": steps, "warmup": warmup,
@@ -999,10 +1025,8 @@ def main():
             "step_weight_stream": {"bytes_per_step": step_bytes,
                                    "achieved_gbs": step_bytes / (results[w0] / steps) / 1e9,
                                    "frac_of_%s_hbm" % peak_kind: step_bytes / (results[w0] / steps) / 1e9 / hbm_peak},
-            "roofline": {"bound": "hbm", "kernel": roof_kernel, "achieved": ach, "peak": hbm_peak,
-                         "peak_kind": peak_kind, "unit": "GB/s", "frac": ach / hbm_peak,
-                         "avg_launch_us": sec_per_launch * 1e6, "alg_bytes_per_launch": bytes_per_launch,
-                         "traffic": measured_traffic(roof_kernel.split("<")[0])},
+            "roofline": roof_entry(*roof),
+            "roofline_matmul_launches": roof_entry(*roof_launches),
             "e2e": {"value": e2e_tok_s[w0], "unit": UNIT, "h2d_bytes_per_step": e2e_res[w0][1],
                     "d2h_bytes_per_step": e2e_res[w0][2]},
             "prefill_ms": prefill_ms,      # prompt pass of PROMPT_LEN tokens (not part of the decode metric)
