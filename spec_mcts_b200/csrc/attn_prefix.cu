@@ -159,8 +159,8 @@ static int prefix_splits(int B, int H, int Hkv, int prefix_len, int64_t own) {
   int want = (148 * per_sm) / (Hkv * rblocks);
   if (want < 1) want = 1;
   if (want > tiles) want = tiles;
-  // How many tiles a split has.  A tile costs it 1.0 us (1.9 with eight warps); the merge has 16 splits of a row on their way at once and reads further ones one by
-  // one, 0.07 us each; a second CTA on an SM costs 2.3 us that matter less the longer splits are.  Us by splits, 8 query heads a kv head:
+  // How many tiles a split has.  A tile costs it 1.0 us (1.9 with eight warps); the merge has 16 splits of a row on their way at once (8 where a row has two
+  // warps) and reads further ones one by one, 0.07 us each, more behind many own keys; a second CTA on an SM costs 2.3 us that matter less the longer splits are.  Us by splits, 8 query heads a kv head:
   // 1 kv head, 1 branch, 2048 keys 16 splits 6.1, 32 7.3; 8192 keys 16 12.4, 32 10.4, 128 14.1; 32768 keys 16 37.3, 64 16.8, 256 24.9; 8 kv heads
   // x 4, 4 branches, 2048 keys 16 7.7, 32 10.6; 32768 keys 16 44.1, 32 30.5.  Over 448 sizes of 1 to 32 kv heads and 512 to 32768 keys 5 % less
   // time than with as many splits as SMs take, four of them 3 to 9 % more (1 kv head x 4, 34 branches, 8192 keys 15.9 and 17.3)

@@ -7,8 +7,8 @@
 // in global memory.  Operands are the reference's: fp16(code * scale), fp32 sums.
 //
 // What bounds it: instructions of the expansion (about 230 a warp and 128 k of 16 rows, of which 100 make operands) and a warp's chain
-// of loads, four of 1 KB on their way.  Microseconds, here and by gemv_nk_kernel (64 rows x part of k per CTA, scratch and
-// tickets): 10 rows x 4096 x 11008 13.7 and 18.2, x 11008 x 4096 17.8 and 18.7; 1 row x 4096 x 4096 5.8 and 7.6, x 11008 x 11008
+// of loads, four of 1 KB on their way.  Microseconds of the launch alone with W in L2, here and by gemv_nk_kernel (64 rows x part of k per CTA,
+// scratch and tickets): 10 rows x 4096 x 11008 13.7 and 18.2 (calls of linear_q40 one after the other: 14.3 and 18.4), x 11008 x 4096 17.8 and 18.7; 1 row x 4096 x 4096 5.8 and 7.6, x 11008 x 11008
 // 24.0 and 27.7; 10 rows x 1024 x 1000 4.0 and 7.0; 20 rows x 4096 x 11008 20.1 and 29.3.  No gain: weights prefetched to L2 at the
 // start (14.2).
 #include <cooperative_groups.h>

@@ -236,8 +236,8 @@ class Transformer(nn.Module):
         # written to tensor memory); False: B <= 16 as B <= narrow_max, above the tensor-core matmul on the checkpoint layout
         self.use_tiled_tc = True
         # steps of more branches than this take it: where a layer's launches, three more of them, have enough to do.  Us a step of 8
-        # layers (prompt 512, 64 own keys), the narrow matmuls and it: dim 4096, 4 branches 534 and 551, 5 565 and 545, 8 608 and 557;
-        # dim 2048, 5 branches 390 and 333; dim 1024, 5 255 and 269, 8 291 and 270; dim 512, 5 212 and 257, 8 233 and 256
+        # layers (prompt 512, 64 own keys), the narrow matmuls and it: dim 4096, 4 branches 528 and 549, 5 560 and 548, 8 605 and 560;
+        # dim 2048, 5 branches 403 and 344; dim 1024, 5 260 and 276, 8 298 and 280; dim 512, 5 213 and 256, 8 222 and 257
         self.narrow_max = 4 if tp_world == 1 and params.dim >= 2048 else 8
         # tensor parallel: all-reduce + residual add + RMSNorm as one launch over peer-mapped buffers (plain
         # stores into the peers' memory); False: torch.distributed all_reduce + the norm kernel
@@ -266,9 +266,8 @@ class Transformer(nn.Module):
         # False: the cluster-reduced launch on the same tiled copies (faster on B200, the default)
         self.use_stream = False
         self.stream_smem_budget = 0      # 0 = the library's default (two launches' CTAs share an SM)
-        # width <= 16: rotary embedding, cache append and attention as one cluster launch
         # single-launch attention (rotary + append + attention) up to this width; wider steps read the
-        # shared prompt once for all branches with the three-launch path
+        # shared prompt once for all branches (see `_attn_step`)
         # width <= 8: final RMSNorm, fp16 lm_head, arg-max and position bump as one launch (above, the
         # library GEMM is faster than the streaming kernel).  Us of a step of 8 layers behind the
         # tensor-core matmuls, with torch's product and arg-max and with it: dim 4096, 5 branches 545 and 549, with feedback
@@ -572,7 +571,7 @@ class Transformer(nn.Module):
         return True
 
     def _gemm_multi(self, bufs, x, lins, outs, st):
-        """Several projections of the same activations: one tensor-core launch above 8 rows when the
+        """Several projections of the same activations: one tensor-core launch above `narrow_max` rows when the
         shapes allow it, one launch per matrix otherwise."""
         M, n = x.shape[0], len(lins)
         if M > self.narrow_max and self.use_tiled and self.use_tiled_tc and x.stride(0) % 8 == 0:
