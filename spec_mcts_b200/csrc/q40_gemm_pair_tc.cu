@@ -24,25 +24,22 @@
 // pair waits for lower-numbered pairs only, and those publish before they wait, so that no order of scheduling can make
 // them wait for each other.  Results depend on nothing but operands and grid.
 //
-// What bounds it, per 128 k of a tile (cycles): up to 96 rows the dequantisers' instructions (460; two thousand issue slots of
-// four schedulers), at 112 and 128 rows the MMAs (500 and 545 with their gaps, 450 and 512 without), above, with all SMs
-// busy, loads from L2 (512 rows x 4096 x 11008: 26 bytes a cycle and SM over a launch).  A launch adds 4 to 5.4 us: set-up and the first stages'
-// latency 2, the last accumulator's way out 1 to 2, draining.  Microseconds, here and by the kernels before (one CTA per
-// tile, k split over clusters; up to 16 rows q40_gemv_tiled): 10 rows x 11008 x 4096 13.0 and 16.8, two x 4096 x 11008 16.9 and
-// 22.9; 100 rows x 11008 x 4096 15.7 and 20.8, two x 4096 x 11008 21.8 and 34.1; 512 rows x 4096 x 11008 45.4 and 61.4,
-// three x 4096 x 4096 45.5 and 82.5, x 11008 x 4096 37.2 and 48.6.  With the SiLU product: 10 rows 17.1 (18.8 while w1's and w3's
-// sums met through the other CTA's shared memory), 77 rows 21.9 (23.0), 100 rows 25.0 (27.7), 512 rows 72 (76); expf and the
-// division are half of what it costs (100 rows: 22.6 with approximate ones).
+// What bounds it, per 128 k of a tile (cycles): up to 96 rows the dequantisers (430; their loop alone takes 343, of which 260 are the
+// half-rate fp16 subtractions and multiplications), at 112 and 128 rows the MMAs (500 and 545 with their gaps, 450 and 512 without), above,
+// with all SMs busy, loads from L2 (512 rows x 4096 x 11008: 26 bytes a cycle and SM over a launch).  A launch adds 3.4 to 5: what its CTAs do
+// first (1.2, beside the launch in front where that leaves SMs free), activations 0.8, the last accumulator's way out 0.6 to 1.5, the end 0.6.
+// As many A buffers as tensor memory has room for (seven up to 32 rows, with four a dequantiser waited half its time for the MMAs of the
+// block before), the first of them filled while the launch in front still writes the activations; one warp of the epilogue polls.
+// Microseconds, launches in a row, before these and now: 10 rows x 4096 x 4096 8.2 and 6.9, three of them 13.2 and 12.6, x 11008 x 4096
+// 13.1 and 12.0; 100 rows 10.0 and 9.2, 16.1 and 14.5, 15.3 and 14.7.  With the SiLU product: 10 rows x 4096 x 11008 17.5 and 16.4, 64 rows
+// 22.7 and 20.2, 100 rows 28.5 and 25.2, 512 rows 87.8 and 79.9 (eight quotients in flight at once: see silu); 512 rows without it,
+// whose k blocks wait for L2, 45.8 and 48.0 x 11008, 42.5 and 43.0 x 11008 x 4096.
 //
 // Every wait is bounded (by seconds): on expiry an error word is set and no more copies are requested; what is still
 // multiplied and stored is undefined, as is the scratch.  Copies and MMAs in flight are waited for, tensor memory is freed.
-#include <cooperative_groups.h>
-
 #include <algorithm>
 
 #include "q40_tc_common.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace q40 {
 namespace ttc {
@@ -60,11 +57,11 @@ constexpr int RAW_BYTES = RAW_W + RAW_S;
 constexpr int RAW_PAD = 9216;                   // next multiple of 1024 (the B tiles want that alignment)
 constexpr int S_MAX = 16;                       // ring stages
 constexpr int A_COLS = 32 * BLK;                // tensor-memory columns of an A buffer
-constexpr int NA_MAX = 4;
+constexpr int NA_MAX = 8;
 constexpr int TMEM_COLS = 512;
 constexpr int CUT = 2;                          // a k range is cut at multiples of so many blocks
 constexpr int GROUPS = 1 + DSETS;               // of four warps, one per tensor-memory quadrant, that finish a pair's last tile
-constexpr int BAR_BYTES = 16 * S_MAX + 8 * NA_MAX + 64;
+constexpr int BAR_BYTES = 24 * S_MAX + 8 * NA_MAX + 64;
 constexpr uint32_t FLAG_POLLS = 1u << 22;       // of one flag, before giving up: seconds, like the other waits
 constexpr int OUT_LD = FEATS + 8;              // halves between rows that wait in shared memory
 constexpr int MAX_PAIRS = 128;
@@ -85,9 +82,9 @@ struct Params {
                            // the sums of a tile's ranges are added in order
   int cut;                 // tiles may be shared between pairs along k (scratch given)
   int share, rest;         // cut: a pair has share units of CUT blocks, the first `rest` pairs one more
-  int bps;                 // SPLIT: blocks of a rank
-  int stages, nacc;        // ring stages, accumulators
-  int run_off, out_off, bar_off;           // byte offsets in the aligned shared memory
+  int bps, own;            // SPLIT: blocks of a rank, and of the four-row groups that it finishes
+  int stages, nacc, na;    // ring stages, accumulators, A buffers
+  int run_off, out_off, bar_off;           // byte offsets in the aligned shared memory (run: SPLIT: sums of the other ranks)
   int silu;                // c[0] = silu(A @ deq(B_0)) * (A @ deq(B_1)): a tile is 128 features of
                            // both, of which a CTA has 64 (its A rows 0..63 those of matrix 0)
   int vec;                 // outputs take 16-byte stores
@@ -114,7 +111,7 @@ struct Slot {
   int i = 0;
   uint32_t turn = 0;
   __device__ __forceinline__ void next(int n) { if (++i == n) { i = 0; turn ^= 1; } }
-  __device__ __forceinline__ void next4(int n) { i += 4; if (i >= n) { i -= n; turn ^= 1; } }     // n >= 4
+  __device__ __forceinline__ void next4(int n) { for (i += 4; i >= n; i -= n) turn ^= 1; }
 };
 __device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
   uint32_t r;
@@ -126,6 +123,30 @@ __device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
 // dequantiser warp 1100 cycles
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// Four values into the shared memory of a CTA of the cluster, counted by a barrier there
+__device__ __forceinline__ void push4(uint32_t dst, const uint32_t (&v)[4], uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+               ::"r"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void ld4(uint32_t taddr, uint32_t (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
+}
+__device__ __forceinline__ void wait_ld4(uint32_t (&r)[4]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]) :: "memory");
+}
+// x / (1 + exp(-x)) for x that fp16 can hold, rounded once as the division operator does, without its branch for operands that cannot
+// occur here: eight of them in flight take a fifth of the time.  The quotient by one Newton step for the reciprocal and the
+// remainder of the product (P. Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, 1990).
+// Beyond 32 the divisor is 1; below -80 the result is -0 in fp16 whatever the exponential
+__device__ __forceinline__ float silu(float x) {
+  const float d = 1.0f + expf(fminf(-x, 80.0f));
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  r = fmaf(fmaf(-d, r, 1.0f), r, r);
+  const float q = x * r;
+  return x > 32.0f ? x : fmaf(fmaf(-d, q, x), r, q);
 }
 __device__ __forceinline__ void commit2(uint32_t bar, uint16_t mask) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
@@ -163,7 +184,7 @@ __device__ __forceinline__ void store_rows(const __half* o, __half* c, int64_t l
 // First block of pair q
 __device__ __forceinline__ int first_block(const Params& p, int q, int npairs) {
   if (q >= npairs) return p.ntiles * p.nblk;
-  if (!p.cut) return (int)((int64_t)p.ntiles * q / npairs) * p.nblk;
+  if (!p.cut) return (int)((uint32_t)p.ntiles * (uint32_t)q / (uint32_t)npairs) * p.nblk;
   return CUT * (q * p.share + min(q, p.rest));
 }
 
@@ -188,12 +209,12 @@ struct KCursor {
 struct Work {
   int u0, u1, nblk, t0, t1, np;
   bool pub;
-  __device__ __forceinline__ Work(int a, int b, int n) : u0(a), u1(b), nblk(n) {
-    t0 = u0 / n;
-    t1 = u1 > u0 ? (u1 - 1) / n : t0;
+  __device__ __forceinline__ Work(int4 w, int n) : u0(w.x), u1(w.y), nblk(n), t0(w.z), t1(w.w) {
     np = u1 > u0 ? t1 - t0 + 1 : 0;
     pub = u1 > u0 && u1 < (t1 + 1) * n;
   }
+  // First and last block (exclusive) of the pair, and their tiles
+  static __device__ __forceinline__ int4 share(int a, int b, int n) { return make_int4(a, b, a / n, (max(b, a + 1) - 1) / n); }
   __device__ __forceinline__ void piece(int k, int& tile, int& b0, int& b1) const {
     tile = k == np - 1 ? t0 : (pub ? (k == 0 ? t1 : t0 + k) : t0 + 1 + k);
     b0 = tile == t0 ? u0 - tile * nblk : 0;
@@ -205,38 +226,35 @@ struct Work {
 // distributed shared memory.  Otherwise a cluster is a pair.
 // CUT: tiles may be shared between pairs along k; SILU: see Params (compiled for each, to keep the registers of all roles
 // below the 80 that 24 warps leave)
-template <bool SPLIT, int NA, bool CUT_K, bool SILU>
+template <bool SPLIT, bool CUT_K, bool SILU>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
   extern __shared__ unsigned char smem_raw[];
-  cg::cluster_group cluster = cg::this_cluster();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int half = blockIdx.x & 1, me = blockIdx.x >> 1, npairs = gridDim.x >> 1;
   const uint32_t lead = SPLIT ? 2 * blockIdx.y : 0;          // rank of the pair's even CTA in the cluster
-  const int S = p.stages;                                    // at least as many as A buffers, and four
+  const int S = p.stages, NA = p.na;                         // at least as many stages as A buffers, and four
   const uint32_t b_bytes = (uint32_t)p.npad * 64u;           // B tile of a k step: npad / 2 rows x 64 k x 2 B
   const uint32_t stage_bytes = RAW_PAD + BLK * b_bytes;
 
   const uint32_t raw0 = smem_u32(smem_raw);
   const uint32_t ring = (raw0 + 1023u) & ~1023u;
   unsigned char* gbase = smem_raw + (ring - raw0);
-  // Block i has stage and barriers i % S and A buffer i % NA.  full: its weights and activations have landed in this
-  // CTA; mdone: its MMAs are complete, in both CTAs; accfull[b]: an accumulator is complete.  In the even CTA, for both:
-  // afull: the A operand is written (and the activations have landed); accfree[b]: an accumulator has been read.
-  const uint32_t bar_full = ring + (uint32_t)p.bar_off, bar_mdone = bar_full + 8 * S_MAX, bar_afull = bar_mdone + 8 * S_MAX,
-                 bar_accfull = bar_afull + 8 * NA_MAX, bar_accfree = bar_accfull + 16, bar_done = bar_accfree + 16, bar_last = bar_done + 8;
+  // Block i has stage and barriers i % S and A buffer i % NA.  full: its weights have landed in this
+  // CTA (act: its activations); mdone: its MMAs are complete, in both CTAs; accfull[b]: an accumulator is complete.  In the even CTA, for
+  // both: afull: the A operand is written (and the activations have landed); accfree[b]: an accumulator has been read.
+  const uint32_t bar_full = ring + (uint32_t)p.bar_off, bar_act = bar_full + 8 * S_MAX, bar_mdone = bar_act + 8 * S_MAX,
+                 bar_afull = bar_mdone + 8 * S_MAX, bar_accfull = bar_afull + 8 * NA_MAX, bar_accfree = bar_accfull + 16,
+                 bar_done = bar_accfree + 16, bar_last = bar_done + 8, bar_flags = bar_last + 8, bar_recv = bar_flags + 8;
   unsigned char* tail = gbase + p.bar_off + BAR_BYTES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail);
   volatile int* s_failed = reinterpret_cast<volatile int*>(tail + 8);
   volatile int* s_acc = reinterpret_cast<volatile int*>(tail + 24);        // accumulator of a pair's last tile
-  volatile int* s_copied = reinterpret_cast<volatile int*>(tail + 16);     // [2] blocks whose copies were requested
+  volatile int* s_copied = reinterpret_cast<volatile int*>(tail + 16);     // [2] see copy_blocks
+  int4* s_share = reinterpret_cast<int4*>(tail + 32);                      // see Work::share
   float* run = reinterpret_cast<float*>(gbase + p.run_off);                // [npad][128] sums of earlier ranges
   __half* out_s = reinterpret_cast<__half*>(gbase + p.out_off);            // [2][16][OUT_LD] finished rows on their way out
 
-  const int sb0 = SPLIT ? blockIdx.y * p.bps : 0, sb1 = SPLIT ? min(p.nblk, sb0 + p.bps) : 0;
-  const Work wk(SPLIT ? me * p.nblk + sb0 : first_block(p, me, npairs),
-                SPLIT ? me * p.nblk + sb1 : first_block(p, me + 1, npairs), p.nblk);
-  const int total = wk.u1 - wk.u0;                    // blocks of this pair
   // matrix, span, 128-feature half of this CTA (SiLU: of the tile, in both matrices) and first row of a tile
   auto decode = [&](int tile, int& pi, int& span, int& fh, int& m0) {
     span = tile / p.chunks;
@@ -254,103 +272,113 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
   bool failed = false;
   uint32_t limit = SPIN_LIMIT;                               // see wait_limited
 
-  // ---- weights: they do not depend on the previous launch, so the first stages are requested before anything else ----
-  int wi = 0;                                                // blocks requested
-  Slot wslot;
-  auto stream_weights = [&](int limit) {
-    int i = 0;
-    for (int k = 0; k < wk.np && wi < limit && !failed; ++k) {
+  // ---- copies of blocks first .. last - 1 of the pair, weights or activations.  `first`: 0, or S where the first S have been requested:
+  // weights do not depend on the previous launch, so their first stages are, before anything else ----
+  int requested = 0;
+  auto copy_blocks = [&](const Work& wk, int first, int last, bool weights) {
+    int i = 0;                                               // first block of a piece
+    Slot sl;
+    sl.turn = first > 0;
+    requested = first;
+    for (int k = 0; k < wk.np && i < last; ++k) {
       int tile, b0, b1, pi, span, fh, m0;
       wk.piece(k, tile, b0, b1);
-      if (i + b1 - b0 <= wi) { i += b1 - b0; continue; }
+      const int from = max(first - i, 0), to = min(b1 - b0, last - i);
+      i += b1 - b0;
+      if (from >= to) continue;
       decode(tile, pi, span, fh, m0);
-      KCursor kc(p, b0 + (wi - i));
-      for (int b = b0 + (wi - i); b < b1 && wi < limit; ++b, kc.next(p)) {
-        const int s = wslot.i;
-        if (wi >= S && !mbar_wait(bar_mdone + 8 * s, wslot.turn ^ 1)) { failed = true; break; }
+      KCursor kc(p, b0 + from);
+      for (int b = from; b < to; ++b, kc.next(p)) {
+        const int s = sl.i;
+        if (requested >= S) wait_limited(bar_mdone + 8 * s, sl.turn ^ 1, limit);
+        if (limit == 0) return;
         const uint32_t dst = ring + s * stage_bytes;
-        const int step = (span * p.k64 + kc.k) * 4;
-        mbar_expect_tx(bar_full + 8 * s, RAW_BYTES);
-        if constexpr (SILU) {                                                    // a 64-column group of each matrix
+        if (weights) {
+          const int step = (span * p.k64 + kc.k) * 4;
+          mbar_expect_tx(bar_full + 8 * s, RAW_BYTES);
+          if constexpr (SILU) {                                                  // a 64-column group of each matrix
 #pragma unroll
-          for (int m = 0; m < 2; ++m) {
-            tma_2d(dst + m * (RAW_W / 2), &maps.w[m], fh * 256 + half * 128, step, bar_full + 8 * s);    // x in words of four bytes
-            tma_2d(dst + RAW_W + m * (RAW_S / 2), &maps.s[m], 512 + fh * 16 + half * 8, step, bar_full + 8 * s);
+            for (int m = 0; m < 2; ++m) {
+              tma_2d(dst + m * (RAW_W / 2), &maps.w[m], fh * 256 + half * 128, step, bar_full + 8 * s);    // x in words of four bytes
+              tma_2d(dst + RAW_W + m * (RAW_S / 2), &maps.s[m], 512 + fh * 16 + half * 8, step, bar_full + 8 * s);
+            }
+          } else {
+            tma_2d(dst, &maps.w[pi], fh * 256, step, bar_full + 8 * s);
+            tma_2d(dst + RAW_W, &maps.s[pi], 512 + fh * 16, step, bar_full + 8 * s);
           }
         } else {
-          tma_2d(dst, &maps.w[pi], fh * 256, step, bar_full + 8 * s);
-          tma_2d(dst + RAW_W, &maps.s[pi], 512 + fh * 16, step, bar_full + 8 * s);
+          // the second k step of a range's last block may be the next range's or beyond K (zeros): not multiplied
+          mbar_expect_tx(bar_act + 8 * s, BLK * b_bytes);
+#pragma unroll
+          for (int h = 0; h < BLK; ++h)
+            tma_2d(dst + RAW_PAD + h * b_bytes, &maps.act, (kc.k + h) * BK, m0 + half * (p.npad / 2), bar_act + 8 * s);
         }
-        wslot.next(S);
-        ++wi;
+        ++requested;
+        sl.next(S);
       }
-      i += b1 - b0;
     }
   };
+  // Until then, only the warps that have something to do run: with all 24 finding out their share (five divisions) first, the first
+  // weights were requested 1.4 to 1.9 us after the start of a CTA
   if (warp == 0) {
     if (lane == 0) {
       *s_failed = 0;
-      for (int s = 0; s < S; ++s) {
-        mbar_init(bar_full + 8 * s, 2);
-        mbar_init(bar_mdone + 8 * s, 1);
-      }
-      for (int s = 0; s < NA; ++s) mbar_init(bar_afull + 8 * s, 8);
-      for (int s = 0; s < 2; ++s) { mbar_init(bar_accfull + 8 * s, 1); mbar_init(bar_accfree + 8 * s, 8); }
       mbar_init(bar_done, 1);
       mbar_init(bar_last, 4);
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      mbar_init(bar_flags, 4);
+      mbar_init(bar_recv, 1);
+      if (SPLIT) {
+        const int own = min(p.own, (p.M + 3) / 4 - (int)blockIdx.y * p.own);
+        if (own > 0) mbar_expect_tx(bar_recv, (gridDim.y - 1) * own * FEATS * 16);
+      }
+    }
+    if (lane < S) {
+      mbar_init(bar_full + 8 * lane, 1);
+      mbar_init(bar_act + 8 * lane, 1);
+      mbar_init(bar_mdone + 8 * lane, 1);
+    }
+    if (lane < NA) mbar_init(bar_afull + 8 * lane, 8);
+    if (lane < 2) { mbar_init(bar_accfull + 8 * lane, 1); mbar_init(bar_accfree + 8 * lane, 8); }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    const int sb0 = SPLIT ? blockIdx.y * p.bps : 0, sb1 = SPLIT ? min(p.nblk, sb0 + p.bps) : 0;
+    const int4 share = Work::share(SPLIT ? me * p.nblk + sb0 : first_block(p, me, npairs),
+                                   SPLIT ? me * p.nblk + sb1 : first_block(p, me + 1, npairs), p.nblk);
+    if (lane == 0) *s_share = share;
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    if (elect_one()) copy_blocks(Work(share, p.nblk), 0, S, true);
+    __syncwarp();
+  } else {
+    if (warp == 1) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(TMEM_COLS));
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    } else if (warp == 3 && lane <= 6) {
+      const CUtensorMap* m = lane == 0 ? &maps.act : lane <= 3 ? &maps.w[lane - 1] : &maps.s[lane - 4];
+      asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
     }
     __syncwarp();
-  } else if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(TMEM_COLS));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  if (warp == 0) {
-    if (elect_one()) stream_weights(min(S, total));
-    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   }
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");     // both CTAs' barriers and tensor memory are there
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  constexpr uint32_t A_COL0 = TMEM_COLS - A_COLS * NA;
+  const Work wk(*s_share, p.nblk);
+  const int total = wk.u1 - wk.u0;                    // blocks of this pair
+  const uint32_t A_COL0 = TMEM_COLS - A_COLS * NA;
   asm volatile("griddepcontrol.launch_dependents;");
 
-  if (warp == 0) {
+  if (warp == 0 || warp == 2) {
     if (elect_one()) {
-      wi = min(S, total);
-      wslot.i = wi % S;
-      wslot.turn = wi / S;
-      stream_weights(total);
-      s_copied[0] = wi;
-    }
-    __syncwarp();
-  } else if (warp == 2) {
-    if (elect_one()) {
-      asm volatile("griddepcontrol.wait;" ::: "memory");
-      int i = 0;
-      Slot sl;
-      for (int k = 0; k < wk.np && !failed; ++k) {
-        int tile, b0, b1, pi, span, fh, m0;
-        wk.piece(k, tile, b0, b1);
-        decode(tile, pi, span, fh, m0);
-        KCursor kc(p, b0);
-        for (int b = b0; b < b1; ++b, kc.next(p)) {
-          const int s = sl.i;
-          if (i >= S && !mbar_wait(bar_mdone + 8 * s, sl.turn ^ 1)) { failed = true; break; }
-          // the second k step of a range's last block may be the next range's or beyond K (zeros): not multiplied
-          mbar_expect_tx(bar_full + 8 * s, BLK * b_bytes);
-#pragma unroll
-          for (int h = 0; h < BLK; ++h)
-            tma_2d(ring + s * stage_bytes + RAW_PAD + h * b_bytes, &maps.act, (kc.k + h) * BK, m0 + half * (p.npad / 2),
-                   bar_full + 8 * s);
-          sl.next(S);
-          ++i;
-        }
+      if (warp == 0) {
+        if (total > S) copy_blocks(wk, S, total, true);
+      } else {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        copy_blocks(wk, 0, total, false);
       }
-      s_copied[1] = i;
+      failed = limit == 0;
+      s_copied[warp >> 1] = requested;
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -359,33 +387,37 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
       const uint32_t idesc = (1u << 4) | ((uint32_t)(p.npad >> 3) << 17) | ((uint32_t)(2 * FEATS >> 4) << 24);
       const uint16_t both = (uint16_t)(3u << lead);
       const uint64_t bdesc = kmajor_desc(ring + RAW_PAD);
+      const uint32_t b_step = b_bytes >> 4, stage_step = stage_bytes >> 4;
       if (elect_one()) {
         Slot sl, sa, sc;                                     // stage, A buffer, accumulator
+        uint32_t bofs = 0;                                   // of the stage, in the operand descriptor's unit
         int g = 0;
         for (int k = 0; k < wk.np; ++k) {
           int tile, b, b1;
           wk.piece(k, tile, b, b1);
-          KCursor kc(p, b);
           while (b < b1) {                                   // a range, or the pair's share of it
+            const int r = b / p.rblk, e = min(b1, (r + 1) * p.rblk);
+            // its last block may be one k step
+            const int odd = min(p.k64, (r + 1) * p.range) - (r * p.range + (e - 1 - r * p.rblk) * BLK) < BLK ? e - 1 : -1;
             if (g >= p.nacc) wait_limited(bar_accfree + 8 * sc.i, sc.turn ^ 1, limit);
             const uint32_t acc = tmem + sc.i * p.npad;
             uint32_t accum = 0;
-            for (bool last = false; b < b1 && !last; ++b) {
+            for (; b < e; ++b) {
               wait_limited(bar_afull + 8 * sa.i, sa.turn, limit);
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-              const uint64_t bd0 = bdesc + (uint64_t)((sl.i * stage_bytes) >> 4), bd1 = bd0 + (uint64_t)(b_bytes >> 4);
-              const uint32_t ta = tmem + A_COL0 + sa.i * A_COLS;
+              const uint64_t bd0 = bdesc + bofs, bd1 = bd0 + b_step;
+              const uint32_t ta = tmem + A_COL0 + sa.i * A_COLS, done = bar_mdone + 8 * sl.i;
+              sl.next(S);
+              sa.next(NA);
+              bofs = sl.i ? bofs + stage_step : 0;
 #pragma unroll
               for (int ks = 0; ks < BK / 16; ++ks) mma2_ts(acc, ta + ks * 8, bd0 + (uint64_t)(ks * 2), idesc, ks ? 1u : accum);
-              if (kc.end - kc.k >= BLK) {
+              if (b != odd) {
 #pragma unroll
                 for (int ks = 0; ks < BK / 16; ++ks) mma2_ts(acc, ta + 32 + ks * 8, bd1 + (uint64_t)(ks * 2), idesc, 1);
               }
-              commit2(bar_mdone + 8 * sl.i, both);
+              commit2(done, both);
               accum = 1;
-              sl.next(S);
-              sa.next(NA);
-              last = kc.next(p);
             }
             commit2(bar_accfull + 8 * sc.i, both);
             sc.next(p.nacc);
@@ -406,24 +438,22 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
     constexpr int WSTEP = SILU ? 512 : 1024, SSTEP = SILU ? 32 : 64, WGRP = SILU ? RAW_W / 2 : 512, SGRP = SILU ? RAW_S / 2 : 32;
     const unsigned char* lane_w = gbase + q * WGRP + lane * 16 + (quad & 1) * 8;
     const unsigned char* lane_s = gbase + RAW_W + q * SGRP + t * 8;
-    const uint32_t afull_lead = mapa(bar_afull, lead) + 8 * (dset % NA);
-    const uint32_t ta = tmem + ((uint32_t)(32 * quad) << 16) + A_COL0 + dset % NA * A_COLS;
-    Slot sl, sw;                                 // stage of this block, and of the one that used its A buffer before
-    sl.i = dset;
-    const int w0 = dset >= NA ? dset - NA : dset + DSETS - NA;
-    sw.i = w0 % S;
-    sw.turn = w0 / S;
+    const uint32_t afull_lead = mapa(bar_afull, lead), ta0 = tmem + ((uint32_t)(32 * quad) << 16) + A_COL0;
+    Slot sl, sa, sw;                             // stage and A buffer of this block, and stage of the one that used the buffer before
+    for (sl.i = dset, sa.i = dset; sa.i >= NA; sa.i -= NA) sa.turn ^= 1;
+    for (sw.i = dset; sw.i < NA;) sw.i += DSETS;
+    sw.i -= NA;                                  // of the first block that waits for one; below DSETS
     for (int i = dset; i < total; i += DSETS) {
       // The MMAs of the block that last used this A buffer are complete.  As the ring has at least NA stages, the block that
-      // last used this stage is through as well, and the stage's barrier, which tells only odd from even phases, is in one
-      // of the two phases that it can tell apart
+      // last used this stage is through as well, and the stage's barriers, which tell only odd from even phases, are in one
+      // of the two phases that they can tell apart
       if (i >= NA) {
         wait_limited(bar_mdone + 8 * sw.i, sw.turn, limit);
         sw.next4(S);
       }
       wait_limited(bar_full + 8 * sl.i, sl.turn, limit);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t so = sl.i * stage_bytes;
+      const uint32_t so = sl.i * stage_bytes, ta = ta0 + sa.i * A_COLS;
 #pragma unroll
       for (int h = 0; h < BLK; ++h) {
         uint32_t r[2][16];
@@ -433,10 +463,13 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
         st_16x256b_x4(ta + 32 * h + (16u << 16), r[1]);
       }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      // the first blocks are expanded while the launch in front still writes the activations
+      wait_limited(bar_act + 8 * sl.i, sl.turn, limit);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(afull_lead);
+      if (lane == 0) mbar_arrive_cluster(afull_lead + 8 * sa.i);
       sl.next4(S);
+      sa.next4(NA);
     }
     failed = limit == 0;
   }
@@ -453,6 +486,8 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
     const int nchunk = p.npad / 16;
     Slot sc;                                                 // accumulator
     int turn = 0;                                            // output buffer
+    const int ranges = CUT_K ? wk.np : wk.np * ((p.nblk + p.rblk - 1) / p.rblk);
+    int gr = 0;                                              // ranges that group 0 has read
     // outputs, scratch and flags may still be in use by the launch in front of this one
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (int k = group == 0 ? 0 : max(0, wk.np - 1); k < wk.np; ++k) {
@@ -480,15 +515,23 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
         const float* first = p.part + ((int64_t)(q0 * 2 + half) * p.npad) * FEATS + feat;
         float v[16];
         if (CUT_K && e == b1 && q0 < me) {
-          for (int q = q0; q < me; ++q) {
-            const int* flag = p.flags + q * 16 + half * 4 + quad;
-            int arrived;
-            uint32_t polls = FLAG_POLLS;
-            do {
-              asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(arrived) : "l"(flag) : "memory");
-              if (arrived < GROUPS) { __nanosleep(64); --polls; }
-            } while (arrived < GROUPS && polls && limit);
-            if (arrived < GROUPS) limit = 0;
+          // group 0 looks at the flags, makes them ready for the next launch and tells the others
+          if (group == 0) {
+            for (int q = q0; q < me; ++q) {
+              int* flag = p.flags + q * 16 + half * 4 + quad;
+              int arrived;
+              uint32_t polls = FLAG_POLLS;
+              do {
+                asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(arrived) : "l"(flag) : "memory");
+                if (arrived < GROUPS) { __nanosleep(64); --polls; }
+              } while (arrived < GROUPS && polls && limit);
+              if (arrived < GROUPS) limit = 0;
+              __syncwarp();
+              if (lane == 0) *flag = 0;
+            }
+            if (lane == 0) mbar_arrive(bar_flags);
+          } else {
+            wait_limited(bar_flags, 0, limit);
           }
           if (ch0 < nchunk) {                                // while the last MMAs run
 #pragma unroll
@@ -498,8 +541,10 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
         // (a barrier's parity tells a phase from its neighbours only: the other groups, which have not followed accfull,
         // wait for the end of all MMAs and for group 0, which has)
         if (group == 0) {
-          wait_limited(bar_accfull + 8 * sc.i, sc.turn, limit);
-          __syncwarp();
+          // one warp polls for the four (polls are issue slots: with all of them, and three more warps that had nothing else to do, a
+          // third of all instructions)
+          if (quad == 2) wait_limited(bar_accfull + 8 * sc.i, sc.turn, limit);
+          asm volatile("bar.sync %0, 128;" ::"n"(1 + GROUPS) : "memory");
           if (all && lane == 0) {
             *s_acc = sc.i;
             mbar_arrive(bar_last);
@@ -570,11 +615,8 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
             x.v = *xchg(feat);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              if (ch * 16 + 8 * hi + 2 * j >= rows) break;   // padding: its share of exponentials and divisions is issue slots
-                                                             // the dequantisers want (100 rows 25.0 us, with it 27.0)
               const float2 f = __half22float2(hi ? x.h[j] : mine.h[j]);
-              const __half2 sg = __floats2half2_rn(f.x / (1.0f + expf(-f.x)), f.y / (1.0f + expf(-f.y)));
-              const __half2 y = __hmul2(sg, hi ? mine.h[j] : x.h[j]);
+              const __half2 y = __hmul2(__floats2half2_rn(silu(f.x), silu(f.y)), hi ? mine.h[j] : x.h[j]);
               o[(8 * hi + 2 * j) * OUT_LD + f64] = __low2half(y);
               o[(8 * hi + 2 * j + 1) * OUT_LD + f64] = __high2half(y);
             }
@@ -592,16 +634,9 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        if (!all && lane == 0) mbar_arrive_cluster(mapa(bar_accfree, lead) + 8 * sc.i);
+        // an arrival that nobody waits for could find the even CTA gone
+        if (!all && ++gr + p.nacc <= ranges && lane == 0) mbar_arrive_cluster(mapa(bar_accfree, lead) + 8 * sc.i);
         sc.next(p.nacc);
-      }
-      if (CUT_K && q0 < me) {
-        // read: the last group makes the flags ready for the next launch
-        __syncwarp();
-        for (int q = q0 + lane; q < me; q += 32) {
-          int* flag = p.flags + q * 16 + half * 4 + quad;
-          if (atomicAdd(flag + 8, 1) == GROUPS - 1) { flag[0] = 0; flag[8] = 0; }
-        }
       }
       if (CUT_K && !whole) {
         // published: GROUPS arrivals per flag, whoever drained the accumulator
@@ -612,61 +647,75 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
     }
     failed = failed || limit == 0;
   }
-  if (!mbar_wait(bar_done, 0) || failed) *s_failed = 1;
+  if (warp >= DQ_WARP0 && (!SPLIT || warp < EPI_WARP0)) wait_limited(bar_done, 0, limit);
+  if (failed || limit == 0) *s_failed = 1;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   __syncthreads();
   failed = *s_failed != 0;
   if (failed && tid == 0) {
     // the copies still on their way, those of the last S blocks at most: none may land in shared memory that has been given back
     q40_set_error(p.err);
-    const int n = max(s_copied[0], s_copied[1]);
-    for (int i = max(0, n - S); i < n; ++i) mbar_wait(bar_full + 8 * (i % S), (uint32_t)((i / S) & 1));
+    for (int h = 0; h < 2; ++h)
+      for (int n = s_copied[h], i = max(0, n - S); i < n; ++i) mbar_wait((h ? bar_act : bar_full) + 8 * (i % S), (uint32_t)((i / S) & 1));
   }
 
-  if (SPLIT && !failed && warp >= DQ_WARP0) {
-    // accumulators -> fp32 tile [npad][128] over the ring, which is idle by now
-    float* tile_f = reinterpret_cast<float*>(gbase);
-    const int quad = warp & 3, set = (warp - DQ_WARP0) >> 2, feat = 32 * quad + lane;
-    for (int ch = set; ch < p.npad / 16; ch += (THREADS / 32 - DQ_WARP0) / 4) {
-      uint32_t r[16];
-      ld16(tmem + ((uint32_t)(32 * quad) << 16) + ch * 16, r);
-      wait_ld16(r);
-#pragma unroll
-      for (int j = 0; j < 16; ++j) tile_f[(ch * 16 + j) * FEATS + feat] = __uint_as_float(r[j]);
+  if (SPLIT && warp >= DQ_WARP0) {
+    // The ranks of a cluster have the sums of a k range each.  Of the groups of four rows, rank r finishes p.own: it gets the others' from
+    // them, as they come to their end, and adds all in k order
+    const int quad = warp & 3, group = (warp - DQ_WARP0) >> 2, feat = 32 * quad + lane;
+    const int nranks = (int)gridDim.y, rank = (int)blockIdx.y;
+    int pi, span, fh, m0;
+    decode(me, pi, span, fh, m0);
+    const int rows = min(p.npad, p.M - m0), ngroups = (rows + 3) / 4;
+    const int g0 = min(ngroups, rank * p.own), g1 = min(ngroups, g0 + p.own);
+    const uint32_t acc = tmem + ((uint32_t)(32 * quad) << 16);
+    const uint32_t recv = ring + (uint32_t)p.run_off;        // [rank, without this one's][group][feature][row]
+    if (!failed) {
+      for (int g = group; g < ngroups; g += GROUPS) {
+        const int to = g / p.own;
+        if (to == rank) continue;
+        uint32_t r[4];
+        ld4(acc + 4 * g, r);
+        wait_ld4(r);
+        const int slot = rank < to ? rank : rank - 1;
+        push4(mapa(recv, 2 * to + half) + (uint32_t)(((slot * p.own + g - to * p.own) * FEATS + feat) * 16), r, mapa(bar_recv, 2 * to + half));
+      }
+    }
+    if (g0 < g1 && !failed) {
+      wait_limited(bar_recv, 0, limit);
+      __half* o = reinterpret_cast<__half*>(gbase) + group * 4 * OUT_LD;     // over the ring, which is idle
+      const float4* in = reinterpret_cast<const float4*>(gbase + p.run_off) + feat;
+      __half* c = p.c[pi] + (int64_t)m0 * p.ldc[pi] + span * SPAN + fh * FEATS;
+      for (int g = g0 + group; g < g1; g += GROUPS) {
+        uint32_t r[4];
+        ld4(acc + 4 * g, r);
+        wait_ld4(r);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < nranks; ++k) {
+          float4 t = make_float4(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]), __uint_as_float(r[3]));
+          if (k != rank) t = in[((k < rank ? k : k - 1) * p.own + g - g0) * FEATS];
+          v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+        }
+        o[feat] = __float2half_rn(v.x);
+        o[OUT_LD + feat] = __float2half_rn(v.y);
+        o[2 * OUT_LD + feat] = __float2half_rn(v.z);
+        o[3 * OUT_LD + feat] = __float2half_rn(v.w);
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+        store_rows<FEATS>(o, c + (int64_t)(4 * g) * p.ldc[pi], p.ldc[pi], min(4, rows - 4 * g), feat, p.vec);
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+      }
+      if (limit == 0) q40_set_error(p.err);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  cluster.sync();
+  // No ordinary store is meant for another CTA, and what a CTA still sends another is waited for there: execution alone meets here (with the
+  // default release, for the stores of the output: half a microsecond more)
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TMEM_COLS));
   }
-  if (!SPLIT) return;
-  // split-K: the r-th CTA of this half finishes the r-th slice of the (row, feature) pairs, adding the tiles in k order
-  float* tile_f = reinterpret_cast<float*>(gbase);
-  int pi, span, fh, m0;
-  decode(me, pi, span, fh, m0);
-  const int nranks = (int)gridDim.y, rank = (int)blockIdx.y;
-  const int rows = min(p.npad, p.M - m0), n_el = rows * FEATS;
-  const int per = ((n_el / 4 + nranks - 1) / nranks) * 4;
-  const int e0 = rank * per, e1 = min(n_el, e0 + per);
-  __half* c = p.c[pi] + (int64_t)m0 * p.ldc[pi] + span * SPAN + fh * FEATS;
-  if (!failed) {
-    for (int e = e0 + tid * 4; e < e1; e += THREADS * 4) {
-      float4 tt[4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-        tt[r] = (r < nranks) ? *reinterpret_cast<const float4*>(cluster.map_shared_rank(tile_f + e, 2 * r + half))
-                             : make_float4(0.f, 0.f, 0.f, 0.f);
-      float4 v = tt[0];
-#pragma unroll
-      for (int r = 1; r < 4; ++r) { v.x += tt[r].x; v.y += tt[r].y; v.z += tt[r].z; v.w += tt[r].w; }
-      __half2* dst = reinterpret_cast<__half2*>(c + (int64_t)(e / FEATS) * p.ldc[pi] + e % FEATS);
-      dst[0] = __floats2half2_rn(v.x, v.y);
-      dst[1] = __floats2half2_rn(v.z, v.w);
-    }
-  }
-  cluster.sync();       // every rank has read the tiles: shared memory may go away
 }
 
 }  // namespace pair
@@ -675,17 +724,15 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
 
 using PairKernel = void (*)(const q40::ttc::pair::Params, const q40::ttc::pair::Maps);
 
-// [0] SPLIT; else 1 + NA == 4, + 2 SiLU, + 4 cut
+// [0] SPLIT; else 1 + 1 SiLU + 2 cut
 static PairKernel pair_kernel(int which) {
   using namespace q40::ttc::pair;
   switch (which) {
-    case 0: return gemm_pair_kernel<true, 4, false, false>;
-    case 1: return gemm_pair_kernel<false, 2, false, false>;
-    case 2: return gemm_pair_kernel<false, 4, false, false>;
-    case 3: return gemm_pair_kernel<false, 2, false, true>;
-    case 4: return gemm_pair_kernel<false, 4, false, true>;
-    case 6: return gemm_pair_kernel<false, 4, true, false>;
-    default: return gemm_pair_kernel<false, 4, true, true>;
+    case 0: return gemm_pair_kernel<true, false, false>;
+    case 1: return gemm_pair_kernel<false, false, false>;
+    case 2: return gemm_pair_kernel<false, false, true>;
+    case 3: return gemm_pair_kernel<false, true, false>;
+    default: return gemm_pair_kernel<false, true, true>;
   }
 }
 
@@ -722,30 +769,32 @@ namespace q40 {
 namespace ttc {
 namespace pair {
 
-// Shared memory of a launch, or 0 if it does not fit: [ring][run][rows on their way out][barriers]
-static size_t layout(Params& p, int na, bool split) {
+// Rows of a tile
+static void tile_rows(Params& p, int npad) {
+  p.npad = npad;
+  p.chunks = (p.M + npad - 1) / npad;
+}
+
+// Shared memory of a launch, or 0 if it does not fit: [ring][run][rows on their way out][barriers]; ring stages, accumulators and A
+// buffers.  `single`: no pair has more than one tile, of one range, and a second accumulator would be for nothing.  Else two where
+// they fit tensor memory beside at least two A buffers
+static size_t layout(Params& p, int split, bool single) {
   const size_t tile = (size_t)p.npad * FEATS * 4, stage = RAW_PAD + (size_t)p.npad * 64 * BLK;
-  const size_t run = p.range < p.k64 ? tile : 0, out = split ? 0 : 2 * 16 * OUT_LD * 2;
+  p.own = ((p.M + 3) / 4 + split - 1) / split;
+  const size_t run = split > 1 ? (size_t)(split - 1) * p.own * FEATS * 16 : p.range < p.k64 ? tile : 0;
+  const size_t out = split > 1 ? 0 : 2 * 16 * OUT_LD * 2;
   const size_t fixed = 1024 /* alignment */ + BAR_BYTES + 64 /* tail */ + run + out;
-  if (fixed + NA_MAX * stage > (size_t)SMEM_MAX) return 0;
-  p.stages = (int)((SMEM_MAX - fixed) / stage);
-  if (p.stages > S_MAX) p.stages = S_MAX;
-  size_t off = p.stages * stage;
-  if (split && off < tile) off = tile;                       // the fp32 tile of a split takes the ring's place
+  if (fixed + DSETS * stage > (size_t)SMEM_MAX) return 0;
+  p.stages = std::min(S_MAX, (int)((SMEM_MAX - fixed) / stage));
+  p.nacc = !single && 2 * p.npad + 2 * A_COLS <= TMEM_COLS ? 2 : 1;
+  p.na = std::min({NA_MAX, p.stages, (TMEM_COLS - p.nacc * p.npad) / A_COLS});
+  const size_t off = p.stages * stage;
   p.run_off = (int)off;
   p.out_off = (int)(off + run);
   p.bar_off = (int)(off + run + out);
   // more than half of an SM's: two pairs of different launches that each got one SM's tensor memory would wait for the other's
   const size_t smem = off + fixed;
   return smem < 116 * 1024 ? 116 * 1024 : smem;
-}
-
-// Rows of a tile -> accumulators and A buffers: two accumulators where they fit tensor memory beside at least two A buffers
-static int tile_rows(Params& p, int npad) {
-  p.npad = npad;
-  p.chunks = (p.M + npad - 1) / npad;
-  p.nacc = 2 * npad + 2 * A_COLS <= TMEM_COLS ? 2 : 1;
-  return TMEM_COLS - p.nacc * npad >= NA_MAX * A_COLS ? NA_MAX : 2;
 }
 
 // k steps -> blocks; `range` k steps are summed in tensor memory
@@ -790,16 +839,16 @@ int q40_pair_gemm(int nmat, const void* a, int64_t lda, const void* const* bw_ti
   p.nprob = nmat; p.M = M; p.K = K; p.err = err; p.silu = silu;
   p.k64 = K / BK;
   pair::k_blocks(p, ranges > 1 ? (p.k64 + ranges - 1) / ranges : p.k64);
-  if ((int64_t)spans * ((M + 63) / 64) * p.nblk > 0x7fffffffLL) return Q40_E_UNSUPPORTED;
+  if ((int64_t)spans * ((M + 63) / 64) * std::max(p.nblk, pair::MAX_PAIRS) > 0x7fffffffLL) return Q40_E_UNSUPPORTED;
   // the kernels' attributes come first: the runtime is asked how many fit with the shared memory that they allow
-  static std::atomic<uint64_t> ready[9];
+  static std::atomic<uint64_t> ready[5];
   auto kernel = [&](int which) -> PairKernel {
     PairKernel k = pair_kernel(which);
     if (q40_allow_smem(ready[which], (const void*)k, SMEM_MAX) == cudaSuccess) return k;
     (void)cudaGetLastError();
     return nullptr;
   };
-  PairKernel plain = kernel(2), in_clusters = kernel(0);
+  PairKernel plain = kernel(1), in_clusters = kernel(0);
   if (!plain || !in_clusters) return Q40_E_UNSUPPORTED;
   const int fit = pair_max_clusters(plain, 1) < pair::MAX_PAIRS ? pair_max_clusters(plain, 1) : pair::MAX_PAIRS;
   if (fit < 1) return Q40_E_UNSUPPORTED;
@@ -822,8 +871,8 @@ int q40_pair_gemm(int nmat, const void* a, int64_t lda, const void* const* bw_ti
     for (int n = 64; n <= pair::MAX_ROWS; n += 16) {
       const int chunks = (M + n - 1) / n;
       if (((M + chunks - 1) / chunks + 15) / 16 * 16 != n) continue;           // the same chunks with fewer rows of padding
-      const int na = pair::tile_rows(p, n);
-      if (pair::layout(p, na, false) == 0) continue;
+      pair::tile_rows(p, n);
+      if (pair::layout(p, 1, false) == 0) continue;
       const double waves = (double)(((int64_t)spans * chunks + fit - 1) / fit);
       const double block = n <= 128 ? 165 + 1.8 * n : 395 + 2.8 * (n - 128);
       const int nr = (p.k64 + p.range - 1) / p.range;
@@ -834,7 +883,7 @@ int q40_pair_gemm(int nmat, const void* a, int64_t lda, const void* const* bw_ti
   }
   if (npad == 0) return Q40_E_UNSUPPORTED;
 
-  const int na = pair::tile_rows(p, npad);
+  pair::tile_rows(p, npad);
   p.ntiles = spans * p.chunks;                   // SiLU: as many, of half a span of both matrices
   p.cut = cut;
   if (cut) {
@@ -850,9 +899,9 @@ int q40_pair_gemm(int nmat, const void* a, int64_t lda, const void* const* bw_ti
     p.share = units / npairs;
     p.rest = units % npairs;
   }
-  const size_t smem = pair::layout(p, na, split > 1);
+  const size_t smem = pair::layout(p, split, split > 1 || (!cut && p.ntiles <= npairs && p.range == p.k64));
   if (smem == 0 || smem > (size_t)SMEM_MAX) return Q40_E_UNSUPPORTED;
-  PairKernel kern = kernel(split > 1 ? 0 : 1 + (na == pair::NA_MAX) + 2 * silu + 4 * cut);      // shared tiles have at most 128 rows: four A buffers
+  PairKernel kern = kernel(split > 1 ? 0 : 1 + silu + 2 * cut);
   if (!kern) return Q40_E_UNSUPPORTED;
   pair::Maps maps;
   const cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)M};

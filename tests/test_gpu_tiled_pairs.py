@@ -103,6 +103,39 @@ def test_silu_product_is_that_of_the_separate_launches(K, M, Kd, n):
     assert (g == want).float().mean() > 0.97
 
 
+def test_silu_of_every_fp16_value(K):
+    """The product's SiLU rounds like the launch that divides: x and y are the activation itself, which takes every value."""
+    Kd, n, M = 64, 256, 65536
+    q, s = np.zeros((Kd * n // 128, 64), np.int8), np.zeros((Kd * n // 64,), np.float16)
+    q[:n // 128], s[:n // 64] = 0x11, 1                          # the first row of the matrix: ones
+    tiled = [K.relayout_tiled(torch.from_numpy(q).cuda(), torch.from_numpy(s).cuda(), (Kd, n))] * 2
+    x = torch.arange(M, dtype=torch.int32, device="cuda").to(torch.int16).view(torch.float16)
+    a = torch.zeros((M, Kd), dtype=torch.float16, device="cuda")
+    a[:, 0] = x
+    g = torch.empty((M, n), dtype=torch.float16, device="cuda")
+    launch(a, tiled, [g, g], (n, n), 1, scratch(K, M))
+    want = K.silu_mul(x, x)
+    assert torch.equal(g.view(torch.int16)[~want.isnan()], want.view(torch.int16)[~want.isnan()].view(-1, 1).expand(-1, n)) and g[want.isnan()].isnan().all()
+
+
+# the k range of a tile over two, three and four pairs of a cluster, each finishing some groups of four rows: one group and none for
+# some ranks, the last one ragged, as many as divide and not
+@pytest.mark.parametrize("M", [1, 4, 9, 13, 17, 36, 100, 128])
+@pytest.mark.parametrize("Kd,n", [(1024, 1024), (4096, 4096), (11008, 256), (8256, 512)])
+def test_k_split_over_a_cluster(K, M, Kd, n):
+    rng = np.random.default_rng(M + Kd)
+    packed, tiled = mats(K, rng, Kd, (n,))
+    a = rng.standard_normal((M, Kd)).astype(np.float16)
+    a_d, out = torch.from_numpy(a).cuda(), torch.full((M + 1, n + 8), 7.0, dtype=torch.float16, device="cuda")
+    launch(a_d, tiled, [out[:M, :n]], (n,), 0, scratch(K, M))
+    close(out[:M, :n], O.matmul_q40(a, *packed[0], (Kd, n)))
+    assert (out[M] == 7).all() and (out[:, n:] == 7).all()
+    again = torch.empty((M, n), dtype=torch.float16, device="cuda")
+    for _ in range(3):
+        launch(a_d, tiled, [again], (n,), 0, scratch(K, M), 1)
+        assert torch.equal(again, out[:M, :n])
+
+
 # as many tiles as take more than a wave of pairs, or less than one, with k ranges long enough to be worth sharing, whether 60 or
 # 74 pairs run: a tile on two pairs or on three (40 tiles), blocks that do and do not divide among them, one and several
 # 16-row chunks
