@@ -1,5 +1,7 @@
 // Declarations shared by the attention kernels.
 #pragma once
+#include <math_constants.h>
+
 #include "q40_common.cuh"
 
 namespace q40 {
@@ -13,6 +15,13 @@ __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// acc + a.x b.x + a.y b.y: the products of fp16 values are exact, each sum rounds once
+__device__ __forceinline__ float dot2(__half2 a, __half2 b, float acc) {
+  asm("{\n\t.reg .b16 a0, a1, b0, b1;\n\tmov.b32 {a0, a1}, %1;\n\tmov.b32 {b0, b1}, %2;\n\t"
+      "fma.rn.f32.f16 %0, a0, b0, %0;\n\tfma.rn.f32.f16 %0, a1, b1, %0;\n\t}" : "+f"(acc) : "r"(h2_as_u32(a)), "r"(h2_as_u32(b)));
+  return acc;
 }
 
 struct BranchArgs {
@@ -34,7 +43,7 @@ struct BranchArgs {
   int nsp;
   int beside_prefix;      // the prefix pass is the launch in front of this one: its results are waited for at the merge
   float scale_log2;       // 1/sqrt(D) * log2(e)
-  // Q4_0 suffix cache (mode 3): packed rows [B, max_t, Hkv, 64] + scales [B, max_t, Hkv, 2];
+  // Q4_0 suffix cache: packed rows [B, max_t, Hkv, 64] + scales [B, max_t, Hkv, 2];
   // the branch's suffix length is pos[b] - prefix_len[0] (device values)
   const int8_t* kq;
   const __half* ksc;
@@ -49,8 +58,8 @@ struct BranchArgs {
   int64_t cur_stride;
 };
 
-// mode 4: mode 3 with q and cur_k from before their rotary embedding (tables [n_pos, 64], 16-byte aligned), which is done here, and the
-// token's key and value appended to the cache.  A struct of its own: a launch takes longer with more arguments, also where they are not
+// The Q4_0 cache; with tables ([n_pos, 64], 16-byte aligned) q and cur_k are from before their rotary embedding, which is done here, and
+// the token's key and value are appended to the cache.  A struct of its own: a launch takes longer with more arguments, also where they are not
 // used (a call of q40_attn_decode 3.33 us with 216 bytes, 3.68 with 240).
 struct BranchRotArgs : BranchArgs {
   const __half* cos_tbl;
@@ -58,8 +67,77 @@ struct BranchRotArgs : BranchArgs {
   int n_pos;
 };
 
-// defined in attn_branch.cu; mode 0 contiguous, 1 paged/int16 ids, 2 paged/int32 ids, 3 Q4_0 cache
+// The end of a row (branch, head) of RT threads: its own keys' partial results, NG of them in shared memory, and those of a prefix pass
+// become the output.  Thread tr owns output dims tr, tr + RT, ... (RT above the head's 128: the first four warps)
+template <int NG, int RT>
+struct RowMerge {
+  static constexpr int DP = RT >= ATTN_D ? 1 : ATTN_D / RT, PB = 16 / DP;
+  float pm_l, pl_l, po[PB][DP];
+  // The prefix partials, once they are there and before the row's warps meet: lane sp holds the maximum and the sum of split sp
+  // (further splits are read at the end), and the first splits' outputs are all requested together
+  __device__ __forceinline__ void load(const BranchArgs& a, int64_t bh, int tr, int lane) {
+    pm_l = lane < a.nsp ? a.pm[(int64_t)lane * a.rows + bh] : -CUDART_INF_F;
+    pl_l = lane < a.nsp ? a.pl[(int64_t)lane * a.rows + bh] : 0.f;
+    if (a.nsp > 0) {
+#pragma unroll
+      for (int i = 0; i < PB; ++i)
+#pragma unroll
+        for (int j = 0; j < DP; ++j)
+          po[i][j] = i < a.nsp && (RT <= ATTN_D || tr < ATTN_D) ? a.po[((int64_t)i * a.rows + bh) * ATTN_D + tr + j * RT] : 0.f;
+    }
+  }
+  __device__ __forceinline__ void finish(const BranchArgs& a, int64_t bh, int tr, int lane, const float* sm_m, const float* sm_l,
+                                         const float (*sm_o)[ATTN_D]) {
+    if (RT > ATTN_D && tr >= ATTN_D) return;
+    float M = -CUDART_INF_F;
+#pragma unroll
+    for (int g = 0; g < NG; ++g) M = fmaxf(M, sm_m[g]);
+    M = fmaxf(M, warp_max(pm_l));
+    for (int sp = 32; sp < a.nsp; ++sp) M = fmaxf(M, a.pm[(int64_t)sp * a.rows + bh]);
+    float Lsum = 0.f, acc[DP];
+#pragma unroll
+    for (int j = 0; j < DP; ++j) acc[j] = 0.f;
+    if (M > -CUDART_INF_F) {
+#pragma unroll
+      for (int g = 0; g < NG; ++g) {
+        const float w = ex2(sm_m[g] - M);         // exp2(-inf) = 0 for empty groups
+        Lsum = fmaf(sm_l[g], w, Lsum);
+#pragma unroll
+        for (int j = 0; j < DP; ++j) acc[j] = fmaf(sm_o[g][tr + j * RT], w, acc[j]);
+      }
+      if (a.nsp > 0) {
+        const float pw_l = ex2(pm_l - M);
+#pragma unroll
+        for (int i = 0; i < PB; ++i) {            // splits from nsp on: weight and sum are 0
+          const float w = __shfl_sync(0xffffffffu, pw_l, i);
+          Lsum = fmaf(__shfl_sync(0xffffffffu, pl_l, i), w, Lsum);
+#pragma unroll
+          for (int j = 0; j < DP; ++j) acc[j] = fmaf(po[i][j], w, acc[j]);
+        }
+        for (int sp = PB; sp < min(a.nsp, 32); ++sp) {
+          const float w = __shfl_sync(0xffffffffu, pw_l, sp);
+          Lsum = fmaf(__shfl_sync(0xffffffffu, pl_l, sp), w, Lsum);
+#pragma unroll
+          for (int j = 0; j < DP; ++j) acc[j] = fmaf(a.po[((int64_t)sp * a.rows + bh) * ATTN_D + tr + j * RT], w, acc[j]);
+        }
+      }
+      for (int sp = 32; sp < a.nsp; ++sp) {
+        const int64_t r = (int64_t)sp * a.rows + bh;
+        const float w = ex2(a.pm[r] - M);
+        Lsum = fmaf(a.pl[r], w, Lsum);
+#pragma unroll
+        for (int j = 0; j < DP; ++j) acc[j] = fmaf(a.po[r * ATTN_D + tr + j * RT], w, acc[j]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < DP; ++j) a.o[bh * ATTN_D + tr + j * RT] = __float2half_rn((Lsum > 0.f) ? acc[j] / Lsum : 0.f);
+  }
+};
+
+// defined in attn_branch_q4.cu; `rotate`: see BranchRotArgs
+int launch_branch_q4(const BranchRotArgs& a, bool rotate, cudaStream_t st);
+// defined in attn_branch.cu; mode 0 contiguous, 1 paged/int16 ids, 2 paged/int32 ids
 int launch_branch(BranchArgs a, int mode, int B, cudaStream_t st);
-int launch_branch(BranchRotArgs a, int B, cudaStream_t st);   // mode 4
+int launch_branch_q4(BranchRotArgs a, int B, cudaStream_t st);         // the Q4_0 cache, with rotation where there are tables
 
 }  // namespace q40

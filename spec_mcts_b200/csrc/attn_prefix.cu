@@ -307,7 +307,7 @@ static int tree_decode(const void* q, int64_t q_stride, const void* prefix_k, co
   br.vq = (const int8_t*)cache_vq; br.vsc = (const __half*)cache_vs;
   br.pos = pos_dev; br.prefix_len = prefix_len_dev; br.max_t = max_t;
   br.cur_k = (const __half*)cur_k; br.cur_v = (const __half*)cur_v; br.cur_stride = cur_stride;
-  return cos_tbl ? launch_branch(br, B, st) : launch_branch((const BranchArgs&)br, 3, B, st);
+  return launch_branch_q4(br, B, st);
 }
 
 extern "C" int q40_attn_tree_decode(const void* q, int64_t q_stride, const void* prefix_k, const void* prefix_v,

@@ -187,16 +187,21 @@ __device__ __forceinline__ void rotate_dims(uint4& lo, uint4& hi, const uint4& c
   }
 }
 
-// dims 8i.. (high nibbles) and 64 + 8i.. (low nibbles) of a head -> 8 packed bytes per lane and the row's two scales
+// dims 8i.. (high nibbles) and 64 + 8i.. (low nibbles) of a head -> 8 packed bytes per lane and the row's two scales.  The eight lanes of a
+// head are STRIDE apart; of others that hold the same, `writes` is false
+template <int STRIDE = 1>
 __device__ __forceinline__ void append_row(const uint4& lo, const uint4& hi, int8_t* codes, __half* scales, int i,
-                                           unsigned gmask) {
+                                           unsigned gmask, bool writes = true) {
   const uint32_t ew[4] = {lo.x, lo.y, lo.z, lo.w}, ow[4] = {hi.x, hi.y, hi.z, hi.w};
   __half2 m = quant_max(ew, ow);
 #pragma unroll
-  for (int off = 4; off > 0; off >>= 1) m = __hmax2(m, u32_as_h2(__shfl_xor_sync(gmask, h2_as_u32(m), off)));
+  for (int off = 4; off > 0; off >>= 1) m = __hmax2(m, u32_as_h2(__shfl_xor_sync(gmask, h2_as_u32(m), off * STRIDE)));
   __half2 sc;
-  *reinterpret_cast<uint2*>(codes + 8 * i) = quant_codes(ew, ow, m, sc);
-  if (i == 0) *reinterpret_cast<__half2*>(scales) = sc;
+  const uint2 out = quant_codes(ew, ow, m, sc);
+  if (writes) {
+    *reinterpret_cast<uint2*>(codes + 8 * i) = out;
+    if (i == 0) *reinterpret_cast<__half2*>(scales) = sc;
+  }
 }
 
 __device__ __forceinline__ float warp_max(float v) {

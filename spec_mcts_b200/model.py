@@ -849,26 +849,12 @@ class Transformer(nn.Module):
         check(rc, "q40_decode_chain")
         return True
 
-    def _rotates_in_attention(self, B):
-        return B * self._H <= 1408
-
     def _attn_step(self, att, q, k, v, ld, ao, B, ws, st):
-        """Rotary embedding, cache append and attention of a step's new tokens (rows of `ld` values).  Up to 1408 (branch, head) pairs as two
-        launches, prompt and branches; with more of them each would rotate in too many places, and a launch of its own does as well or
-        better.  Us of a step of 32 layers with 32 heads, in three launches and two a layer, prompt 512 and 64 own keys / 100 and 200:
-        6 branches 2067 and 2026 / 2186 and 2107, 20 2266 and 2215 / 2486 and 2445, 44 2482 and 2435 / 2920 and 2898, 48 2512 and
-        2503 / 2964 and 3003, 64 2703 and 2692 / 3212 and 3198, 100 3218 and 3239 / 3982 and 3990."""
+        """Rotary embedding, cache append and attention of a step's new tokens (rows of `ld` values), as two launches, prompt and branches.
+        With a launch of its own for rotation and append (q40_rope_kv_append) a step is slower at all widths: us for 8 layers with 32 heads,
+        prompt 512, 64 and 200 own keys, 6 branches 528 and 545 / 548 and 563, 44 branches 612 and 622 / 685 and 693, 100 branches
+        761 and 765 / 892 and 909."""
         p, pk, pv = self.params, att.cache_prompt_k, att.cache_prompt_v
-        if not self._rotates_in_attention(B):
-            caches = [t.data_ptr() for t in (att.cache_k, att.cache_k_s, att.cache_v, att.cache_v_s)]
-            pos, plen = self._pos_dev.data_ptr(), self._prefix_len_dev.data_ptr()
-            check(lib.q40_rope_kv_append(q.data_ptr(), ld, k.data_ptr(), ld, v.data_ptr(), ld, pos, plen, self._cos.data_ptr(),
-                                         self._sin.data_ptr(), self._n_pos, *caches, B, self._H, self._Hkv, self._D, p.max_seq_len, st),
-                  "q40_rope_kv_append")
-            check(lib.q40_attn_tree_decode(q.data_ptr(), ld, pk.data_ptr(), pv.data_ptr(), p.max_prompt_seq_len, plen, pk.stride(0),
-                                           pk.stride(1), *caches, p.max_seq_len, pos, k.data_ptr(), v.data_ptr(), ld, ao.data_ptr(), B,
-                                           self._H, self._Hkv, self._D, ws.data_ptr(), ws.numel(), st), "q40_attn_tree_decode")
-            return
         check(lib.q40_attn_tree_step(q.data_ptr(), ld, k.data_ptr(), v.data_ptr(), ld, pk.data_ptr(), pv.data_ptr(), p.max_prompt_seq_len,
                                      self._prefix_len_dev.data_ptr(), pk.stride(0), pk.stride(1), att.cache_k.data_ptr(),
                                      att.cache_k_s.data_ptr(), att.cache_v.data_ptr(), att.cache_v_s.data_ptr(), p.max_seq_len,
@@ -1144,8 +1130,6 @@ class Transformer(nn.Module):
             self.launches_per_step = 2
             return
         per_layer = (5 if self._fused_attn_for(B) else 6) if fused else (8 if self._silu_pair(B, self.layers[0].feed_forward) else 9)
-        if not (fused and per_layer == 5 or self._rotates_in_attention(B)):
-            per_layer += 1
         self.launches_per_step = self.params.n_layers * per_layer + (2 if self._narrow(B) else 1) + (not fused and self._fused_tail(B))
 
 
