@@ -438,6 +438,19 @@ int q40_silu_mul(const void* a, const void* b, void* y, int64_t n, void* stream)
 int q40_attn_causal(const void* q, int64_t ldq, const void* k, int64_t ldk, const void* v, int64_t ldv, void* o,
                     int64_t ldo, int S, int H, int Hkv, int D, void* stream);
 
+/* The layers of a prompt pass, enqueued by one call: per layer q40_rmsnorm (adding the previous layer's output), q40_gemm_tiled_tc_multi
+ * for wq, wk and wv (keys and values into the prompt cache), q40_rope_qk, q40_attn_causal, wo, q40_rmsnorm, q40_gemm_tiled_tc_ws with the SiLU
+ * product for w1 and w3, and w2, under the rules of those calls (head size 128, row-major buffers without padding).  `layers`, in host
+ * memory, has Q40_PROMPT_LAYER_POINTERS addresses per layer: the tiled copies of wq, wk, wv, wo, w1, w3, w2, the weights of the two
+ * norms, the first rows of the layer's prompt keys and values.  h [S, dim] holds the embeddings and is updated; the last layer's
+ * output is left in f, not added.  xn, o, f [S, dim]; q, ao [S, H*128]; g [S, hidden] are scratch.  A status other than 0 is that of the call
+ * that failed; the launches before it have been enqueued.  Replaces the loop over TransformerBlock of Transformer.forward
+ * (hf_model_q40_kv_shared.py:505-507) for start_pos == 0. */
+#define Q40_PROMPT_LAYER_POINTERS 11
+int q40_prompt_layers(const void* const* layers, int n_layers, int S, int dim, int hidden, int H, int Hkv, float eps, void* h,
+                      void* xn, void* q, void* ao, void* o, void* g, void* f, const int32_t* pos, const void* cos_tbl,
+                      const void* sin_tbl, void* workspace, size_t workspace_bytes, int* err, int use_pdl, void* stream);
+
 /* ---- tensor-parallel all-reduce fused with residual add and RMSNorm (no counterpart in the reference beyond
  * the torch.distributed all_reduce after wo and w2, hf_model_q40_kv_shared.py:258-261) ----
  * One process per GPU.  Every rank allocates one buffer (q40_tp_alloc: cudaMalloc + zero fill + CUDA IPC handle of

@@ -127,6 +127,8 @@ SIGNATURES = {
                          c_void_p]),
     "q40_rope_qk": (c_int, [c_void_p, c_int, c_int64, c_void_p, c_int, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_int,
                             c_void_p]),
+    "q40_prompt_layers": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                  c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p, c_int, c_void_p]),
     "q40_silu_mul": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_void_p]),
 }
 

@@ -356,6 +356,14 @@ class Transformer(nn.Module):
         scratch = K._tiled_tc_workspace(h.device, S) if any(mm[2][1] is not None for *_, mm in plan) else None
         silu_ws = self._tc_ws_args(scratch)
         pending = None     # output of the previous sub-block, added to h by the next norm kernel
+        table = self._prompt_table(plan) if self.tp_world == 1 else None
+        if table is not None:
+            check(lib.q40_prompt_layers(table, len(plan), S, p.dim, hid, H, Hkv, float(p.norm_eps), h.data_ptr(), xn.data_ptr(), q.data_ptr(),
+                                        ao.data_ptr(), o.data_ptr(), g.data_ptr(), f.data_ptr(), pos.data_ptr(), self._cos.data_ptr(),
+                                        self._sin.data_ptr(), *silu_ws, err.data_ptr(), 1 if self.use_pdl else 0, st), "q40_prompt_layers")
+            for att, *_ in plan:
+                att.cache_prompt_len = S
+            plan, pending = (), f
         for att, attn_norm, ffn_norm, (qkv, wo, w13, w2) in plan:
             # keys and values go straight to their place in the prompt cache
             ck, cv = att.cache_prompt_k[:S], att.cache_prompt_v[:S]
@@ -395,6 +403,21 @@ class Transformer(nn.Module):
         if self.prefill_tiled_tc:
             self._check_prompt()
         return logits
+
+    def _prompt_table(self, plan):
+        """The addresses that q40_prompt_layers reads, or None where a layer is not multiplied through tiled copies alone or its buffers are
+        not laid out for it."""
+        rows = []
+        rest = (self._Hkv * self._D, self._D, 1)
+        for att, attn_norm, ffn_norm, sites in plan:
+            ck, cv = att.cache_prompt_k, att.cache_prompt_v
+            if (any(tiled is None for _, tiled in sites) or ck.stride() != rest or cv.stride() != rest or
+                    not (attn_norm.is_contiguous() and ffn_norm.is_contiguous())):
+                return None
+            for _, tiled in sites:
+                rows += tiled
+            rows += (attn_norm, ffn_norm, ck, cv)
+        return (ctypes.c_void_p * len(rows))(*[t.data_ptr() for t in rows]) if rows else None
 
     def _check_prompt(self):
         """Raise if a bounded wait inside a tensor-core matmul of the last prompt pass expired: waits for the pass, so
