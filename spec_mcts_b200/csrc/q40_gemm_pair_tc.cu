@@ -84,6 +84,8 @@ struct Params {
   int share, rest;         // cut: a pair has share units of CUT blocks, the first `rest` pairs one more
   int bps, own;            // SPLIT: blocks of a rank, and of the four-row groups that it finishes
   int stages, nacc, na;    // ring stages, accumulators, A buffers
+  int dsets, egroups;      // sets that dequantise, and groups that finish tiles beside the main loop: four and one; all five where there is
+                           // but one tile; three and two where finishing takes longer (see layout)
   int run_off, out_off, bar_off;           // byte offsets in the aligned shared memory (run: SPLIT: sums of the other ranks)
   int silu;                // c[0] = silu(A @ deq(B_0)) * (A @ deq(B_1)): a tile is 128 features of
                            // both, of which a CTA has 64 (its A rows 0..63 those of matrix 0)
@@ -111,7 +113,7 @@ struct Slot {
   int i = 0;
   uint32_t turn = 0;
   __device__ __forceinline__ void next(int n) { if (++i == n) { i = 0; turn ^= 1; } }
-  __device__ __forceinline__ void next4(int n) { for (i += 4; i >= n; i -= n) turn ^= 1; }
+  __device__ __forceinline__ void skip(int by, int n) { for (i += by; i >= n; i -= n) turn ^= 1; }
 };
 __device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
   uint32_t r;
@@ -338,7 +340,7 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
       mbar_init(bar_mdone + 8 * lane, 1);
     }
     if (lane < NA) mbar_init(bar_afull + 8 * lane, 8);
-    if (lane < 2) { mbar_init(bar_accfull + 8 * lane, 1); mbar_init(bar_accfree + 8 * lane, 8); }
+    if (lane < 2) { mbar_init(bar_accfull + 8 * lane, 1); mbar_init(bar_accfree + 8 * lane, 8 * p.egroups); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     const int sb0 = SPLIT ? blockIdx.y * p.bps : 0, sb1 = SPLIT ? min(p.nblk, sb0 + p.bps) : 0;
@@ -429,10 +431,10 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
       }
       __syncwarp();
     }
-  } else if (warp >= DQ_WARP0 && warp < EPI_WARP0) {
+  } else if (warp >= DQ_WARP0 && (warp - DQ_WARP0) >> 2 < p.dsets) {
     // warp = (set, quadrant): 32 feature rows = two 16-row tiles of one 64-column group, all k of a block.  Lane (g, t) holds, per
     // 16-row tile and 16 k, rows g and g + 8 at k = 4t .. 4t + 3
-    const int quad = warp & 3, dset = (warp - DQ_WARP0) >> 2;
+    const int quad = warp & 3, dset = (warp - DQ_WARP0) >> 2, dsets = p.dsets;
     const int q = quad >> 1, t = lane & 3;
     // bytes between half steps of a group, and between groups: of one matrix, side by side; with SiLU each of its own
     constexpr int WSTEP = SILU ? 512 : 1024, SSTEP = SILU ? 32 : 64, WGRP = SILU ? RAW_W / 2 : 512, SGRP = SILU ? RAW_S / 2 : 32;
@@ -441,15 +443,15 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
     const uint32_t afull_lead = mapa(bar_afull, lead), ta0 = tmem + ((uint32_t)(32 * quad) << 16) + A_COL0;
     Slot sl, sa, sw;                             // stage and A buffer of this block, and stage of the one that used the buffer before
     for (sl.i = dset, sa.i = dset; sa.i >= NA; sa.i -= NA) sa.turn ^= 1;
-    for (sw.i = dset; sw.i < NA;) sw.i += DSETS;
-    sw.i -= NA;                                  // of the first block that waits for one; below DSETS
-    for (int i = dset; i < total; i += DSETS) {
+    for (sw.i = dset; sw.i < NA;) sw.i += dsets;
+    sw.i -= NA;                                  // of the first block that waits for one; below dsets, and so below S
+    for (int i = dset; i < total; i += dsets) {
       // The MMAs of the block that last used this A buffer are complete.  As the ring has at least NA stages, the block that
       // last used this stage is through as well, and the stage's barriers, which tell only odd from even phases, are in one
       // of the two phases that they can tell apart
       if (i >= NA) {
         wait_limited(bar_mdone + 8 * sw.i, sw.turn, limit);
-        sw.next4(S);
+        sw.skip(dsets, S);
       }
       wait_limited(bar_full + 8 * sl.i, sl.turn, limit);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -468,29 +470,30 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(afull_lead + 8 * sa.i);
-      sl.next4(S);
-      sa.next4(NA);
+      sl.skip(dsets, S);
+      sa.skip(dsets, NA);
     }
     failed = limit == 0;
   }
   if (!SPLIT && warp >= DQ_WARP0) {
     // ================= accumulators -> output =================
-    // Group 0 (warps 20..23) finishes every tile but the pair's last beside the main loop; the last one (the last range of it)
-    // falls to all groups, the dequantisers having come to their end: 16-row chunks group, group + GROUPS, ...
+    // Group 0 (warps 20..23; with it group 1, of warps 16..19, if p.egroups is 2) finishes every tile but the pair's last beside the main
+    // loop; the last one (the last range of it) falls to all groups, the dequantisers having come to their end: 16-row chunks group,
+    // group + GROUPS, ...
     // No wait leaves these loops early, so that the warps of a group always meet at its (plain) barrier.
-    const int group = warp >= EPI_WARP0 ? 0 : 1 + ((warp - DQ_WARP0) >> 2);
+    const int group = DSETS - ((warp - DQ_WARP0) >> 2), E = SILU && !CUT_K ? 1 : p.egroups;
     const int quad = warp & 3, feat = 32 * quad + lane;
     const uint32_t lane_base = tmem + ((uint32_t)(32 * quad) << 16);
-    // two buffers of 16 finished rows per group; those of groups 1.. over the ring, which is idle by then
-    __half* out_g = group == 0 ? out_s : reinterpret_cast<__half*>(gbase) + (group - 1) * 2 * 16 * OUT_LD;
+    // two buffers of 16 finished rows per group; those of groups E.. over the ring, which is idle by then
+    __half* out_g = (group < E ? out_s + group * 2 * 16 * OUT_LD : reinterpret_cast<__half*>(gbase) + (group - E) * 2 * 16 * OUT_LD);
     const int nchunk = p.npad / 16;
     Slot sc;                                                 // accumulator
     int turn = 0;                                            // output buffer
     const int ranges = CUT_K ? wk.np : wk.np * ((p.nblk + p.rblk - 1) / p.rblk);
-    int gr = 0;                                              // ranges that group 0 has read
+    int gr = 0;                                              // ranges that this group has read
     // outputs, scratch and flags may still be in use by the launch in front of this one
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (int k = group == 0 ? 0 : max(0, wk.np - 1); k < wk.np; ++k) {
+    for (int k = group < E ? 0 : max(0, wk.np - 1); k < wk.np; ++k) {
       int tile, b0, b1, pi, span, fh, m0;
       wk.piece(k, tile, b0, b1);
       decode(tile, pi, span, fh, m0);
@@ -510,8 +513,8 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
         const bool add_run = b > b0;
         b = e;
         all = e == b1 && k == wk.np - 1;
-        if (group > 0 && !all) continue;
-        const int ch0 = all ? group : 0, step = all ? GROUPS : 1;
+        if (group >= E && !all) continue;
+        const int ch0 = group, step = all ? GROUPS : E;
         const float* first = p.part + ((int64_t)(q0 * 2 + half) * p.npad) * FEATS + feat;
         float v[16];
         if (CUT_K && e == b1 && q0 < me) {
@@ -540,12 +543,12 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
         }
         // (a barrier's parity tells a phase from its neighbours only: the other groups, which have not followed accfull,
         // wait for the end of all MMAs and for group 0, which has)
-        if (group == 0) {
+        if (group < E) {
           // one warp polls for the four (polls are issue slots: with all of them, and three more warps that had nothing else to do, a
           // third of all instructions)
           if (quad == 2) wait_limited(bar_accfull + 8 * sc.i, sc.turn, limit);
-          asm volatile("bar.sync %0, 128;" ::"n"(1 + GROUPS) : "memory");
-          if (all && lane == 0) {
+          asm volatile("bar.sync %0, 128;" ::"r"(1 + GROUPS + group) : "memory");
+          if (all && group == 0 && lane == 0) {
             *s_acc = sc.i;
             mbar_arrive(bar_last);
           }
@@ -642,12 +645,12 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
         // published: GROUPS arrivals per flag, whoever drained the accumulator
         __threadfence();
         __syncwarp();
-        if (lane == 0) atomicAdd(p.flags + me * 16 + half * 4 + quad, all ? 1 : GROUPS);
+        if (lane == 0) atomicAdd(p.flags + me * 16 + half * 4 + quad, all || group > 0 ? 1 : GROUPS - (E - 1));
       }
     }
     failed = failed || limit == 0;
   }
-  if (warp >= DQ_WARP0 && (!SPLIT || warp < EPI_WARP0)) wait_limited(bar_done, 0, limit);
+  if (warp >= DQ_WARP0) wait_limited(bar_done, 0, limit);
   if (failed || limit == 0) *s_failed = 1;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   __syncthreads();
@@ -777,17 +780,23 @@ static void tile_rows(Params& p, int npad) {
 
 // Shared memory of a launch, or 0 if it does not fit: [ring][run][rows on their way out][barriers]; ring stages, accumulators and A
 // buffers.  `single`: no pair has more than one tile, of one range, and a second accumulator would be for nothing.  Else two where
-// they fit tensor memory beside at least two A buffers
+// they fit tensor memory beside at least two A buffers.
+// Two groups finish tiles where that is what a pair waits for: the sums of ranges of few blocks (three matrices of 512 rows x 4096 x 4096, eight
+// blocks: 54.4 us with one, 52.4; 300 rows 39.0 and 34.9; but 22 blocks, x 11008 x 4096, 43.3 and 46.4), and many rows of a SiLU product
+// with shared tiles (x 4096 x 11008, 100 rows 26.2 and 24.5, 128 28.8 and 26.2; 77 21.7 and 22.0).  Where there is one tile a pair, its warps
+// dequantise too (10 rows x 4096 x 12288 12.1 and 11.8, x 11008 x 4096 11.6 and 11.4, 64 rows 12.7 and 12.3, 100 the same)
 static size_t layout(Params& p, int split, bool single) {
   const size_t tile = (size_t)p.npad * FEATS * 4, stage = RAW_PAD + (size_t)p.npad * 64 * BLK;
   p.own = ((p.M + 3) / 4 + split - 1) / split;
   const size_t run = split > 1 ? (size_t)(split - 1) * p.own * FEATS * 16 : p.range < p.k64 ? tile : 0;
-  const size_t out = split > 1 ? 0 : 2 * 16 * OUT_LD * 2;
+  p.egroups = !single && (p.silu ? p.cut && p.npad >= 96 : 8 * p.rblk <= p.npad) ? 2 : 1;
+  const size_t out = split > 1 ? 0 : p.egroups * 2 * 16 * OUT_LD * 2;
   const size_t fixed = 1024 /* alignment */ + BAR_BYTES + 64 /* tail */ + run + out;
   if (fixed + DSETS * stage > (size_t)SMEM_MAX) return 0;
   p.stages = std::min(S_MAX, (int)((SMEM_MAX - fixed) / stage));
   p.nacc = !single && 2 * p.npad + 2 * A_COLS <= TMEM_COLS ? 2 : 1;
   p.na = std::min({NA_MAX, p.stages, (TMEM_COLS - p.nacc * p.npad) / A_COLS});
+  p.dsets = single && p.stages > DSETS ? GROUPS : GROUPS - p.egroups;
   const size_t off = p.stages * stage;
   p.run_off = (int)off;
   p.out_off = (int)(off + run);
