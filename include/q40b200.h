@@ -159,6 +159,7 @@ int q40_gemm_kn_static_error(int* host_out, int clear, void* stream);
 
 /* Y[M,N] = X[M,K] @ deq(W)[N,K]^T, W quantised from a row-major [N,K] matrix (groups
  * along K): wq viewed as [N*K/(2*group), group], ws as [N*K/group].  K % (2*group) == 0.
+ * More than 8 rows may run on tcgen05, whose bounded waits report expiry in the int at byte 4092 of the workspace.
  * Replaces: dequantize_q40 + F.linear in LinearQ4_0.forward (quantize.py:235-246,
  * hf_model_q40.py:222-233). */
 int q40_gemm_nk(const void* x, int64_t ldx, const void* wq, const void* ws, void* y,

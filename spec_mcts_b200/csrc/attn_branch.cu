@@ -143,7 +143,7 @@ attn_branch_kernel(const BranchArgs a) {
 
   if (a.beside_prefix) asm volatile("griddepcontrol.wait;" ::: "memory");
   RowMerge<NG, RT> merge;
-  merge.load(a, bh, tr, lane);
+  merge.load(a, rows, bh, tr, lane);
 
   const int g0 = slot * NG;
   if (sub == 0) { sm_m[g0 + grp] = m; sm_l[g0 + grp] = l; }
@@ -154,7 +154,7 @@ attn_branch_kernel(const BranchArgs a) {
   else if (WPR == 1) __syncwarp();
   else asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "n"(RT) : "memory");
 
-  merge.finish(a, bh, tr, lane, sm_m + g0, sm_l + g0, sm_o + g0);
+  merge.finish(a, rows, bh, tr, lane, sm_m + g0, sm_l + g0, sm_o + g0);
 }
 
 template <int MODE, int NW, int WPR, int U>

@@ -290,11 +290,11 @@ attn_branch_q4_kernel(const Q4Args<ROT> a) {
       : t == 2 ? make_float4(o[8], o[9], o[10], o[11]) : make_float4(o[12], o[13], o[14], o[15]);
   if (a.beside_prefix) asm volatile("griddepcontrol.wait;" ::: "memory");
   RowMerge<WPR, RT> merge;
-  merge.load(a, bh, part * 32 + lane, lane);
+  merge.load(a, rows, bh, part * 32 + lane, lane);
   if (WPR == 1) __syncwarp();
   else if (WPR == Q4_NW) __syncthreads();
   else asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "n"(RT) : "memory");
-  merge.finish(a, bh, part * 32 + lane, lane, sm_m + slot * WPR, sm_l + slot * WPR, sm_o + slot * WPR);
+  merge.finish(a, rows, bh, part * 32 + lane, lane, sm_m + slot * WPR, sm_l + slot * WPR, sm_o + slot * WPR);
 }
 
 template <bool ROT, int WPR, bool SC4>

@@ -75,25 +75,25 @@ struct RowMerge {
   float pm_l, pl_l, po[PB][DP];
   // The prefix partials, once they are there and before the row's warps meet: lane sp holds the maximum and the sum of split sp
   // (further splits are read at the end), and the first splits' outputs are all requested together
-  __device__ __forceinline__ void load(const BranchArgs& a, int64_t bh, int tr, int lane) {
-    pm_l = lane < a.nsp ? a.pm[(int64_t)lane * a.rows + bh] : -CUDART_INF_F;
-    pl_l = lane < a.nsp ? a.pl[(int64_t)lane * a.rows + bh] : 0.f;
+  __device__ __forceinline__ void load(const BranchArgs& a, int64_t rows, int64_t bh, int tr, int lane) {
+    pm_l = lane < a.nsp ? a.pm[(int64_t)lane * rows + bh] : -CUDART_INF_F;
+    pl_l = lane < a.nsp ? a.pl[(int64_t)lane * rows + bh] : 0.f;
     if (a.nsp > 0) {
 #pragma unroll
       for (int i = 0; i < PB; ++i)
 #pragma unroll
         for (int j = 0; j < DP; ++j)
-          po[i][j] = i < a.nsp && (RT <= ATTN_D || tr < ATTN_D) ? a.po[((int64_t)i * a.rows + bh) * ATTN_D + tr + j * RT] : 0.f;
+          po[i][j] = i < a.nsp && (RT <= ATTN_D || tr < ATTN_D) ? a.po[((int64_t)i * rows + bh) * ATTN_D + tr + j * RT] : 0.f;
     }
   }
-  __device__ __forceinline__ void finish(const BranchArgs& a, int64_t bh, int tr, int lane, const float* sm_m, const float* sm_l,
+  __device__ __forceinline__ void finish(const BranchArgs& a, int64_t rows, int64_t bh, int tr, int lane, const float* sm_m, const float* sm_l,
                                          const float (*sm_o)[ATTN_D]) {
     if (RT > ATTN_D && tr >= ATTN_D) return;
     float M = -CUDART_INF_F;
 #pragma unroll
     for (int g = 0; g < NG; ++g) M = fmaxf(M, sm_m[g]);
     M = fmaxf(M, warp_max(pm_l));
-    for (int sp = 32; sp < a.nsp; ++sp) M = fmaxf(M, a.pm[(int64_t)sp * a.rows + bh]);
+    for (int sp = 32; sp < a.nsp; ++sp) M = fmaxf(M, a.pm[(int64_t)sp * rows + bh]);
     float Lsum = 0.f, acc[DP];
 #pragma unroll
     for (int j = 0; j < DP; ++j) acc[j] = 0.f;
@@ -118,11 +118,11 @@ struct RowMerge {
           const float w = __shfl_sync(0xffffffffu, pw_l, sp);
           Lsum = fmaf(__shfl_sync(0xffffffffu, pl_l, sp), w, Lsum);
 #pragma unroll
-          for (int j = 0; j < DP; ++j) acc[j] = fmaf(a.po[((int64_t)sp * a.rows + bh) * ATTN_D + tr + j * RT], w, acc[j]);
+          for (int j = 0; j < DP; ++j) acc[j] = fmaf(a.po[((int64_t)sp * rows + bh) * ATTN_D + tr + j * RT], w, acc[j]);
         }
       }
       for (int sp = 32; sp < a.nsp; ++sp) {
-        const int64_t r = (int64_t)sp * a.rows + bh;
+        const int64_t r = (int64_t)sp * rows + bh;
         const float w = ex2(a.pm[r] - M);
         Lsum = fmaf(a.pl[r], w, Lsum);
 #pragma unroll

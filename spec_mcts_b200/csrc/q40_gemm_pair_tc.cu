@@ -90,6 +90,8 @@ struct Params {
   int silu;                // c[0] = silu(A @ deq(B_0)) * (A @ deq(B_1)): a tile is 128 features of
                            // both, of which a CTA has 64 (its A rows 0..63 those of matrix 0)
   int vec;                 // outputs take 16-byte stores
+  const __half* nk_s;      // NK: scales [n_cols][K / 64]
+  int n_cols;
   float* part;             // scratch slots: [pair][half][npad][128]
   int* flags;              // per pair: see FLAG_BYTES
   int* err;
@@ -162,6 +164,14 @@ __device__ __forceinline__ void mma2_ts(uint32_t tmem_d, uint32_t tmem_a, uint64
       ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accum) : "memory");
 }
 
+// 16 columns of the lane's own row of tensor memory
+__device__ __forceinline__ void st_32x32b_x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+
 // Waits for tensor-memory loads; naming the registers keeps their uses behind it
 __device__ __forceinline__ void wait_ld16(uint32_t (&r)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;"
@@ -170,9 +180,12 @@ __device__ __forceinline__ void wait_ld16(uint32_t (&r)[16]) {
 }
 
 // `n` finished rows of W features from shared memory to the output, by the 128 threads t of a group
-template <int W>
-__device__ __forceinline__ void store_rows(const __half* o, __half* c, int64_t ldc, int n, int t, int vec) {
-  if (vec) {
+template <int W, bool RAGGED = false>
+__device__ __forceinline__ void store_rows(const __half* o, __half* c, int64_t ldc, int n, int t, int vec, int cols = W) {
+  if (RAGGED && (cols < W || vec == 2)) {                    // fewer features than W, or rows at any address
+    for (int row = t / 32; row < n; row += 4)
+      for (int col = t % 32; col < cols; col += 32) c[row * ldc + col] = o[row * OUT_LD + col];
+  } else if (vec) {
     const int col = t % (W / 8) * 8;
     for (int row = t / (W / 8); row < n; row += 1024 / W)
       *reinterpret_cast<uint4*>(c + row * ldc + col) = *reinterpret_cast<const uint4*>(o + row * OUT_LD + col);
@@ -206,6 +219,32 @@ struct KCursor {
   }
 };
 
+// NK: 64 bytes of a row, 16 at a time, are 64 k of one group in their high nibbles and 64 k of the next in their low ones, and a lane's columns of
+// the A buffer from ta on and from ta + 32 on: fp16(code * scale) of k pairs.  The 16-byte pieces lie swizzled (64 bytes)
+__device__ __forceinline__ void dequant_row(const unsigned char* row, int swizzle, uint32_t scales, uint32_t ta) {
+  constexpr uint32_t HI = 0x54805480u, LO = 0x64086408u;     // see dequant_step; both codes are two's complement here
+  const __half2 sh = __low2half2(u32_as_h2(scales)), sl = __high2half2(u32_as_h2(scales));
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t hi[16], lo[16];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const uint4 v = *reinterpret_cast<const uint4*>(row + (((2 * h + c) ^ swizzle) << 4));
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t p0 = prmt(w[j], w[j], 0x1100), p1 = prmt(w[j], w[j], 0x3322);       // bytes 0 and 1, 2 and 3, to 16 bits each
+        hi[8 * c + 2 * j] = deq_pair<HI>(lop3_and_xor(p0, 0x00F000F0u, HI), sh);
+        hi[8 * c + 2 * j + 1] = deq_pair<HI>(lop3_and_xor(p1, 0x00F000F0u, HI), sh);
+        lo[8 * c + 2 * j] = deq_pair<LO>(lop3_and_xor(p0, 0x000F000Fu, LO), sl);
+        lo[8 * c + 2 * j + 1] = deq_pair<LO>(lop3_and_xor(p1, 0x000F000Fu, LO), sl);
+      }
+    }
+    st_32x32b_x16(ta + 16 * h, hi);
+    st_32x32b_x16(ta + 32 + 16 * h, lo);
+  }
+}
+
 // The pieces of tiles that a pair works on, in the order it takes them: the one it publishes first (the last tile, if its
 // k range goes on beyond the pair's share), the one it may have to wait for last (the first tile)
 struct Work {
@@ -228,7 +267,8 @@ struct Work {
 // distributed shared memory.  Otherwise a cluster is a pair.
 // CUT: tiles may be shared between pairs along k; SILU: see Params (compiled for each, to keep the registers of all roles
 // below the 80 that 24 warps leave)
-template <bool SPLIT, bool CUT_K, bool SILU>
+// NK: one matrix [n_cols, K] with groups along K, as quantised in memory (not a tiled copy): a lane expands its own feature's row
+template <bool SPLIT, bool CUT_K, bool SILU, bool NK = false>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
   extern __shared__ unsigned char smem_raw[];
@@ -297,8 +337,10 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
         const uint32_t dst = ring + s * stage_bytes;
         if (weights) {
           const int step = (span * p.k64 + kc.k) * 4;
-          mbar_expect_tx(bar_full + 8 * s, RAW_BYTES);
-          if constexpr (SILU) {                                                  // a 64-column group of each matrix
+          mbar_expect_tx(bar_full + 8 * s, NK ? RAW_W : RAW_BYTES);
+          if constexpr (NK) {
+            tma_2d(dst, &maps.w[0], kc.k * 32, span * SPAN + half * FEATS, bar_full + 8 * s);                  // x in bytes
+          } else if constexpr (SILU) {                                                  // a 64-column group of each matrix
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
               tma_2d(dst + m * (RAW_W / 2), &maps.w[m], fh * 256 + half * 128, step, bar_full + 8 * s);    // x in words of four bytes
@@ -349,15 +391,18 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
     if (lane == 0) *s_share = share;
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    if (elect_one()) copy_blocks(Work(share, p.nblk), 0, S, true);
+    if (elect_one()) {
+      if (NK) asm volatile("griddepcontrol.wait;" ::: "memory");       // the launch in front may be the one that writes the weights
+      copy_blocks(Work(share, p.nblk), 0, S, true);
+    }
     __syncwarp();
   } else {
     if (warp == 1) {
       asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(TMEM_COLS));
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    } else if (warp == 3 && lane <= 6) {
-      const CUtensorMap* m = lane == 0 ? &maps.act : lane <= 3 ? &maps.w[lane - 1] : &maps.s[lane - 4];
+    } else if (warp == 3 && lane <= (NK ? 1 : 2 * p.nprob)) {
+      const CUtensorMap* m = lane == 0 ? &maps.act : lane <= p.nprob ? &maps.w[lane - 1] : &maps.s[lane - 1 - p.nprob];
       asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
     }
     __syncwarp();
@@ -445,6 +490,31 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
     for (sl.i = dset, sa.i = dset; sa.i >= NA; sa.i -= NA) sa.turn ^= 1;
     for (sw.i = dset; sw.i < NA;) sw.i += dsets;
     sw.i -= NA;                                  // of the first block that waits for one; below dsets, and so below S
+    // NK: the lane's row, where this block's scales are, and how many blocks of the piece begin there; scales are read a block ahead
+    const __half* sc = nullptr;
+    int piece = 0, kb = dset, len = 1;
+    uint32_t scales = 0;
+    auto next_scales = [&]() {
+      if (sc == nullptr || kb >= len) {
+        if (sc != nullptr) { kb -= len; ++piece; }
+        for (;; ++piece) {
+          int tile, b0, b1, pi, span, fh, m0;
+          wk.piece(piece, tile, b0, b1);
+          decode(tile, pi, span, fh, m0);
+          len = b1 - b0;
+          sc = p.nk_s + (int64_t)min(span * SPAN + fh * FEATS + 32 * quad + lane, p.n_cols - 1) * (p.K / 64) + 2 * b0;
+          if (kb < len) break;
+          kb -= len;
+        }
+      }
+      scales = __ldg(reinterpret_cast<const uint32_t*>(sc + 2 * kb));
+      kb += dsets;
+    };
+    const int frow = 32 * quad + lane;
+    if constexpr (NK) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (dset < total) next_scales();
+    }
     for (int i = dset; i < total; i += dsets) {
       // The MMAs of the block that last used this A buffer are complete.  As the ring has at least NA stages, the block that
       // last used this stage is through as well, and the stage's barriers, which tell only odd from even phases, are in one
@@ -456,6 +526,11 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
       wait_limited(bar_full + 8 * sl.i, sl.turn, limit);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t so = sl.i * stage_bytes, ta = ta0 + sa.i * A_COLS;
+      if constexpr (NK) {
+        const uint32_t now = scales;
+        if (i + dsets < total) next_scales();
+        dequant_row(gbase + so + frow * 64, (frow >> 1) & 3, now, ta);
+      } else
 #pragma unroll
       for (int h = 0; h < BLK; ++h) {
         uint32_t r[2][16];
@@ -498,7 +573,7 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
       wk.piece(k, tile, b0, b1);
       decode(tile, pi, span, fh, m0);
       const bool whole = !CUT_K || b1 == p.nblk;                       // this pair has the tile's last blocks and finishes it
-      const int rows = min(p.npad, p.M - m0);
+      const int rows = min(p.npad, p.M - m0), cols = NK ? min(FEATS, p.n_cols - span * SPAN - fh * FEATS) : FEATS;
       const int64_t ldc = p.ldc[pi];
       __half* c = p.c[pi] + (int64_t)m0 * ldc + span * SPAN + fh * FEATS + (SILU ? half * (FEATS / 2) : 0);
       // the pairs with its first blocks, whose sums are added in k order
@@ -632,7 +707,7 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) o[j * OUT_LD + feat] = __float2half_rn(__uint_as_float(r[j]));
             asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
-            store_rows<FEATS>(o, c + (int64_t)ch * 16 * ldc, ldc, min(16, rows - ch * 16), feat, p.vec);
+            store_rows<FEATS, NK>(o, c + (int64_t)ch * 16 * ldc, ldc, min(16, rows - ch * 16), feat, p.vec, cols);
           }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -704,7 +779,8 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
         o[2 * OUT_LD + feat] = __float2half_rn(v.z);
         o[3 * OUT_LD + feat] = __float2half_rn(v.w);
         asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
-        store_rows<FEATS>(o, c + (int64_t)(4 * g) * p.ldc[pi], p.ldc[pi], min(4, rows - 4 * g), feat, p.vec);
+        store_rows<FEATS, NK>(o, c + (int64_t)(4 * g) * p.ldc[pi], p.ldc[pi], min(4, rows - 4 * g), feat, p.vec,
+                              NK ? min(FEATS, p.n_cols - span * SPAN - fh * FEATS) : FEATS);
         asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
       }
       if (limit == 0) q40_set_error(p.err);
@@ -727,7 +803,7 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
 
 using PairKernel = void (*)(const q40::ttc::pair::Params, const q40::ttc::pair::Maps);
 
-// [0] SPLIT; else 1 + 1 SiLU + 2 cut
+// [0] SPLIT; else 1 + 1 SiLU + 2 cut; [5], [6] SPLIT and not, with groups along K
 static PairKernel pair_kernel(int which) {
   using namespace q40::ttc::pair;
   switch (which) {
@@ -735,7 +811,9 @@ static PairKernel pair_kernel(int which) {
     case 1: return gemm_pair_kernel<false, false, false>;
     case 2: return gemm_pair_kernel<false, false, true>;
     case 3: return gemm_pair_kernel<false, true, false>;
-    default: return gemm_pair_kernel<false, true, true>;
+    case 4: return gemm_pair_kernel<false, true, true>;
+    case 5: return gemm_pair_kernel<true, false, false, true>;
+    default: return gemm_pair_kernel<false, false, false, true>;
   }
 }
 
@@ -818,8 +896,6 @@ static void k_blocks(Params& p, int range) {
 }  // namespace ttc
 }  // namespace q40
 
-// The launch that q40_gemm_tiled_tc_multi and q40_gemm_tiled_tc_ws make: see q40_tc_common.cuh.  Arguments are checked.
-//
 // Which launch: the one of least estimated time.  Nanoseconds on a B200, weights from HBM, launches in a row; npad = rows
 // of a tile, a block = 128 k of 256 features:
 //   a block           232 + npad / 4, or the MMAs' 2.2 npad (one tile per pair; 16 rows 236, 112 rows 258, 128 rows 283);
@@ -829,35 +905,25 @@ static void k_blocks(Params& p, int range) {
 // 10 rows x 4096 x 11008, two matrices: 16.8 us shared, 21.9 not, 29.3 split in two; 100 rows x 11008 x 4096: 15.7 split in
 // three, 17.6 in two, 27.5 not; 512 rows x 4096 x 11008: 128-row tiles 41.3, 112 39.5, 176 45.4, 256 57.2: there the
 // estimate, 39.9 for 176 rows and 40.4 for 112, takes the slower one.
-int q40_pair_gemm(int nmat, const void* a, int64_t lda, const void* const* bw_tiled, void* const* c, const int64_t* ldc,
-                  const int* n_cols, int M, int K, int ranges, int silu, void* workspace, size_t workspace_bytes, double beat_ns,
-                  int* err, int use_pdl, void* stream) {
+// The launch of p's matmul (matrices, sizes and k blocks are in it) as the variant of least estimated time, if that is below beat_ns
+template <typename EncodeWeights>
+static int pair_run(q40::ttc::pair::Params& p, bool nk, int spans, const void* a, int64_t lda, void* workspace, size_t workspace_bytes, double beat_ns,
+                    int use_pdl, void* stream, EncodeWeights encode_weights) {
   using namespace q40;
   using namespace q40::ttc;
-  pair::Params p{};
-  int spans = 0;
-  p.vec = 1;
-  for (int i = 0; i < nmat; ++i) {
-    p.c[i] = (__half*)c[i]; p.ldc[i] = ldc[i];
-    p.spans[i] = n_cols[i] / SPAN;
-    p.vec &= q40_aligned(c[i], 16) && ldc[i] % 8 == 0;
-    spans += p.spans[i];
-  }
+  const int M = p.M, K = p.K, silu = p.silu;
   EncodeTiledFn encode = ttc_encode_fn();
   if (!encode) return Q40_E_UNSUPPORTED;
-  p.nprob = nmat; p.M = M; p.K = K; p.err = err; p.silu = silu;
-  p.k64 = K / BK;
-  pair::k_blocks(p, ranges > 1 ? (p.k64 + ranges - 1) / ranges : p.k64);
   if ((int64_t)spans * ((M + 63) / 64) * std::max(p.nblk, pair::MAX_PAIRS) > 0x7fffffffLL) return Q40_E_UNSUPPORTED;
   // the kernels' attributes come first: the runtime is asked how many fit with the shared memory that they allow
-  static std::atomic<uint64_t> ready[5];
+  static std::atomic<uint64_t> ready[7];
   auto kernel = [&](int which) -> PairKernel {
     PairKernel k = pair_kernel(which);
     if (q40_allow_smem(ready[which], (const void*)k, SMEM_MAX) == cudaSuccess) return k;
     (void)cudaGetLastError();
     return nullptr;
   };
-  PairKernel plain = kernel(1), in_clusters = kernel(0);
+  PairKernel plain = kernel(nk ? 6 : 1), in_clusters = kernel(nk ? 5 : 0);
   if (!plain || !in_clusters) return Q40_E_UNSUPPORTED;
   const int fit = pair_max_clusters(plain, 1) < pair::MAX_PAIRS ? pair_max_clusters(plain, 1) : pair::MAX_PAIRS;
   if (fit < 1) return Q40_E_UNSUPPORTED;
@@ -910,7 +976,7 @@ int q40_pair_gemm(int nmat, const void* a, int64_t lda, const void* const* bw_ti
   }
   const size_t smem = pair::layout(p, split, split > 1 || (!cut && p.ntiles <= npairs && p.range == p.k64));
   if (smem == 0 || smem > (size_t)SMEM_MAX) return Q40_E_UNSUPPORTED;
-  PairKernel kern = kernel(split > 1 ? 0 : 1 + silu + 2 * cut);
+  PairKernel kern = split > 1 ? in_clusters : nk ? plain : kernel(1 + silu + 2 * cut);
   if (!kern) return Q40_E_UNSUPPORTED;
   pair::Maps maps;
   const cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)M};
@@ -921,16 +987,7 @@ int q40_pair_gemm(int nmat, const void* a, int64_t lda, const void* const* bw_ti
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return Q40_E_UNSUPPORTED;
-  for (int i = 0; i < nmat; ++i) {
-    const cuuint64_t wdim[2] = {STEP_BYTES / 4, (cuuint64_t)p.spans[i] * (K / 16)};
-    const cuuint64_t wstride[1] = {STEP_BYTES};
-    const cuuint32_t wbox[2] = {silu ? 128u : 256u, 4 * pair::BLK}, sbox[2] = {silu ? 8u : 16u, 4 * pair::BLK};
-    for (int j = 0; j < 2; ++j)
-      if (encode(j ? &maps.s[i] : &maps.w[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, (void*)bw_tiled[i], wdim, wstride, j ? sbox : wbox,
-                 estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return Q40_E_UNSUPPORTED;
-  }
+  if (!encode_weights(encode, maps)) return Q40_E_UNSUPPORTED;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(2 * npairs, split, 1);
   cfg.blockDim = dim3(pair::THREADS, 1, 1);
@@ -948,6 +1005,62 @@ int q40_pair_gemm(int nmat, const void* a, int64_t lda, const void* const* bw_ti
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p, maps);
   if (e != cudaSuccess) return (int)e;
   return Q40_OK;
+}
+
+// The launch that q40_gemm_tiled_tc_multi and q40_gemm_tiled_tc_ws make: see q40_tc_common.cuh.  Arguments are checked.
+int q40_pair_gemm(int nmat, const void* a, int64_t lda, const void* const* bw_tiled, void* const* c, const int64_t* ldc,
+                  const int* n_cols, int M, int K, int ranges, int silu, void* workspace, size_t workspace_bytes, double beat_ns,
+                  int* err, int use_pdl, void* stream) {
+  using namespace q40;
+  using namespace q40::ttc;
+  pair::Params p{};
+  int spans = 0;
+  p.vec = 1;
+  for (int i = 0; i < nmat; ++i) {
+    p.c[i] = (__half*)c[i]; p.ldc[i] = ldc[i];
+    p.spans[i] = n_cols[i] / SPAN;
+    p.vec &= q40_aligned(c[i], 16) && ldc[i] % 8 == 0;
+    spans += p.spans[i];
+  }
+  p.nprob = nmat; p.M = M; p.K = K; p.err = err; p.silu = silu;
+  p.k64 = K / BK;
+  pair::k_blocks(p, ranges > 1 ? (p.k64 + ranges - 1) / ranges : p.k64);
+  return pair_run(p, false, spans, a, lda, workspace, workspace_bytes, beat_ns, use_pdl, stream, [&](EncodeTiledFn encode, pair::Maps& maps) {
+    const cuuint32_t estr[2] = {1, 1};
+    for (int i = 0; i < nmat; ++i) {
+      const cuuint64_t wdim[2] = {STEP_BYTES / 4, (cuuint64_t)p.spans[i] * (K / 16)};
+      const cuuint64_t wstride[1] = {STEP_BYTES};
+      const cuuint32_t wbox[2] = {silu ? 128u : 256u, 4 * pair::BLK}, sbox[2] = {silu ? 8u : 16u, 4 * pair::BLK};
+      for (int j = 0; j < 2; ++j)
+        if (encode(j ? &maps.s[i] : &maps.w[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, (void*)bw_tiled[i], wdim, wstride, j ? sbox : wbox,
+                   estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+          return false;
+    }
+    return true;
+  });
+}
+
+// Y[M, N] = X[M, K] @ deq(W)^T for W [N, K] with groups of 64 along K: see q40_gemm_nk, whose arguments are checked.  K % 128 == 0; x on 16-byte
+// boundaries, rows too.  Weights may be what the launch in front writes: they are requested behind the wait for it
+int q40_pair_linear(const void* x, int64_t ldx, const void* wq, const void* ws, void* y, int64_t ldy, int M, int N, int K, double beat_ns,
+                    int* err, void* stream) {
+  using namespace q40;
+  using namespace q40::ttc;
+  pair::Params p{};
+  p.c[0] = (__half*)y; p.ldc[0] = ldy;
+  p.spans[0] = (N + SPAN - 1) / SPAN;
+  p.vec = q40_aligned(y, 16) && ldy % 8 == 0 ? 1 : q40_aligned(y, 4) && ldy % 2 == 0 ? 0 : 2;
+  p.nprob = 1; p.M = M; p.K = K; p.err = err;
+  p.nk_s = (const __half*)ws; p.n_cols = N;
+  p.k64 = K / BK;
+  pair::k_blocks(p, p.k64);
+  return pair_run(p, true, p.spans[0], x, ldx, nullptr, 0, beat_ns, 1, stream, [&](EncodeTiledFn encode, pair::Maps& maps) {
+    const cuuint64_t dim[2] = {(cuuint64_t)K / 2, (cuuint64_t)N}, pitch[1] = {(cuuint64_t)K / 2};
+    const cuuint32_t box[2] = {64, pair::FEATS}, estr[2] = {1, 1};
+    return encode(&maps.w[0], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)wq, dim, pitch, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  });
 }
 
 // Scratch of q40_gemm_tiled_tc_ws: flags and one slot of sums per pair (0: none is used for so many rows)

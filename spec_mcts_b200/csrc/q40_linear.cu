@@ -61,6 +61,9 @@ template <int MT>
 __global__ void __launch_bounds__(THREADS, 1) linear_kernel(const Args p) {
   extern __shared__ __align__(16) unsigned char smem[];
   cg::cluster_group cluster = cg::this_cluster();
+  // started while the launch in front drains (which may be the one that writes the weights): 0.9 us of a call
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   __half* xs = reinterpret_cast<__half*>(smem);                       // [M][xk + XPAD], in fours of the order x0 x2 x1 x3
   float* slab = reinterpret_cast<float*>(smem + p.off_slab);          // [kw][TILES][MT * 8][M_LD]
   float* out = reinterpret_cast<float*>(smem + p.off_out);            // [TILES][MT * 8][16] this CTA's sums
@@ -255,33 +258,29 @@ static int launch(Args& p, int c, int clusters, size_t smem, cudaStream_t st) {
   cfg.blockDim = dim3(THREADS, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = c; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   const cudaError_t l = cudaLaunchKernelEx(&cfg, linear_kernel<MT>, p);
   return l == cudaSuccess ? Q40_OK : (int)l;
 }
 
-}  // namespace nk
-}  // namespace q40
-
-// q40_gemm_nk for up to 32 rows and groups of 64, or Q40_E_UNSUPPORTED.  Arguments are checked.
-int q40_linear(const void* x, int64_t ldx, const void* wq, const void* ws, void* y, int64_t ldy, int M, int N, int K, void* stream) {
-  using namespace q40;
-  using namespace q40::nk;
-  if (M > 32) return Q40_E_UNSUPPORTED;
-  const int mt = M <= 8 ? 1 : (M <= 16 ? 2 : 4), tiles = (N + 15) / 16, ksteps = K / STEP;
+// The launch of least estimated time (`ns`, of what differs between launches); c == 0: none, gemv_nk_kernel takes the call
+struct Plan {
   Args p{};
-  p.wide_s = K % 256 == 0 && q40_aligned(ws, 8);
-  p.wide_x = q40_aligned(x, 16) && ldx % 8 == 0;
-  p.x = (const __half*)x; p.ldx = ldx; p.w = (const uint8_t*)wq; p.s = (const __half*)ws; p.y = (__half*)y; p.ldy = ldy;
+  int c = 0, clusters = 0, busiest = 0;            // CTAs of a cluster, clusters, steps of the busiest warp
+  size_t smem = 0;
+  double ns = 1e30;
+};
+static Plan make_plan(int M, int N, int K) {
+  const int mt = M <= 8 ? 1 : (M <= 16 ? 2 : 4), tiles = (N + 15) / 16, ksteps = K / STEP;
+  Plan best;
+  Args p{};
   p.M = M; p.N = N; p.K = K;
-  double best = 1e30;
-  int bc = 0, bclusters = 0, busiest = 0;
-  size_t bsmem = 0;
-  Args bp{};
   for (int c = 1; c <= 4; c *= 2) {
     if (c > ksteps) break;
     const int fit = c == 1 ? 148 : (c == 2 ? 74 : 33);
@@ -301,19 +300,42 @@ int q40_linear(const void* x, int64_t ldx, const void* wq, const void* ws, void*
       // costs.  (Without the quarter 1 row x 2048 x 10711, where a warp had five single steps, 10.2 us, 8.8 by gemv_nk_kernel; now 7.3)
       const int tw = WARPS / p.kw, warp_tiles = (p.tiles + tw - 1) / tw, warp_steps = (p.ksteps + p.kw - 1) / p.kw;
       const double ns = warp_tiles * (warp_steps + 0.25 * (warp_steps & 1)) * (160.0 + 110.0 * mt) + p.xk * M * 0.03 + p.kw * 20.0 + (c > 1 ? 1200 : 0);
-      if (ns < best) { best = ns; busiest = warp_tiles * warp_steps; bc = c; bclusters = clusters; bsmem = off; bp = p; }
+      if (ns < best.ns) best = {p, c, clusters, warp_tiles * warp_steps, off, ns};
     }
   }
-  if (bc == 0) return Q40_E_UNSUPPORTED;
   // gemv_nk_kernel instead, where it is the faster one with weights from HBM (us here and there).  Above eight rows, where activations leave room for
   // few warps' sums, so that one has a long chain of steps: 16 rows x 7040 x 9825 45.4 and 31.9, 55 steps; 9 x 11008 x 11008 43.5 and 36.9, 43; 24 x
   // 8320 x 3197 29.7 and 28.1, 33; but 12 x 8704 x 8754 27.8 and 31.1, 34, with tiles spread evenly; 16 x 6528 x 8146 25.9 and 27.7, 26.  Up to four,
   // where CTAs have a quarter less to do on average than the busiest and scales lie so that a step's come in two loads: 1 row x 4224 x 4963 10.0
   // and 9.0, 4 rows x 10880 x 2893 14.2 and 12.3, x 6016 x 5185 12.6 and 12.1; but 1 x 1152 x 2596, 2 steps, 4.3 and 5.0.  (From L2 this
   // kernel is the faster one of most of these: 32.3 and 28.6, 30.6 and 33.4, 22.8 and 24.2 above eight rows, 8.2 and 8.6, 11.7 and 11.5, 10.2 and 10.9.)
-  const double even = (double)tiles * ksteps / (148.0 * bp.tiles * bp.ksteps);
-  if (M > 8 ? busiest >= (even < 0.9 ? 30 : 40) : M <= 4 && K % 256 != 0 && even < 0.75 && busiest >= 6) return Q40_E_UNSUPPORTED;
-  if (mt == 1) return launch<1>(bp, bc, bclusters, bsmem, (cudaStream_t)stream);
-  if (mt == 2) return launch<2>(bp, bc, bclusters, bsmem, (cudaStream_t)stream);
-  return launch<4>(bp, bc, bclusters, bsmem, (cudaStream_t)stream);
+  const double even = !best.c ? 1 : (double)tiles * ksteps / (148.0 * best.p.tiles * best.p.ksteps);
+  if (best.c && (M > 8 ? best.busiest >= (even < 0.9 ? 30 : 40) : M <= 4 && K % 256 != 0 && even < 0.75 && best.busiest >= 6)) best.c = 0;
+  return best;
+}
+
+}  // namespace nk
+}  // namespace q40
+
+// About how long q40_linear takes for 9 to 32 rows, nanoseconds (1e30: it does not take the call).  Measured, and by this: 10 rows x 1024 x 1000
+// 3.6 and 3.8 us, 16 x 2048 x 2048 4.9 and 5.3, x 4096 x 11008 13.1 and 12.9 (14.7 with weights from HBM), 20 rows 17.3 and 17.6
+double q40_linear_ns(int M, int N, int K) {
+  const q40::nk::Plan p = q40::nk::make_plan(M, N, K);
+  return p.c ? 2200 + 1.75 * p.ns : 1e30;
+}
+
+// q40_gemm_nk for up to 32 rows and groups of 64, or Q40_E_UNSUPPORTED.  Arguments are checked.
+int q40_linear(const void* x, int64_t ldx, const void* wq, const void* ws, void* y, int64_t ldy, int M, int N, int K, void* stream) {
+  using namespace q40;
+  using namespace q40::nk;
+  if (M > 32) return Q40_E_UNSUPPORTED;
+  Plan plan = make_plan(M, N, K);
+  if (plan.c == 0) return Q40_E_UNSUPPORTED;
+  Args& p = plan.p;
+  p.wide_s = K % 256 == 0 && q40_aligned(ws, 8);
+  p.wide_x = q40_aligned(x, 16) && ldx % 8 == 0;
+  p.x = (const __half*)x; p.ldx = ldx; p.w = (const uint8_t*)wq; p.s = (const __half*)ws; p.y = (__half*)y; p.ldy = ldy;
+  if (M <= 8) return launch<1>(p, plan.c, plan.clusters, plan.smem, (cudaStream_t)stream);
+  if (M <= 16) return launch<2>(p, plan.c, plan.clusters, plan.smem, (cudaStream_t)stream);
+  return launch<4>(p, plan.c, plan.clusters, plan.smem, (cudaStream_t)stream);
 }

@@ -473,7 +473,7 @@ def _tc_error_page(dev, st) -> torch.Tensor:
 
 
 def tc_error_flag(dev=None) -> int:
-    """1 if a tensor-core matmul launched through matmul_q40 or a prompt pass on the current stream of `dev` gave up
+    """1 if a tensor-core matmul launched through matmul_q40, linear_q40 or a prompt pass on the current stream of `dev` gave up
     on one of its bounded waits since the workspace was created (synchronises the device).  Not reported: matmuls
     captured on a stream on which no call that needs a workspace was made outside of a capture before."""
     dev = _indexed(dev)

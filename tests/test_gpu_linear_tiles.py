@@ -11,7 +11,11 @@ pytestmark = pytest.mark.gpu
                                    (13, 2944, 2368), (5, 2048, 2369),
                                    # what the other kernel takes, and its neighbours: long chains of steps above eight rows, uneven CTAs up to four, a remainder of 32
                                    (16, 7040, 9825), (17, 6144, 6165), (33, 6144, 6165), (1, 4224, 4963), (4, 4224, 4963), (5, 4224, 4963), (36, 4224, 4963),
-                                   (2, 1152, 2596), (1, 2048, 10711)])
+                                   (2, 1152, 2596), (1, 2048, 10711),
+                                   # pairs of CTAs: one block of k and one feature, ragged features on either CTA of a pair, odd rows of the result, k split over two to
+                                   # four pairs, more tiles than pairs, rows on both sides of 128 and of 256
+                                   (33, 128, 1), (40, 128, 129), (48, 256, 255), (100, 4096, 257), (33, 11008, 383), (64, 2048, 1000), (77, 384, 20001), (100, 4096, 11008),
+                                   (128, 640, 511), (129, 640, 640), (256, 256, 20000), (300, 1152, 1003), (513, 128, 300), (12, 8704, 8754), (9, 7040, 7001)])
 def test_against_64_bits(M, K, N):
     """What is rounded: operands fp16(code * scale), by half a step (2^-11) of each product; sums in fp32 (1e-5 of the sum of magnitudes
     covers 2^-24 per addition over K); the result, by half an fp16 step (2^-11, subnormals 2^-25)."""
@@ -28,6 +32,33 @@ def test_against_64_bits(M, K, N):
     want = xd @ w.t()
     bound = want.abs() * 2 ** -11 + 2 ** -25 + (xd.abs() @ w.abs().t()) * (1e-5 + 2 ** -11)
     assert ((y - want).abs() <= bound).all(), ((y - want).abs() / bound).max()
+    assert KK.tc_error_flag() == 0
+
+
+@pytest.mark.parametrize("M,K,N", [(40, 1024, 515), (100, 512, 20001), (64, 4096, 300)])
+def test_what_lies_around_the_result_stays_and_weights_just_written_are_read(M, K, N):
+    """Behind a launch that writes the weights, as a dependent launch of its own; the result is column ranges of wider rows."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from spec_mcts_b200 import kernels as KK
+    from spec_mcts_b200._lib import check, lib
+    g = torch.Generator(device="cuda").manual_seed(N)
+    ws = torch.zeros(lib.q40_gemm_workspace_bytes(M, N, K), dtype=torch.uint8, device="cuda")
+    x = torch.randn((M, K + 8), generator=g, device="cuda").half()[:, :K]
+    st = torch.cuda.current_stream().cuda_stream
+    q, s = torch.zeros((N * K // 128, 64), dtype=torch.int8, device="cuda"), torch.zeros(N * K // 64, dtype=torch.float16, device="cuda")
+    for first in (8, 1, 2):
+        w = (torch.randn((N, K), generator=g, device="cuda") * 0.05).half()
+        y = torch.full((M + 1, N + 11), 7.0, dtype=torch.float16, device="cuda")
+        torch.cuda.synchronize()
+        check(lib.q40_quantize(w.data_ptr(), q.data_ptr(), s.data_ptr(), N * K, 64, st))
+        check(lib.q40_gemm_nk(x.data_ptr(), x.stride(0), q.data_ptr(), s.data_ptr(), y[:, first:].data_ptr(), y.stride(0), M, N, K, 64, ws.data_ptr(), ws.numel(), st))
+        want = x.double() @ KK.dequantize_q40(q, s, 64, (N, K)).double().t()
+        got = y[:M, first:first + N].double()
+        # as above, without the operands' rounding: fp32 sums and the result's half step
+        assert ((got - want).abs() <= want.abs() * 2 ** -11 + 2 ** -25 + 1e-5 * (x.double().abs() @ KK.dequantize_q40(q, s, 64, (N, K)).double().abs().t())).all()
+        assert (y[M] == 7).all() and (y[:, :first] == 7).all() and (y[:, first + N:] == 7).all()
+        assert not ws.any()                                   # no counter, no error word
 
 
 def test_infinities_and_nan_stay_in_their_row_and_column():
