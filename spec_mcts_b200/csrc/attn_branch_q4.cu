@@ -7,7 +7,7 @@
 //   scores   A = codes of K as fp16 (16 keys x 128 dims, exact), B = the query in every column; the two scales of a key multiply the
 //            fp32 sums of its two halves
 //   output   A = V transposed (dims x 16 keys), fp16(code * scale), B = the weights: column pairs hold fp16(p) and fp16(p - fp16(p)),
-//            so that weights keep 22 bits and the sums of both columns are the row's
+//            so that weights keep 22 bits and the sums of both columns are the row's (weight_parts)
 // Dims and keys of a contraction may be in any order as long as both operands agree, so lanes take them as memory has them: lane
 // (g, t) of eight times four holds bytes 16t.. of keys g and g + 8 for the scores (a warp's load covers eight whole rows) and bytes 8g.. of
 // keys 2t, 2t + 1, 2t + 8 and 2t + 9 for the output.  All four lanes of a key end up with its score, and all four lanes t with the
@@ -30,6 +30,16 @@ constexpr int RING_BYTES = Q4_NW * STAGES * STAGE_BYTES;
 __device__ __forceinline__ int v_at(int r, int at) {
   return (r >> 1) * 128 + 32 * ((2 * (r & 1) + (at >> 5)) ^ ((r >> 1) & 3)) + (at & 31);
 }
+
+// A weight p as two fp16: fp16(p) and what that leaves.  Weights come times 2^14, so that 22 bits are kept of all above 2^-28 of a row's
+// largest, and 2^-39 of it of the others.  The first is never 0: an infinite value has to come out infinite, however small its weight
+constexpr float WEIGHT_BITS = 14.f;
+__device__ __forceinline__ uint32_t weight_parts(float p) {
+  const __half h = __hmax_nan(__float2half_rn(p), __ushort_as_half(1));
+  return h2_as_u32(__halves2half2(h, __float2half_rn(p - __half2float(h))));
+}
+// A row's sum from those over the two parts.  An infinite value is infinite in the first, and no number times a rest of 0
+__device__ __forceinline__ float both_parts(float a, float b) { return fabsf(a) <= 3.402823466e38f ? a + b : a; }
 
 template <bool ROT>
 using Q4Args = std::conditional_t<ROT, BranchRotArgs, BranchArgs>;
@@ -112,7 +122,7 @@ attn_branch_q4_kernel(const Q4Args<ROT> a) {
     }
   q72 += __shfl_xor_sync(0xffffffffu, q72, 1);
   q72 = 72.f * (q72 + __shfl_xor_sync(0xffffffffu, q72, 2));
-  float m = -CUDART_INF_F, l = 0.f;              // l: of this lane's keys
+  float m = -CUDART_INF_F, l = 0.f;              // m: WEIGHT_BITS below the largest score; l: of this lane's keys
   float acc[8][4];                               // dims 8g + 2i (columns: both parts of the weights) and 8g + 2i + 1; from 4: 64 + ..
 #pragma unroll
   for (int i = 0; i < 8; ++i)
@@ -181,7 +191,7 @@ attn_branch_q4_kernel(const Q4Args<ROT> a) {
       for (int r = 0; r < 2; ++r) {              // columns are alike: rows g and g + 8 of one
         const float2 sc = __half22float2(*reinterpret_cast<const __half2*>(st + KS_OFF + 4 * (16 * i + 8 * r + g)));
         s[i][r] = t0 + 16 * i + 8 * r + g < len ? fmaf(sc.x, ch[2 * r] - q72, sc.y * cl[2 * r]) * a.scale_log2 : -CUDART_INF_F;
-        mnew = fmaxf(mnew, s[i][r]);
+        mnew = fmaxf(mnew, s[i][r] - WEIGHT_BITS);
       }
     }
     mnew = max_g(mnew);
@@ -201,8 +211,7 @@ attn_branch_q4_kernel(const Q4Args<ROT> a) {
       for (int r = 0; r < 2; ++r) {
         const float p = ex2(s[i][r] - m);
         l += p;
-        const __half ph = __float2half_rn(p);
-        pk[r] = h2_as_u32(__halves2half2(ph, __float2half_rn(p - __half2float(ph))));
+        pk[r] = weight_parts(p);
       }
       const auto of_key = [&](const uint32_t (&v)[2], int r) { return __shfl_sync(0xffffffffu, v[r >> 1], 8 * t + 4 * (r & 1)); };
       const uint32_t sel = g & 1 ? 0x7632u : 0x5410u;                     // odd columns: the rest
@@ -240,8 +249,8 @@ attn_branch_q4_kernel(const Q4Args<ROT> a) {
   float o[16];                                   // dims 8g .. and 64 + 8g ..
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    o[2 * i] = acc[i][0] + acc[i][1];
-    o[2 * i + 1] = acc[i][2] + acc[i][3];
+    o[2 * i] = both_parts(acc[i][0], acc[i][1]);
+    o[2 * i + 1] = both_parts(acc[i][2], acc[i][3]);
   }
 
   // the token being decoded attends to its own, un-quantised K/V: one more key for a row's first warp

@@ -51,3 +51,31 @@ def test_own_keys_against_float64(B, H, Hkv, plen, cur, shift, size):
     # scores are fp32 sums over 128 dims of products up to some hundred: 2^-24 times 128 times those, as a relative error of a weight
     bound = (2 * 2 ** -11 + (2 ** -11 if plen else 0) + 1e-3 * 2 ** -4) * size_of + 2 * 2 ** -25
     assert ((got - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("H", [4, 64])                # four and two warps a row
+@pytest.mark.parametrize("code", [-1, 2])             # of the infinite value; its weight: 1, 2^-13, 2^-52 of the largest
+@pytest.mark.parametrize("lead", [0.0, 9.0, 36.0])
+def test_infinities(H, code, lead):
+    """A value of infinite scale makes its dims infinite, whatever its weight; the token's own key with a score of -inf counts for nothing."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from spec_mcts_b200._lib import check, lib
+    B, D, n = 20, 128, 40
+    q = torch.zeros(B, H, D, dtype=torch.float16, device="cuda")
+    q[..., 0] = 1
+    z = lambda *s: torch.zeros(s, dtype=torch.float16, device="cuda")
+    kq, vq = torch.zeros(B, n, H, 64, dtype=torch.int8, device="cuda"), torch.full((B, n, H, 64), 0x11, dtype=torch.int8, device="cuda")
+    ks, vs = z(B, n, H, 2), z(B, n, H, 2) + 1
+    kq[:, 7, :, 0], ks[:, 7, :, 0] = 16, lead * math.sqrt(D)             # key 7 leads
+    vq[:, 21], vs[:, 21, :, 0] = (code & 15) * 17 - (256 if code < 0 else 0), math.inf
+    pos, zero, out = torch.full((B,), n, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda"), z(B, H * D)
+    ck, cv = z(B, H, D), z(B, H * D) + 1
+    ck[..., 0] = -math.inf
+    pk, ws = z(64, H, D), torch.empty(lib.q40_attn_shared_prefix_workspace_bytes(B, H, D, 64), dtype=torch.uint8, device="cuda")
+    check(lib.q40_attn_tree_decode(q.data_ptr(), H * D, pk.data_ptr(), pk.data_ptr(), 64, zero.data_ptr(), pk.stride(0), pk.stride(1), kq.data_ptr(),
+                                   ks.data_ptr(), vq.data_ptr(), vs.data_ptr(), n, pos.data_ptr(), ck.data_ptr(), cv.data_ptr(), H * D, out.data_ptr(), B, H, H, D,
+                                   ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream))
+    out = out.view(B, H, 2, 64)
+    assert (out[:, :, 0] == math.copysign(math.inf, code)).all()
+    assert out[:, :, 1].isfinite().all()
