@@ -1,6 +1,7 @@
 // Decode attention for one query token per branch over that branch's own keys: a
 // contiguous [B,Hkv,L,D] cache or a paged pool (the packed Q4_0 cache: attn_branch_q4.cu).  Two, four or eight warps per row
-// (branch, query head), one or two rows per CTA: see launch_branch_mode.
+// (branch, query head), one or two rows per CTA: see launch_branch_mode.  Calls that several heads of a kv head, or matrix instructions,
+// make faster go to attn_branch_f16.cu, which says which.
 //
 // Eight lanes share a key: lane i owns dims 8i..8i+7 and 64+8i..64+8i+7 of the head (two 16-byte loads of K, two of
 // V, each of which covers 128 contiguous bytes over the lanes), the partial dot products are summed with three shuffles, and every group of
@@ -23,17 +24,6 @@ namespace q40 {
 //
 // A CTA has NW warps; WPR of them share a row (branch, head).  What bounds a row is latency (ids -> keys -> sums
 // -> merge), so the split is the one that keeps the warps of all rows resident at once: see launch_branch_mode.
-
-// Slot of key t of branch b: in the pool (paged), or just t (contiguous).  `row` is the branch's first page id.  (With a division
-// by the page size and 64-bit products per key, slots were a third of a paged row's instructions.)
-template <int MODE>  // 0 contiguous, 1 paged with int16 ids, 2 paged with int32 ids
-__device__ __forceinline__ int key_slot(const BranchArgs& a, const void* row, int t) {
-  if (MODE == 0) return t;
-  const int pg = a.page_shift >= 0 ? t >> a.page_shift : t / a.page_size, in = t - pg * a.page_size;
-  const int id = MODE == 1 ? (int)(uint16_t) reinterpret_cast<const int16_t*>(row)[pg] : reinterpret_cast<const int32_t*>(row)[pg];
-  // a bad page id must not turn into a wild read: clamp into the pool
-  return min(min(max(id, 0), a.last_page) * a.page_size + in, a.P - 1);
-}
 
 template <int MODE, int NW, int WPR, int U>    // U: keys per 8-lane group in flight
 __global__ void __launch_bounds__(NW * 32, U > 2 ? 16 / NW : NW == 8 ? 3 : 5)
@@ -154,7 +144,7 @@ attn_branch_kernel(const BranchArgs a) {
   else if (WPR == 1) __syncwarp();
   else asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "n"(RT) : "memory");
 
-  merge.finish(a, rows, bh, tr, lane, sm_m + g0, sm_l + g0, sm_o + g0);
+  merge.finish(a, rows, bh, tr, lane, sm_m + g0, sm_l + g0, sm_o[g0]);
 }
 
 template <int MODE, int NW, int WPR, int U>
@@ -168,7 +158,7 @@ static int launch_rows(const BranchArgs& a, cudaStream_t st) {
 // four keys, three with two keys, four of four warps with four keys, five with two.  A row's chain of iterations is its
 // time while all rows are resident: eight warps while they are, then four; then what counts is that a row's start and
 // merge occupy few warps: two, with two rows a CTA.  Microseconds, written warps / keys (2 / 4 has two rows a CTA):
-//   paged, 512 keys: 256 rows 8 / 4 10.2, 8 / 2 13.3, 4 / 4 14.7; 416 rows 8 / 2 15.2, 4 / 4 16.7, 8 / 4 18.2; 256 keys: 512 rows
+//   paged, 512 keys: 256 rows 8 / 4 10.2, 8 / 2 13.3, 4 / 4 14.7; 256 keys: 512 rows
 //     4 / 4 10.1, 4 / 2 12.3, 8 / 4 12.0; 608 rows 4 / 2 13.1, 4 / 4 14.9, 2 / 4 15.3; 1024 rows 2 / 4 17.0, 4 / 4 19.0; 3200 rows
 //     2 / 4 50, 4 / 4 53.8; of up to 64: 768 rows 2 / 4 5.8, 4 / 4 6.5, 4 / 2 7.4.  Behind a prefix: 3200 rows of up to 64
 //     2 / 4 23.2, 4 / 4 30.1, of up to 256 49.7 and 52.1
@@ -179,7 +169,6 @@ static int launch_branch_mode(const BranchArgs& a, cudaStream_t st) {
   const int64_t rows = a.rows;
   if constexpr (MODE == 1 || MODE == 2) {
     if (rows <= 2 * 148) return launch_rows<MODE, 8, 8, 4>(a, st);
-    if (rows <= 3 * 148) return launch_rows<MODE, 8, 8, 2>(a, st);
     if (rows > 5 * 148 || (rows > 4 * 148 && a.L <= 128)) return launch_rows<MODE, 4, 2, 4>(a, st);
     if (rows > 4 * 148) return launch_rows<MODE, 4, 4, 2>(a, st);
   } else {
@@ -200,6 +189,7 @@ static void fill_derived(BranchArgs& a, int B) {
 
 int launch_branch(BranchArgs a, int mode, int B, cudaStream_t st) {
   fill_derived(a, B);
+  if (int rc; launch_branch_f16(a, mode, st, rc)) return rc;
   if (mode == 0) return launch_branch_mode<0>(a, st);
   if (mode == 1) return launch_branch_mode<1>(a, st);
   return launch_branch_mode<2>(a, st);

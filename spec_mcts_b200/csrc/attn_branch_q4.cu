@@ -31,16 +31,6 @@ __device__ __forceinline__ int v_at(int r, int at) {
   return (r >> 1) * 128 + 32 * ((2 * (r & 1) + (at >> 5)) ^ ((r >> 1) & 3)) + (at & 31);
 }
 
-// A weight p as two fp16: fp16(p) and what that leaves.  Weights come times 2^14, so that 22 bits are kept of all above 2^-28 of a row's
-// largest, and 2^-39 of it of the others.  The first is never 0: an infinite value has to come out infinite, however small its weight
-constexpr float WEIGHT_BITS = 14.f;
-__device__ __forceinline__ uint32_t weight_parts(float p) {
-  const __half h = __hmax_nan(__float2half_rn(p), __ushort_as_half(1));
-  return h2_as_u32(__halves2half2(h, __float2half_rn(p - __half2float(h))));
-}
-// A row's sum from those over the two parts.  An infinite value is infinite in the first, and no number times a rest of 0
-__device__ __forceinline__ float both_parts(float a, float b) { return fabsf(a) <= 3.402823466e38f ? a + b : a; }
-
 template <bool ROT>
 using Q4Args = std::conditional_t<ROT, BranchRotArgs, BranchArgs>;
 
@@ -303,7 +293,7 @@ attn_branch_q4_kernel(const Q4Args<ROT> a) {
   if (WPR == 1) __syncwarp();
   else if (WPR == Q4_NW) __syncthreads();
   else asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "n"(RT) : "memory");
-  merge.finish(a, rows, bh, part * 32 + lane, lane, sm_m + slot * WPR, sm_l + slot * WPR, sm_o + slot * WPR);
+  merge.finish(a, rows, bh, part * 32 + lane, lane, sm_m + slot * WPR, sm_l + slot * WPR, sm_o[slot * WPR]);
 }
 
 template <bool ROT, int WPR, bool SC4>

@@ -67,6 +67,27 @@ struct BranchRotArgs : BranchArgs {
   int n_pos;
 };
 
+// A weight p as two fp16: fp16(p) and what that leaves.  Weights come times 2^14, so that 22 bits are kept of all above 2^-28 of a row's
+// largest, and 2^-39 of it of the others.  The first is never 0: an infinite value has to come out infinite, however small its weight
+constexpr float WEIGHT_BITS = 14.f;
+__device__ __forceinline__ uint32_t weight_parts(float p) {
+  const __half h = __hmax_nan(__float2half_rn(p), __ushort_as_half(1));
+  return h2_as_u32(__halves2half2(h, __float2half_rn(p - __half2float(h))));
+}
+// A row's sum from those over the two parts.  An infinite value is infinite in the first, and no number times a rest of 0
+__device__ __forceinline__ float both_parts(float a, float b) { return fabsf(a) <= 3.402823466e38f ? a + b : a; }
+
+// Slot of key t of branch b: in the pool (paged), or just t (contiguous).  `row` is the branch's first page id.  (With a division
+// by the page size and 64-bit products per key, slots were a third of a paged row's instructions.)
+template <int MODE>  // 0 contiguous, 1 paged with int16 ids, 2 paged with int32 ids
+__device__ __forceinline__ int key_slot(const BranchArgs& a, const void* row, int t) {
+  if (MODE == 0) return t;
+  const int pg = a.page_shift >= 0 ? t >> a.page_shift : t / a.page_size, in = t - pg * a.page_size;
+  const int id = MODE == 1 ? (int)(uint16_t) reinterpret_cast<const int16_t*>(row)[pg] : reinterpret_cast<const int32_t*>(row)[pg];
+  // a bad page id must not turn into a wild read: clamp into the pool
+  return min(min(max(id, 0), a.last_page) * a.page_size + in, a.P - 1);
+}
+
 // The end of a row (branch, head) of RT threads: its own keys' partial results, NG of them in shared memory, and those of a prefix pass
 // become the output.  Thread tr owns output dims tr, tr + RT, ... (RT above the head's 128: the first four warps)
 template <int NG, int RT>
@@ -86,8 +107,9 @@ struct RowMerge {
           po[i][j] = i < a.nsp && (RT <= ATTN_D || tr < ATTN_D) ? a.po[((int64_t)i * rows + bh) * ATTN_D + tr + j * RT] : 0.f;
     }
   }
+  template <int STRIDE = ATTN_D>                // floats between the outputs of two
   __device__ __forceinline__ void finish(const BranchArgs& a, int64_t rows, int64_t bh, int tr, int lane, const float* sm_m, const float* sm_l,
-                                         const float (*sm_o)[ATTN_D]) {
+                                         const float* sm_o) {
     if (RT > ATTN_D && tr >= ATTN_D) return;
     float M = -CUDART_INF_F;
 #pragma unroll
@@ -103,7 +125,7 @@ struct RowMerge {
         const float w = ex2(sm_m[g] - M);         // exp2(-inf) = 0 for empty groups
         Lsum = fmaf(sm_l[g], w, Lsum);
 #pragma unroll
-        for (int j = 0; j < DP; ++j) acc[j] = fmaf(sm_o[g][tr + j * RT], w, acc[j]);
+        for (int j = 0; j < DP; ++j) acc[j] = fmaf(sm_o[g * STRIDE + tr + j * RT], w, acc[j]);
       }
       if (a.nsp > 0) {
         const float pw_l = ex2(pm_l - M);
@@ -138,6 +160,8 @@ struct RowMerge {
 int launch_branch_q4(const BranchRotArgs& a, bool rotate, cudaStream_t st);
 // defined in attn_branch.cu; mode 0 contiguous, 1 paged/int16 ids, 2 paged/int32 ids
 int launch_branch(BranchArgs a, int mode, int B, cudaStream_t st);
+// defined in attn_branch_f16.cu; false, and nothing launched, where attn_branch_kernel is faster
+bool launch_branch_f16(const BranchArgs& a, int mode, cudaStream_t st, int& rc);
 int launch_branch_q4(BranchRotArgs a, int B, cudaStream_t st);         // the Q4_0 cache, with rotation where there are tables
 
 }  // namespace q40
