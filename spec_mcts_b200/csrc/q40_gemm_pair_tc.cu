@@ -17,7 +17,8 @@
 //                 and write fp16(code * scale), the reference's operand value (triton_kernels.py:444-445), to
 //                 tensor memory (see q40_gemm_tiled_tc.cu)
 //   warps 20..23  accumulators -> output
-// The pair's last tile is finished by the dequantiser warps as well.
+// The pair's last tile is finished by the dequantiser warps as well.  Where it is the only one, warps 20..23 are a fifth set; where finishing
+// is what a pair waits for, warps 16..19 finish too (see layout).
 //
 // A tile whose k range is cut between pairs: all but the last leave their fp32 sums in a scratch slot (first thing,
 // each has one at most) and raise flags; the pair with the last k blocks does them last and adds the slots in order.  A
@@ -1044,7 +1045,7 @@ int q40_pair_gemm(int nmat, const void* a, int64_t lda, const void* const* bw_ti
 // Y[M, N] = X[M, K] @ deq(W)^T for W [N, K] with groups of 64 along K: see q40_gemm_nk, whose arguments are checked.  K % 128 == 0; x on 16-byte
 // boundaries, rows too.  Weights may be what the launch in front writes: they are requested behind the wait for it
 int q40_pair_linear(const void* x, int64_t ldx, const void* wq, const void* ws, void* y, int64_t ldy, int M, int N, int K, double beat_ns,
-                    int* err, void* stream) {
+                    void* staged, int* err, void* stream) {
   using namespace q40;
   using namespace q40::ttc;
   pair::Params p{};
@@ -1055,7 +1056,11 @@ int q40_pair_linear(const void* x, int64_t ldx, const void* wq, const void* ws, 
   p.nk_s = (const __half*)ws; p.n_cols = N;
   p.k64 = K / BK;
   pair::k_blocks(p, p.k64);
-  return pair_run(p, true, p.spans[0], x, ldx, nullptr, 0, beat_ns, 1, stream, [&](EncodeTiledFn encode, pair::Maps& maps) {
+  return pair_run(p, true, p.spans[0], staged ? staged : x, staged ? K : ldx, nullptr, 0, beat_ns, 1, stream, [&](EncodeTiledFn encode, pair::Maps& maps) {
+    if (staged && cudaMemcpy2DAsync(staged, (size_t)K * 2, x, (size_t)ldx * 2, (size_t)K * 2, M, cudaMemcpyDeviceToDevice, (cudaStream_t)stream) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return false;
+    }
     const cuuint64_t dim[2] = {(cuuint64_t)K / 2, (cuuint64_t)N}, pitch[1] = {(cuuint64_t)K / 2};
     const cuuint32_t box[2] = {64, pair::FEATS}, estr[2] = {1, 1};
     return encode(&maps.w[0], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)wq, dim, pitch, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,

@@ -1,5 +1,5 @@
 // y[M, N] = x[M, K] @ deq(W)^T for W [N, K] with groups of 64 along K (the layout of quantize_q40 on a Linear weight), up to 32 rows a
-// launch.
+// launch (from 9 on where q40_pair_linear, on tcgen05, is not the faster one: see q40_gemm_nk).
 //
 // One CTA per SM: up to five 16-row tiles of W over the whole k range, or, where the activations do not fit shared memory or
 // tiles are few, a cluster of two or four CTAs that share it.  The activations are staged once, W comes straight into the
@@ -8,9 +8,9 @@
 //
 // What bounds it: instructions of the expansion (about 230 a warp and 128 k of 16 rows, of which 100 make operands) and a warp's chain
 // of loads, four of 1 KB on their way.  Microseconds of the launch alone with W in L2, here and by gemv_nk_kernel (64 rows x part of k per CTA,
-// scratch and tickets): 10 rows x 4096 x 11008 13.7 and 18.2 (calls of linear_q40 one after the other: 14.3 and 18.4), x 11008 x 4096 17.8 and 18.7; 1 row x 4096 x 4096 5.8 and 7.6, x 11008 x 11008
-// 24.0 and 27.7; 10 rows x 1024 x 1000 4.0 and 7.0; 20 rows x 4096 x 11008 20.1 and 29.3.  No gain: weights prefetched to L2 at the
-// start (14.2).
+// scratch and tickets): 10 rows x 4096 x 11008 13.7 and 18.2 (calls of linear_q40 one after the other: 12.0, without programmatic launch
+// 14.3, and 18.4), x 11008 x 4096 17.8 and 18.7; 1 row x 4096 x 4096 5.8 and 7.6, x 11008 x 11008 24.0 and 27.7; 10 rows x 1024 x 1000 4.0 and
+// 7.0; 20 rows x 4096 x 11008 20.1 and 29.3.  No gain: weights prefetched to L2 at the start (14.2).
 #include <cooperative_groups.h>
 
 #include <algorithm>

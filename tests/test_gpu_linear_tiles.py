@@ -78,3 +78,30 @@ def test_infinities_and_nan_stay_in_their_row_and_column():
     assert torch.isnan(y[2]).all() and (y[1, clean] == float("inf")).all() and y[1, 3] == -float("inf")
     rows = [m for m in range(10) if m not in (1, 2)]
     assert (y[rows, 7] == float("inf")).all() and torch.isfinite(y[rows][:, clean]).all()
+
+
+@pytest.mark.parametrize("M,K,N", [(33, 256, 300), (100, 1152, 2050)])
+def test_rows_off_16_bytes_have_the_same_bits_captured_too(M, K, N):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from spec_mcts_b200 import kernels as KK
+    from spec_mcts_b200._lib import check, lib
+    g = torch.Generator(device="cuda").manual_seed(M)
+    q, s = KK.quantize_q40((torch.randn((N, K), generator=g, device="cuda") * 0.05).half())
+    x = torch.randn((M, K), generator=g, device="cuda").half()
+    off = torch.zeros(4 + M * (K + 4), dtype=torch.float16, device="cuda")[4:].view(M, K + 4)[:, :K].copy_(x)
+    ws = torch.zeros(max(lib.q40_gemm_workspace_bytes(M, N, K), 4096 + 2 * M * K), dtype=torch.uint8, device="cuda")
+
+    def call(x, y):
+        check(lib.q40_gemm_nk(x.data_ptr(), x.stride(0), q.data_ptr(), s.data_ptr(), y.data_ptr(), N, M, N, K, 64, ws.data_ptr(), ws.numel(),
+                              torch.cuda.current_stream().cuda_stream))
+        return y
+    y = [torch.zeros((M, N), dtype=torch.float16, device="cuda") for _ in range(3)]
+    call(x, y[0])
+    call(off, y[1])
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call(off, y[2])
+    graph.replay()
+    assert torch.equal(y[0], y[1]) and torch.equal(y[0], y[2])
