@@ -195,9 +195,11 @@ struct F16Form { int heads, warps, stages; };
 static F16Form f16_form(const BranchArgs& a, int mode) {
   constexpr int64_t SMS = 148;
   const bool prefix = a.beside_prefix;
-  const int rep = a.H / a.Hkv, L = a.L;
+  // Keys of a branch: with lengths (on the device) a.L only bounds them, and what is between does not change the result, so it must not change the
+  // form, whose sums have an order of their own.  The pool's share of a branch instead
+  const int rep = a.H / a.Hkv, L = a.seq_lens ? (int)(a.P / (a.rows / a.H)) : a.L;
   // As many heads as leave rows for the SMs.  Us by heads (of 4 a kv head) at their best number of warps: paged, 300 keys, 96 rows of one head
-  // 5.13 / 5.48 / 6.51 with 1 / 2 / 4, 224 rows 7.2 / 5.49 / 6.57, 384 rows 8.5 / 7.6 / 6.9; 20 keys, 640 rows 3.8 / 3.8 / 4.5; 40 keys behind
+  // 5.13 / 5.48 / 6.51 with 1 / 2 / 4, 224 rows 7.2 / 5.49 / 6.57, 384 rows 8.5 / 7.6 / 6.9; 20 keys, 640 rows 3.8 / 3.8 / 4.5 (contiguous 3.5 / 3.4 / 3.8, attn_branch_kernel 3.1); 40 keys behind
   // 400, 640 rows 8.2 / 7.6 / 8.6, 1600 rows 12.7 / 10.9 / 11.2
   const int64_t enough = L <= 64 ? (prefix ? 300 : 200) : prefix ? SMS : SMS / 2;
   const int heads = rep % 4 == 0 && a.rows / 4 > enough ? 4 : rep % 2 == 0 && a.rows / 2 > enough ? 2 : 1;
@@ -206,6 +208,7 @@ static F16Form f16_form(const BranchArgs& a, int mode) {
   // 160 rows 27.7 / 15.4 / 11.4 (three stages 11.0) / 14.0 (19.1); 100 keys, 320 rows 10.1 / 7.5 / 6.2 / 12.0 (11.0), 800 rows 11.5 / 8.6 / 10.9 / 23.6
   // (18.8); contiguous, 300 keys, 800 rows 23.2 / 21.8 / 23.7 / 35.2 (42.4); 40 keys behind 400, 448 rows 10.3 / 8.2 / 11.3 / 17.1 (10.1)
   if (heads > 1) {
+    if (mode == 0 && L < 32 && a.rows <= 8 * SMS) return {0, 0, 0};
     if (prefix && L <= 64) return {heads, 2, 2};
     if (rows <= SMS && !prefix) return {heads, 8, 2};
     if (rows <= 2 * SMS) return {heads, 4, 3};
@@ -213,10 +216,10 @@ static F16Form f16_form(const BranchArgs& a, int mode) {
     return {heads, rows <= 8 * SMS || prefix ? 2 : 1, 2};
   }
   // One, beside the prefix pass.  Us of attn_branch_kernel and here: 320 rows of up to 130 9.5, 8.6, of 40 8.2, 7.6; 480 of 250 11.6, 12.3;
-  // 160 of 236 9.9, 10.6; 832 of 300 18.9, 16.2; 2048 of 138 17.0, 18.6, of 256 behind 2048 37.4, 36.5, 3200 of 250 37.9, 36.1
+  // 160 of 161 9.2, 9.5, 192 of 142 7.5, 7.1; 832 of 300 18.9, 16.2; 2048 of 138 17.0, 18.6, of 256 behind 2048 37.4, 36.5, 3200 of 250 37.9, 36.1
   if (prefix) {
     if (rep > 1 && L <= 64 && rows > SMS && rows <= 3 * SMS) return {1, 2, 2};
-    if (rows <= 2 * SMS) return {rows <= SMS || L <= 200, 4, 3};
+    if (rows <= 2 * SMS) return {rows <= SMS || L <= 150, 4, 3};
     if (rows <= 3 * SMS) return {1, 4, 2};
     return {rows > 5 * SMS && L > 240, 2, 2};
   }
