@@ -13,8 +13,8 @@
 // cat(prompt.expand(B), suffix) for SDPA (hf_model_q40_kv_shared.py:375-376, 405).
 //
 // Algorithmic traffic: prefix K/V once per (kv head, row block); Q and the partials are
-// small next to it.  What bounds it: a warp's chain of MMAs and softmax per tile (2.1 us; see attn_tile.cuh), start, first
-// tile and partials around it.
+// small next to it.  What bounds it: a warp's chain of MMAs and softmax per tile (2.1 us, a quarter where four warps share it; see
+// attn_tile.cuh), start, first tile and partials around it.
 #include <climits>
 
 #include "attn_tile.cuh"
@@ -39,12 +39,12 @@ struct PrefixArgs {
   int n_pos;
 };
 
-// grid: (nsp, Hkv, row blocks); block: NWARPS*32 threads, 16 query rows per warp.
-template <int NWARPS, bool ROT>
+// grid: (nsp, Hkv, row blocks); block: NWARPS*32 threads, 16 query rows per KW warps, which share the keys of a tile.
+template <int NWARPS, int KW, bool ROT>
 __global__ void __launch_bounds__(NWARPS * 32)
 attn_prefix_kernel(const PrefixArgs a) {
   constexpr int D = ATTN_D;
-  constexpr int RB = NWARPS * 16;
+  constexpr int RB = NWARPS / KW * 16, KEYS = TILE_KEYS / KW;
   constexpr int NT = NWARPS * 32;
   extern __shared__ __align__(128) unsigned char smem[];
   // [Q rows][stage][K tile | V tile]
@@ -105,20 +105,21 @@ attn_prefix_kernel(const PrefixArgs a) {
   __syncthreads();
   WarpRows w;
   w.init();
-  w.load_q(sbase, warp * 16, lane);
+  const int wrow = warp / KW * 16, kfirst = warp % KW * KEYS;   // of this warp
+  w.load_q(sbase, wrow, lane);
 
-  const bool any_row = row0 + warp * 16 < rows;      // a warp without rows only helps to load
+  const bool any_row = row0 + wrow < rows;      // a warp without rows only helps to load
   for (int tile = 0; tile < ntiles; ++tile) {
     const int stage = tile & 1;
     if (tile + 1 < ntiles) load(tile + 1, stage ^ 1);
     cp_async_commit();
     cp_async_wait<1>();   // the tile for this iteration has landed
     __syncthreads();
-    const uint32_t kt = stages + stage * 2 * TILE_BYTES, vt = kt + TILE_BYTES;
-    const int n = k_end - k_begin - tile * TILE_KEYS;          // every tile holds at least one key
-    if (any_row) {
-      if (n >= TILE_KEYS) w.step<false>(kt, vt, a.scale_log2, 0, 0, lane);
-      else w.step<true>(kt, vt, a.scale_log2, n, n, lane);
+    const uint32_t kt = stages + stage * 2 * TILE_BYTES + kfirst * TILE_ROW_BYTES, vt = kt + TILE_BYTES;
+    const int n = k_end - k_begin - tile * TILE_KEYS - kfirst;
+    if (any_row && n > 0) {
+      if (n >= KEYS) w.template step<false, KEYS>(kt, vt, a.scale_log2, 0, 0, lane);
+      else w.template step<true, KEYS>(kt, vt, a.scale_log2, n, n, lane);
     }
     __syncthreads();  // all warps are done with this stage before it is refilled
   }
@@ -127,17 +128,57 @@ attn_prefix_kernel(const PrefixArgs a) {
   // ---- write the partial (m, l, O) of rows g and g+8 ----
   w.finish();
   const int64_t total_rows = (int64_t)a.B * a.H;
+  if constexpr (KW > 1) {
+    // the warps of a row meet in the tiles' memory; eight threads a row, 16 dims each
+    constexpr int LD = D + 4;
+    float *so = reinterpret_cast<float*>(smem), *sm = so + KW * RB * LD, *sl = sm + KW * RB;
+    __syncthreads();                                  // (no tile: the queries are still being read)
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    const int gr = row0 + warp * 16 + g + r * 8;
-    if (gr >= rows) continue;
-    const int b = gr / rep, j = gr % rep;
-    const int64_t ridx = (int64_t)sp * total_rows + (int64_t)b * a.H + hk * rep + j;
-    if (t == 0) { a.pm[ridx] = w.m[r]; a.pl[ridx] = w.l[r]; }
-    float* dst = a.po + ridx * D;
+    for (int r = 0; r < 2; ++r) {
+      const int at = warp % KW * RB + wrow + g + r * 8;
+      if (t == 0) { sm[at] = w.m[r]; sl[at] = w.l[r]; }
 #pragma unroll
-    for (int dt = 0; dt < 16; ++dt)
-      *reinterpret_cast<float2*>(dst + dt * 8 + 2 * t) = make_float2(w.o[dt][2 * r], w.o[dt][2 * r + 1]);
+      for (int dt = 0; dt < 16; ++dt) *reinterpret_cast<float2*>(so + at * LD + dt * 8 + 2 * t) = make_float2(w.o[dt][2 * r], w.o[dt][2 * r + 1]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < RB * 8 / NT; ++i) {
+      const int r = (tid + i * NT) >> 3, part = tid & 7, gr = row0 + r;
+      if (gr >= rows) continue;
+      float M = -CUDART_INF_F, l = 0.f, f[KW];
+#pragma unroll
+      for (int k = 0; k < KW; ++k) M = fmaxf(M, sm[k * RB + r]);
+#pragma unroll
+      for (int k = 0; k < KW; ++k) {                  // no finite score: sums and outputs are 0
+        f[k] = M > -CUDART_INF_F ? ex2(sm[k * RB + r] - M) : 1.f;
+        l = fmaf(sl[k * RB + r], f[k], l);
+      }
+      const int64_t ridx = (int64_t)sp * total_rows + (int64_t)(gr / rep) * a.H + hk * rep + gr % rep;
+      if (part == 0) { a.pm[ridx] = M; a.pl[ridx] = l; }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < KW; ++k) {
+          const float4 x = *reinterpret_cast<const float4*>(so + (k * RB + r) * LD + 32 * c + 4 * part);
+          v.x = fmaf(x.x, f[k], v.x); v.y = fmaf(x.y, f[k], v.y); v.z = fmaf(x.z, f[k], v.z); v.w = fmaf(x.w, f[k], v.w);
+        }
+        *reinterpret_cast<float4*>(a.po + ridx * D + 32 * c + 4 * part) = v;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int gr = row0 + wrow + g + r * 8;
+      if (gr >= rows) continue;
+      const int b = gr / rep, j = gr % rep;
+      const int64_t ridx = (int64_t)sp * total_rows + (int64_t)b * a.H + hk * rep + j;
+      if (t == 0) { a.pm[ridx] = w.m[r]; a.pl[ridx] = w.l[r]; }
+      float* dst = a.po + ridx * D;
+#pragma unroll
+      for (int dt = 0; dt < 16; ++dt)
+        *reinterpret_cast<float2*>(dst + dt * 8 + 2 * t) = make_float2(w.o[dt][2 * r], w.o[dt][2 * r + 1]);
+    }
   }
 }
 
@@ -178,15 +219,26 @@ static int launch_prefix(PrefixArgs& pa, int nsp, cudaStream_t st) {
   const int tiles = (pa.prefix_len + TILE_KEYS - 1) / TILE_KEYS;
   pa.keys_per_split = ((tiles + nsp - 1) / nsp) * TILE_KEYS;
   const int rep = pa.H / pa.Hkv, rows = pa.B * rep;
-  const auto smem = [](int warps) { return (size_t)warps * 16 * TILE_ROW_BYTES + 4 * TILE_BYTES; };      // the Q rows, two stages of K and V
-  const auto launch = [&](std::atomic<uint64_t>& ready, auto kern, int warps) {
-    const cudaError_t e = q40_allow_smem(ready, (const void*)kern, (int)smem(warps));
-    return e != cudaSuccess ? e : q40_launch_pdl(kern, dim3(nsp, pa.Hkv, (rows + warps * 16 - 1) / (warps * 16)), dim3(warps * 32), smem(warps), st, pa);
+  const auto launch = [&](std::atomic<uint64_t>& ready, auto kern, int warps, int kw) {
+    const int rb = warps / kw * 16;
+    // the Q rows, two stages of K and V; as much with shared tiles, so that no three CTAs crowd on an SM (20 branches, 200 own
+    // keys: 19.3 us, 17.7 so)
+    const size_t smem = (size_t)warps * 16 * TILE_ROW_BYTES + 4 * TILE_BYTES;
+    const cudaError_t e = q40_allow_smem(ready, (const void*)kern, (int)smem);
+    return e != cudaSuccess ? e : q40_launch_pdl(kern, dim3(nsp, pa.Hkv, (rows + rb - 1) / rb), dim3(warps * 32), smem, st, pa);
   };
-  static std::atomic<uint64_t> ready[4];
+  static std::atomic<uint64_t> ready[8];
+  const bool rot = pa.cos_tbl != nullptr;
   cudaError_t e;
-  if (rows <= 64) e = pa.cos_tbl ? launch(ready[0], attn_prefix_kernel<4, true>, 4) : launch(ready[1], attn_prefix_kernel<4, false>, 4);
-  else e = pa.cos_tbl ? launch(ready[2], attn_prefix_kernel<8, true>, 8) : launch(ready[3], attn_prefix_kernel<8, false>, 8);
+  // Warps that would have no rows take a part of each tile's keys: up to 16 rows all four, up to 32 two a row where splits have more than one tile
+  // (half of one tile is what the merge of the warps takes again).  The same with and without rotation, whose results are the same bits.  Us with one
+  // warp a row and so, with the branch pass: 10 branches behind 2048 keys 11.6 and 9.9, 2 behind 70 5.1 and 4.5; rotating, 5 behind 512 8.9 and 8.5, 10
+  // 9.6 and 9.1, 16 10.6 and 9.9; 17 behind 2048 13.7 and 11.6, behind 600 9.1 and 8.4; but rotating, 20 behind 512 (eight splits) 11.3 and 11.6
+  if (rows <= 16) e = rot ? launch(ready[0], attn_prefix_kernel<4, 4, true>, 4, 4) : launch(ready[1], attn_prefix_kernel<4, 4, false>, 4, 4);
+  else if (rows <= 32 && pa.keys_per_split > TILE_KEYS)
+    e = rot ? launch(ready[2], attn_prefix_kernel<4, 2, true>, 4, 2) : launch(ready[3], attn_prefix_kernel<4, 2, false>, 4, 2);
+  else if (rows <= 64) e = rot ? launch(ready[4], attn_prefix_kernel<4, 1, true>, 4, 1) : launch(ready[5], attn_prefix_kernel<4, 1, false>, 4, 1);
+  else e = rot ? launch(ready[6], attn_prefix_kernel<8, 1, true>, 8, 1) : launch(ready[7], attn_prefix_kernel<8, 1, false>, 8, 1);
   if (e != cudaSuccess) return (int)e;
   return Q40_OK;
 }

@@ -87,32 +87,33 @@ struct WarpRows {
     for (int ks = 0; ks < 8; ++ks) ldsm_x4(tile + tile_off(row, 2 * ks + (mi >> 1)), qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3]);
   }
 
-  // One tile: S = Q K^T, online softmax, O += P V.  With MASK, key i of the tile counts for row g below n0 and for row g + 8
+  // KEYS keys of a tile: S = Q K^T, online softmax, O += P V.  With MASK, key i of the tile counts for row g below n0 and for row g + 8
   // below n1.  A row all of whose scores so far are -inf keeps its sum and outputs at zero.
-  template <bool MASK>
+  template <bool MASK, int KEYS = TILE_KEYS>
   __device__ __forceinline__ void step(uint32_t kt, uint32_t vt, float scale_log2, int n0, int n1, int lane) {
     const int t = lane & 3;
-    float s[8][4];
+    constexpr int NT = KEYS / 8;
+    float s[NT][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < NT; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
 #pragma unroll
     for (int ks = 0; ks < 8; ks += 2) {
       // eight sums in turn: one after the other, each MMA would wait for the one before it
-      uint32_t kb[8][4];
+      uint32_t kb[NT][4];
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt)
+      for (int nt = 0; nt < NT; ++nt)
         ldsm_x4(kt + tile_off(nt * 8 + (lane & 7), 2 * ks + (lane >> 3)), kb[nt][0], kb[nt][1], kb[nt][2], kb[nt][3]);
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt) mma_f16(s[nt], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], kb[nt][0], kb[nt][1]);
+      for (int nt = 0; nt < NT; ++nt) mma_f16(s[nt], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], kb[nt][0], kb[nt][1]);
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt)
+      for (int nt = 0; nt < NT; ++nt)
         mma_f16(s[nt], qa[ks + 1][0], qa[ks + 1][1], qa[ks + 1][2], qa[ks + 1][3], kb[nt][2], kb[nt][3]);
     }
     float mx[2] = {-CUDART_INF_F, -CUDART_INF_F};
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
+    for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         s[nt][j] *= scale_log2;
@@ -131,7 +132,7 @@ struct WarpRows {
     }
     float ls[2] = {0.f, 0.f};
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
+    for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float p = ex2(s[nt][j] - m[j >> 1]);
@@ -148,7 +149,7 @@ struct WarpRows {
       }
     }
 #pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
+    for (int kk = 0; kk < KEYS / 16; ++kk) {
       const uint32_t a0 = pack_h2(s[2 * kk][0], s[2 * kk][1]);
       const uint32_t a1 = pack_h2(s[2 * kk][2], s[2 * kk][3]);
       const uint32_t a2 = pack_h2(s[2 * kk + 1][0], s[2 * kk + 1][1]);

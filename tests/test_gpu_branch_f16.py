@@ -71,7 +71,9 @@ def test_own_keys_against_float64(B, H, Hkv, L, page, ids):
 
 
 @pytest.mark.parametrize("B,H,Hkv,L,plen", [(29, 32, 8, 64, 70), (20, 32, 8, 129, 300), (29, 32, 8, 160, 513), (58, 32, 8, 97, 64), (13, 32, 8, 33, 1), (13, 32, 16, 160, 130),
-                                            (4, 32, 32, 257, 70), (29, 6, 6, 160, 64), (29, 12, 12, 257, 600), (29, 28, 28, 256, 200), (29, 32, 32, 257, 128)])
+                                            (4, 32, 32, 257, 70), (29, 6, 6, 160, 64), (29, 12, 12, 257, 600), (29, 28, 28, 256, 200), (29, 32, 32, 257, 128),
+                                            # up to 16 and up to 32 rows a kv head, whose warps share a tile's keys: 1, 15 to 17, 63 to 65 keys, none in the last part
+                                            (1, 4, 4, 33, 1), (2, 32, 4, 33, 15), (16, 4, 4, 33, 16), (5, 12, 4, 33, 17), (17, 4, 4, 33, 63), (4, 32, 4, 33, 65), (8, 16, 4, 33, 33), (16, 4, 4, 33, 600), (32, 4, 4, 33, 1100), (33, 4, 4, 33, 65)])
 def test_behind_a_prompt_against_float64(B, H, Hkv, L, plen):
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
