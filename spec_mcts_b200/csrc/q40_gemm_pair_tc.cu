@@ -984,7 +984,7 @@ static int pair_run(q40::ttc::pair::Params& p, bool nk, int spans, const void* a
   const cuuint64_t gstride[1] = {(cuuint64_t)lda * 2};
   const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)p.npad / 2};
   const cuuint32_t estr[2] = {1, 1};
-  if (encode(&maps.act, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)a, gdim, gstride, box, estr,
+  if (ttc_encode(encode, &maps.act, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)a, gdim, gstride, box, estr,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return Q40_E_UNSUPPORTED;
@@ -1033,7 +1033,7 @@ int q40_pair_gemm(int nmat, const void* a, int64_t lda, const void* const* bw_ti
       const cuuint64_t wstride[1] = {STEP_BYTES};
       const cuuint32_t wbox[2] = {silu ? 128u : 256u, 4 * pair::BLK}, sbox[2] = {silu ? 8u : 16u, 4 * pair::BLK};
       for (int j = 0; j < 2; ++j)
-        if (encode(j ? &maps.s[i] : &maps.w[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, (void*)bw_tiled[i], wdim, wstride, j ? sbox : wbox,
+        if (ttc_encode(encode, j ? &maps.s[i] : &maps.w[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, (void*)bw_tiled[i], wdim, wstride, j ? sbox : wbox,
                    estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
           return false;
@@ -1063,7 +1063,7 @@ int q40_pair_linear(const void* x, int64_t ldx, const void* wq, const void* ws, 
     }
     const cuuint64_t dim[2] = {(cuuint64_t)K / 2, (cuuint64_t)N}, pitch[1] = {(cuuint64_t)K / 2};
     const cuuint32_t box[2] = {64, pair::FEATS}, estr[2] = {1, 1};
-    return encode(&maps.w[0], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)wq, dim, pitch, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    return ttc_encode(encode, &maps.w[0], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)wq, dim, pitch, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   });
 }

@@ -385,7 +385,7 @@ static int tiled_tc(int nmat, const void* a, int64_t lda, const void* const* bw_
   const cuuint64_t gstride[1] = {(cuuint64_t)lda * 2};
   const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)p.Mpad};
   const cuuint32_t estr[2] = {1, 1};
-  if (encode(&amap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)a, gdim, gstride, box, estr,
+  if (ttc_encode(encode, &amap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)a, gdim, gstride, box, estr,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return Q40_E_UNSUPPORTED;

@@ -146,6 +146,15 @@ static inline EncodeTiledFn ttc_encode_fn() {
   cached.store(fn, std::memory_order_release);
   return (EncodeTiledFn)fn;
 }
+// A call of it.  The driver wants the device's context current in the calling thread, which a thread that has made no call of the runtime so far
+// does not have (all that a launch asks of the runtime before may be known already)
+template <typename... Args>
+static CUresult ttc_encode(EncodeTiledFn fn, Args... args) {
+  const CUresult r = fn(args...);
+  int dev = 0;
+  if (r == CUDA_SUCCESS || cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return r;
+  return fn(args...);
+}
 
 // q40_gemm_pair_tc.cu: C_i[M, N_i] = A[M, K] @ deq(B_i) on tiled copies by pairs of CTAs, or, with `silu` and two matrices, c[0] =
 // silu(A @ deq(B_0)) * (A @ deq(B_1)).  M <= 128: any order of the sums over k; above: the sums of `ranges` equal k

@@ -132,3 +132,17 @@ def test_without_the_extension(K, monkeypatch):
     c, y = K.matmul_q40(a, q, s, shape), K.linear_q40(a, q, s, (512, 256))
     monkeypatch.setattr(K, "_host_calls", None)
     assert torch.equal(K.matmul_q40(a, q, s, shape), c) and torch.equal(K.linear_q40(a, q, s, (512, 256)), y)
+
+
+@pytest.mark.parametrize("op,M", [("matmul_q40", 1), ("matmul_q40", 9), ("matmul_q40", 40), ("matmul_q40", 130), ("linear_q40", 1), ("linear_q40", 40), ("linear_q40", 300)])
+def test_the_first_call_of_a_thread_is_like_any_other(K, op, M):
+    """A thread that has made no call of the CUDA runtime gets the bits, and so the route, of the others."""
+    import threading
+    a, q, s, shape = data(K, M, 4096, 4096)
+    for _ in range(2):                                        # the copy is made, the output's memory is there
+        want = getattr(K, op)(a, q, s, shape)
+    got = []
+    t = threading.Thread(target=lambda: got.append(getattr(K, op)(a, q, s, shape)))
+    t.start()
+    t.join()
+    assert got and torch.equal(got[0], want)
