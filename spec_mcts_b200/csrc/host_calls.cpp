@@ -121,7 +121,7 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
       K > INT32_MAX || N > INT32_MAX || x->scalar_type() != at::kHalf || !x->is_contiguous() || !w->is_contiguous() || !s->is_contiguous())
     Py_RETURN_NONE;
   const int64_t M = x->size(0);
-  if (M < 1 || M > INT32_MAX) Py_RETURN_NONE;
+  if (M < 1 || M > INT32_MAX || (M > 32 && (uintptr_t)x->data_ptr() % 16 == 8)) Py_RETURN_NONE;      // those are copied first
   const auto stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
   PyObject* st = PyLong_FromVoidPtr(stream);
   if (!st) return nullptr;

@@ -638,7 +638,7 @@ extern "C" int q40_gemm_kn(const void* a, int64_t lda, const void* bw, const voi
 
 // q40_gemm_pair_tc.cu
 int q40_pair_linear(const void* x, int64_t ldx, const void* wq, const void* ws, void* y, int64_t ldy, int M, int N, int K, double beat_ns,
-                    void* staged, int* err, void* stream);
+                    int* err, void* stream);
 // q40_linear.cu
 double q40_linear_ns(int M, int N, int K);
 int q40_linear(const void* x, int64_t ldx, const void* wq, const void* ws, void* y, int64_t ldy, int M, int N, int K, void* stream);
@@ -693,19 +693,16 @@ extern "C" int q40_gemm_nk(const void* x, int64_t ldx, const void* wq, const voi
   // From 9 rows on tensor-core products by pairs of CTAs, where that is the faster one (above 32 rows always).  Us by launches of 32 rows at most, and by
   // pairs, weights from HBM: 10 rows x 4096 x 11008 13.3 and 14.0, 16 rows 14.7 and 14.0, 20 19.1 and 14.0, 32 36.0 and 14.3, 64 68.4 and 14.7, 100 113
   // and 15.6; 10 x 11008 x 4096 16.9 and 13.5, x 1024 x 1000 3.6 and 5.1; 16 x 2048 x 2048 4.9 and 6.4, 64 13.6 and 7.2; 128 x 11008 x 11008 308 and 33
-  // Activations that no tensor copy takes are laid out in the scratch first, if it has room for them: the same sums in the same order
-  const bool plain_x = q40_aligned(x, 16) && ldx % 8 == 0;
-  if (M > 8 && group == 64 && workspace && workspace_bytes >= (size_t)q40::COUNTER_BYTES + (plain_x ? 0 : (size_t)M * K * 2) &&
-      p.nblocks * 4 < q40::COUNTER_BYTES && q40_aligned(workspace, 16)) {
+  if (M > 8 && group == 64 && workspace && workspace_bytes >= (size_t)q40::COUNTER_BYTES && p.nblocks * 4 < q40::COUNTER_BYTES &&
+      q40_aligned(workspace, 16)) {
     const double beat = M > 32 ? 1e30 : q40_linear_ns(M, N, K) - 1000;       // what the pairs' estimate leaves out
-    char* const scratch = (char*)workspace + q40::COUNTER_BYTES;
-    const int rc = q40_pair_linear(x, ldx, wq, ws, y, ldy, M, N, K, beat, plain_x ? nullptr : scratch, reinterpret_cast<int*>(scratch - 4), stream);
+    const int rc = q40_pair_linear(x, ldx, wq, ws, y, ldy, M, N, K, beat, reinterpret_cast<int*>((char*)workspace + q40::COUNTER_BYTES - 4), stream);
     if (rc != Q40_E_UNSUPPORTED) return rc;
   }
-  // Otherwise (no scratch, activations that no tensor copy takes) 32 rows at a time with one CTA per SM, where the tiles allow it.  Above 32 rows a short k range over many CTAs is the exception, for which
-  // 64 rows a launch keep the SMs busy.  Microseconds by launches of 32 and by the launches below: 64 rows x 2048 x 2048 14.5 and 27.9,
-  // x 4096 x 5500 29.6 and 46.3; 100 rows x 1280 x 9000 30.9 and 57.5, x 3072 x 11008 59.6 and 92.6; 64 rows x 1024 x 6000 13.0 and 14.2, x
-  // 8000 14.5 and 14.0, x 11008 18.3 and 17.3
+  // Otherwise (up to 32 rows the pairs' estimate is the longer one; no scratch, no tensor maps) 32 rows at a time with one CTA per SM, where the
+  // tiles allow it.  Above 32 rows a short k range over many CTAs is the exception, for which 64 rows a launch keep the SMs busy.  Microseconds by
+  // launches of 32 and by the launches below: 64 rows x 2048 x 2048 14.5 and 27.9, x 4096 x 5500 29.6 and 46.3; 100 rows x 1280 x 9000 30.9 and
+  // 57.5, x 3072 x 11008 59.6 and 92.6; 64 rows x 1024 x 6000 13.0 and 14.2, x 8000 14.5 and 14.0, x 11008 18.3 and 17.3
   if (group == 64 && (M <= 32 || K > 1152 || N <= 6500)) {
     for (; m0 < M; m0 += 32) {
       const int rc = q40_linear(xh + m0 * ldx, ldx, wq, ws, yh + m0 * ldy, ldy, M - m0 < 32 ? M - m0 : 32, N, K, stream);

@@ -92,6 +92,8 @@ struct Params {
                            // both, of which a CTA has 64 (its A rows 0..63 those of matrix 0)
   int vec;                 // outputs take 16-byte stores
   const __half* nk_s;      // NK: scales [n_cols][K / 64]
+  const __half* x;         // NK: activations that no tensor copy takes (8-byte boundaries), or null
+  int64_t ldx;
   int n_cols;
   float* part;             // scratch slots: [pair][half][npad][128]
   int* flags;              // per pair: see FLAG_BYTES
@@ -363,6 +365,56 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
       }
     }
   };
+  // The activations of all blocks, eight bytes a lane, one k step of each by this warp; four blocks on their way.  Rows of the tile behind the last
+  // keep what was there: nothing is stored of their products.  Here, and by tensor copies behind a launch that copies the rows to 16 bytes: 10 rows
+  // x 11008 x 4096 15.4 and 15.9 us, 40 x 4096 x 11008 20.3 and 16.7, 100 rows 28.9 and 18.2 (by one warp 81, with rows of zeros; copies of eight
+  // bytes are what it waits for).  In place all the same: two threads on a stream may have their copies and products in any order
+  auto copy_rows = [&](const Work& wk, int h) {
+    constexpr int AHEAD = 3;                                 // below the number of stages
+    const int at = lane & 15, r0 = lane >> 4;
+    uint32_t to[4];                                          // rows r0, r0 + 2, .. + 6 of every eight
+#pragma unroll
+    for (int j = 0; j < 4; ++j) to[j] = RAW_PAD + h * b_bytes + (r0 + 2 * j) * 128 + (((at >> 1) ^ (r0 + 2 * j)) << 4) + 8 * (at & 1);
+    Slot sl, landed;
+    int n = 0, arrived = 0;
+    const auto arrive = [&]() {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the products read them through another proxy
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_act + 8 * landed.i);
+      landed.next(S);
+      ++arrived;
+    };
+    for (int k = 0; k < wk.np && limit; ++k) {
+      int tile, b0, b1, pi, span, fh, m0;
+      wk.piece(k, tile, b0, b1);
+      decode(tile, pi, span, fh, m0);
+      m0 += half * (p.npad / 2);
+      const int rows = min(p.npad / 2, p.M - m0) - r0;
+      const __half* src = p.x + (m0 + r0) * p.ldx + (b0 * BLK + h) * BK + 4 * at;
+      for (int b = b0; b < b1; ++b, src += BLK * BK) {
+        if (n >= S) wait_limited(bar_mdone + 8 * sl.i, sl.turn ^ 1, limit);
+        limit = __all_sync(0xffffffffu, limit != 0) ? limit : 0;
+        if (limit == 0) break;
+        uint32_t dst = ring + sl.i * stage_bytes;
+        const __half* from = src;
+        for (int r = 0; r < rows; r += 8, dst += 1024, from += 8 * p.ldx) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (r + 2 * j < rows)
+              asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + to[j]), "l"(from + 2 * j * p.ldx) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        sl.next(S);
+        if (++n > AHEAD) {
+          asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD) : "memory");
+          arrive();
+        }
+      }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    while (arrived < n) arrive();
+    failed = limit == 0;
+  };
   // Until then, only the warps that have something to do run: with all 24 finding out their share (five divisions) first, the first
   // weights were requested 1.4 to 1.9 us after the start of a CTA
   if (warp == 0) {
@@ -379,7 +431,7 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
     }
     if (lane < S) {
       mbar_init(bar_full + 8 * lane, 1);
-      mbar_init(bar_act + 8 * lane, 1);
+      mbar_init(bar_act + 8 * lane, NK && p.x ? BLK : 1);
       mbar_init(bar_mdone + 8 * lane, 1);
     }
     if (lane < NA) mbar_init(bar_afull + 8 * lane, 8);
@@ -402,7 +454,7 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
       asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(TMEM_COLS));
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    } else if (warp == 3 && lane <= (NK ? 1 : 2 * p.nprob)) {
+    } else if (warp == 3 && lane <= (NK ? 1 : 2 * p.nprob) && !(NK && lane == 0 && p.x)) {
       const CUtensorMap* m = lane == 0 ? &maps.act : lane <= p.nprob ? &maps.w[lane - 1] : &maps.s[lane - 1 - p.nprob];
       asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
     }
@@ -417,7 +469,11 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
   const uint32_t A_COL0 = TMEM_COLS - A_COLS * NA;
   asm volatile("griddepcontrol.launch_dependents;");
 
-  if (warp == 0 || warp == 2) {
+  if (NK && p.x && (warp == 2 || warp == 3)) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    copy_rows(wk, warp - 2);
+    s_copied[1] = 0;
+  } else if (warp == 0 || warp == 2) {
     if (elect_one()) {
       if (warp == 0) {
         if (total > S) copy_blocks(wk, S, total, true);
@@ -979,12 +1035,12 @@ static int pair_run(q40::ttc::pair::Params& p, bool nk, int spans, const void* a
   if (smem == 0 || smem > (size_t)SMEM_MAX) return Q40_E_UNSUPPORTED;
   PairKernel kern = split > 1 ? in_clusters : nk ? plain : kernel(1 + silu + 2 * cut);
   if (!kern) return Q40_E_UNSUPPORTED;
-  pair::Maps maps;
+  pair::Maps maps{};
   const cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)M};
   const cuuint64_t gstride[1] = {(cuuint64_t)lda * 2};
   const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)p.npad / 2};
   const cuuint32_t estr[2] = {1, 1};
-  if (ttc_encode(encode, &maps.act, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)a, gdim, gstride, box, estr,
+  if (!p.x && ttc_encode(encode, &maps.act, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)a, gdim, gstride, box, estr,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return Q40_E_UNSUPPORTED;
@@ -1042,10 +1098,10 @@ int q40_pair_gemm(int nmat, const void* a, int64_t lda, const void* const* bw_ti
   });
 }
 
-// Y[M, N] = X[M, K] @ deq(W)^T for W [N, K] with groups of 64 along K: see q40_gemm_nk, whose arguments are checked.  K % 128 == 0; x on 16-byte
+// Y[M, N] = X[M, K] @ deq(W)^T for W [N, K] with groups of 64 along K: see q40_gemm_nk, whose arguments are checked.  K % 128 == 0; x on 8-byte
 // boundaries, rows too.  Weights may be what the launch in front writes: they are requested behind the wait for it
 int q40_pair_linear(const void* x, int64_t ldx, const void* wq, const void* ws, void* y, int64_t ldy, int M, int N, int K, double beat_ns,
-                    void* staged, int* err, void* stream) {
+                    int* err, void* stream) {
   using namespace q40;
   using namespace q40::ttc;
   pair::Params p{};
@@ -1054,13 +1110,10 @@ int q40_pair_linear(const void* x, int64_t ldx, const void* wq, const void* ws, 
   p.vec = q40_aligned(y, 16) && ldy % 8 == 0 ? 1 : q40_aligned(y, 4) && ldy % 2 == 0 ? 0 : 2;
   p.nprob = 1; p.M = M; p.K = K; p.err = err;
   p.nk_s = (const __half*)ws; p.n_cols = N;
+  if (!q40_aligned(x, 16) || ldx % 8 != 0) { p.x = (const __half*)x; p.ldx = ldx; }
   p.k64 = K / BK;
   pair::k_blocks(p, p.k64);
-  return pair_run(p, true, p.spans[0], staged ? staged : x, staged ? K : ldx, nullptr, 0, beat_ns, 1, stream, [&](EncodeTiledFn encode, pair::Maps& maps) {
-    if (staged && cudaMemcpy2DAsync(staged, (size_t)K * 2, x, (size_t)ldx * 2, (size_t)K * 2, M, cudaMemcpyDeviceToDevice, (cudaStream_t)stream) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return false;
-    }
+  return pair_run(p, true, p.spans[0], x, ldx, nullptr, 0, beat_ns, 1, stream, [&](EncodeTiledFn encode, pair::Maps& maps) {
     const cuuint64_t dim[2] = {(cuuint64_t)K / 2, (cuuint64_t)N}, pitch[1] = {(cuuint64_t)K / 2};
     const cuuint32_t box[2] = {64, pair::FEATS}, estr[2] = {1, 1};
     return ttc_encode(encode, &maps.w[0], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)wq, dim, pitch, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,

@@ -105,3 +105,59 @@ def test_rows_off_16_bytes_have_the_same_bits_captured_too(M, K, N):
         call(off, y[2])
     graph.replay()
     assert torch.equal(y[0], y[1]) and torch.equal(y[0], y[2])
+
+
+# one block of k; more blocks than the ring has stages; k split over a cluster and not; rows that fill no pair of eight; several chunks of rows
+@pytest.mark.parametrize("M,K,N", [(33, 128, 300), (40, 11008, 1000), (100, 4096, 20001), (20, 4096, 11008), (64, 11008, 128), (128, 2048, 515), (129, 640, 640), (300, 4096, 700), (513, 128, 300)])
+def test_rows_8_bytes_off_have_the_same_bits_whatever_the_scratch(M, K, N, monkeypatch):
+    """What a call computes, and how, does not depend on where its activations lie, nor on the calls before it."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from spec_mcts_b200 import kernels as KK
+    from spec_mcts_b200._lib import check, lib
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    q, s = KK.quantize_q40((torch.randn((N, K), generator=g, device="cuda") * 0.05).half())
+    x = torch.randn((M, K), generator=g, device="cuda").half()
+    off = torch.zeros(4 + M * K, dtype=torch.float16, device="cuda")[4:].view(M, K).copy_(x)
+    assert off.data_ptr() % 16 == 8
+    want = KK.linear_q40(x, q, s, (N, K))
+    monkeypatch.setattr(KK, "_workspaces", {})
+    for _ in range(2):                                        # a first call, and one that the native way may take
+        assert torch.equal(KK.linear_q40(off, q, s, (N, K)), want)
+    with pytest.raises(KK.Q40Error):                          # nearer than 8 bytes: refused as ever
+        KK.linear_q40(torch.zeros(1 + M * K, dtype=torch.float16, device="cuda")[1:].view(M, K), q, s, (N, K))
+    assert KK.tc_error_flag() == 0
+    # rows further apart, and a result that is column ranges of wider rows
+    wide = torch.full((M, K + 12), 9.0, dtype=torch.float16, device="cuda")
+    y = torch.full((M + 1, N + 3), 7.0, dtype=torch.float16, device="cuda")
+    wide[:, 4:4 + K] = x
+    ws = torch.zeros(lib.q40_gemm_workspace_bytes(M, N, K), dtype=torch.uint8, device="cuda")
+    check(lib.q40_gemm_nk(wide[:, 4:].data_ptr(), K + 12, q.data_ptr(), s.data_ptr(), y[:, 1:].data_ptr(), N + 3, M, N, K, 64, ws.data_ptr(), ws.numel(),
+                          torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(y[:M, 1:1 + N], want) and (y[M] == 7).all() and (y[:, 0] == 7).all() and (y[:, 1 + N:] == 7).all()
+    assert not ws.any()
+
+
+def test_rows_8_bytes_off_from_two_threads_on_one_stream():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import threading
+    from spec_mcts_b200 import kernels as KK
+    g = torch.Generator(device="cuda").manual_seed(1)
+    M, K, N = 40, 2048, 1000
+    q, s = KK.quantize_q40((torch.randn((N, K), generator=g, device="cuda") * 0.05).half())
+    xs = [torch.zeros(4 + M * K, dtype=torch.float16, device="cuda")[4:].view(M, K).copy_(torch.randn((M, K), generator=g, device="cuda")) for _ in range(2)]
+    want = [KK.linear_q40(x.clone(), q, s, (N, K)) for x in xs]
+    out = [[], []]
+
+    def work(i):
+        for _ in range(300):
+            out[i].append(KK.linear_q40(xs[i], q, s, (N, K)))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert all(len(o) == 300 and all(torch.equal(y, w) for y in o) for o, w in zip(out, want))
