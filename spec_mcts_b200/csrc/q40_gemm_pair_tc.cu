@@ -30,11 +30,11 @@
 // with all SMs busy, loads from L2 (512 rows x 4096 x 11008: 26 bytes a cycle and SM over a launch).  A launch adds 3.4 to 5: what its CTAs do
 // first (1.2, beside the launch in front where that leaves SMs free), activations 0.8, the last accumulator's way out 0.6 to 1.5, the end 0.6.
 // As many A buffers as tensor memory has room for (seven up to 32 rows, with four a dequantiser waited half its time for the MMAs of the
-// block before), the first of them filled while the launch in front still writes the activations; one warp of the epilogue polls.
-// Microseconds, launches in a row, before these and now: 10 rows x 4096 x 4096 8.2 and 6.9, three of them 13.2 and 12.6, x 11008 x 4096
-// 13.1 and 12.0; 100 rows 10.0 and 9.2, 16.1 and 14.5, 15.3 and 14.7.  With the SiLU product: 10 rows x 4096 x 11008 17.5 and 16.4, 64 rows
-// 22.7 and 20.2, 100 rows 28.5 and 25.2, 512 rows 87.8 and 79.9 (eight quotients in flight at once: see silu); 512 rows without it,
-// whose k blocks wait for L2, 45.8 and 48.0 x 11008, 42.5 and 43.0 x 11008 x 4096.
+// block before); one warp of the epilogue polls.
+// Microseconds, launches in a row out of a graph, six sets of weights in turn, the power limit active above 64 rows; before these and now: 10 rows
+// x 4096 x 4096 8.2 and 6.9, three of them 13.3 and 12.3, x 11008 x 4096 13.3 and 12.0; 102 rows 9.9 and 9.2, 17.3 and 15.6, 15.8 and 15.4. With the
+// SiLU product: 10 rows x 4096 x 11008 17.7 and 16.2, 64 rows 24.3 and 21.2, 100 rows 31.4 and 25.6, 512 rows 94.5 and 82.5 (eight quotients in flight
+// at once: see silu). 512 rows without it, whose k blocks wait for L2: 49.6 and 48.3 x 11008, 45.4 and 44.9 x 11008 x 4096.
 //
 // Every wait is bounded (by seconds): on expiry an error word is set and no more copies are requested; what is still
 // multiplied and stored is undefined, as is the scratch.  Copies and MMAs in flight are waited for, tensor memory is freed.
@@ -62,7 +62,8 @@ constexpr int NA_MAX = 8;
 constexpr int TMEM_COLS = 512;
 constexpr int CUT = 2;                          // a k range is cut at multiples of so many blocks
 constexpr int GROUPS = 1 + DSETS;               // of four warps, one per tensor-memory quadrant, that finish a pair's last tile
-constexpr int BAR_BYTES = 24 * S_MAX + 8 * NA_MAX + 64;
+template <bool EARLY>
+constexpr int BAR_BYTES = (EARLY ? 24 : 16) * S_MAX + 8 * NA_MAX + 64;
 constexpr uint32_t FLAG_POLLS = 1u << 22;       // of one flag, before giving up: seconds, like the other waits
 constexpr int OUT_LD = FEATS + 8;              // halves between rows that wait in shared memory
 constexpr int MAX_PAIRS = 128;
@@ -92,11 +93,15 @@ struct Params {
                            // both, of which a CTA has 64 (its A rows 0..63 those of matrix 0)
   int vec;                 // outputs take 16-byte stores
   const __half* nk_s;      // NK: scales [n_cols][K / 64]
-  const __half* x;         // NK: activations that no tensor copy takes (8-byte boundaries), or null
-  int64_t ldx;
   int n_cols;
-  float* part;             // scratch slots: [pair][half][npad][128]
-  int* flags;              // per pair: see FLAG_BYTES
+  union {                  // (NK never cuts tiles; arguments are launch time)
+    float* part;           // scratch slots: [pair][half][npad][128]
+    const __half* x;       // NK: activations that no tensor copy takes (8-byte boundaries), or null
+  };
+  union {
+    int* flags;            // per pair: see FLAG_BYTES
+    int64_t ldx;
+  };
   int* err;
 };
 
@@ -271,7 +276,10 @@ struct Work {
 // CUT: tiles may be shared between pairs along k; SILU: see Params (compiled for each, to keep the registers of all roles
 // below the 80 that 24 warps leave)
 // NK: one matrix [n_cols, K] with groups along K, as quantised in memory (not a tiled copy): a lane expands its own feature's row
-template <bool SPLIT, bool CUT_K, bool SILU, bool NK = false>
+// EARLY: weights are expanded before their block's activations have landed, which the launch in front may still write.  Where a pair has one tile:
+// 10 rows x 4096 x 4096 6.9 us, 7.2 without; 100 rows 9.2 and 9.6.  Where it has several the wait of its own costs more: 512 rows x 4096 x 11008 46.4
+// without and 49.6, x 11008 x 4096 43.2 and 44.4, 100 x 11008 x 11008 33.1 and 34.1 (for a pair's first blocks alone: 48.4, 44.3, 33.3)
+template <bool EARLY, bool SPLIT, bool CUT_K, bool SILU, bool NK = false>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
   extern __shared__ unsigned char smem_raw[];
@@ -285,17 +293,17 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
   const uint32_t raw0 = smem_u32(smem_raw);
   const uint32_t ring = (raw0 + 1023u) & ~1023u;
   unsigned char* gbase = smem_raw + (ring - raw0);
-  // Block i has stage and barriers i % S and A buffer i % NA.  full: its weights have landed in this
-  // CTA (act: its activations); mdone: its MMAs are complete, in both CTAs; accfull[b]: an accumulator is complete.  In the even CTA, for
+  // Block i has stage and barriers i % S and A buffer i % NA.  full: its weights and activations have landed in this
+  // CTA (EARLY: its weights; act: its activations); mdone: its MMAs are complete, in both CTAs; accfull[b]: an accumulator is complete.  In the even CTA, for
   // both: afull: the A operand is written (and the activations have landed); accfree[b]: an accumulator has been read.
-  const uint32_t bar_full = ring + (uint32_t)p.bar_off, bar_act = bar_full + 8 * S_MAX, bar_mdone = bar_act + 8 * S_MAX,
+  const uint32_t bar_full = ring + (uint32_t)p.bar_off, bar_act = EARLY ? bar_full + 8 * S_MAX : bar_full, bar_mdone = bar_act + 8 * S_MAX,
                  bar_afull = bar_mdone + 8 * S_MAX, bar_accfull = bar_afull + 8 * NA_MAX, bar_accfree = bar_accfull + 16,
                  bar_done = bar_accfree + 16, bar_last = bar_done + 8, bar_flags = bar_last + 8, bar_recv = bar_flags + 8;
-  unsigned char* tail = gbase + p.bar_off + BAR_BYTES;
+  unsigned char* tail = gbase + p.bar_off + BAR_BYTES<EARLY>;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail);
   volatile int* s_failed = reinterpret_cast<volatile int*>(tail + 8);
   volatile int* s_acc = reinterpret_cast<volatile int*>(tail + 24);        // accumulator of a pair's last tile
-  volatile int* s_copied = reinterpret_cast<volatile int*>(tail + 16);     // [2] see copy_blocks
+  volatile int* s_copied = reinterpret_cast<volatile int*>(tail + 16);     // blocks requested: [0] weights, [1] activations, [3] copy_rows' second warp
   int4* s_share = reinterpret_cast<int4*>(tail + 32);                      // see Work::share
   float* run = reinterpret_cast<float*>(gbase + p.run_off);                // [npad][128] sums of earlier ranges
   __half* out_s = reinterpret_cast<__half*>(gbase + p.out_off);            // [2][16][OUT_LD] finished rows on their way out
@@ -413,6 +421,7 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     while (arrived < n) arrive();
+    s_copied[h ? 3 : 1] = n;
     failed = limit == 0;
   };
   // Until then, only the warps that have something to do run: with all 24 finding out their share (five divisions) first, the first
@@ -430,8 +439,9 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
       }
     }
     if (lane < S) {
-      mbar_init(bar_full + 8 * lane, 1);
-      mbar_init(bar_act + 8 * lane, NK && p.x ? BLK : 1);
+      const int acts = NK && p.x ? BLK : 1;                  // arrivals of a block's activations
+      mbar_init(bar_full + 8 * lane, EARLY ? 1 : 1 + acts);
+      if (EARLY) mbar_init(bar_act + 8 * lane, acts);
       mbar_init(bar_mdone + 8 * lane, 1);
     }
     if (lane < NA) mbar_init(bar_afull + 8 * lane, 8);
@@ -472,7 +482,6 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
   if (NK && p.x && (warp == 2 || warp == 3)) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     copy_rows(wk, warp - 2);
-    s_copied[1] = 0;
   } else if (warp == 0 || warp == 2) {
     if (elect_one()) {
       if (warp == 0) {
@@ -597,8 +606,7 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
         st_16x256b_x4(ta + 32 * h + (16u << 16), r[1]);
       }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-      // the first blocks are expanded while the launch in front still writes the activations
-      wait_limited(bar_act + 8 * sl.i, sl.turn, limit);
+      if constexpr (EARLY) wait_limited(bar_act + 8 * sl.i, sl.turn, limit);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(afull_lead + 8 * sa.i);
@@ -790,8 +798,16 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
   if (failed && tid == 0) {
     // the copies still on their way, those of the last S blocks at most: none may land in shared memory that has been given back
     q40_set_error(p.err);
-    for (int h = 0; h < 2; ++h)
-      for (int n = s_copied[h], i = max(0, n - S); i < n; ++i) mbar_wait((h ? bar_act : bar_full) + 8 * (i % S), (uint32_t)((i / S) & 1));
+    if constexpr (EARLY) {
+      for (int h = 0; h < 2; ++h)
+        for (int n = h && NK && p.x ? min(s_copied[1], s_copied[3]) : s_copied[h], i = max(0, n - S); i < n; ++i)
+          mbar_wait((h ? bar_act : bar_full) + 8 * (i % S), (uint32_t)((i / S) & 1));
+    } else {
+      // (first in the place of those that gave up before they requested a block that another did)
+      for (int h = 0, n = max(s_copied[0], s_copied[1]); h < (NK && p.x ? 3 : 2); ++h)
+        for (int i = s_copied[h == 2 ? 3 : h]; i < n; ++i) mbar_arrive(bar_full + 8 * (i % S));
+      for (int n = max(s_copied[0], s_copied[1]), i = max(0, n - S); i < n; ++i) mbar_wait(bar_full + 8 * (i % S), (uint32_t)((i / S) & 1));
+    }
   }
 
   if (SPLIT && warp >= DQ_WARP0) {
@@ -860,17 +876,19 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
 
 using PairKernel = void (*)(const q40::ttc::pair::Params, const q40::ttc::pair::Maps);
 
-// [0] SPLIT; else 1 + 1 SiLU + 2 cut; [5], [6] SPLIT and not, with groups along K
+// [0] SPLIT; [1] EARLY; else 2 + 1 SiLU + 2 cut; [6] .. [8] with groups along K: SPLIT, EARLY, neither
 static PairKernel pair_kernel(int which) {
   using namespace q40::ttc::pair;
   switch (which) {
-    case 0: return gemm_pair_kernel<true, false, false>;
-    case 1: return gemm_pair_kernel<false, false, false>;
-    case 2: return gemm_pair_kernel<false, false, true>;
-    case 3: return gemm_pair_kernel<false, true, false>;
-    case 4: return gemm_pair_kernel<false, true, true>;
-    case 5: return gemm_pair_kernel<true, false, false, true>;
-    default: return gemm_pair_kernel<false, false, false, true>;
+    case 0: return gemm_pair_kernel<true, true, false, false>;
+    case 1: return gemm_pair_kernel<true, false, false, false>;
+    case 2: return gemm_pair_kernel<false, false, false, false>;
+    case 3: return gemm_pair_kernel<false, false, false, true>;
+    case 4: return gemm_pair_kernel<false, false, true, false>;
+    case 5: return gemm_pair_kernel<false, false, true, true>;
+    case 6: return gemm_pair_kernel<true, true, false, false, true>;
+    case 7: return gemm_pair_kernel<true, false, false, false, true>;
+    default: return gemm_pair_kernel<false, false, false, false, true>;
   }
 }
 
@@ -924,9 +942,10 @@ static size_t layout(Params& p, int split, bool single) {
   const size_t tile = (size_t)p.npad * FEATS * 4, stage = RAW_PAD + (size_t)p.npad * 64 * BLK;
   p.own = ((p.M + 3) / 4 + split - 1) / split;
   const size_t run = split > 1 ? (size_t)(split - 1) * p.own * FEATS * 16 : p.range < p.k64 ? tile : 0;
+  const bool early = single && !p.silu;
   p.egroups = !single && (p.silu ? p.cut && p.npad >= 96 : 8 * p.rblk <= p.npad) ? 2 : 1;
   const size_t out = split > 1 ? 0 : p.egroups * 2 * 16 * OUT_LD * 2;
-  const size_t fixed = 1024 /* alignment */ + BAR_BYTES + 64 /* tail */ + run + out;
+  const size_t fixed = 1024 /* alignment */ + (early ? BAR_BYTES<true> : BAR_BYTES<false>) + 64 /* tail */ + run + out;
   if (fixed + DSETS * stage > (size_t)SMEM_MAX) return 0;
   p.stages = std::min(S_MAX, (int)((SMEM_MAX - fixed) / stage));
   p.nacc = !single && 2 * p.npad + 2 * A_COLS <= TMEM_COLS ? 2 : 1;
@@ -973,14 +992,14 @@ static int pair_run(q40::ttc::pair::Params& p, bool nk, int spans, const void* a
   if (!encode) return Q40_E_UNSUPPORTED;
   if ((int64_t)spans * ((M + 63) / 64) * std::max(p.nblk, pair::MAX_PAIRS) > 0x7fffffffLL) return Q40_E_UNSUPPORTED;
   // the kernels' attributes come first: the runtime is asked how many fit with the shared memory that they allow
-  static std::atomic<uint64_t> ready[7];
+  static std::atomic<uint64_t> ready[9];
   auto kernel = [&](int which) -> PairKernel {
     PairKernel k = pair_kernel(which);
     if (q40_allow_smem(ready[which], (const void*)k, SMEM_MAX) == cudaSuccess) return k;
     (void)cudaGetLastError();
     return nullptr;
   };
-  PairKernel plain = kernel(nk ? 6 : 1), in_clusters = kernel(nk ? 5 : 0);
+  PairKernel plain = kernel(nk ? 8 : 2), in_clusters = kernel(nk ? 6 : 0);
   if (!plain || !in_clusters) return Q40_E_UNSUPPORTED;
   const int fit = pair_max_clusters(plain, 1) < pair::MAX_PAIRS ? pair_max_clusters(plain, 1) : pair::MAX_PAIRS;
   if (fit < 1) return Q40_E_UNSUPPORTED;
@@ -1031,16 +1050,17 @@ static int pair_run(q40::ttc::pair::Params& p, bool nk, int spans, const void* a
     p.share = units / npairs;
     p.rest = units % npairs;
   }
-  const size_t smem = pair::layout(p, split, split > 1 || (!cut && p.ntiles <= npairs && p.range == p.k64));
+  const bool single = split > 1 || (!cut && p.ntiles <= npairs && p.range == p.k64);
+  const size_t smem = pair::layout(p, split, single);
   if (smem == 0 || smem > (size_t)SMEM_MAX) return Q40_E_UNSUPPORTED;
-  PairKernel kern = split > 1 ? in_clusters : nk ? plain : kernel(1 + silu + 2 * cut);
+  PairKernel kern = split > 1 ? in_clusters : single && !silu ? kernel(nk ? 7 : 1) : nk ? plain : kernel(2 + silu + 2 * cut);
   if (!kern) return Q40_E_UNSUPPORTED;
   pair::Maps maps{};
   const cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)M};
   const cuuint64_t gstride[1] = {(cuuint64_t)lda * 2};
   const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)p.npad / 2};
   const cuuint32_t estr[2] = {1, 1};
-  if (!p.x && ttc_encode(encode, &maps.act, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)a, gdim, gstride, box, estr,
+  if (!(nk && p.x) && ttc_encode(encode, &maps.act, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)a, gdim, gstride, box, estr,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return Q40_E_UNSUPPORTED;
