@@ -937,15 +937,19 @@ static void tile_rows(Params& p, int npad) {
 // Two groups finish tiles where that is what a pair waits for: the sums of ranges of few blocks (three matrices of 512 rows x 4096 x 4096, eight
 // blocks: 54.4 us with one, 52.4; 300 rows 39.0 and 34.9; but 22 blocks, x 11008 x 4096, 43.3 and 46.4), and many rows of a SiLU product
 // with shared tiles (x 4096 x 11008, 100 rows 26.2 and 24.5, 128 28.8 and 26.2; 77 21.7 and 22.0).  Where there is one tile a pair, its warps
-// dequantise too (10 rows x 4096 x 12288 12.1 and 11.8, x 11008 x 4096 11.6 and 11.4, 64 rows 12.7 and 12.3, 100 the same)
-static size_t layout(Params& p, int split, bool single) {
+// dequantise too (10 rows x 4096 x 12288 12.1 and 11.8, x 11008 x 4096 11.6 and 11.4, 64 rows 12.7 and 12.3, 100 the same).
+// `alone`: no pair has more than one tile.  Then one group, where the output rows of two leave no room for the ring (three x 4096 x 4096 in tiles of
+// 176 rows: 171 rows 25.2 us, in tiles of 96 with two groups 26.7); where pairs have more, smaller tiles are the faster ones (512 rows 55.8 and 52.8)
+static size_t layout(Params& p, int split, bool single, bool alone) {
   const size_t tile = (size_t)p.npad * FEATS * 4, stage = RAW_PAD + (size_t)p.npad * 64 * BLK;
   p.own = ((p.M + 3) / 4 + split - 1) / split;
   const size_t run = split > 1 ? (size_t)(split - 1) * p.own * FEATS * 16 : p.range < p.k64 ? tile : 0;
   const bool early = single && !p.silu;
   p.egroups = !single && (p.silu ? p.cut && p.npad >= 96 : 8 * p.rblk <= p.npad) ? 2 : 1;
-  const size_t out = split > 1 ? 0 : p.egroups * 2 * 16 * OUT_LD * 2;
-  const size_t fixed = 1024 /* alignment */ + (early ? BAR_BYTES<true> : BAR_BYTES<false>) + 64 /* tail */ + run + out;
+  const auto out_bytes = [&]() { return split > 1 ? (size_t)0 : (size_t)p.egroups * 2 * 16 * OUT_LD * 2; };
+  const size_t rest = 1024 /* alignment */ + (early ? BAR_BYTES<true> : BAR_BYTES<false>) + 64 /* tail */ + run;
+  if (alone && rest + out_bytes() + DSETS * stage > (size_t)SMEM_MAX) p.egroups = 1;
+  const size_t out = out_bytes(), fixed = rest + out;
   if (fixed + DSETS * stage > (size_t)SMEM_MAX) return 0;
   p.stages = std::min(S_MAX, (int)((SMEM_MAX - fixed) / stage));
   p.nacc = !single && 2 * p.npad + 2 * A_COLS <= TMEM_COLS ? 2 : 1;
@@ -1023,7 +1027,7 @@ static int pair_run(q40::ttc::pair::Params& p, bool nk, int spans, const void* a
       const int chunks = (M + n - 1) / n;
       if (((M + chunks - 1) / chunks + 15) / 16 * 16 != n) continue;           // the same chunks with fewer rows of padding
       pair::tile_rows(p, n);
-      if (pair::layout(p, 1, false) == 0) continue;
+      if (pair::layout(p, 1, false, (int64_t)spans * chunks <= fit) == 0) continue;
       const double waves = (double)(((int64_t)spans * chunks + fit - 1) / fit);
       const double block = n <= 128 ? 165 + 1.8 * n : 395 + 2.8 * (n - 128);
       const int nr = (p.k64 + p.range - 1) / p.range;
@@ -1051,7 +1055,7 @@ static int pair_run(q40::ttc::pair::Params& p, bool nk, int spans, const void* a
     p.rest = units % npairs;
   }
   const bool single = split > 1 || (!cut && p.ntiles <= npairs && p.range == p.k64);
-  const size_t smem = pair::layout(p, split, single);
+  const size_t smem = pair::layout(p, split, single, p.ntiles <= npairs);
   if (smem == 0 || smem > (size_t)SMEM_MAX) return Q40_E_UNSUPPORTED;
   PairKernel kern = split > 1 ? in_clusters : single && !silu ? kernel(nk ? 7 : 1) : nk ? plain : kernel(2 + silu + 2 * cut);
   if (!kern) return Q40_E_UNSUPPORTED;

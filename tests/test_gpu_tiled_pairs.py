@@ -197,3 +197,23 @@ def test_a_share_that_never_comes_is_given_up_after_seconds(K):
     ws[:8192].zero_()
     launch(a, tiled, [g, g], (n, n), 1, ws, 1)
     assert torch.equal(g, want)
+
+
+@pytest.mark.parametrize("M", [161, 171, 176, 177])     # tiles of 176 rows, and the smaller ones of the next more
+def test_largest_tiles_with_sums_of_ranges(K, M):
+    """k in ranges that are summed one after the other, in tiles whose ring has just the room it needs, against float64."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    Kd, Ns = 4096, (4096, 4096, 4096)
+    packed = [K.quantize_q40((torch.randn((Kd, n), generator=g, device="cuda") * 0.05).half()) for n in Ns]
+    tiled = [K.relayout_tiled(q, s, (Kd, n)) for (q, s), n in zip(packed, Ns)]
+    a, ws = torch.randn((M, Kd), generator=g, device="cuda").half(), scratch(K, M)
+    outs = [torch.full((M, n), float("nan"), dtype=torch.float16, device="cuda") for n in Ns]
+    launch(a, tiled, outs, Ns, 0, ws)
+    for o, (q, s), n in zip(outs, packed, Ns):
+        w = K.dequantize_q40(q, s, 64, (Kd, n)).double()         # the operand as it is multiplied
+        want, size = a.double() @ w, a.double().abs() @ w.abs()
+        # fp32 sums (2^-24 per addition, 1e-5 covers 4096 of them in any grouping) and the result's half step
+        assert ((o.double() - want).abs() <= want.abs() * 2 ** -11 + 2 ** -25 + 1e-5 * size).all()
+    again = [torch.empty_like(o) for o in outs]
+    launch(a, tiled, again, Ns, 0, ws, 1)
+    assert all(torch.equal(x, y) for x, y in zip(outs, again))
