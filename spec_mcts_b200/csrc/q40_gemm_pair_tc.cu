@@ -148,17 +148,18 @@ __device__ __forceinline__ void ld4(uint32_t taddr, uint32_t (&r)[4]) {
 __device__ __forceinline__ void wait_ld4(uint32_t (&r)[4]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]) :: "memory");
 }
-// x / (1 + exp(-x)) for x that fp16 can hold, rounded once as the division operator does, without its branch for operands that cannot
-// occur here: eight of them in flight take a fifth of the time.  The quotient by one Newton step for the reciprocal and the
-// remainder of the product (P. Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, 1990).
-// Beyond 32 the divisor is 1; below -80 the result is -0 in fp16 whatever the exponential
+// x / (1 + exp(-x)) for x that fp16 can hold.  The quotient by one Newton step for the reciprocal and the remainder of the product
+// (P. Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, 1990): eight of them in flight take a fifth of the
+// time of eight divisions one after the other.  Rounded to fp16 it is what those give for every fp16 x, which is what the tests compare.
+// Beyond 32 the divisor is 1; below -80 the result is -0 in fp16 whatever the exponential; a zero keeps its sign
+// (a remainder of +0 times -r, which is -0, added to it)
 __device__ __forceinline__ float silu(float x) {
   const float d = 1.0f + expf(fminf(-x, 80.0f));
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
   r = fmaf(fmaf(-d, r, 1.0f), r, r);
   const float q = x * r;
-  return x > 32.0f ? x : fmaf(fmaf(-d, q, x), r, q);
+  return x > 32.0f ? x : fmaf(fmaf(d, q, -x), -r, q);
 }
 __device__ __forceinline__ void commit2(uint32_t bar, uint16_t mask) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"

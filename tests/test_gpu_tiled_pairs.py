@@ -118,6 +118,24 @@ def test_silu_of_every_fp16_value(K):
     assert torch.equal(g.view(torch.int16)[~want.isnan()], want.view(torch.int16)[~want.isnan()].view(-1, 1).expand(-1, n)) and g[want.isnan()].isnan().all()
 
 
+@pytest.mark.parametrize("M,n", [(16, 256), (10, 9728), (129, 512)])
+def test_silu_of_a_sum_that_rounds_to_minus_zero(K, M, n):
+    """x is a negative sum below the smallest fp16, y is 1: the product is -0, as by the launch that divides."""
+    Kd, rows = 64, n // 128
+    mats = [(np.zeros((Kd * rows, 64), np.int8), np.zeros((Kd * n // 64,), np.float16)) for _ in range(2)]
+    for k, (q, s) in enumerate(mats):                            # row k of matrix k: 2^-14 in the first, ones in the second
+        q[k * rows:(k + 1) * rows], s[k * n // 64:(k + 1) * n // 64] = 0x11, 1 if k else 2 ** -14
+    tiled = [K.relayout_tiled(torch.from_numpy(q).cuda(), torch.from_numpy(s).cuda(), (Kd, n)) for q, s in mats]
+    a = torch.zeros((M, Kd), dtype=torch.float16, device="cuda")
+    a[:, 0], a[:, 1] = -2.0 ** -24, 1
+    g, ws = torch.empty((M, n), dtype=torch.float16, device="cuda"), scratch(K, M)
+    launch(a, tiled, [g, g], (n, n), 1, ws)
+    outs = [torch.empty((M, n), dtype=torch.float16, device="cuda") for _ in range(2)]
+    launch(a, tiled, outs, (n, n), 0, ws)
+    assert (outs[0].view(torch.int16) == -0x8000).all() and (outs[1] == 1).all()
+    assert torch.equal(g.view(torch.int16), K.silu_mul(*outs).view(torch.int16)) and torch.signbit(g).all()
+
+
 # the k range of a tile over two, three and four pairs of a cluster, each finishing some groups of four rows: one group and none for
 # some ranks, the last one ragged, as many as divide and not
 @pytest.mark.parametrize("M", [1, 4, 9, 13, 17, 36, 100, 128])
