@@ -164,6 +164,7 @@ static int launch_rows(const BranchArgs& a, cudaStream_t st) {
 //     2 / 4 23.2, 4 / 4 30.1, of up to 256 49.7 and 52.1
 //   contiguous, 512 keys: 256 rows 8 / 4 12.6, 4 / 4 14.7; 416 rows 8 / 2 19.3, 4 / 4 19.9; 768 rows 4 / 4 35.9, 2 / 4 36.1; 3200 rows
 //     of 256 4 / 4 63.1, 2 / 4 67.0; of 64: 64 rows 4 / 4 2.6, 8 / 4 3.1; 768 rows 2 / 4 5.1, 4 / 4 5.9
+// (a.L is the length here: rows whose lengths are on the device come by their number alone, see f16_form_of_rows, and not between 4 and 6 SMs')
 template <int MODE>
 static int launch_branch_mode(const BranchArgs& a, cudaStream_t st) {
   const int64_t rows = a.rows;

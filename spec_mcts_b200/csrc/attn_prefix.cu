@@ -182,7 +182,7 @@ attn_prefix_kernel(const PrefixArgs a) {
   }
 }
 
-// `own`: keys that the branches have of their own in front of a head, about; 0: not known
+// `own`: keys that the branches have of their own in front of a head, about; 0: not known, -1: their lengths are on the device
 static int prefix_splits(int B, int H, int Hkv, int prefix_len, int64_t own) {
   const int rep = H / Hkv;
   const int rows = B * rep;
@@ -195,7 +195,10 @@ static int prefix_splits(int B, int H, int Hkv, int prefix_len, int64_t own) {
   // partials and leaves SMs to them (64 branches of up to 256 own keys behind 512: 34.6 us with two, 31.4; 34 behind 471 22.2 and 21.4; at four
   // times the prefix no difference, below it one is slower: 10 behind 2048 16.6 and 18.5; and with fewer than eight tiles: 64 branches
   // of up to 100 behind 300 17.9 and 18.7)
-  const bool hidden = tiles >= 8 && own > 6 * (int64_t)prefix_len;
+  // With lengths on the device neither the table's width nor anything else that they leave open may decide (splits have their own order of
+  // sums): one up to ten tiles, which 64, 34 and 10 branches of up to 16 / 64 / 128 / 256 / 500 keys behind 512 take 0.87 to 1.04 times as long with as
+  // with two, behind 700 0.92 to 1.08, behind 1024 0.87 to 1.18, behind 2048 0.94 to 1.39; 8 kv heads no difference
+  const bool hidden = tiles >= 8 && (own < 0 ? tiles <= 10 : own > 6 * (int64_t)prefix_len);
   const int per_sm = rows <= 64 && !hidden ? 2 : 1;
   int want = (148 * per_sm) / (Hkv * rblocks);
   if (want < 1) want = 1;
@@ -284,10 +287,8 @@ extern "C" int q40_attn_shared_prefix(const void* q, const void* prefix_k, const
   br.scale_log2 = attn_scale_log2(D);
 
   if (prefix_len > 0) {
-    // lengths are on the device; Lmax is taken for twice their mean up to 256 keys.  A wider table is more likely one that branches can grow
-    // into (64 branches of 64 keys with room for 4096, behind 8192: 71 us if they count as 2048 each, 47), and long rows gain nothing (34
-    // branches of 1000 behind 512: 89.7 and 89.9)
-    const int nsp = prefix_splits(B, H, Hkv, prefix_len, Lmax <= 256 ? (int64_t)B * Lmax / 2 : 0);
+    // (long rows gain nothing from fewer splits: 34 branches of 1000 behind 512 89.7 us and 89.9)
+    const int nsp = prefix_splits(B, H, Hkv, prefix_len, seq_lens && Lmax > 0 ? -1 : Lmax <= 256 ? (int64_t)B * Lmax / 2 : 0);
     const size_t need = (size_t)nsp * rows_total * (D + 2) * sizeof(float);
     if (!workspace || workspace_bytes < need) return Q40_E_WORKSPACE;
     if (!q40_aligned(workspace, 16)) return Q40_E_ALIGN;

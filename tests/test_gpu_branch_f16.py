@@ -105,3 +105,38 @@ def test_infinities(B, Hkv, lead):
     assert (out[..., 3] == -math.inf).all() and (out[..., 100] == math.inf).all()
     out[..., 3] = out[..., 100] = 1
     assert (out == 1).all()
+
+
+@pytest.mark.parametrize("B,H,Hkv", [(1, 32, 32), (4, 32, 32), (5, 32, 32), (7, 32, 32), (9, 32, 32), (12, 32, 32), (16, 32, 32), (20, 32, 32), (23, 32, 32), (27, 32, 32),
+                                     (30, 32, 32), (40, 32, 32), (60, 32, 32), (70, 32, 32), (4, 32, 8), (6, 32, 8), (12, 32, 8), (18, 32, 8), (20, 32, 8), (30, 32, 8),
+                                     (39, 32, 8), (70, 32, 8), (30, 32, 16), (3, 24, 8)])
+def test_bits_do_not_depend_on_what_only_bounds_the_lengths(B, H, Hkv):
+    """With lengths, neither the table's width, nor max_suffix, nor the pool's size changes a bit, behind no prompt and behind ones of one to many splits."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from spec_mcts_b200 import kernels as K
+    page, pages, longest = 16, 3, 48
+    q, k, v, table = _case(B, H, Hkv, longest, page, B)
+    g = torch.Generator(device="cuda").manual_seed(B)
+    lens = torch.randint(0, longest + 1, (B,), generator=g, device="cuda", dtype=torch.int32)
+    P = k.shape[1]
+    k2, v2 = (torch.zeros((Hkv, 40 * P, 128), dtype=torch.float16, device="cuda") for _ in range(2))
+    k2[:, :P], v2[:, :P] = k, v
+    k1, v1 = (t[:, :max(page, int(table[:, :].max()) * page + page)].contiguous() for t in (k, v))
+    tables = []
+    for width in (pages, 8, 9, 16, 17, 40):               # 48, 128, 144, 256, 272 and 640 keys
+        t = torch.zeros((B, width), dtype=torch.int32, device="cuda")
+        t[:, :pages] = table
+        tables.append(t)
+    for plen in (0, 20, 512, 600, 1300):
+        pk, pv = (torch.randn((max(plen, 1), Hkv, 128), generator=g, device="cuda").half() for _ in range(2))
+        want = None
+        for t in tables:
+            for kk, vv in ((k, v), (k2, v2), (k1, v1)):
+                n = t.shape[1] * page
+                if plen:
+                    got = K.shared_prefix_attn(q, pk, pv, plen, t, lens, kk, vv, page_size=page, max_suffix=n)
+                else:
+                    got = K.page_flash_attn(t, q, kk, vv, kk.shape[1], B, n, H, 128, page_size=page, seq_lens=lens)
+                want = got if want is None else want
+                assert torch.equal(got, want), (plen, n, kk.shape[1])
