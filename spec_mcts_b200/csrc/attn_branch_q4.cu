@@ -315,10 +315,13 @@ static int launch_q4(const BranchRotArgs& a, cudaStream_t st) {
 // 40.2, 3200 rows 23.6 / 29.9 / 41.1 / 57.9 (18.8 / 22.9 / 29.4 / 41.9 here).  Keys and values straight to registers instead of through
 // the ring: 20.4 / 25.2 / 33.8 / 47.6; three stages, which leave the prefix pass no room beside: 18.8 / 23.3 / 32.6 / 45.6; five CTAs
 // an SM, with spills: 19.5 / 23.5 / 30.9 / 44.2
+// Scales off four bytes by the same rule (without rotation, 32 heads, 200 own keys behind 40, two warps a row and so: 6 branches 14.3 us and 10.2, 10
+// 14.4 and 11.1; 20 own keys behind 512, 100 branches 19.7 and 16.4)
 int launch_branch_q4(const BranchRotArgs& a, bool rotate, cudaStream_t st) {
   const int w = a.rows <= 3 * 148 ? 4 : a.rows <= 10 * 148 ? 2 : 1;
   if (rotate) return w == 1 ? launch_q4<true, 1, true>(a, st) : w == 2 ? launch_q4<true, 2, true>(a, st) : launch_q4<true, 4, true>(a, st);
-  if (!q40_aligned(a.ksc, 4) || !q40_aligned(a.vsc, 4)) return launch_q4<false, 2, false>(a, st);
+  if (!q40_aligned(a.ksc, 4) || !q40_aligned(a.vsc, 4))
+    return w == 1 ? launch_q4<false, 1, false>(a, st) : w == 2 ? launch_q4<false, 2, false>(a, st) : launch_q4<false, 4, false>(a, st);
   return w == 1 ? launch_q4<false, 1, true>(a, st) : w == 2 ? launch_q4<false, 2, true>(a, st) : launch_q4<false, 4, true>(a, st);
 }
 
