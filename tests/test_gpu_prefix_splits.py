@@ -37,3 +37,26 @@ def test_long_prefixes(B, H, Hkv, prefix):
     """More splits than a merge has on their way at once, up to more than a warp has lanes; a last split that is shorter, or a single key."""
     test_against_64_bits(B, H, Hkv, prefix, 40, 16)
 
+
+def test_two_threads_on_one_stream():
+    """The partial results of a call are merged by that call, whatever another thread enqueues on the same stream."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import threading
+    from spec_mcts_b200 import kernels as K
+    g = torch.Generator(device="cuda").manual_seed(1)
+    normal = lambda *s: torch.randn(s, generator=g, device="cuda").half()
+    calls = [(normal(10, 8, 128), normal(1024, 8, 128), normal(1024, 8, 128), 1024, None, None, None, None) for _ in range(2)]
+    want, out = [K.shared_prefix_attn(*c) for c in calls], [[], []]
+
+    def work(i):
+        for _ in range(500):
+            out[i].append(K.shared_prefix_attn(*calls[i]))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert all(len(o) == 500 and all(torch.equal(y, w) for y in o) for o, w in zip(out, want))
