@@ -188,9 +188,9 @@ static void fill_derived(BranchArgs& a, int B) {
   a.rows = (int64_t)B * a.H;
 }
 
-int launch_branch(BranchArgs a, int mode, int B, int prompt, cudaStream_t st) {
+int launch_branch(BranchArgs a, int mode, int B, cudaStream_t st) {
   fill_derived(a, B);
-  if (int rc; launch_branch_f16(a, mode, prompt, st, rc)) return rc;
+  if (int rc; launch_branch_f16(a, mode, st, rc)) return rc;
   if (mode == 0) return launch_branch_mode<0>(a, st);
   if (mode == 1) return launch_branch_mode<1>(a, st);
   return launch_branch_mode<2>(a, st);
@@ -224,7 +224,7 @@ extern "C" int q40_attn_decode(const void* q, const void* k, const void* v, void
   a.q = (const __half*)q; a.q_stride = (int64_t)H * D; a.k = (const __half*)k; a.v = (const __half*)v; a.o = (__half*)o;
   a.L = L; a.H = H; a.Hkv = Hkv; a.P = 0; a.page_size = 1;
   a.scale_log2 = q40::attn_scale_log2(D);
-  return q40::launch_branch(a, 0, B, 0, (cudaStream_t)stream);
+  return q40::launch_branch(a, 0, B, (cudaStream_t)stream);
 }
 
 extern "C" int q40_attn_paged(const void* page_tbl, int idx_bytes, int64_t tbl_stride,
@@ -245,5 +245,5 @@ extern "C" int q40_attn_paged(const void* page_tbl, int idx_bytes, int64_t tbl_s
   a.tbl = page_tbl; a.tbl_stride = tbl_stride; a.seq_lens = seq_lens;
   a.L = Lmax; a.H = H; a.Hkv = Hkv; a.P = P; a.page_size = page_size;
   a.scale_log2 = q40::attn_scale_log2(D);
-  return q40::launch_branch(a, idx_bytes == 2 ? 1 : 2, B, 0, (cudaStream_t)stream);
+  return q40::launch_branch(a, idx_bytes == 2 ? 1 : 2, B, (cudaStream_t)stream);
 }

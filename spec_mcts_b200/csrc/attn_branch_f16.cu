@@ -197,12 +197,10 @@ struct F16Form { int heads, warps, stages; };
 // 256 and 500, uniform from 0: 3 to 8 % behind the best form of each, in the geometric mean over up to 53 numbers of branches (1 to 100) behind no
 // prompt, 300, 512 and 2048 keys; 32 and 8 kv heads for 32 heads.  Forms by the table's width: 3 to 8 % too, and 5 to 12 % with a pool of 512 keys a branch
 // that counted as length.  Us for lengths up to 16 / 128 / 500: 20 branches 3.7 / 6.2 / 19.0 (four warps a row by scalar products 5.2 / 6.7 / 18.9);
-// 50 branches 4.3 / 13.1 / 35.9 (two warps 6.2 / 13.7 / 33.4).  Many rows behind a long
-// prompt (38 to 64 branches behind 1536 to 4096 keys): two warps take 0.985 to 1.012 times as long over the five lengths together as scalar
-// products, 1.02 to 1.14 times for the shortest, 0.94 to 0.98 times for the longest; behind 1024 keys 0.994 to 1.020, behind 512 more
-static F16Form f16_form_of_rows(int64_t all, int rep, int prompt) {
+// 50 branches 4.3 / 13.1 / 35.9 (two warps 6.2 / 13.7 / 33.4); 64 behind 2048 keys by scalar products 18.2 for up to 16, 38.2 for up to 256 (two
+// warps on matrix instructions 21.1 and 37.1)
+static F16Form f16_form_of_rows(int64_t all, int rep, bool prefix) {
   constexpr int64_t SMS = 148;
-  const bool prefix = prompt > 0;
   const int heads = rep % 4 == 0 && all > (prefix ? 4 : 6) * SMS ? 4 : rep % 2 == 0 && all > SMS ? 2 : 1;
   const int64_t rows = all / heads;
   if (heads > 1 && prefix) return {heads, rows <= 2 * SMS ? 4 : 2, 2};
@@ -210,15 +208,15 @@ static F16Form f16_form_of_rows(int64_t all, int rep, int prompt) {
   if (rows <= (prefix ? 200 : SMS)) return {0, 0, 0};
   if (rows <= 3 * SMS) return {1, 4, rows <= 2 * SMS ? 3 : 2};
   if (rows <= 4 * SMS) return {0, 0, 0};
-  if (rows <= 6 * SMS || (prompt > 1280 && rows > 8 * SMS && rows <= 14 * SMS)) return {1, 2, 2};
+  if (rows <= 6 * SMS) return {1, 2, 2};
   return {rows > (prefix ? 14 : 8) * SMS, 1, 2};
 }
 
-static F16Form f16_form(const BranchArgs& a, int mode, int prompt) {
+static F16Form f16_form(const BranchArgs& a, int mode) {
   constexpr int64_t SMS = 148;
   const bool prefix = a.beside_prefix;
   const int rep = a.H / a.Hkv, L = a.L;
-  if (a.seq_lens) return f16_form_of_rows(a.rows, rep, prompt);
+  if (a.seq_lens) return f16_form_of_rows(a.rows, rep, prefix);
   // As many heads as leave rows for the SMs.  Us by heads (of 4 a kv head) at their best number of warps: paged, 300 keys, 96 rows of one head
   // 5.13 / 5.48 / 6.51 with 1 / 2 / 4, 224 rows 7.2 / 5.49 / 6.57, 384 rows 8.5 / 7.6 / 6.9; 20 keys, 640 rows 3.8 / 3.8 / 4.5 (contiguous 3.5 / 3.4 / 3.8, attn_branch_kernel 3.1); 40 keys behind
   // 400, 640 rows 8.2 / 7.6 / 8.6, 1600 rows 12.7 / 10.9 / 11.2
@@ -270,8 +268,8 @@ static int launch_f16_heads(const BranchArgs& a, const F16Form& f, cudaStream_t 
   return f.heads == 4 ? launch_f16_form<MODE, 4>(a, f, st) : f.heads == 2 ? launch_f16_form<MODE, 2>(a, f, st) : launch_f16_form<MODE, 1>(a, f, st);
 }
 
-bool launch_branch_f16(const BranchArgs& a, int mode, int prompt, cudaStream_t st, int& rc) {
-  const F16Form f = f16_form(a, mode, prompt);
+bool launch_branch_f16(const BranchArgs& a, int mode, cudaStream_t st, int& rc) {
+  const F16Form f = f16_form(a, mode);
   if (f.heads == 0) return false;
   rc = mode == 0 ? launch_f16_heads<0>(a, f, st) : mode == 1 ? launch_f16_heads<1>(a, f, st) : launch_f16_heads<2>(a, f, st);
   return true;
