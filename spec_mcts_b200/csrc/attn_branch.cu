@@ -164,13 +164,13 @@ static int launch_rows(const BranchArgs& a, cudaStream_t st) {
 //     2 / 4 23.2, 4 / 4 30.1, of up to 256 49.7 and 52.1
 //   contiguous, 512 keys: 256 rows 8 / 4 12.6, 4 / 4 14.7; 416 rows 8 / 2 19.3, 4 / 4 19.9; 768 rows 4 / 4 35.9, 2 / 4 36.1; 3200 rows
 //     of 256 4 / 4 63.1, 2 / 4 67.0; of 64: 64 rows 4 / 4 2.6, 8 / 4 3.1; 768 rows 2 / 4 5.1, 4 / 4 5.9
-// (a.L is the length here: rows whose lengths are on the device come by their number alone, see f16_form_of_rows, and not between 4 and 6 SMs')
+// (a.L is the length here.  Rows whose lengths are on the device are split by their number alone, see f16_form_of_rows)
 template <int MODE>
 static int launch_branch_mode(const BranchArgs& a, cudaStream_t st) {
   const int64_t rows = a.rows;
   if constexpr (MODE == 1 || MODE == 2) {
     if (rows <= 2 * 148) return launch_rows<MODE, 8, 8, 4>(a, st);
-    if (rows > 5 * 148 || (rows > 4 * 148 && a.L <= 128)) return launch_rows<MODE, 4, 2, 4>(a, st);
+    if (rows > 5 * 148 || (rows > 4 * 148 && (a.L <= 128 || a.seq_lens))) return launch_rows<MODE, 4, 2, 4>(a, st);
     if (rows > 4 * 148) return launch_rows<MODE, 4, 4, 2>(a, st);
   } else {
     if (a.L > 128 && rows <= 2 * 148) return launch_rows<MODE, 8, 8, 4>(a, st);
@@ -188,9 +188,9 @@ static void fill_derived(BranchArgs& a, int B) {
   a.rows = (int64_t)B * a.H;
 }
 
-int launch_branch(BranchArgs a, int mode, int B, cudaStream_t st) {
+int launch_branch(BranchArgs a, int mode, int B, int prompt, cudaStream_t st) {
   fill_derived(a, B);
-  if (int rc; launch_branch_f16(a, mode, st, rc)) return rc;
+  if (int rc; launch_branch_f16(a, mode, prompt, st, rc)) return rc;
   if (mode == 0) return launch_branch_mode<0>(a, st);
   if (mode == 1) return launch_branch_mode<1>(a, st);
   return launch_branch_mode<2>(a, st);
@@ -224,7 +224,7 @@ extern "C" int q40_attn_decode(const void* q, const void* k, const void* v, void
   a.q = (const __half*)q; a.q_stride = (int64_t)H * D; a.k = (const __half*)k; a.v = (const __half*)v; a.o = (__half*)o;
   a.L = L; a.H = H; a.Hkv = Hkv; a.P = 0; a.page_size = 1;
   a.scale_log2 = q40::attn_scale_log2(D);
-  return q40::launch_branch(a, 0, B, (cudaStream_t)stream);
+  return q40::launch_branch(a, 0, B, 0, (cudaStream_t)stream);
 }
 
 extern "C" int q40_attn_paged(const void* page_tbl, int idx_bytes, int64_t tbl_stride,
@@ -245,5 +245,5 @@ extern "C" int q40_attn_paged(const void* page_tbl, int idx_bytes, int64_t tbl_s
   a.tbl = page_tbl; a.tbl_stride = tbl_stride; a.seq_lens = seq_lens;
   a.L = Lmax; a.H = H; a.Hkv = Hkv; a.P = P; a.page_size = page_size;
   a.scale_log2 = q40::attn_scale_log2(D);
-  return q40::launch_branch(a, idx_bytes == 2 ? 1 : 2, B, (cudaStream_t)stream);
+  return q40::launch_branch(a, idx_bytes == 2 ? 1 : 2, B, 0, (cudaStream_t)stream);
 }

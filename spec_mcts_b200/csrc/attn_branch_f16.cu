@@ -193,30 +193,35 @@ static int launch_f16(const BranchArgs& a, cudaStream_t st) {
 // a time: one CTA of eight warps, two of four with three stages, three of four with two.
 struct F16Form { int heads, warps, stages; };
 // With lengths, which are on the device.  The table's width only bounds them, and the pool may be larger or shared: neither changes the result,
-// so neither may change the form, whose sums have an order of their own.  By rows alone, then, for what loses least over lengths of up to 16, 64, 128,
-// 256 and 500, uniform from 0: 3 to 8 % behind the best form of each, in the geometric mean over up to 53 numbers of branches (1 to 100) behind no
-// prompt, 300, 512 and 2048 keys; 32 and 8 kv heads for 32 heads.  Forms by the table's width: 3 to 8 % too, and 5 to 12 % with a pool of 512 keys a branch
-// that counted as length.  Us for lengths up to 16 / 128 / 500: 20 branches 3.7 / 6.2 / 19.0 (four warps a row by scalar products 5.2 / 6.7 / 18.9);
-// 50 branches 4.3 / 13.1 / 35.9 (two warps 6.2 / 13.7 / 33.4); 64 behind 2048 keys by scalar products 18.2 for up to 16, 38.2 for up to 256 (two
-// warps on matrix instructions 21.1 and 37.1)
-static F16Form f16_form_of_rows(int64_t all, int rep, bool prefix) {
+// so neither may change the form, whose sums have an order of their own.  By rows and prompt alone, then, for what loses least over lengths of up to 16,
+// 64, 128, 256 and 500, uniform from 0, in the geometric mean (below: times as long as attn_branch_kernel, least and most of single lengths):
+//   4 heads a kv head behind 200 keys, 20 / 26 / 33 branches: two heads a row, two warps 0.85 / 0.85 / 0.75 (0.67 to 1.07), four heads, four warps 0.88 /
+//     0.87 / 0.75 (0.51 to 1.26); behind 850, 20 / 26 / 33: two heads, two warps 1.15 / 1.02 / 0.78, four 0.85 / 0.76 / 0.94, four heads, four 0.94 / 0.84 /
+//     0.76.  (A long prompt leaves the branches fewer SMs at a time; two heads of a kv head behind 1024, 20 / 26 branches, two warps 1.19 / 1.03,
+//     four 0.89 / 0.77; behind 100, 26 branches 0.90 and 0.99)
+//   one head, 20 / 24 / 27 branches (four and a bit rows an SM), two warps: behind 200 keys 1.08 / 1.01 / 1.00 (to 1.26), behind 700 0.95 / 0.87 / 0.88
+//   one head and no prompt, one warp a row: 38 / 42 / 44 / 48 branches 1.15 / 1.02 / 0.95 / 0.92
+// Us for lengths up to 16 / 128 / 500: 20 branches 3.4 / 6.5 / 16.7 (four warps a row by scalar products 3.7 / 7.3 / 17.2); 48 branches 4.0 / 10.2 / 34.9
+// (5.8 / 10.0 / 36.4)
+static F16Form f16_form_of_rows(int64_t all, int rep, int prompt) {
   constexpr int64_t SMS = 148;
-  const int heads = rep % 4 == 0 && all > (prefix ? 4 : 6) * SMS ? 4 : rep % 2 == 0 && all > SMS ? 2 : 1;
+  const bool prefix = prompt > 0, far = prompt > 640;
+  const int heads = rep % 4 == 0 && all > (prefix && !far ? 8 : 6) * SMS ? 4 : rep % 2 == 0 && all > SMS ? 2 : 1;
   const int64_t rows = all / heads;
-  if (heads > 1 && prefix) return {heads, rows <= 2 * SMS ? 4 : 2, 2};
+  if (heads > 1 && prefix) return {heads, rows <= (heads == 2 && far ? 3 : 2) * SMS ? 4 : 2, 2};
   if (heads > 1) return {heads, rows <= SMS ? 8 : rows <= 3 * SMS ? 4 : 2, rows > SMS && rows <= 2 * SMS ? 3 : 2};
   if (rows <= (prefix ? 200 : SMS)) return {0, 0, 0};
   if (rows <= 3 * SMS) return {1, 4, rows <= 2 * SMS ? 3 : 2};
   if (rows <= 4 * SMS) return {0, 0, 0};
-  if (rows <= 6 * SMS) return {1, 2, 2};
-  return {rows > (prefix ? 14 : 8) * SMS, 1, 2};
+  if (rows <= 6 * SMS) return {!prefix || far, 2, 2};
+  return {4 * rows > (prefix ? 56 : 37) * SMS, 1, 2};
 }
 
-static F16Form f16_form(const BranchArgs& a, int mode) {
+static F16Form f16_form(const BranchArgs& a, int mode, int prompt) {
   constexpr int64_t SMS = 148;
   const bool prefix = a.beside_prefix;
   const int rep = a.H / a.Hkv, L = a.L;
-  if (a.seq_lens) return f16_form_of_rows(a.rows, rep, prefix);
+  if (a.seq_lens) return f16_form_of_rows(a.rows, rep, prompt);
   // As many heads as leave rows for the SMs.  Us by heads (of 4 a kv head) at their best number of warps: paged, 300 keys, 96 rows of one head
   // 5.13 / 5.48 / 6.51 with 1 / 2 / 4, 224 rows 7.2 / 5.49 / 6.57, 384 rows 8.5 / 7.6 / 6.9; 20 keys, 640 rows 3.8 / 3.8 / 4.5 (contiguous 3.5 / 3.4 / 3.8, attn_branch_kernel 3.1); 40 keys behind
   // 400, 640 rows 8.2 / 7.6 / 8.6, 1600 rows 12.7 / 10.9 / 11.2
@@ -268,8 +273,8 @@ static int launch_f16_heads(const BranchArgs& a, const F16Form& f, cudaStream_t 
   return f.heads == 4 ? launch_f16_form<MODE, 4>(a, f, st) : f.heads == 2 ? launch_f16_form<MODE, 2>(a, f, st) : launch_f16_form<MODE, 1>(a, f, st);
 }
 
-bool launch_branch_f16(const BranchArgs& a, int mode, cudaStream_t st, int& rc) {
-  const F16Form f = f16_form(a, mode);
+bool launch_branch_f16(const BranchArgs& a, int mode, int prompt, cudaStream_t st, int& rc) {
+  const F16Form f = f16_form(a, mode, prompt);
   if (f.heads == 0) return false;
   rc = mode == 0 ? launch_f16_heads<0>(a, f, st) : mode == 1 ? launch_f16_heads<1>(a, f, st) : launch_f16_heads<2>(a, f, st);
   return true;

@@ -158,10 +158,10 @@ struct RowMerge {
 
 // defined in attn_branch_q4.cu; `rotate`: see BranchRotArgs
 int launch_branch_q4(const BranchRotArgs& a, bool rotate, cudaStream_t st);
-// defined in attn_branch.cu; mode 0 contiguous, 1 paged/int16 ids, 2 paged/int32 ids
-int launch_branch(BranchArgs a, int mode, int B, cudaStream_t st);
+// defined in attn_branch.cu; mode 0 contiguous, 1 paged/int16 ids, 2 paged/int32 ids; `prompt`: keys of the prefix pass, 0: none
+int launch_branch(BranchArgs a, int mode, int B, int prompt, cudaStream_t st);
 // defined in attn_branch_f16.cu; false, and nothing launched, where attn_branch_kernel is faster
-bool launch_branch_f16(const BranchArgs& a, int mode, cudaStream_t st, int& rc);
+bool launch_branch_f16(const BranchArgs& a, int mode, int prompt, cudaStream_t st, int& rc);
 int launch_branch_q4(BranchRotArgs a, int B, cudaStream_t st);         // the Q4_0 cache, with rotation where there are tables
 
 }  // namespace q40

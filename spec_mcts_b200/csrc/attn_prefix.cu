@@ -308,7 +308,7 @@ extern "C" int q40_attn_shared_prefix(const void* q, const void* prefix_k, const
   // Lmax == 0: the branch kernel only merges the prefix partials
   const int mode = (Lmax == 0) ? 0 : (idx_bytes == 2 ? 1 : 2);
   if (Lmax == 0) { br.seq_lens = nullptr; br.L = 0; }
-  return launch_branch(br, mode, B, st);
+  return launch_branch(br, mode, B, prefix_len, st);
 }
 
 // cos_tbl != NULL: q and cur_k are rotated and the token is appended (q40_attn_tree_step)
