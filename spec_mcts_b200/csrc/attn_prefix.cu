@@ -192,22 +192,24 @@ static int prefix_splits(int B, int H, int Hkv, int prefix_len, int64_t own) {
   // rows), one for the 128-row variant; never round up past whole waves (a 149th CTA doubles the time
   // of one SM)
   // ... one, too, where the branches' own keys are so many that the pass is over long before they are: it then gets by with half of the
-  // partials and leaves SMs to them (64 branches of up to 256 own keys behind 512: 34.6 us with two, 31.4; 34 behind 471 22.2 and 21.4; at four
-  // times the prefix no difference, below it one is slower: 10 behind 2048 16.6 and 18.5; and with fewer than eight tiles: 64 branches
-  // of up to 100 behind 300 17.9 and 18.7)
+  // partials and leaves SMs to them (64 branches of 256 own keys behind 512: 52.0 us with two, 47.6; of up to 256 35.0 and 32.0, 34 behind 471 18.5
+  // and 17.6; below some times the prefix one is slower: 10 of up to 64 behind 2048 9.1 and 11.1; and with fewer than eight tiles: 64
+  // of up to 100 behind 300 15.1 and 15.8)
   // With lengths on the device neither the table's width nor anything else that they leave open may decide (splits have their own order of
   // sums): one up to ten tiles, which 64, 34 and 10 branches of up to 16 / 64 / 128 / 256 / 500 keys behind 512 take 0.87 to 1.04 times as long with as
-  // with two, behind 700 0.92 to 1.08, behind 1024 0.87 to 1.18, behind 2048 0.94 to 1.39; 8 kv heads no difference
+  // with two, behind 700 0.92 to 1.08, behind 1024 0.87 to 1.18, behind 2048 0.94 to 1.39; 8 kv heads no difference (53 of up to 39 behind 499
+  // 13.3 with one and 12.1, the most that is lost)
   const bool hidden = tiles >= 8 && (own < 0 ? tiles <= 10 : own > 6 * (int64_t)prefix_len);
   const int per_sm = rows <= 64 && !hidden ? 2 : 1;
   int want = (148 * per_sm) / (Hkv * rblocks);
   if (want < 1) want = 1;
   if (want > tiles) want = tiles;
-  // How many tiles a split has.  A tile costs it 1.0 us (1.9 with eight warps); the merge has 16 splits of a row on their way at once (8 where a row has two
+  // How many tiles a split has.  A tile costs it 1.0 us (1.9 with eight warps, 0.8 where two warps share a row's keys, 0.56 where four do); the merge has 16 splits of a row on their way at once (8 where a row has two
   // warps) and reads further ones one by one, 0.07 us each, more behind many own keys; a second CTA on an SM costs 2.3 us that matter less the longer splits are.  Us by splits, 8 query heads a kv head:
-  // 1 kv head, 1 branch, 2048 keys 16 splits 6.1, 32 7.3; 8192 keys 16 12.4, 32 10.4, 128 14.1; 32768 keys 16 37.3, 64 16.8, 256 24.9; 8 kv heads
-  // x 4, 4 branches, 2048 keys 16 7.7, 32 10.6; 32768 keys 16 44.1, 32 30.5.  Over 448 sizes of 1 to 32 kv heads and 512 to 32768 keys 5 % less
-  // time than with as many splits as SMs take, four of them 3 to 9 % more (1 kv head x 4, 34 branches, 8192 keys 15.9 and 17.3)
+  // 1 kv head, 1 branch, 2048 keys 16 splits 4.5, 32 6.5; 8192 keys 16 8.0, 32 8.1, 128 12.8; 32768 keys 16 21.4, 64 12.6, 256 24.4; 8 kv heads
+  // x 4, 4 branches, 2048 keys 16 6.2, 32 8.7; 32768 keys 16 31.6, 32 27.9.  Before warps shared tiles, over 448 sizes of 1 to 32 kv heads and 512 to
+  // 32768 keys, 5 % less time than with as many splits as SMs take, four of them 3 to 9 % more (1 kv head x 4, 34 branches, 8192 keys 15.9 and
+  // 17.3).  The line is that of tiles that no warps share: up to 16 rows it has more splits than are best from 8192 keys on (1 kv head, 8192 keys 43, 9.4)
   int best = tiles, least = INT_MAX;
   for (int per = (tiles + want - 1) / want;; ++per) {
     const int n = (tiles + per - 1) / per;                  // every split is non-empty

@@ -35,6 +35,8 @@
 // x 4096 x 4096 8.2 and 6.9, three of them 13.3 and 12.3, x 11008 x 4096 13.3 and 12.0; 102 rows 9.9 and 9.2, 17.3 and 15.6, 15.8 and 15.4. With the
 // SiLU product: 10 rows x 4096 x 11008 17.7 and 16.2, 64 rows 24.3 and 21.2, 100 rows 31.4 and 25.6, 512 rows 94.5 and 82.5 (eight quotients in flight
 // at once: see silu). 512 rows without it, whose k blocks wait for L2: 49.6 and 48.3 x 11008, 45.4 and 44.9 x 11008 x 4096.
+// With pauses, off the power limit: 144 rows x 4096 x 11008 21.9 and 17.0, 256 rows 25.9 and 24.3, 400 and 512 rows with the SiLU product 73.4 and 61.3, 73.9
+// and 70.2; 300 and 400 rows x 11008 x 4096 31.6 and 30.4, 34.2 and 34.3.
 //
 // Every wait is bounded (by seconds): on expiry an error word is set and no more copies are requested; what is still
 // multiplied and stored is undefined, as is the scratch.  Copies and MMAs in flight are waited for, tensor memory is freed.
@@ -67,7 +69,7 @@ constexpr int BAR_BYTES = (EARLY ? 24 : 16) * S_MAX + 8 * NA_MAX + 64;
 constexpr uint32_t FLAG_POLLS = 1u << 22;       // of one flag, before giving up: seconds, like the other waits
 constexpr int OUT_LD = FEATS + 8;              // halves between rows that wait in shared memory
 constexpr int MAX_PAIRS = 128;
-constexpr int FLAG_BYTES = MAX_PAIRS * 64;      // at the start of the scratch, per pair: [half][quadrant] arrivals, then departures
+constexpr int FLAG_BYTES = MAX_PAIRS * 64;      // at the start of the scratch, per pair: [half][quadrant] arrivals, and as many words without use
 
 // Tensor maps: the activations, and per matrix the weights (box 1024 bytes x 8 steps, half of it with SiLU) and scales (64 bytes x
 // 8 steps, or half) of a tiled copy read as rows of one step
@@ -757,6 +759,8 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
             *xchg(feat ^ 64) = x.v;
             asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
             x.v = *xchg(feat);
+            // (Also where all eight are padding.  With a branch around these the whole takes longer: 8 rows x 4096 x 11008 15.5 and 15.9 us, 64
+            // 17.6 and 19.2, 100 23.1 and 24.0)
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const float2 f = __half22float2(hi ? x.h[j] : mine.h[j]);
