@@ -67,6 +67,9 @@ constexpr int GROUPS = 1 + DSETS;               // of four warps, one per tensor
 template <bool EARLY>
 constexpr int BAR_BYTES = (EARLY ? 24 : 16) * S_MAX + 8 * NA_MAX + 64;
 constexpr uint32_t FLAG_POLLS = 1u << 22;       // of one flag, before giving up: seconds, like the other waits
+// Of the other waits: 10 s.  Roles that are there early wait for what the launch in front leaves, which may take the 4 s in which its flags run out; with less
+// than that theirs would run out too.  (griddepcontrol.wait ahead of the first of them, by each role: three matrices of 10 rows x 4096 x 4096 11.9 us, 12.3)
+constexpr uint32_t WAIT_POLLS = 4 * SPIN_LIMIT;
 constexpr int OUT_LD = FEATS + 8;              // halves between rows that wait in shared memory
 constexpr int MAX_PAIRS = 128;
 constexpr int FLAG_BYTES = MAX_PAIRS * 64;      // at the start of the scratch, per pair: [half][quadrant] arrivals, and as many words without use
@@ -326,7 +329,7 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
     while (pi < p.nprob - 1 && span >= p.spans[pi]) { span -= p.spans[pi]; ++pi; }
   };
   bool failed = false;
-  uint32_t limit = SPIN_LIMIT;                               // see wait_limited
+  uint32_t limit = WAIT_POLLS;                               // see wait_limited
 
   // ---- copies of blocks first .. last - 1 of the pair, weights or activations.  `first`: 0, or S where the first S have been requested:
   // weights do not depend on the previous launch, so their first stages are, before anything else ----
@@ -803,6 +806,7 @@ gemm_pair_kernel(const Params p, const __grid_constant__ Maps maps) {
   if (failed && tid == 0) {
     // the copies still on their way, those of the last S blocks at most: none may land in shared memory that has been given back
     q40_set_error(p.err);
+    mbar_wait(bar_done, 0);                                  // MMAs, too: a wait that is over asked for them only once
     if constexpr (EARLY) {
       for (int h = 0; h < 2; ++h)
         for (int n = h && NK && p.x ? min(s_copied[1], s_copied[3]) : s_copied[h], i = max(0, n - S); i < n; ++i)

@@ -117,6 +117,8 @@ gemm_tiled_wide_kernel(const Params p, const __grid_constant__ CUtensorMap amap)
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
   asm volatile("griddepcontrol.launch_dependents;");
+  // the time that the launch in front takes, whose waits may run out, is not that of this one's waits
+  if (warp != 0) asm volatile("griddepcontrol.wait;" ::: "memory");
 
   bool failed = false;
   if (warp == 0) {

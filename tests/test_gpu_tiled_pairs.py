@@ -235,3 +235,33 @@ def test_largest_tiles_with_sums_of_ranges(K, M):
     again = [torch.empty_like(o) for o in outs]
     launch(a, tiled, again, Ns, 0, ws, 1)
     assert all(torch.equal(x, y) for x, y in zip(outs, again))
+
+
+@pytest.mark.parametrize("M,n,silu", [(16, 5120, 1), (100, 4096, 0), (300, 4096, 0)])     # shared tiles; one tile a pair; ranges and chunks of rows
+def test_a_launch_behind_one_that_waits_for_seconds(K, M, n, silu):
+    """A dependent launch is there early.  It does not count the time that the launch in front takes (here one whose wait runs out) as its own."""
+    from spec_mcts_b200._lib import check, lib
+    rng = np.random.default_rng(M)
+    m, Kd, n0 = 16, 8064, 5120
+    _, front = mats(K, rng, Kd, (n0, n0))
+    _, tiled = mats(K, rng, Kd, (n,) * (1 + silu))
+    x, a = (torch.from_numpy(rng.standard_normal((r, Kd)).astype(np.float16)).cuda() for r in (m, M))
+    ws0, ws = scratch(K, m), scratch(K, M)
+    want, got = (torch.empty((M, n), dtype=torch.float16, device="cuda") for _ in range(2))
+    launch(a, tiled, [want] * (1 + silu), (n,) * (1 + silu), silu, ws)
+    g = torch.empty((m, n0), dtype=torch.float16, device="cuda")
+    err = torch.zeros(2, dtype=torch.int32).pin_memory()
+    ws0[:8192].view(torch.int32)[:8] = -1000
+    torch.cuda.synchronize()
+
+    def one(mats_, x_, out, N, s, w, e):
+        k = len(mats_)
+        P = ctypes.c_void_p * k
+        check(lib.q40_gemm_tiled_tc_ws(k, x_.data_ptr(), x_.stride(0), P(*[t.data_ptr() for t in mats_]), P(*[out.data_ptr()] * k), (ctypes.c_int64 * k)(*[N] * k),
+                                       (ctypes.c_int * k)(*[N] * k), x_.shape[0], Kd, s, w.data_ptr() if w.numel() else None, w.numel(), e.data_ptr(), 1,
+                                       torch.cuda.current_stream().cuda_stream), "q40_gemm_tiled_tc_ws")
+
+    one(front, x, g, n0, 1, ws0, err[:1])
+    one(tiled, a, got, n, silu, ws, err[1:])
+    torch.cuda.synchronize()
+    assert err.tolist() == [1, 0] and torch.equal(got, want)
