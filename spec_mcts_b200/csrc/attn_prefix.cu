@@ -16,6 +16,7 @@
 // small next to it.  What bounds it: a warp's chain of MMAs and softmax per tile (2.1 us, a quarter where four warps share it; see
 // attn_tile.cuh), start, first tile and partials around it.
 #include <climits>
+#include <mutex>
 
 #include "attn_tile.cuh"
 
@@ -288,7 +289,12 @@ extern "C" int q40_attn_shared_prefix(const void* q, const void* prefix_k, const
   br.L = Lmax; br.H = H; br.Hkv = Hkv; br.P = P; br.page_size = page_size;
   br.scale_log2 = attn_scale_log2(D);
 
+  // The first of two launches leaves the other its partial results in the scratch.  Callers that share one, as threads on one stream may, enqueue both before
+  // the next does (a lock from Python costs 0.3 us of a call)
+  static std::mutex turns[64];
+  std::unique_lock<std::mutex> turn;
   if (prefix_len > 0) {
+    turn = std::unique_lock<std::mutex>(turns[(uintptr_t)workspace / 512 % 64]);
     // (long rows gain nothing from fewer splits: 34 branches of 1000 behind 512 89.7 us and 89.9)
     const int nsp = prefix_splits(B, H, Hkv, prefix_len, seq_lens && Lmax > 0 ? -1 : Lmax <= 256 ? (int64_t)B * Lmax / 2 : 0);
     const size_t need = (size_t)nsp * rows_total * (D + 2) * sizeof(float);

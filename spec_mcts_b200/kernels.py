@@ -10,7 +10,6 @@ from __future__ import annotations
 
 import ctypes
 import math
-import threading
 import weakref
 from typing import Optional, Sequence
 
@@ -84,7 +83,6 @@ _workspaces: dict = {}
 _outgrown: list = []                # ... whose place a larger one has taken, and whose address a graph may have
 _SMALL_WORKSPACE = 64 << 20
 _large_in_graphs: set = set()       # keys of larger ones that a capture has used
-_attn_locks: dict = {}              # (device, stream) -> see shared_prefix_attn
 _capture_workspaces: dict = {}      # the same keys -> (id of the stream's last capture, buffer made in it)
 
 
@@ -773,14 +771,11 @@ def shared_prefix_attn(q, prefix_k, prefix_v, prefix_len, p, seq_lens, kpool, vp
         idx_bytes, P, Lmax, tbl_stride = 4, 0, 0, 0
     o = torch.empty((B, H, D), device=dev, dtype=torch.float16)
     nbytes = lib.q40_attn_shared_prefix_workspace_bytes(B, H, D, max(prefix_len, 1))
-    st = _stream(dev)
-    # two launches, of which one leaves the other partial results in the scratch: those of two threads on a stream must not alternate
-    with _attn_locks.setdefault((dev.index, st), threading.Lock()):
-        ws = _workspace("attn", dev, nbytes, zero=False)
-        check(lib.q40_attn_shared_prefix(q.data_ptr(), _ptr(prefix_k), _ptr(prefix_v), prefix_len, ks, hs,
-                                         _ptr(p), idx_bytes, tbl_stride, _ptr(seq_lens), _ptr(kpool),
-                                         _ptr(vpool), o.data_ptr(), P, B, Lmax, H, Hkv, D, page_size,
-                                         ws.data_ptr(), ws.numel(), st), "q40_attn_shared_prefix")
+    ws = _workspace("attn", dev, nbytes, zero=False)
+    check(lib.q40_attn_shared_prefix(q.data_ptr(), _ptr(prefix_k), _ptr(prefix_v), prefix_len, ks, hs,
+                                     _ptr(p), idx_bytes, tbl_stride, _ptr(seq_lens), _ptr(kpool),
+                                     _ptr(vpool), o.data_ptr(), P, B, Lmax, H, Hkv, D, page_size,
+                                     ws.data_ptr(), ws.numel(), _stream(dev)), "q40_attn_shared_prefix")
     return o
 
 
