@@ -183,7 +183,7 @@ attn_prefix_kernel(const PrefixArgs a) {
   }
 }
 
-// `own`: keys that the branches have of their own in front of a head, about; 0: not known, -1: their lengths are on the device
+// `own`: keys that the branches have of their own in front of a head, about; 0: not known
 static int prefix_splits(int B, int H, int Hkv, int prefix_len, int64_t own) {
   const int rep = H / Hkv;
   const int rows = B * rep;
@@ -196,11 +196,7 @@ static int prefix_splits(int B, int H, int Hkv, int prefix_len, int64_t own) {
   // partials and leaves SMs to them (64 branches of 256 own keys behind 512: 52.0 us with two, 47.6; of up to 256 35.0 and 32.0, 34 behind 471 18.5
   // and 17.6; below some times the prefix one is slower: 10 of up to 64 behind 2048 9.1 and 11.1; and with fewer than eight tiles: 64
   // of up to 100 behind 300 15.1 and 15.8)
-  // With lengths on the device neither the table's width nor anything else that they leave open may decide (splits have their own order of
-  // sums): one up to ten tiles, which 64, 34 and 10 branches of up to 16 / 64 / 128 / 256 / 500 keys behind 512 take 0.87 to 1.04 times as long with as
-  // with two, behind 700 0.92 to 1.08, behind 1024 0.87 to 1.18, behind 2048 0.94 to 1.39; 8 kv heads no difference (53 of up to 39 behind 499
-  // 13.3 with one and 12.1, the most that is lost)
-  const bool hidden = tiles >= 8 && (own < 0 ? tiles <= 10 : own > 6 * (int64_t)prefix_len);
+  const bool hidden = tiles >= 8 && own > 6 * (int64_t)prefix_len;
   const int per_sm = rows <= 64 && !hidden ? 2 : 1;
   int want = (148 * per_sm) / (Hkv * rblocks);
   if (want < 1) want = 1;
@@ -295,8 +291,10 @@ extern "C" int q40_attn_shared_prefix(const void* q, const void* prefix_k, const
   std::unique_lock<std::mutex> turn;
   if (prefix_len > 0) {
     turn = std::unique_lock<std::mutex>(turns[(uintptr_t)workspace / 512 % 64]);
-    // (long rows gain nothing from fewer splits: 34 branches of 1000 behind 512 89.7 us and 89.9)
-    const int nsp = prefix_splits(B, H, Hkv, prefix_len, seq_lens && Lmax > 0 ? -1 : Lmax <= 256 ? (int64_t)B * Lmax / 2 : 0);
+    // lengths are on the device; Lmax is taken for twice their mean up to 256 keys.  A wider table is more likely one that branches can grow
+    // into (64 branches of 64 keys with room for 4096, behind 8192: 71 us if they count as 2048 each, 47), and long rows gain nothing (34
+    // branches of 1000 behind 512: 89.7 and 89.9).  (So Lmax may move a result's last bits, by another number of splits, behind 449 keys and more)
+    const int nsp = prefix_splits(B, H, Hkv, prefix_len, Lmax <= 256 ? (int64_t)B * Lmax / 2 : 0);
     const size_t need = (size_t)nsp * rows_total * (D + 2) * sizeof(float);
     if (!workspace || workspace_bytes < need) return Q40_E_WORKSPACE;
     if (!q40_aligned(workspace, 16)) return Q40_E_ALIGN;

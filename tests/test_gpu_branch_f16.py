@@ -111,7 +111,8 @@ def test_infinities(B, Hkv, lead):
                                      (30, 32, 32), (40, 32, 32), (60, 32, 32), (70, 32, 32), (4, 32, 8), (6, 32, 8), (12, 32, 8), (18, 32, 8), (20, 32, 8), (30, 32, 8),
                                      (39, 32, 8), (70, 32, 8), (30, 32, 16), (3, 24, 8)])
 def test_bits_do_not_depend_on_what_only_bounds_the_lengths(B, H, Hkv):
-    """With lengths, neither the table's width, nor max_suffix, nor the pool's size changes a bit, behind no prompt and behind ones of one to many splits."""
+    """With lengths, neither the table's width, nor max_suffix, nor the pool's size changes a bit; but behind a prompt of eight tiles and more
+    max_suffix says how many splits it has."""
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     from spec_mcts_b200 import kernels as K
@@ -128,10 +129,10 @@ def test_bits_do_not_depend_on_what_only_bounds_the_lengths(B, H, Hkv):
         t = torch.zeros((B, width), dtype=torch.int32, device="cuda")
         t[:, :pages] = table
         tables.append(t)
-    for plen in (0, 20, 512, 600, 1300):
+    for plen in (0, 20, 400, 512, 1300):
         pk, pv = (torch.randn((max(plen, 1), Hkv, 128), generator=g, device="cuda").half() for _ in range(2))
         want = None
-        for t in tables:
+        for t in tables if plen < 449 else tables[-1:]:
             for kk, vv in ((k, v), (k2, v2), (k1, v1)):
                 n = t.shape[1] * page
                 if plen:
