@@ -197,8 +197,8 @@ struct F16Form { int heads, warps, stages; };
 // 64, 128, 256 and 500, uniform from 0, in the geometric mean (below: times as long as attn_branch_kernel, least and most of single lengths):
 //   4 heads a kv head behind 200 keys, 20 / 26 / 33 branches: two heads a row, two warps 0.85 / 0.85 / 0.75 (0.67 to 1.07), four heads, four warps 0.88 /
 //     0.87 / 0.75 (0.51 to 1.26); behind 850, 20 / 26 / 33: two heads, two warps 1.15 / 1.02 / 0.78, four 0.85 / 0.76 / 0.94, four heads, four 0.94 / 0.84 /
-//     0.76.  (A long prompt leaves the branches fewer SMs at a time; two heads of a kv head behind 1024, 20 / 26 branches, two warps 1.19 / 1.03,
-//     four 0.89 / 0.77; behind 100, 26 branches 0.90 and 0.99)
+//     0.76, two 1.23 / 1.11 / 0.84; 36 branches four 0.83, two 0.83, behind 2048 0.86 and 0.84.  (A long prompt leaves the branches fewer SMs at a
+//     time; two heads a kv head behind 1024, 20 / 26 branches, two warps 1.19 / 1.03, four 0.89 / 0.77; behind 100, 26 branches 0.90 and 0.99)
 //   one head, 20 / 24 / 27 branches (four and a bit rows an SM), two warps: behind 200 keys 1.08 / 1.01 / 1.00 (to 1.26), behind 700 0.95 / 0.87 / 0.88
 //   one head and no prompt, one warp a row: 38 / 42 / 44 / 48 branches 1.15 / 1.02 / 0.95 / 0.92
 // Us for lengths up to 16 / 128 / 500: 20 branches 3.4 / 6.5 / 16.7 (four warps a row by scalar products 3.7 / 7.3 / 17.2); 48 branches 4.0 / 10.2 / 34.9
@@ -208,7 +208,8 @@ static F16Form f16_form_of_rows(int64_t all, int rep, int prompt) {
   const bool prefix = prompt > 0, far = prompt > 640;
   const int heads = rep % 4 == 0 && all > (prefix && !far ? 8 : 6) * SMS ? 4 : rep % 2 == 0 && all > SMS ? 2 : 1;
   const int64_t rows = all / heads;
-  if (heads > 1 && prefix) return {heads, rows <= (heads == 2 && far ? 3 : 2) * SMS ? 4 : 2, 2};
+  if (heads == 4 && prefix) return {4, 4 * all <= 29 * SMS ? 4 : 2, 2};
+  if (heads > 1 && prefix) return {heads, rows <= (far ? 3 : 2) * SMS ? 4 : 2, 2};
   if (heads > 1) return {heads, rows <= SMS ? 8 : rows <= 3 * SMS ? 4 : 2, rows > SMS && rows <= 2 * SMS ? 3 : 2};
   if (rows <= (prefix ? 200 : SMS)) return {0, 0, 0};
   if (rows <= 3 * SMS) return {1, 4, rows <= 2 * SMS ? 3 : 2};
